@@ -289,6 +289,11 @@ int pb200_facet2facet_backward_padded(int64_t Nf, int64_t NiK, int Cin, int Cout
  * torch_sph_harm_reorder (picasso/math_utils.py:10-62).  xyz (N,3) contiguous. */
 int pb200_sph_harm_coeff(int64_t N, int L, const float* xyz, float* out, void* stream);
 
+/* filter (3,C) = corners (3,K) @ weights (K,C): the vertex2facet filter of a layer from its spherical-harmonic
+ * coefficients (picasso/mesh/layers.py:110-112), and gradWeights (K,C) = corners^T @ gradFilter. */
+int pb200_corner_filter(int K, int C, const float* corners, const float* weights, float* filter, void* stream);
+int pb200_corner_filter_backward(int K, int C, const float* corners, const float* gradFilter, float* gradWeights, void* stream);
+
 /* geometry[f] = [unit normal (3), plane intercept d, area].  Replaces
  * compute_triangle_geometry_ (picasso/mesh/pi_modules/decimate.py:70-85).  `vertex` has
  * `vstride` floats per row, of which the first three are xyz. */

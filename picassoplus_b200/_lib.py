@@ -24,6 +24,13 @@ if not os.path.exists(LIB_PATH):
 
 _lib = C.CDLL(LIB_PATH)
 
+try:
+    import torch as _torch  # noqa: F401  (the extension links against the libraries torch has loaded)
+    from . import _torch_ops as ops  # noqa: F401  the native host path: checks, allocation, launches, autograd nodes
+except ImportError as e:
+    raise ImportError(f"picassoplus_b200._torch_ops is missing or does not load ({e}): build it with "
+                      "`python -m picassoplus_b200.build`") from e
+
 i64, i32, vp, sz, f32 = C.c_int64, C.c_int, C.c_void_p, C.c_size_t, C.c_float
 
 
@@ -96,6 +103,8 @@ SIGNATURES = {
     "pb200_rows_contract_workspace_bytes": (sz, [i64, i32, i32]),
     "pb200_rows_contract": (i32, [i64, i32, i32, vp, vp, vp, vp, i32, vp, sz, vp]),
     "pb200_sph_harm_coeff": (i32, [i64, i32, vp, vp, vp]),
+    "pb200_corner_filter": (i32, [i32, i32, vp, vp, vp, vp]),
+    "pb200_corner_filter_backward": (i32, [i32, i32, vp, vp, vp, vp]),
     "pb200_triangle_geometry": (i32, [i64, i64, i32, vp, vp, vp, vp]),
     "pb200_expand_rows_forward": (i32, [i64, i64, i32, vp, vp, vp, vp]),
     "pb200_expand_rows_backward": (i32, [i64, i64, i32, vp, vp, vp, vp]),

@@ -18,7 +18,7 @@ import torch
 
 from . import _lib
 from .mesh.pi_modules import conv3d
-from .topology import FaceMeans, face_means, ptr, stream_ptr
+from .topology import FaceMeans, face_means, ptr, stream_ptr, vertex_csr
 
 
 class _ExpandRows(torch.autograd.Function):
@@ -90,36 +90,27 @@ def one_sample_forward(face_rows, filter, weights, weights_padded=None):
     return out
 
 
-class _SharedRowsF2F(torch.autograd.Function):
-    """facet2facet over one row per face shared by the face's samples: forward through the one-sample entry,
-    backward through the general operator's backward over (rows, per-face mean weights, one sample per face)."""
-
-    @staticmethod
-    def forward(ctx, face_rows, filter, weights, one_each, weights_padded):
-        face_rows, filter = face_rows.contiguous(), filter.contiguous()
-        ctx.save_for_backward(face_rows, filter, weights, one_each)
-        ctx.weights_padded = weights_padded
-        return one_sample_forward(face_rows, filter, weights, weights_padded)
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        face_rows, filter, weights, one_each = ctx.saved_tensors
-        gin, gf = conv3d.facet2facet_backward(grad_output.contiguous(), face_rows, filter, weights, one_each,
-                                              baryPadded=ctx.weights_padded)
-        return gin, gf, None, None, None
-
-
 def facet2facet_shared_rows(face_rows, filter, bary_sh, cum):
     """facet2facet(repeat_interleave(face_rows, samples per face), filter, bary_sh, cum) without the expanded rows.
     bary_sh: the (NiK, F) sample weights, or their per-face means as topology.face_means / face_means_sph_harm
     return them (then cum is not looked at)."""
     fm = bary_sh if isinstance(bary_sh, FaceMeans) else face_means(bary_sh, cum)
-    return _SharedRowsF2F.apply(face_rows, filter, fm.rows, fm.one_each, fm.rows_padded)
+    return _lib.ops.facet2facet_shared_rows(face_rows, filter, fm.rows, fm.one_each, fm.rows_padded, conv3d._f2f_precision)
 
 
 def conv_block(x, Wv, Wf, Wo, face, cum, bary_sh, coeff, nf_count, vt_map, sh_eye):
-    cin = x.shape[1]
-    spatial = (sh_eye @ Wv).reshape(3, cin, 1)
-    y = conv3d.vertex2facet(x, spatial, face)
-    z = facet2facet_shared_rows(y, Wf, bary_sh, cum)
-    return conv3d.facet2vertex(z, Wo, coeff, face, nf_count, vt_map)
+    """One native autograd node for the three operators: forward and backward run without the interpreter."""
+    if sh_eye.requires_grad:                      # its gradient comes from the product with Wv: operator by operator
+        y = conv3d.vertex2facet(x, (sh_eye @ Wv).reshape(3, x.shape[1], 1), face)
+        z = facet2facet_shared_rows(y, Wf, bary_sh, cum)
+        return conv3d.facet2vertex(z, Wo, coeff, face, nf_count, vt_map)
+    conv3d._check(face, "face", 2, torch.int32)
+    conv3d._check(vt_map, "vt_map", 1, torch.int32)
+    fm = bary_sh if isinstance(bary_sh, FaceMeans) else face_means(bary_sh, cum)
+    v_rowptr = v_entries = None
+    if torch.is_grad_enabled():
+        pull = vertex_csr(face, None, x.shape[0], x.shape[0])
+        v_rowptr, v_entries = pull.rowptr, pull.entries
+    push = vertex_csr(face, vt_map, vt_map.shape[0], nf_count.shape[0])
+    return _lib.ops.conv_block(x, Wv, Wf, Wo, sh_eye, face, fm.rows, fm.one_each, fm.rows_padded, coeff, nf_count, vt_map,
+                               v_rowptr, v_entries, push.rowptr, push.entries, conv3d._f2f_precision)

@@ -1,10 +1,11 @@
-"""Builds libpicasso_b200.so from csrc/*.cu with nvcc for sm_100a, in-tree.
+"""Builds libpicasso_b200.so from csrc/*.cu with nvcc for sm_100a, and the torch extension _torch_ops.so (the native
+host path over the library's C ABI) from csrc/torch_ops.cpp with g++, in-tree.
 
     python -m picassoplus_b200.build [--force] [--verbose]
 
 Objects are rebuilt only when their source (or a header) is newer.  The library links the
 CUDA runtime statically, exports the C ABI declared in include/picasso_b200.h, and
-has no dependency on torch.
+has no dependency on torch; the extension links the library and torch.
 """
 from __future__ import annotations
 
@@ -18,6 +19,7 @@ ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(CSRC, "_obj")
 LIB = os.path.join(PKG, "libpicasso_b200.so")
+OPS = os.path.join(PKG, "_torch_ops.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -48,6 +50,21 @@ def _headers_mtime() -> float:
     return max(os.path.getmtime(h) for h in hs)
 
 
+def _ops_command(out: str):
+    """g++ command of the torch extension: torch's own headers, libraries and C++ ABI."""
+    import sysconfig
+    import torch
+    t = os.path.join(os.path.dirname(torch.__file__))
+    inc, lib = os.path.join(t, "include"), os.path.join(t, "lib")
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    return (["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_torch_ops",
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] +
+            [a for d in (inc, os.path.join(inc, "torch", "csrc", "api", "include"), os.path.join(cuda, "include"),
+                         sysconfig.get_paths()["include"]) for a in ("-isystem", d)] +
+            [os.path.join(CSRC, "torch_ops.cpp"), "-o", out, "-L" + PKG, "-l:libpicasso_b200.so", "-L" + lib, "-lc10", "-lc10_cuda",
+             "-ltorch_cpu", "-ltorch", "-ltorch_python", "-Wl,-rpath,$ORIGIN:" + lib])
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OBJ, exist_ok=True)
     nvcc = _nvcc()
@@ -66,13 +83,16 @@ def build(force: bool = False, verbose: bool = False) -> str:
         r = subprocess.run(cmd, capture_output=True, text=True)
         return cmd, r
 
+    def check(cmd, r):
+        if verbose or r.returncode != 0:
+            sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+        if r.returncode != 0:
+            raise RuntimeError("build step failed: " + " ".join(cmd[-3:]))
+
     if jobs:
         with ThreadPoolExecutor(max_workers=min(8, len(jobs))) as ex:
             for cmd, r in ex.map(run, jobs):
-                if verbose or r.returncode != 0:
-                    sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
-                if r.returncode != 0:
-                    raise RuntimeError("nvcc failed for " + cmd[-3])
+                check(cmd, r)
     if jobs or not os.path.exists(LIB):
         cmd = [nvcc, "-shared", "-o", LIB] + objs + ["-cudart", "static",
                "-gencode", "arch=compute_100a,code=sm_100a"]
@@ -80,6 +100,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    ops_src = os.path.join(CSRC, "torch_ops.cpp")
+    if force or not os.path.exists(OPS) or os.path.getmtime(OPS) < max(os.path.getmtime(ops_src), hm):
+        check(*run(_ops_command(OPS)))
     return LIB
 
 

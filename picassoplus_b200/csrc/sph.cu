@@ -66,9 +66,50 @@ face_mean_sph_harm_kernel(int64_t Nf, int64_t NiK, int L, const float* __restric
     }
 }
 
+// The three-row vertex2facet filter of a layer, corners (3,K) @ weights (K,C), and its gradient corners^T @ gradFilter:
+// K <= 36 terms, a few thousand results.  Both are one short launch; as library GEMMs they were two of the step's
+// larger host costs.
+__global__ void corner_filter_kernel(int K, int C, const float* __restrict__ corners, const float* __restrict__ weights,
+                                     float* __restrict__ filter) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= 3 * C) return;
+    const int j = i / C, c = i - j * C;
+    float acc = 0.f;
+    for (int k = 0; k < K; ++k) acc = fmaf(__ldg(corners + j * K + k), __ldg(weights + (int64_t)k * C + c), acc);
+    filter[i] = acc;
+}
+
+__global__ void corner_filter_bwd_kernel(int K, int C, const float* __restrict__ corners, const float* __restrict__ gfilter,
+                                         float* __restrict__ gweights) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= K * C) return;
+    const int k = i / C, c = i - k * C;
+    float acc = 0.f;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) acc = fmaf(__ldg(corners + j * K + k), __ldg(gfilter + j * C + c), acc);
+    gweights[i] = acc;
+}
+
 }  // namespace pb
 
 using namespace pb;
+
+extern "C" int pb200_corner_filter(int K, int C, const float* corners, const float* weights, float* filter, void* stream) {
+    PB_REQUIRE(K > 0 && C > 0 && K <= (1 << 15) && C <= (1 << 15), PB200_EINVAL, "corner_filter: bad sizes");
+    PB_REQUIRE(corners && weights && filter, PB200_EINVAL, "corner_filter: null pointer");
+    PB_LAUNCH("corner_filter", corner_filter_kernel, (unsigned)ceil_div(3 * C, 128), 128, 0, (cudaStream_t)stream, K, C, corners,
+              weights, filter);
+    return PB200_OK;
+}
+
+extern "C" int pb200_corner_filter_backward(int K, int C, const float* corners, const float* gradFilter, float* gradWeights,
+                                            void* stream) {
+    PB_REQUIRE(K > 0 && C > 0 && K <= (1 << 15) && C <= (1 << 15), PB200_EINVAL, "corner_filter_backward: bad sizes");
+    PB_REQUIRE(corners && gradFilter && gradWeights, PB200_EINVAL, "corner_filter_backward: null pointer");
+    PB_LAUNCH("corner_filter_bwd", corner_filter_bwd_kernel, (unsigned)ceil_div(K * C, 128), 128, 0, (cudaStream_t)stream, K, C,
+              corners, gradFilter, gradWeights);
+    return PB200_OK;
+}
 
 extern "C" int pb200_face_mean_sph_harm(int64_t Nf, int64_t NiK, int L, const float* xyz, const int32_t* numInterior,
                                         float* out, void* stream_) {

@@ -13,6 +13,8 @@ import torch
 from ... import _lib
 from ...topology import vertex_csr, ptr, stream_ptr
 
+_ops = _lib.ops
+
 _f2f_precision = _lib.PREC_FP32
 
 
@@ -208,6 +210,8 @@ def facet2vertex_backward(grad_output, input, filter, coeff, face, nfCount, vtMa
 
 
 # ------------------------------------------------------------------ autograd Functions
+# The three calls facet2facet / vertex2facet / facet2vertex go through the native nodes of _torch_ops (same kernels, same
+# gradients, a tenth of the host time); the Function classes are the reference's names for callers that use them directly.
 class f2f_Function(torch.autograd.Function):
     @staticmethod
     def forward(ctx, textureIn, filter, baryCoeff, numTexture):
@@ -236,7 +240,9 @@ def facet2facet(textureIn, filter, baryCoeff, numTexture):
     Output:
         output:      (concat_NfIn, out_channels) float32
     '''
-    return f2f_Function.apply(textureIn, filter, baryCoeff, numTexture)
+    baryCoeff.requires_grad = False
+    numTexture.requires_grad = False
+    return _ops.facet2facet(textureIn, filter, baryCoeff, numTexture, _f2f_precision)
 
 
 class v2f_Function(torch.autograd.Function):
@@ -263,7 +269,13 @@ def vertex2facet(input, filter, face):
     Output:
         output: (concat_NfIn, in_channels*multiplier) float32
     '''
-    return v2f_Function.apply(input, filter, face)
+    face.requires_grad = False
+    rowptr = entries = None
+    if torch.is_grad_enabled() and (input.requires_grad or filter.requires_grad):
+        _check(face, "face", 2, torch.int32)
+        csr = vertex_csr(face, None, input.shape[0], input.shape[0])
+        rowptr, entries = csr.rowptr, csr.entries
+    return _ops.vertex2facet(input, filter, face, rowptr, entries)
 
 
 class f2v_Function(torch.autograd.Function):
@@ -296,4 +308,11 @@ def facet2vertex(input, filter, coeff, face, nfCount, vtMap):
     Output:
         output:  (concat_NvOut, in_channels*multiplier) float32
     '''
-    return f2v_Function.apply(input, filter, coeff, face, nfCount, vtMap)
+    coeff.requires_grad = False
+    face.requires_grad = False
+    nfCount.requires_grad = False
+    vtMap.requires_grad = False
+    _check(face, "face", 2, torch.int32)
+    _check(vtMap, "vt_map", 1, torch.int32)
+    csr = vertex_csr(face, vtMap, vtMap.shape[0], nfCount.shape[0])
+    return _ops.facet2vertex(input, filter, coeff, face, nfCount, vtMap, csr.rowptr, csr.entries)
