@@ -226,6 +226,71 @@ size_t pb200_rows_contract_workspace_bytes(int64_t Nrows, int M, int N);
 int pb200_rows_contract(int64_t Nrows, int M, int N, const float* A, const float* B, float* out, float* colsum,
                         int precision, void* workspace, size_t workspace_bytes, void* stream);
 
+/* ---- whole layers: operator, pointwise stage and batch normalisation --------------------------------------------
+ * The three pointwise forwards with what a layer module adds around them (picasso/mesh/layers.py:109-120,166-175):
+ *   features   (rows, C): the operator's output, written as a by-product for the backward pass (NULL = not wanted; the
+ *              rows entry ignores it);
+ *   mean, var, gamma, beta, eps: running statistics the outputs are normalised with (inference; var NULL = not).  */
+typedef struct {
+    float* features;
+    const float *mean, *var, *gamma, *beta;
+    float eps;
+} pb200_pointwise_extra;
+int pb200_vertex2facet_layer_forward(int64_t Nf, int64_t Nv, int C, int Cout, const float* input, const float* filter,
+                                     const int32_t* face, const float* depthWeights, const float* bias, int relu,
+                                     float* output, int precision, const pb200_pointwise_extra* extra, void* workspace,
+                                     size_t workspace_bytes, void* stream);
+int pb200_facet2vertex_layer_forward(int64_t Nf, int64_t NvOut, int C, int K, int Cout, const float* input,
+                                     const float* filter, const float* coeff, const int32_t* nfCount, const int32_t* rowptr,
+                                     const int32_t* entries, const float* depthWeights, const float* bias, int relu,
+                                     float* output, int precision, const pb200_pointwise_extra* extra, void* workspace,
+                                     size_t workspace_bytes, void* stream);
+int pb200_rows_layer_forward(int64_t Nrows, int C, int Cout, const float* rows, const float* weights, const float* bias,
+                             int relu, float* output, int precision, const pb200_pointwise_extra* extra, void* workspace,
+                             size_t workspace_bytes, void* stream);
+
+/* Gradient of the rows a pointwise stage consumed: (gradOutput taken back through the normalisation `norm` and, with relu,
+ * through the activation, both by the activated rows `mask`) @ weights; maskedRows (may be NULL) receives the first factor.
+ * transposed != 0: weights holds the transposed matrix, (Cout, C) row-major. */
+typedef struct { const float *mean, *scale, *k1, *k2; } pb200_norm_gradient;
+int pb200_gradient_rows_matmul(int64_t Nrows, int C, int Cout, const float* rows, const float* mask, int relu,
+                               const pb200_norm_gradient* norm, const float* weights, int transposed, float* output,
+                               float* maskedRows, int precision, void* workspace, size_t workspace_bytes, void* stream);
+
+/* Batch normalisation over the rows of (N, C) (torch.nn.BatchNorm1d), in the pieces a layer needs.
+ *   bias_act_stats       rows <- act(rows + bias) in place and partial (pb200_norm_parts(N, C), 3, C) statistics of the result;
+ *                        *nparts (host) = partials written
+ *   norm_finalize        merges partials into mean and invstd (C each); moves the running statistics (unbiased variance)
+ *                        and adds one to *batches when they are given
+ *   norm_invstd          invstd = 1 / sqrt(var + eps) for statistics that come from elsewhere; adds one to *batches
+ *   norm_apply           out = gamma * (act - mean) * invstd + beta (gamma, beta may be NULL)
+ *   norm_backward_reduce gradients of gamma and beta, and scale, k1, k2 with
+ *                        gradAct = scale * gradOutput + k2 * (act - mean) + k1
+ *                        (partial: pb200_norm_parts(N, C) * 2 * C floats)
+ *   norm_backward_apply  masked = gradAct (mean NULL: gradOutput) where the activation let the value through; gradBias = its
+ *                        column sums (partial: pb200_norm_parts(N, C) * C floats) */
+int pb200_norm_parts(int64_t N, int C);
+int pb200_bias_act_stats(int64_t N, int C, float* rows, const float* bias, int relu, float* partial, int* nparts, void* stream);
+int pb200_norm_finalize(int nparts, int C, const float* partial, float eps, float momentum, float* runningMean,
+                        float* runningVar, int64_t* batches, float* mean, float* invstd, void* stream);
+int pb200_norm_invstd(int C, const float* var, float eps, int64_t* batches, float* invstd, void* stream);
+int pb200_norm_apply(int64_t N, int C, const float* act, const float* mean, const float* invstd, const float* gamma,
+                     const float* beta, float* out, void* stream);
+int pb200_norm_backward_reduce(int64_t N, int C, const float* gradOutput, const float* act, const float* mean,
+                               const float* invstd, const float* gamma, float* partial, float* gradGamma, float* gradBeta,
+                               float* scale, float* k1, float* k2, void* stream);
+int pb200_norm_backward_apply(int64_t N, int C, const float* gradOutput, const float* act, const float* mean, const float* scale,
+                              const float* k1, const float* k2, int relu, float* masked, float* partial, float* gradBias,
+                              void* stream);
+
+/* out (B, C) = mean over the rows of every sample; `ends` (B,) = running number of rows up to and including the sample
+ * (int64, ends[B-1] == N).  Replaces the scatter of GlobalPool3d (picasso/mesh/layers.py:242-260). */
+size_t pb200_segment_mean_workspace_bytes(int64_t N, int B, int C);
+int pb200_segment_mean(int64_t N, int B, int C, const float* rows, const int64_t* ends, float* out, void* workspace,
+                       size_t workspace_bytes, void* stream);
+int pb200_segment_mean_backward(int64_t N, int B, int C, const float* gradOutput, const int64_t* ends, float* gradInput,
+                                void* stream);
+
 /* ---- facet2facet --------------------------------------------------------------------
  * A[f,d,ci] = (1/T_f) sum_{k in samples(f)} bary[k,d]*input[k,ci];
  * output[f,co] = sum_{d,ci} A[f,d,ci]*filter[co,ci,d];  samples(f) = rows
@@ -281,6 +346,11 @@ int pb200_facet2facet_backward_padded(int64_t Nf, int64_t NiK, int Cin, int Cout
                                       const float* input, const float* filter, const float* bary, const float* baryPadded,
                                       const int32_t* numInterior, float* gradInput, float* gradFilter,
                                       int precision, void* workspace, size_t workspace_bytes, void* stream);
+
+/* The filter gradient alone (same workspace), for samples that are data and need no gradient. */
+int pb200_facet2facet_filter_gradient(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, const float* gradOutput,
+                                      const float* input, const float* bary, const float* baryPadded, const int32_t* numInterior,
+                                      float* gradFilter, int precision, void* workspace, size_t workspace_bytes, void* stream);
 
 /* ---- spherical-harmonic basis and triangle geometry -----------------------------------
  * out[i, 0..(L+1)^2) = real/imaginary spherical-harmonic components of xyz[i] projected

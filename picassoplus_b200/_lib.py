@@ -78,6 +78,7 @@ SIGNATURES = {
     "pb200_facet2facet_backward_workspace_bytes": (sz, [i64, i64, i32, i32, i32, i32]),
     "pb200_facet2facet_backward": (i32, [i64, i64, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, i32, vp, sz, vp]),
     "pb200_facet2facet_backward_padded": (i32, [i64, i64, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, i32, vp, sz, vp]),
+    "pb200_facet2facet_filter_gradient": (i32, [i64, i64, i32, i32, i32, vp, vp, vp, vp, vp, vp, i32, vp, sz, vp]),
     "pb200_level_prepare": (i32, [i64, i64, i64, i32, vp, vp, vp, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, sz, vp]),
     "pb200_cluster_csr_workspace_bytes": (sz, [i64, i64]),
     "pb200_build_cluster_csr": (i32, [i64, i64, vp, vp, vp, vp, vp, vp, vp, sz, vp]),
@@ -98,6 +99,21 @@ SIGNATURES = {
                                   vp, sz, vp]),
     "pb200_combine_clusters": (i32, [i64, i64, vp, vp, vp, vp, vp, vp, vp, vp, sz, vp]),
     "pb200_rows_pointwise_forward": (i32, [i64, i32, i32, vp, vp, vp, i32, vp, i32, vp, sz, vp]),
+    "pb200_vertex2facet_layer_forward": (i32, [i64, i64, i32, i32, vp, vp, vp, vp, vp, i32, vp, i32, vp, vp, sz, vp]),
+    "pb200_facet2vertex_layer_forward": (i32, [i64, i64, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, i32, vp, i32,
+                                               vp, vp, sz, vp]),
+    "pb200_rows_layer_forward": (i32, [i64, i32, i32, vp, vp, vp, i32, vp, i32, vp, vp, sz, vp]),
+    "pb200_gradient_rows_matmul": (i32, [i64, i32, i32, vp, vp, i32, vp, vp, i32, vp, vp, i32, vp, sz, vp]),
+    "pb200_norm_parts": (i32, [i64, i32]),
+    "pb200_bias_act_stats": (i32, [i64, i32, vp, vp, i32, vp, vp, vp]),
+    "pb200_norm_finalize": (i32, [i32, i32, vp, f32, f32, vp, vp, vp, vp, vp, vp]),
+    "pb200_norm_invstd": (i32, [i32, vp, f32, vp, vp, vp]),
+    "pb200_norm_apply": (i32, [i64, i32, vp, vp, vp, vp, vp, vp, vp]),
+    "pb200_norm_backward_reduce": (i32, [i64, i32, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]),
+    "pb200_norm_backward_apply": (i32, [i64, i32, vp, vp, vp, vp, vp, vp, i32, vp, vp, vp, vp]),
+    "pb200_segment_mean_workspace_bytes": (sz, [i64, i32, i32]),
+    "pb200_segment_mean": (i32, [i64, i32, i32, vp, vp, vp, vp, sz, vp]),
+    "pb200_segment_mean_backward": (i32, [i64, i32, i32, vp, vp, vp, vp]),
     "pb200_masked_rows_matmul_workspace_bytes": (sz, [i32, i32]),
     "pb200_masked_rows_matmul": (i32, [i64, i32, i32, vp, vp, vp, vp, vp, i32, vp, sz, vp]),
     "pb200_rows_contract_workspace_bytes": (sz, [i64, i32, i32]),

@@ -161,7 +161,7 @@ size_t pb200_facet2facet_backward_workspace_bytes(int64_t Nf, int64_t NiK, int C
 static int f2f_backward_impl(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, const float* gradOutput,
                              const float* input, const float* filter, const float* bary, const float* baryPadded,
                              const int32_t* numInterior, float* gradInput, float* gradFilter, int precision,
-                             void* workspace, size_t workspace_bytes, void* stream_) {
+                             void* workspace, size_t workspace_bytes, void* stream_, bool want_gin) {
     cudaStream_t stream = (cudaStream_t)stream_;
     PB_REQUIRE(f2f_sizes_ok(Nf, NiK, Cin, Cout, F), PB200_EINVAL,
                "facet2facet_backward: bad sizes (F must be in 1..50)");
@@ -172,7 +172,7 @@ static int f2f_backward_impl(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, 
         PB_CUDA(cudaMemsetAsync(gradFilter, 0, sizeof(float) * (size_t)Cout * Cin * F, stream));
         return PB200_OK;
     }
-    PB_REQUIRE(gradOutput && filter && numInterior && (NiK == 0 || (input && bary && gradInput)), PB200_EINVAL,
+    PB_REQUIRE(gradOutput && (filter || !want_gin) && numInterior && (NiK == 0 || (input && bary && (gradInput || !want_gin))), PB200_EINVAL,
                "facet2facet_backward: null pointer");
     PB_REQUIRE(workspace && workspace_bytes >= pb200_facet2facet_backward_workspace_bytes(Nf, NiK, Cin, Cout, F, precision),
                PB200_EWORKSPACE, "facet2facet_backward: workspace too small");
@@ -199,7 +199,7 @@ static int f2f_backward_impl(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, 
         }
     }
     if (tg) {
-        if (NiK > 0) {
+        if (NiK > 0 && want_gin) {
             int rc = tc::gin::backward_input(Nf, Cin, Cout, F, gradOutput, filter, bary, bary_p, Fp, numInterior,
                                              gradInput, precision, w, stream, false);
             if (rc) return rc;
@@ -221,9 +221,9 @@ static int f2f_backward_impl(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, 
                                               precision, w, stream);
         if (rc) return rc;
     }
-    if (tg && tf) return PB200_OK;
+    if ((tg || !want_gin) && tf) return PB200_OK;
     return f2f_simt_backward(Nf, NiK, Cin, Cout, F, gradOutput, input, filter, bary, numInterior, gradInput,
-                             gradFilter, simt_ws, stream, !tg, !tf);
+                             gradFilter, simt_ws, stream, !tg && want_gin, !tf);
 }
 
 extern "C" {
@@ -233,7 +233,7 @@ int pb200_facet2facet_backward(int64_t Nf, int64_t NiK, int Cin, int Cout, int F
                                const int32_t* numInterior, float* gradInput, float* gradFilter, int precision,
                                void* workspace, size_t workspace_bytes, void* stream) {
     return f2f_backward_impl(Nf, NiK, Cin, Cout, F, gradOutput, input, filter, bary, nullptr, numInterior, gradInput,
-                             gradFilter, precision, workspace, workspace_bytes, stream);
+                             gradFilter, precision, workspace, workspace_bytes, stream, true);
 }
 
 int pb200_facet2facet_backward_padded(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, const float* gradOutput,
@@ -241,7 +241,15 @@ int pb200_facet2facet_backward_padded(int64_t Nf, int64_t NiK, int Cin, int Cout
                                       const int32_t* numInterior, float* gradInput, float* gradFilter, int precision,
                                       void* workspace, size_t workspace_bytes, void* stream) {
     return f2f_backward_impl(Nf, NiK, Cin, Cout, F, gradOutput, input, filter, bary, baryPadded, numInterior, gradInput,
-                             gradFilter, precision, workspace, workspace_bytes, stream);
+                             gradFilter, precision, workspace, workspace_bytes, stream, true);
+}
+
+// for callers whose samples are data (raw textures): the input gradient, a third of the backward pass, is left out
+int pb200_facet2facet_filter_gradient(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, const float* gradOutput,
+                                      const float* input, const float* bary, const float* baryPadded, const int32_t* numInterior,
+                                      float* gradFilter, int precision, void* workspace, size_t workspace_bytes, void* stream) {
+    return f2f_backward_impl(Nf, NiK, Cin, Cout, F, gradOutput, input, nullptr, bary, baryPadded, numInterior, nullptr, gradFilter,
+                             precision, workspace, workspace_bytes, stream, false);
 }
 
 int pb200_padded_row_floats(int F) { return F > 0 ? tc::padded_F(F) : 0; }

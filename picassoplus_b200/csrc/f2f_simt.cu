@@ -202,8 +202,9 @@ int f2f_simt_backward(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, const f
     int64_t FC = f2f_chunk_faces(Nf, Q);
     float* A = (float*)w;   w += align_up(sizeof(float) * (size_t)FC * Q, 256);
     float* gA = (float*)w;
-    PB_LAUNCH("f2f_transpose_filter", f2f_transpose_filter_kernel, persistent_blocks((int64_t)Q * Cout, 256, 8), 256, 0,
-              stream, F, Cin, Cout, filter, Wt);
+    if (want_gin)
+        PB_LAUNCH("f2f_transpose_filter", f2f_transpose_filter_kernel, persistent_blocks((int64_t)Q * Cout, 256, 8), 256, 0,
+                  stream, F, Cin, Cout, filter, Wt);
     PB_CUDA(cudaMemsetAsync(gWt, 0, sizeof(float) * (size_t)Q * Cout, stream));
     for (int64_t f0 = 0; f0 < Nf; f0 += FC) {
         int64_t nf = Nf - f0 < FC ? Nf - f0 : FC;

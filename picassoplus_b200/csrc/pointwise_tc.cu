@@ -40,7 +40,8 @@ constexpr int W_TILE_BYTES = UM * 64;
 constexpr int KB = 32;                      // channels per stage (one 64-byte bf16 operand row)
 
 // weight image: Wimg[kb][split][co 0..127][32 bf16, 64B-swizzled], element (co, k) = Wd[kb*32 + k][co0 + co]
-__global__ void pw_prep_weights_kernel(int Cmid, int Cout, int co0, int cchunk, int nkb, int nsplit,
+// at wd[k * sk + n * sn]: (sk, sn) = (Cout, 1) for the layer's weights as they are, (1, Cin) for their transpose
+__global__ void pw_prep_weights_kernel(int Cmid, int64_t sk, int64_t sn, int co0, int cchunk, int nkb, int nsplit,
                                        const float* __restrict__ wd, uint8_t* __restrict__ wimg) {
     const int64_t total = (int64_t)nkb * UM * 4;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -54,7 +55,7 @@ __global__ void pw_prep_weights_kernel(int Cmid, int Cout, int co0, int cchunk, 
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 const int ci = kb * KB + c * 8 + 2 * j + e;
-                v[e] = (co < cchunk && ci < Cmid) ? __ldg(wd + (int64_t)ci * Cout + co0 + co) : 0.f;
+                v[e] = (co < cchunk && ci < Cmid) ? __ldg(wd + ci * sk + (co0 + co) * sn) : 0.f;
             }
             if (nsplit == 1) { hi[j] = pack_bf16x2(v[0], v[1]); lo[j] = 0u; }
             else split_bf16x2(v[0], v[1], hi[j], lo[j]);
@@ -86,11 +87,19 @@ struct Params {
     const int32_t* nfCount;
     // masked rows (backward of the pointwise stage)
     const float* rows;        // (Nrows, C) upstream gradient
-    const float* mask;        // (Nrows, C) activated output: the gradient passes where it is > 0; NULL = no mask
+    const float* mask;        // (Nrows, C) activated output; NULL = neither mask nor normalisation
+    int relu_mask;            // the gradient passes where the activated output is > 0
     float* masked_out;        // (Nrows, C) the masked gradient, written as a by-product; NULL = not wanted
+    // gradient through a batch normalisation behind the activation: rows <- scale * rows + k2 * (mask - mean) + k1, per channel,
+    // before the mask is applied (norm.cu); NULL = none
+    const float *bn_mean, *bn_scale, *bn_k1, *bn_k2;
+    float* feat_out;          // (Nrows, C) the gathered rows, written as a by-product for the backward pass; NULL = not wanted
     const uint8_t* wimg;
     const float* bias;        // (Cout chunk) or NULL
     float* out;               // first output channel of the chunk
+    // inference: outputs are normalised with the running statistics (first channel of the chunk); ev_var NULL = not
+    const float *ev_mean, *ev_var, *ev_gamma, *ev_beta;
+    float ev_eps;
     int* async_err;
     int wait_budget;
 };
@@ -208,10 +217,26 @@ __global__ void __launch_bounds__(NTHREADS, 1) rows_pointwise_tc_kernel(Params p
                             if (p.mask) {
                                 const float4* mk = reinterpret_cast<const float4*>(p.mask + row * C + c);
                                 const float4 m0 = ldg4(mk), m1 = ldg4(mk + 1);
+                                if (p.bn_mean) {
+                                    auto through = [&](float4& a, const float4& x, int o) {
+                                        const float4 mu = ldg4(reinterpret_cast<const float4*>(p.bn_mean + c) + o);
+                                        const float4 sc = ldg4(reinterpret_cast<const float4*>(p.bn_scale + c) + o);
+                                        const float4 k1 = ldg4(reinterpret_cast<const float4*>(p.bn_k1 + c) + o);
+                                        const float4 k2 = ldg4(reinterpret_cast<const float4*>(p.bn_k2 + c) + o);
+                                        a.x = fmaf(sc.x, a.x, fmaf(k2.x, x.x - mu.x, k1.x));
+                                        a.y = fmaf(sc.y, a.y, fmaf(k2.y, x.y - mu.y, k1.y));
+                                        a.z = fmaf(sc.z, a.z, fmaf(k2.z, x.z - mu.z, k1.z));
+                                        a.w = fmaf(sc.w, a.w, fmaf(k2.w, x.w - mu.w, k1.w));
+                                    };
+                                    through(a0, m0, 0);
+                                    through(a1, m1, 1);
+                                }
+                                if (p.relu_mask) {
                                 a0 = make_float4(m0.x > 0.f ? a0.x : 0.f, m0.y > 0.f ? a0.y : 0.f, m0.z > 0.f ? a0.z : 0.f,
                                                  m0.w > 0.f ? a0.w : 0.f);
                                 a1 = make_float4(m1.x > 0.f ? a1.x : 0.f, m1.y > 0.f ? a1.y : 0.f, m1.z > 0.f ? a1.z : 0.f,
                                                  m1.w > 0.f ? a1.w : 0.f);
+                                }
                             }
                             if (p.masked_out) {
                                 float4* mo = reinterpret_cast<float4*>(p.masked_out + row * C + c);
@@ -228,6 +253,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) rows_pointwise_tc_kernel(Params p
                         }
                         if (end > beg) { a0 = scale4(a0, inv_n); a1 = scale4(a1, inv_n); }
                     }
+                    if (MODE != 2 && p.feat_out && valid) {
+                        float4* fo = reinterpret_cast<float4*>(p.feat_out + row * C + c);
+                        fo[0] = a0; fo[1] = a1;
+                    }
                 }
                 if (!publish(a0, a1, b16)) { alive = false; break; }
             }
@@ -241,6 +270,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) rows_pointwise_tc_kernel(Params p
             const int q = warp & 3, g = warp >> 2;
             const int co = q * 32 + lane;
             const float bv = (p.bias && co < Cout) ? __ldg(p.bias + co) : 0.f;
+            float ev_m = 0.f, ev_s = 1.f, ev_b = 0.f;
+            if (p.ev_var && co < Cout) {
+                ev_m = __ldg(p.ev_mean + co);
+                ev_s = 1.f / sqrtf(__ldg(p.ev_var + co) + p.ev_eps);
+                if (p.ev_gamma) ev_s *= __ldg(p.ev_gamma + co);
+                if (p.ev_beta) ev_b = __ldg(p.ev_beta + co);
+            }
 #pragma unroll 1
             for (int half = 0; half < 2; ++half) {
                 const int col = g * 64 + half * 32;
@@ -248,12 +284,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) rows_pointwise_tc_kernel(Params p
                 tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)col, r);
                 tmem_ld_wait();
                 if (co < Cout) {
+                    const int64_t left = p.Nrows - (r0 + col);
+                    const int cnt = left < 32 ? (int)left : 32;              // rows of this half (<= 0: none)
+                    float* o = p.out + (r0 + col) * p.out_stride + co;
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
-                        const int64_t ro = r0 + col + j;
                         float v = __uint_as_float(r[j]) + bv;
                         if (p.relu) v = fmaxf(v, 0.f);
-                        if (ro < p.Nrows) __stcs(p.out + ro * p.out_stride + co, v);
+                        v = fmaf(v - ev_m, ev_s, ev_b);
+                        if (j < cnt) __stcs(o + (int64_t)j * p.out_stride, v);
                     }
                 }
             }
@@ -341,9 +380,19 @@ static Plan plan(int C, int precision) {
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
+// What a layer adds around the product: normalisation of the outputs, the by-product (pb200_pointwise_extra).
+static int set_extra(Params& p, const pb200_pointwise_extra* x, const char* where) {
+    if (!x) return PB200_OK;
+    PB_REQUIRE(!x->features || aligned16(x->features), PB200_EINVAL, "%s: features must be 16-byte aligned", where);
+    PB_REQUIRE(!x->var || x->mean, PB200_EINVAL, "%s: variance without mean", where);
+    p.feat_out = x->features;
+    p.ev_mean = x->mean; p.ev_var = x->var; p.ev_gamma = x->gamma; p.ev_beta = x->beta; p.ev_eps = x->eps;
+    return PB200_OK;
+}
+
 template <int MODE>
 static int run(Params p, int Cout, const float* wd, const float* bias, float* out, int precision, void* ws,
-               cudaStream_t stream) {
+               cudaStream_t stream, bool transposed = false) {
     int rc = tc::check_async_error("pointwise fusion");
     if (rc) return rc;
     const Plan pl = plan(p.C, precision);
@@ -353,13 +402,16 @@ static int run(Params p, int Cout, const float* wd, const float* bias, float* ou
     p.wait_budget = tc::wait_budget_kclocks();
     const int64_t ntiles = ceil_div(p.Nrows, TILE_R);
     const int grid = (int)(ntiles < sm_count() ? ntiles : sm_count());
+    const Params all = p;
     for (int co0 = 0; co0 < Cout; co0 += UM) {
         const int cchunk = Cout - co0 < UM ? Cout - co0 : UM;
         PB_LAUNCH("pw_prep_weights", pw_prep_weights_kernel, persistent_blocks((int64_t)pl.nkb * UM * 4, 256, 8), 256, 0, stream,
-                  p.C, Cout, co0, cchunk, pl.nkb, pl.nsplit, wd, wimg);
+                  p.C, (int64_t)(transposed ? 1 : Cout), (int64_t)(transposed ? p.C : 1), co0, cchunk, pl.nkb, pl.nsplit, wd, wimg);
         p.Cout = cchunk; p.wimg = wimg; p.bias = bias ? bias + co0 : nullptr; p.out = out + co0;
+        p.ev_mean = all.ev_var ? all.ev_mean + co0 : nullptr; p.ev_var = all.ev_var ? all.ev_var + co0 : nullptr;
+        p.ev_gamma = all.ev_gamma ? all.ev_gamma + co0 : nullptr; p.ev_beta = all.ev_beta ? all.ev_beta + co0 : nullptr;
         const char* label = MODE == 0 ? "v2f_pointwise_tc" : (MODE == 1 ? "f2v_pointwise_tc" : "masked_rows_tc");
-        if (MODE == 2 && co0 > 0) p.masked_out = nullptr;      // the by-product is written by the first chunk's launch
+        if (co0 > 0) { p.masked_out = nullptr; p.feat_out = nullptr; }      // by-products are written by the first chunk's launch
         if (pl.nsplit == 2) {
             PB_CUDA(cudaFuncSetAttribute(rows_pointwise_tc_kernel<2, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
             PB_LAUNCH(label, (rows_pointwise_tc_kernel<2, MODE>), grid, NTHREADS, pl.smem, stream, p);
@@ -385,8 +437,15 @@ size_t pb200_vertex2facet_pointwise_workspace_bytes(int C, int precision) {
 
 int pb200_vertex2facet_pointwise_forward(int64_t Nf, int64_t Nv, int C, int Cout, const float* input, const float* filter,
                                          const int32_t* face, const float* depthWeights, const float* bias, int relu,
-                                         float* output, int precision, void* workspace, size_t workspace_bytes,
-                                         void* stream_) {
+                                         float* output, int precision, void* workspace, size_t workspace_bytes, void* stream) {
+    return pb200_vertex2facet_layer_forward(Nf, Nv, C, Cout, input, filter, face, depthWeights, bias, relu, output, precision, nullptr,
+                                            workspace, workspace_bytes, stream);
+}
+
+int pb200_vertex2facet_layer_forward(int64_t Nf, int64_t Nv, int C, int Cout, const float* input, const float* filter,
+                                         const int32_t* face, const float* depthWeights, const float* bias, int relu,
+                                         float* output, int precision, const pb200_pointwise_extra* extra, void* workspace,
+                                         size_t workspace_bytes, void* stream_) {
     cudaStream_t stream = (cudaStream_t)stream_;
     PB_REQUIRE(Nf >= 0 && Nv >= 0 && C > 0 && Cout > 0 && C % 8 == 0 && Nf < (1LL << 31) && Nv < (1LL << 31), PB200_EINVAL,
                "vertex2facet_pointwise_forward: bad sizes (channels must be a multiple of 8)");
@@ -401,6 +460,7 @@ int pb200_vertex2facet_pointwise_forward(int64_t Nf, int64_t Nv, int C, int Cout
     pw::Params p = {};
     p.Nrows = Nf; p.C = C; p.relu = relu;
     p.vin = input; p.vfilt = filter; p.face = face; p.Nv = Nv;
+    if (int rc = pw::set_extra(p, extra, "vertex2facet_pointwise_forward")) return rc;
     return pw::run<0>(p, Cout, depthWeights, bias, output, precision, workspace, stream);
 }
 
@@ -410,10 +470,19 @@ size_t pb200_facet2vertex_pointwise_workspace_bytes(int64_t Nf, int C, int preci
 }
 
 int pb200_facet2vertex_pointwise_forward(int64_t Nf, int64_t NvOut, int C, int K, int Cout, const float* input,
+                                         const float* filter, const float* coeff, const int32_t* nfCount, const int32_t* rowptr,
+                                         const int32_t* entries, const float* depthWeights, const float* bias, int relu,
+                                         float* output, int precision, void* workspace, size_t workspace_bytes, void* stream) {
+    return pb200_facet2vertex_layer_forward(Nf, NvOut, C, K, Cout, input, filter, coeff, nfCount, rowptr, entries, depthWeights, bias,
+                                            relu, output, precision, nullptr, workspace, workspace_bytes, stream);
+}
+
+int pb200_facet2vertex_layer_forward(int64_t Nf, int64_t NvOut, int C, int K, int Cout, const float* input,
                                          const float* filter, const float* coeff, const int32_t* nfCount,
                                          const int32_t* rowptr, const int32_t* entries, const float* depthWeights,
-                                         const float* bias, int relu, float* output, int precision, void* workspace,
-                                         size_t workspace_bytes, void* stream_) {
+                                         const float* bias, int relu, float* output, int precision,
+                                         const pb200_pointwise_extra* extra, void* workspace, size_t workspace_bytes,
+                                         void* stream_) {
     cudaStream_t stream = (cudaStream_t)stream_;
     PB_REQUIRE(Nf >= 0 && NvOut >= 0 && C > 0 && K > 0 && Cout > 0 && C % 8 == 0 && f2v_face_products_supported(C, K) &&
                    Nf < (1LL << 29) && NvOut < (1LL << 31),
@@ -436,6 +505,7 @@ int pb200_facet2vertex_pointwise_forward(int64_t Nf, int64_t NvOut, int C, int K
     pw::Params p = {};
     p.Nrows = NvOut; p.C = C; p.relu = relu;
     p.wx = wx; p.rowptr = rowptr; p.entries = entries; p.nfCount = nfCount;
+    if (int rc = pw::set_extra(p, extra, "facet2vertex_pointwise_forward")) return rc;
     return pw::run<1>(p, Cout, depthWeights, bias, output, precision, workspace, stream);
 }
 
@@ -445,8 +515,14 @@ size_t pb200_masked_rows_matmul_workspace_bytes(int C, int precision) {
 }
 
 int pb200_rows_pointwise_forward(int64_t Nrows, int C, int Cout, const float* rows, const float* weights, const float* bias,
-                                 int relu, float* output, int precision, void* workspace, size_t workspace_bytes,
-                                 void* stream_) {
+                                 int relu, float* output, int precision, void* workspace, size_t workspace_bytes, void* stream) {
+    return pb200_rows_layer_forward(Nrows, C, Cout, rows, weights, bias, relu, output, precision, nullptr, workspace, workspace_bytes,
+                                    stream);
+}
+
+int pb200_rows_layer_forward(int64_t Nrows, int C, int Cout, const float* rows, const float* weights, const float* bias,
+                                 int relu, float* output, int precision, const pb200_pointwise_extra* extra, void* workspace,
+                                 size_t workspace_bytes, void* stream_) {
     cudaStream_t stream = (cudaStream_t)stream_;
     PB_REQUIRE(Nrows >= 0 && C > 0 && Cout > 0 && C % 8 == 0 && Nrows < (1LL << 31), PB200_EINVAL,
                "rows_pointwise_forward: bad sizes (the row width must be a multiple of 8)");
@@ -461,12 +537,20 @@ int pb200_rows_pointwise_forward(int64_t Nrows, int C, int Cout, const float* ro
     pw::Params p = {};
     p.Nrows = Nrows; p.C = C; p.relu = relu;
     p.rows = rows;
+    if (int rc = pw::set_extra(p, extra, "rows_pointwise_forward")) return rc;
     return pw::run<2>(p, Cout, weights, bias, output, precision, workspace, stream);
 }
 
 int pb200_masked_rows_matmul(int64_t Nrows, int C, int Cout, const float* rows, const float* mask, const float* weights,
                              float* output, float* maskedRows, int precision, void* workspace, size_t workspace_bytes,
-                             void* stream_) {
+                             void* stream) {
+    return pb200_gradient_rows_matmul(Nrows, C, Cout, rows, mask, 1, nullptr, weights, 0, output, maskedRows, precision, workspace,
+                                      workspace_bytes, stream);
+}
+
+int pb200_gradient_rows_matmul(int64_t Nrows, int C, int Cout, const float* rows, const float* mask, int relu,
+                               const pb200_norm_gradient* norm, const float* weights, int transposed, float* output, float* maskedRows,
+                               int precision, void* workspace, size_t workspace_bytes, void* stream_) {
     cudaStream_t stream = (cudaStream_t)stream_;
     PB_REQUIRE(Nrows >= 0 && C > 0 && Cout > 0 && C % 8 == 0 && Nrows < (1LL << 31), PB200_EINVAL,
                "masked_rows_matmul: bad sizes (the row width must be a multiple of 8)");
@@ -480,8 +564,14 @@ int pb200_masked_rows_matmul(int64_t Nrows, int C, int Cout, const float* rows, 
                "masked_rows_matmul: workspace too small");
     pw::Params p = {};
     p.Nrows = Nrows; p.C = C; p.relu = 0;
-    p.rows = rows; p.mask = mask; p.masked_out = maskedRows;
-    return pw::run<2>(p, Cout, weights, nullptr, output, precision, workspace, stream);
+    p.rows = rows; p.mask = mask; p.masked_out = maskedRows; p.relu_mask = relu;
+    if (norm) {
+        PB_REQUIRE(mask && norm->mean && norm->scale && norm->k1 && norm->k2 && pw::aligned16(norm->mean) && pw::aligned16(norm->scale) &&
+                       pw::aligned16(norm->k1) && pw::aligned16(norm->k2),
+                   PB200_EINVAL, "masked_rows_matmul: normalisation needs the activated rows and 16-byte aligned per-channel arrays");
+        p.bn_mean = norm->mean; p.bn_scale = norm->scale; p.bn_k1 = norm->k1; p.bn_k2 = norm->k2;
+    }
+    return pw::run<2>(p, Cout, weights, nullptr, output, precision, workspace, stream, transposed != 0);
 }
 
 }  // extern "C"

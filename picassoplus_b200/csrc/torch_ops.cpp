@@ -145,15 +145,20 @@ Tensor f2f_one_sample_forward(const Scope& s, const Tensor& input, const Tensor&
 }
 
 void f2f_backward(const Scope& s, const Tensor& g, const Tensor& input, const Tensor& filter, const Tensor& bary,
-                  const Tensor& bary_padded, const Tensor& cum, int precision, Tensor& gin, Tensor& gf) {
+                  const Tensor& bary_padded, const Tensor& cum, int precision, Tensor& gin, Tensor& gf, bool want_gin) {
     const int64_t NiK = input.size(0), Cin = input.size(1), Cout = filter.size(0), F = filter.size(2), Nf = cum.size(0);
-    gin = s.floats({NiK, Cin});
+    if (want_gin) gin = s.floats({NiK, Cin});
     gf = s.floats({Cout, Cin, F});
     const size_t nb = pb200_facet2facet_backward_workspace_bytes(Nf, NiK, (int)Cin, (int)Cout, (int)F, precision);
     Tensor ws = s.bytes(nb);
-    call(pb200_facet2facet_backward_padded(Nf, NiK, (int)Cin, (int)Cout, (int)F, fp(g), fp(input), fp(filter), fp(bary),
-                                           fp(bary_padded), ip(cum), fpm(gin), fpm(gf), precision, ws.data_ptr(), nb, s.stream),
-         "pb200_facet2facet_backward_padded");
+    if (want_gin)
+        call(pb200_facet2facet_backward_padded(Nf, NiK, (int)Cin, (int)Cout, (int)F, fp(g), fp(input), fp(filter), fp(bary),
+                                               fp(bary_padded), ip(cum), fpm(gin), fpm(gf), precision, ws.data_ptr(), nb, s.stream),
+             "pb200_facet2facet_backward_padded");
+    else
+        call(pb200_facet2facet_filter_gradient(Nf, NiK, (int)Cin, (int)Cout, (int)F, fp(g), fp(input), fp(bary), fp(bary_padded), ip(cum),
+                                               fpm(gf), precision, ws.data_ptr(), nb, s.stream),
+             "pb200_facet2facet_filter_gradient");
 }
 
 // --------------------------------------------------------------------------------------------------------- checks
@@ -240,7 +245,7 @@ struct F2F : Node {
         const Tensor x = input.unpack();
         Scope s(x);
         f2f_backward(s, aligned(upstream(grads)), aligned(x), filter.unpack(), aligned(bary.unpack()), bary_padded.unpack(),
-                     cum.unpack(), precision, out[0], out[1]);
+                     cum.unpack(), precision, out[0], out[1], task_should_compute_output(0));
         return out;
     }
     void release_variables() override {
@@ -265,7 +270,7 @@ struct ConvBlock : Node {
         f2v_backward(s, upstream(grads), z.unpack(), filter_out.unpack(), coeff.unpack(), fc, nf_count.unpack(), vt_map.unpack(),
                      gz, out[3]);
         f2f_backward(s, gz, y.unpack(), filter.unpack(), weights.unpack(), weights_padded.unpack(), one_each.unpack(), precision,
-                     gy, out[2]);
+                     gy, out[2], true);
         gz.reset();
         v2f_backward(s, gy, xin, sp, fc, rowptr.unpack(), entries.unpack(), out[0], gs);
         if (task_should_compute_output(1)) {
@@ -441,6 +446,588 @@ Tensor conv_block(const Tensor& x, const Tensor& wv_in, const Tensor& wf_in, con
     return out;
 }
 
+// ------------------------------------------------------------------------------------------------------------ layers
+// What stands behind the operator of a layer: product with depth_weights, bias, ReLU or nothing, batch normalisation.
+enum NormMode { NORM_NONE = 0, NORM_BATCH = 1, NORM_RUNNING = 2 };
+struct Tail {
+    int mode = NORM_NONE;
+    bool relu = false;
+    Tensor gamma, beta, running_mean, running_var, batches;
+    double momentum = 0, eps = 0;
+};
+
+// Mean and 1 / deviation of every channel
+struct NormStats { Tensor mean, invstd; };
+void bump(const Tensor& t) { if (t.defined()) t.unsafeGetTensorImpl()->bump_version(); }
+int64_t* counter(const Tensor& t) { return t.defined() ? static_cast<int64_t*>(t.data_ptr()) : nullptr; }
+
+// Statistics of activated rows with torch's own reduction (norm.cu says why); it moves the running statistics too.
+NormStats batch_stats(const Scope& s, const Tail& t, const Tensor& act) {
+    NormStats st;
+    Tensor var;
+    std::tie(st.mean, var) = at::batch_norm_update_stats(act, t.running_mean, t.running_var, t.momentum);
+    st.invstd = s.floats({act.size(1)});
+    call(pb200_norm_invstd((int)act.size(1), fp(var), (float)t.eps, counter(t.batches), fpm(st.invstd), s.stream), "pb200_norm_invstd");
+    bump(t.running_mean);
+    bump(t.running_var);
+    bump(t.batches);
+    return st;
+}
+
+// Statistics from the partials of pb200_bias_act_stats
+NormStats finalize(const Scope& s, const Tail& t, int64_t C, int nparts, const Tensor& partial) {
+    NormStats st{s.floats({C}), s.floats({C})};
+    call(pb200_norm_finalize(nparts, (int)C, fp(partial), (float)t.eps, (float)t.momentum, fpm(t.running_mean), fpm(t.running_var),
+                             counter(t.batches), fpm(st.mean), fpm(st.invstd), s.stream),
+         "pb200_norm_finalize");
+    bump(t.running_mean);
+    bump(t.running_var);
+    bump(t.batches);
+    return st;
+}
+
+Tensor normalise(const Scope& s, const Tail& t, const Tensor& act, const NormStats& st) {
+    Tensor out = s.floats(act.sizes());
+    call(pb200_norm_apply(act.size(0), (int)act.size(1), fp(act), fp(st.mean), fp(st.invstd), fp(t.gamma), fp(t.beta), fpm(out), s.stream),
+         "pb200_norm_apply");
+    return out;
+}
+
+// The per-channel factors that take a gradient back through the normalisation, each array on a 16-byte boundary, and the
+// gradients of gamma and beta
+struct NormGrads {
+    Tensor buffer, gamma, beta;
+    pb200_norm_gradient factors = {nullptr, nullptr, nullptr, nullptr};
+};
+NormGrads norm_backward(const Scope& s, const Tensor& g, const Tensor& act, const NormStats& st, const Tensor& gamma) {
+    const int64_t rows = act.size(0), C = act.size(1), pitch = (C + 3) / 4 * 4;
+    NormGrads r{s.floats({3, pitch}), s.floats({C}), s.floats({C})};
+    float *scale = fpm(r.buffer), *k1 = scale + pitch, *k2 = k1 + pitch;
+    Tensor partial = s.floats({pb200_norm_parts(rows, (int)C), 2, C});
+    call(pb200_norm_backward_reduce(rows, (int)C, fp(g), fp(act), fp(st.mean), fp(st.invstd), fp(gamma), fpm(partial), fpm(r.gamma),
+                                    fpm(r.beta), scale, k1, k2, s.stream),
+         "pb200_norm_backward_reduce");
+    r.factors = {fp(st.mean), scale, k1, k2};
+    return r;
+}
+
+// The gradient in front of the activation, as an array of its own, and its column sums
+void masked_gradient(const Scope& s, const Tensor& g, const Tensor& act, const NormGrads& n, bool relu, Tensor& gm, Tensor& bias) {
+    const int64_t rows = act.size(0), C = act.size(1);
+    gm = s.floats({rows, C});
+    bias = s.floats({1, C});
+    Tensor partial = s.floats({pb200_norm_parts(rows, (int)C), C});
+    call(pb200_norm_backward_apply(rows, (int)C, fp(g), fp(act), n.factors.mean, n.factors.scale, n.factors.k1, n.factors.k2, relu ? 1 : 0,
+                                   fpm(gm), fpm(partial), fpm(bias), s.stream),
+         "pb200_norm_backward_apply");
+}
+
+// The pointwise stage of a forward pass.  `launch` runs the operator's layer entry with the extras it is handed; what
+// the backward pass needs stays in `act`, `features` and `stats`.
+struct Staged { Tensor out, act, features; NormStats stats; };
+template <typename Launch>
+Staged run_stage(const Scope& s, const Tail& t, int64_t rows, int64_t C, int64_t Cout, bool keep_features, Launch&& launch) {
+    Staged r;
+    r.act = s.floats({rows, Cout});
+    pb200_pointwise_extra x = {};
+    if (keep_features) { r.features = s.floats({rows, C}); x.features = fpm(r.features); }
+    if (t.mode == NORM_RUNNING) {
+        x.mean = fp(t.running_mean); x.var = fp(t.running_var); x.gamma = fp(t.gamma); x.beta = fp(t.beta); x.eps = (float)t.eps;
+    }
+    launch(fpm(r.act), &x);
+    r.out = r.act;
+    if (t.mode == NORM_BATCH) {
+        r.stats = batch_stats(s, t, r.act);
+        r.out = normalise(s, t, r.act, r.stats);
+    }
+    return r;
+}
+
+struct StageGrads { Tensor features, weights, bias, gamma, beta; };
+
+// Gradients of out = norm(act(features @ weights + bias)) for upstream g.
+StageGrads stage_backward(const Scope& s, const Tensor& g_in, const Tensor& act, const Tensor& features, const Tensor& weights,
+                          const NormStats& st, const Tensor& gamma, bool relu, bool want_features, int precision) {
+    const int64_t rows = act.size(0), C = weights.size(0), Cout = act.size(1);
+    StageGrads r;
+    const Tensor g = aligned(g_in);
+    const bool normed = st.mean.defined();
+    NormGrads n;
+    if (normed) {
+        n = norm_backward(s, g, act, st, gamma);
+        r.gamma = n.gamma;
+        r.beta = n.beta;
+    }
+    Tensor gm = g;
+    if (Cout % 8 == 0 && rows > 0 && want_features) {
+        r.features = s.floats({rows, C});
+        if (relu || normed) gm = s.floats({rows, Cout});
+        const size_t nb = pb200_masked_rows_matmul_workspace_bytes((int)Cout, precision);
+        Tensor ws = s.bytes(nb);
+        call(pb200_gradient_rows_matmul(rows, (int)Cout, (int)C, fp(g), relu || normed ? fp(act) : nullptr, relu ? 1 : 0,
+                                        normed ? &n.factors : nullptr, fp(weights), 1, fpm(r.features),
+                                        gm.is_same(g) ? nullptr : fpm(gm), precision, ws.data_ptr(), nb, s.stream),
+             "pb200_gradient_rows_matmul");
+    } else {
+        if (rows > 0 && (relu || normed)) masked_gradient(s, g, act, n, relu, gm, r.bias);
+        if (want_features) r.features = at::matmul(gm, weights.t());
+    }
+    if (C % 4 == 0 && Cout % 4 == 0 && rows > 0) {
+        const Tensor a = aligned(features);
+        r.weights = s.floats({C, Cout});
+        r.bias = s.floats({1, Cout});
+        const size_t nb = pb200_rows_contract_workspace_bytes(rows, (int)C, (int)Cout);
+        Tensor ws = s.bytes(nb);
+        call(pb200_rows_contract(rows, (int)C, (int)Cout, fp(a), fp(gm), fpm(r.weights), fpm(r.bias), precision, ws.data_ptr(), nb,
+                                 s.stream),
+             "pb200_rows_contract");
+    } else {
+        r.weights = at::matmul(features.t(), gm);
+        if (!r.bias.defined()) r.bias = gm.sum(0, true);
+    }
+    return r;
+}
+
+Tensor flat(const Tensor& bias) { return bias.defined() ? bias.reshape({-1}).contiguous() : bias; }
+void check_stage(const Tensor& weights, int64_t C) {
+    check(weights, "depth_weights", 2, at::kFloat);
+    if (weights.size(0) != C) fail("depth_weights must have shape (channels, out_channels)");
+}
+// gradients that the node's edges ask for only
+#define PUT(i, t) do { if (task_should_compute_output(i)) out[i] = (t); } while (0)
+
+struct V2FLayer : Node {
+    SavedVariable input, filter, corners, face, rowptr, entries, weights, act, features, mean, invstd, gamma;
+    bool relu = false;
+    int precision = 0;
+    variable_list apply(variable_list&& grads) override {
+        variable_list out(6);
+        if (!grads[0].defined()) return out;
+        std::lock_guard<std::mutex> lock(mutex_);
+        const Tensor x = input.unpack(), eye = corners.unpack();
+        Scope s(x);
+        StageGrads r = stage_backward(s, upstream(grads), act.unpack(shared_from_this()), features.unpack(), weights.unpack(), NormStats{mean.unpack(), invstd.unpack()},
+                                      gamma.unpack(), relu,
+                                      task_should_compute_output(0) || task_should_compute_output(1), precision);
+        if (r.features.defined()) {
+            Tensor gf;
+            v2f_backward(s, r.features, x, filter.unpack(), face.unpack(), rowptr.unpack(), entries.unpack(), out[0], gf);
+            if (task_should_compute_output(1)) {
+                out[1] = s.floats({eye.size(1), x.size(1)});
+                call(pb200_corner_filter_backward((int)eye.size(1), (int)x.size(1), fp(eye), fp(gf), fpm(out[1]), s.stream),
+                     "pb200_corner_filter_backward");
+            }
+        }
+        PUT(2, r.weights);
+        PUT(3, r.bias);
+        PUT(4, r.gamma);
+        PUT(5, r.beta);
+        return out;
+    }
+    void release_variables() override {
+        std::lock_guard<std::mutex> lock(mutex_);
+        for (SavedVariable* v : {&input, &filter, &corners, &face, &rowptr, &entries, &weights, &act, &features, &mean, &invstd, &gamma}) v->reset_data();
+    }
+    std::string name() const override { return "VertexToFacetLayerBackward"; }
+};
+
+struct F2VLayer : Node {
+    SavedVariable input, filter, coeff, face, nf_count, vt_map, weights, act, features, mean, invstd, gamma;
+    bool relu = false;
+    int precision = 0;
+    variable_list apply(variable_list&& grads) override {
+        variable_list out(6);
+        if (!grads[0].defined()) return out;
+        std::lock_guard<std::mutex> lock(mutex_);
+        const Tensor x = input.unpack();
+        Scope s(x);
+        StageGrads r = stage_backward(s, upstream(grads), act.unpack(shared_from_this()), features.unpack(), weights.unpack(), NormStats{mean.unpack(), invstd.unpack()},
+                                      gamma.unpack(), relu,
+                                      task_should_compute_output(0) || task_should_compute_output(1), precision);
+        if (r.features.defined())
+            f2v_backward(s, r.features, x, filter.unpack(), coeff.unpack(), face.unpack(), nf_count.unpack(), vt_map.unpack(), out[0],
+                         out[1]);
+        PUT(2, r.weights);
+        PUT(3, r.bias);
+        PUT(4, r.gamma);
+        PUT(5, r.beta);
+        return out;
+    }
+    void release_variables() override {
+        std::lock_guard<std::mutex> lock(mutex_);
+        for (SavedVariable* v : {&input, &filter, &coeff, &face, &nf_count, &vt_map, &weights, &act, &features, &mean, &invstd, &gamma}) v->reset_data();
+    }
+    std::string name() const override { return "FacetToVertexLayerBackward"; }
+};
+
+struct RowsLayer : Node {
+    SavedVariable rows, weights, act, mean, invstd, gamma;
+    bool relu = false;
+    int precision = 0;
+    variable_list apply(variable_list&& grads) override {
+        variable_list out(5);
+        if (!grads[0].defined()) return out;
+        std::lock_guard<std::mutex> lock(mutex_);
+        const Tensor x = rows.unpack();
+        Scope s(x);
+        StageGrads r = stage_backward(s, upstream(grads), act.unpack(shared_from_this()), x, weights.unpack(), NormStats{mean.unpack(), invstd.unpack()},
+                                      gamma.unpack(), relu,
+                                      task_should_compute_output(0), precision);
+        PUT(0, r.features);
+        PUT(1, r.weights);
+        PUT(2, r.bias);
+        PUT(3, r.gamma);
+        PUT(4, r.beta);
+        return out;
+    }
+    void release_variables() override {
+        std::lock_guard<std::mutex> lock(mutex_);
+        for (SavedVariable* v : {&rows, &weights, &act, &mean, &invstd, &gamma}) v->reset_data();
+    }
+    std::string name() const override { return "RowsLayerBackward"; }
+};
+
+struct F2FLayer : Node {
+    SavedVariable input, filter, bary, cum, act, mean, invstd, gamma;
+    bool relu = false;
+    int precision = 0;
+    variable_list apply(variable_list&& grads) override {
+        variable_list out(5);
+        if (!grads[0].defined()) return out;
+        std::lock_guard<std::mutex> lock(mutex_);
+        const Tensor x = input.unpack(), a = act.unpack(shared_from_this()), g = aligned(upstream(grads));
+        const NormStats st{mean.unpack(), invstd.unpack()};
+        Scope s(x);
+        NormGrads n;
+        if (st.mean.defined()) {
+            n = norm_backward(s, g, a, st, gamma.unpack());
+            out[3] = n.gamma;
+            out[4] = n.beta;
+        }
+        Tensor gm;
+        masked_gradient(s, g, a, n, relu, gm, out[2]);
+        f2f_backward(s, gm, aligned(x), filter.unpack(), aligned(bary.unpack()), Tensor(), cum.unpack(), precision, out[0], out[1],
+                     task_should_compute_output(0));
+        return out;
+    }
+    void release_variables() override {
+        std::lock_guard<std::mutex> lock(mutex_);
+        for (SavedVariable* v : {&input, &filter, &bary, &cum, &act, &mean, &invstd, &gamma}) v->reset_data();
+    }
+    std::string name() const override { return "FacetToFacetLayerBackward"; }
+};
+
+Tail make_tail(bool relu, int mode, const OptTensor& gamma, const OptTensor& beta, const OptTensor& mean, const OptTensor& var,
+               const OptTensor& batches, double momentum, double eps) {
+    return Tail{mode, relu, or_undefined(gamma), or_undefined(beta), or_undefined(mean), or_undefined(var), or_undefined(batches),
+                momentum, eps};
+}
+#define TAIL_PARAMS bool relu, int norm_mode, const OptTensor &gamma, const OptTensor &beta, const OptTensor &running_mean, \
+        const OptTensor &running_var, const OptTensor &batches, double momentum, double eps, int precision
+#define TAIL_ARGS relu, norm_mode, gamma, beta, running_mean, running_var, batches, momentum, eps
+
+// vertex2facet with the filter corners @ spatial_weights, then the pointwise stage
+Tensor v2f_layer(const Tensor& x_in, const Tensor& face, const OptTensor& rowptr, const OptTensor& entries, const Tensor& corners,
+                 const Tensor& spatial, const Tensor& weights_in, const OptTensor& bias_in, TAIL_PARAMS) {
+    const Tail t = make_tail(TAIL_ARGS);
+    const Tensor bias0 = or_undefined(bias_in);
+    std::shared_ptr<V2FLayer> node;
+    if (torch::autograd::compute_requires_grad(x_in, spatial, weights_in, bias0, t.gamma, t.beta))
+        node = node_for<V2FLayer>(x_in, spatial, weights_in, bias0, t.gamma, t.beta);
+    at::AutoDispatchBelowADInplaceOrView below;
+    check(x_in, "input", 2, at::kFloat);
+    check(face, "face", 2, at::kInt);
+    check(spatial, "spatial_weights", 2, at::kFloat);
+    check_stage(weights_in, x_in.size(1));
+    const int64_t Nv = x_in.size(0), C = x_in.size(1), Nf = face.size(0), Cout = weights_in.size(1), K = corners.size(1);
+    if (spatial.size(0) != K || spatial.size(1) != C) fail("spatial_weights must have shape (number of bases, channels)");
+    if (Nf > 0 && face.size(1) != 3) fail("face must have shape (NfIn, 3)");
+    Scope s(x_in);
+    const Tensor x = aligned(x_in), bias = flat(bias0);
+    // the library product, whose rounding the separate modules share (norm.cu says why bits matter between layers)
+    const Tensor filter = at::matmul(corners, spatial).view({3, C, 1});
+    const size_t nb = pb200_vertex2facet_pointwise_workspace_bytes((int)C, precision);
+    Tensor ws = s.bytes(nb);
+    Staged r = run_stage(s, t, Nf, C, Cout, (bool)node, [&](float* out, const pb200_pointwise_extra* extra) {
+        call(pb200_vertex2facet_layer_forward(Nf, Nv, (int)C, (int)Cout, fp(x), fp(filter), ip(face), fp(weights_in), fp(bias), relu, out,
+                                              precision, extra, ws.data_ptr(), nb, s.stream),
+             "pb200_vertex2facet_layer_forward");
+    });
+    if (node) {
+        node->input = keep(x);
+        node->filter = keep(filter);
+        node->corners = keep(corners);
+        node->face = keep(face);
+        node->rowptr = keep(or_undefined(rowptr));
+        node->entries = keep(or_undefined(entries));
+        node->weights = keep(weights_in);
+        node->features = keep(r.features);
+        node->mean = keep(r.stats.mean);
+        node->invstd = keep(r.stats.invstd);
+        node->gamma = keep(t.gamma);
+        node->relu = relu;
+        node->precision = precision;
+        torch::autograd::set_history(r.out, node);
+        node->act = SavedVariable(r.act, r.act.is_same(r.out));
+    }
+    return r.out;
+}
+
+Tensor f2v_layer(const Tensor& x_in, const Tensor& face, const Tensor& nf_count, const Tensor& vt_map, const Tensor& rowptr,
+                 const Tensor& entries, const Tensor& coeff, const Tensor& filter_in, const Tensor& weights, const OptTensor& bias_in,
+                 TAIL_PARAMS) {
+    const Tail t = make_tail(TAIL_ARGS);
+    const Tensor bias0 = or_undefined(bias_in);
+    std::shared_ptr<F2VLayer> node;
+    if (torch::autograd::compute_requires_grad(x_in, filter_in, weights, bias0, t.gamma, t.beta))
+        node = node_for<F2VLayer>(x_in, filter_in, weights, bias0, t.gamma, t.beta);
+    at::AutoDispatchBelowADInplaceOrView below;
+    check_f2v(x_in, filter_in, coeff, face, nf_count, vt_map);
+    check_stage(weights, x_in.size(1));
+    const int64_t Nf = x_in.size(0), C = x_in.size(1), K = filter_in.size(0), NvOut = nf_count.size(0), Cout = weights.size(1);
+    if (filter_in.size(2) != 1) fail("filter must have shape (K, C, 1)");
+    Scope s(x_in);
+    const Tensor x = aligned(x_in), filter = aligned(filter_in), bias = flat(bias0);
+    const size_t nb = pb200_facet2vertex_pointwise_workspace_bytes(Nf, (int)C, precision);
+    Tensor ws = s.bytes(nb);
+    Staged r = run_stage(s, t, NvOut, C, Cout, (bool)node, [&](float* out, const pb200_pointwise_extra* extra) {
+        call(pb200_facet2vertex_layer_forward(Nf, NvOut, (int)C, (int)K, (int)Cout, fp(x), fp(filter), fp(coeff), ip(nf_count), ip(rowptr),
+                                              ip(entries), fp(weights), fp(bias), relu, out, precision, extra, ws.data_ptr(), nb, s.stream),
+             "pb200_facet2vertex_layer_forward");
+    });
+    if (node) {
+        node->input = keep(x);
+        node->filter = keep(filter);
+        node->coeff = keep(coeff);
+        node->face = keep(face);
+        node->nf_count = keep(nf_count);
+        node->vt_map = keep(vt_map);
+        node->weights = keep(weights);
+        node->features = keep(r.features);
+        node->mean = keep(r.stats.mean);
+        node->invstd = keep(r.stats.invstd);
+        node->gamma = keep(t.gamma);
+        node->relu = relu;
+        node->precision = precision;
+        torch::autograd::set_history(r.out, node);
+        node->act = SavedVariable(r.act, r.act.is_same(r.out));
+    }
+    return r.out;
+}
+
+Tensor rows_layer(const Tensor& rows_in, const Tensor& weights, const OptTensor& bias_in, TAIL_PARAMS) {
+    const Tail t = make_tail(TAIL_ARGS);
+    const Tensor bias0 = or_undefined(bias_in);
+    std::shared_ptr<RowsLayer> node;
+    if (torch::autograd::compute_requires_grad(rows_in, weights, bias0, t.gamma, t.beta))
+        node = node_for<RowsLayer>(rows_in, weights, bias0, t.gamma, t.beta);
+    at::AutoDispatchBelowADInplaceOrView below;
+    check(rows_in, "inputs", 2, at::kFloat);
+    check(weights, "weights", 2, at::kFloat);
+    const int64_t N = rows_in.size(0), C = rows_in.size(1), Cout = weights.size(1);
+    if (weights.size(0) != C) fail("weights must have shape (in_channels, out_channels)");
+    Scope s(rows_in);
+    const Tensor rows = aligned(rows_in), bias = flat(bias0);
+    const size_t nb = pb200_masked_rows_matmul_workspace_bytes((int)C, precision);
+    Tensor ws = s.bytes(nb);
+    Staged r = run_stage(s, t, N, C, Cout, false, [&](float* out, const pb200_pointwise_extra* extra) {
+        call(pb200_rows_layer_forward(N, (int)C, (int)Cout, fp(rows), fp(weights), fp(bias), relu, out, precision, extra, ws.data_ptr(), nb,
+                                      s.stream),
+             "pb200_rows_layer_forward");
+    });
+    if (node) {
+        node->rows = keep(rows);
+        node->weights = keep(weights);
+        node->mean = keep(r.stats.mean);
+        node->invstd = keep(r.stats.invstd);
+        node->gamma = keep(t.gamma);
+        node->relu = relu;
+        node->precision = precision;
+        torch::autograd::set_history(r.out, node);
+        node->act = SavedVariable(r.act, r.act.is_same(r.out));
+    }
+    return r.out;
+}
+
+// facet2facet over the samples of every face (`counts` per face), then bias, ReLU or nothing, normalisation
+Tensor f2f_layer(const Tensor& input, const Tensor& filter, const Tensor& bary, const Tensor& counts, const Tensor& bias0, TAIL_PARAMS) {
+    const Tail t = make_tail(TAIL_ARGS);
+    std::shared_ptr<F2FLayer> node;
+    if (torch::autograd::compute_requires_grad(input, filter, bias0, t.gamma, t.beta))
+        node = node_for<F2FLayer>(input, filter, bias0, t.gamma, t.beta);
+    at::AutoDispatchBelowADInplaceOrView below;
+    check_f2f(input, filter, bary);
+    const Tensor cum = at::cumsum(counts, 0, at::kInt), bias = flat(bias0);
+    check(cum, "num_texture", 1, at::kInt);
+    Scope s(input);
+    Tensor act = f2f_forward(s, aligned(input), filter, bary, cum, precision);
+    const int64_t rows = act.size(0), C = act.size(1);
+    Tensor out = act;
+    NormStats st;
+    Tensor partial = s.floats({pb200_norm_parts(rows, (int)C), 3, C});
+    int parts = 0;
+    call(pb200_bias_act_stats(rows, (int)C, fpm(act), fp(bias), relu, fpm(partial), &parts, s.stream), "pb200_bias_act_stats");
+    if (t.mode == NORM_BATCH) {
+        st = finalize(s, t, C, parts, partial);
+        out = normalise(s, t, act, st);
+    } else if (t.mode == NORM_RUNNING) {
+        const NormStats running{t.running_mean, s.floats({C})};
+        call(pb200_norm_invstd((int)C, fp(t.running_var), (float)t.eps, nullptr, fpm(running.invstd), s.stream), "pb200_norm_invstd");
+        out = normalise(s, t, act, running);
+    }
+    if (node) {
+        node->input = keep(input);
+        node->filter = keep(filter);
+        node->bary = keep(bary);
+        node->cum = keep(cum);
+        node->mean = keep(st.mean);
+        node->invstd = keep(st.invstd);
+        node->gamma = keep(t.gamma);
+        node->relu = relu;
+        node->precision = precision;
+        torch::autograd::set_history(out, node);
+        node->act = SavedVariable(act, act.is_same(out));
+    }
+    return out;
+}
+
+// ------------------------------------------------------------------------------------------- pooling over clusters
+struct Pool : Node {
+    enum Kind { MAX, AVG, UNPOOL } kind = MAX;
+    SavedVariable max_index, vt_replace;
+    Tensor key, rowptr, members;                               // cluster arrays of the cache: never written in place
+    std::vector<int64_t> in_shape;
+    variable_list apply(variable_list&& grads) override {
+        variable_list out(1);
+        if (!grads[0].defined()) return out;
+        std::lock_guard<std::mutex> lock(mutex_);
+        const Tensor g = upstream(grads);
+        Scope s(g);
+        out[0] = s.floats(in_shape);
+        const int64_t n = in_shape[0], C = in_shape[1], m = g.size(0);
+        if (kind == MAX)
+            call(pb200_mesh_max_pool_backward_clusters(n, m, (int)C, ip(max_index.unpack()), fp(g), ip(key), ip(rowptr), fpm(out[0]), s.stream),
+                 "pb200_mesh_max_pool_backward_clusters");
+        else if (kind == AVG)
+            call(pb200_mesh_avg_pool_backward(n, m, (int)C, fp(g), ip(vt_replace.unpack()), ip(key), fpm(out[0]), s.stream),
+                 "pb200_mesh_avg_pool_backward");
+        else
+            call(pb200_mesh_unpool_backward(n, m, (int)C, fp(g), ip(rowptr), ip(members), fpm(out[0]), s.stream),
+                 "pb200_mesh_unpool_backward");
+        return out;
+    }
+    void release_variables() override {
+        std::lock_guard<std::mutex> lock(mutex_);
+        max_index.reset_data();
+        vt_replace.reset_data();
+        key.reset(); rowptr.reset(); members.reset();
+    }
+    std::string name() const override { return "MeshPoolBackward"; }
+};
+
+std::shared_ptr<Pool> pool_node(Pool::Kind kind, const Tensor& input, const Tensor& key, const Tensor& rowptr, const Tensor& members) {
+    std::shared_ptr<Pool> node;
+    if (torch::autograd::compute_requires_grad(input)) {
+        node = node_for<Pool>(input);
+        node->kind = kind;
+        node->in_shape = input.sizes().vec();
+        node->key = key; node->rowptr = rowptr; node->members = members;
+    }
+    return node;
+}
+
+Tensor max_pool(const Tensor& input, int64_t nv_out, const Tensor& key, const Tensor& rowptr, const Tensor& members) {
+    auto node = pool_node(Pool::MAX, input, key, rowptr, members);
+    Tensor out, index;
+    {
+        at::AutoDispatchBelowADInplaceOrView below;
+        Scope s(input);
+        const int64_t C = input.size(1);
+        out = s.floats({nv_out, C});
+        index = at::empty({nv_out, C}, s.f32.dtype(at::kInt));
+        call(pb200_mesh_max_pool_forward(input.size(0), nv_out, (int)C, fp(input), ip(rowptr), ip(members), fpm(out),
+                                         static_cast<int32_t*>(index.data_ptr()), s.stream),
+             "pb200_mesh_max_pool_forward");
+    }
+    if (node) {
+        node->max_index = keep(index);
+        torch::autograd::set_history(out, node);
+    }
+    return out;
+}
+
+Tensor avg_pool(const Tensor& input, int64_t nv_out, const Tensor& vt_replace, const Tensor& key, const Tensor& rowptr,
+                const Tensor& members) {
+    auto node = pool_node(Pool::AVG, input, key, rowptr, members);
+    Tensor out;
+    {
+        at::AutoDispatchBelowADInplaceOrView below;
+        Scope s(input);
+        out = s.floats({nv_out, input.size(1)});
+        call(pb200_mesh_avg_pool_forward(input.size(0), nv_out, (int)input.size(1), fp(input), ip(vt_replace), ip(rowptr), ip(members),
+                                         fpm(out), s.stream),
+             "pb200_mesh_avg_pool_forward");
+    }
+    if (node) {
+        node->vt_replace = keep(vt_replace);
+        torch::autograd::set_history(out, node);
+    }
+    return out;
+}
+
+Tensor unpool(const Tensor& input, int64_t nv_fine, const Tensor& key, const Tensor& rowptr, const Tensor& members) {
+    auto node = pool_node(Pool::UNPOOL, input, key, rowptr, members);
+    Tensor out;
+    {
+        at::AutoDispatchBelowADInplaceOrView below;
+        Scope s(input);
+        out = s.floats({nv_fine, input.size(1)});
+        call(pb200_mesh_unpool_forward(input.size(0), nv_fine, (int)input.size(1), fp(input), ip(key), fpm(out), s.stream),
+             "pb200_mesh_unpool_forward");
+    }
+    if (node) torch::autograd::set_history(out, node);
+    return out;
+}
+
+struct SegmentMean : Node {
+    Tensor ends;                                               // of the cache: never written in place
+    int64_t rows = 0, channels = 0;
+    variable_list apply(variable_list&& grads) override {
+        variable_list out(1);
+        if (!grads[0].defined()) return out;
+        const Tensor g = upstream(grads);
+        Scope s(g);
+        out[0] = s.floats({rows, channels});
+        call(pb200_segment_mean_backward(rows, (int)g.size(0), (int)channels, fp(g), ends.data_ptr<int64_t>(), fpm(out[0]), s.stream),
+             "pb200_segment_mean_backward");
+        return out;
+    }
+    std::string name() const override { return "SegmentMeanBackward"; }
+};
+
+Tensor segment_mean(const Tensor& input, const Tensor& ends) {
+    std::shared_ptr<SegmentMean> node;
+    if (torch::autograd::compute_requires_grad(input)) node = node_for<SegmentMean>(input);
+    Tensor out;
+    {
+        at::AutoDispatchBelowADInplaceOrView below;
+        Scope s(input);
+        const int64_t N = input.size(0), C = input.size(1), B = ends.size(0);
+        out = s.floats({B, C});
+        const size_t nb = pb200_segment_mean_workspace_bytes(N, (int)B, (int)C);
+        Tensor ws = s.bytes(nb);
+        call(pb200_segment_mean(N, (int)B, (int)C, fp(input), ends.data_ptr<int64_t>(), fpm(out), ws.data_ptr(), nb, s.stream),
+             "pb200_segment_mean");
+    }
+    if (node) {
+        node->ends = ends;
+        node->rows = input.size(0);
+        node->channels = input.size(1);
+        torch::autograd::set_history(out, node);
+    }
+    return out;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -450,4 +1037,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("facet2facet", &facet2facet);
     m.def("facet2facet_shared_rows", &facet2facet_shared_rows);
     m.def("conv_block", &conv_block);
+    m.def("v2f_layer", &v2f_layer);
+    m.def("f2v_layer", &f2v_layer);
+    m.def("rows_layer", &rows_layer);
+    m.def("f2f_layer", &f2f_layer);
+    m.def("max_pool", &max_pool);
+    m.def("avg_pool", &avg_pool);
+    m.def("unpool", &unpool);
+    m.def("segment_mean", &segment_mean);
 }

@@ -25,3 +25,20 @@ def sph_harm_coeff(L: int, cart_coords: torch.Tensor) -> torch.Tensor:
         out = torch.empty(xyz.shape[0], (L + 1) ** 2, dtype=torch.float32, device=dev)
         _lib.call("pb200_sph_harm_coeff", xyz.shape[0], L, ptr(xyz), ptr(out), stream_ptr(dev))
     return out
+
+
+_corners = {}
+
+
+def corner_basis(L: int, device) -> torch.Tensor:
+    """sph_harm_coeff(L, eye(3)): the basis at the three corner directions, (3, (L+1)^2), a constant of the degree that every
+    vertex2facet layer multiplies its weights with.  One table per degree and device is kept; it is complete before it is
+    handed out, so every stream may read it."""
+    table = _corners.get((L, device))
+    if table is None:
+        table = sph_harm_coeff(L, torch.eye(3, device=device))
+        if torch.cuda.is_current_stream_capturing():      # memory of a graph's pool: good for this graph only
+            return table
+        torch.cuda.current_stream(device).synchronize()
+        _corners[(L, device)] = table
+    return table

@@ -12,7 +12,9 @@ import torch
 import torch.nn as nn
 
 from .pi_modules import conv3d, fused, pool3d, unpool3d
-from ..math_utils import sph_harm_coeff
+from .. import _lib
+from ..math_utils import corner_basis, sph_harm_coeff
+from ..topology import sample_ends
 
 
 _fusion = True
@@ -24,6 +26,10 @@ def set_fusion(on: bool) -> None:
     reference's sequence of separate kernels.  Batch norm stays a torch module either way."""
     global _fusion
     _fusion = bool(on)
+
+
+def _plain_activation(fn):
+    return fn is None or type(fn) is nn.ReLU
 
 
 def _filter_variable_(shape, stddev=1.0, use_xavier=True):
@@ -40,6 +46,31 @@ class SphHarmCoeff(nn.Module):
 
     def __call__(self, cart_coords):
         return sph_harm_coeff(self.l, cart_coords)
+
+
+def _norm_args(bn, rows, device, needs_grad):
+    """How the native layers run the module's batch norm: (mode, weight, bias, running mean, running var, batches, momentum,
+    eps) with mode 1 = statistics of the batch, 2 = running statistics, or None when the torch module has to run itself (a
+    subclass or a hook, cumulative averages, parameters elsewhere, inference statistics under autograd, a single row)."""
+    if (type(bn) is not nn.BatchNorm1d or bn._forward_hooks or bn._forward_pre_hooks or bn._backward_hooks or
+            bn._backward_pre_hooks or _has_global_hooks()):
+        return None
+    p, b = bn._parameters, bn._buffers
+    weight, bias, mean, var, batches = p["weight"], p["bias"], b["running_mean"], b["running_var"], b["num_batches_tracked"]
+    for t in (weight, bias, mean, var):
+        if t is not None and (t.device != device or t.dtype != torch.float32 or not t.is_contiguous()):
+            return None
+    if (mean is None) != (var is None) or (mean is None) != (batches is None):
+        return None
+    if bn.training or mean is None:
+        if rows < 2 or (mean is not None and (bn.momentum is None or batches.device != device or batches.dtype != torch.int64)):
+            return None
+        return 1, weight, bias, mean, var, batches, bn.momentum or 0.0, bn.eps
+    return None if needs_grad else (2, weight, bias, mean, var, None, 0.0, bn.eps)
+
+
+_has_global_hooks = nn.modules.module._has_any_global_hook
+_NO_NORM = (0, None, None, None, None, None, 0.0, 0.0)
 
 
 class _PointwiseTail(nn.Module):
@@ -63,8 +94,17 @@ class _PointwiseTail(nn.Module):
     def _fusable(self, x, channels, multiplier):
         return _fusion and fused.eligible(x, channels, multiplier, self.activation_fn)
 
-    def _after_fused(self, x):
-        return self.BatchNorm(x) if self.with_bn else x
+    def _native(self, rows, x, run):
+        """run(relu, norm mode, norm arrays ..., precision) = the whole layer as one native call; batch norm included where
+        _norm_args allows it, by the torch module behind it otherwise."""
+        norm = _NO_NORM
+        if self.with_bn:
+            needs_grad = torch.is_grad_enabled() and (x.requires_grad or any(q.requires_grad for q in self._parameters.values()))
+            norm = _norm_args(self._modules["BatchNorm"], rows, x.device, needs_grad)
+        relu = self.activation_fn is not None
+        if norm is None:
+            return self.BatchNorm(run(relu, *_NO_NORM))
+        return run(relu, *norm)
 
 
 class F2FConv3d(_PointwiseTail):
@@ -83,6 +123,10 @@ class F2FConv3d(_PointwiseTail):
     def forward(self, input_texture, bary_coeff, num_texture):
         assert self.in_channels == input_texture.shape[-1]
         assert self.num_basis == bary_coeff.shape[-1]
+        if input_texture.is_cuda and _fusion and _plain_activation(self.activation_fn) and num_texture.shape[0] > 0:
+            bary_coeff.requires_grad = False
+            return self._native(num_texture.shape[0], input_texture, lambda *tail: _lib.ops.f2f_layer(
+                input_texture, self.weights, bary_coeff, num_texture, self.biases, *tail, conv3d._f2f_precision))
         running = torch.cumsum(num_texture, dim=0, dtype=torch.int)   # the operator wants the running count
         return self._tail(conv3d.facet2facet(input_texture, self.weights, bary_coeff, running))
 
@@ -103,11 +147,11 @@ class V2FConv3d(_PointwiseTail):
         self._init_tail(out_channels, activation_fn, with_bn, bn_momentum)
 
     def forward(self, inputs, face):
-        corners = sph_harm_coeff(self.L, torch.eye(3, device=inputs.device))
-        spatial = (corners @ self.spatial_weights).reshape(3, self.in_channels, self.multiplier)
+        corners = corner_basis(self.L, inputs.device)
         if self._fusable(inputs, self.in_channels, self.multiplier):
-            return self._after_fused(fused.vertex2facet_pointwise(inputs, spatial, face, self.depth_weights, self.biases,
-                                                                  self.activation_fn is not None))
+            return self._native(face.shape[0], inputs, lambda *tail: fused.vertex2facet_layer(
+                inputs, face, corners, self.spatial_weights, self.depth_weights, self.biases, tail))
+        spatial = (corners @ self.spatial_weights).reshape(3, self.in_channels, self.multiplier)
         feats = conv3d.vertex2facet(inputs, spatial, face)
         return self._tail(feats @ self.depth_weights)
 
@@ -129,9 +173,8 @@ class F2VConv3d(_PointwiseTail):
 
     def forward(self, inputs, face, nf_count, vt_map, filt_coeff):
         if self._fusable(inputs, self.in_channels, self.multiplier):
-            return self._after_fused(fused.facet2vertex_pointwise(inputs, self.spatial_weights, filt_coeff, face, nf_count,
-                                                                  vt_map, self.depth_weights, self.biases,
-                                                                  self.activation_fn is not None))
+            return self._native(nf_count.shape[0], inputs, lambda *tail: fused.facet2vertex_layer(
+                inputs, self.spatial_weights, filt_coeff, face, nf_count, vt_map, self.depth_weights, self.biases, tail))
         feats = conv3d.facet2vertex(inputs, self.spatial_weights, filt_coeff, face, nf_count, vt_map)
         return self._tail(feats @ self.depth_weights)
 
@@ -176,7 +219,7 @@ class Unpool3d(nn.Module):
         return unpool3d.interpolate(inputs, vt_replace, vt_map)
 
 
-class PerItemConv3d(nn.Module):
+class PerItemConv3d(_PointwiseTail):
     """Pointwise layer (per vertex, per facet, per point): matmul -> + biases -> activation -> batch norm, the
     reference's module of the same name (picasso/mesh/layers.py:198-240), parameters `weights`
     (in_channels, out_channels), `biases` (1, out_channels), `BatchNorm`.  With fusion on, an input width that is
@@ -188,20 +231,14 @@ class PerItemConv3d(nn.Module):
         super().__init__()
         self.in_channels, self.out_channels = in_channels, out_channels
         self.use_xavier, self.stddev = use_xavier, stddev
-        self.with_bn, self.activation_fn = with_bn, activation_fn
-        if with_bn:
-            self.BatchNorm = nn.BatchNorm1d(out_channels, eps=0.001, momentum=bn_momentum)
         self.weights = _filter_variable_([in_channels, out_channels], stddev=stddev, use_xavier=use_xavier)
-        self.biases = nn.Parameter(torch.zeros(1, out_channels))
+        self._init_tail(out_channels, activation_fn, with_bn, bn_momentum)
 
     def forward(self, inputs):
-        if _fusion and inputs.dim() == 2 and fused.eligible(inputs, self.in_channels, 1, self.activation_fn):
-            outputs = fused.rows_pointwise(inputs.contiguous(), self.weights, self.biases, self.activation_fn is not None)
-        else:
-            outputs = torch.matmul(inputs, self.weights) + self.biases
-            if self.activation_fn is not None:
-                outputs = self.activation_fn(outputs)
-        return self.BatchNorm(outputs) if self.with_bn else outputs
+        if inputs.dim() == 2 and self._fusable(inputs, self.in_channels, 1):
+            return self._native(inputs.shape[0], inputs, lambda *tail: fused.rows_layer(
+                inputs.contiguous(), self.weights, self.biases, tail))
+        return self._tail(torch.matmul(inputs, self.weights))
 
 
 class GlobalPool3d(nn.Module):
@@ -214,10 +251,12 @@ class GlobalPool3d(nn.Module):
         self.method = method
 
     def forward(self, inputs, nv_in):
-        lengths = nv_in.to(torch.int64)
         if self.method == 'avg':
-            return torch.segment_reduce(inputs, 'mean', lengths=lengths)
+            if inputs.is_cuda and inputs.dtype == torch.float32 and inputs.dim() == 2 and nv_in.dim() == 1 and nv_in.device == inputs.device:
+                return _lib.ops.segment_mean(inputs.contiguous(), sample_ends(nv_in, inputs.shape[0]))
+            return torch.segment_reduce(inputs, 'mean', lengths=nv_in.to(torch.int64))
         if self.method == 'max':
+            lengths = nv_in.to(torch.int64)
             values = torch.segment_reduce(inputs, 'max', lengths=lengths)
             # position of the first vertex that attains the maximum, as an index into `inputs`
             B = lengths.shape[0]

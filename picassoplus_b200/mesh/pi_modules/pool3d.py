@@ -111,7 +111,13 @@ class MaxPoolFunction(torch.autograd.Function):
 
 
 def maxPool(input, vt_replace, vt_map, vt_out):
-    return MaxPoolFunction.apply(input, vt_replace, vt_map, vt_out)
+    _pool_checks(input, vt_replace, vt_map, vt_out)
+    vt_replace.requires_grad = False
+    vt_map.requires_grad = False
+    if vt_out.is_leaf:
+        vt_out.requires_grad = False
+    cl = cluster_csr(vt_replace, vt_map, vt_out.shape[0])
+    return _lib.ops.max_pool(input, vt_out.shape[0], cl.key, cl.rowptr, cl.members)
 
 
 class AvgPoolFunction(torch.autograd.Function):
@@ -132,4 +138,10 @@ class AvgPoolFunction(torch.autograd.Function):
 
 
 def avgPool(input, vt_replace, vt_map, vt_out):
-    return AvgPoolFunction.apply(input, vt_replace, vt_map, vt_out)
+    _pool_checks(input, vt_replace, vt_map, vt_out)
+    vt_replace.requires_grad = False
+    vt_map.requires_grad = False
+    if vt_out.is_leaf:
+        vt_out.requires_grad = False
+    cl = cluster_csr(vt_replace, vt_map, vt_out.shape[0])
+    return _lib.ops.avg_pool(input, vt_out.shape[0], vt_replace, cl.key, cl.rowptr, cl.members)

@@ -66,4 +66,12 @@ class InterpolateFunction(torch.autograd.Function):
 
 
 def interpolate(input, vt_replace, vt_map):
-    return InterpolateFunction.apply(input, vt_replace, vt_map)
+    _check(input, "input", 2, torch.float32)
+    _check(vt_replace, "vt_replace", 1, torch.int32)
+    _check(vt_map, "vt_map", 1, torch.int32)
+    if vt_replace.shape[0] != vt_map.shape[0]:
+        raise RuntimeError("vt_replace and vt_map must have one entry per fine vertex")
+    vt_replace.requires_grad = False
+    vt_map.requires_grad = False
+    cl = cluster_csr(vt_replace, vt_map, input.shape[0])
+    return _lib.ops.unpool(input, vt_map.shape[0], cl.key, cl.rowptr, cl.members)

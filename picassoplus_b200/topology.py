@@ -392,6 +392,37 @@ def face_means_sph_harm(L: int, sample_xyz: torch.Tensor, num_interior: torch.Te
     return fm
 
 
+class SampleEnds:
+    """Running number of rows up to and including every sample (B,) int64."""
+
+    def __init__(self, ends, keep, versions):
+        self.ends = ends
+        self._keep = keep
+        self._versions = versions
+        self.nbytes = 8 * ends.numel()
+
+
+def sample_ends(counts: torch.Tensor, n_rows: int) -> torch.Tensor:
+    """Cached running totals of the samples' row counts; same cache, budget and validation modes as vertex_csr.  They must
+    add up to n_rows."""
+    slot = ("samples", counts.device.index, counts.data_ptr(), counts.dtype, counts.shape[0], int(n_rows))
+    versions = (counts._version,)
+    hit = _lookup(slot, versions)
+    if hit is not None:
+        return hit.ends
+    ends = torch.cumsum(counts.detach(), 0, dtype=torch.int64)
+    bad = ends[-1:] != n_rows if counts.shape[0] else torch.full((1,), n_rows != 0, device=counts.device)
+    bad = bad | (counts < 0).any()
+    msg = "the samples' row counts must be non-negative and add up to the number of rows"
+    if _validation == "deferred":
+        with _lock:
+            _deferred.append((bad.to(torch.int32), msg))
+    elif bool(bad.item()):
+        raise RuntimeError(msg)
+    _store(slot, SampleEnds(ends, (counts,), versions))
+    return ends
+
+
 def check_num_interior(num_interior: torch.Tensor, nik: int) -> None:
     """Validates a running sample count (non-decreasing, inside [0, nik], ends at nik) on the
     device: raises in 'sync' mode, queues the status word in 'deferred' mode.  The facet2facet

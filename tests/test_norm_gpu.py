@@ -1,0 +1,98 @@
+"""Batch normalisation inside the native layers and the per-sample mean, against torch in fp64 at the sizes where their
+kernels' work split changes (one row per block, remainders of the unrolled loops, channels that are no multiple of four,
+more than one chunk of 32 thread columns)."""
+import pytest
+import torch
+import torch.nn as nn
+
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def norm_err(a, b):
+    a, b = a.detach().double(), b.detach().double()
+    return float((a - b).norm() / b.norm())
+
+
+@pytest.mark.parametrize("rows,C", [(2, 8), (33, 5), (1000, 32), (4097, 100), (70001, 128), (513, 260)])
+@pytest.mark.parametrize("relu", [True, False])
+def test_rows_layer_with_batch_norm(rows, C, relu):
+    """PerItemConv3d in training (two steps: running statistics), then in inference, forward and backward."""
+    from picassoplus_b200.mesh.layers import PerItemConv3d
+    torch.manual_seed(rows + C)
+    m = PerItemConv3d(16, C, activation_fn=nn.ReLU() if relu else None).cuda().train()
+    with torch.no_grad():
+        m.biases.normal_(0, 0.3)
+        m.BatchNorm.weight.uniform_(0.5, 1.5)
+        m.BatchNorm.bias.normal_()
+    bn = nn.BatchNorm1d(C, eps=1e-3).cuda().double().train()
+    bn.load_state_dict(m.BatchNorm.state_dict())
+    for step in range(2):
+        x = (torch.randn(rows, 16, device="cuda") * 0.5 + 1.0).requires_grad_()
+        g = torch.randn(rows, C, device="cuda")
+        y = m(x)
+        got = torch.autograd.grad(y, [x, m.weights, m.biases, m.BatchNorm.weight, m.BatchNorm.bias], g)
+        xd = x.detach().double().requires_grad_()
+        p = [t.detach().double().requires_grad_() for t in (m.weights, m.biases)]
+        z = xd @ p[0] + p[1]
+        # a pre-activation within rounding of zero may fall on either side of the ReLU: gradients get more room with it
+        act = torch.relu(z) if relu else z
+        want_y = bn(act)
+        want = torch.autograd.grad(want_y, [xd, p[0], p[1], bn.weight, bn.bias], g.double())
+        assert rel_err(y, want_y) <= 2e-4
+        for i, (a, b) in enumerate(zip(got, want)):
+            if rows > 2 and (relu or i != 2):       # two rows normalise to +-1: rounding noise; without ReLU the bias has no gradient
+                assert norm_err(a, b) <= (2e-2 if relu else 1e-3)
+    assert rel_err(m.BatchNorm.running_mean, bn.running_mean) <= 1e-4
+    assert rel_err(m.BatchNorm.running_var, bn.running_var) <= 1e-4
+    assert int(m.BatchNorm.num_batches_tracked) == 2
+    m.eval(), bn.eval()
+    x = torch.randn(rows, 16, device="cuda")
+    z = x.double() @ m.weights.double() + m.biases.double()
+    want = bn(torch.relu(z) if relu else z)
+    with torch.no_grad():
+        assert rel_err(m(x), want) <= 2e-4          # running statistics inside the kernel
+    assert rel_err(m(x), want) <= 2e-4              # under autograd: the torch module behind the kernel
+
+
+@pytest.mark.parametrize("rows,C", [(2, 3), (777, 12), (50000, 32)])
+def test_facet_layer_statistics(rows, C):
+    """F2FConv3d: bias, ReLU and statistics in one pass, running and batch statistics, data without gradient."""
+    from picassoplus_b200.mesh.layers import F2FConv3d
+    torch.manual_seed(rows)
+    m = F2FConv3d(3, C, 2).cuda().train()
+    counts = torch.randint(1, 4, (rows,), device="cuda", dtype=torch.int32)
+    n = int(counts.sum())
+    tex, bary = torch.rand(n, 3, device="cuda"), torch.randn(n, 9, device="cuda")
+    seg = torch.repeat_interleave(torch.arange(rows, device="cuda"), counts)
+    A = torch.zeros(rows, 9, 3, device="cuda", dtype=torch.float64).index_add_(0, seg, bary.double()[:, :, None] * tex.double()[:, None])
+    z = torch.einsum("fdc,ocd->fo", A / counts[:, None, None], m.weights.double()) + m.biases.double()
+    bn = nn.BatchNorm1d(C, eps=1e-3).cuda().double().train()
+    want = bn(torch.relu(z))
+    got = m(tex, bary, counts)
+    assert rel_err(got, want) <= 1e-3 if rows == 2 else rel_err(got, want) <= 2e-4
+    assert rel_err(m.BatchNorm.running_var, bn.running_var) <= 1e-4
+    g = torch.randn(rows, C, device="cuda")
+    gw, = torch.autograd.grad(got, [m.weights], g)
+    if rows > 2:
+        gw_want, = torch.autograd.grad(want, [m.weights], g.double())
+        assert norm_err(gw, gw_want) <= 2e-2
+    m.eval(), bn.eval()
+    with torch.no_grad():
+        assert rel_err(m(tex, bary, counts), bn(torch.relu(z))) <= 2e-4
+
+
+@pytest.mark.parametrize("lengths,C", [([1], 1), ([5, 1, 1000, 3], 40), ([512, 512, 511, 513], 128), ([100] * 130, 33), ([70000], 4)])
+def test_global_mean(lengths, C):
+    from picassoplus_b200.mesh.layers import GlobalPool3d
+    x = torch.randn(sum(lengths), C, device="cuda").requires_grad_()
+    nv = torch.tensor(lengths, device="cuda", dtype=torch.int32)
+    out = GlobalPool3d("avg")(x, nv)
+    g = torch.randn_like(out)
+    gx, = torch.autograd.grad(out, x, g)
+    parts = torch.split(x.detach().double(), lengths)
+    assert rel_err(out, torch.stack([p.mean(0) for p in parts])) <= 1e-5
+    assert rel_err(gx, torch.repeat_interleave(g / nv[:, None], nv.long(), 0)) <= 1e-6
+    with pytest.raises(RuntimeError):
+        GlobalPool3d("avg")(x, nv + 1)
