@@ -486,14 +486,29 @@ int pb200_pcloud_conv3d_backward(int64_t Np, int64_t Mp, int64_t Nout, int F, in
  * Edges of a face that names a vertex twice are no candidates.
  * edgeCost (3*Nf floats, may be NULL) receives the cost of every distinct edge in (lower, higher) order;
  * info (HOST pointer to 4 int64, may be NULL) = {distinct edges, matching rounds run on the whole grid, edges
- * handed to the single-block finish, 0}.  The call synchronises the stream a few times (it reads back three
- * counters and the 2*B sample totals) and returns PB200_EINDEX for a vertex id outside [0, Nv). */
+ * handed to the single-block finish, 0} (batches of small samples run without a grid: 0, 0).  The call synchronises the
+ * stream twice (it reads back the 2*B sample totals, and a status word at the end) and returns PB200_EINDEX for a vertex id
+ * outside [0, Nv) or a face that joins vertices of two samples. */
 size_t pb200_mesh_simplify_workspace_bytes(int64_t B, int64_t Nv, int64_t Nf);
 int pb200_mesh_simplify(int useArea, float wgtBnd, int64_t B, int64_t D, int64_t Nv, int64_t Nf,
                         const int32_t* nvIn, const int32_t* mfIn, const int32_t* nv2Remove, const float* vertexIn,
                         const int32_t* faceIn, const float* planeIn, int32_t* nvOut, int32_t* mfOut, float* vertexOut,
                         int32_t* faceOut, int32_t* vtReplace, int32_t* vtMap, uint8_t* isDegenerate, float* edgeCost,
                         int64_t* info, void* workspace, size_t workspace_bytes, void* stream);
+/* The same pass in two halves for callers that go on with the decimated meshes alone (the pass loop of mesh_decimation,
+ * picasso/mesh/pi_modules/decimate.py:30-46): begin queues everything up to the sizes of the result without a
+ * synchronisation, finish writes the kept vertices and faces behind one another (new ids) with the faces' geometry.
+ * nv, mf, target: vertices, faces and wanted vertices of every sample (B each; nv and mf must add up to Nv and Nf),
+ * mostFaces = the largest of mf.  Between the two calls the caller reads nvOut, mfOut (B each) and *status (0, PB200_EINDEX, 1 =
+ * a face joins vertices of two samples, PB200_ECUDA) and allocates vertexOut (sum nvOut, D), faceOut (sum mfOut, 3), geometryOut
+ * (sum mfOut, 5).  Same workspace (pb200_mesh_simplify_workspace_bytes), untouched in between. */
+int pb200_decimate_begin(int useArea, float wgtBnd, int64_t B, int64_t D, int64_t Nv, int64_t Nf, int64_t mostFaces, const int32_t* nv,
+                         const int32_t* mf, const int32_t* target, const float* vertexIn, const int32_t* faceIn, const float* planeIn,
+                         int32_t* nvOut, int32_t* mfOut, int32_t* status, int32_t* vtReplace, int32_t* vtMap, void* workspace,
+                         size_t workspace_bytes, void* stream);
+int pb200_decimate_finish(int64_t B, int64_t D, int64_t Nv, int64_t Nf, const float* vertexIn, const int32_t* vtReplace,
+                          const int32_t* vtMap, float* vertexOut, int32_t* faceOut, float* geometryOut, void* workspace,
+                          size_t workspace_bytes, void* stream);
 /* Clusters of a mesh A (repA, mapA over its nvA vertices) merged with the clusters of its decimated
  * version B (repB, mapB over nvB vertices) into clusters of A over the vertices B kept.  Replaces
  * combineClustersLauncher (decimate_gpu.cu:750-812; binding CombineClusters, `combine_clusters`).

@@ -97,6 +97,8 @@ SIGNATURES = {
     "pb200_mesh_simplify_workspace_bytes": (sz, [i64, i64, i64]),
     "pb200_mesh_simplify": (i32, [i32, f32, i64, i64, i64, i64, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp,
                                   vp, sz, vp]),
+    "pb200_decimate_begin": (i32, [i32, f32, i64, i64, i64, i64, i64, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, sz, vp]),
+    "pb200_decimate_finish": (i32, [i64, i64, i64, i64, vp, vp, vp, vp, vp, vp, vp, sz, vp]),
     "pb200_combine_clusters": (i32, [i64, i64, vp, vp, vp, vp, vp, vp, vp, vp, sz, vp]),
     "pb200_rows_pointwise_forward": (i32, [i64, i32, i32, vp, vp, vp, i32, vp, i32, vp, sz, vp]),
     "pb200_vertex2facet_layer_forward": (i32, [i64, i64, i32, i32, vp, vp, vp, vp, vp, i32, vp, i32, vp, vp, sz, vp]),

@@ -2,6 +2,7 @@
 // scatter-shaped kernel pulls through, triangle geometry, and row expansion by sample
 // counts.  All integer work; results are bit-exact and independent of scheduling.
 #include "common.cuh"
+#include "scan.cuh"
 #include "sph_core.cuh"
 
 namespace pb {
@@ -19,57 +20,6 @@ __global__ void corner_count_kernel(int64_t ncorner, int64_t NvIn, int64_t NvOut
     int vo = vtMap ? vtMap[vi] : vi;
     if (vo >= NvOut || vo < -1) { if (status) *status = PB200_EINDEX; return; }
     if (vo >= 0) atomicAdd(&cnt[vo], 1);
-}
-
-// ------------------------------------------------------------------------ exclusive scan
-constexpr int SCAN_THREADS = 256;
-constexpr int SCAN_ITEMS = 8;
-constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
-
-__global__ void scan_tiles_kernel(const int32_t* __restrict__ in, int64_t n, int32_t* __restrict__ out,
-                                  int32_t* __restrict__ tile_sum) {
-    __shared__ int32_t warp_tot[SCAN_THREADS / 32];
-    int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
-    int32_t v[SCAN_ITEMS];
-    int32_t run = 0;
-#pragma unroll
-    for (int j = 0; j < SCAN_ITEMS; ++j) {
-        int32_t x = (base + j < n) ? in[base + j] : 0;
-        v[j] = run;
-        run += x;
-    }
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int32_t inc = run;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        int32_t t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += t;
-    }
-    if (lane == 31) warp_tot[warp] = inc;
-    __syncthreads();
-    int32_t warp_off = 0;
-    for (int w = 0; w < warp; ++w) warp_off += warp_tot[w];
-    int32_t excl = warp_off + inc - run;
-#pragma unroll
-    for (int j = 0; j < SCAN_ITEMS; ++j)
-        if (base + j < n) out[base + j] = excl + v[j];
-    if (threadIdx.x == SCAN_THREADS - 1) tile_sum[blockIdx.x] = warp_off + inc;
-}
-
-__global__ void scan_tile_sums_kernel(int32_t* __restrict__ tile_sum, int ntiles, int32_t* __restrict__ total_out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    int32_t run = 0;
-    for (int t = 0; t < ntiles; ++t) { int32_t x = tile_sum[t]; tile_sum[t] = run; run += x; }
-    *total_out = run;
-}
-
-__global__ void scan_finish_kernel(int32_t* __restrict__ rowptr, int64_t n, const int32_t* __restrict__ tile_off,
-                                   int32_t* __restrict__ cursor) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int32_t v = rowptr[i] + tile_off[i / SCAN_TILE];
-    rowptr[i] = v;
-    cursor[i] = v;
 }
 
 // -------------------------------------------------------------------------------- fill
@@ -142,49 +92,41 @@ __global__ void cluster_fill_kernel(int64_t NvIn, const int32_t* __restrict__ ke
 
 // Rows come out of the atomic fill in arbitrary order; sorting each row ascending makes
 // the CSR (and every reduction that walks it) independent of scheduling.
+// A thread sorts a short row by insertion.  A long row is handed to the whole warp: every element finds its rank by
+// counting smaller ones (all entries of a row are distinct), writes itself to that slot of `tmp`, and the row is copied back.
 constexpr int SHORT_ROW = 32;
 
-__global__ void sort_short_rows_kernel(int64_t nrows, const int32_t* __restrict__ rowptr,
-                                       int32_t* __restrict__ entries, int32_t* __restrict__ long_rows,
-                                       int32_t* __restrict__ n_long) {
-    int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= nrows) return;
-    int beg = rowptr[v], end = rowptr[v + 1];
-    int deg = end - beg;
-    if (deg <= 1) return;
-    if (deg > SHORT_ROW) { long_rows[atomicAdd(n_long, 1)] = (int32_t)v; return; }
-    int32_t a[SHORT_ROW];
-    for (int i = 0; i < deg; ++i) a[i] = entries[beg + i];
-    for (int i = 1; i < deg; ++i) {
-        int32_t x = a[i];
-        int j = i - 1;
-        while (j >= 0 && a[j] > x) { a[j + 1] = a[j]; --j; }
-        a[j + 1] = x;
+__global__ void __launch_bounds__(128)
+sort_rows_kernel(int64_t nrows, const int32_t* __restrict__ rowptr, int32_t* __restrict__ entries, int32_t* __restrict__ tmp) {
+    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    int beg = 0, end = 0;
+    if (v < nrows) { beg = rowptr[v]; end = rowptr[v + 1]; }
+    const int deg = end - beg;
+    if (deg > 1 && deg <= SHORT_ROW) {
+        int32_t a[SHORT_ROW];
+        for (int i = 0; i < deg; ++i) a[i] = entries[beg + i];
+        for (int i = 1; i < deg; ++i) {
+            int32_t x = a[i];
+            int j = i - 1;
+            while (j >= 0 && a[j] > x) { a[j + 1] = a[j]; --j; }
+            a[j + 1] = x;
+        }
+        for (int i = 0; i < deg; ++i) entries[beg + i] = a[i];
     }
-    for (int i = 0; i < deg; ++i) entries[beg + i] = a[i];
-}
-
-// One warp per long row: every element finds its rank by counting smaller elements
-// (all entries of a row are distinct), writes itself to that slot of `tmp`, then the
-// row is copied back.
-__global__ void sort_long_rows_kernel(const int32_t* __restrict__ rowptr, int32_t* __restrict__ entries,
-                                      const int32_t* __restrict__ long_rows, const int32_t* __restrict__ n_long,
-                                      int32_t* __restrict__ tmp) {
-    int lane = threadIdx.x & 31;
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int nwarps = (gridDim.x * blockDim.x) >> 5;
-    int total = *n_long;
-    for (int r = warp; r < total; r += nwarps) {
-        int v = long_rows[r];
-        int beg = rowptr[v], end = rowptr[v + 1];
-        for (int i = beg + lane; i < end; i += 32) {
-            int32_t x = entries[i];
+    unsigned waiting = __ballot_sync(0xffffffffu, deg > SHORT_ROW);
+    while (waiting) {
+        const int owner = __ffs(waiting) - 1;
+        waiting &= waiting - 1;
+        const int b = __shfl_sync(0xffffffffu, beg, owner), e = __shfl_sync(0xffffffffu, end, owner);
+        for (int i = b + lane; i < e; i += 32) {
+            const int32_t x = entries[i];
             int rank = 0;
-            for (int j = beg; j < end; ++j) rank += (entries[j] < x);
-            tmp[beg + rank] = x;
+            for (int j = b; j < e; ++j) rank += entries[j] < x;
+            tmp[b + rank] = x;
         }
         __syncwarp();
-        for (int i = beg + lane; i < end; i += 32) entries[i] = tmp[i];
+        for (int i = b + lane; i < e; i += 32) entries[i] = tmp[i];
         __syncwarp();
     }
 }
@@ -289,11 +231,6 @@ level_prepare_kernel(int64_t Nf, int64_t NvIn, int64_t NvOut, int vstride, const
     }
 }
 
-__global__ void copy_counts_kernel(int64_t n, const int32_t* __restrict__ src, int32_t* __restrict__ dst) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dst[i] = src[i];
-}
-
 // ------------------------------------------------------------------------ row expansion
 // out[f] = mean of the rows of face f's samples, added in ascending order (0 for a face without samples)
 template <int VEC>
@@ -382,24 +319,44 @@ __global__ void check_running_count_kernel(int64_t Nf, int64_t NiK, const int32_
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// second half of the vertex-CSR build: exclusive scan of the corner counts in cursor[0..NvOut]
-// (last slot 0) -> rowptr, atomic-cursor fill, per-row sort
-static int finish_vertex_csr(int64_t Nf, int64_t NvIn, int64_t NvOut, const int32_t* face, const int32_t* vtMap,
-                             int32_t* rowptr, int32_t* entries, int32_t* cursor, int32_t* tile_sum, int32_t* long_rows,
-                             int32_t* tmp, int32_t* n_long, cudaStream_t stream) {
-    const int ntiles = (int)ceil_div(NvOut + 1, SCAN_TILE);
-    PB_LAUNCH("scan_tiles", scan_tiles_kernel, ntiles, SCAN_THREADS, 0, stream,
-              (const int32_t*)cursor, NvOut + 1, rowptr, tile_sum);
-    PB_LAUNCH("scan_tile_sums", scan_tile_sums_kernel, 1, 32, 0, stream, tile_sum, ntiles, tile_sum + ntiles);
-    PB_LAUNCH("scan_finish", scan_finish_kernel, (unsigned)ceil_div(NvOut + 1, 256), 256, 0, stream,
-              rowptr, NvOut + 1, (const int32_t*)tile_sum, cursor);
+// Workspace of a CSR build over `rows` rows and `items` items
+struct CsrWork {
+    int32_t *cursor, *tile_sum, *tmp;
+    CsrWork(void* ws, int64_t rows) {
+        char* w = (char*)ws;
+        cursor = (int32_t*)w;   w += align_up(sizeof(int32_t) * (size_t)(rows + 1), 256);
+        tile_sum = (int32_t*)w; w += align_up(sizeof(int32_t) * (size_t)scan::tiles(rows), 256);
+        tmp = (int32_t*)w;
+    }
+    static size_t bytes(int64_t rows, int64_t items) {
+        return align_up(sizeof(int32_t) * (size_t)(rows + 1), 256) + align_up(sizeof(int32_t) * (size_t)scan::tiles(rows), 256) +
+               align_up(sizeof(int32_t) * (size_t)(items + 1), 256) + 256;
+    }
+};
+
+// counts in w.cursor -> rowptr (and a copy of the counts), cursor = row starts
+static int row_starts(int64_t rows, const CsrWork& w, int32_t* rowptr, int32_t* counts, cudaStream_t stream) {
+    if (rows == 0) { PB_CUDA(cudaMemsetAsync(rowptr, 0, sizeof(int32_t), stream)); return PB200_OK; }
+    const int nt = scan::tiles(rows);
+    PB_LAUNCH("scan_tile_totals", scan::tile_totals_kernel, nt, scan::THREADS, 0, stream, (const int32_t*)w.cursor, rows, w.tile_sum);
+    PB_LAUNCH("scan_row_starts", scan::row_starts_kernel, nt, scan::THREADS, 0, stream, (const int32_t*)w.cursor, rows,
+              (const int32_t*)w.tile_sum, rowptr, w.cursor, counts);
+    return PB200_OK;
+}
+
+static int sort_rows(int64_t rows, const int32_t* rowptr, int32_t* entries, const CsrWork& w, cudaStream_t stream) {
+    PB_LAUNCH("sort_rows", sort_rows_kernel, (unsigned)ceil_div(rows, 128), 128, 0, stream, rows, rowptr, entries, w.tmp);
+    return PB200_OK;
+}
+
+// second half of the vertex-CSR build: corner counts in w.cursor -> rowptr, atomic-cursor fill, per-row sort
+static int finish_vertex_csr(int64_t Nf, int64_t NvIn, int64_t NvOut, const int32_t* face, const int32_t* vtMap, int32_t* rowptr,
+                             int32_t* entries, int32_t* counts, const CsrWork& w, cudaStream_t stream) {
+    if (int rc = row_starts(NvOut, w, rowptr, counts, stream)) return rc;
     if (Nf > 0 && NvOut > 0) {
         PB_LAUNCH("corner_fill", corner_fill_kernel, (unsigned)ceil_div(3 * Nf, 256), 256, 0, stream,
-                  3 * Nf, NvIn, NvOut, face, vtMap, cursor, entries);
-        PB_LAUNCH("sort_short_rows", sort_short_rows_kernel, (unsigned)ceil_div(NvOut, 128), 128, 0, stream,
-                  NvOut, (const int32_t*)rowptr, entries, long_rows, n_long);
-        PB_LAUNCH("sort_long_rows", sort_long_rows_kernel, 2 * sm_count(), 256, 0, stream,
-                  (const int32_t*)rowptr, entries, (const int32_t*)long_rows, (const int32_t*)n_long, tmp);
+                  3 * Nf, NvIn, NvOut, face, vtMap, w.cursor, entries);
+        return sort_rows(NvOut, rowptr, entries, w, stream);
     }
     return PB200_OK;
 }
@@ -425,11 +382,7 @@ int pb200_count_vertex_adjface(int64_t Nf, int64_t NvIn, int64_t NvOut, const in
 
 size_t pb200_vertex_csr_workspace_bytes(int64_t Nf, int64_t NvOut) {
     if (Nf < 0 || NvOut < 0) return 0;
-    size_t cursor = align_up(sizeof(int32_t) * (size_t)(NvOut + 1), 256);
-    size_t tiles = align_up(sizeof(int32_t) * (size_t)(ceil_div(NvOut + 1, SCAN_TILE) + 1), 256);
-    size_t longs = align_up(sizeof(int32_t) * (size_t)(NvOut + 1), 256);
-    size_t tmp = align_up(sizeof(int32_t) * (size_t)(3 * Nf + 1), 256);
-    return cursor + tiles + longs + tmp + 256;
+    return CsrWork::bytes(NvOut, 3 * Nf);
 }
 
 int pb200_build_vertex_csr(int64_t Nf, int64_t NvIn, int64_t NvOut, const int32_t* face,
@@ -441,22 +394,13 @@ int pb200_build_vertex_csr(int64_t Nf, int64_t NvIn, int64_t NvOut, const int32_
     PB_REQUIRE(rowptr && status && (Nf == 0 || (face && entries)), PB200_EINVAL, "build_vertex_csr: null pointer");
     PB_REQUIRE(workspace && workspace_bytes >= pb200_vertex_csr_workspace_bytes(Nf, NvOut), PB200_EWORKSPACE,
                "build_vertex_csr: workspace too small");
-    char* w = (char*)workspace;
-    int32_t* cursor = (int32_t*)w;  w += align_up(sizeof(int32_t) * (size_t)(NvOut + 1), 256);
-    int ntiles = (int)ceil_div(NvOut + 1, SCAN_TILE);
-    int32_t* tile_sum = (int32_t*)w; w += align_up(sizeof(int32_t) * (size_t)(ntiles + 1), 256);
-    int32_t* long_rows = (int32_t*)w; w += align_up(sizeof(int32_t) * (size_t)(NvOut + 1), 256);
-    int32_t* tmp = (int32_t*)w;      w += align_up(sizeof(int32_t) * (size_t)(3 * Nf + 1), 256);
-    int32_t* n_long = (int32_t*)w;
-
+    const CsrWork w(workspace, NvOut);
     PB_CUDA(cudaMemsetAsync(status, 0, sizeof(int32_t), stream));
-    PB_CUDA(cudaMemsetAsync(cursor, 0, sizeof(int32_t) * (NvOut + 1), stream));
-    PB_CUDA(cudaMemsetAsync(n_long, 0, sizeof(int32_t), stream));
+    PB_CUDA(cudaMemsetAsync(w.cursor, 0, sizeof(int32_t) * (NvOut + 1), stream));
     if (Nf > 0)
         PB_LAUNCH("corner_count", corner_count_kernel, (unsigned)ceil_div(3 * Nf, 256), 256, 0, stream,
-                  3 * Nf, NvIn, NvOut, face, vtMap, cursor, status);
-    return pb::finish_vertex_csr(Nf, NvIn, NvOut, face, vtMap, rowptr, entries, cursor, tile_sum, long_rows, tmp, n_long,
-                                 stream);
+                  3 * Nf, NvIn, NvOut, face, vtMap, w.cursor, status);
+    return pb::finish_vertex_csr(Nf, NvIn, NvOut, face, vtMap, rowptr, entries, nullptr, w, stream);
 }
 
 int pb200_level_prepare(int64_t Nf, int64_t NvIn, int64_t NvOut, int vstride, const float* vertex, const int32_t* face,
@@ -471,37 +415,23 @@ int pb200_level_prepare(int64_t Nf, int64_t NvIn, int64_t NvOut, int vstride, co
                "level_prepare: null pointer");
     PB_REQUIRE(workspace && workspace_bytes >= pb200_vertex_csr_workspace_bytes(Nf, NvOut), PB200_EWORKSPACE,
                "level_prepare: workspace too small");
-    char* w = (char*)workspace;
-    int32_t* cursor = (int32_t*)w;  w += align_up(sizeof(int32_t) * (size_t)(NvOut + 1), 256);
-    int ntiles = (int)ceil_div(NvOut + 1, SCAN_TILE);
-    int32_t* tile_sum = (int32_t*)w; w += align_up(sizeof(int32_t) * (size_t)(ntiles + 1), 256);
-    int32_t* long_rows = (int32_t*)w; w += align_up(sizeof(int32_t) * (size_t)(NvOut + 1), 256);
-    int32_t* tmp = (int32_t*)w;      w += align_up(sizeof(int32_t) * (size_t)(3 * Nf + 1), 256);
-    int32_t* n_long = (int32_t*)w;
+    const CsrWork w(workspace, NvOut);
     PB_CUDA(cudaMemsetAsync(status, 0, sizeof(int32_t), stream));
-    PB_CUDA(cudaMemsetAsync(cursor, 0, sizeof(int32_t) * (NvOut + 1), stream));
-    PB_CUDA(cudaMemsetAsync(n_long, 0, sizeof(int32_t), stream));
+    PB_CUDA(cudaMemsetAsync(w.cursor, 0, sizeof(int32_t) * (NvOut + 1), stream));
     if (Nf > 0) {
         static const SphConst cst = make_sph_const();
         const int K = (L + 1) * (L + 1);
         PB_LAUNCH("level_prepare", level_prepare_kernel, (unsigned)ceil_div(Nf, PREP_BLOCK), PREP_BLOCK,
                   sizeof(float) * PREP_BLOCK * (K + 1), stream, Nf, NvIn, NvOut, vstride, vertex, face, vtMap, L, orient, cst,
-                  geometry, normals, coeff, cursor, status);
+                  geometry, normals, coeff, w.cursor, status);
     }
-    if (NvOut > 0)      // the corner counts are the reference's nfCount; the scan below overwrites the cursor
-        PB_LAUNCH("copy_counts", copy_counts_kernel, (unsigned)ceil_div(NvOut, 256), 256, 0, stream, NvOut,
-                  (const int32_t*)cursor, nfCount);
-    return pb::finish_vertex_csr(Nf, NvIn, NvOut, face, vtMap, rowptr, entries, cursor, tile_sum, long_rows, tmp, n_long,
-                                 stream);
+    // the corner counts are the reference's nfCount
+    return pb::finish_vertex_csr(Nf, NvIn, NvOut, face, vtMap, rowptr, entries, nfCount, w, stream);
 }
 
 size_t pb200_cluster_csr_workspace_bytes(int64_t NvIn, int64_t NvOut) {
     if (NvIn < 0 || NvOut < 0) return 0;
-    size_t cursor = align_up(sizeof(int32_t) * (size_t)(NvOut + 1), 256);
-    size_t tiles = align_up(sizeof(int32_t) * (size_t)(ceil_div(NvOut + 1, SCAN_TILE) + 1), 256);
-    size_t longs = align_up(sizeof(int32_t) * (size_t)(NvOut + 1), 256);
-    size_t tmp = align_up(sizeof(int32_t) * (size_t)(NvIn + 1), 256);
-    return cursor + tiles + longs + tmp + 256;
+    return CsrWork::bytes(NvOut, NvIn);
 }
 
 int pb200_build_cluster_csr(int64_t NvIn, int64_t NvOut, const int32_t* vtReplace, const int32_t* vtMap,
@@ -514,31 +444,17 @@ int pb200_build_cluster_csr(int64_t NvIn, int64_t NvOut, const int32_t* vtReplac
                "build_cluster_csr: null pointer");
     PB_REQUIRE(workspace && workspace_bytes >= pb200_cluster_csr_workspace_bytes(NvIn, NvOut), PB200_EWORKSPACE,
                "build_cluster_csr: workspace too small");
-    char* w = (char*)workspace;
-    int32_t* cursor = (int32_t*)w;  w += align_up(sizeof(int32_t) * (size_t)(NvOut + 1), 256);
-    int ntiles = (int)ceil_div(NvOut + 1, SCAN_TILE);
-    int32_t* tile_sum = (int32_t*)w; w += align_up(sizeof(int32_t) * (size_t)(ntiles + 1), 256);
-    int32_t* long_rows = (int32_t*)w; w += align_up(sizeof(int32_t) * (size_t)(NvOut + 1), 256);
-    int32_t* tmp = (int32_t*)w;      w += align_up(sizeof(int32_t) * (size_t)(NvIn + 1), 256);
-    int32_t* n_long = (int32_t*)w;
+    const CsrWork w(workspace, NvOut);
     PB_CUDA(cudaMemsetAsync(status, 0, sizeof(int32_t), stream));
-    PB_CUDA(cudaMemsetAsync(cursor, 0, sizeof(int32_t) * (NvOut + 1), stream));
-    PB_CUDA(cudaMemsetAsync(n_long, 0, sizeof(int32_t), stream));
+    PB_CUDA(cudaMemsetAsync(w.cursor, 0, sizeof(int32_t) * (NvOut + 1), stream));
     if (NvIn > 0)
         PB_LAUNCH("cluster_count", cluster_count_kernel, (unsigned)ceil_div(NvIn, 256), 256, 0, stream,
-                  NvIn, NvOut, vtReplace, vtMap, key, cursor, status);
-    PB_LAUNCH("scan_tiles", scan_tiles_kernel, ntiles, SCAN_THREADS, 0, stream,
-              (const int32_t*)cursor, NvOut + 1, rowptr, tile_sum);
-    PB_LAUNCH("scan_tile_sums", scan_tile_sums_kernel, 1, 32, 0, stream, tile_sum, ntiles, tile_sum + ntiles);
-    PB_LAUNCH("scan_finish", scan_finish_kernel, (unsigned)ceil_div(NvOut + 1, 256), 256, 0, stream,
-              rowptr, NvOut + 1, (const int32_t*)tile_sum, cursor);
+                  NvIn, NvOut, vtReplace, vtMap, key, w.cursor, status);
+    if (int rc = row_starts(NvOut, w, rowptr, nullptr, stream)) return rc;
     if (NvIn > 0 && NvOut > 0) {
         PB_LAUNCH("cluster_fill", cluster_fill_kernel, (unsigned)ceil_div(NvIn, 256), 256, 0, stream,
-                  NvIn, (const int32_t*)key, cursor, members);
-        PB_LAUNCH("sort_short_rows", sort_short_rows_kernel, (unsigned)ceil_div(NvOut, 128), 128, 0, stream,
-                  NvOut, (const int32_t*)rowptr, members, long_rows, n_long);
-        PB_LAUNCH("sort_long_rows", sort_long_rows_kernel, 2 * sm_count(), 256, 0, stream,
-                  (const int32_t*)rowptr, members, (const int32_t*)long_rows, (const int32_t*)n_long, tmp);
+                  NvIn, (const int32_t*)key, w.cursor, members);
+        return sort_rows(NvOut, rowptr, members, w, stream);
     }
     return PB200_OK;
 }
@@ -551,31 +467,17 @@ int pb200_build_key_csr(int64_t N, int64_t NvOut, const int32_t* key, int key_st
     PB_REQUIRE(rowptr && status && (N == 0 || (key && members)), PB200_EINVAL, "build_key_csr: null pointer");
     PB_REQUIRE(workspace && workspace_bytes >= pb200_cluster_csr_workspace_bytes(N, NvOut), PB200_EWORKSPACE,
                "build_key_csr: workspace too small");
-    char* w = (char*)workspace;
-    int32_t* cursor = (int32_t*)w;  w += align_up(sizeof(int32_t) * (size_t)(NvOut + 1), 256);
-    int ntiles = (int)ceil_div(NvOut + 1, SCAN_TILE);
-    int32_t* tile_sum = (int32_t*)w; w += align_up(sizeof(int32_t) * (size_t)(ntiles + 1), 256);
-    int32_t* long_rows = (int32_t*)w; w += align_up(sizeof(int32_t) * (size_t)(NvOut + 1), 256);
-    int32_t* tmp = (int32_t*)w;      w += align_up(sizeof(int32_t) * (size_t)(N + 1), 256);
-    int32_t* n_long = (int32_t*)w;
+    const CsrWork w(workspace, NvOut);
     PB_CUDA(cudaMemsetAsync(status, 0, sizeof(int32_t), stream));
-    PB_CUDA(cudaMemsetAsync(cursor, 0, sizeof(int32_t) * (NvOut + 1), stream));
-    PB_CUDA(cudaMemsetAsync(n_long, 0, sizeof(int32_t), stream));
+    PB_CUDA(cudaMemsetAsync(w.cursor, 0, sizeof(int32_t) * (NvOut + 1), stream));
     if (N > 0)
         PB_LAUNCH("key_count", key_count_kernel, (unsigned)ceil_div(N, 256), 256, 0, stream, N, NvOut, key, key_stride,
-                  cursor, status);
-    PB_LAUNCH("scan_tiles", scan_tiles_kernel, ntiles, SCAN_THREADS, 0, stream,
-              (const int32_t*)cursor, NvOut + 1, rowptr, tile_sum);
-    PB_LAUNCH("scan_tile_sums", scan_tile_sums_kernel, 1, 32, 0, stream, tile_sum, ntiles, tile_sum + ntiles);
-    PB_LAUNCH("scan_finish", scan_finish_kernel, (unsigned)ceil_div(NvOut + 1, 256), 256, 0, stream,
-              rowptr, NvOut + 1, (const int32_t*)tile_sum, cursor);
+                  w.cursor, status);
+    if (int rc = row_starts(NvOut, w, rowptr, nullptr, stream)) return rc;
     if (N > 0 && NvOut > 0) {
         PB_LAUNCH("key_fill", key_fill_kernel, (unsigned)ceil_div(N, 256), 256, 0, stream, N, NvOut, key, key_stride,
-                  cursor, members);
-        PB_LAUNCH("sort_short_rows", sort_short_rows_kernel, (unsigned)ceil_div(NvOut, 128), 128, 0, stream,
-                  NvOut, (const int32_t*)rowptr, members, long_rows, n_long);
-        PB_LAUNCH("sort_long_rows", sort_long_rows_kernel, 2 * sm_count(), 256, 0, stream,
-                  (const int32_t*)rowptr, members, (const int32_t*)long_rows, (const int32_t*)n_long, tmp);
+                  w.cursor, members);
+        return sort_rows(NvOut, rowptr, members, w, stream);
     }
     return PB200_OK;
 }

@@ -4,204 +4,43 @@
 //
 // The reference sorts edge indices with a comparator sort, loops over the samples of the batch
 // on the host (unique / cost / sort per sample), copies the sorted candidates to the host and
-// clusters vertices there in two sequential sweeps.  Here one pass is:
-//   1. edge keys (lower vertex, higher vertex) -> stable LSD radix sort -> boundary flags
-//      (an edge seen once) and the list of distinct candidates, for the whole batch at once;
-//   2. vertex quadrics pulled through the vertex CSR in ascending (face, corner) order
-//      (no float atomics: run-to-run deterministic), boundary quadrics in the same walk;
-//   3. candidate costs, one radix sort by (sample, cost) -> every candidate's rank;
-//   4. the first sequential sweep (an edge is taken when neither end is covered) is the greedy
-//      matching in rank order.  It equals the fixed point of "take every edge whose rank is
-//      the smallest among the live edges at both of its ends", computed in parallel rounds
-//      (atomicMin per vertex); the sweep's early stop is a prefix count over ranks;
-//   5. the second sweep attaches every still-uncovered vertex through its lowest-ranked
+// clusters vertices there in two sequential sweeps.  Here one pass is, for the whole batch at once:
+//   1. the vertex CSR of the faces; a thread per vertex sorts its row, collects the other ends of the
+//      edges it owns (an edge belongs to its lower vertex), sorts those and so knows its distinct
+//      candidate edges and, by their multiplicity, the boundary edges (seen once): candidates come out
+//      in (lower, higher) order after one prefix sum, without sorting the edges of the batch;
+//   2. vertex quadrics pulled through the CSR in ascending (face, corner) order (no float atomics:
+//      run-to-run deterministic), boundary quadrics in the same walk; candidate costs.  A candidate's
+//      place in the cost order is the 64-bit key (cost, candidate): nothing is sorted by cost;
+//   3. the first sequential sweep (an edge is taken when neither end is covered) is the greedy
+//      matching in key order.  It equals the fixed point of "take every edge whose key is the
+//      smallest among the live edges at both of its ends", computed in parallel rounds
+//      (atomicMin per vertex).  The sweep's early stop keeps the first want[s] matched edges in key
+//      order: their last key is found by radix selection among the matched edges;
+//   4. the second sweep attaches every still-uncovered vertex through its lowest-keyed
 //      edge: after a complete first sweep no edge joins two uncovered vertices, so these
-//      choices are independent; its early stop is again a prefix count;
-//   6. cluster positions (members added in ascending vertex id), relabelled faces, degenerate
+//      choices are independent; its early stop is the same selection;
+//   5. cluster positions (members added in ascending vertex id), relabelled faces, degenerate
 //      flags, vertex map and the per-sample output sizes.
-// Results equal the sequential procedure's for any input; the host reads back three counters
-// (a few stream synchronisations), never mesh data.
+// Results equal the sequential procedure's for any input.
+//
+// A pass is a chain of dependent steps over small arrays: what it costs is launches, grid-wide
+// synchronisations and latency far more than bytes.  Radix sorts of the edges and of the costs took 70 of
+// its 170 launches; steps 3 and 4, thirty-odd steps of their own, are ONE kernel: a block per sample where
+// samples are small (steps separated by block barriers), a cooperative grid with a bounded barrier
+// otherwise.  Two scenes of 490 000 vertices, three levels of 1/4: 9.2 -> 4.6 ms; 64 shapes of 642
+// vertices, two levels: 4.6 -> 1.26 ms (host loop and level preparation included).
 //
 // This file is compiled with --fmad=false: every float operation is rounded on its own, so the
 // costs (and therefore the clustering) can be reproduced exactly by a plain C restatement.
 #include "common.cuh"
+#include "scan.cuh"
 
 namespace pb {
 namespace dec {
 
-constexpr uint32_t NO_RANK = 0xffffffffu;
-
-// ------------------------------------------------------------------ exclusive scan (int32)
-// out[0..n] (n + 1 values): out[i] = sum of in[0..i); in place allowed.
-constexpr int SC_THREADS = 256, SC_ITEMS = 8, SC_TILE = SC_THREADS * SC_ITEMS;
-
-__global__ void scan_tiles_kernel(const int32_t* in, int64_t n, int32_t* out, int32_t* __restrict__ tile_sum) {
-    __shared__ int32_t warp_tot[SC_THREADS / 32];
-    const int64_t base = (int64_t)blockIdx.x * SC_TILE + (int64_t)threadIdx.x * SC_ITEMS;
-    int32_t v[SC_ITEMS], run = 0;
-#pragma unroll
-    for (int j = 0; j < SC_ITEMS; ++j) {
-        const int32_t x = (base + j < n) ? in[base + j] : 0;
-        v[j] = run;
-        run += x;
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int32_t inc = run;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int32_t t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += t;
-    }
-    if (lane == 31) warp_tot[warp] = inc;
-    __syncthreads();
-    int32_t warp_off = 0;
-    for (int w = 0; w < warp; ++w) warp_off += warp_tot[w];
-    const int32_t excl = warp_off + inc - run;
-#pragma unroll
-    for (int j = 0; j < SC_ITEMS; ++j)
-        if (base + j <= n) out[base + j] = excl + v[j];
-    if (threadIdx.x == SC_THREADS - 1) tile_sum[blockIdx.x] = warp_off + inc;
-}
-
-// one block: exclusive scan of the tile totals, 1024 at a time with a carry
-__global__ void scan_sums_kernel(int32_t* __restrict__ tile_sum, int ntiles) {
-    __shared__ int32_t wt[32];
-    __shared__ int32_t carry;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int base = 0; base < ntiles; base += 1024) {
-        const int i = base + threadIdx.x;
-        const int32_t x = i < ntiles ? tile_sum[i] : 0;
-        int32_t inc = x;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int32_t t = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += t;
-        }
-        if (lane == 31) wt[warp] = inc;
-        __syncthreads();
-        if (warp == 0) {
-            const int32_t w = wt[lane];
-            int32_t winc = w;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int32_t t = __shfl_up_sync(0xffffffffu, winc, o);
-                if (lane >= o) winc += t;
-            }
-            wt[lane] = winc - w;
-        }
-        __syncthreads();
-        const int32_t excl = carry + wt[warp] + inc - x;
-        if (i < ntiles) tile_sum[i] = excl;
-        __syncthreads();
-        if (threadIdx.x == 1023) carry = excl + x;
-        __syncthreads();
-    }
-}
-
-__global__ void scan_add_kernel(int32_t* __restrict__ out, int64_t n, const int32_t* __restrict__ tile_off) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i <= n) out[i] += tile_off[i / SC_TILE];
-}
-
-static size_t scan_tiles_for(int64_t n) { return (size_t)ceil_div(n + 1, SC_TILE); }
-
-static int exclusive_scan(const int32_t* in, int64_t n, int32_t* out, int32_t* tile_sum, cudaStream_t stream) {
-    const int ntiles = (int)scan_tiles_for(n);
-    PB_LAUNCH("dec_scan_tiles", scan_tiles_kernel, ntiles, SC_THREADS, 0, stream, in, n, out, tile_sum);
-    if (ntiles > 1) {
-        PB_LAUNCH("dec_scan_sums", scan_sums_kernel, 1, 1024, 0, stream, tile_sum, ntiles);
-        PB_LAUNCH("dec_scan_add", scan_add_kernel, (unsigned)ceil_div(n + 1, 256), 256, 0, stream, out, n,
-                  (const int32_t*)tile_sum);
-    }
-    return PB200_OK;
-}
-
-// ------------------------------------------------ stable LSD radix sort, 8 bits per pass
-// 64-bit keys with a 32-bit payload.  A block owns a tile of 2048 consecutive elements, a warp
-// 256 consecutive ones in 8 rounds of 32: the rank of an element among equal digits follows
-// the element order, which makes every pass stable.
-constexpr int RS_THREADS = 256, RS_ROUNDS = 8, RS_TILE = RS_THREADS * RS_ROUNDS, RS_WARPS = RS_THREADS / 32;
-
-__global__ void rs_hist_kernel(const uint64_t* __restrict__ keys, int64_t n, int shift, int nblocks,
-                               int32_t* __restrict__ hist) {
-    __shared__ int32_t h[256];
-    h[threadIdx.x] = 0;
-    __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * RS_TILE;
-#pragma unroll
-    for (int j = 0; j < RS_ROUNDS; ++j) {
-        const int64_t i = base + j * RS_THREADS + threadIdx.x;
-        if (i < n) atomicAdd(&h[(int)((keys[i] >> shift) & 255u)], 1);
-    }
-    __syncthreads();
-    hist[(int64_t)threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
-}
-
-__global__ void rs_scatter_kernel(const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin,
-                                  uint64_t* __restrict__ kout, uint32_t* __restrict__ vout, int64_t n, int shift,
-                                  int nblocks, const int32_t* __restrict__ hist_scan) {
-    __shared__ int32_t wc[RS_WARPS][256];
-    for (int i = threadIdx.x; i < RS_WARPS * 256; i += RS_THREADS) (&wc[0][0])[i] = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t seg = (int64_t)blockIdx.x * RS_TILE + (int64_t)warp * (RS_ROUNDS * 32);
-    uint64_t k[RS_ROUNDS];
-    uint32_t v[RS_ROUNDS];
-    int32_t lr[RS_ROUNDS];
-#pragma unroll
-    for (int j = 0; j < RS_ROUNDS; ++j) {
-        const int64_t i = seg + j * 32 + lane;
-        const bool valid = i < n;
-        k[j] = valid ? kin[i] : 0;
-        v[j] = valid ? vin[i] : 0;
-        const int d = valid ? (int)((k[j] >> shift) & 255u) : 256 + lane;     // elements past the end: groups of one
-        const unsigned mask = __match_any_sync(0xffffffffu, d);
-        const int leader = __ffs(mask) - 1;
-        int32_t old = 0;
-        if (valid && lane == leader) { old = wc[warp][d]; wc[warp][d] = old + __popc(mask); }
-        old = __shfl_sync(0xffffffffu, old, leader);
-        lr[j] = old + __popc(mask & ((1u << lane) - 1u));
-        __syncwarp();
-    }
-    __syncthreads();
-    {
-        const int d = threadIdx.x;
-        int32_t run = hist_scan[(int64_t)d * nblocks + blockIdx.x];
-#pragma unroll
-        for (int w = 0; w < RS_WARPS; ++w) { const int32_t t = wc[w][d]; wc[w][d] = run; run += t; }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < RS_ROUNDS; ++j) {
-        const int64_t i = seg + j * 32 + lane;
-        if (i < n) {
-            const int32_t pos = wc[warp][(int)((k[j] >> shift) & 255u)] + lr[j];
-            kout[pos] = k[j];
-            vout[pos] = v[j];
-        }
-    }
-}
-
-// sorts (k, v) by the low `bits` bits of k; on return k / v point at the sorted arrays
-static int radix_sort(uint64_t*& k, uint64_t*& kalt, uint32_t*& v, uint32_t*& valt, int64_t n, int bits,
-                      int32_t* hist, int32_t* tile_sum, cudaStream_t stream) {
-    if (n <= 1) return PB200_OK;
-    const int nblocks = (int)ceil_div(n, RS_TILE);
-    for (int shift = 0; shift < bits; shift += 8) {
-        PB_LAUNCH("dec_sort_hist", rs_hist_kernel, nblocks, RS_THREADS, 0, stream, (const uint64_t*)k, n, shift, nblocks, hist);
-        int rc = exclusive_scan(hist, (int64_t)256 * nblocks, hist, tile_sum, stream);
-        if (rc != PB200_OK) return rc;
-        PB_LAUNCH("dec_sort_scatter", rs_scatter_kernel, nblocks, RS_THREADS, 0, stream, (const uint64_t*)k,
-                  (const uint32_t*)v, kalt, valt, n, shift, nblocks, (const int32_t*)hist);
-        uint64_t* tk = k; k = kalt; kalt = tk;
-        uint32_t* tv = v; v = valt; valt = tv;
-    }
-    return PB200_OK;
-}
-
-static int bit_length(int64_t x) { int b = 0; while (x > 0) { ++b; x >>= 1; } return b; }
+typedef unsigned long long u64;
+constexpr u64 NO_KEY = ~0ull;
 
 // ------------------------------------------------------------------------ small helpers
 // sample that owns vertex (or face) id x: first s with x < cum[s]; B when none
@@ -222,48 +61,194 @@ __device__ __forceinline__ void warp_append(bool pred, uint32_t value, uint32_t*
     if (pred) list[base + __popc(m & ((1u << lane) - 1u))] = value;
 }
 
+// counter[key] += 1 for the lanes with key >= 0, one atomic per distinct key of the warp; called by whole warps
+__device__ __forceinline__ void warp_count(int key, int32_t* counter) {
+    const int lane = threadIdx.x & 31;
+    const unsigned m = __match_any_sync(0xffffffffu, key >= 0 ? key : -1 - lane);
+    if (key >= 0 && lane == __ffs(m) - 1) atomicAdd(&counter[key], __popc(m));
+}
+
 // face edge slots as the reference numbers them (decimate_gpu.cu:262-308):
 // slot 0 joins corners (0,1), slot 1 corners (0,2), slot 2 corners (1,2)
 __device__ __forceinline__ int slot_a(int k) { return k == 2 ? 1 : 0; }
 __device__ __forceinline__ int slot_b(int k) { return k == 0 ? 1 : 2; }
 
-// ------------------------------------------------------------------------------ edges
-__global__ void edge_keys_kernel(int64_t Ne, int64_t Nv, int vbits, const int32_t* __restrict__ face,
-                                 uint64_t* __restrict__ key, uint32_t* __restrict__ val, int32_t* __restrict__ status) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= Ne) return;
-    const int64_t f = e / 3;
-    const int k = (int)(e - 3 * f);
-    int a = face[3 * f + slot_a(k)], b = face[3 * f + slot_b(k)];
-    if (a < 0 || b < 0 || a >= Nv || b >= Nv) { *status = PB200_EINDEX; a = b = (int)Nv; }
-    const uint64_t lo = (uint64_t)(a <= b ? a : b), hi = (uint64_t)(a <= b ? b : a);
-    key[e] = (lo << vbits) | hi;
-    val[e] = (uint32_t)e;
+// ------------------------------------------------------------------ vertex CSR and edges
+// a face with an id outside [0, Nv) is reported and takes part in nothing
+__device__ __forceinline__ bool read_face(const int32_t* __restrict__ face, int64_t f, int64_t Nv, int (&v)[3]) {
+    v[0] = face[3 * f]; v[1] = face[3 * f + 1]; v[2] = face[3 * f + 2];
+    return v[0] >= 0 && v[1] >= 0 && v[2] >= 0 && v[0] < Nv && v[1] < Nv && v[2] < Nv;
 }
 
-// over the sorted edges: boundary flag of the edge instance, first-of-run flag
-__global__ void edge_flags_kernel(int64_t Ne, int64_t Nv, int vbits, const uint64_t* __restrict__ skey,
-                                  const uint32_t* __restrict__ sval, uint8_t* __restrict__ bnd, int32_t* __restrict__ uflag) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= Ne) return;
-    const uint64_t k = skey[i];
-    const bool valid = (int64_t)(k >> vbits) < Nv;
-    const bool same_prev = i > 0 && skey[i - 1] == k;
-    const bool same_next = i + 1 < Ne && skey[i + 1] == k;
-    bnd[sval[i]] = (valid && !same_prev && !same_next) ? 1 : 0;
-    uflag[i] = (valid && !same_prev) ? 1 : 0;
+__global__ void count_corners_kernel(int64_t Nf, int64_t Nv, const int32_t* __restrict__ face, int32_t* __restrict__ cnt,
+                                     int32_t* __restrict__ status) {
+    const int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= Nf) return;
+    int v[3];
+    if (!read_face(face, f, Nv, v)) { *status = PB200_EINDEX; return; }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) atomicAdd(&cnt[v[c]], 1);
 }
 
-__global__ void unique_write_kernel(int64_t Ne, int vbits, const uint64_t* __restrict__ skey,
-                                    const int32_t* __restrict__ uflag_scan, int32_t* __restrict__ ulo,
-                                    int32_t* __restrict__ uhi) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= Ne) return;
-    if (uflag_scan[i + 1] == uflag_scan[i]) return;
-    const uint64_t k = skey[i];
-    const int u = uflag_scan[i];
-    ulo[u] = (int32_t)(k >> vbits);
-    uhi[u] = (int32_t)(k & ((1ull << vbits) - 1ull));
+__global__ void fill_corners_kernel(int64_t Nf, int64_t Nv, const int32_t* __restrict__ face, int32_t* __restrict__ cursor,
+                                    int32_t* __restrict__ entries) {
+    const int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= Nf) return;
+    int v[3];
+    if (!read_face(face, f, Nv, v)) return;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) entries[atomicAdd(&cursor[v[c]], 1)] = (int32_t)((f << 2) | c);
+}
+
+// The edge of corner (f, c), s-th of two: its slot, the other end, and whether corner c owns the instance (it is the lower
+// end; of a degenerate edge the corner that the slot names first)
+__device__ __forceinline__ bool corner_edge(const int32_t* __restrict__ face, int32_t entry, int v, int s, int& other, uint32_t& e) {
+    const int64_t f = entry >> 2;
+    const int c = entry & 3;
+    const int k = c == 0 ? s : (c == 1 ? 2 * s : 1 + s);
+    const int oc = slot_a(k) == c ? slot_b(k) : slot_a(k);
+    other = face[3 * f + oc];
+    e = (uint32_t)(3 * f + k);
+    return other > v || (other == v && slot_a(k) == c);
+}
+
+// Per vertex: row sorted; distinct other ends of its own edges, ascending, to hi[2 * rowptr[v] ...], their number to
+// ucnt[v]; boundary flag of every edge instance.  Long rows (more than SHORT corners) are taken by the whole warp:
+// ranks by counting, with room in tmp (two int32 per entry of the row, twice).
+constexpr int SHORT = 16;
+
+__global__ void __launch_bounds__(128)
+vertex_edges_kernel(int64_t Nv, const int32_t* __restrict__ face, const int32_t* __restrict__ rowptr, int32_t* entries,
+                    int32_t* hi, int32_t* __restrict__ ucnt, uint8_t* __restrict__ bnd, int32_t* tmpA, uint32_t* tmpB,
+                    int32_t* __restrict__ tile_sum) {
+    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    int beg = 0, end = 0;
+    if (v < Nv) { beg = rowptr[v]; end = rowptr[v + 1]; }
+    const int deg = end - beg;
+    int found = 0;
+    if (deg > 0 && deg <= SHORT) {
+        int32_t a[SHORT];
+        for (int i = 0; i < deg; ++i) {
+            const int32_t x = entries[beg + i];
+            int j = i - 1;
+            while (j >= 0 && a[j] > x) { a[j + 1] = a[j]; --j; }
+            a[j + 1] = x;
+        }
+        int32_t o[2 * SHORT];
+        uint32_t id[2 * SHORT];
+        int n = 0;
+        for (int i = 0; i < deg; ++i) {
+            entries[beg + i] = a[i];
+            for (int s = 0; s < 2; ++s) {
+                int other;
+                uint32_t e;
+                if (!corner_edge(face, a[i], (int)v, s, other, e)) continue;
+                int j = n++ - 1;
+                while (j >= 0 && o[j] > other) { o[j + 1] = o[j]; id[j + 1] = id[j]; --j; }
+                o[j + 1] = other; id[j + 1] = e;
+            }
+        }
+        for (int i = 0; i < n; ++i) {
+            const bool first = i == 0 || o[i - 1] != o[i], last = i + 1 == n || o[i + 1] != o[i];
+            bnd[id[i]] = first && last;
+            if (first) hi[2 * (int64_t)beg + found++] = o[i];
+        }
+    }
+    unsigned waiting = __ballot_sync(0xffffffffu, deg > SHORT);
+    while (waiting) {
+        const int owner = __ffs(waiting) - 1;
+        waiting &= waiting - 1;
+        const int64_t b = __shfl_sync(0xffffffffu, beg, owner);
+        const int d = __shfl_sync(0xffffffffu, deg, owner);
+        const int vv = (int)(v - lane + owner);
+        // the row, sorted
+        for (int i = lane; i < d; i += 32) {
+            const int32_t x = entries[b + i];
+            int rank = 0;
+            for (int j = 0; j < d; ++j) rank += entries[b + j] < x;
+            tmpA[2 * b + rank] = x;
+        }
+        __syncwarp();
+        for (int i = lane; i < d; i += 32) entries[b + i] = tmpA[2 * b + i];
+        __syncwarp();
+        // own edges, in row order: other end to tmpA, instance to tmpB
+        int n = 0;
+        for (int i0 = 0; i0 < 2 * d; i0 += 32) {
+            const int i = i0 + lane;
+            int other = 0;
+            uint32_t e = 0;
+            const bool own = i < 2 * d && corner_edge(face, entries[b + (i >> 1)], vv, i & 1, other, e);
+            const unsigned m = __ballot_sync(0xffffffffu, own);
+            if (own) {
+                const int at = n + __popc(m & ((1u << lane) - 1u));
+                tmpA[2 * b + at] = other;
+                tmpB[2 * b + at] = e;
+            }
+            n += __popc(m);
+        }
+        __syncwarp();
+        for (int i = lane; i < n; i += 32) {
+            const int x = tmpA[2 * b + i];
+            int same = 0, before = 0;
+            for (int j = 0; j < n; ++j) { const bool eq = tmpA[2 * b + j] == x; same += eq; before += eq && j < i; }
+            bnd[tmpB[2 * b + i]] = same == 1;
+            tmpB[2 * b + i] = before == 0;                       // first of its run (the instance is not needed any more)
+        }
+        __syncwarp();
+        int total = 0;
+        for (int i0 = 0; i0 < n; i0 += 32) {
+            const int i = i0 + lane;
+            const bool first = i < n && tmpB[2 * b + i] != 0;
+            if (first) {
+                const int x = tmpA[2 * b + i];
+                int rank = 0;
+                for (int j = 0; j < n; ++j) rank += tmpB[2 * b + j] != 0 && tmpA[2 * b + j] < x;
+                hi[2 * b + rank] = x;
+            }
+            total += __popc(__ballot_sync(0xffffffffu, first));
+        }
+        if (lane == owner) found = total;
+        __syncwarp();
+    }
+    if (v < Nv) ucnt[v] = found;
+    const int sum = __reduce_add_sync(0xffffffffu, found);
+    if (lane == 0 && sum > 0) atomicAdd(&tile_sum[v / scan::TILE], sum);
+}
+
+// candidates in (lower, higher) order; ustart[v] = first candidate of vertex v, ustart[Nv] = their number.  Samples are
+// clustered independently of one another: an edge between two of them is reported and nothing is clustered.
+constexpr int32_t ECROSS = 1;
+
+__global__ void __launch_bounds__(scan::THREADS)
+candidates_kernel(int64_t Nv, int B, const int32_t* __restrict__ nvIn, int32_t* __restrict__ status, const int32_t* __restrict__ ucnt, const int32_t* __restrict__ tile_sum, const int32_t* __restrict__ rowptr,
+                  const int32_t* __restrict__ hi, int32_t* __restrict__ ustart, int32_t* __restrict__ ulo, int32_t* __restrict__ uhi) {
+    __shared__ int sh[scan::THREADS / 32];
+    const int before = scan::tiles_before(tile_sum, blockIdx.x, sh);
+    const int64_t base = (int64_t)blockIdx.x * scan::TILE + (int64_t)threadIdx.x * scan::ITEMS;
+    int n[scan::ITEMS], s = 0;
+    scan::load_items(ucnt, Nv, base, n);
+#pragma unroll
+    for (int j = 0; j < scan::ITEMS; ++j) s += n[j];
+    int run = before + scan::block_exclusive(s, sh);
+    int sample = base < Nv ? sample_of((int)base, nvIn, B) : B;
+#pragma unroll
+    for (int j = 0; j < scan::ITEMS; ++j) {
+        const int64_t v = base + j;
+        if (v >= Nv) break;
+        ustart[v] = run;
+        while (sample < B && nvIn[sample] <= v) ++sample;
+        const int end = sample < B ? nvIn[sample] : 0;
+        const int64_t src = 2 * (int64_t)rowptr[v];
+        for (int i = 0; i < n[j]; ++i) {
+            const int other = hi[src + i];
+            ulo[run + i] = (int32_t)v;
+            uhi[run + i] = other;
+            if (other >= end) *status = ECROSS;
+        }
+        run += n[j];
+        if (v + 1 == Nv) ustart[Nv] = run;
+    }
 }
 
 // ---------------------------------------------------------------------------- quadrics
@@ -390,316 +375,531 @@ __device__ __forceinline__ uint32_t cost_key(float c) {
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-// one thread per candidate (decimate_gpu.cu:378-416); sort key = (sample, cost), payload = candidate
-__global__ void edge_cost_kernel(int64_t nu, int64_t Nv, int D, int B, const int32_t* __restrict__ nvIn,
-                                 const int32_t* __restrict__ ulo, const int32_t* __restrict__ uhi,
-                                 const float* __restrict__ vertex, const float* __restrict__ Qv,
-                                 uint64_t* __restrict__ key, uint32_t* __restrict__ val, float* __restrict__ costOut) {
-    const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= nu) return;
-    const int vi = ulo[u], vj = uhi[u];
-    float q[10];
+// one candidate per thread (decimate_gpu.cu:378-416); order key = (cost, candidate)
+__global__ void __launch_bounds__(128)
+edge_cost_kernel(int64_t Nv, int D, const int32_t* __restrict__ ustart, const int32_t* __restrict__ ulo, const int32_t* __restrict__ uhi,
+                 const float* __restrict__ vertex, const float* __restrict__ Qv, u64* __restrict__ key, float* __restrict__ costOut) {
+    const int nu = ustart[Nv];
+    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < nu; u += gridDim.x * blockDim.x) {
+        const int vi = ulo[u], vj = uhi[u];
+        float q[10];
 #pragma unroll
-    for (int t = 0; t < 10; ++t) q[t] = Qv[10 * (int64_t)vi + t] + Qv[10 * (int64_t)vj + t];
-    const float A[3][3] = {{q[0], q[1], q[2]}, {q[1], q[3], q[4]}, {q[2], q[4], q[5]}};
-    const float b[3] = {q[6], q[7], q[8]};
-    float x[3], cost;
-    const float rc = reduce_system(A, b, x);
-    if (rc > 1e-6f) cost = quadric_error(x, A, b, q[9]);
-    else {
-        const float ei = quadric_error(vertex + (int64_t)vi * D, A, b, q[9]);
-        const float ej = quadric_error(vertex + (int64_t)vj * D, A, b, q[9]);
-        cost = ei < ej ? ei : ej;
-    }
-    key[u] = ((uint64_t)sample_of(vi, nvIn, B) << 32) | cost_key(cost);
-    val[u] = (uint32_t)u;
-    if (costOut) costOut[u] = cost;
-}
-
-// first candidate of every sample (candidates are in ascending lower-vertex order)
-__global__ void segment_kernel(int B, int64_t nu, const int32_t* __restrict__ nvIn, const int32_t* __restrict__ ulo,
-                               int32_t* __restrict__ segstart) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s > B) return;
-    const int bound = s == 0 ? 0 : nvIn[s - 1];
-    int64_t lo = 0, hi = nu;
-    while (lo < hi) { const int64_t mid = (lo + hi) >> 1; if (ulo[mid] < bound) lo = mid + 1; else hi = mid; }
-    segstart[s] = (int32_t)lo;
-}
-
-__global__ void rank_kernel(int64_t nu, const uint32_t* __restrict__ sorted_u, uint32_t* __restrict__ rank) {
-    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < nu) rank[sorted_u[r]] = (uint32_t)r;
-}
-
-// ---------------------------------------------------------------------------- matching
-// live list of the first sweep: candidates of samples that still have vertices to remove
-__global__ void match_init_kernel(int64_t nu, int B, const int32_t* __restrict__ nvIn, const int32_t* __restrict__ want,
-                                  const int32_t* __restrict__ ulo, const int32_t* __restrict__ uhi,
-                                  uint32_t* __restrict__ list, int32_t* __restrict__ count) {
-    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x; i0 < nu; i0 += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t u = i0 + threadIdx.x;
-        bool take = false;
-        if (u < nu) {
-            const int lo = ulo[u], hi = uhi[u];
-            const int s = sample_of(lo, nvIn, B);
-            take = lo != hi && s < B && want[s] > 0;
+        for (int t = 0; t < 10; ++t) q[t] = Qv[10 * (int64_t)vi + t] + Qv[10 * (int64_t)vj + t];
+        const float A[3][3] = {{q[0], q[1], q[2]}, {q[1], q[3], q[4]}, {q[2], q[4], q[5]}};
+        const float b[3] = {q[6], q[7], q[8]};
+        float x[3], cost;
+        const float rc = reduce_system(A, b, x);
+        if (rc > 1e-6f) cost = quadric_error(x, A, b, q[9]);
+        else {
+            const float ei = quadric_error(vertex + (int64_t)vi * D, A, b, q[9]);
+            const float ej = quadric_error(vertex + (int64_t)vj * D, A, b, q[9]);
+            cost = ei < ej ? ei : ej;
         }
-        warp_append(take, (uint32_t)u, list, count);
+        key[u] = ((u64)cost_key(cost) << 32) | (u64)(uint32_t)u;
+        if (costOut) costOut[u] = cost;
     }
 }
 
-// round, first half: every live edge posts its rank at both ends
-__global__ void match_post_kernel(const uint32_t* __restrict__ list, const int32_t* __restrict__ count,
-                                  int32_t* __restrict__ next_count, const int32_t* __restrict__ ulo,
-                                  const int32_t* __restrict__ uhi, const uint32_t* __restrict__ rank,
-                                  const uint8_t* __restrict__ covered, uint32_t* __restrict__ vmin) {
-    const int n = *count;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *next_count = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t u = list[i];
-        const int lo = ulo[u], hi = uhi[u];
-        if (covered[lo] | covered[hi]) continue;
-        const uint32_t r = rank[u];
-        atomicMin(&vmin[lo], r);
-        atomicMin(&vmin[hi], r);
+// ---------------------------------------------------------------------------- clustering
+// All of both sweeps in one kernel.  Arrays that one step writes and a later one reads are read with __ldcg (the steps'
+// writers are other threads, in grid mode on other SMs).
+struct Cluster {
+    int64_t Nv;
+    int B;
+    const int32_t *nvIn, *want, *ustart, *ulo, *uhi;
+    const u64* key;
+    uint8_t* covered;
+    u64 *vminA, *vminB, *vminC;
+    uint32_t *listA, *listB, *taken, *joined;
+    int32_t *matched, *attached;          // (B) edges of the first / second sweep per sample
+    // grid mode only
+    u64* prefix;                          // (B) selection: key digits fixed so far
+    int32_t* rest;                        // (B) selection: how many are still to take
+    int32_t* hist;                        // (B << digit bits)
+    int digit_bits;
+    int32_t* counters;                    // 8 ints, zero
+    unsigned* barrier;                    // 2 words, zero: arrivals, give-up flag
+    int32_t* rounds;                      // rounds on the grid, live edges handed to the tail
+    int32_t* status;
+    int32_t *vtReplace, *head, *next;     // clusters as linked lists: head[root], next[member] hold id + 1, 0 = end
+};
+
+// The steps of a group of threads: a block over one sample's candidates, or the grid over all of them.
+constexpr int TAIL = 8192;                // live edges below which one block goes on alone: its rounds cost a block barrier
+constexpr long long BARRIER_CLOCKS = 4000000000ll;       // about two seconds
+
+__device__ __forceinline__ bool grid_barrier(unsigned* bar, int32_t* status) {
+    __shared__ int ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        ok = 1;
+        __threadfence();
+        const unsigned target = (atomicAdd(&bar[0], 1u) / gridDim.x + 1u) * gridDim.x;
+        const long long t0 = clock64();
+        unsigned seen, gone;
+        do {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&bar[0]) : "memory");
+            asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(gone) : "l"(&bar[1]) : "memory");
+            if (gone || clock64() - t0 > BARRIER_CLOCKS) { ok = 0; break; }
+        } while ((int)(seen - target) < 0);
+        if (!ok) { atomicExch(&bar[1], 1u); *status = PB200_ECUDA; }
+        __threadfence();
     }
+    __syncthreads();
+    return ok != 0;
 }
 
-// round, second half: an edge that holds the minimum at both ends is taken; edges with two
-// free ends stay live and clear the slots of the other minimum array for the next round
-__global__ void match_take_kernel(const uint32_t* __restrict__ list, const int32_t* __restrict__ count,
-                                  uint32_t* __restrict__ next_list, int32_t* __restrict__ next_count,
-                                  const int32_t* __restrict__ ulo, const int32_t* __restrict__ uhi,
-                                  const uint32_t* __restrict__ rank, uint8_t* covered,
-                                  const uint32_t* __restrict__ vmin, uint32_t* __restrict__ vmin_next,
-                                  int32_t* __restrict__ mflag) {
-    const int n = *count;
-    for (int i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
-        const int i = i0 + threadIdx.x;
-        bool live = false;
-        uint32_t u = 0;
-        if (i < n) {
-            u = list[i];
-            const int lo = ulo[u], hi = uhi[u];
-            const uint32_t r = rank[u];
-            if (vmin[lo] == r && vmin[hi] == r) {
-                mflag[r] = 1;
-                covered[lo] = 1;
-                covered[hi] = 1;
-            } else if (!(covered[lo] | covered[hi])) {
-                live = true;
-                vmin_next[lo] = NO_RANK;
-                vmin_next[hi] = NO_RANK;
-            }
-        }
-        warp_append(live, u, next_list, next_count);
+__device__ __forceinline__ bool is_covered(const uint8_t* c, int v) { return __ldcg(c + v) != 0; }
+
+// a live edge posts its key at both ends
+__device__ __forceinline__ void post_edge(const Cluster& p, uint32_t u, u64* vmin) {
+    const int lo = p.ulo[u], hi = p.uhi[u];
+    if (is_covered(p.covered, lo) || is_covered(p.covered, hi)) return;
+    const u64 k = p.key[u];
+    atomicMin(&vmin[lo], k);
+    atomicMin(&vmin[hi], k);
+}
+// 2: taken, 1: still live (the slots of the other array are cleared for the next round), 0: dead
+__device__ __forceinline__ int take_edge(const Cluster& p, uint32_t u, const u64* vmin, u64* vnext) {
+    const int lo = p.ulo[u], hi = p.uhi[u];
+    const u64 k = p.key[u];
+    if (__ldcg(&vmin[lo]) == k && __ldcg(&vmin[hi]) == k) {
+        p.covered[lo] = 1;
+        p.covered[hi] = 1;
+        return 2;
     }
+    if (is_covered(p.covered, lo) || is_covered(p.covered, hi)) return 0;
+    vnext[lo] = NO_KEY;
+    vnext[hi] = NO_KEY;
+    return 1;
+}
+// second sweep: the uncovered end of an edge with one covered end, or -1
+__device__ __forceinline__ int free_end(const Cluster& p, uint32_t u) {
+    const int lo = p.ulo[u], hi = p.uhi[u];
+    if (lo == hi) return -1;
+    const bool cl = is_covered(p.covered, lo), ch = is_covered(p.covered, hi);
+    return cl == ch ? -1 : (cl ? hi : lo);
+}
+__device__ __forceinline__ void join(const Cluster& p, int member, int root) {
+    p.vtReplace[member] = -root;
+    atomicAdd(&p.vtReplace[root], 1);
+    p.next[member] = atomicExch(&p.head[root], member + 1);
+}
+// first sweep applied (decimate_gpu.cu:568-584): the lower vertex is contracted into the higher one
+__device__ __forceinline__ void apply_taken(const Cluster& p, uint32_t u) { join(p, p.ulo[u], p.uhi[u]); }
+// second sweep applied (decimate_gpu.cu:586-612)
+__device__ __forceinline__ void apply_joined(const Cluster& p, uint32_t u) {
+    const int lo = p.ulo[u], hi = p.uhi[u];
+    const bool cl = is_covered(p.covered, lo);
+    const int seed = cl ? lo : hi, joiner = cl ? hi : lo;
+    const int rep = __ldcg(&p.vtReplace[seed]);
+    join(p, joiner, rep < 0 ? -rep : seed);
 }
 
-// the same rounds for a short live list, by one block until the list is empty; every round
-// takes at least the lowest-ranked live edge, so `count + 1` rounds bound the loop
-constexpr int TAIL_THREADS = 1024;
-constexpr int TAIL_LIMIT = 8192;
-__global__ void __launch_bounds__(TAIL_THREADS)
-match_tail_kernel(uint32_t* listA, uint32_t* listB, int32_t* countA, const int32_t* __restrict__ ulo,
-                  const int32_t* __restrict__ uhi, const uint32_t* __restrict__ rank, uint8_t* covered,
-                  uint32_t* vminA, uint32_t* vminB, int32_t* __restrict__ mflag, int32_t* __restrict__ rounds_out) {
-    __shared__ int32_t next_n;
-    uint32_t* list = listA;
-    uint32_t* next = listB;
-    uint32_t* vmin = vminA;
-    uint32_t* vmin_next = vminB;
-    int n = *countA;
-    const int limit = n + 1;
-    int rounds = 0;
-    while (n > 0 && rounds < limit) {
-        if (threadIdx.x == 0) next_n = 0;
-        for (int i = threadIdx.x; i < n; i += TAIL_THREADS) {
-            const uint32_t u = list[i];
-            const int lo = ulo[u], hi = uhi[u];
-            if (covered[lo] | covered[hi]) continue;
-            const uint32_t r = rank[u];
-            atomicMin(&vmin[lo], r);
-            atomicMin(&vmin[hi], r);
+// rounds of one block over the live list `from` (n edges; nullptr: the candidates u0 ... u0 + n) until none is left;
+// taken edges are appended to `taken`.  Every round takes at least the lowest live edge: n + 1 rounds bound the loop.
+template <typename OnTaken>
+__device__ void block_rounds(const Cluster& p, uint32_t u0, uint32_t* from, uint32_t* list0, uint32_t* list1, int n, u64* vmin, u64* vnext,
+                             OnTaken&& on_taken) {
+    __shared__ int32_t live[3];
+    if (threadIdx.x < 3) live[threadIdx.x] = 0;
+    __syncthreads();
+    uint32_t* out = list0;
+    uint32_t* other = list1;
+    int slot = 0;
+    for (int round = 0, limit = n + 1; n > 0 && round < limit; ++round) {
+        if (threadIdx.x == 0) live[(slot + 1) % 3] = 0;
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            const uint32_t u = from ? __ldcg(from + i) : u0 + i;
+            if (p.ulo[u] != p.uhi[u]) post_edge(p, u, vmin);
         }
         __syncthreads();
-        for (int i0 = 0; i0 < n; i0 += TAIL_THREADS) {
+        for (int i0 = 0; i0 < n; i0 += blockDim.x) {
             const int i = i0 + threadIdx.x;
-            bool live = false;
+            int what = 0;
             uint32_t u = 0;
             if (i < n) {
-                u = list[i];
-                const int lo = ulo[u], hi = uhi[u];
-                const uint32_t r = rank[u];
-                if (vmin[lo] == r && vmin[hi] == r) {
-                    mflag[r] = 1;
-                    covered[lo] = 1;
-                    covered[hi] = 1;
-                } else if (!(covered[lo] | covered[hi])) {
-                    live = true;
-                    vmin_next[lo] = NO_RANK;
-                    vmin_next[hi] = NO_RANK;
-                }
+                u = from ? __ldcg(from + i) : u0 + i;
+                if (p.ulo[u] != p.uhi[u]) what = take_edge(p, u, vmin, vnext);
             }
-            warp_append(live, u, next, &next_n);
+            on_taken(what == 2, u);
+            warp_append(what == 1, u, out, &live[slot]);
         }
         __syncthreads();
-        n = next_n;
+        n = live[slot];
+        slot = (slot + 1) % 3;
+        from = out;
+        uint32_t* t = out; out = other; other = t;
+        u64* tv = vmin; vmin = vnext; vnext = tv;
+    }
+    __syncthreads();
+}
+
+// k-th smallest key (k >= 1) among the n listed candidates, by a block: eight bits at a time from the top
+__device__ u64 block_select(const Cluster& p, const uint32_t* list, int n, int k, int ubits) {
+    __shared__ int32_t hist[256];
+    __shared__ int digit, left;
+    u64 prefix = 0;
+    for (int shift = 56; shift >= 0; shift -= 8) {
+        if (shift < 32 && shift >= ubits) { prefix <<= 8; continue; }          // candidate ids have no such digit
+        for (int i = threadIdx.x; i < 256; i += blockDim.x) hist[i] = 0;
         __syncthreads();
-        uint32_t* t = list; list = next; next = t;
-        uint32_t* tv = vmin; vmin = vmin_next; vmin_next = tv;
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            const u64 key = p.key[__ldcg(list + i)];
+            if (shift == 56 || (key >> (shift + 8)) == prefix) atomicAdd(&hist[(int)(key >> shift) & 255], 1);
+        }
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            int c[8], s = 0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) { c[j] = hist[threadIdx.x * 8 + j]; s += c[j]; }
+            int inc = s;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int t = __shfl_up_sync(0xffffffffu, inc, o); if ((int)threadIdx.x >= o) inc += t; }
+            int run = inc - s;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (run < k && run + c[j] >= k) { digit = threadIdx.x * 8 + j; left = k - run; }
+                run += c[j];
+            }
+        }
+        __syncthreads();
+        prefix = (prefix << 8) | (u64)digit;
+        k = left;
+        __syncthreads();
+    }
+    return prefix;
+}
+
+__device__ __forceinline__ int bit_length(int x) { return 32 - __clz(x); }
+
+// A block per sample.
+__global__ void __launch_bounds__(1024) cluster_samples_kernel(Cluster p) {
+    __shared__ int32_t count;
+    if (__ldcg(p.status) != 0) return;
+    for (int s = blockIdx.x; s < p.B; s += gridDim.x) {
+        const int v0 = s > 0 ? p.nvIn[s - 1] : 0, v1 = p.nvIn[s];
+        const int u0 = p.ustart[v0], n = p.ustart[v1] - u0, want = p.want[s];
+        const int ubits = bit_length(u0 + n);
+        uint32_t* taken = p.taken + v0;                        // at most one edge per two vertices
+        uint32_t* joined = p.joined + v0;                      // at most one edge per vertex
+        if (threadIdx.x == 0) count = 0;
+        __syncthreads();
+        if (want <= 0 || n == 0) continue;                     // uniform over the block
+        block_rounds(p, (uint32_t)u0, nullptr, p.listA + u0, p.listB + u0, n, p.vminA, p.vminB,
+                     [&](bool yes, uint32_t u) { warp_append(yes, u, taken, &count); });
+        const int matched = count;
+        const u64 last = matched > want ? block_select(p, taken, matched, want, ubits) : NO_KEY;
+        for (int i = threadIdx.x; i < matched; i += blockDim.x) {
+            const uint32_t u = __ldcg(taken + i);
+            if (p.key[u] <= last) apply_taken(p, u);
+        }
+        __syncthreads();
+        if (matched < want) {
+            if (threadIdx.x == 0) count = 0;
+            for (int i = threadIdx.x; i < n; i += blockDim.x) {
+                const int v = free_end(p, u0 + i);
+                if (v >= 0) atomicMin(&p.vminC[v], p.key[u0 + i]);
+            }
+            __syncthreads();
+            for (int i0 = 0; i0 < n; i0 += blockDim.x) {
+                const int i = i0 + threadIdx.x;
+                bool yes = false;
+                if (i < n) {
+                    const int v = free_end(p, u0 + i);
+                    yes = v >= 0 && __ldcg(&p.vminC[v]) == p.key[u0 + i];
+                }
+                warp_append(yes, u0 + i, joined, &count);
+            }
+            __syncthreads();
+            const int found = count;
+            const u64 end = found > want - matched ? block_select(p, joined, found, want - matched, ubits) : NO_KEY;
+            for (int i = threadIdx.x; i < found; i += blockDim.x) {
+                const uint32_t u = __ldcg(joined + i);
+                if (p.key[u] <= end) apply_joined(p, u);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// The whole grid over the whole batch (cooperative launch).
+constexpr int GRID_THREADS = 512;
+
+__device__ __forceinline__ int select_goal(const Cluster& p, int s, bool second) {      // edges to keep, or -1: all of them
+    const int m = __ldcg(&p.matched[s]), w = p.want[s];
+    if (!second) return m > w ? w : -1;
+    const int need = w - m;
+    return need > 0 && __ldcg(&p.attached[s]) > need ? need : -1;
+}
+
+// prefix[s] = last key to keep of every sample whose list is too long; false: the barrier gave up
+__device__ bool grid_select(const Cluster& p, const uint32_t* list, int n, bool second, int ubits, int32_t* flag) {
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+    for (int s = tid; s < p.B; s += nt) {
+        const int goal = select_goal(p, s, second);
+        p.prefix[s] = 0;
+        p.rest[s] = goal;
+        if (goal >= 0) *flag = 1;
+    }
+    if (!grid_barrier(p.barrier, p.status)) return false;
+    if (__ldcg(flag) == 0) return true;
+    const int bits = p.digit_bits, bins = 1 << bits;
+    for (int shift = 64 - bits; shift >= 0; shift -= bits) {
+        const bool empty = shift < 32 && shift >= ubits;
+        if (!empty) {
+            for (int i = tid; i < n; i += nt) {
+                const uint32_t u = __ldcg(list + i);
+                const int s = sample_of(p.ulo[u], p.nvIn, p.B);
+                if (__ldcg(&p.rest[s]) < 0) continue;
+                const u64 key = p.key[u];
+                if (shift + bits >= 64 || (key >> (shift + bits)) == __ldcg(&p.prefix[s]))
+                    atomicAdd(&p.hist[((int64_t)s << bits) + (int)((key >> shift) & (u64)(bins - 1))], 1);
+            }
+            if (!grid_barrier(p.barrier, p.status)) return false;
+        }
+        const int lane = threadIdx.x & 31;
+        for (int s = tid >> 5; s < p.B; s += nt >> 5) {         // a warp per sample
+            const int k = __ldcg(&p.rest[s]);
+            if (k < 0) continue;
+            u64 digit = 0;
+            int left = k;
+            if (!empty) {
+                int before = 0, at = -1, rem = 0;
+                for (int b0 = 0; b0 < bins; b0 += 32) {
+                    const int64_t h = ((int64_t)s << bits) + b0 + lane;
+                    const int c = b0 + lane < bins ? __ldcg(&p.hist[h]) : 0;
+                    if (b0 + lane < bins) p.hist[h] = 0;
+                    int inc = c;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) { const int t = __shfl_up_sync(0xffffffffu, inc, o); if (lane >= o) inc += t; }
+                    if (before + inc - c < k && before + inc >= k) { at = b0 + lane; rem = k - (before + inc - c); }
+                    before += __shfl_sync(0xffffffffu, inc, 31);
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, at >= 0);
+                const int src = m ? __ffs(m) - 1 : 0;
+                digit = (u64)(unsigned)__shfl_sync(0xffffffffu, at, src);
+                left = __shfl_sync(0xffffffffu, rem, src);
+            }
+            if (lane == 0) { p.prefix[s] = (__ldcg(&p.prefix[s]) << bits) | digit; p.rest[s] = left; }
+        }
+        if (!grid_barrier(p.barrier, p.status)) return false;
+    }
+    return true;
+}
+
+__global__ void __launch_bounds__(GRID_THREADS, 3) cluster_grid_kernel(Cluster p) {
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+    // the barrier's give-up flag shares the word: nobody raises it before everybody has passed the first barrier
+    if (__ldcg(p.status) != 0) return;
+    const int nu = p.ustart[p.Nv];
+    const int ubits = bit_length(nu);
+    int32_t* live = p.counters;             // [3] in turn
+    int32_t* ntaken = p.counters + 3;
+    int32_t* njoined = p.counters + 4;
+    int32_t* flags = p.counters + 5;        // [2]
+    // ---- first sweep
+    uint32_t *from = nullptr, *out = p.listA, *other = p.listB;
+    u64 *vmin = p.vminA, *vnext = p.vminB;
+    int n = nu, slot = 0, rounds = 0;
+    auto eligible = [&](uint32_t u) {
+        const int lo = p.ulo[u];
+        if (lo == p.uhi[u]) return false;
+        const int s = sample_of(lo, p.nvIn, p.B);
+        return s < p.B && p.want[s] > 0;
+    };
+    auto took = [&](bool yes, uint32_t u) {
+        warp_append(yes, u, p.taken, ntaken);
+        if (__any_sync(0xffffffffu, yes)) warp_count(yes ? sample_of(p.ulo[u], p.nvIn, p.B) : -1, p.matched);
+    };
+    while (n > TAIL || (from == nullptr && n > 0)) {
+        if (tid == 0) live[(slot + 1) % 3] = 0;
+        for (int i = tid; i < n; i += nt) {
+            const uint32_t u = from ? __ldcg(from + i) : (uint32_t)i;
+            if (from || eligible(u)) post_edge(p, u, vmin);
+        }
+        if (!grid_barrier(p.barrier, p.status)) return;
+        for (int i0 = blockIdx.x * blockDim.x; i0 < n; i0 += nt) {
+            const int i = i0 + threadIdx.x;
+            int what = 0;
+            uint32_t u = 0;
+            if (i < n) {
+                u = from ? __ldcg(from + i) : (uint32_t)i;
+                if (from || eligible(u)) what = take_edge(p, u, vmin, vnext);
+            }
+            took(what == 2, u);
+            warp_append(what == 1, u, out, &live[slot]);
+        }
+        if (!grid_barrier(p.barrier, p.status)) return;
+        n = __ldcg(&live[slot]);
+        slot = (slot + 1) % 3;
+        from = out;
+        uint32_t* t = out; out = other; other = t;
+        u64* tv = vmin; vmin = vnext; vnext = tv;
         ++rounds;
     }
-    if (threadIdx.x == 0) { *countA = n; *rounds_out = rounds; }
-}
-
-// matched edges per sample (prefix counts over ranks)
-__global__ void segment_count_kernel(int B, const int32_t* __restrict__ segstart, const int32_t* __restrict__ scan,
-                                     int32_t* __restrict__ per_sample) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < B) per_sample[s] = scan[segstart[s + 1]] - scan[segstart[s]];
-}
-
-// first sweep applied: the first want[s] matched edges of every sample in rank order
-// (decimate_gpu.cu:568-584): the lower vertex is contracted into the higher one
-__global__ void apply_matched_kernel(int64_t nu, int B, const int32_t* __restrict__ want, const int32_t* __restrict__ segstart,
-                                     const uint64_t* __restrict__ skey, const uint32_t* __restrict__ sorted_u,
-                                     const int32_t* __restrict__ mflag, const int32_t* __restrict__ mscan,
-                                     const int32_t* __restrict__ ulo, const int32_t* __restrict__ uhi,
-                                     int32_t* __restrict__ vtReplace) {
-    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= nu || !mflag[r]) return;
-    const int s = (int)(skey[r] >> 32);
-    if (s >= B) return;
-    if (mscan[r] - mscan[segstart[s]] >= want[s]) return;
-    const uint32_t u = sorted_u[r];
-    const int lo = ulo[u], hi = uhi[u];
-    vtReplace[lo] = -hi;
-    atomicAdd(&vtReplace[hi], 1);
-}
-
-// second sweep (decimate_gpu.cu:586-612), only where the first one ran out of edges before it
-// reached want[s]: an uncovered vertex joins through its lowest-ranked edge
-__global__ void attach_post_kernel(int64_t nu, int B, const int32_t* __restrict__ nvIn, const int32_t* __restrict__ want,
-                                   const int32_t* __restrict__ matched, const int32_t* __restrict__ ulo,
-                                   const int32_t* __restrict__ uhi, const uint32_t* __restrict__ rank,
-                                   const uint8_t* __restrict__ covered, uint32_t* __restrict__ vmin) {
-    const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= nu) return;
-    const int lo = ulo[u], hi = uhi[u];
-    if (lo == hi) return;
-    const int s = sample_of(lo, nvIn, B);
-    if (s >= B || matched[s] >= want[s]) return;
-    const int cl = covered[lo], ch = covered[hi];
-    if (cl == ch) return;
-    atomicMin(&vmin[cl ? hi : lo], rank[u]);
-}
-
-__global__ void attach_flag_kernel(int64_t nu, int B, const int32_t* __restrict__ nvIn, const int32_t* __restrict__ want,
-                                   const int32_t* __restrict__ matched, const int32_t* __restrict__ ulo,
-                                   const int32_t* __restrict__ uhi, const uint32_t* __restrict__ rank,
-                                   const uint8_t* __restrict__ covered, const uint32_t* __restrict__ vmin,
-                                   int32_t* __restrict__ aflag) {
-    const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= nu) return;
-    const int lo = ulo[u], hi = uhi[u];
-    if (lo == hi) return;
-    const int s = sample_of(lo, nvIn, B);
-    if (s >= B || matched[s] >= want[s]) return;
-    const int cl = covered[lo], ch = covered[hi];
-    if (cl == ch) return;
-    const uint32_t r = rank[u];
-    if (vmin[cl ? hi : lo] == r) aflag[r] = 1;
-}
-
-__global__ void apply_attach_kernel(int64_t nu, int B, const int32_t* __restrict__ want, const int32_t* __restrict__ matched,
-                                    const int32_t* __restrict__ segstart, const uint64_t* __restrict__ skey,
-                                    const uint32_t* __restrict__ sorted_u, const int32_t* __restrict__ aflag,
-                                    const int32_t* __restrict__ ascan, const int32_t* __restrict__ ulo,
-                                    const int32_t* __restrict__ uhi, const uint8_t* __restrict__ covered,
-                                    int32_t* vtReplace) {
-    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= nu || !aflag[r]) return;
-    const int s = (int)(skey[r] >> 32);
-    if (s >= B) return;
-    if (ascan[r] - ascan[segstart[s]] >= want[s] - matched[s]) return;
-    const uint32_t u = sorted_u[r];
-    const int lo = ulo[u], hi = uhi[u];
-    const int seed = covered[lo] ? lo : hi, joiner = covered[lo] ? hi : lo;
-    const int rep = vtReplace[seed];
-    const int root = rep < 0 ? -rep : seed;
-    vtReplace[joiner] = -root;
-    atomicAdd(&vtReplace[root], 1);
+    if (tid == 0 && p.rounds) { p.rounds[0] = rounds; p.rounds[1] = n; }
+    if (n > 0 && blockIdx.x == 0) block_rounds(p, 0u, from, out, other, n, vmin, vnext, took);
+    if (!grid_barrier(p.barrier, p.status)) return;
+    const int matched = __ldcg(ntaken);
+    if (!grid_select(p, p.taken, matched, false, ubits, &flags[0])) return;
+    for (int i = tid; i < matched; i += nt) {
+        const uint32_t u = __ldcg(p.taken + i);
+        const int s = sample_of(p.ulo[u], p.nvIn, p.B);
+        if (__ldcg(&p.rest[s]) < 0 || p.key[u] <= __ldcg(&p.prefix[s])) apply_taken(p, u);
+    }
+    // ---- second sweep, in the samples that the first one left short
+    auto short_of = [&](uint32_t u) {
+        const int s = sample_of(p.ulo[u], p.nvIn, p.B);
+        return s < p.B && __ldcg(&p.matched[s]) < p.want[s];
+    };
+    for (int s = tid; s < p.B; s += nt)
+        if (__ldcg(&p.matched[s]) < p.want[s]) flags[1] = 1;
+    if (!grid_barrier(p.barrier, p.status)) return;
+    if (__ldcg(&flags[1]) == 0) return;
+    for (int i = tid; i < nu; i += nt) {
+        const int v = free_end(p, i);
+        if (v >= 0 && short_of(i)) atomicMin(&p.vminC[v], p.key[i]);
+    }
+    if (!grid_barrier(p.barrier, p.status)) return;
+    for (int i0 = blockIdx.x * blockDim.x; i0 < nu; i0 += nt) {
+        const int i = i0 + threadIdx.x;
+        bool yes = false;
+        if (i < nu) {
+            const int v = free_end(p, i);
+            yes = v >= 0 && short_of(i) && __ldcg(&p.vminC[v]) == p.key[i];
+        }
+        warp_append(yes, (uint32_t)i, p.joined, njoined);
+        if (__any_sync(0xffffffffu, yes)) warp_count(yes ? sample_of(p.ulo[i], p.nvIn, p.B) : -1, p.attached);
+    }
+    if (!grid_barrier(p.barrier, p.status)) return;
+    const int found = __ldcg(njoined);
+    if (tid == 0) flags[0] = 0;
+    if (!grid_barrier(p.barrier, p.status)) return;
+    if (!grid_select(p, p.joined, found, true, ubits, &flags[0])) return;
+    for (int i = tid; i < found; i += nt) {
+        const uint32_t u = __ldcg(p.joined + i);
+        const int s = sample_of(p.ulo[u], p.nvIn, p.B);
+        if (__ldcg(&p.rest[s]) < 0 || p.key[u] <= __ldcg(&p.prefix[s])) apply_joined(p, u);
+    }
 }
 
 // -------------------------------------------------------------------- contraction, faces
-__global__ void cluster_key_kernel(int64_t Nv, const int32_t* __restrict__ vtReplace, int32_t* __restrict__ key) {
+// decimate_gpu.cu:403-441: a representative moves to the mean of its cluster (members added in ascending id), a vertex on its
+// own keeps its row, a contracted vertex's row is zero.  map: rows go to map[v] and rows with map[v] < 0 nowhere; NULL: to v.
+__global__ void __launch_bounds__(128)
+contract_kernel(int64_t Nv, int D, const int32_t* __restrict__ vtReplace, const int32_t* __restrict__ head, const int32_t* __restrict__ next,
+                const float* __restrict__ vertexIn, const int32_t* __restrict__ map, float* __restrict__ vertexOut) {
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < Nv) key[v] = vtReplace[v] < 0 ? -vtReplace[v] : -1;
-}
-
-// decimate_gpu.cu:403-441: a representative moves to the mean of its cluster, a vertex on its
-// own keeps its row, a contracted vertex's row is zero
-__global__ void contract_kernel(int64_t Nv, int D, const int32_t* __restrict__ vtReplace, const int32_t* __restrict__ rowptr,
-                                const int32_t* __restrict__ members, const float* __restrict__ vertexIn,
-                                float* __restrict__ vertexOut) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= Nv * D) return;
-    const int64_t v = i / D;
-    const int t = (int)(i - v * D);
+    if (v >= Nv) return;
+    const int64_t to = map ? map[v] : v;
+    if (to < 0) return;
     const int rep = vtReplace[v];
-    float out = 0.f;
-    if (rep > 0) {
-        float acc = 0.f;
-        for (int p = rowptr[v]; p < rowptr[v + 1]; ++p) acc += vertexIn[(int64_t)members[p] * D + t];
-        out = (acc + vertexIn[i]) / (rep + 1);
-    } else if (rep == 0) {
-        out = vertexIn[i];
+    const float* own = vertexIn + v * D;
+    float* out = vertexOut + to * D;
+    if (rep <= 0) {
+        for (int t = 0; t < D; ++t) out[t] = rep == 0 ? own[t] : 0.f;
+        return;
     }
-    vertexOut[i] = out;
+    constexpr int FEW = 16;
+    int id[FEW];
+    if (rep <= FEW) {
+        int n = 0;
+        for (int m = head[v]; m != 0 && n < rep; m = next[m - 1]) {
+            int j = n++ - 1;
+            while (j >= 0 && id[j] > m) { id[j + 1] = id[j]; --j; }
+            id[j + 1] = m;
+        }
+        for (int t = 0; t < D; ++t) {
+            float acc = 0.f;
+            for (int i = 0; i < n; ++i) acc += vertexIn[(int64_t)(id[i] - 1) * D + t];
+            out[t] = (acc + own[t]) / (rep + 1);
+        }
+    } else {
+        for (int t = 0; t < D; ++t) out[t] = 0.f;
+        for (int last = 0, i = 0; i < rep; ++i) {               // the next larger member, by a walk over the list
+            int m = 0x7fffffff;
+            for (int x = head[v], left = rep; x != 0 && left > 0; x = next[x - 1], --left) if (x > last && x < m) m = x;
+            if (m == 0x7fffffff) break;
+            for (int t = 0; t < D; ++t) out[t] += vertexIn[(int64_t)(m - 1) * D + t];
+            last = m;
+        }
+        for (int t = 0; t < D; ++t) out[t] = (out[t] + own[t]) / (rep + 1);
+    }
 }
 
-// decimate_gpu.cu:444-507
-__global__ void face_relabel_kernel(int64_t Nf, int B, const int32_t* __restrict__ mfIn, const int32_t* __restrict__ vtReplace,
-                                    const int32_t* __restrict__ faceIn, int32_t* __restrict__ faceOut,
-                                    uint8_t* __restrict__ isDegenerate, int32_t* __restrict__ kept, int32_t* __restrict__ mfOut) {
-    for (int64_t f0 = (int64_t)blockIdx.x * blockDim.x; f0 < Nf; f0 += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t f = f0 + threadIdx.x;
-        int s = -1 - (int)(threadIdx.x & 31);                   // lanes without a kept face: groups of one
+// decimate_gpu.cu:444-507; a block per scan tile of faces, whose kept ones it also counts
+__global__ void __launch_bounds__(scan::THREADS)
+face_relabel_kernel(int64_t Nf, int64_t Nv, int B, const int32_t* __restrict__ mfIn, const int32_t* __restrict__ vtReplace,
+                    const int32_t* __restrict__ faceIn, int32_t* __restrict__ faceOut, uint8_t* __restrict__ isDegenerate,
+                    int32_t* __restrict__ kept, int32_t* __restrict__ mfOut, int32_t* __restrict__ tile_sum) {
+    __shared__ int sh[scan::THREADS / 32];
+    int mine = 0;
+#pragma unroll 1
+    for (int j = 0; j < scan::ITEMS; ++j) {
+        const int64_t f = (int64_t)blockIdx.x * scan::TILE + j * scan::THREADS + threadIdx.x;
+        int s = -1;
         if (f < Nf) {
             int v[3];
+            bool deg = !read_face(faceIn, f, Nv, v);
+            if (!deg) {
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                v[c] = faceIn[3 * f + c];
-                const int rep = vtReplace[v[c]];
-                if (rep < 0) v[c] = -rep;
-                faceOut[3 * f + c] = v[c];
+                for (int c = 0; c < 3; ++c) {
+                    const int rep = vtReplace[v[c]];
+                    if (rep < 0) v[c] = -rep;
+                }
+                deg = v[0] == v[1] || v[0] == v[2] || v[1] == v[2];
             }
-            const bool deg = v[0] == v[1] || v[0] == v[2] || v[1] == v[2];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) faceOut[3 * f + c] = v[c];
             isDegenerate[f] = deg ? 1 : 0;
             if (!deg) {
                 kept[v[0]] = 1; kept[v[1]] = 1; kept[v[2]] = 1;
                 s = sample_of((int)f, mfIn, B);
                 if (s > B - 1) s = B - 1;
+                ++mine;
             }
         }
-        const unsigned m = __match_any_sync(0xffffffffu, s);
-        if (s >= 0 && (int)(threadIdx.x & 31) == __ffs(m) - 1) atomicAdd(&mfOut[s], __popc(m));
+        warp_count(s, mfOut);
     }
+    mine = scan::block_sum(mine, sh);
+    if (threadIdx.x == 0) tile_sum[blockIdx.x] = mine;
+}
+
+// kept vertices of a scan tile and of every sample
+__global__ void __launch_bounds__(scan::THREADS)
+kept_totals_kernel(int64_t Nv, int B, const int32_t* __restrict__ nvIn, const int32_t* __restrict__ kept, int32_t* __restrict__ tile_sum,
+                   int32_t* __restrict__ nvOut) {
+    __shared__ int sh[scan::THREADS / 32];
+    int mine = 0;
+#pragma unroll 1
+    for (int j = 0; j < scan::ITEMS; ++j) {
+        const int64_t v = (int64_t)blockIdx.x * scan::TILE + j * scan::THREADS + threadIdx.x;
+        const bool k = v < Nv && kept[v] != 0;
+        const int s = k ? sample_of((int)v, nvIn, B) : -1;
+        warp_count(s < B ? s : -1, nvOut);
+        mine += k;
+    }
+    mine = scan::block_sum(mine, sh);
+    if (threadIdx.x == 0) tile_sum[blockIdx.x] = mine;
 }
 
 // decimate_gpu.cu:509-533: kept vertices are numbered in order, the others map to -1
-__global__ void vertex_map_kernel(int64_t Nv, const int32_t* __restrict__ kept, const int32_t* __restrict__ kscan,
-                                  int32_t* __restrict__ vtMap) {
-    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < Nv) vtMap[v] = kept[v] ? kscan[v] : -1;
-}
-
-__global__ void sample_sizes_kernel(int B, const int32_t* __restrict__ nvIn, const int32_t* __restrict__ kscan,
-                                    int32_t* __restrict__ nvOut) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < B) nvOut[s] = kscan[nvIn[s]] - kscan[s == 0 ? 0 : nvIn[s - 1]];
+__global__ void __launch_bounds__(scan::THREADS)
+vertex_map_kernel(int64_t Nv, const int32_t* __restrict__ kept, const int32_t* __restrict__ tile_sum, int32_t* __restrict__ vtMap) {
+    __shared__ int sh[scan::THREADS / 32];
+    const int before = scan::tiles_before(tile_sum, blockIdx.x, sh);
+    const int64_t base = (int64_t)blockIdx.x * scan::TILE + (int64_t)threadIdx.x * scan::ITEMS;
+    int k[scan::ITEMS], s = 0;
+    scan::load_items(kept, Nv, base, k);
+#pragma unroll
+    for (int j = 0; j < scan::ITEMS; ++j) s += k[j];
+    int run = before + scan::block_exclusive(s, sh);
+#pragma unroll
+    for (int j = 0; j < scan::ITEMS; ++j) {
+        if (base + j < Nv) vtMap[base + j] = k[j] ? run : -1;
+        run += k[j];
+    }
 }
 
 __global__ void face_update_kernel(int64_t Nf, const int32_t* __restrict__ vtMap, const uint8_t* __restrict__ isDegenerate,
@@ -710,19 +910,98 @@ __global__ void face_update_kernel(int64_t Nf, const int32_t* __restrict__ vtMap
     for (int c = 0; c < 3; ++c) faceOut[3 * f + c] = vtMap[faceOut[3 * f + c]];
 }
 
+// The kept faces behind one another with the new vertex ids, and their geometry (the arithmetic of
+// triangle_geometry_kernel in adjacency.cu)
+__global__ void __launch_bounds__(scan::THREADS)
+emit_faces_kernel(int64_t Nf, int D, const int32_t* __restrict__ tile_sum, const uint8_t* __restrict__ isDegenerate,
+                  const int32_t* __restrict__ relabelled, const int32_t* __restrict__ vtMap, const float* __restrict__ vertex,
+                  int32_t* __restrict__ faceOut, float* __restrict__ geom) {
+    __shared__ int sh[scan::THREADS / 32];
+    __shared__ int step[scan::ITEMS + 1][scan::THREADS / 32];
+    const int before = scan::tiles_before(tile_sum, blockIdx.x, sh);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t base = (int64_t)blockIdx.x * scan::TILE;
+    unsigned keeps[scan::ITEMS];
+#pragma unroll
+    for (int j = 0; j < scan::ITEMS; ++j) {
+        const int64_t f = base + j * scan::THREADS + threadIdx.x;
+        keeps[j] = __ballot_sync(0xffffffffu, f < Nf && !isDegenerate[f]);
+        if (lane == 0) step[j][warp] = __popc(keeps[j]);
+    }
+    __syncthreads();
+    int run = before;
+#pragma unroll 1
+    for (int j = 0; j < scan::ITEMS; ++j) {
+        int at = run;
+        for (int w = 0; w < scan::THREADS / 32; ++w) { if (w < warp) at += step[j][w]; run += step[j][w]; }
+        if (!((keeps[j] >> lane) & 1u)) continue;
+        at += __popc(keeps[j] & ((1u << lane) - 1u));
+        const int64_t f = base + j * scan::THREADS + threadIdx.x;
+        int v[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) { v[c] = vtMap[relabelled[3 * f + c]]; faceOut[3 * (int64_t)at + c] = v[c]; }
+        const float *a = vertex + (int64_t)v[0] * D, *b = vertex + (int64_t)v[1] * D, *c = vertex + (int64_t)v[2] * D;
+        const float ax = a[0], ay = a[1], az = a[2];
+        const float ux = b[0] - ax, uy = b[1] - ay, uz = b[2] - az;
+        const float vx = c[0] - ax, vy = c[1] - ay, vz = c[2] - az;
+        float nx = uy * vz - uz * vy, ny = uz * vx - ux * vz, nz = ux * vy - uy * vx;
+        const float l2 = sqrtf(nx * nx + ny * ny + nz * nz);
+        const float den = l2 + 1e-10f;
+        nx = nx / den; ny = ny / den; nz = nz / den;
+        float* g = geom + 5 * (int64_t)at;
+        g[0] = nx; g[1] = ny; g[2] = nz;
+        g[3] = -(nx * ax + ny * ay + nz * az);
+        g[4] = l2 / 2.f;
+    }
+}
+
+// running totals of the samples' sizes and what is to be removed of each
+__global__ void __launch_bounds__(1024)
+begin_pass_kernel(int B, const int32_t* __restrict__ nv, const int32_t* __restrict__ mf, const int32_t* __restrict__ target,
+                  int32_t* __restrict__ nvCum, int32_t* __restrict__ mfCum, int32_t* __restrict__ want) {
+    __shared__ int wt[2][32];
+    __shared__ int carry[2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x < 2) carry[threadIdx.x] = 0;
+    __syncthreads();
+    for (int s0 = 0; s0 < B; s0 += 1024) {
+        const int s = s0 + threadIdx.x;
+        int x[2] = {s < B ? nv[s] : 0, s < B ? mf[s] : 0};
+        int inc[2] = {x[0], x[1]};
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+            for (int t = 0; t < 2; ++t) { const int y = __shfl_up_sync(0xffffffffu, inc[t], o); if (lane >= o) inc[t] += y; }
+        if (lane == 31) { wt[0][warp] = inc[0]; wt[1][warp] = inc[1]; }
+        __syncthreads();
+        int tot[2] = {carry[0], carry[1]};
+        for (int w = 0; w < 32; ++w)
+            for (int t = 0; t < 2; ++t) { if (w < warp) inc[t] += wt[t][w]; tot[t] += wt[t][w]; }
+        if (s < B) { nvCum[s] = carry[0] + inc[0]; mfCum[s] = carry[1] + inc[1]; want[s] = x[0] - target[s]; }
+        __syncthreads();
+        if (threadIdx.x < 2) carry[threadIdx.x] = tot[threadIdx.x];
+        __syncthreads();
+    }
+}
+
 // ------------------------------------------------------------------------ cluster merge
 // decimate_gpu.cu:750-812.  repB_work[vo] of a vertex B kept becomes its id in A; a vertex of A
 // whose representative was contracted in B follows that contraction.
-__global__ void merge_back_kernel(int64_t nvA, int64_t nvB, const int32_t* __restrict__ mapA, int32_t* __restrict__ repB_work) {
+__global__ void merge_back_kernel(int64_t nvA, int64_t nvB, const int32_t* __restrict__ repA, const int32_t* __restrict__ mapA,
+                                  int32_t* __restrict__ repB_work, int32_t* __restrict__ repOut) {
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nvA) return;
+    repOut[v] = repA[v];
     const int vo = mapA[v];
     if (vo >= 0 && vo < nvB && repB_work[vo] >= 0) repB_work[vo] = (int32_t)v;
 }
 __global__ void merge_follow_kernel(int64_t nvA, int64_t nvB, const int32_t* __restrict__ repA, const int32_t* __restrict__ mapA,
-                                    const int32_t* __restrict__ repB_work, int32_t* repOut, int32_t* __restrict__ status) {
+                                    const int32_t* __restrict__ repB_work, const int32_t* __restrict__ mapB, int32_t* repOut,
+                                    int32_t* __restrict__ mapOut, int32_t* __restrict__ status) {
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nvA) return;
+    const int own = mapA[v];
+    mapOut[v] = (own >= 0 && own < nvB) ? mapB[own] : -1;
     int64_t vi = v;
     if (repA[v] < 0) vi = -(int64_t)repA[v];
     if (vi >= nvA) { *status = PB200_EINDEX; return; }
@@ -738,13 +1017,6 @@ __global__ void merge_follow_kernel(int64_t nvA, int64_t nvB, const int32_t* __r
     repOut[v] = -root_a;
     atomicAdd(&repOut[root_a], 1);
 }
-__global__ void merge_map_kernel(int64_t nvA, int64_t nvB, const int32_t* __restrict__ mapA, const int32_t* __restrict__ mapB,
-                                 int32_t* __restrict__ mapOut) {
-    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= nvA) return;
-    const int vo = mapA[v];
-    mapOut[v] = (vo >= 0 && vo < nvB) ? mapB[vo] : -1;
-}
 
 // ---------------------------------------------------------------------------- workspace
 struct Carve {
@@ -759,47 +1031,118 @@ struct Carve {
 };
 
 struct Work {
-    uint64_t *keyA, *keyB;
-    uint32_t *valA, *valB, *rank, *listA, *listB, *vminA, *vminB;
-    int32_t *hist, *tile_sum, *flag, *scan, *ulo, *uhi, *segstart, *matched, *counters, *rowptr, *entries, *key,
-            *crowptr, *members, *kept, *kscan, *status;
-    uint8_t *bnd, *covered;
+    // cleared to 0 / to 0xff by one memset each
+    char *zero_begin, *ones_begin;
+    size_t zero_bytes, ones_bytes;
+    int32_t *cnt, *utile, *head, *kept, *matched, *attached, *hist, *counters, *status, *rounds;
+    unsigned* barrier;
+    uint8_t* covered;
+    u64 *vminA, *vminB, *vminC;
+    // written before they are read
+    int32_t *nvCum, *mfCum, *want, *rowptr, *entries, *hi, *ucnt, *ustart, *ulo, *uhi, *next, *tile, *ftile, *rest, *relabelled;
+    uint32_t *listA, *listB, *taken, *joined;
+    u64 *key, *prefix;
+    uint8_t *bnd, *degenerate;
     float* Q;
-    void *csr_ws, *ccsr_ws;
-    size_t csr_ws_bytes, ccsr_ws_bytes, total;
+    int digit_bits;
+    size_t total;
 };
 
 static Work carve(void* base, int64_t B, int64_t Nv, int64_t Nf) {
     Work w;
     Carve c(base);
-    const size_t Ne = (size_t)(3 * Nf);
-    const size_t nblocks = (size_t)ceil_div((int64_t)Ne, RS_TILE) + 1;
-    w.keyA = c.take<uint64_t>(Ne);  w.keyB = c.take<uint64_t>(Ne);
-    w.valA = c.take<uint32_t>(Ne);  w.valB = c.take<uint32_t>(Ne);
-    w.rank = c.take<uint32_t>(Ne);  w.listA = c.take<uint32_t>(Ne);  w.listB = c.take<uint32_t>(Ne);
-    w.vminA = c.take<uint32_t>((size_t)Nv);  w.vminB = c.take<uint32_t>((size_t)Nv);
-    w.hist = c.take<int32_t>(256 * nblocks + 1);
-    size_t longest = 256 * nblocks + 1;
-    if (Ne + 1 > longest) longest = Ne + 1;
-    if ((size_t)Nv + 1 > longest) longest = (size_t)Nv + 1;
-    w.tile_sum = c.take<int32_t>(scan_tiles_for((int64_t)longest) + 1);
-    w.flag = c.take<int32_t>(Ne + 1);  w.scan = c.take<int32_t>(Ne + 1);
+    const size_t Ne = (size_t)(3 * Nf), V = (size_t)Nv, S = (size_t)B;
+    w.digit_bits = B <= 4096 ? 8 : 4;                           // selection histograms of every sample: at most 64 MB
+    w.zero_begin = c.p;
+    w.cnt = c.take<int32_t>(V + 1);
+    w.utile = c.take<int32_t>((size_t)scan::tiles(Nv));
+    w.head = c.take<int32_t>(V);  w.kept = c.take<int32_t>(V + 1);  w.covered = c.take<uint8_t>(V);
+    w.matched = c.take<int32_t>(S);  w.attached = c.take<int32_t>(S);  w.hist = c.take<int32_t>(S << w.digit_bits);
+    w.counters = c.take<int32_t>(8);  w.barrier = c.take<unsigned>(2);  w.rounds = c.take<int32_t>(2);  w.status = c.take<int32_t>(1);
+    w.zero_bytes = c.used;
+    w.ones_begin = c.p ? c.p + c.used : nullptr;
+    w.vminA = c.take<u64>(V);  w.vminB = c.take<u64>(V);  w.vminC = c.take<u64>(V);
+    w.ones_bytes = c.used - w.zero_bytes;
+    w.nvCum = c.take<int32_t>(S);  w.mfCum = c.take<int32_t>(S);  w.want = c.take<int32_t>(S);
+    w.rowptr = c.take<int32_t>(V + 1);  w.entries = c.take<int32_t>(Ne);  w.hi = c.take<int32_t>(2 * Ne);
+    w.ucnt = c.take<int32_t>(V);  w.ustart = c.take<int32_t>(V + 1);
     w.ulo = c.take<int32_t>(Ne);  w.uhi = c.take<int32_t>(Ne);
-    w.segstart = c.take<int32_t>((size_t)B + 2);  w.matched = c.take<int32_t>((size_t)B + 1);
-    w.counters = c.take<int32_t>(8);
-    w.rowptr = c.take<int32_t>((size_t)Nv + 1);  w.entries = c.take<int32_t>(Ne);
-    w.key = c.take<int32_t>((size_t)Nv);
-    w.crowptr = c.take<int32_t>((size_t)Nv + 1);  w.members = c.take<int32_t>((size_t)Nv);
-    w.kept = c.take<int32_t>((size_t)Nv + 1);  w.kscan = c.take<int32_t>((size_t)Nv + 1);
-    w.status = c.take<int32_t>(4);
-    w.bnd = c.take<uint8_t>(Ne);  w.covered = c.take<uint8_t>((size_t)Nv);
-    w.Q = c.take<float>(10 * (size_t)Nv);
-    w.csr_ws_bytes = pb200_vertex_csr_workspace_bytes(Nf, Nv);
-    w.csr_ws = c.take<char>(w.csr_ws_bytes);
-    w.ccsr_ws_bytes = pb200_cluster_csr_workspace_bytes(Nv, Nv);
-    w.ccsr_ws = c.take<char>(w.ccsr_ws_bytes);
+    w.next = c.take<int32_t>(V);
+    w.tile = c.take<int32_t>((size_t)scan::tiles(Nv));  w.ftile = c.take<int32_t>((size_t)scan::tiles(Nf));
+    w.rest = c.take<int32_t>(S);  w.prefix = c.take<u64>(S);
+    w.key = c.take<u64>(Ne);                                    // long rows use it before the costs exist
+    w.listA = c.take<uint32_t>(2 * Ne);                         // and this (listA, listB)
+    w.listB = w.listA ? w.listA + Ne : nullptr;
+    w.taken = c.take<uint32_t>(V);  w.joined = c.take<uint32_t>(V);
+    w.relabelled = c.take<int32_t>(Ne);
+    w.bnd = c.take<uint8_t>(Ne);  w.degenerate = c.take<uint8_t>((size_t)Nf);
+    w.Q = c.take<float>(10 * V);
     w.total = c.used + 256;
     return w;
+}
+
+// Samples with at most this many faces go to a block each: their candidates (three per two faces) are some twenty per
+// thread, and a step then costs a block barrier instead of a grid barrier.
+constexpr int64_t SAMPLE_FACES = 16384;
+
+// Clustering, relabelled faces and vertex map of one pass: everything up to the sizes of its result.
+static int cluster_pass(const Work& w, int useArea, float wgtBnd, int64_t B, int64_t D, int64_t Nv, int64_t Nf, int64_t most_faces,
+                        const int32_t* nvIn, const int32_t* mfIn, const int32_t* want, const float* vertexIn, const int32_t* faceIn,
+                        const float* planeIn, int32_t* nvOut, int32_t* mfOut, int32_t* vtReplace, int32_t* vtMap, int32_t* relabelled,
+                        uint8_t* isDegenerate, float* edgeCost, cudaStream_t stream) {
+    PB_CUDA(cudaMemsetAsync(w.zero_begin, 0, w.zero_bytes, stream));
+    PB_CUDA(cudaMemsetAsync(nvOut, 0, sizeof(int32_t) * B, stream));
+    PB_CUDA(cudaMemsetAsync(mfOut, 0, sizeof(int32_t) * B, stream));
+    if (Nv == 0) return PB200_OK;
+    PB_CUDA(cudaMemsetAsync(vtReplace, 0, sizeof(int32_t) * Nv, stream));
+    const int vt = scan::tiles(Nv);
+    if (Nf > 0) {
+        PB_CUDA(cudaMemsetAsync(w.ones_begin, 0xff, w.ones_bytes, stream));
+        const unsigned fgrid = (unsigned)ceil_div(Nf, 256);
+        PB_LAUNCH("dec_count_corners", count_corners_kernel, fgrid, 256, 0, stream, Nf, Nv, faceIn, w.cnt, w.status);
+        PB_LAUNCH("scan_tile_totals", scan::tile_totals_kernel, vt, scan::THREADS, 0, stream, (const int32_t*)w.cnt, Nv, w.tile);
+        PB_LAUNCH("scan_row_starts", scan::row_starts_kernel, vt, scan::THREADS, 0, stream, (const int32_t*)w.cnt, Nv, (const int32_t*)w.tile,
+                  w.rowptr, w.cnt, (int32_t*)nullptr);
+        PB_LAUNCH("dec_fill_corners", fill_corners_kernel, fgrid, 256, 0, stream, Nf, Nv, faceIn, w.cnt, w.entries);
+        PB_LAUNCH("dec_vertex_edges", vertex_edges_kernel, (unsigned)ceil_div(Nv, 128), 128, 0, stream, Nv, faceIn, (const int32_t*)w.rowptr,
+                  w.entries, w.hi, w.ucnt, w.bnd, (int32_t*)w.key, w.listA, w.utile);
+        PB_LAUNCH("dec_candidates", candidates_kernel, vt, scan::THREADS, 0, stream, Nv, (int)B, nvIn, w.status,
+                  (const int32_t*)w.ucnt, (const int32_t*)w.utile,
+                  (const int32_t*)w.rowptr, (const int32_t*)w.hi, w.ustart, w.ulo, w.uhi);
+        PB_LAUNCH("dec_vertex_quadric", vertex_quadric_kernel, (unsigned)ceil_div(Nv, 128), 128, 0, stream, Nv, (int)D, useArea ? 1 : 0, wgtBnd,
+                  (const int32_t*)w.rowptr, (const int32_t*)w.entries, faceIn, planeIn, vertexIn, (const uint8_t*)w.bnd, w.Q);
+        PB_LAUNCH("dec_edge_cost", edge_cost_kernel, persistent_blocks(3 * Nf, 128, 16), 128, 0, stream, Nv, (int)D, (const int32_t*)w.ustart,
+                  (const int32_t*)w.ulo, (const int32_t*)w.uhi, vertexIn, (const float*)w.Q, w.key, edgeCost);
+        Cluster p;
+        p.Nv = Nv; p.B = (int)B; p.nvIn = nvIn; p.want = want; p.ustart = w.ustart; p.ulo = w.ulo; p.uhi = w.uhi; p.key = w.key;
+        p.covered = w.covered; p.vminA = w.vminA; p.vminB = w.vminB; p.vminC = w.vminC;
+        p.listA = w.listA; p.listB = w.listB; p.taken = w.taken; p.joined = w.joined; p.matched = w.matched; p.attached = w.attached;
+        p.prefix = w.prefix; p.rest = w.rest; p.hist = w.hist; p.digit_bits = w.digit_bits; p.counters = w.counters; p.barrier = w.barrier;
+        p.rounds = w.rounds; p.status = w.status; p.vtReplace = vtReplace; p.head = w.head; p.next = w.next;
+        if (most_faces <= SAMPLE_FACES) {
+            const int threads = most_faces <= 512 ? 256 : (most_faces <= 2048 ? 512 : 1024);
+            PB_LAUNCH("dec_cluster_samples", cluster_samples_kernel, (unsigned)(B < 65535 ? B : 65535), threads, 0, stream, p);
+        } else {
+            // as many blocks as have work and fit at once
+            int64_t blocks = ceil_div(3 * Nf, GRID_THREADS * 4);
+            int per_sm = 0;
+            PB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cluster_grid_kernel, GRID_THREADS, 0));
+            if (blocks > (int64_t)sm_count() * per_sm) blocks = (int64_t)sm_count() * per_sm;
+            PB_REQUIRE(blocks > 0, PB200_ECUDA, "mesh_simplify: the clustering kernel does not fit this device");
+            void* args[] = {&p};
+            LaunchScope scope("dec_cluster_grid", stream);
+            PB_CUDA(cudaLaunchCooperativeKernel((void*)cluster_grid_kernel, dim3((unsigned)blocks), dim3(GRID_THREADS), args, 0, stream));
+        }
+        PB_LAUNCH("dec_face_relabel", face_relabel_kernel, scan::tiles(Nf), scan::THREADS, 0, stream, Nf, Nv, (int)B, mfIn,
+                  (const int32_t*)vtReplace, faceIn, relabelled, isDegenerate, w.kept, mfOut, w.ftile);
+    }
+    PB_LAUNCH("dec_kept_totals", kept_totals_kernel, vt, scan::THREADS, 0, stream, Nv, (int)B, nvIn, (const int32_t*)w.kept, w.tile, nvOut);
+    PB_LAUNCH("dec_vertex_map", vertex_map_kernel, vt, scan::THREADS, 0, stream, Nv, (const int32_t*)w.kept, (const int32_t*)w.tile, vtMap);
+    return PB200_OK;
+}
+
+static bool sizes_ok(int64_t B, int64_t D, int64_t Nv, int64_t Nf) {
+    return B >= 1 && B < (1 << 20) && D >= 3 && D <= 4096 && Nv >= 0 && Nf >= 0 && Nf < (1LL << 29) && Nv < (1LL << 30);
 }
 
 }  // namespace dec
@@ -821,8 +1164,7 @@ int pb200_mesh_simplify(int useArea, float wgtBnd, int64_t B, int64_t D, int64_t
                         int32_t* faceOut, int32_t* vtReplace, int32_t* vtMap, uint8_t* isDegenerate, float* edgeCost,
                         int64_t* info, void* workspace, size_t workspace_bytes, void* stream_) {
     cudaStream_t stream = (cudaStream_t)stream_;
-    PB_REQUIRE(B >= 1 && B < (1 << 20) && D >= 3 && D <= 4096 && Nv >= 0 && Nf >= 0 && Nf < (1LL << 29) && Nv < (1LL << 30),
-               PB200_EINVAL, "mesh_simplify: bad sizes");
+    PB_REQUIRE(sizes_ok(B, D, Nv, Nf), PB200_EINVAL, "mesh_simplify: bad sizes");
     PB_REQUIRE(Nv > 0 || Nf == 0, PB200_EINVAL, "mesh_simplify: faces without vertices");
     PB_REQUIRE(nvIn && mfIn && nv2Remove && nvOut && mfOut, PB200_EINVAL, "mesh_simplify: null pointer");
     PB_REQUIRE(Nv == 0 || (vertexIn && vertexOut && vtReplace && vtMap), PB200_EINVAL, "mesh_simplify: null pointer");
@@ -832,6 +1174,7 @@ int pb200_mesh_simplify(int useArea, float wgtBnd, int64_t B, int64_t D, int64_t
     if (info) info[0] = info[1] = info[2] = info[3] = 0;
 
     // the per-sample running totals decide the segmentation: check them on the host (B values each)
+    int64_t most_faces = 0;
     {
         int32_t* h = (int32_t*)malloc(sizeof(int32_t) * 2 * (size_t)B);
         PB_REQUIRE(h, PB200_EINVAL, "mesh_simplify: out of host memory");
@@ -842,156 +1185,71 @@ int pb200_mesh_simplify(int useArea, float wgtBnd, int64_t B, int64_t D, int64_t
         for (int64_t s = 0; ok && s < B; ++s) {
             const int32_t pv = s ? h[s - 1] : 0, pf = s ? h[B + s - 1] : 0;
             ok = h[s] >= pv && h[B + s] >= pf;
+            if (h[B + s] - pf > most_faces) most_faces = h[B + s] - pf;
         }
         ok = ok && h[B - 1] == Nv && h[2 * B - 1] == Nf;
         free(h);
         if (e != cudaSuccess) return cuda_fail(e, "mesh_simplify: reading the sample sizes");
         PB_REQUIRE(ok, PB200_EINVAL, "mesh_simplify: nvIn / mfIn must be non-decreasing running totals ending at Nv / Nf");
     }
-
-    Work w = carve(workspace, B, Nv, Nf);
-    const int64_t Ne = 3 * Nf;
-    PB_CUDA(cudaMemsetAsync(w.status, 0, sizeof(int32_t) * 4, stream));
-    PB_CUDA(cudaMemsetAsync(w.counters, 0, sizeof(int32_t) * 8, stream));
-    PB_CUDA(cudaMemsetAsync(mfOut, 0, sizeof(int32_t) * B, stream));
-    if (Nv > 0) {
-        PB_CUDA(cudaMemsetAsync(vtReplace, 0, sizeof(int32_t) * Nv, stream));
-        PB_CUDA(cudaMemsetAsync(w.covered, 0, (size_t)Nv, stream));
-        PB_CUDA(cudaMemsetAsync(w.kept, 0, sizeof(int32_t) * (Nv + 1), stream));
-        PB_CUDA(cudaMemsetAsync(w.vminA, 0xff, sizeof(uint32_t) * Nv, stream));
-        PB_CUDA(cudaMemsetAsync(w.vminB, 0xff, sizeof(uint32_t) * Nv, stream));
-    }
-
-    int64_t nu = 0;
-    uint64_t* skey = w.keyA;       // (sample, cost) keys in rank order, once sorted
-    uint32_t* sorted_u = w.valA;   // candidate of every rank
-    if (Ne > 0 && Nv > 0) {
-        // ---- 1. edges
-        const int vbits = bit_length(Nv);
-        PB_LAUNCH("dec_edge_keys", edge_keys_kernel, (unsigned)ceil_div(Ne, 256), 256, 0, stream, Ne, Nv, vbits, faceIn,
-                  w.keyA, w.valA, w.status);
-        uint64_t *k = w.keyA, *kalt = w.keyB;
-        uint32_t *v = w.valA, *valt = w.valB;
-        int rc = radix_sort(k, kalt, v, valt, Ne, 2 * vbits, w.hist, w.tile_sum, stream);
-        if (rc != PB200_OK) return rc;
-        PB_LAUNCH("dec_edge_flags", edge_flags_kernel, (unsigned)ceil_div(Ne, 256), 256, 0, stream, Ne, Nv, vbits,
-                  (const uint64_t*)k, (const uint32_t*)v, w.bnd, w.flag);
-        rc = exclusive_scan(w.flag, Ne, w.scan, w.tile_sum, stream);
-        if (rc != PB200_OK) return rc;
-        PB_LAUNCH("dec_unique_write", unique_write_kernel, (unsigned)ceil_div(Ne, 256), 256, 0, stream, Ne, vbits,
-                  (const uint64_t*)k, (const int32_t*)w.scan, w.ulo, w.uhi);
-        int32_t h[2] = {0, 0};
-        PB_CUDA(cudaMemcpyAsync(&h[0], w.scan + Ne, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
-        PB_CUDA(cudaMemcpyAsync(&h[1], w.status, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
-        PB_CUDA(cudaStreamSynchronize(stream));
-        PB_REQUIRE(h[1] == 0, PB200_EINDEX, "mesh_simplify: face holds a vertex id outside [0, Nv)");
-        nu = h[0];
-
-        // ---- 2. quadrics
-        rc = pb200_build_vertex_csr(Nf, Nv, Nv, faceIn, nullptr, w.rowptr, w.entries, w.status + 1, w.csr_ws, w.csr_ws_bytes,
-                                    stream_);
-        if (rc != PB200_OK) return rc;
-        PB_LAUNCH("dec_vertex_quadric", vertex_quadric_kernel, (unsigned)ceil_div(Nv, 128), 128, 0, stream, Nv, (int)D,
-                  useArea ? 1 : 0, wgtBnd, (const int32_t*)w.rowptr, (const int32_t*)w.entries, faceIn, planeIn, vertexIn,
-                  (const uint8_t*)w.bnd, w.Q);
-    }
-    if (nu > 0) {
-        // ---- 3. costs and ranks
-        PB_LAUNCH("dec_edge_cost", edge_cost_kernel, (unsigned)ceil_div(nu, 128), 128, 0, stream, nu, Nv, (int)D, (int)B, nvIn,
-                  (const int32_t*)w.ulo, (const int32_t*)w.uhi, vertexIn, (const float*)w.Q, w.keyA, w.valA, edgeCost);
-        uint64_t *k = w.keyA, *kalt = w.keyB;
-        uint32_t *v = w.valA, *valt = w.valB;
-        int rc = radix_sort(k, kalt, v, valt, nu, 32 + bit_length(B), w.hist, w.tile_sum, stream);
-        if (rc != PB200_OK) return rc;
-        skey = k; sorted_u = v;
-        PB_LAUNCH("dec_rank", rank_kernel, (unsigned)ceil_div(nu, 256), 256, 0, stream, nu, (const uint32_t*)sorted_u, w.rank);
-        PB_LAUNCH("dec_segments", segment_kernel, (unsigned)ceil_div(B + 1, 128), 128, 0, stream, (int)B, nu, nvIn,
-                  (const int32_t*)w.ulo, w.segstart);
-
-        // ---- 4. first sweep as parallel rounds
-        PB_CUDA(cudaMemsetAsync(w.flag, 0, sizeof(int32_t) * (nu + 1), stream));
-        int32_t* count[2] = {w.counters, w.counters + 1};
-        uint32_t* list[2] = {w.listA, w.listB};
-        uint32_t* vmin[2] = {w.vminA, w.vminB};
-        const int grid = 4 * sm_count();
-        PB_LAUNCH("dec_match_init", match_init_kernel, grid, 256, 0, stream, nu, (int)B, nvIn, nv2Remove,
-                  (const int32_t*)w.ulo, (const int32_t*)w.uhi, list[0], count[0]);
-        int cur = 0;
-        int32_t live = 0;
-        int64_t rounds = 0;
-        PB_CUDA(cudaMemcpyAsync(&live, count[0], sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
-        PB_CUDA(cudaStreamSynchronize(stream));
-        while (live > TAIL_LIMIT) {
-            for (int r = 0; r < 4; ++r) {
-                PB_LAUNCH("dec_match_post", match_post_kernel, grid, 256, 0, stream, (const uint32_t*)list[cur],
-                          (const int32_t*)count[cur], count[cur ^ 1], (const int32_t*)w.ulo, (const int32_t*)w.uhi,
-                          (const uint32_t*)w.rank, (const uint8_t*)w.covered, vmin[cur]);
-                PB_LAUNCH("dec_match_take", match_take_kernel, grid, 256, 0, stream, (const uint32_t*)list[cur],
-                          (const int32_t*)count[cur], list[cur ^ 1], count[cur ^ 1], (const int32_t*)w.ulo,
-                          (const int32_t*)w.uhi, (const uint32_t*)w.rank, w.covered, (const uint32_t*)vmin[cur],
-                          vmin[cur ^ 1], w.flag);
-                cur ^= 1;
-                ++rounds;
-            }
-            PB_CUDA(cudaMemcpyAsync(&live, count[cur], sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
-            PB_CUDA(cudaStreamSynchronize(stream));
-        }
-        if (info) { info[1] = rounds; info[2] = live; }
-        if (live > 0) {
-            PB_LAUNCH("dec_match_tail", match_tail_kernel, 1, TAIL_THREADS, 0, stream, list[cur], list[cur ^ 1], count[cur],
-                      (const int32_t*)w.ulo, (const int32_t*)w.uhi, (const uint32_t*)w.rank, w.covered, vmin[cur],
-                      vmin[cur ^ 1], w.flag, w.counters + 2);
-        }
-        int rc2 = exclusive_scan(w.flag, nu, w.scan, w.tile_sum, stream);
-        if (rc2 != PB200_OK) return rc2;
-        PB_LAUNCH("dec_segment_count", segment_count_kernel, (unsigned)ceil_div(B, 128), 128, 0, stream, (int)B,
-                  (const int32_t*)w.segstart, (const int32_t*)w.scan, w.matched);
-        PB_LAUNCH("dec_apply_matched", apply_matched_kernel, (unsigned)ceil_div(nu, 256), 256, 0, stream, nu, (int)B, nv2Remove,
-                  (const int32_t*)w.segstart, (const uint64_t*)skey, (const uint32_t*)sorted_u, (const int32_t*)w.flag,
-                  (const int32_t*)w.scan, (const int32_t*)w.ulo, (const int32_t*)w.uhi, vtReplace);
-
-        // ---- 5. second sweep
-        PB_CUDA(cudaMemsetAsync(w.vminA, 0xff, sizeof(uint32_t) * Nv, stream));
-        PB_CUDA(cudaMemsetAsync(w.flag, 0, sizeof(int32_t) * (nu + 1), stream));
-        PB_LAUNCH("dec_attach_post", attach_post_kernel, (unsigned)ceil_div(nu, 256), 256, 0, stream, nu, (int)B, nvIn, nv2Remove,
-                  (const int32_t*)w.matched, (const int32_t*)w.ulo, (const int32_t*)w.uhi, (const uint32_t*)w.rank,
-                  (const uint8_t*)w.covered, w.vminA);
-        PB_LAUNCH("dec_attach_flag", attach_flag_kernel, (unsigned)ceil_div(nu, 256), 256, 0, stream, nu, (int)B, nvIn, nv2Remove,
-                  (const int32_t*)w.matched, (const int32_t*)w.ulo, (const int32_t*)w.uhi, (const uint32_t*)w.rank,
-                  (const uint8_t*)w.covered, (const uint32_t*)w.vminA, w.flag);
-        rc2 = exclusive_scan(w.flag, nu, w.scan, w.tile_sum, stream);
-        if (rc2 != PB200_OK) return rc2;
-        PB_LAUNCH("dec_apply_attach", apply_attach_kernel, (unsigned)ceil_div(nu, 256), 256, 0, stream, nu, (int)B, nv2Remove,
-                  (const int32_t*)w.matched, (const int32_t*)w.segstart, (const uint64_t*)skey, (const uint32_t*)sorted_u,
-                  (const int32_t*)w.flag, (const int32_t*)w.scan, (const int32_t*)w.ulo, (const int32_t*)w.uhi,
-                  (const uint8_t*)w.covered, vtReplace);
-    }
-    if (info) info[0] = nu;
-
-    // ---- 6. contraction, faces, vertex map
-    if (Nv > 0) {
-        PB_LAUNCH("dec_cluster_key", cluster_key_kernel, (unsigned)ceil_div(Nv, 256), 256, 0, stream, Nv,
-                  (const int32_t*)vtReplace, w.key);
-        int rc = pb200_build_key_csr(Nv, Nv, w.key, 1, w.crowptr, w.members, w.status + 2, w.ccsr_ws, w.ccsr_ws_bytes, stream_);
-        if (rc != PB200_OK) return rc;
-        PB_LAUNCH("dec_contract", contract_kernel, (unsigned)ceil_div(Nv * D, 256), 256, 0, stream, Nv, (int)D,
-                  (const int32_t*)vtReplace, (const int32_t*)w.crowptr, (const int32_t*)w.members, vertexIn, vertexOut);
-    }
-    if (Nf > 0)
-        PB_LAUNCH("dec_face_relabel", face_relabel_kernel, 4 * sm_count(), 256, 0, stream, Nf, (int)B, mfIn,
-                  (const int32_t*)vtReplace, faceIn, faceOut, isDegenerate, w.kept, mfOut);
-    {
-        int rc = exclusive_scan(w.kept, Nv, w.kscan, w.tile_sum, stream);
-        if (rc != PB200_OK) return rc;
-        if (Nv > 0)
-            PB_LAUNCH("dec_vertex_map", vertex_map_kernel, (unsigned)ceil_div(Nv, 256), 256, 0, stream, Nv,
-                      (const int32_t*)w.kept, (const int32_t*)w.kscan, vtMap);
-        PB_LAUNCH("dec_sample_sizes", sample_sizes_kernel, (unsigned)ceil_div(B, 128), 128, 0, stream, (int)B, nvIn,
-                  (const int32_t*)w.kscan, nvOut);
-    }
+    const Work w = carve(workspace, B, Nv, Nf);
+    int rc = cluster_pass(w, useArea, wgtBnd, B, D, Nv, Nf, most_faces, nvIn, mfIn, nv2Remove, vertexIn, faceIn, planeIn, nvOut, mfOut,
+                          vtReplace, vtMap, faceOut, isDegenerate, edgeCost, stream);
+    if (rc) return rc;
+    if (Nv > 0)
+        PB_LAUNCH("dec_contract", contract_kernel, (unsigned)ceil_div(Nv, 128), 128, 0, stream, Nv, (int)D, (const int32_t*)vtReplace,
+                  (const int32_t*)w.head, (const int32_t*)w.next, vertexIn, (const int32_t*)nullptr, vertexOut);
     if (Nf > 0)
         PB_LAUNCH("dec_face_update", face_update_kernel, (unsigned)ceil_div(Nf, 256), 256, 0, stream, Nf,
                   (const int32_t*)vtMap, (const uint8_t*)isDegenerate, faceOut);
+    int32_t status = 0, counts[3] = {0, 0, 0};
+    PB_CUDA(cudaMemcpyAsync(&status, w.status, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
+    if (info && Nf > 0) {
+        PB_CUDA(cudaMemcpyAsync(&counts[0], w.ustart + Nv, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
+        PB_CUDA(cudaMemcpyAsync(&counts[1], w.rounds, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
+    }
+    PB_CUDA(cudaStreamSynchronize(stream));
+    PB_REQUIRE(status != PB200_EINDEX, PB200_EINDEX, "mesh_simplify: face holds a vertex id outside [0, Nv)");
+    PB_REQUIRE(status != ECROSS, PB200_EINDEX, "mesh_simplify: a face joins vertices of two samples");
+    PB_REQUIRE(status == 0, PB200_ECUDA, "mesh_simplify: a wait inside the clustering kernel ran out");
+    if (info) { info[0] = counts[0]; info[1] = counts[1]; info[2] = counts[2]; }
+    return PB200_OK;
+}
+
+int pb200_decimate_begin(int useArea, float wgtBnd, int64_t B, int64_t D, int64_t Nv, int64_t Nf, int64_t mostFaces, const int32_t* nv,
+                         const int32_t* mf, const int32_t* target, const float* vertexIn, const int32_t* faceIn, const float* planeIn,
+                         int32_t* nvOut, int32_t* mfOut, int32_t* status, int32_t* vtReplace, int32_t* vtMap, void* workspace,
+                         size_t workspace_bytes, void* stream_) {
+    cudaStream_t stream = (cudaStream_t)stream_;
+    PB_REQUIRE(sizes_ok(B, D, Nv, Nf) && Nv > 0, PB200_EINVAL, "decimate_begin: bad sizes");
+    PB_REQUIRE(nv && mf && target && nvOut && mfOut && status && vertexIn && vtReplace && vtMap && (Nf == 0 || (faceIn && planeIn)),
+               PB200_EINVAL, "decimate_begin: null pointer");
+    PB_REQUIRE(workspace && workspace_bytes >= pb200_mesh_simplify_workspace_bytes(B, Nv, Nf), PB200_EWORKSPACE,
+               "decimate_begin: workspace too small");
+    const Work w = carve(workspace, B, Nv, Nf);
+    PB_LAUNCH("dec_begin_pass", begin_pass_kernel, 1, 1024, 0, stream, (int)B, nv, mf, target, w.nvCum, w.mfCum, w.want);
+    int rc = cluster_pass(w, useArea, wgtBnd, B, D, Nv, Nf, mostFaces, w.nvCum, w.mfCum, w.want, vertexIn, faceIn, planeIn, nvOut, mfOut,
+                          vtReplace, vtMap, w.relabelled, w.degenerate, nullptr, stream);
+    if (rc) return rc;
+    PB_CUDA(cudaMemcpyAsync(status, w.status, sizeof(int32_t), cudaMemcpyDeviceToDevice, stream));
+    return PB200_OK;
+}
+
+int pb200_decimate_finish(int64_t B, int64_t D, int64_t Nv, int64_t Nf, const float* vertexIn, const int32_t* vtReplace,
+                          const int32_t* vtMap, float* vertexOut, int32_t* faceOut, float* geometryOut, void* workspace,
+                          size_t workspace_bytes, void* stream_) {
+    cudaStream_t stream = (cudaStream_t)stream_;
+    PB_REQUIRE(sizes_ok(B, D, Nv, Nf) && Nv > 0, PB200_EINVAL, "decimate_finish: bad sizes");
+    PB_REQUIRE(vertexIn && vtReplace && vtMap && vertexOut && (Nf == 0 || (faceOut && geometryOut)), PB200_EINVAL,
+               "decimate_finish: null pointer");
+    PB_REQUIRE(workspace && workspace_bytes >= pb200_mesh_simplify_workspace_bytes(B, Nv, Nf), PB200_EWORKSPACE,
+               "decimate_finish: workspace too small");
+    const Work w = carve(workspace, B, Nv, Nf);
+    PB_LAUNCH("dec_contract", contract_kernel, (unsigned)ceil_div(Nv, 128), 128, 0, stream, Nv, (int)D, vtReplace, (const int32_t*)w.head,
+              (const int32_t*)w.next, vertexIn, vtMap, vertexOut);
+    if (Nf > 0)
+        PB_LAUNCH("dec_emit_faces", emit_faces_kernel, scan::tiles(Nf), scan::THREADS, 0, stream, Nf, (int)D, (const int32_t*)w.ftile,
+                  (const uint8_t*)w.degenerate, (const int32_t*)w.relabelled, vtMap, (const float*)vertexOut, faceOut, geometryOut);
     return PB200_OK;
 }
 
@@ -1009,12 +1267,10 @@ int pb200_combine_clusters(int64_t nvA, int64_t nvB, const int32_t* repA, const 
     if (nvA == 0) return PB200_OK;
     int32_t* rb = (int32_t*)workspace;
     if (nvB > 0) PB_CUDA(cudaMemcpyAsync(rb, repB, sizeof(int32_t) * nvB, cudaMemcpyDeviceToDevice, stream));
-    PB_CUDA(cudaMemcpyAsync(repOut, repA, sizeof(int32_t) * nvA, cudaMemcpyDeviceToDevice, stream));
     const unsigned grid = (unsigned)ceil_div(nvA, 256);
-    PB_LAUNCH("dec_merge_back", merge_back_kernel, grid, 256, 0, stream, nvA, nvB, mapA, rb);
-    PB_LAUNCH("dec_merge_follow", merge_follow_kernel, grid, 256, 0, stream, nvA, nvB, repA, mapA, (const int32_t*)rb, repOut,
-              status);
-    PB_LAUNCH("dec_merge_map", merge_map_kernel, grid, 256, 0, stream, nvA, nvB, mapA, mapB, mapOut);
+    PB_LAUNCH("dec_merge_back", merge_back_kernel, grid, 256, 0, stream, nvA, nvB, repA, mapA, rb, repOut);
+    PB_LAUNCH("dec_merge_follow", merge_follow_kernel, grid, 256, 0, stream, nvA, nvB, repA, mapA, (const int32_t*)rb, mapB, repOut,
+              mapOut, status);
     return PB200_OK;
 }
 

@@ -15,9 +15,13 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
 
+#include <array>
+#include <list>
 #include <mutex>
 #include <stdexcept>
 #include <string>
+#include <unordered_map>
+#include <vector>
 
 #include "../../include/picasso_b200.h"
 
@@ -1028,6 +1032,224 @@ Tensor segment_mean(const Tensor& input, const Tensor& ends) {
     return out;
 }
 
+// -------------------------------------------------------------------------------------------------------- decimation
+Tensor on_device(const std::vector<int64_t>& values, const Tensor& like) {
+    return at::tensor(values, at::TensorOptions().dtype(at::kInt)).to(like.device());
+}
+std::vector<int64_t> on_host(const Tensor& t) {
+    const Tensor h = t.cpu();
+    const int32_t* p = h.data_ptr<int32_t>();
+    return std::vector<int64_t>(p, p + h.numel());
+}
+
+// The pass loop of mesh_decimation (picasso/mesh/pi_modules/decimate.py:5-48) with one synchronisation per pass: the host
+// reads the samples' new sizes, which it needs to allocate the result, and decides on the next pass by them.
+// nv_host / mf_host / target_host: the samples' sizes where the caller knows them already (empty: read here).
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, std::vector<int64_t>, std::vector<int64_t>>
+mesh_decimation(const Tensor& vertex_in, const Tensor& face_in, const Tensor& geometry_in, const Tensor& nv_in, const Tensor& mf_in,
+                const OptTensor& target_in, bool use_area, double wgt_bnd, std::vector<int64_t> nv_host, std::vector<int64_t> mf_host,
+                std::vector<int64_t> target_host) {
+    c10::InferenceMode inference(false);
+    at::NoGradGuard no_grad;
+    Tensor vertex = vertex_in.contiguous(), face = face_in.contiguous(), geometry = geometry_in.contiguous();
+    check(vertex, "vertexIn", 2, at::kFloat);
+    check(face, "faceIn", 2, at::kInt);
+    check(geometry, "planeIn", 2, at::kFloat);
+    if (vertex.size(1) < 3) fail("The shape of input vertex should be (Nv, 3+)).");
+    if (face.size(1) != 3) fail("The shape of input face should be (Nf, 3)).");
+    if (geometry.size(0) != face.size(0) || geometry.size(1) != 5) fail("The shape of input face normals should be (Nf, 5)).");
+    Scope s(vertex);
+    const auto i32 = s.f32.dtype(at::kInt);
+    const int64_t D = vertex.size(1), B = nv_in.size(0);
+    Tensor nv = nv_in, mf = mf_in, rep, map;
+    if (nv_host.empty()) {
+        const std::vector<int64_t> all = on_host(at::cat({nv_in.to(at::kInt), mf_in.to(at::kInt), target_in.value().to(at::kInt)}));
+        nv_host.assign(all.begin(), all.begin() + B);
+        mf_host.assign(all.begin() + B, all.begin() + 2 * B);
+        target_host.assign(all.begin() + 2 * B, all.end());
+    }
+    auto sum = [](const std::vector<int64_t>& v) { int64_t t = 0; for (int64_t x : v) t += x; return t; };
+    auto more = [&] { for (int64_t k = 0; k < B; ++k) if (nv_host[k] > target_host[k]) return true; return false; };
+    const bool any = more();
+    if (any && (sum(nv_host) != vertex.size(0) || sum(mf_host) != face.size(0)))
+        fail("mesh_simplify: nvIn / mfIn must be the samples' vertex and face counts");
+    const Tensor target = target_in.has_value() ? target_in->to(vertex.device(), at::kInt).contiguous() : on_device(target_host, vertex);
+    while (more()) {
+        const int64_t Nv = vertex.size(0), Nf = face.size(0);
+        const Tensor sizes = at::empty({2 * B + 1}, i32), vt_replace = at::empty({Nv}, i32), vt_map = at::empty({Nv}, i32);
+        int32_t* sz = sizes.data_ptr<int32_t>();
+        const size_t nb = pb200_mesh_simplify_workspace_bytes(B, Nv, Nf);
+        Tensor ws = s.bytes(nb);
+        const Tensor nv32 = nv.to(at::kInt).contiguous(), mf32 = mf.to(at::kInt).contiguous();
+        int64_t most = 0;
+        for (int64_t m : mf_host) most = m > most ? m : most;
+        call(pb200_decimate_begin(use_area, (float)wgt_bnd, B, D, Nv, Nf, most, ip(nv32), ip(mf32), ip(target), fp(vertex), ip(face),
+                                  fp(geometry), sz, sz + B, sz + 2 * B, vt_replace.data_ptr<int32_t>(), vt_map.data_ptr<int32_t>(),
+                                  ws.data_ptr(), nb, s.stream),
+             "pb200_decimate_begin");
+        const std::vector<int64_t> now = on_host(sizes);
+        if (now[2 * B] == PB200_EINDEX) fail("mesh_simplify: face holds a vertex id outside [0, Nv)");
+        if (now[2 * B] == 1) fail("mesh_simplify: a face joins vertices of two samples");
+        if (now[2 * B] != 0) fail("mesh_simplify: a wait inside the clustering kernel ran out");
+        bool removed = false;
+        for (int64_t k = 0; k < B; ++k) removed |= now[k] < nv_host[k];
+        if (!removed) break;               // nothing left to contract (no candidate edges): the reference would loop forever
+        nv_host.assign(now.begin(), now.begin() + B);
+        mf_host.assign(now.begin() + B, now.begin() + 2 * B);
+        const int64_t Nv2 = sum(nv_host), Nf2 = sum(mf_host);
+        Tensor vertex2 = s.floats({Nv2, D}), face2 = at::empty({Nf2, 3}, i32), geometry2 = s.floats({Nf2, 5});
+        // an empty result still needs addresses for the checks of the call; nothing is written there
+        call(pb200_decimate_finish(B, D, Nv, Nf, fp(vertex), ip(vt_replace), ip(vt_map), Nv2 ? fpm(vertex2) : fpm(geometry),
+                                   Nf2 ? face2.data_ptr<int32_t>() : sz, Nf2 ? fpm(geometry2) : fpm(geometry), ws.data_ptr(), nb, s.stream),
+             "pb200_decimate_finish");
+        if (!rep.defined()) {
+            rep = vt_replace;
+            map = vt_map;
+        } else {
+            const int64_t nvA = rep.size(0);
+            Tensor rep2 = at::empty({nvA}, i32), map2 = at::empty({nvA}, i32), work = at::empty({Nv + 2}, i32);
+            int32_t* w = work.data_ptr<int32_t>();
+            call(pb200_combine_clusters(nvA, Nv, ip(rep), ip(map), ip(vt_replace), ip(vt_map), rep2.data_ptr<int32_t>(),
+                                        map2.data_ptr<int32_t>(), w + Nv + 1, w, sizeof(int32_t) * (size_t)(Nv + 1), s.stream),
+                 "pb200_combine_clusters");
+            rep = rep2;
+            map = map2;
+        }
+        vertex = vertex2;
+        face = face2;
+        geometry = geometry2;
+        nv = sizes.narrow(0, 0, B);
+        mf = sizes.narrow(0, B, B);
+    }
+    if (!rep.defined()) {
+        rep = at::zeros({vertex.size(0)}, i32);
+        map = at::arange(vertex.size(0), i32);
+        return {vertex_in, face_in, geometry_in, nv, mf, rep, map, nv_host, mf_host};
+    }
+    return {vertex, face, geometry, nv, mf, rep, map, nv_host, mf_host};
+}
+
+// One mesh level: what topology.prepare_level returns, with the status word of the CSR build.
+std::tuple<OptTensor, OptTensor, Tensor, Tensor, Tensor, Tensor, Tensor>
+level_prepare(const Tensor& vertex, const Tensor& face, const OptTensor& vt_map, int64_t nv_out, int L, bool orient, bool want_geometry,
+              bool want_normals) {
+    at::NoGradGuard no_grad;
+    Scope s(face);
+    const auto i32 = s.f32.dtype(at::kInt);
+    const int64_t nv_in = vertex.size(0), nf = face.size(0), K = (int64_t)(L + 1) * (L + 1);
+    OptTensor geometry, normals;
+    if (want_geometry) geometry = s.floats({nf, 5});
+    if (want_normals) normals = s.floats({nf, 3});
+    Tensor coeff = s.floats({nf, K}), nf_count = at::empty({nv_out}, i32), rowptr = at::empty({nv_out + 1}, i32),
+           entries = at::empty({nf > 0 ? 3 * nf : 1}, i32), status = at::empty({1}, i32);
+    const size_t nb = pb200_vertex_csr_workspace_bytes(nf, nv_out);
+    Tensor ws = s.bytes(nb);
+    call(pb200_level_prepare(nf, nv_in, nv_out, (int)vertex.size(1), fp(vertex), ip(face), vt_map.has_value() ? ip(*vt_map) : nullptr, L,
+                             orient ? 1 : 0, geometry.has_value() ? fpm(*geometry) : nullptr, normals.has_value() ? fpm(*normals) : nullptr,
+                             fpm(coeff), nf_count.data_ptr<int32_t>(), rowptr.data_ptr<int32_t>(), entries.data_ptr<int32_t>(),
+                             status.data_ptr<int32_t>(), ws.data_ptr(), nb, s.stream),
+         "pb200_level_prepare");
+    return {geometry, normals, coeff, nf_count, rowptr, entries, status};
+}
+
+// -------------------------------------------------------------------------------------------------- topology cache
+// Structures derived from index tensors (CSRs, sample means, running totals), found again by the tensors they were made
+// from.  An entry is named by kind, addresses and two numbers; it is good while the index tensors' storages are the ones it
+// was made from (weak references: the cache does not keep a batch's tensors alive, and memory that was freed and handed out
+// again is another storage) and their version counters have not moved.  Entries of storages that are gone are dropped at
+// the next insertion: a program that brings a new batch every step holds the structures of the batches it holds, no more.
+// Otherwise least recently used ones go when the bytes exceed the budget.  A structure used on a stream other than the one
+// it was made on is recorded there, so that dropping it is safe at any time.  All calls run under the GIL.
+struct TopologyCache {
+    struct Source {
+        c10::weak_intrusive_ptr<c10::StorageImpl> storage;
+        int64_t version;
+        explicit Source(const Tensor& t) : storage(t.storage().getWeakStorageImpl()), version(t._version()) {}
+        bool is(const Tensor& t) const {
+            return !storage.expired() && storage._unsafe_get_target() == t.storage().unsafeGetStorageImpl() && version == (int64_t)t._version();
+        }
+    };
+    struct Entry {
+        std::vector<Source> sources;
+        std::vector<Tensor> tensors;
+        py::object value;
+        int64_t bytes;
+        c10::cuda::CUDAStream stream;
+    };
+    using Key = std::array<int64_t, 8>;
+    struct Hash {
+        size_t operator()(const Key& k) const {
+            uint64_t h = 0x9e3779b97f4a7c15ull;
+            for (int64_t x : k) h = (h ^ (uint64_t)x) * 0xff51afd7ed558ccdull, h ^= h >> 32;
+            return (size_t)h;
+        }
+    };
+    using List = std::list<std::pair<Key, Entry>>;
+    List order;                                  // least recently used first
+    std::unordered_map<Key, List::iterator, Hash> at;
+    int64_t bytes = 0, budget = 2ll << 30;
+
+    static Key key(int kind, const Tensor& a, const OptTensor& b, int64_t m, int64_t n) {
+        return {kind, a.device().index(), (int64_t)a.data_ptr(), a.size(0), b.has_value() ? (int64_t)b->data_ptr() : -1,
+                b.has_value() ? b->size(0) : -1, m, n};
+    }
+    void erase(List::iterator it) {
+        bytes -= it->second.bytes;
+        at.erase(it->first);
+        order.erase(it);
+    }
+    Entry* find(const Key& k, const Tensor& a, const OptTensor& b) {
+        auto it = at.find(k);
+        if (it == at.end()) return nullptr;
+        Entry& e = it->second->second;
+        if (!e.sources[0].is(a) || (b.has_value() && !e.sources[1].is(*b))) return nullptr;
+        order.splice(order.end(), order, it->second);
+        const auto now = c10::cuda::getCurrentCUDAStream(a.device().index());
+        if (now != e.stream)
+            for (const Tensor& t : e.tensors) t.record_stream(now);
+        return &e;
+    }
+    void put(const Key& k, const Tensor& a, const OptTensor& b, std::vector<Tensor> tensors, py::object value, int64_t size) {
+        auto old = at.find(k);
+        if (old != at.end()) erase(old->second);
+        for (auto it = order.begin(); it != order.end();) {
+            auto here = it++;
+            bool gone = false;
+            for (const Source& src : here->second.sources) gone |= src.storage.expired();
+            if (gone) erase(here);
+        }
+        if (budget <= 0) return;
+        Entry e{{Source(a)}, std::move(tensors), std::move(value), size, c10::cuda::getCurrentCUDAStream(a.device().index())};
+        if (b.has_value()) e.sources.emplace_back(*b);
+        at[k] = order.insert(order.end(), {k, std::move(e)});
+        bytes += size;
+        while (!order.empty() && bytes > budget) erase(order.begin());
+    }
+};
+TopologyCache& cache() {
+    static TopologyCache* c = new TopologyCache();          // never destroyed: it holds Python objects
+    return *c;
+}
+py::object cache_find(int kind, const Tensor& a, const OptTensor& b, int64_t m, int64_t n) {
+    TopologyCache::Entry* e = cache().find(TopologyCache::key(kind, a, b, m, n), a, b);
+    return e ? e->value : py::object(py::none());
+}
+void cache_put(int kind, const Tensor& a, const OptTensor& b, int64_t m, int64_t n, std::vector<Tensor> tensors, py::object value,
+               int64_t bytes) {
+    cache().put(TopologyCache::key(kind, a, b, m, n), a, b, std::move(tensors), std::move(value), bytes);
+}
+void cache_budget(int64_t n) {
+    TopologyCache& c = cache();
+    c.budget = n;
+    while (!c.order.empty() && c.bytes > c.budget) c.erase(c.order.begin());
+}
+py::tuple cache_stats() { return py::make_tuple(cache().order.size(), cache().bytes, cache().budget); }
+void cache_clear() {
+    cache().at.clear();
+    cache().order.clear();
+    cache().bytes = 0;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -1045,4 +1267,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("avg_pool", &avg_pool);
     m.def("unpool", &unpool);
     m.def("segment_mean", &segment_mean);
+    m.def("mesh_decimation", &mesh_decimation);
+    m.def("level_prepare", &level_prepare);
+    m.def("cache_find", &cache_find);
+    m.def("cache_put", &cache_put);
+    m.def("cache_budget", &cache_budget);
+    m.def("cache_stats", &cache_stats);
+    m.def("cache_clear", &cache_clear);
 }

@@ -135,24 +135,7 @@ def combine_clusters_(repA, mapA, repB, mapB):
 
 def mesh_decimation_(vertexIn, faceIn, geometryIn, nvIn, mfIn, nvOut, useArea=True, wgtBnd=5):
     '''Decimates every sample of the batch to nvOut vertices (decimate.py:5-48): passes of `simplify`
-    until every sample has shed its vertices, clusters merged across the passes.
+    until every sample has shed its vertices, clusters merged across the passes; the loop runs natively with one
+    synchronisation per pass.
     Returns vertexOut, faceOut, geometryOut, nvOut, mfOut, vtReplace, vtMap.'''
-    nv2Remove = nvIn - nvOut
-    repIn = torch.zeros(vertexIn.shape[0], dtype=torch.int32, device=vertexIn.device)
-    mapIn = torch.arange(vertexIn.shape[0], dtype=torch.int32, device=vertexIn.device)
-    while bool(torch.any(nv2Remove > 0)):
-        nvIn_cumsum = torch.cumsum(nvIn, dim=-1, dtype=torch.int32)
-        mfIn_cumsum = torch.cumsum(mfIn, dim=-1, dtype=torch.int32)
-        vertexOut, faceOut, isDegenerate, repOut, mapOut, nvOut, mfOut = simplify(
-            vertexIn.contiguous(), faceIn.contiguous(), geometryIn.contiguous(), nvIn_cumsum, mfIn_cumsum,
-            nv2Remove.to(torch.int32).contiguous(), useArea, wgtBnd)
-        removed = nvIn - nvOut
-        if not bool(torch.any(removed > 0)):
-            break          # nothing left to contract (no candidate edges): the reference would loop forever
-        faceIn = faceOut[~isDegenerate, :]
-        vertexIn = vertexOut[mapOut >= 0, :]
-        geometryIn = compute_triangle_geometry_(vertexIn, faceIn)
-        nv2Remove = nv2Remove - removed
-        repIn, mapIn = combine_clusters_(repIn, mapIn, repOut, mapOut)
-        nvIn, mfIn = nvOut, mfOut
-    return vertexIn, faceIn, geometryIn, nvIn, mfIn, repIn, mapIn
+    return _lib.ops.mesh_decimation(vertexIn, faceIn, geometryIn, nvIn, mfIn, nvOut, bool(useArea), float(wgtBnd), [], [], [])[:7]

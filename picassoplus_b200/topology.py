@@ -6,13 +6,13 @@ operator calls per step in the reference's encoder blocks,
 picasso/networks/pi2_blocks.py:88-92), so the CSR is built once per (face, vtMap) pair
 and looked up afterwards.
 
-Cache policy.  A slot is named by the storage of the index tensors (device, data pointer,
-length); the slot remembers the tensors' version counters.  A lookup whose versions differ
-(the tensors were overwritten in place, as a streaming loader does with its device buffers)
-rebuilds the CSR and REPLACES the slot, so stale entries never pile up.  Slots hold a
-reference to their index tensors, so the memory behind a key cannot be recycled while the
-slot lives.  The cache is bounded by bytes (`set_cache_budget`, default 2 GiB of CSR arrays
-per process) and evicts least-recently-used slots; `set_cache_budget(0)` turns it off.
+Cache policy (TopologyCache in csrc/torch_ops.cpp).  An entry is named by the storage of the index
+tensors (device, data pointer, length) and good while those storages live and their version counters
+stand still.  A lookup whose versions differ (the tensors were overwritten in place, as a streaming
+loader does with its device buffers) rebuilds the structure and REPLACES the entry, so stale entries
+never pile up; entries whose tensors are gone are dropped at the next insertion, so neither do those of
+past batches.  The cache is bounded by bytes (`set_cache_budget`, default 2 GiB of CSR arrays
+per process) and evicts least-recently-used entries; `set_cache_budget(0)` turns it off.
 Callers that manage topologies themselves can pass a prebuilt `VertexCSR` to the operator
 wrappers (`csr=`) and skip the cache altogether.
 
@@ -26,16 +26,14 @@ kept and `check_deferred()` reads them all at a point where the caller synchroni
 from __future__ import annotations
 
 import threading
-from collections import OrderedDict
 from typing import List, Optional
 
 import torch
 
 from . import _lib
 
-_budget_bytes = 2 << 30
-_cache: "OrderedDict[tuple, VertexCSR]" = OrderedDict()
-_cache_bytes = 0
+_ops = _lib.ops
+_VERTEX, _CLUSTER, _PAIRS, _MEANS, _MEANS_SH, _SAMPLES = range(6)      # kinds of cache entries
 _lock = threading.Lock()
 _validation = "sync"
 _deferred: List[tuple] = []          # (status tensor, message)
@@ -51,10 +49,7 @@ def ptr(t: Optional[torch.Tensor]):
 
 def set_cache_budget(nbytes: int) -> None:
     """Upper bound on the bytes of CSR arrays the cache keeps (0 = no caching)."""
-    global _budget_bytes
-    with _lock:
-        _budget_bytes = int(nbytes)
-        _evict_locked()
+    _ops.cache_budget(int(nbytes))
 
 
 def set_validation(mode: str) -> None:
@@ -83,28 +78,18 @@ def check_deferred() -> None:
 class VertexCSR:
     """rowptr (NvOut+1,), entries (3*Nf,) int32: row v lists (f << 2 | corner) ascending."""
 
-    def __init__(self, rowptr, entries, keep, versions=None, shared=False):
+    def __init__(self, rowptr, entries):
         self.rowptr = rowptr
         self.entries = entries
-        self._keep = keep
-        self._versions = versions
-        self.nbytes = 0 if shared else rowptr.numel() * 4 + entries.numel() * 4
+
+    def _tensors(self):
+        return [self.rowptr, self.entries]
 
 
-def _slot(face, vt_map, nv_in, nv_out):
-    vk = None if vt_map is None else (vt_map.data_ptr(), vt_map.shape[0])
-    return (face.device.index, face.data_ptr(), face.shape[0], vk, int(nv_in), int(nv_out))
-
-
-def _versions(face, vt_map):
-    return (face._version, None if vt_map is None else vt_map._version)
-
-
-def _evict_locked():
-    global _cache_bytes
-    while _cache and _cache_bytes > _budget_bytes:
-        _, old = _cache.popitem(last=False)
-        _cache_bytes -= old.nbytes
+def _store(kind, a, b, m, n, value, shared=False):
+    """Puts a structure made from the index tensors a (and b) into the cache; shared: its arrays belong to another entry."""
+    tensors = value._tensors()
+    _ops.cache_put(kind, a, b, m, n, tensors, value, 0 if shared else sum(t.numel() * t.element_size() for t in tensors))
 
 
 def _launch_build(face, vt_map, nv_in, nv_out):
@@ -134,28 +119,7 @@ def build_vertex_csr(face: torch.Tensor, vt_map: Optional[torch.Tensor], nv_in: 
                 _deferred.append((status, _bad_index_message(nv_in, nv_out)))
         elif int(status.item()) != 0:
             raise RuntimeError(_bad_index_message(nv_in, nv_out))
-    return VertexCSR(rowptr, entries, (face, vt_map), _versions(face, vt_map))
-
-
-def _lookup(slot, versions):
-    with _lock:
-        hit = _cache.get(slot)
-        if hit is not None and hit._versions == versions:
-            _cache.move_to_end(slot)
-            return hit
-    return None
-
-
-def _store(slot, csr):
-    global _cache_bytes
-    with _lock:
-        old = _cache.pop(slot, None)
-        if old is not None:
-            _cache_bytes -= old.nbytes
-        if _budget_bytes > 0:
-            _cache[slot] = csr
-            _cache_bytes += csr.nbytes
-            _evict_locked()
+    return VertexCSR(rowptr, entries)
 
 
 def vertex_csr(face: torch.Tensor, vt_map: Optional[torch.Tensor], nv_in: int, nv_out: int) -> VertexCSR:
@@ -163,16 +127,12 @@ def vertex_csr(face: torch.Tensor, vt_map: Optional[torch.Tensor], nv_in: int, n
     In 'sync' mode an identity vtMap over nv_in == nv_out vertices shares the arrays of
     vt_map=None (the identity test rides on the build's one synchronisation); in 'deferred'
     mode nothing is read back and the CSR is built from vtMap as given."""
-    slot = _slot(face, vt_map, nv_in, nv_out)
-    versions = _versions(face, vt_map)
-    hit = _lookup(slot, versions)
+    hit = _ops.cache_find(_VERTEX, face, vt_map, nv_in, nv_out)
     if hit is not None:
         return hit
-    csr = None
     may_be_identity = vt_map is not None and nv_in == nv_out and vt_map.shape[0] == nv_in
     if may_be_identity and _validation == "sync":
-        base_slot = _slot(face, None, nv_in, nv_out)
-        base = _lookup(base_slot, _versions(face, None))
+        base = _ops.cache_find(_VERTEX, face, None, nv_in, nv_out)
         with torch.cuda.device(face.device):
             ident = (vt_map == torch.arange(nv_in, dtype=vt_map.dtype, device=vt_map.device)).all().to(torch.int32)
             if base is None:
@@ -181,15 +141,15 @@ def vertex_csr(face: torch.Tensor, vt_map: Optional[torch.Tensor], nv_in: int, n
                 code, is_ident = torch.stack([status[0], ident]).tolist()
                 if code != 0:
                     raise RuntimeError(_bad_index_message(nv_in, nv_out))
-                base = VertexCSR(rowptr, entries, (face, None), _versions(face, None))
-                _store(base_slot, base)
+                base = VertexCSR(rowptr, entries)
+                _store(_VERTEX, face, None, nv_in, nv_out, base)
             else:
                 is_ident = int(ident.item())
         if is_ident:
-            csr = VertexCSR(base.rowptr, base.entries, (face, vt_map), versions, shared=True)
-    if csr is None:
-        csr = build_vertex_csr(face, vt_map, nv_in, nv_out)
-    _store(slot, csr)
+            _store(_VERTEX, face, vt_map, nv_in, nv_out, base, shared=True)
+            return base
+    csr = build_vertex_csr(face, vt_map, nv_in, nv_out)
+    _store(_VERTEX, face, vt_map, nv_in, nv_out, csr)
     return csr
 
 
@@ -209,28 +169,15 @@ def prepare_level(vertex: torch.Tensor, face: torch.Tensor, vt_map: Optional[tor
         raise RuntimeError("vertex must have shape (Nv, >=3) and face (Nf, 3)")
     vertex, face = vertex.contiguous(), face.contiguous()
     nv_in, nf = vertex.shape[0], face.shape[0]
-    dev = face.device
-    K = (L + 1) ** 2
-    with torch.cuda.device(dev):
-        geometry = torch.empty(nf, 5, dtype=torch.float32, device=dev) if want_geometry else None
-        normals = torch.empty(nf, 3, dtype=torch.float32, device=dev) if want_normals else None
-        coeff = torch.empty(nf, K, dtype=torch.float32, device=dev)
-        nf_count = torch.empty(nv_out, dtype=torch.int32, device=dev)
-        rowptr = torch.empty(nv_out + 1, dtype=torch.int32, device=dev)
-        entries = torch.empty(max(3 * nf, 1), dtype=torch.int32, device=dev)
-        status = torch.empty(1, dtype=torch.int32, device=dev)
-        wbytes = _lib.query("pb200_vertex_csr_workspace_bytes", nf, nv_out)
-        ws = torch.empty(wbytes, dtype=torch.uint8, device=dev)
-        _lib.call("pb200_level_prepare", nf, nv_in, nv_out, vertex.shape[1], ptr(vertex), ptr(face), ptr(vt_map), L,
-                  1 if orient else 0, ptr(geometry), ptr(normals), ptr(coeff), ptr(nf_count), ptr(rowptr), ptr(entries),
-                  ptr(status), ptr(ws), wbytes, stream_ptr(dev))
-        if _validation == "deferred":
-            with _lock:
-                _deferred.append((status, _bad_index_message(nv_in, nv_out)))
-        elif int(status.item()) != 0:
-            raise RuntimeError(_bad_index_message(nv_in, nv_out))
-    csr = VertexCSR(rowptr, entries, (face, vt_map), _versions(face, vt_map))
-    _store(_slot(face, vt_map, nv_in, nv_out), csr)
+    geometry, normals, coeff, nf_count, rowptr, entries, status = _lib.ops.level_prepare(
+        vertex, face, vt_map, nv_out, L, bool(orient), bool(want_geometry), bool(want_normals))
+    if _validation == "deferred":
+        with _lock:
+            _deferred.append((status, _bad_index_message(nv_in, nv_out)))
+    elif int(status.item()) != 0:
+        raise RuntimeError(_bad_index_message(nv_in, nv_out))
+    csr = VertexCSR(rowptr, entries)
+    _store(_VERTEX, face, vt_map, nv_in, nv_out, csr)
     return dict(geometry=geometry, normals=normals, coeff=coeff, nf_count=nf_count, csr=csr)
 
 
@@ -238,13 +185,13 @@ class ClusterCSR:
     """Decimation clusters of a fine level: key (NvIn,) = coarse id of each fine vertex or -1;
     rowptr (NvOut+1,), members (NvIn,) = member fine vertices of every coarse vertex, ascending."""
 
-    def __init__(self, key, rowptr, members, keep, versions):
+    def __init__(self, key, rowptr, members):
         self.key = key
         self.rowptr = rowptr
         self.members = members
-        self._keep = keep
-        self._versions = versions
-        self.nbytes = 4 * (key.numel() + rowptr.numel() + members.numel())
+
+    def _tensors(self):
+        return [self.key, self.rowptr, self.members]
 
 
 def cluster_csr(vt_replace: torch.Tensor, vt_map: torch.Tensor, nv_out: int) -> ClusterCSR:
@@ -252,9 +199,7 @@ def cluster_csr(vt_replace: torch.Tensor, vt_map: torch.Tensor, nv_out: int) -> 
     vertex_csr).  One pooling level is used by a pool in the encoder and an unpool in the decoder,
     forward and backward: four lookups per step, one build."""
     nv_in = vt_replace.shape[0]
-    slot = ("cluster", vt_replace.device.index, vt_replace.data_ptr(), vt_map.data_ptr(), nv_in, int(nv_out))
-    versions = (vt_replace._version, vt_map._version)
-    hit = _lookup(slot, versions)
+    hit = _ops.cache_find(_CLUSTER, vt_replace, vt_map, nv_out, 0)
     if hit is not None:
         return hit
     dev = vt_replace.device
@@ -273,8 +218,8 @@ def cluster_csr(vt_replace: torch.Tensor, vt_map: torch.Tensor, nv_out: int) -> 
                 _deferred.append((status, msg))
         elif int(status.item()) != 0:
             raise RuntimeError(msg)
-    csr = ClusterCSR(key, rowptr, members, (vt_replace, vt_map), versions)
-    _store(slot, csr)
+    csr = ClusterCSR(key, rowptr, members)
+    _store(_CLUSTER, vt_replace, vt_map, nv_out, 0, csr)
     return csr
 
 
@@ -282,21 +227,19 @@ class PairCSR:
     """Neighbour pairs grouped by one column of nnIndex: rowptr (rows+1,), members (pairs,) = pair ids
     of every row, ascending."""
 
-    def __init__(self, rowptr, members, keep, versions):
+    def __init__(self, rowptr, members):
         self.rowptr = rowptr
         self.members = members
-        self._keep = keep
-        self._versions = versions
-        self.nbytes = 4 * (rowptr.numel() + members.numel())
+
+    def _tensors(self):
+        return [self.rowptr, self.members]
 
 
 def pair_csr(nn_index: torch.Tensor, column: int, n_rows: int) -> PairCSR:
     """Cached grouping of the neighbour pairs of a point-cloud convolution by their output point
     (column 0) or input point (column 1); same cache, budget and validation modes as vertex_csr."""
     npairs = nn_index.shape[0]
-    slot = ("pairs", nn_index.device.index, nn_index.data_ptr(), npairs, int(column), int(n_rows))
-    versions = (nn_index._version,)
-    hit = _lookup(slot, versions)
+    hit = _ops.cache_find(_PAIRS, nn_index, None, column, n_rows)
     if hit is not None:
         return hit
     dev = nn_index.device
@@ -315,8 +258,8 @@ def pair_csr(nn_index: torch.Tensor, column: int, n_rows: int) -> PairCSR:
                 _deferred.append((status, msg))
         elif int(status.item()) != 0:
             raise RuntimeError(msg)
-    csr = PairCSR(rowptr, members, (nn_index,), versions)
-    _store(slot, csr)
+    csr = PairCSR(rowptr, members)
+    _store(_PAIRS, nn_index, None, column, n_rows, csr)
     return csr
 
 
@@ -324,15 +267,15 @@ class FaceMeans:
     """Per-face mean of the sample rows of a batch (Nf, F) and the running count 1, 2, ..., Nf that says
     'one sample per face'."""
 
-    def __init__(self, rows, one_each, keep, versions):
+    def __init__(self, rows, one_each):
         self.rows = rows
         self.one_each = one_each
         # the copy with rows padded to a multiple of four floats that the tensor-core kernels read (None when the row
         # length is such a multiple already): made once here instead of in every forward and backward call
         self.rows_padded = pad_rows(rows)
-        self._keep = keep
-        self._versions = versions
-        self.nbytes = 4 * (rows.numel() + one_each.numel() + (0 if self.rows_padded is None else self.rows_padded.numel()))
+
+    def _tensors(self):
+        return [t for t in (self.rows, self.one_each, self.rows_padded) if t is not None]
 
 
 def pad_rows(rows: torch.Tensor):
@@ -352,10 +295,7 @@ def face_means(sample_rows: torch.Tensor, num_interior: torch.Tensor) -> FaceMea
     """Cached mean over every face's samples of sample_rows (NiK, F) (num_interior = inclusive running sample
     count, as facet2facet takes it); same cache and budget as vertex_csr.  Forward and backward of a step share it."""
     nf, nik = num_interior.shape[0], sample_rows.shape[0]
-    slot = ("face_means", sample_rows.device.index, sample_rows.data_ptr(), num_interior.data_ptr(), nik, nf,
-            sample_rows.shape[1])
-    versions = (sample_rows._version, num_interior._version)
-    hit = _lookup(slot, versions)
+    hit = _ops.cache_find(_MEANS, sample_rows, num_interior, sample_rows.shape[1], 0)
     if hit is not None:
         return hit
     dev = sample_rows.device
@@ -365,8 +305,8 @@ def face_means(sample_rows: torch.Tensor, num_interior: torch.Tensor) -> FaceMea
         _lib.call("pb200_face_mean_rows", nf, nik, sample_rows.shape[1], ptr(sample_rows), ptr(num_interior), ptr(rows),
                   stream_ptr(dev))
         one_each = torch.arange(1, nf + 1, dtype=torch.int32, device=dev)
-    fm = FaceMeans(rows, one_each, (sample_rows, num_interior), versions)
-    _store(slot, fm)
+    fm = FaceMeans(rows, one_each)
+    _store(_MEANS, sample_rows, num_interior, sample_rows.shape[1], 0, fm)
     return fm
 
 
@@ -374,9 +314,7 @@ def face_means_sph_harm(L: int, sample_xyz: torch.Tensor, num_interior: torch.Te
     """face_means(sph_harm_coeff(L, sample_xyz), num_interior) in one kernel (identical bits), without the
     (NiK, (L+1)^2) array; cached the same way."""
     nf, nik = num_interior.shape[0], sample_xyz.shape[0]
-    slot = ("face_means_sh", sample_xyz.device.index, sample_xyz.data_ptr(), num_interior.data_ptr(), nik, nf, int(L))
-    versions = (sample_xyz._version, num_interior._version)
-    hit = _lookup(slot, versions)
+    hit = _ops.cache_find(_MEANS_SH, sample_xyz, num_interior, L, 0)
     if hit is not None:
         return hit
     if sample_xyz.dim() != 2 or sample_xyz.shape[1] != 3 or sample_xyz.dtype != torch.float32 or not sample_xyz.is_contiguous():
@@ -387,27 +325,25 @@ def face_means_sph_harm(L: int, sample_xyz: torch.Tensor, num_interior: torch.Te
         rows = torch.empty(nf, (L + 1) ** 2, dtype=torch.float32, device=dev)
         _lib.call("pb200_face_mean_sph_harm", nf, nik, int(L), ptr(sample_xyz), ptr(num_interior), ptr(rows), stream_ptr(dev))
         one_each = torch.arange(1, nf + 1, dtype=torch.int32, device=dev)
-    fm = FaceMeans(rows, one_each, (sample_xyz, num_interior), versions)
-    _store(slot, fm)
+    fm = FaceMeans(rows, one_each)
+    _store(_MEANS_SH, sample_xyz, num_interior, L, 0, fm)
     return fm
 
 
 class SampleEnds:
     """Running number of rows up to and including every sample (B,) int64."""
 
-    def __init__(self, ends, keep, versions):
+    def __init__(self, ends):
         self.ends = ends
-        self._keep = keep
-        self._versions = versions
-        self.nbytes = 8 * ends.numel()
+
+    def _tensors(self):
+        return [self.ends]
 
 
 def sample_ends(counts: torch.Tensor, n_rows: int) -> torch.Tensor:
     """Cached running totals of the samples' row counts; same cache, budget and validation modes as vertex_csr.  They must
     add up to n_rows."""
-    slot = ("samples", counts.device.index, counts.data_ptr(), counts.dtype, counts.shape[0], int(n_rows))
-    versions = (counts._version,)
-    hit = _lookup(slot, versions)
+    hit = _ops.cache_find(_SAMPLES, counts, None, n_rows, counts.element_size())
     if hit is not None:
         return hit.ends
     ends = torch.cumsum(counts.detach(), 0, dtype=torch.int64)
@@ -419,7 +355,7 @@ def sample_ends(counts: torch.Tensor, n_rows: int) -> torch.Tensor:
             _deferred.append((bad.to(torch.int32), msg))
     elif bool(bad.item()):
         raise RuntimeError(msg)
-    _store(slot, SampleEnds(ends, (counts,), versions))
+    _store(_SAMPLES, counts, None, n_rows, counts.element_size(), SampleEnds(ends))
     return ends
 
 
@@ -441,12 +377,9 @@ def check_num_interior(num_interior: torch.Tensor, nik: int) -> None:
 
 
 def cache_stats():
-    with _lock:
-        return {"slots": len(_cache), "bytes": _cache_bytes, "budget": _budget_bytes}
+    slots, nbytes, budget = _ops.cache_stats()
+    return {"slots": slots, "bytes": nbytes, "budget": budget}
 
 
 def clear_cache() -> None:
-    global _cache_bytes
-    with _lock:
-        _cache.clear()
-        _cache_bytes = 0
+    _ops.cache_clear()
