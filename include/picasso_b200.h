@@ -226,6 +226,11 @@ size_t pb200_rows_contract_workspace_bytes(int64_t Nrows, int M, int N);
 int pb200_rows_contract(int64_t Nrows, int M, int N, const float* A, const float* B, float* out, float* colsum,
                         int precision, void* workspace, size_t workspace_bytes, void* stream);
 
+/* The same contraction in fp32 multiply-adds (no rounding of the operands), any widths; no column sums. */
+size_t pb200_rows_contract_f32_workspace_bytes(int64_t rows, int M, int N);
+int pb200_rows_contract_f32(int64_t rows, int M, int N, const float* A, const float* B, float* out, void* workspace,
+                            size_t workspace_bytes, void* stream);
+
 /* ---- whole layers: operator, pointwise stage and batch normalisation --------------------------------------------
  * The three pointwise forwards with what a layer module adds around them (picasso/mesh/layers.py:109-120,166-175):
  *   features   (rows, C): the operator's output, written as a by-product for the backward pass (NULL = not wanted; the

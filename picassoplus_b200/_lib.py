@@ -120,6 +120,8 @@ SIGNATURES = {
     "pb200_masked_rows_matmul": (i32, [i64, i32, i32, vp, vp, vp, vp, vp, i32, vp, sz, vp]),
     "pb200_rows_contract_workspace_bytes": (sz, [i64, i32, i32]),
     "pb200_rows_contract": (i32, [i64, i32, i32, vp, vp, vp, vp, i32, vp, sz, vp]),
+    "pb200_rows_contract_f32_workspace_bytes": (sz, [i64, i32, i32]),
+    "pb200_rows_contract_f32": (i32, [i64, i32, i32, vp, vp, vp, vp, sz, vp]),
     "pb200_sph_harm_coeff": (i32, [i64, i32, vp, vp, vp]),
     "pb200_corner_filter": (i32, [i32, i32, vp, vp, vp, vp]),
     "pb200_corner_filter_backward": (i32, [i32, i32, vp, vp, vp, vp]),

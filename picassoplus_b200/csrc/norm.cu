@@ -41,8 +41,7 @@ template <int V> __device__ __forceinline__ void store(float* p, const Vec<V>& x
 
 struct Moments { float n, mean, m2; };
 __device__ __forceinline__ void merge(Moments& a, const Moments& b) {
-    if (b.n == 0.f) return;
-    const float n = a.n + b.n, d = b.mean - a.mean, f = b.n / n;
+    const float n = a.n + b.n, d = b.mean - a.mean, f = b.n > 0.f ? __fdividef(b.n, n) : 0.f;      // no branch: loads run ahead
     a.mean = fmaf(d, f, a.mean);
     a.m2 += b.m2 + d * d * a.n * f;
     a.n = n;
@@ -106,7 +105,7 @@ stats_kernel(int64_t N, int C, float* __restrict__ rows, const float* __restrict
     }
 }
 
-// Merges the partials of every channel: 32 slices side by side, then the slices in order.  Writes what the transform and
+// Merges the partials of every channel: 32 slices side by side, then the slices pairwise.  Writes what the transform and
 // the backward pass need and moves the running statistics (unbiased variance, as torch's batch norm does).
 constexpr int FS = 32;
 __global__ void __launch_bounds__(32 * FS)
@@ -117,15 +116,21 @@ finalize_kernel(int nparts, int C, const float* __restrict__ partial, float eps,
     const int c = blockIdx.x * 32 + threadIdx.x, y = threadIdx.y;
     const int per = (nparts + FS - 1) / FS;
     Moments m{0.f, 0.f, 0.f};
-    if (c < C)
-        for (int b = y * per; b < nparts && b < (y + 1) * per; ++b) {
+    if (c < C) {
+        const int end = nparts < (y + 1) * per ? nparts : (y + 1) * per;
+#pragma unroll 4
+        for (int b = y * per; b < end; ++b) {
             const float* p = partial + (int64_t)b * 3 * C + c;
             merge(m, Moments{p[0], p[C], p[2 * C]});
         }
+    }
     red[y][threadIdx.x] = m;
-    __syncthreads();
+#pragma unroll
+    for (int h = FS / 2; h > 0; h >>= 1) {
+        __syncthreads();
+        if (y < h) { merge(m, red[y + h][threadIdx.x]); red[y][threadIdx.x] = m; }
+    }
     if (y == 0 && c < C) {
-        for (int k = 1; k < FS; ++k) merge(m, red[k][threadIdx.x]);
         const float var = m.m2 / m.n;
         mean[c] = m.mean;
         invstd[c] = rsqrtf(var + eps);

@@ -159,20 +159,110 @@ __global__ void conv_fwd_vec_kernel(int64_t Np, int64_t Mp, int F, int CV, int T
     }
 }
 
+// An input point that many output points name (a padded neighbour list names point 0 over and over) would keep one group of
+// lanes walking long after the others are done: 800 pairs took 300 us of a 370 us launch.  Rows longer than this get a block
+// each.
+constexpr int LONG_ROW = 64;
+
+// The long rows of the input gradient, a role of the launch's first blocks so that they run beside the others.  A block looks
+// through LONG_SCAN rows.  For a long one, all threads fetch the next STAGE pairs (index, 1 / count, bins, weights) into shared
+// memory, then the block's groups of CV lanes walk equal consecutive parts of them, four row gathers in flight; the groups'
+// sums are added in group order.
+constexpr int LONG_SCAN = 1024, STAGE = 256, STAGED_BINS = 3;
+static inline int long_blocks(int64_t Np) { return (int)ceil_div(Np, LONG_SCAN); }
+
+__device__ __noinline__ void bwd_input_long_rows(int64_t first, int64_t Np, int64_t Mp, int F, int CV, int T,
+                                                    const float4* __restrict__ gout, const float4* __restrict__ filter,
+                                                    const int32_t* __restrict__ nnCount, const int32_t* __restrict__ nnIndex,
+                                                    const int32_t* __restrict__ bin, const float* __restrict__ coeff,
+                                                    const int32_t* __restrict__ rowptr, const int32_t* __restrict__ members,
+                                                    float4* __restrict__ gin, float4* sfilt) {
+    __shared__ float4 red[256];
+    __shared__ int rows[LONG_SCAN], nrows;
+    __shared__ int sp[STAGE], so[STAGE], sb[STAGE][STAGED_BINS];
+    __shared__ float srn[STAGE], sc[STAGE][STAGED_BINS];
+    if (threadIdx.x == 0) nrows = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < LONG_SCAN; i += blockDim.x) {
+        const int64_t n = first + i;
+        if (n < Np && __ldg(rowptr + n + 1) - __ldg(rowptr + n) > LONG_ROW) rows[atomicAdd(&nrows, 1)] = i;
+    }
+    __syncthreads();
+    const int total = nrows;
+    if (total == 0) return;
+    for (int i = threadIdx.x; i < F * CV; i += blockDim.x) sfilt[i] = filter[i];
+    const int G = blockDim.x / CV, g = threadIdx.x / CV, cg = threadIdx.x - g * CV;
+    const bool staged = T <= STAGED_BINS;
+    for (int k = 0; k < total; ++k) {
+        const int64_t n = first + rows[k];
+        const int e0 = __ldg(rowptr + n), e1 = __ldg(rowptr + n + 1);
+        float4 acc = zero4();
+        for (int s0 = e0; s0 < e1; s0 += STAGE) {
+            const int cnt = e1 - s0 < STAGE ? e1 - s0 : STAGE;
+            __syncthreads();
+            for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
+                const int p = __ldg(members + s0 + i);
+                const int o = __ldg(nnIndex + 2 * (int64_t)p);
+                const bool ok = o >= 0 && o < Mp;
+                sp[i] = p;
+                so[i] = ok ? o : -1;
+                srn[i] = ok ? 1.f / (float)__ldg(nnCount + o) : 0.f;
+                if (staged)
+                    for (int t = 0; t < T; ++t) {
+                        const int f = __ldg(bin + (int64_t)p * T + t);
+                        const bool in = f >= 0 && f < F;
+                        sb[i][t] = in ? f : 0;
+                        sc[i][t] = in ? (coeff ? __ldg(coeff + (int64_t)p * T + t) : 1.f) : 0.f;
+                    }
+            }
+            __syncthreads();
+            const int per = (cnt + G - 1) / G, b = g * per;
+            const int e = g < G ? (b + per < cnt ? b + per : cnt) : 0;
+            for (int q = b; q < e; q += 4) {
+                float4 x[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) x[u] = q + u < e && so[q + u] >= 0 ? ldg4(gout + (int64_t)so[q + u] * CV + cg) : zero4();
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    if (q + u >= e) break;
+                    float4 w = zero4();
+                    if (staged) for (int t = 0; t < T; ++t) fma4s(w, sc[q + u][t], sfilt[sb[q + u][t] * CV + cg]);
+                    else w = pair_weight4(sp[q + u], cg, CV, F, T, bin, coeff, sfilt);
+                    fma4(acc, scale4(x[u], srn[q + u]), w);
+                }
+            }
+        }
+        red[threadIdx.x] = acc;
+        __syncthreads();
+        if (g == 0) {
+            for (int t = 1; t < G; ++t) add4(acc, red[t * CV + cg]);
+            gin[n * CV + cg] = acc;
+        }
+        __syncthreads();
+    }
+}
+
 __global__ void conv_bwd_input_vec_kernel(int64_t Np, int64_t Mp, int F, int CV, int T, const float4* __restrict__ gout,
                                           const float4* __restrict__ filter, const int32_t* __restrict__ nnCount,
                                           const int32_t* __restrict__ nnIndex, const int32_t* __restrict__ bin,
                                           const float* __restrict__ coeff, const int32_t* __restrict__ rowptr,
-                                          const int32_t* __restrict__ members, float4* __restrict__ gin) {
+                                          const int32_t* __restrict__ members, int nlong, float4* __restrict__ gin) {
     extern __shared__ float4 sfilt[];
+    if ((int)blockIdx.x < nlong) {
+        bwd_input_long_rows((int64_t)blockIdx.x * LONG_SCAN, Np, Mp, F, CV, T, gout, filter, nnCount, nnIndex, bin, coeff, rowptr, members,
+                            gin, sfilt);
+        return;
+    }
     for (int i = threadIdx.x; i < F * CV; i += blockDim.x) sfilt[i] = filter[i];
     __syncthreads();
-    const int64_t total = Np * CV;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t total = Np * CV, nblocks = gridDim.x - nlong;
+    for (int64_t i = (int64_t)(blockIdx.x - nlong) * blockDim.x + threadIdx.x; i < total; i += nblocks * blockDim.x) {
         const int64_t n = i / CV;
         const int cg = (int)(i - n * CV);
         float4 acc = zero4();
-        for (int e = __ldg(rowptr + n); e < __ldg(rowptr + n + 1); ++e) {
+        const int e0 = __ldg(rowptr + n), e1 = __ldg(rowptr + n + 1);
+        if (e1 - e0 > LONG_ROW) continue;
+        for (int e = e0; e < e1; ++e) {
             const int64_t p = __ldg(members + e);
             const int o = __ldg(nnIndex + 2 * p);
             if (o < 0 || o >= Mp) continue;
@@ -232,90 +322,24 @@ static bool sizes_ok(int64_t Np, int64_t Mp, int64_t Nout, int F, int C, int r, 
            Nout < (1LL << 31) && (int64_t)F * C * r * 4 <= 200 * 1024;
 }
 // ------------------------------------------------------------------------ cooperative kernels
-// C of 32, 64 or 128: the CV = C / 4 lanes of a point sit in one warp, so lane j fetches the indices of the j-th
-// pair of a run and the run is walked with shuffles, four pairs at a time: the four row gathers and the bin
-// fetches of a step are in flight together. TT: 1 = one bin per pair, 3 = three weighted bins, 0 = any T.
+// C of 32, 64 or 128: the lanes of a point sit in one warp, so lane j fetches the indices of the j-th
+// pair of a run and the run is walked with shuffles, a few pairs at a time: the row gathers of a step are in
+// flight together. TT: 1 = one bin per pair, 3 = three weighted bins, 0 = any T.
 // Same order of additions as the vector kernels.
 template <int CV>
 __device__ __forceinline__ unsigned group_mask(int gbase) {
     return CV == 32 ? 0xffffffffu : (((1u << (CV & 31)) - 1u) << gbase);
 }
 
-template <int TT, int CV>
-__device__ __forceinline__ float4 pair_weight4t(int64_t p, int cg, int F, int T, const int32_t* __restrict__ bin,
-                                                const float* __restrict__ coeff, const float4* __restrict__ sfilt) {
-    if constexpr (TT == 0) {
-        return pair_weight4(p, cg, CV, F, T, bin, coeff, sfilt);
-    } else if constexpr (TT == 1) {
-        const int f = __ldg(bin + p);
-        const bool ok = (unsigned)f < (unsigned)F;
-        const float4 w = sfilt[(ok ? f : 0) * CV + cg];
-        return ok ? w : zero4();
-    } else {
-    int f[3];
-    float c[3];
-#pragma unroll
-    for (int t = 0; t < 3; ++t) {
-        f[t] = __ldg(bin + p * 3 + t);
-        c[t] = __ldg(coeff + p * 3 + t);
-    }
-    float4 w = zero4();
-#pragma unroll
-    for (int t = 0; t < 3; ++t) {
-        const bool ok = (unsigned)f[t] < (unsigned)F;
-        fma4s(w, ok ? c[t] : 0.f, sfilt[(ok ? f[t] : 0) * CV + cg]);
-    }
-    return w;
-    }
-}
+// A lane owns VPL float4 of the row, LN lanes a point: with two per lane (64 and 128 channels) the index fetches, shuffles and
+// bin look-ups of a pair are shared by twice the channels, which is what these kernels are short of (the load/store pipe), and
+// U = 2 pairs per step keep as many row gathers in flight per warp as four with one float4.
+template <int CV> struct Lanes {
+    static constexpr int VPL = CV >= 16 ? 2 : 1, LN = CV / VPL, U = VPL == 2 ? 2 : 4;
+};
 
-template <int TT, int CV>
-__global__ void __launch_bounds__(256)
-conv_fwd_coop_kernel(int64_t Np, int64_t Mp, int F, int T, const float4* __restrict__ input,
-                     const float4* __restrict__ filter, const int32_t* __restrict__ nnCount,
-                     const int32_t* __restrict__ nnIndex, const int32_t* __restrict__ bin, const float* __restrict__ coeff,
-                     const int32_t* __restrict__ rowptr, const int32_t* __restrict__ members, float4* __restrict__ output) {
-    extern __shared__ float4 sfilt[];
-    for (int i = threadIdx.x; i < F * CV; i += blockDim.x) sfilt[i] = filter[i];
-    __syncthreads();
-    const int lane = threadIdx.x & 31, cg = lane % CV, gbase = lane - cg;
-    const unsigned mask = group_mask<CV>(gbase);
-    const int64_t stride = (int64_t)gridDim.x * (blockDim.x / CV);
-    for (int64_t o = (int64_t)blockIdx.x * (blockDim.x / CV) + threadIdx.x / CV; o < Mp; o += stride) {
-        const int e0 = __ldg(rowptr + o), e1 = __ldg(rowptr + o + 1);
-        const float rn = 1.f / (float)__ldg(nnCount + o);
-        float4 acc = zero4();
-        for (int e = e0; e < e1; e += CV) {
-            int p_mine = 0, in_mine = -1;
-            if (e + cg < e1) {
-                p_mine = __ldg(members + e + cg);
-                in_mine = __ldg(nnIndex + 2 * (int64_t)p_mine + 1);
-            }
-            const int n = e1 - e < CV ? e1 - e : CV;
-            for (int j = 0; j < n; j += 4) {
-                float4 x[4], w[4];
-                int pp[4];
-                bool ok[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int src = gbase + ((j + u) & (CV - 1));
-                    pp[u] = __shfl_sync(mask, p_mine, src);
-                    const int in = __shfl_sync(mask, in_mine, src);
-                    ok[u] = j + u < n && in >= 0 && in < Np;
-                    x[u] = ok[u] ? ldg4(input + (int64_t)in * CV + cg) : zero4();
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) w[u] = pair_weight4t<TT, CV>(pp[u], cg, F, T, bin, coeff, sfilt);
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (ok[u]) fma4(acc, scale4(x[u], rn), w[u]);
-            }
-        }
-        output[o * CV + cg] = acc;
-    }
-}
-
-// The bins and weights of the pair a lane fetched (TT of 1 or 3), handed to the group's lanes by shuffles.
+// The bins and weights of the pair a lane fetched (TT of 1 or 3), handed to the group's lanes by shuffles.  A bin outside
+// [0, F) becomes bin 0 with weight 0.
 template <int TT>
 struct LaneBins {
     int f[TT == 3 ? 3 : 1];
@@ -323,114 +347,174 @@ struct LaneBins {
 };
 
 template <int TT>
-__device__ __forceinline__ void load_bins(LaneBins<TT>& b, bool have, int64_t p, const int32_t* __restrict__ bin,
+__device__ __forceinline__ void load_bins(LaneBins<TT>& b, bool have, int64_t p, int F, const int32_t* __restrict__ bin,
                                           const float* __restrict__ coeff) {
 #pragma unroll
     for (int t = 0; t < (TT == 3 ? 3 : 1); ++t) {
         b.f[t] = have ? __ldg(bin + p * (TT == 3 ? 3 : 1) + t) : -1;
         b.c[t] = TT == 3 ? (have ? __ldg(coeff + p * 3 + t) : 0.f) : 1.f;
+        if ((unsigned)b.f[t] >= (unsigned)F) { b.f[t] = 0; b.c[t] = 0.f; }
     }
+}
+
+// out += x * rn * weight of the pair, for the lane's float4
+template <int TT, int CV>
+__device__ __forceinline__ void add_pair(float4 (&acc)[Lanes<CV>::VPL], const float4 (&x)[Lanes<CV>::VPL], float rn, const LaneBins<TT>& b, int64_t p,
+                                         unsigned mask, int src, int ln, bool ok, int F, int T, const int32_t* __restrict__ bin,
+                                         const float* __restrict__ coeff, const float4* __restrict__ sfilt) {
+    constexpr int VPL = Lanes<CV>::VPL, LN = Lanes<CV>::LN;
+    float4 w[VPL];
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) w[i] = zero4();
+    if constexpr (TT == 0) {
+        if (ok)
+#pragma unroll
+            for (int i = 0; i < VPL; ++i) w[i] = pair_weight4(p, ln + i * LN, CV, F, T, bin, coeff, sfilt);
+    } else {
+#pragma unroll
+        for (int t = 0; t < TT; ++t) {
+            const int f = __shfl_sync(mask, b.f[t], src);            // out of range: bin 0 with weight 0
+            const float c = __shfl_sync(mask, b.c[t], src);
+#pragma unroll
+            for (int i = 0; i < VPL; ++i) fma4s(w[i], c, sfilt[f * CV + ln + i * LN]);
+        }
+    }
+    if (ok)
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) fma4(acc[i], scale4(x[i], rn), w[i]);
 }
 
 template <int TT, int CV>
-__device__ __forceinline__ float4 shuffled_weight4(const LaneBins<TT>& b, unsigned mask, int src, int cg, int F,
-                                                   const float4* __restrict__ sfilt) {
-    float4 w = zero4();
+__global__ void __launch_bounds__(256, 4)
+conv_fwd_coop_kernel(int64_t Np, int64_t Mp, int F, int T, const float4* __restrict__ input,
+                     const float4* __restrict__ filter, const int32_t* __restrict__ nnCount,
+                     const int32_t* __restrict__ nnIndex, const int32_t* __restrict__ bin, const float* __restrict__ coeff,
+                     const int32_t* __restrict__ rowptr, const int32_t* __restrict__ members, float4* __restrict__ output) {
+    constexpr int VPL = Lanes<CV>::VPL, LN = Lanes<CV>::LN, U = Lanes<CV>::U;
+    extern __shared__ float4 sfilt[];
+    for (int i = threadIdx.x; i < F * CV; i += blockDim.x) sfilt[i] = filter[i];
+    __syncthreads();
+    const int lane = threadIdx.x & 31, ln = lane % LN, gbase = lane - ln;
+    const unsigned mask = group_mask<LN>(gbase);
+    const int64_t stride = (int64_t)gridDim.x * (blockDim.x / LN);
+    for (int64_t o = (int64_t)blockIdx.x * (blockDim.x / LN) + threadIdx.x / LN; o < Mp; o += stride) {
+        const int e0 = __ldg(rowptr + o), e1 = __ldg(rowptr + o + 1);
+        const float rn = 1.f / (float)__ldg(nnCount + o);
+        float4 acc[VPL];
 #pragma unroll
-    for (int t = 0; t < (TT == 3 ? 3 : 1); ++t) {
-        const int f = __shfl_sync(mask, b.f[t], src);
-        const float c = TT == 3 ? __shfl_sync(mask, b.c[t], src) : 1.f;
-        const bool ok = (unsigned)f < (unsigned)F;
-        fma4s(w, ok ? c : 0.f, sfilt[(ok ? f : 0) * CV + cg]);
+        for (int i = 0; i < VPL; ++i) acc[i] = zero4();
+        for (int e = e0; e < e1; e += LN) {
+            int p_mine = 0, in_mine = -1;
+            LaneBins<TT> mybins;
+            const bool have = e + ln < e1;
+            if (have) {
+                p_mine = __ldg(members + e + ln);
+                in_mine = __ldg(nnIndex + 2 * (int64_t)p_mine + 1);
+            }
+            if constexpr (TT != 0) load_bins<TT>(mybins, have, p_mine, F, bin, coeff);
+            const int n = e1 - e < LN ? e1 - e : LN;
+            for (int j = 0; j < n; j += U) {
+                float4 x[U][VPL];
+                int pp[U];
+                bool ok[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int src = gbase + ((j + u) & (LN - 1));
+                    pp[u] = TT == 0 ? __shfl_sync(mask, p_mine, src) : 0;
+                    const int in = __shfl_sync(mask, in_mine, src);
+                    ok[u] = j + u < n && in >= 0 && in < Np;
+#pragma unroll
+                    for (int i = 0; i < VPL; ++i) x[u][i] = ok[u] ? ldg4(input + (int64_t)in * CV + ln + i * LN) : zero4();
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    add_pair<TT, CV>(acc, x[u], rn, mybins, pp[u], mask, gbase + ((j + u) & (LN - 1)), ln, ok[u], F, T, bin, coeff, sfilt);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) output[o * CV + ln + i * LN] = acc[i];
     }
-    return w;
 }
 
-// one step of the input gradient: up to four pairs whose indices sit in the lanes of the group, slots j .. j + 3
-// of [j, end); the four rows of the output gradient and the bin fetches are in flight together
-template <int TT, int CV>
-__device__ __forceinline__ void bwd_input_step(float4& acc, int j, int end, unsigned mask, int gbase, int cg, int p_mine,
-                                               int o_mine, float rn_mine, const LaneBins<TT>& mybins, int64_t Mp, int F, int T,
-                                               const float4* __restrict__ gout, const int32_t* __restrict__ bin,
-                                               const float* __restrict__ coeff, const float4* __restrict__ sfilt) {
-    float4 x[4], w[4];
-    int pp[4];
-    float rn[4];
-    bool ok[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        const int src = gbase + ((j + u) & (CV - 1));
-        pp[u] = __shfl_sync(mask, p_mine, src);
-        const int o = __shfl_sync(mask, o_mine, src);
-        rn[u] = __shfl_sync(mask, rn_mine, src);
-        ok[u] = j + u < end && o >= 0 && o < Mp;
-        x[u] = ok[u] ? ldg4(gout + (int64_t)o * CV + cg) : zero4();
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        if constexpr (TT == 0) w[u] = pair_weight4(pp[u], cg, CV, F, T, bin, coeff, sfilt);
-        else w[u] = shuffled_weight4<TT, CV>(mybins, mask, gbase + ((j + u) & (CV - 1)), cg, F, sfilt);
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-        if (ok[u]) fma4(acc, scale4(x[u], rn[u]), w[u]);
-}
-
-// A group takes W = CV / 4 consecutive input points per step: their pairs are one contiguous run of the grouping,
+// A group takes W = LN / 4 consecutive input points per step: their pairs are one contiguous run of the grouping,
 // and when it fits the group's lanes (the usual case: an input point is the neighbour of a few output points) one
 // fetch of the indices serves all W points.
 template <int TT, int CV>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(256, 3)
 conv_bwd_input_coop_kernel(int64_t Np, int64_t Mp, int F, int T, const float4* __restrict__ gout,
                            const float4* __restrict__ filter, const int32_t* __restrict__ nnCount,
                            const int32_t* __restrict__ nnIndex, const int32_t* __restrict__ bin,
                            const float* __restrict__ coeff, const int32_t* __restrict__ rowptr,
-                           const int32_t* __restrict__ members, float4* __restrict__ gin) {
-    constexpr int W = CV / 4;
+                           const int32_t* __restrict__ members, int nlong, float4* __restrict__ gin) {
+    constexpr int VPL = Lanes<CV>::VPL, LN = Lanes<CV>::LN, U = Lanes<CV>::U, W = LN / 4;
     extern __shared__ float4 sfilt[];
+    if ((int)blockIdx.x < nlong) {
+        bwd_input_long_rows((int64_t)blockIdx.x * LONG_SCAN, Np, Mp, F, CV, T, gout, filter, nnCount, nnIndex, bin, coeff, rowptr, members,
+                            gin, sfilt);
+        return;
+    }
     for (int i = threadIdx.x; i < F * CV; i += blockDim.x) sfilt[i] = filter[i];
     __syncthreads();
-    const int lane = threadIdx.x & 31, cg = lane % CV, gbase = lane - cg;
-    const unsigned mask = group_mask<CV>(gbase);
-    const int64_t stride = (int64_t)gridDim.x * (blockDim.x / CV) * W;
-    for (int64_t base = ((int64_t)blockIdx.x * (blockDim.x / CV) + threadIdx.x / CV) * W; base < Np; base += stride) {
+    const int lane = threadIdx.x & 31, ln = lane % LN, gbase = lane - ln;
+    const unsigned mask = group_mask<LN>(gbase);
+    const int64_t stride = (int64_t)(gridDim.x - nlong) * (blockDim.x / LN) * W;
+    for (int64_t base = ((int64_t)(blockIdx.x - nlong) * (blockDim.x / LN) + threadIdx.x / LN) * W; base < Np; base += stride) {
         int rp_mine = 0;
-        if (cg <= W) rp_mine = __ldg(rowptr + (base + cg < Np ? base + cg : Np));
+        if (ln <= W) rp_mine = __ldg(rowptr + (base + ln < Np ? base + ln : Np));
         const int E0 = __shfl_sync(mask, rp_mine, gbase), EW = __shfl_sync(mask, rp_mine, gbase + W);
-        const bool together = EW - E0 <= CV;
+        const bool together = EW - E0 <= LN;
         int p_mine = 0, o_mine = -1;
         float rn_mine = 0.f;
         LaneBins<TT> mybins;
-        if (together) {
-            const bool have = E0 + cg < EW;
-            if (have) p_mine = __ldg(members + E0 + cg);
+        auto fetch = [&](int e, bool have) {
+            p_mine = 0, o_mine = -1, rn_mine = 0.f;
+            if (have) p_mine = __ldg(members + e);
             if (have) o_mine = __ldg(nnIndex + 2 * (int64_t)p_mine);
-            if constexpr (TT != 0) load_bins<TT>(mybins, have, p_mine, bin, coeff);
-            if (o_mine >= 0 && o_mine < Mp) rn_mine = 1.f / (float)__ldg(nnCount + o_mine);
-        }
+            if constexpr (TT != 0) load_bins<TT>(mybins, have, p_mine, F, bin, coeff);
+            if (o_mine >= Mp) o_mine = -1;
+            if (o_mine >= 0) rn_mine = 1.f / (float)__ldg(nnCount + o_mine);
+        };
+        float4 acc[VPL];
+        // pairs of the fetched run, slots [j, end)
+        auto walk = [&](int j, int end) {
+            for (; j < end; j += U) {
+                float4 x[U][VPL];
+                int pp[U];
+                float rn[U];
+                bool ok[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int src = gbase + ((j + u) & (LN - 1));
+                    pp[u] = TT == 0 ? __shfl_sync(mask, p_mine, src) : 0;
+                    const int o = __shfl_sync(mask, o_mine, src);
+                    rn[u] = __shfl_sync(mask, rn_mine, src);
+                    ok[u] = j + u < end && o >= 0;
+#pragma unroll
+                    for (int i = 0; i < VPL; ++i) x[u][i] = ok[u] ? ldg4(gout + (int64_t)o * CV + ln + i * LN) : zero4();
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    add_pair<TT, CV>(acc, x[u], rn[u], mybins, pp[u], mask, gbase + ((j + u) & (LN - 1)), ln, ok[u], F, T, bin, coeff, sfilt);
+            }
+        };
+        if (together) fetch(E0 + ln, E0 + ln < EW);
 #pragma unroll 1
         for (int k = 0; k < W; ++k) {
             const int e0 = __shfl_sync(mask, rp_mine, gbase + k), e1 = __shfl_sync(mask, rp_mine, gbase + k + 1);
-            float4 acc = zero4();
+            if (e1 - e0 > LONG_ROW) continue;
+#pragma unroll
+            for (int i = 0; i < VPL; ++i) acc[i] = zero4();
             if (together) {
-                for (int j = e0 - E0; j < e1 - E0; j += 4)
-                    bwd_input_step<TT, CV>(acc, j, e1 - E0, mask, gbase, cg, p_mine, o_mine, rn_mine, mybins, Mp, F, T, gout, bin,
-                                           coeff, sfilt);
+                walk(e0 - E0, e1 - E0);
             } else {
-                for (int e = e0; e < e1; e += CV) {
-                    p_mine = 0, o_mine = -1, rn_mine = 0.f;
-                    const bool have = e + cg < e1;
-                    if (have) p_mine = __ldg(members + e + cg);
-                    if (have) o_mine = __ldg(nnIndex + 2 * (int64_t)p_mine);
-                    if constexpr (TT != 0) load_bins<TT>(mybins, have, p_mine, bin, coeff);
-                    if (o_mine >= 0 && o_mine < Mp) rn_mine = 1.f / (float)__ldg(nnCount + o_mine);
-                    const int n = e1 - e < CV ? e1 - e : CV;
-                    for (int j = 0; j < n; j += 4)
-                        bwd_input_step<TT, CV>(acc, j, n, mask, gbase, cg, p_mine, o_mine, rn_mine, mybins, Mp, F, T, gout, bin,
-                                               coeff, sfilt);
+                for (int e = e0; e < e1; e += LN) {
+                    fetch(e + ln, e + ln < e1);
+                    walk(0, e1 - e < LN ? e1 - e : LN);
                 }
             }
-            if (base + k < Np) gin[(base + k) * CV + cg] = acc;
+            if (base + k < Np)
+#pragma unroll
+                for (int i = 0; i < VPL; ++i) gin[(base + k) * CV + ln + i * LN] = acc[i];
         }
     }
 }
@@ -466,7 +550,7 @@ conv_bwd_filter_coop_kernel(int64_t Np, int64_t Mp, int64_t Nout, int pairs_per_
             o_mine = __ldg(nnIndex + 2 * (q + cg));
             in_mine = __ldg(nnIndex + 2 * (q + cg) + 1);
         }
-        if constexpr (TT != 0) load_bins<TT>(mybins, have, q + cg, bin, coeff);
+        if constexpr (TT != 0) load_bins<TT>(mybins, have, q + cg, F, bin, coeff);
         if (o_mine >= 0 && o_mine < Mp) rn_mine = 1.f / (float)__ldg(nnCount + o_mine);
         const int n = q1 - q < CV ? (int)(q1 - q) : CV;
         for (int j = 0; j < n; j += 4) {
@@ -491,8 +575,8 @@ conv_bwd_filter_coop_kernel(int64_t Np, int64_t Mp, int64_t Nout, int pairs_per_
 #pragma unroll
                     for (int t = 0; t < (TT == 3 ? 3 : 1); ++t) {
                         const int f = __shfl_sync(mask, mybins.f[t], src);
-                        const float c = TT == 3 ? __shfl_sync(mask, mybins.c[t], src) : 1.f;
-                        if (ok[u] && (unsigned)f < (unsigned)F) fma4s(mine[f * CV + cg], c, d);
+                        const float c = __shfl_sync(mask, mybins.c[t], src);
+                        if (ok[u] && c != 0.f) fma4s(mine[f * CV + cg], c, d);
                     }
                 } else if (ok[u]) {
                     const int64_t p = q + j + u;
@@ -522,8 +606,13 @@ static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // the vector kernels: depth multiplier 1, channels a multiple of 4 and at most 1024 (one group of lanes per point),
 // and a filter table that leaves room in shared memory for at least one accumulator copy
 static bool vec_ok(int F, int C, int r) { return r == 1 && C % 4 == 0 && C <= 1024 && (size_t)F * C * 4 <= 48 * 1024; }
-constexpr int VEC_PAIRS_PER_BLOCK = 2048;
-static int vec_filter_blocks(int64_t Nout) { return (int)ceil_div(Nout > 0 ? Nout : 1, VEC_PAIRS_PER_BLOCK); }
+// pairs of a filter-gradient block: 2048 (partial tables stay small against the gathers), fewer where that would leave less
+// than six blocks per SM to hide the gathers' latency, 256 at least
+static int vec_pairs_per_block(int64_t Nout) {
+    int64_t n = ceil_div(ceil_div(Nout > 0 ? Nout : 1, 6 * (int64_t)sm_count()), 32) * 32;
+    return (int)(n < 256 ? 256 : n > 2048 ? 2048 : n);
+}
+static int vec_filter_blocks(int64_t Nout) { return (int)ceil_div(Nout > 0 ? Nout : 1, vec_pairs_per_block(Nout)); }
 static int vec_sub_groups(int F, int C) {
     int sub = 256 / (C / 4);
     if (sub < 1) sub = 1;
@@ -545,7 +634,7 @@ template <int TT, int CV>
 static int launch_fwd_coop(int64_t Np, int64_t Mp, int F, int T, const float* input, const float* filter, const int32_t* nnCount,
                            const int32_t* nnIndex, const int32_t* bin, const float* coeff, const int32_t* rowptr,
                            const int32_t* members, float* output, cudaStream_t stream) {
-    PB_LAUNCH("pcloud_conv_fwd", (conv_fwd_coop_kernel<TT, CV>), persistent_blocks(Mp * CV, 256, 8), 256, sizeof(float4) * F * CV,
+    PB_LAUNCH("pcloud_conv_fwd", (conv_fwd_coop_kernel<TT, CV>), persistent_blocks(Mp * Lanes<CV>::LN, 256, 8), 256, sizeof(float4) * F * CV,
               stream, Np, Mp, F, T, (const float4*)input, (const float4*)filter, nnCount, nnIndex, bin, coeff, rowptr, members,
               (float4*)output);
     return PB200_OK;
@@ -556,15 +645,17 @@ static int launch_bwd_coop(int64_t Np, int64_t Mp, int64_t Nout, int nb, int F, 
                            const float* gout, const int32_t* nnCount, const int32_t* nnIndex, const int32_t* bin,
                            const float* coeff, const int32_t* rowptr, const int32_t* members, float* gin, float* partial,
                            cudaStream_t stream) {
-    if (Np > 0)
-        PB_LAUNCH("pcloud_conv_bwd_input", (conv_bwd_input_coop_kernel<TT, CV>), persistent_blocks(Np * CV, 256, 8), 256,
+    if (Np > 0) {
+        const int nlong = Nout > LONG_ROW ? long_blocks(Np) : 0;
+        PB_LAUNCH("pcloud_conv_bwd_input", (conv_bwd_input_coop_kernel<TT, CV>), nlong + persistent_blocks(Np * Lanes<CV>::LN, 256, 8), 256,
                   sizeof(float4) * F * CV, stream, Np, Mp, F, T, (const float4*)gout, (const float4*)filter, nnCount, nnIndex, bin,
-                  coeff, rowptr, members, (float4*)gin);
+                  coeff, rowptr, members, nlong, (float4*)gin);
+    }
     const int sub = coop_sub_groups(F, 4 * CV);
     const size_t smem = sizeof(float4) * (size_t)sub * F * CV;
     PB_CUDA(cudaFuncSetAttribute(conv_bwd_filter_coop_kernel<TT, CV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     PB_LAUNCH("pcloud_conv_bwd_filter", (conv_bwd_filter_coop_kernel<TT, CV>), nb, sub * CV, smem, stream, Np, Mp, Nout,
-              VEC_PAIRS_PER_BLOCK, sub, F, T, (const float4*)input, (const float4*)gout, nnCount, nnIndex, bin, coeff,
+              vec_pairs_per_block(Nout), sub, F, T, (const float4*)input, (const float4*)gout, nnCount, nnIndex, bin, coeff,
               (float4*)partial);
     return PB200_OK;
 }
@@ -645,16 +736,18 @@ int pb200_pcloud_conv3d_backward(int64_t Np, int64_t Mp, int64_t Nout, int F, in
             if (rc != PB200_OK) return rc;
             return reduce_partials((const float*)workspace, nbc, (int64_t)F * C, gradFilter, stream);
         }
-        if (Np > 0)
-            PB_LAUNCH("pcloud_conv_bwd_input", conv_bwd_input_vec_kernel, persistent_blocks(Np * CV, 256, 8), 256,
+        if (Np > 0) {
+            const int nlong = Nout > LONG_ROW ? long_blocks(Np) : 0;
+            PB_LAUNCH("pcloud_conv_bwd_input", conv_bwd_input_vec_kernel, nlong + persistent_blocks(Np * CV, 256, 8), 256,
                       sizeof(float) * F * C, stream, Np, Mp, F, CV, T, (const float4*)gradOutput, (const float4*)filter, nnCount,
-                      nnIndex, binIndex, binCoeff, rowptr_in, members_in, (float4*)gradInput);
+                      nnIndex, binIndex, binCoeff, rowptr_in, members_in, nlong, (float4*)gradInput);
+        }
         const int nbv = vec_filter_blocks(Nout), sub = vec_sub_groups(F, C);
         const size_t smemv = sizeof(float) * (size_t)sub * F * C;
         const int threads = sub * CV < 32 ? 32 : ((sub * CV + 31) / 32) * 32;
         PB_CUDA(cudaFuncSetAttribute(conv_bwd_filter_vec_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemv));
         PB_LAUNCH("pcloud_conv_bwd_filter", conv_bwd_filter_vec_kernel, nbv, threads, smemv, stream, Np, Mp, Nout,
-                  VEC_PAIRS_PER_BLOCK, F, CV, T, sub, (const float4*)input, (const float4*)gradOutput, nnCount, nnIndex, binIndex,
+                  vec_pairs_per_block(Nout), F, CV, T, sub, (const float4*)input, (const float4*)gradOutput, nnCount, nnIndex, binIndex,
                   binCoeff, (float4*)workspace);
         return reduce_partials((const float*)workspace, nbv, (int64_t)F * C, gradFilter, stream);
     }

@@ -853,6 +853,25 @@ Tensor rows_layer(const Tensor& rows_in, const Tensor& weights, const OptTensor&
     return r.out;
 }
 
+// act <- activation(act + bias) in place, out = its normalisation (act itself without one); the statistics used
+NormStats bias_act_norm(const Scope& s, const Tail& t, const Tensor& act, const Tensor& bias, Tensor& out) {
+    const int64_t rows = act.size(0), C = act.size(1);
+    Tensor partial = s.floats({pb200_norm_parts(rows, (int)C), 3, C});
+    int parts = 0;
+    call(pb200_bias_act_stats(rows, (int)C, fpm(act), fp(bias), t.relu, fpm(partial), &parts, s.stream), "pb200_bias_act_stats");
+    out = act;
+    NormStats st;
+    if (t.mode == NORM_BATCH) {
+        st = finalize(s, t, C, parts, partial);
+        out = normalise(s, t, act, st);
+    } else if (t.mode == NORM_RUNNING) {
+        const NormStats running{t.running_mean, s.floats({C})};
+        call(pb200_norm_invstd((int)C, fp(t.running_var), (float)t.eps, nullptr, fpm(running.invstd), s.stream), "pb200_norm_invstd");
+        out = normalise(s, t, act, running);
+    }
+    return st;
+}
+
 // facet2facet over the samples of every face (`counts` per face), then bias, ReLU or nothing, normalisation
 Tensor f2f_layer(const Tensor& input, const Tensor& filter, const Tensor& bary, const Tensor& counts, const Tensor& bias0, TAIL_PARAMS) {
     const Tail t = make_tail(TAIL_ARGS);
@@ -864,21 +883,8 @@ Tensor f2f_layer(const Tensor& input, const Tensor& filter, const Tensor& bary, 
     const Tensor cum = at::cumsum(counts, 0, at::kInt), bias = flat(bias0);
     check(cum, "num_texture", 1, at::kInt);
     Scope s(input);
-    Tensor act = f2f_forward(s, aligned(input), filter, bary, cum, precision);
-    const int64_t rows = act.size(0), C = act.size(1);
-    Tensor out = act;
-    NormStats st;
-    Tensor partial = s.floats({pb200_norm_parts(rows, (int)C), 3, C});
-    int parts = 0;
-    call(pb200_bias_act_stats(rows, (int)C, fpm(act), fp(bias), relu, fpm(partial), &parts, s.stream), "pb200_bias_act_stats");
-    if (t.mode == NORM_BATCH) {
-        st = finalize(s, t, C, parts, partial);
-        out = normalise(s, t, act, st);
-    } else if (t.mode == NORM_RUNNING) {
-        const NormStats running{t.running_mean, s.floats({C})};
-        call(pb200_norm_invstd((int)C, fp(t.running_var), (float)t.eps, nullptr, fpm(running.invstd), s.stream), "pb200_norm_invstd");
-        out = normalise(s, t, act, running);
-    }
+    Tensor act = f2f_forward(s, aligned(input), filter, bary, cum, precision), out;
+    const NormStats st = bias_act_norm(s, t, act, bias, out);
     if (node) {
         node->input = keep(input);
         node->filter = keep(filter);
@@ -1028,6 +1034,170 @@ Tensor segment_mean(const Tensor& input, const Tensor& ends) {
         node->rows = input.size(0);
         node->channels = input.size(1);
         torch::autograd::set_history(out, node);
+    }
+    return out;
+}
+
+// ----------------------------------------------------------------------------------------------- point-cloud convolution
+// The neighbour pairs and the two groupings of them (rowptr / members by output and by input point)
+struct Pairs { Tensor nn_count, nn_index, bin_index, bin_coeff; };
+int bins_per_pair(const Pairs& q) { return q.bin_coeff.defined() ? (int)q.bin_index.size(1) : 1; }
+
+void check_pairs(const Tensor& input, const Tensor& filter, const Pairs& q) {
+    check(input, "input", 2, at::kFloat);
+    check(filter, "filter", 3, at::kFloat);
+    check(q.nn_count, "nn_count", 1, at::kInt);
+    check(q.nn_index, "nn_index", 2, at::kInt);
+    check(q.bin_index, "bin_index", q.bin_coeff.defined() ? 2 : 1, at::kInt);
+    if (q.bin_coeff.defined()) {
+        check(q.bin_coeff, "bin_coeff", 2, at::kFloat);
+        if (q.bin_coeff.sizes() != q.bin_index.sizes()) fail("bin_coeff and bin_index must have the same shape");
+    }
+    if (filter.size(1) != input.size(1)) fail("Input Channel size error of the filter");
+    if (q.nn_index.size(0) > 0 && q.nn_index.size(1) != 2) fail("nn_index must have shape (pairs, 2)");
+    if (q.bin_index.size(0) != q.nn_index.size(0)) fail("bin_index must have one row per neighbor pair");
+}
+
+Tensor pairs_forward(const Scope& s, const Tensor& input, const Tensor& filter, const Pairs& q, const Tensor& rowptr, const Tensor& members) {
+    const int64_t Np = input.size(0), C = input.size(1), F = filter.size(0), r = filter.size(2), Mp = q.nn_count.size(0);
+    Tensor out = s.floats({Mp, C * r});
+    call(pb200_pcloud_conv3d_forward(Np, Mp, q.nn_index.size(0), (int)F, (int)C, (int)r, bins_per_pair(q), fp(input), fp(filter),
+                                     ip(q.nn_count), ip(q.nn_index), ip(q.bin_index), fp(q.bin_coeff), ip(rowptr), ip(members), fpm(out),
+                                     s.stream),
+         "pb200_pcloud_conv3d_forward");
+    return out;
+}
+
+void pairs_backward(const Scope& s, const Tensor& g, const Tensor& input, const Tensor& filter, const Pairs& q, const Tensor& rowptr,
+                    const Tensor& members, Tensor& gin, Tensor& gf) {
+    const int64_t Np = input.size(0), C = input.size(1), F = filter.size(0), r = filter.size(2), Mp = q.nn_count.size(0), n = q.nn_index.size(0);
+    gin = s.floats({Np, C});
+    gf = s.floats({F, C, r});
+    const size_t nb = pb200_pcloud_conv3d_backward_workspace_bytes(n, (int)F, (int)C, (int)r);
+    Tensor ws = s.bytes(nb);
+    call(pb200_pcloud_conv3d_backward(Np, Mp, n, (int)F, (int)C, (int)r, bins_per_pair(q), fp(g), fp(input), fp(filter), ip(q.nn_count),
+                                      ip(q.nn_index), ip(q.bin_index), fp(q.bin_coeff), ip(rowptr), ip(members), fpm(gin), fpm(gf),
+                                      ws.data_ptr(), nb, s.stream),
+         "pb200_pcloud_conv3d_backward");
+}
+
+struct PairsNode : Node {
+    SavedVariable input, filter, nn_count, nn_index, bin_index, bin_coeff, rowptr, members;
+    void keep_pairs(const Tensor& x, const Tensor& f, const Pairs& q, const Tensor& by_in_rowptr, const Tensor& by_in_members) {
+        input = keep(x);
+        filter = keep(f);
+        nn_count = keep(q.nn_count);
+        nn_index = keep(q.nn_index);
+        bin_index = keep(q.bin_index);
+        bin_coeff = keep(q.bin_coeff);
+        rowptr = keep(by_in_rowptr);
+        members = keep(by_in_members);
+    }
+    void pairs_gradient(const Scope& s, const Tensor& g, const Tensor& x, Tensor& gin, Tensor& gf) {
+        pairs_backward(s, g, x, filter.unpack(), Pairs{nn_count.unpack(), nn_index.unpack(), bin_index.unpack(), bin_coeff.unpack()},
+                       rowptr.unpack(), members.unpack(), gin, gf);
+    }
+    variable_list apply(variable_list&& grads) override {
+        variable_list out(2);
+        if (!grads[0].defined()) return out;
+        std::lock_guard<std::mutex> lock(mutex_);
+        const Tensor x = input.unpack();
+        Scope s(x);
+        pairs_gradient(s, upstream(grads), x, out[0], out[1]);
+        return out;
+    }
+    void release_variables() override {
+        std::lock_guard<std::mutex> lock(mutex_);
+        for (SavedVariable* v : {&input, &filter, &nn_count, &nn_index, &bin_index, &bin_coeff, &rowptr, &members}) v->reset_data();
+    }
+    std::string name() const override { return "PointConvBackward"; }
+};
+
+// convolution, product with depth_weights (fp32), bias, ReLU or nothing, normalisation
+struct PointLayer : PairsNode {
+    SavedVariable features, weights, act, mean, invstd, gamma;
+    bool relu = false;
+    variable_list apply(variable_list&& grads) override {
+        variable_list out(6);
+        if (!grads[0].defined()) return out;
+        std::lock_guard<std::mutex> lock(mutex_);
+        const Tensor x = input.unpack(), a = act.unpack(shared_from_this()), w = weights.unpack(), feats = features.unpack(),
+                     g = aligned(upstream(grads));
+        const NormStats st{mean.unpack(), invstd.unpack()};
+        Scope s(x);
+        NormGrads n;
+        if (st.mean.defined()) {
+            n = norm_backward(s, g, a, st, gamma.unpack());
+            out[4] = n.gamma;
+            out[5] = n.beta;
+        }
+        Tensor gm;
+        masked_gradient(s, g, a, n, relu, gm, out[3]);
+        const int64_t rows = a.size(0), M = w.size(0), N = w.size(1);
+        out[2] = s.floats({M, N});
+        const size_t nb = pb200_rows_contract_f32_workspace_bytes(rows, (int)M, (int)N);
+        Tensor ws = s.bytes(nb);
+        call(pb200_rows_contract_f32(rows, (int)M, (int)N, fp(feats), fp(gm), fpm(out[2]), ws.data_ptr(), nb, s.stream),
+             "pb200_rows_contract_f32");
+        if (task_should_compute_output(0) || task_should_compute_output(1))
+            pairs_gradient(s, at::matmul(gm, w.t()), x, out[0], out[1]);
+        return out;
+    }
+    void release_variables() override {
+        PairsNode::release_variables();
+        std::lock_guard<std::mutex> lock(mutex_);
+        for (SavedVariable* v : {&features, &weights, &act, &mean, &invstd, &gamma}) v->reset_data();
+    }
+    std::string name() const override { return "PointLayerBackward"; }
+};
+
+Tensor point_conv(const Tensor& input, const Tensor& filter, const Tensor& nn_count, const Tensor& nn_index, const Tensor& bin_index,
+                  const OptTensor& bin_coeff, const Tensor& out_rowptr, const Tensor& out_members, const OptTensor& in_rowptr,
+                  const OptTensor& in_members) {
+    const Pairs q{nn_count, nn_index, bin_index, or_undefined(bin_coeff)};
+    check_pairs(input, filter, q);
+    std::shared_ptr<PairsNode> node;
+    if (torch::autograd::compute_requires_grad(input, filter)) node = node_for<PairsNode>(input, filter);
+    Tensor out;
+    {
+        at::AutoDispatchBelowADInplaceOrView below;
+        Scope s(input);
+        out = pairs_forward(s, input, filter, q, out_rowptr, out_members);
+    }
+    if (node) {
+        node->keep_pairs(input, filter, q, or_undefined(in_rowptr), or_undefined(in_members));
+        torch::autograd::set_history(out, node);
+    }
+    return out;
+}
+
+Tensor point_layer(const Tensor& input, const Tensor& filter, const Tensor& nn_count, const Tensor& nn_index, const Tensor& bin_index,
+                   const OptTensor& bin_coeff, const Tensor& out_rowptr, const Tensor& out_members, const OptTensor& in_rowptr,
+                   const OptTensor& in_members, const Tensor& weights, const Tensor& bias0, bool relu, int norm_mode, const OptTensor& gamma,
+                   const OptTensor& beta, const OptTensor& running_mean, const OptTensor& running_var, const OptTensor& batches,
+                   double momentum, double eps) {
+    const Tail t = make_tail(TAIL_ARGS);
+    const Pairs q{nn_count, nn_index, bin_index, or_undefined(bin_coeff)};
+    check_pairs(input, filter, q);
+    check_stage(weights, filter.size(1) * filter.size(2));
+    std::shared_ptr<PointLayer> node;
+    if (torch::autograd::compute_requires_grad(input, filter, weights, bias0, t.gamma, t.beta))
+        node = node_for<PointLayer>(input, filter, weights, bias0, t.gamma, t.beta);
+    at::AutoDispatchBelowADInplaceOrView below;
+    Scope s(input);
+    Tensor feats = pairs_forward(s, input, filter, q, out_rowptr, out_members);
+    Tensor act = at::matmul(feats, weights), out;
+    const NormStats st = bias_act_norm(s, t, act, flat(bias0), out);
+    if (node) {
+        node->keep_pairs(input, filter, q, or_undefined(in_rowptr), or_undefined(in_members));
+        node->features = keep(feats);
+        node->weights = keep(weights);
+        node->mean = keep(st.mean);
+        node->invstd = keep(st.invstd);
+        node->gamma = keep(t.gamma);
+        node->relu = relu;
+        torch::autograd::set_history(out, node);
+        node->act = SavedVariable(act, act.is_same(out));
     }
     return out;
 }
@@ -1263,6 +1433,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("f2v_layer", &f2v_layer);
     m.def("rows_layer", &rows_layer);
     m.def("f2f_layer", &f2f_layer);
+    m.def("point_conv", &point_conv);
+    m.def("point_layer", &point_layer);
     m.def("max_pool", &max_pool);
     m.def("avg_pool", &avg_pool);
     m.def("unpool", &unpool);

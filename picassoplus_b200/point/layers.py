@@ -5,6 +5,8 @@ from __future__ import annotations
 
 import torch.nn as nn
 
+from .. import _lib
+from ..mesh import layers as _layers
 from ..mesh.layers import _PointwiseTail, _filter_variable_
 from .pi_modules import conv3d
 
@@ -22,6 +24,10 @@ class PCloudConv3d(_PointwiseTail):
         self._init_tail(out_channels, activation_fn, with_bn, bn_momentum)
 
     def forward(self, inputs, nn_count, nn_index, filt_index, filt_coeff=None):
+        if _layers._fusion and inputs.is_cuda and _layers._plain_activation(self.activation_fn) and nn_count.shape[0] > 0:
+            pairs = (nn_count, nn_index, filt_index, filt_coeff)
+            return self._native(nn_count.shape[0], inputs, lambda *tail: _lib.ops.point_layer(
+                inputs, self.spatial_weights, *pairs, *conv3d.groupings(inputs, *pairs), self.depth_weights, self.biases, *tail))
         if filt_coeff is None:
             feats = conv3d.conv3d(inputs, self.spatial_weights, nn_count, nn_index, filt_index)
         else:

@@ -106,8 +106,24 @@ class ConvFunction(torch.autograd.Function):
         return grad_input, grad_filter, None, None, None
 
 
+def groupings(input, nn_count, nn_index, bin_index, bin_coeff):
+    """Marks the index arrays as data and returns the pairs grouped by output point and, when a gradient is needed, by input
+    point: (rowptr, members, rowptr, members)."""
+    for t in (nn_count, nn_index, bin_index, bin_coeff):
+        if t is not None:
+            t.requires_grad = False
+    _check(nn_count, "nn_count", 1, torch.int32)
+    _check(nn_index, "nn_index", 2, torch.int32)
+    by_out = pair_csr(nn_index, 0, nn_count.shape[0])
+    if torch.is_grad_enabled():
+        by_in = pair_csr(nn_index, 1, input.shape[0])
+        return by_out.rowptr, by_out.members, by_in.rowptr, by_in.members
+    return by_out.rowptr, by_out.members, None, None
+
+
 def conv3d(input, filter, nn_count, nn_index, bin_index):
-    return ConvFunction.apply(input, filter, nn_count, nn_index, bin_index)
+    return _lib.ops.point_conv(input, filter, nn_count, nn_index, bin_index, None,
+                               *groupings(input, nn_count, nn_index, bin_index, None))
 
 
 class FuzzyConv3dFunction(torch.autograd.Function):
@@ -129,4 +145,5 @@ class FuzzyConv3dFunction(torch.autograd.Function):
 
 
 def fuzzyconv3d(input, filter, nn_count, nn_index, bin_index, bin_coeff):
-    return FuzzyConv3dFunction.apply(input, filter, nn_count, nn_index, bin_index, bin_coeff)
+    return _lib.ops.point_conv(input, filter, nn_count, nn_index, bin_index, bin_coeff,
+                               *groupings(input, nn_count, nn_index, bin_index, bin_coeff))
