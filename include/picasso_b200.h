@@ -352,6 +352,13 @@ int pb200_facet2facet_backward_padded(int64_t Nf, int64_t NiK, int Cin, int Cout
                                       const int32_t* numInterior, float* gradInput, float* gradFilter,
                                       int precision, void* workspace, size_t workspace_bytes, void* stream);
 
+/* pb200_facet2facet_backward for faces with exactly one sample each (the counterpart of pb200_facet2facet_one_sample_forward):
+ * oneEach = 1, 2, ..., Nf on the device; workspace of pb200_facet2facet_backward_workspace_bytes(Nf, Nf, ...). */
+int pb200_facet2facet_one_sample_backward(int64_t Nf, int Cin, int Cout, int F, const float* gradOutput, const float* input,
+                                          const float* filter, const float* weights, const float* weightsPadded,
+                                          const int32_t* oneEach, float* gradInput, float* gradFilter, int precision,
+                                          void* workspace, size_t workspace_bytes, void* stream);
+
 /* The filter gradient alone (same workspace), for samples that are data and need no gradient. */
 int pb200_facet2facet_filter_gradient(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, const float* gradOutput,
                                       const float* input, const float* bary, const float* baryPadded, const int32_t* numInterior,

@@ -24,6 +24,12 @@ int backward_input(int64_t Nf, int Cin, int Cout, int F, const float* gout, cons
                    const float* bary_p, int Fp, const int32_t* cum, float* gin, int precision, void* ws,
                    cudaStream_t stream, bool transposed);
 }  // namespace gin
+namespace one {
+bool supported(int Cn, int Ck, int F, int precision);
+size_t workspace_bytes(int Cn, int Ck, int F, int precision);
+int run(int64_t Nf, int Cn, int Ck, int F, const float* rows, const float* filter, const float* w, int Fp, float* out, int precision,
+        void* ws, cudaStream_t stream, bool forward);
+}  // namespace one
 namespace gfilter {
 bool supported(int Cin, int Cout, int F);
 bool fits(int64_t Nf, int Cin, int Cout, int F, int precision);
@@ -91,12 +97,19 @@ int pb200_facet2facet_forward(int64_t Nf, int64_t NiK, int Cin, int Cout, int F,
 // One sample per face: output[f,co] = sum_d weights[f,d] * (sum_ci input[f,ci] * filter[co,ci,d]).  The inner
 // sum is a plain GEMM over the input rows (no face operand of F * Cin products to build, split and store) and
 // the outer one an epilogue over the accumulator: the input-gradient kernel with the channel roles exchanged.
-static bool one_sample_on_gin(int Cin, int Cout, int F, int precision) { return use_tc_gin(Cout, Cin, F, precision); }
+static bool one_sample_on_gin(int Cin, int Cout, int F, int precision) {
+    return tc::one::supported(Cout, Cin, F, precision) || use_tc_gin(Cout, Cin, F, precision);
+}
+// workspace of the one-sample product (Cn channels out of Ck): its own kernel, else the input-gradient kernel's
+static size_t one_sample_ws(int Cn, int Ck, int F, int precision) {
+    return tc::one::supported(Cn, Ck, F, precision) ? tc::one::workspace_bytes(Cn, Ck, F, precision)
+                                                    : tc::gin::workspace_bytes(Cn, Ck, F, precision);
+}
 
 size_t pb200_facet2facet_one_sample_forward_workspace_bytes(int64_t Nf, int Cin, int Cout, int F, int precision) {
     if (!f2f_sizes_ok(Nf, Nf, Cin, Cout, F)) return 0;
     if (one_sample_on_gin(Cin, Cout, F, precision))
-        return tc::gin::workspace_bytes(Cout, Cin, F, precision) + tc::padded_bary_bytes(Nf, F);
+        return one_sample_ws(Cout, Cin, F, precision) + tc::padded_bary_bytes(Nf, F);
     return align_up(sizeof(int32_t) * (size_t)(Nf > 0 ? Nf : 1), 256) +
            pb200_facet2facet_forward_workspace_bytes(Nf, Nf, Cin, Cout, F, precision);
 }
@@ -128,11 +141,13 @@ int pb200_facet2facet_one_sample_forward(int64_t Nf, int Cin, int Cout, int F, c
                        "facet2facet_one_sample_forward: weightsPadded must be 16-byte aligned");
             wp = weightsPadded;
         } else if (F % 4 != 0) {
-            float* dst = (float*)(w + tc::gin::workspace_bytes(Cout, Cin, F, precision));
+            float* dst = (float*)(w + one_sample_ws(Cout, Cin, F, precision));
             int rc = tc::pad_bary(Nf, F, weights, dst, stream);
             if (rc) return rc;
             wp = dst;
         }
+        if (tc::one::supported(Cout, Cin, F, precision))
+            return tc::one::run(Nf, Cout, Cin, F, input, filter, wp, Fp, output, precision, w, stream, true);
         return tc::gin::backward_input(Nf, Cout, Cin, F, input, filter, weights, wp, Fp, nullptr, output, precision, w,
                                        stream, true);
     }
@@ -143,11 +158,18 @@ int pb200_facet2facet_one_sample_forward(int64_t Nf, int Cin, int Cout, int F, c
                                      workspace_bytes - (size_t)(w - (char*)workspace), stream_);
 }
 
+// room for the filter image of either input-gradient kernel
+static size_t gin_ws(int Cin, int Cout, int F, int precision) {
+    const size_t a = tc::gin::workspace_bytes(Cin, Cout, F, precision);
+    const size_t b = tc::one::supported(Cin, Cout, F, precision) ? tc::one::workspace_bytes(Cin, Cout, F, precision) : 0;
+    return a > b ? a : b;
+}
+
 size_t pb200_facet2facet_backward_workspace_bytes(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, int precision) {
     if (!f2f_sizes_ok(Nf, NiK, Cin, Cout, F)) return 0;
     const bool tg = use_tc_gin(Cin, Cout, F, precision), tf = use_tc_gf(Nf, Cin, Cout, F, precision);
     size_t n = (tg && tf) ? 0 : f2f_simt_bwd_ws(Nf, Cin, Cout, F);
-    if (tg) n += tc::gin::workspace_bytes(Cin, Cout, F, precision);
+    if (tg) n += gin_ws(Cin, Cout, F, precision);
     if (tf) n += tc::gfilter::workspace_bytes(Nf, Cin, Cout, F, precision);
     if (tg || tf) n += tc::padded_bary_bytes(NiK, F);
     if (tf) n += tc::padded_input_bytes(NiK, Cin);
@@ -161,7 +183,7 @@ size_t pb200_facet2facet_backward_workspace_bytes(int64_t Nf, int64_t NiK, int C
 static int f2f_backward_impl(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, const float* gradOutput,
                              const float* input, const float* filter, const float* bary, const float* baryPadded,
                              const int32_t* numInterior, float* gradInput, float* gradFilter, int precision,
-                             void* workspace, size_t workspace_bytes, void* stream_, bool want_gin) {
+                             void* workspace, size_t workspace_bytes, void* stream_, bool want_gin, bool one_each) {
     cudaStream_t stream = (cudaStream_t)stream_;
     PB_REQUIRE(f2f_sizes_ok(Nf, NiK, Cin, Cout, F), PB200_EINVAL,
                "facet2facet_backward: bad sizes (F must be in 1..50)");
@@ -191,7 +213,7 @@ static int f2f_backward_impl(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, 
             PB_REQUIRE(aligned16(baryPadded), PB200_EINVAL, "facet2facet_backward: baryPadded must be 16-byte aligned");
             bary_p = baryPadded;
         } else {
-            char* wp = w + (tg ? tc::gin::workspace_bytes(Cin, Cout, F, precision) : 0) +
+            char* wp = w + (tg ? gin_ws(Cin, Cout, F, precision) : 0) +
                        (tf ? tc::gfilter::workspace_bytes(Nf, Cin, Cout, F, precision) : 0);
             int rc = tc::pad_bary(NiK, F, bary, (float*)wp, stream);
             if (rc) return rc;
@@ -200,11 +222,13 @@ static int f2f_backward_impl(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, 
     }
     if (tg) {
         if (NiK > 0 && want_gin) {
-            int rc = tc::gin::backward_input(Nf, Cin, Cout, F, gradOutput, filter, bary, bary_p, Fp, numInterior,
-                                             gradInput, precision, w, stream, false);
+            int rc = one_each && tc::one::supported(Cin, Cout, F, precision)
+                         ? tc::one::run(Nf, Cin, Cout, F, gradOutput, filter, bary_p, Fp, gradInput, precision, w, stream, false)
+                         : tc::gin::backward_input(Nf, Cin, Cout, F, gradOutput, filter, bary, bary_p, Fp, numInterior, gradInput,
+                                                   precision, w, stream, false);
             if (rc) return rc;
         }
-        w += tc::gin::workspace_bytes(Cin, Cout, F, precision);
+        w += gin_ws(Cin, Cout, F, precision);
     }
     if (tf) {
         // the filter-gradient kernel reads 16 input channels per CTA with 16-byte copies: channel counts that
@@ -233,7 +257,7 @@ int pb200_facet2facet_backward(int64_t Nf, int64_t NiK, int Cin, int Cout, int F
                                const int32_t* numInterior, float* gradInput, float* gradFilter, int precision,
                                void* workspace, size_t workspace_bytes, void* stream) {
     return f2f_backward_impl(Nf, NiK, Cin, Cout, F, gradOutput, input, filter, bary, nullptr, numInterior, gradInput,
-                             gradFilter, precision, workspace, workspace_bytes, stream, true);
+                             gradFilter, precision, workspace, workspace_bytes, stream, true, false);
 }
 
 int pb200_facet2facet_backward_padded(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, const float* gradOutput,
@@ -241,7 +265,7 @@ int pb200_facet2facet_backward_padded(int64_t Nf, int64_t NiK, int Cin, int Cout
                                       const int32_t* numInterior, float* gradInput, float* gradFilter, int precision,
                                       void* workspace, size_t workspace_bytes, void* stream) {
     return f2f_backward_impl(Nf, NiK, Cin, Cout, F, gradOutput, input, filter, bary, baryPadded, numInterior, gradInput,
-                             gradFilter, precision, workspace, workspace_bytes, stream, true);
+                             gradFilter, precision, workspace, workspace_bytes, stream, true, false);
 }
 
 // for callers whose samples are data (raw textures): the input gradient, a third of the backward pass, is left out
@@ -249,7 +273,15 @@ int pb200_facet2facet_filter_gradient(int64_t Nf, int64_t NiK, int Cin, int Cout
                                       const float* input, const float* bary, const float* baryPadded, const int32_t* numInterior,
                                       float* gradFilter, int precision, void* workspace, size_t workspace_bytes, void* stream) {
     return f2f_backward_impl(Nf, NiK, Cin, Cout, F, gradOutput, input, nullptr, bary, baryPadded, numInterior, nullptr, gradFilter,
-                             precision, workspace, workspace_bytes, stream, false);
+                             precision, workspace, workspace_bytes, stream, false, false);
+}
+
+int pb200_facet2facet_one_sample_backward(int64_t Nf, int Cin, int Cout, int F, const float* gradOutput, const float* input,
+                                          const float* filter, const float* weights, const float* weightsPadded, const int32_t* oneEach,
+                                          float* gradInput, float* gradFilter, int precision, void* workspace, size_t workspace_bytes,
+                                          void* stream) {
+    return f2f_backward_impl(Nf, Nf, Cin, Cout, F, gradOutput, input, filter, weights, weightsPadded, oneEach, gradInput, gradFilter,
+                             precision, workspace, workspace_bytes, stream, true, true);
 }
 
 int pb200_padded_row_floats(int F) { return F > 0 ? tc::padded_F(F) : 0; }

@@ -38,57 +38,6 @@ constexpr int NTHREADS = (EWARPS + 2 + GWARPS) * 32;
 constexpr int G_KTILE_BYTES = TILE_M * 64;      // one 16-channel block of the gradOutput tile
 constexpr int W_STAGE_BYTES = NCOLS * 64;       // one 16-channel block of a filter slice
 
-// ---- TMEM loads of 1/4/8/16/32 consecutive columns (lane = row)
-__device__ __forceinline__ void tmem_ld1(uint32_t taddr, float* v) {
-    uint32_t r0;
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r0) : "r"(taddr) : "memory");
-    v[0] = __uint_as_float(r0);
-}
-__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float* v) {
-    uint32_t r[4];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
-#pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
-}
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
-    uint32_t r[8];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr) : "memory");
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
-    uint32_t r[16];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                 "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                   "=r"(r[15])
-                 : "r"(taddr) : "memory");
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-__device__ __forceinline__ void tmem_ld32f(uint32_t taddr, float* v) {
-    uint32_t r[32];
-    tmem_ld32(taddr, r);
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// F consecutive columns -> v[0..F)
-template <int F>
-__device__ __forceinline__ void tmem_ld_row(uint32_t taddr, float* v) {
-    int o = 0;
-    if (F & 32) { tmem_ld32f(taddr + o, v + o); o += 32; }
-    if (F & 16) { tmem_ld16(taddr + o, v + o); o += 16; }
-    if (F & 8)  { tmem_ld8(taddr + o, v + o); o += 8; }
-    if (F & 4)  { tmem_ld4(taddr + o, v + o); o += 4; }
-    if (F & 2)  { tmem_ld1(taddr + o, v + o); tmem_ld1(taddr + o + 1, v + o + 1); o += 2; }
-    if (F & 1)  { tmem_ld1(taddr + o, v + o); }
-}
-
 // ---- filter image: Wimg[slice][kst][split][row 0..255][16 floats, 64B-swizzled];
 //      row = cil*F + d, element (row, kk) = filter[co = kst*16 + kk][ci = slice*NQ + cil][d]
 //      (co counts from the chunk's first output channel co0)
@@ -124,16 +73,16 @@ __global__ void f2f_tc_gin_prep_filter_kernel(int F, int Cin, int co0, int Cout,
 }
 
 // ---- bf16 filter image: Wimg[slice][kst][split][row 0..255][32 bf16, 64B-swizzled];
-//      row = cil*F + d, element (row, kk) = filter[co = kst*32 + kk][ci = slice*NQ + cil][d]
+//      row = cil*F + d (`rows` of them), element (row, kk) = filter[co = kst*32 + kk][ci = slice*NQ + cil][d]
 __global__ void f2f_tc_gin_prep_filter_bf16_kernel(int F, int Cin, int co0, int Cout, int nq, int nslices, int kst,
-                                                   int nsplit, int64_t s_co, int64_t s_ci,
+                                                   int nsplit, int rows, int64_t s_co, int64_t s_ci,
                                                    const float* __restrict__ filter, uint8_t* __restrict__ wimg) {
-    int64_t total = (int64_t)nslices * kst * NCOLS * 4;
+    int64_t total = (int64_t)nslices * kst * rows * 4;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (int64_t)gridDim.x * blockDim.x) {
         int c = (int)(i & 3);
-        int row = (int)((i >> 2) % NCOLS);
-        int64_t blk = i / (4 * NCOLS);
+        int row = (int)((i >> 2) % rows);
+        int64_t blk = i / (4 * rows);
         int ks = (int)(blk % kst);
         int slice = (int)(blk / kst);
         int cil = row / F, d = row - cil * F;
@@ -150,11 +99,18 @@ __global__ void f2f_tc_gin_prep_filter_bf16_kernel(int F, int Cin, int co0, int 
             if (nsplit == 1) { hi[j] = pack_bf16x2(v[0], v[1]); lo[j] = 0u; }
             else split_bf16x2(v[0], v[1], hi[j], lo[j]);
         }
-        uint8_t* base = wimg + blk * (int64_t)nsplit * W_STAGE_BYTES;
+        uint8_t* base = wimg + blk * (int64_t)nsplit * rows * 64;
         uint32_t off = swz64_offset((uint32_t)row, (uint32_t)c);
         *reinterpret_cast<uint4*>(base + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        if (nsplit == 2) *reinterpret_cast<uint4*>(base + W_STAGE_BYTES + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        if (nsplit == 2) *reinterpret_cast<uint4*>(base + rows * 64 + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
     }
+}
+
+int prep_filter_bf16(int F, int Cin, int co0, int Cout, int nq, int nslices, int kst, int nsplit, int rows, int64_t s_co, int64_t s_ci,
+                     const float* filter, uint8_t* wimg, cudaStream_t stream) {
+    PB_LAUNCH("f2f_tc_gin_prep_filter", f2f_tc_gin_prep_filter_bf16_kernel, persistent_blocks((int64_t)nslices * kst * rows * 4, 256, 8), 256, 0,
+              stream, F, Cin, co0, Cout, nq, nslices, kst, nsplit, rows, s_co, s_ci, filter, wimg);
+    return PB200_OK;
 }
 
 // running sample count after face f; a null array stands for one sample per face
@@ -686,8 +642,8 @@ int backward_input(int64_t Nf, int Cin, int Cout, int F, const float* gout, cons
         const int kst = pl.bf ? (cchunk + 31) / 32 : (cchunk + KS - 1) / KS;
         const int64_t items = (int64_t)pl.nslices * kst * NCOLS * 4;
         if (pl.bf) {
-            PB_LAUNCH("f2f_tc_gin_prep_filter", f2f_tc_gin_prep_filter_bf16_kernel, persistent_blocks(items, 256, 8), 256, 0,
-                      stream, F, Cin, co0, cchunk, pl.nq, pl.nslices, kst, pl.nsplit, s_co, s_ci, filter, wimg);
+            rc = prep_filter_bf16(F, Cin, co0, cchunk, pl.nq, pl.nslices, kst, pl.nsplit, NCOLS, s_co, s_ci, filter, wimg, stream);
+            if (rc) return rc;
         } else {
             PB_LAUNCH("f2f_tc_gin_prep_filter", f2f_tc_gin_prep_filter_kernel, persistent_blocks(items, 256, 8), 256, 0,
                       stream, F, Cin, co0, cchunk, pl.nq, pl.nslices, kst, pl.nsplit, s_co, s_ci, filter, wimg);

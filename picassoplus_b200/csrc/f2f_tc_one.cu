@@ -1,0 +1,427 @@
+// facet2facet for faces with exactly one sample each, forward and input gradient, on tcgen05 + TMEM:
+//
+//   out[f, cn] = sum_d w[f, d] * sum_ck rows[f, ck] * W[ck, cn, d]
+//
+// (forward: rows = input, ck counts input channels, cn output channels; input gradient: rows = gradOutput, the roles
+// exchanged).  The inner sum is a product on the tensor cores, the outer one an epilogue over the accumulator: the scheme
+// of f2f_tc_gin.cu, whose kernel serves faces with several samples.  There the two warps of a TMEM quadrant share the
+// SAMPLES of a face; with one sample half of them did nothing but read the same columns again, and the other half's chain of
+// TMEM loads and sums per slice was three times as long as the slice's products at 64 channels (two scenes of 880 000 faces,
+// 64 -> 64, 16 bases: 924 us, products alone 300 us).  Here
+//   * 16 epilogue warps (thread = face) in two groups of eight, one group per accumulator, so a group has the time of two
+//     slices to drain one; the two warps of a quadrant in a group take the slice's channel quadruples in turn, load a
+//     quadruple's columns together, hand the accumulator back as soon as the last columns are in registers, and store 16 bytes
+//     per quadruple;
+//   * a slice holds a multiple of four channels (NQ), its filter image exactly the rows the product reads;
+//   * a work item is a tile of 128 faces and a run of slices: few tiles are spread over the chip by splitting their slices.
+// Loaders, filter stream and MMA issue as in f2f_tc_gin.cu.  What bounds it now: the three products per term at 64 channels
+// and more (bf16 hi + lo), the epilogue below and in bf16 mode.  All waits are bounded.
+#include "common.cuh"
+#include "tc_ptx.cuh"
+#include "tc_runtime.cuh"
+
+namespace pb {
+namespace tc {
+
+namespace gin {
+int prep_filter_bf16(int F, int Cin, int co0, int Cout, int nq, int nslices, int kst, int nsplit, int rows, int64_t s_co, int64_t s_ci,
+                     const float* filter, uint8_t* wimg, cudaStream_t stream);
+}
+
+namespace one {
+
+using namespace ptx;
+
+constexpr int TILE_M = 128;
+constexpr int NCOLS = 256;                       // accumulator columns
+constexpr int EWARPS = 16;                       // epilogue warps: 2 groups x 4 TMEM quadrants x 2
+constexpr int GWARPS = 2;                        // row loaders
+constexpr int NTHREADS = (EWARPS + 2 + GWARPS) * 32;
+constexpr int KTILE_BYTES = TILE_M * 64;         // 32 channels of the tile's rows
+constexpr int MAX_CK = 256;                      // contracted channels per launch
+
+struct Params {
+    int64_t Nf;
+    int Cn, Ck;
+    int nslices, kst, nmma;
+    int nstages, kb, gbufs;          // filter stages, K-blocks of 32 channels in one stage (divides kst)
+    int groups, per_group;           // slice groups of a tile, slices of a group
+    const float* rows;
+    int stride;                      // floats per row
+    int accumulate;                  // later chunks of contracted channels add to out
+    const float* w;                  // weight rows padded to Fp floats
+    int Fp;
+    const uint8_t* wimg;
+    float* out;
+    int* async_err;
+    int wait_budget;
+};
+
+template <int F> constexpr int NQ = F == 4 ? 64 : F == 9 ? 28 : F == 16 ? 16 : 10;      // channels of a slice
+template <int F> constexpr int G = F == 25 ? 2 : 4;                                     // channels of a step
+
+// sum over the F columns in v with the weights b: packed pairs, two chains
+template <int F>
+__device__ __forceinline__ float weighted(const float* v, const float (&b)[(F + 3) / 4 * 4]) {
+    float2 s0 = make_float2(0.f, 0.f), s1 = s0;
+#pragma unroll
+    for (int i = 0; i < F / 2; ++i) {
+        const float2 x = make_float2(v[2 * i], v[2 * i + 1]), y = make_float2(b[2 * i], b[2 * i + 1]);
+        if (i & 1) s1 = __ffma2_rn(y, x, s1);
+        else s0 = __ffma2_rn(y, x, s0);
+    }
+    float s = (s0.x + s1.x) + (s0.y + s1.y);
+    if (F & 1) s = fmaf(b[F - 1], v[F - 1], s);
+    return s;
+}
+
+template <int NSPLIT, int F>
+__global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p) {
+    constexpr int nq = NQ<F>;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int S = p.nstages, KST = p.kst;
+    const uint32_t gtile_bytes = (uint32_t)NSPLIT * KST * KTILE_BYTES;
+    const uint32_t w_bytes = (uint32_t)p.nmma * 64, wblk_bytes = NSPLIT * w_bytes, wstage_bytes = wblk_bytes * p.kb;
+    uint8_t* gtile = smem;
+    uint8_t* wst = smem + (size_t)p.gbufs * gtile_bytes;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(wst + (size_t)S * wstage_bytes);
+    uint64_t* w_full = bars;                  // [S]
+    uint64_t* w_empty = bars + S;             // [S]
+    uint64_t* acc_full = bars + 2 * S;        // [2]
+    uint64_t* acc_empty = bars + 2 * S + 2;   // [2]
+    uint64_t* g_full = bars + 2 * S + 4;      // [2] row tile buffer written
+    uint64_t* g_empty = bars + 2 * S + 6;     // [2] all products of the item done with the buffer
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S + 8);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    if (tid == 0) {
+        for (int s = 0; s < S; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], 1); }
+        for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], EWARPS / 2); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&g_full[b], GWARPS); mbar_init(&g_empty[b], 1); }
+        abort_flag[0] = 0;
+        abort_flag[1] = p.wait_budget;
+        fence_barrier_init();
+    }
+    if (warp == EWARPS) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    const int64_t nitems = (p.Nf + TILE_M - 1) / TILE_M * p.groups;
+
+    if (warp < EWARPS) {
+        // ===================== epilogue (thread = face) =====================
+        const int q = warp & 3, sub = (warp >> 2) & 1;
+        const uint32_t mine = (uint32_t)(warp >> 3);              // accumulator of this group
+        const int r = q * 32 + lane;
+        const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + mine * NCOLS;
+        const bool vec = p.Cn % G<F> == 0 && (reinterpret_cast<uintptr_t>(p.out) & (4 * G<F> - 1)) == 0;
+        uint32_t sc = 0;
+        bool alive = true;
+        for (int64_t item = blockIdx.x; item < nitems && alive; item += gridDim.x) {
+            const int64_t f = item / p.groups * TILE_M + r;
+            const int s0 = (int)(item % p.groups) * p.per_group;
+            const int s1 = s0 + p.per_group < p.nslices ? s0 + p.per_group : p.nslices;
+            const bool valid = f < p.Nf;
+            float b[(F + 3) / 4 * 4];
+            {
+                const float4* src = reinterpret_cast<const float4*>(p.w + (valid ? f : 0) * p.Fp);
+#pragma unroll
+                for (int i = 0; i < (F + 3) / 4; ++i) {
+                    const float4 v = valid ? ldg4(src + i) : zero4();
+                    b[4 * i] = v.x; b[4 * i + 1] = v.y; b[4 * i + 2] = v.z; b[4 * i + 3] = v.w;
+                }
+            }
+            float* const row = p.out + f * p.Cn;
+            auto store = [&](int c, const float (&s)[G<F>]) {
+                if (!valid || c >= p.Cn) return;
+                if (vec) {
+                    if constexpr (G<F> == 4) {
+                        float4 v = make_float4(s[0], s[1], s[2], s[3]);
+                        float4* dst = reinterpret_cast<float4*>(row + c);
+                        if (p.accumulate) add4(v, *dst);
+                        *dst = v;
+                    } else {
+                        float2 v = make_float2(s[0], s[1]);
+                        float2* dst = reinterpret_cast<float2*>(row + c);
+                        if (p.accumulate) { v.x += dst->x; v.y += dst->y; }
+                        *dst = v;
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < G<F>; ++j)
+                        if (c + j < p.Cn) row[c + j] = p.accumulate ? row[c + j] + s[j] : s[j];
+                }
+            };
+            for (int slice = s0; slice < s1; ++slice, ++sc) {
+                if ((sc & 1u) != mine) continue;
+                int ok = 1;
+                if (lane == 0) ok = mbar_wait(&acc_full[mine], (sc >> 1) & 1u, abort_flag) ? 1 : 0;
+                if (!__shfl_sync(0xffffffffu, ok, 0)) { alive = false; break; }
+                tc_fence_after();
+                const int c0 = slice * nq;
+                int left = (p.Cn - c0 + G<F> - 1) / G<F>;         // steps of the slice that exist
+                if (left > nq / G<F>) left = nq / G<F>;
+                auto hand_back = [&](int k) {                     // after the loads of this warp's last quadruple
+                    if (k + 2 < left) return;
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&acc_empty[mine]);
+                };
+                if (sub >= left) hand_back(left);                 // nothing of this slice for this warp
+                for (int k = sub; k < left; k += 2) {
+                    float s[G<F>], v[G<F> * F];
+                    const uint32_t t = tbase + (uint32_t)(k * G<F> * F);
+                    if constexpr (F == 16) { tmem_ld32f(t, v); tmem_ld32f(t + 32, v + 32); }
+                    else tmem_ld_row<G<F> * F>(t, v);
+                    tmem_ld_wait();
+                    hand_back(k);
+#pragma unroll
+                    for (int j = 0; j < G<F>; ++j) s[j] = weighted<F>(v + j * F, b);
+                    store(c0 + G<F> * k, s);
+                }
+            }
+        }
+    } else if (warp >= EWARPS + 2) {
+        // ===================== row loaders =====================
+        // a task is one 16-byte operand chunk (8 channels) of one row; consecutive lanes take consecutive chunks
+        const int gt = tid - (EWARPS + 2) * 32;
+        const int cpr = KST * 4, ntasks = TILE_M * cpr;
+        constexpr int U = 6;                                      // tasks in flight per thread
+        uint32_t icount = 0;
+        for (int64_t item = blockIdx.x; item < nitems; item += gridDim.x, ++icount) {
+            const int64_t f0 = item / p.groups * TILE_M;
+            const uint32_t gb = p.gbufs == 2 ? (icount & 1u) : 0u;
+            const uint32_t gph = p.gbufs == 2 ? ((icount >> 1) & 1u) : (icount & 1u);
+            uint8_t* const gdst = gtile + (size_t)gb * gtile_bytes;
+            if (warp == EWARPS + 2 && lane < 2) {                 // the next item's rows and weights, on their way to L2
+                const int64_t n0 = (item + gridDim.x) / p.groups * TILE_M;
+                if (n0 < p.Nf && n0 != f0) {
+                    const int64_t n = p.Nf - n0 < TILE_M ? p.Nf - n0 : TILE_M;
+                    if (lane == 0 && p.stride == p.Ck) prefetch_l2(p.rows + n0 * p.stride, (uint32_t)(n * p.stride * 4));
+                    if (lane == 1) prefetch_l2(p.w + n0 * p.Fp, (uint32_t)(n * p.Fp * 4));
+                }
+            }
+            int ok = 1;
+            if (lane == 0) ok = mbar_wait(&g_empty[gb], gph ^ 1u, abort_flag) ? 1 : 0;
+            if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+            for (int base = 0; base < ntasks; base += U * GWARPS * 32) {
+                float4 u[U], w[U];
+#pragma unroll
+                for (int j = 0; j < U; ++j) {
+                    const int idx = base + j * GWARPS * 32 + gt;
+                    const int rr = idx / cpr, c = idx - rr * cpr;
+                    const int64_t fr = f0 + rr;
+                    const float4* src = reinterpret_cast<const float4*>(p.rows + fr * p.stride);
+                    u[j] = zero4(); w[j] = zero4();
+                    if (idx < ntasks && fr < p.Nf && c * 8 < p.Ck) u[j] = ldg4(src + 2 * c);
+                    if (idx < ntasks && fr < p.Nf && c * 8 + 4 < p.Ck) w[j] = ldg4(src + 2 * c + 1);
+                }
+#pragma unroll
+                for (int j = 0; j < U; ++j) {
+                    const int idx = base + j * GWARPS * 32 + gt;
+                    if (idx >= ntasks) continue;
+                    const int rr = idx / cpr, c = idx - rr * cpr;
+                    uint8_t* dst = gdst + (size_t)(c >> 2) * KTILE_BYTES + swz64_offset((uint32_t)rr, (uint32_t)(c & 3));
+                    uint32_t hi[4], lo[4];
+                    if (NSPLIT == 1) {
+                        hi[0] = pack_bf16x2(u[j].x, u[j].y); hi[1] = pack_bf16x2(u[j].z, u[j].w);
+                        hi[2] = pack_bf16x2(w[j].x, w[j].y); hi[3] = pack_bf16x2(w[j].z, w[j].w);
+                    } else {
+                        split_bf16x2(u[j].x, u[j].y, hi[0], lo[0]); split_bf16x2(u[j].z, u[j].w, hi[1], lo[1]);
+                        split_bf16x2(w[j].x, w[j].y, hi[2], lo[2]); split_bf16x2(w[j].z, w[j].w, hi[3], lo[3]);
+                        *reinterpret_cast<uint4*>(dst + (size_t)KST * KTILE_BYTES) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                    }
+                    *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                }
+            }
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&g_full[gb]);
+        }
+    } else if (warp == EWARPS) {
+        // ===================== filter stream (TMA engine) =====================
+        if (lane == 0) {
+            int s = 0;
+            uint32_t ph = 0;
+            bool alive = true;
+            for (int64_t item = blockIdx.x; item < nitems && alive; item += gridDim.x) {
+                const int s0 = (int)(item % p.groups) * p.per_group;
+                const int s1 = s0 + p.per_group < p.nslices ? s0 + p.per_group : p.nslices;
+                for (int blk = s0 * KST; blk < s1 * KST; blk += p.kb) {
+                    if (!mbar_wait(&w_empty[s], ph ^ 1u, abort_flag)) { alive = false; break; }
+                    mbar_arrive_expect_tx(&w_full[s], wstage_bytes);
+                    bulk_g2s(wst + (size_t)s * wstage_bytes, p.wimg + (size_t)blk * wblk_bytes, wstage_bytes, &w_full[s]);
+                    if (++s == S) { s = 0; ph ^= 1u; }
+                }
+            }
+            if (!alive) {                                         // let copies in flight land before shared memory is released
+                const long long t0 = clock64();
+                while (clock64() - t0 < 2000000) { }
+            }
+        }
+    } else {
+        // ===================== MMA issue =====================
+        if (lane == 0) {
+            const uint32_t idesc = instr_desc(FMT_BF16, TILE_M, (uint32_t)p.nmma);
+            const uint64_t dg_base = smem_desc_kmajor(smem_u32(gtile), 64, SWZ_64B);
+            const uint64_t dw_base = smem_desc_kmajor(smem_u32(wst), 64, SWZ_64B);
+            int s = 0;
+            uint32_t ph = 0, icount = 0, sc = 0;
+            bool alive = true;
+            for (int64_t item = blockIdx.x; item < nitems && alive; item += gridDim.x, ++icount) {
+                const int s0 = (int)(item % p.groups) * p.per_group;
+                const int s1 = s0 + p.per_group < p.nslices ? s0 + p.per_group : p.nslices;
+                const uint32_t gb = p.gbufs == 2 ? (icount & 1u) : 0u;
+                const uint32_t gph = p.gbufs == 2 ? ((icount >> 1) & 1u) : (icount & 1u);
+                const uint64_t dg_tile = dg_base + (uint64_t)((gb * gtile_bytes) >> 4);
+                if (!mbar_wait(&g_full[gb], gph, abort_flag)) break;
+                for (int slice = s0; slice < s1 && alive; ++slice, ++sc) {
+                    const uint32_t a = sc & 1u;
+                    if (!mbar_wait(&acc_empty[a], ((sc >> 1) & 1u) ^ 1u, abort_flag)) { alive = false; break; }
+                    tc_fence_after();
+                    const uint32_t d_tmem = tmem_base + a * NCOLS;
+                    for (int ks0 = 0; ks0 < KST; ks0 += p.kb) {
+                        if (!mbar_wait(&w_full[s], ph, abort_flag)) { alive = false; break; }
+                        tc_fence_after();
+                        for (int kk = 0; kk < p.kb; ++kk) {
+                            const int ks = ks0 + kk;
+                            const uint64_t dg_hi = dg_tile + (uint64_t)(((uint32_t)ks * KTILE_BYTES) >> 4);
+                            const uint64_t dw_hi = dw_base + (uint64_t)(((uint32_t)s * wstage_bytes + kk * wblk_bytes) >> 4);
+#pragma unroll
+                            for (int k2 = 0; k2 < 2; ++k2) {
+                                const uint64_t adv = (uint64_t)(k2 * 2);
+                                const uint32_t first = (ks | k2) != 0;
+                                if (NSPLIT == 1) {
+                                    mma_f16(d_tmem, dg_hi + adv, dw_hi + adv, idesc, first);
+                                } else {
+                                    const uint64_t dg_lo = dg_hi + (uint64_t)(((uint32_t)KST * KTILE_BYTES) >> 4);
+                                    const uint64_t dw_lo = dw_hi + (uint64_t)(w_bytes >> 4);
+                                    mma_f16(d_tmem, dg_lo + adv, dw_hi + adv, idesc, first);
+                                    mma_f16(d_tmem, dg_hi + adv, dw_lo + adv, idesc, 1u);
+                                    mma_f16(d_tmem, dg_hi + adv, dw_hi + adv, idesc, 1u);
+                                }
+                            }
+                        }
+                        tc_commit(&w_empty[s]);
+                        if (++s == S) { s = 0; ph ^= 1u; }
+                    }
+                    if (alive) tc_commit(&acc_full[a]);
+                }
+                if (alive) tc_commit(&g_empty[gb]);
+            }
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == EWARPS) tmem_dealloc(tmem_base, 512);
+    if (tid == 0 && *abort_flag && p.async_err) {
+        *p.async_err = 2;
+        __threadfence_system();
+    }
+}
+
+// ---------------------------------------------------------------------------- host side
+struct Plan { int nsplit, nq, nslices, kst, nmma, nblocks, gbufs; size_t smem, wimg_bytes; };
+
+static int nq_of(int F) { return F == 4 ? NQ<4> : F == 9 ? NQ<9> : F == 16 ? NQ<16> : NQ<25>; }
+
+static Plan plan(int Cn, int CkAll, int F, int precision) {
+    Plan pl;
+    const int Ck = CkAll < MAX_CK ? CkAll : MAX_CK;
+    pl.nsplit = operand_mode(precision).nsplit;
+    pl.nq = nq_of(F);
+    const int g = F == 25 ? G<25> : G<4>, cn = (Cn + g - 1) / g * g;
+    if (pl.nq > cn) pl.nmma = (cn * F + 15) / 16 * 16;
+    else pl.nmma = (pl.nq * F + 15) / 16 * 16;
+    pl.nslices = (Cn + pl.nq - 1) / pl.nq;
+    pl.kst = (Ck + 31) / 32;
+    const size_t budget = 226 * 1024;
+    const size_t gt = (size_t)pl.nsplit * pl.kst * KTILE_BYTES, ws = (size_t)pl.nsplit * pl.nmma * 64;
+    // a second tile buffer takes the row copy off the critical path, when at least three filter stages still fit beside it
+    pl.gbufs = (2 * gt + 1024 + 384 + 3 * ws <= budget) ? 2 : 1;
+    const size_t fixed = pl.gbufs * gt + 1024 + 384;
+    pl.nblocks = (int)((budget - fixed) / ws);
+    if (pl.nblocks > 16) pl.nblocks = 16;
+    pl.smem = fixed + pl.nblocks * ws;
+    pl.wimg_bytes = (size_t)pl.nslices * pl.kst * ws;
+    return pl;
+}
+
+// bf16 operands (hi + lo or single), rows readable 16 bytes at a time
+bool supported(int Cn, int Ck, int F, int precision) {
+    if (precision != PB200_PREC_FP32 && precision != PB200_PREC_BF16) return false;
+    if (!(F == 4 || F == 9 || F == 16 || F == 25) || Cn < 1 || Ck < 4 || Ck % 4 != 0) return false;
+    const Plan pl = plan(Cn, Ck, F, precision);
+    return pl.nblocks >= 2 && pl.smem <= 227 * 1024;
+}
+
+size_t workspace_bytes(int Cn, int Ck, int F, int precision) { return align_up(plan(Cn, Ck, F, precision).wimg_bytes, 256); }
+
+template <int NSPLIT, int F>
+static int launch(const char* label, const Params& p, int grid, size_t smem, cudaStream_t stream) {
+    PB_CUDA(cudaFuncSetAttribute(f2f_one_sample_tc_kernel<NSPLIT, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PB_LAUNCH(label, (f2f_one_sample_tc_kernel<NSPLIT, F>), grid, NTHREADS, smem, stream, p);
+    return PB200_OK;
+}
+
+// forward = true: the operator's forward pass (filter (Cn, Ck, F)); false: its input gradient (filter (Ck, Cn, F))
+int run(int64_t Nf, int Cn, int Ck, int F, const float* rows, const float* filter, const float* w, int Fp, float* out, int precision,
+        void* ws, cudaStream_t stream, bool forward) {
+    const char* label = forward ? "f2f_fwd_one_sample_tc" : "f2f_bwd_gin_tc";
+    int rc = check_async_error(forward ? "facet2facet_forward" : "facet2facet_backward");
+    if (rc) return rc;
+    const Plan pl = plan(Cn, Ck, F, precision);
+    const int64_t s_ck = forward ? (int64_t)F : (int64_t)Cn * F, s_cn = forward ? (int64_t)Ck * F : (int64_t)F;
+    const int64_t ntiles = ceil_div(Nf, TILE_M);
+    const int sms = sm_count();
+    // Slice groups of a tile.  With fewer tiles than SMs a tile's slices go to as many CTAs as there are.  With a few tiles per
+    // SM the last wave is short of tiles: groups are halved while that evens it out, but a group keeps enough products (two
+    // slices of three, four of one) for the copy of the next item's rows to hide behind.
+    int groups = 1;
+    if (ntiles < sms) {
+        groups = (int)(sms / ntiles);
+        if (groups > pl.nslices) groups = pl.nslices;
+    } else {
+        const int keep = pl.nsplit == 2 ? 2 : 4;
+        while (ntiles * groups < 8LL * sms && pl.nslices >= 2 * groups * keep) groups *= 2;
+    }
+    const int per_group = (int)ceil_div(pl.nslices, groups);
+    groups = (int)ceil_div(pl.nslices, per_group);
+    const int64_t items = ntiles * groups;
+    const int grid = (int)(items < sms ? items : sms);
+    for (int k0 = 0; k0 < Ck; k0 += MAX_CK) {
+        const int chunk = Ck - k0 < MAX_CK ? Ck - k0 : MAX_CK;
+        const int kst = (chunk + 31) / 32;
+        rc = gin::prep_filter_bf16(F, Cn, k0, chunk, pl.nq, pl.nslices, kst, pl.nsplit, pl.nmma, s_ck, s_cn, filter, (uint8_t*)ws, stream);
+        if (rc) return rc;
+        Params p;
+        p.Nf = Nf; p.Cn = Cn; p.Ck = chunk;
+        p.nslices = pl.nslices; p.kst = kst; p.nmma = pl.nmma; p.gbufs = pl.gbufs;
+        p.kb = kst;
+        while (p.kb > 1 && (kst % p.kb != 0 || pl.nblocks < 2 * p.kb)) --p.kb;
+        p.nstages = pl.nblocks / p.kb;
+        p.groups = groups; p.per_group = per_group;
+        p.rows = rows + k0; p.stride = Ck; p.accumulate = k0 > 0 ? 1 : 0;
+        p.w = w; p.Fp = Fp; p.wimg = (const uint8_t*)ws; p.out = out;
+        p.async_err = async_error_word();
+        p.wait_budget = wait_budget_kclocks();
+        const bool two = pl.nsplit == 2;
+        switch (F) {
+            case 4: rc = two ? launch<2, 4>(label, p, grid, pl.smem, stream) : launch<1, 4>(label, p, grid, pl.smem, stream); break;
+            case 9: rc = two ? launch<2, 9>(label, p, grid, pl.smem, stream) : launch<1, 9>(label, p, grid, pl.smem, stream); break;
+            case 16: rc = two ? launch<2, 16>(label, p, grid, pl.smem, stream) : launch<1, 16>(label, p, grid, pl.smem, stream); break;
+            default: rc = two ? launch<2, 25>(label, p, grid, pl.smem, stream) : launch<1, 25>(label, p, grid, pl.smem, stream); break;
+        }
+        if (rc) return rc;
+    }
+    return PB200_OK;
+}
+
+}  // namespace one
+}  // namespace tc
+}  // namespace pb

@@ -70,6 +70,10 @@ __device__ __forceinline__ void fence_proxy_async() {
 }
 
 // -------------------------------------------------------------------- bulk (TMA) copies
+// bring a piece of memory towards L2; address 16-byte aligned, size a multiple of 16
+__device__ __forceinline__ void prefetch_l2(const void* src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
 // 1-D bulk copy global -> shared, completion counted in bytes on an mbarrier.  Source and
 // destination 16-byte aligned, size a multiple of 16.
 __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, uint32_t bytes, uint64_t* bar) {
@@ -134,6 +138,57 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// ---- TMEM loads of 1/4/8/16/32 consecutive columns (lane = row)
+__device__ __forceinline__ void tmem_ld1(uint32_t taddr, float* v) {
+    uint32_t r0;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r0) : "r"(taddr) : "memory");
+    v[0] = __uint_as_float(r0);
+}
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float* v) {
+    uint32_t r[4];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr) : "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
+    uint32_t r[16];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                 "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
+                   "=r"(r[15])
+                 : "r"(taddr) : "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void tmem_ld32f(uint32_t taddr, float* v) {
+    uint32_t r[32];
+    tmem_ld32(taddr, r);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// F consecutive columns -> v[0..F)
+template <int F>
+__device__ __forceinline__ void tmem_ld_row(uint32_t taddr, float* v) {
+    int o = 0;
+    if (F & 32) { tmem_ld32f(taddr + o, v + o); o += 32; }
+    if (F & 16) { tmem_ld16(taddr + o, v + o); o += 16; }
+    if (F & 8)  { tmem_ld8(taddr + o, v + o); o += 8; }
+    if (F & 4)  { tmem_ld4(taddr + o, v + o); o += 4; }
+    if (F & 2)  { tmem_ld1(taddr + o, v + o); tmem_ld1(taddr + o + 1, v + o + 1); o += 2; }
+    if (F & 1)  { tmem_ld1(taddr + o, v + o); }
+}
 
 // ---------------------------------------------------------------------- UMMA descriptors
 // Shared-memory matrix descriptor of a K-major operand tile stored as rows of `row_bytes`

@@ -165,6 +165,19 @@ void f2f_backward(const Scope& s, const Tensor& g, const Tensor& input, const Te
              "pb200_facet2facet_filter_gradient");
 }
 
+// one sample per face (one_each = 1, 2, ..., Nf)
+void f2f_one_sample_backward(const Scope& s, const Tensor& g, const Tensor& input, const Tensor& filter, const Tensor& weights,
+                             const Tensor& weights_padded, const Tensor& one_each, int precision, Tensor& gin, Tensor& gf) {
+    const int64_t Nf = input.size(0), Cin = input.size(1), Cout = filter.size(0), F = filter.size(2);
+    gin = s.floats({Nf, Cin});
+    gf = s.floats({Cout, Cin, F});
+    const size_t nb = pb200_facet2facet_backward_workspace_bytes(Nf, Nf, (int)Cin, (int)Cout, (int)F, precision);
+    Tensor ws = s.bytes(nb);
+    call(pb200_facet2facet_one_sample_backward(Nf, (int)Cin, (int)Cout, (int)F, fp(g), fp(input), fp(filter), fp(weights),
+                                               fp(weights_padded), ip(one_each), fpm(gin), fpm(gf), precision, ws.data_ptr(), nb, s.stream),
+         "pb200_facet2facet_one_sample_backward");
+}
+
 // --------------------------------------------------------------------------------------------------------- checks
 void check_v2f(const Tensor& input, const Tensor& filter, const Tensor& face) {
     check(input, "input", 2, at::kFloat);
@@ -242,13 +255,18 @@ struct F2V : Node {
 struct F2F : Node {
     SavedVariable input, filter, bary, bary_padded, cum;
     int precision = 0;
+    bool one_sample = false;
     variable_list apply(variable_list&& grads) override {
         variable_list out(2);
         if (!grads[0].defined()) return out;
         std::lock_guard<std::mutex> lock(mutex_);
         const Tensor x = input.unpack();
         Scope s(x);
-        f2f_backward(s, aligned(upstream(grads)), aligned(x), filter.unpack(), aligned(bary.unpack()), bary_padded.unpack(),
+        if (one_sample)
+            f2f_one_sample_backward(s, aligned(upstream(grads)), aligned(x), filter.unpack(), aligned(bary.unpack()), bary_padded.unpack(),
+                                    cum.unpack(), precision, out[0], out[1]);
+        else
+            f2f_backward(s, aligned(upstream(grads)), aligned(x), filter.unpack(), aligned(bary.unpack()), bary_padded.unpack(),
                      cum.unpack(), precision, out[0], out[1], task_should_compute_output(0));
         return out;
     }
@@ -273,8 +291,8 @@ struct ConvBlock : Node {
         Tensor gz, gy, gs;
         f2v_backward(s, upstream(grads), z.unpack(), filter_out.unpack(), coeff.unpack(), fc, nf_count.unpack(), vt_map.unpack(),
                      gz, out[3]);
-        f2f_backward(s, gz, y.unpack(), filter.unpack(), weights.unpack(), weights_padded.unpack(), one_each.unpack(), precision,
-                     gy, out[2], true);
+        f2f_one_sample_backward(s, gz, y.unpack(), filter.unpack(), weights.unpack(), weights_padded.unpack(), one_each.unpack(),
+                                precision, gy, out[2]);
         gz.reset();
         v2f_backward(s, gy, xin, sp, fc, rowptr.unpack(), entries.unpack(), out[0], gs);
         if (task_should_compute_output(1)) {
@@ -397,6 +415,7 @@ Tensor facet2facet_shared_rows(const Tensor& rows_in, const Tensor& filter_in, c
         node->bary = keep(weights);
         node->bary_padded = keep(or_undefined(weights_padded));
         node->cum = keep(one_each);
+        node->one_sample = true;
         node->precision = precision;
         torch::autograd::set_history(out, node);
     }
