@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_fwd_tc_kernel(FwdParams p) {
         }
     } else if (warp == PWARPS) {
         // ================================ filter loader (TMA engine) ==========================
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t bytes = (uint32_t)(NSPLIT * FILT_TILE_BYTES);
             int s = 0;
             uint32_t ph = 0;
@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_fwd_tc_kernel(FwdParams p) {
         }
     } else {
         // ================================ MMA issuer =========================================
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = instr_desc(BF ? FMT_BF16 : FMT_TF32, UM, TILE_F);
             const uint64_t dbase = smem_desc_kmajor(smem_u32(stages), 64, SWZ_64B);
             int s = 0;

@@ -119,9 +119,6 @@ constexpr int BATOM_BYTES = 1024;
 constexpr int BG_SBO = (UM / 64) * BATOM_BYTES;
 constexpr int BG_TILE_BYTES = (KF / 8) * BG_SBO;
 __host__ __device__ constexpr int at_blocks_b16(int F) { return (F * CG + 63) / 64; }
-__device__ __forceinline__ void sts_u2(uint32_t a, uint32_t x, uint32_t y) {
-    asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(a), "r"(x), "r"(y) : "memory");
-}
 __device__ __forceinline__ void sts_u4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
     asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
@@ -150,16 +147,6 @@ __device__ __forceinline__ void put4_b16(uint32_t a, uint32_t lo_off, const floa
         sts_u2(a, hi[0], hi[1]);
         sts_u2(a + lo_off, lo[0], lo[1]);
     }
-}
-
-// one whole warp waits on an mbarrier phase: every lane probes once, then lane 0 waits (bounded)
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int lane) {
-    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity) ? 1 : 0)) return true;
-    int ok = 1;
-    if (lane == 0) ok = mbar_wait(bar, parity, abort_flag) ? 1 : 0;
-    ok = __shfl_sync(0xffffffffu, ok, 0);
-    if (ok) (void)mbar_try_wait(bar, parity);   // every lane observes the completed phase itself
-    return ok != 0;
 }
 
 // One compute warp's share of a flush: its TMEM lane quadrant, every second group of 32 accumulator
@@ -296,7 +283,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_bwd_gfilter_tc_kernel(Params 
                 const int one = __any_sync(0xffffffffu, T > 1) ? 0 : 1;          // no face of the stage has a second sample
                 if (lane == KF) sts_i4(rb32 + RAW_REC_OFF + KF * 16, slow, one, ks0, ns);
                 __syncwarp();
-                if (lane == 0) {
+                if (elect_one()) {
                     // the stage's bary rows: one bulk copy (rows are 16-byte multiples)
                     const uint32_t bbytes = (uint32_t)(ns * p.Fp * 4);
                     mbar_arrive_expect_tx(bar, bbytes);
@@ -520,7 +507,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_bwd_gfilter_tc_kernel(Params 
         }
     } else {
         // ==================================== MMA issuer ====================================
-        if (lane == 0) {
+        if (elect_one()) {
             const int n1 = NR < 256 ? NR : 256, n2 = NR - n1;
             const uint32_t idesc1 = instr_desc_mnmajor(BF ? FMT_BF16 : FMT_TF32, UM, (uint32_t)n1);
             const uint32_t idesc2 = instr_desc_mnmajor(BF ? FMT_BF16 : FMT_TF32, UM, (uint32_t)(n2 > 0 ? n2 : 16));

@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_bwd_gin_tc_kernel(Params p) {
         }
     } else if (warp == EWARPS) {
         // ===================== filter loader (TMA engine) =====================
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t bytes = (uint32_t)wstage_bytes;
             int s = 0;
             uint32_t ph = 0;
@@ -492,7 +492,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_bwd_gin_tc_kernel(Params p) {
         }
     } else {
         // ===================== MMA issuer =====================
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = instr_desc(BF ? FMT_BF16 : FMT_TF32, TILE_M, (uint32_t)p.nmma);
             const uint64_t dg_base = smem_desc_kmajor(smem_u32(gtile), 64, SWZ_64B);
             const uint64_t dw_base = smem_desc_kmajor(smem_u32(wst), 64, SWZ_64B);

@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
         }
     } else if (warp == EWARPS) {
         // ===================== filter stream (TMA engine) =====================
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0;
             uint32_t ph = 0;
             bool alive = true;
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
         }
     } else {
         // ===================== MMA issue =====================
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = instr_desc(FMT_BF16, TILE_M, (uint32_t)p.nmma);
             const uint64_t dg_base = smem_desc_kmajor(smem_u32(gtile), 64, SWZ_64B);
             const uint64_t dw_base = smem_desc_kmajor(smem_u32(wst), 64, SWZ_64B);

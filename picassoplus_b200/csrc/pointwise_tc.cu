@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) rows_pointwise_tc_kernel(Params p
         }
     } else if (warp == PWARPS) {
         // ================================ weight loader (TMA engine) ==========================
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t bytes = (uint32_t)(NSPLIT * W_TILE_BYTES);
             int s = 0;
             uint32_t ph = 0;
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) rows_pointwise_tc_kernel(Params p
         }
     } else {
         // ================================ MMA issuer =========================================
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = instr_desc(FMT_BF16, UM, TILE_R);
             const uint64_t dbase = smem_desc_kmajor(smem_u32(stages), 64, SWZ_64B);
             int s = 0;

@@ -57,9 +57,6 @@ struct Params {
 
 __host__ __device__ constexpr size_t stage_bytes(int nsplit) { return (size_t)nsplit * (A_TILE + B_TILE); }
 
-__device__ __forceinline__ void sts_u2(uint32_t a, uint32_t x, uint32_t y) {
-    asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(a), "r"(x), "r"(y) : "memory");
-}
 // four consecutive columns of a K-row: one 8-byte piece in the hi tile (and in the lo tile)
 template <int NSPLIT>
 __device__ __forceinline__ void put4(uint32_t a, uint32_t lo_off, const float4& v) {
@@ -184,7 +181,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) rows_contract_tc_kernel(Params p)
             }
             tc_fence_before();
         }
-    } else if (lane == 0) {
+    } else if (elect_one()) {
         // ================================== product issuer ==================================
         const uint32_t idesc = instr_desc_mnmajor(FMT_BF16, UM, (uint32_t)nmma);
         const uint64_t da0 = smem_desc_mnmajor_b16(s32, ATOM, SBO_A);
