@@ -30,6 +30,12 @@ size_t workspace_bytes(int Cn, int Ck, int F, int precision);
 int run(int64_t Nf, int Cn, int Ck, int F, const float* rows, const float* filter, const float* w, int Fp, float* out, int precision,
         void* ws, cudaStream_t stream, bool forward);
 }  // namespace one
+namespace onef {
+bool supported(int Cin, int Cout, int F, int precision);
+size_t workspace_bytes(int64_t Nf, int Cin, int Cout, int F, int precision);
+int backward_filter(int64_t Nf, int Cin, int Cout, int F, const float* gout, const float* input, const float* w, float* gfilter,
+                    int precision, void* ws, cudaStream_t stream);
+}  // namespace onef
 namespace gfilter {
 bool supported(int Cin, int Cout, int F);
 bool fits(int64_t Nf, int Cin, int Cout, int F, int precision);
@@ -165,12 +171,19 @@ static size_t gin_ws(int Cin, int Cout, int F, int precision) {
     return a > b ? a : b;
 }
 
+// room for the partial sums of either filter-gradient kernel
+static size_t gf_ws(int64_t Nf, int Cin, int Cout, int F, int precision) {
+    const size_t a = tc::gfilter::workspace_bytes(Nf, Cin, Cout, F, precision);
+    const size_t b = tc::onef::supported(Cin, Cout, F, precision) ? tc::onef::workspace_bytes(Nf, Cin, Cout, F, precision) : 0;
+    return a > b ? a : b;
+}
+
 size_t pb200_facet2facet_backward_workspace_bytes(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, int precision) {
     if (!f2f_sizes_ok(Nf, NiK, Cin, Cout, F)) return 0;
     const bool tg = use_tc_gin(Cin, Cout, F, precision), tf = use_tc_gf(Nf, Cin, Cout, F, precision);
     size_t n = (tg && tf) ? 0 : f2f_simt_bwd_ws(Nf, Cin, Cout, F);
     if (tg) n += gin_ws(Cin, Cout, F, precision);
-    if (tf) n += tc::gfilter::workspace_bytes(Nf, Cin, Cout, F, precision);
+    if (tf) n += gf_ws(Nf, Cin, Cout, F, precision);
     if (tg || tf) n += tc::padded_bary_bytes(NiK, F);
     if (tf) n += tc::padded_input_bytes(NiK, Cin);
     return n;
@@ -214,7 +227,7 @@ static int f2f_backward_impl(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, 
             bary_p = baryPadded;
         } else {
             char* wp = w + (tg ? gin_ws(Cin, Cout, F, precision) : 0) +
-                       (tf ? tc::gfilter::workspace_bytes(Nf, Cin, Cout, F, precision) : 0);
+                       (tf ? gf_ws(Nf, Cin, Cout, F, precision) : 0);
             int rc = tc::pad_bary(NiK, F, bary, (float*)wp, stream);
             if (rc) return rc;
             bary_p = (const float*)wp;
@@ -230,7 +243,10 @@ static int f2f_backward_impl(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, 
         }
         w += gin_ws(Cin, Cout, F, precision);
     }
-    if (tf) {
+    if (tf && one_each && tc::onef::supported(Cin, Cout, F, precision)) {
+        int rc = tc::onef::backward_filter(Nf, Cin, Cout, F, gradOutput, input, bary_p, gradFilter, precision, w, stream);
+        if (rc) return rc;
+    } else if (tf) {
         // the filter-gradient kernel reads 16 input channels per CTA with 16-byte copies: channel counts that
         // are not a multiple of 16 go through a zero-padded copy at the end of the workspace
         const float* input_p = input;
