@@ -45,7 +45,7 @@ constexpr int TMEM_COLS = 512;
 constexpr int ACOLS = 16;                     // columns of one tile's operand in a stage
 constexpr int MAX_SLOTS = 8;                  // stages of the plain operand in shared memory
 constexpr int MAX_F = 32;
-constexpr int MAX_NT = 8;                      // tiles of a CTA
+constexpr int MAX_NT = 5;                      // tiles of a CTA
 constexpr int MAX_RAW = 8;                    // stages of raw rows in shared memory
 constexpr int FLUSH_FACES = 4096;             // as in f2f_tc_gfilter.cu
 
@@ -107,9 +107,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_gfilter_kernel(Par
     constexpr int FS = FACES<NSPLIT>;
     constexpr int FLUSH = FLUSH_FACES / FS;
     constexpr int W_BYTES = MAX_F * FS * 4;                       // weights of a stage, [basis][face]
-    // A wait tells a barrier's phase from the one before, not from the one two before.  A warp that takes every fourth stage
-    // therefore has rings of 4 or 8 slots, where it has itself seen a slot's last phase.  The operand ring may be shorter: its
-    // barriers belong to stages (mod 4), and the stage st - nbuf that a warp waits for follows one it has waited for before.
+    // A wait tells a barrier's phase from the one before, not from the one two before or behind.  A warp that takes every
+    // fourth stage therefore has rings of 4 or 8 slots, where it has itself seen a slot's last phase; what it waits for of the
+    // products is the end of a stage 2 to 8 stages back, on barriers that come round every 8 stages.
     static_assert(EG == 4 && GWARPS == 4, "see the ring depths");
     const int SLOTS = p.slots;
     extern __shared__ uint8_t smem_raw[];
@@ -125,10 +125,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_gfilter_kernel(Par
     uint8_t* const raw = wring + SLOTS * W_BYTES;
     uint64_t* bars = reinterpret_cast<uint64_t*>(raw + p.nraw * (size_t)raw_bytes);
     uint64_t* g_full = bars;                      // [SLOTS]   plain operand and weights of a stage written
-    uint64_t* g_empty = bars + MAX_SLOTS;         // [SLOTS]   products of the stage done
-    uint64_t* a_full = bars + 2 * MAX_SLOTS;      // [4]       expanded operand of a stage (mod 4) written
-    uint64_t* a_empty = bars + 2 * MAX_SLOTS + 4; // [4]       products of the stage done
-    uint64_t* raw_full = bars + 2 * MAX_SLOTS + 8; // [MAX_RAW] rows of a stage have arrived
+    uint64_t* a_full = bars + MAX_SLOTS;          // [4]       expanded operand of a stage (mod 4) written
+    uint64_t* done = a_full + 4;                  // [8]       products of a stage (mod 8) done
+    uint64_t* raw_full = done + 8;                // [MAX_RAW] rows of a stage have arrived
     uint64_t* raw_free = raw_full + MAX_RAW;      // [MAX_RAW] and have been read
     uint64_t* acc_done = raw_free + MAX_RAW;      // all products issued so far complete
     uint64_t* acc_free = acc_done + 1;            // accumulators read out
@@ -136,8 +135,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_gfilter_kernel(Par
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     if (tid == 0) {
-        for (int s = 0; s < SLOTS; ++s) { mbar_init(&g_full[s], 1); mbar_init(&g_empty[s], 1); }
-        for (int b = 0; b < 4; ++b) { mbar_init(&a_full[b], 4); mbar_init(&a_empty[b], 1); }
+        for (int s = 0; s < SLOTS; ++s) mbar_init(&g_full[s], 1);
+        for (int b = 0; b < 4; ++b) mbar_init(&a_full[b], 4);
+        for (int b = 0; b < 8; ++b) mbar_init(&done[b], 1);
         for (int r = 0; r < p.nraw; ++r) { mbar_init(&raw_full[r], 1); mbar_init(&raw_free[r], 5); }
         mbar_init(acc_done, 1);
         mbar_init(acc_free, EWARPS);
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_gfilter_kernel(Par
             }
             const int slot = gr.i;
             if (!warp_wait(&g_full[slot], gr.ph, abort_flag, lane) ||
-                (st >= p.nbuf && !warp_wait(&a_empty[(st - p.nbuf) & 3], (uint32_t)((st - p.nbuf) >> 2) & 1u, abort_flag, lane))) {
+                (st >= p.nbuf && !warp_wait(&done[(st - p.nbuf) & 7], (uint32_t)((st - p.nbuf) >> 3) & 1u, abort_flag, lane))) {
                 alive = false;
                 break;
             }
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_gfilter_kernel(Par
         for (int st = gw; st < nst; st += GWARPS) {
             const int64_t left = p.Nf - (st0 + st) * FS;
             const int n = left < FS ? (int)left : FS;              // faces of the stage
-            if (!warp_wait(&g_empty[gr.i], gr.ph ^ 1u, abort_flag, lane) ||
+            if ((st >= SLOTS && !warp_wait(&done[(st - SLOTS) & 7], (uint32_t)((st - SLOTS) >> 3) & 1u, abort_flag, lane)) ||
                 !warp_wait(&raw_full[rr.i], rr.ph, abort_flag, lane)) break;
             const uint32_t rb = raw32 + (uint32_t)rr.i * raw_bytes, gdst = g32 + (uint32_t)gr.i * slot_bytes;
             if (p.N <= 32) put_rows(std::integral_constant<int, 8>{}, rb + raw_g, gdst, n);
@@ -326,46 +326,58 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_gfilter_kernel(Par
         // ===================== products =====================
         const uint32_t idesc = instr_desc(FMT_BF16, ROWS, (uint32_t)p.N) | (1u << 16);      // B is MN-major
         const uint64_t dg = smem_desc_mnmajor_b16(smem_u32(gring), 1024, sbo);
-        bool alive = true, fresh = true, wait_free = false;
-        uint32_t fph = 0;
-        int boundary = FLUSH - 1;
-        Ring ar;
-        for (int st = 0; st < nst; ++st) {
-            const int slot = st & (SLOTS - 1);
-            if (wait_free) {
-                wait_free = false;
-                if (!mbar_wait(acc_free, fph, abort_flag)) { alive = false; break; }
-                fph ^= 1u;
-                fresh = true;
-            }
-            // (the warps that report the expanded operand have seen the plain one)
-            if (!mbar_wait(&a_full[st & 3], (uint32_t)(st >> 2) & 1u, abort_flag)) { alive = false; break; }
-            tc_fence_after();
-            const uint64_t g_hi = dg + (uint64_t)(((uint32_t)slot * slot_bytes) >> 4), g_lo = g_hi + (uint64_t)(g_split >> 4);
-            const uint32_t a = tmem_base + (uint32_t)(p.a_col + ar.i * p.nt * ACOLS);
-            auto round = [&](uint32_t acol, uint64_t b, uint32_t acc) {
+        const uint32_t a_first = tmem_base + (uint32_t)p.a_col, a_step = (uint32_t)(p.nt * ACOLS), a_end = a_first + p.nbuf * a_step;
+        const uint64_t g_step = slot_bytes >> 4, g_end = dg + SLOTS * g_step, lo = g_split >> 4;
+        // every instruction of this thread is on the way from one stage to the next: the number of tiles is a constant in it
+        auto products = [&](auto ntc) {
+            constexpr int NT = decltype(ntc)::value;
+            uint32_t d[NT];
 #pragma unroll
-                for (int t = 0; t < MAX_NT; ++t)
-                    if (t < nt) mma_f16_ta(tmem_base + (uint32_t)(t * p.N), a + (uint32_t)(t * ACOLS) + acol, b, idesc, acc);
-            };
-            if (NSPLIT == 2) {
-                round(8, g_hi, fresh ? 0u : 1u);
-                round(0, g_lo, 1u);
-                round(0, g_hi, 1u);
-            } else {
-                round(0, g_hi, fresh ? 0u : 1u);
-                round(8, g_hi + (uint64_t)((2 * sbo) >> 4), 1u);
+            for (int t = 0; t < NT; ++t) d[t] = tmem_base + (uint32_t)(t * p.N);
+            bool wait_free = false;
+            uint32_t fph = 0, accumulate = 0, a = a_first;
+            uint64_t g_hi = dg;
+            int left = FLUSH;                                      // stages until the next flush
+            for (int st = 0; st < nst; ++st) {
+                // (the warps that report the expanded operand have seen the plain one)
+                if (!mbar_wait(&a_full[st & 3], (uint32_t)(st >> 2) & 1u, abort_flag)) return;
+                if (wait_free) {
+                    wait_free = false;
+                    if (!mbar_wait(acc_free, fph, abort_flag)) return;
+                    fph ^= 1u;
+                    accumulate = 0;
+                }
+                tc_fence_after();
+                auto round = [&](uint32_t acol, uint64_t b, uint32_t acc) {
+#pragma unroll
+                    for (int t = 0; t < NT; ++t) mma_f16_ta(d[t], a + (uint32_t)(t * ACOLS) + acol, b, idesc, acc);
+                };
+                if (NSPLIT == 2) {
+                    round(8, g_hi, accumulate);
+                    round(0, g_hi + lo, 1u);
+                    round(0, g_hi, 1u);
+                } else {
+                    round(0, g_hi, accumulate);
+                    round(8, g_hi + (uint64_t)((2 * sbo) >> 4), 1u);
+                }
+                tc_commit(&done[st & 7]);
+                accumulate = 1;
+                if (--left == 0) {
+                    left = FLUSH;
+                    if (st + p.nbuf + EG < nst) { tc_commit(acc_done); wait_free = true; }
+                }
+                if ((a += a_step) == a_end) a = a_first;
+                if ((g_hi += g_step) == g_end) g_hi = dg;
             }
-            fresh = false;
-            tc_commit(&g_empty[slot]);
-            tc_commit(&a_empty[st & 3]);
-            if (st == boundary) {
-                if (boundary + p.nbuf + EG < nst) { tc_commit(acc_done); wait_free = true; }
-                boundary += FLUSH;
-            }
-            ar.step(1, p.nbuf);
+            tc_commit(acc_done);
+        };
+        switch (nt) {
+            case 1: products(std::integral_constant<int, 1>{}); break;
+            case 2: products(std::integral_constant<int, 2>{}); break;
+            case 3: products(std::integral_constant<int, 3>{}); break;
+            case 4: products(std::integral_constant<int, 4>{}); break;
+            default: products(std::integral_constant<int, 5>{}); break;
         }
-        if (alive) tc_commit(acc_done);
     }
     __syncwarp();
     tc_fence_before();
