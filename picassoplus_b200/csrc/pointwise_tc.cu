@@ -34,7 +34,9 @@ using namespace ptx;
 constexpr int TILE_R = 256;                 // rows per tile (UMMA N)
 constexpr int UM = 128;                     // output channels per launch (UMMA M), zero-padded
 constexpr int PWARPS = 16;
-constexpr int NTHREADS = (PWARPS + 2) * 32;
+constexpr int EWARPS = 4;                   // epilogue: one warp per TMEM quadrant
+constexpr int W_WARP = PWARPS + EWARPS, MMA_WARP = W_WARP + 1;
+constexpr int NTHREADS = (MMA_WARP + 1) * 32;
 constexpr int ROW_TILE_BYTES = TILE_R * 64;
 constexpr int W_TILE_BYTES = UM * 64;
 constexpr int KB = 32;                      // channels per stage (one 64-byte bf16 operand row)
@@ -118,18 +120,19 @@ __global__ void __launch_bounds__(NTHREADS, 1) rows_pointwise_tc_kernel(Params p
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)S * sbytes);
     uint64_t* full = bars;                        // [S] producers (16 warps) + weight bytes
     uint64_t* empty = bars + S;                   // [S] MMA done with the stage
-    uint64_t* acc_full = bars + 2 * S;            // accumulator of the tile complete
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S + 1);
+    uint64_t* acc_full = bars + 2 * S;            // [2] accumulator of a tile complete
+    uint64_t* acc_free = bars + 2 * S + 2;        // [2] and read out
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S + 4);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     if (tid == 0) {
         for (int s = 0; s < S; ++s) { mbar_init(&full[s], PWARPS + 1); mbar_init(&empty[s], 1); }
-        mbar_init(acc_full, 1);
+        for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_free[a], EWARPS); }
         abort_flag[0] = 0;
         abort_flag[1] = p.wait_budget;
         fence_barrier_init();
     }
-    if (warp == PWARPS) { tmem_alloc(tmem_slot, TILE_R); tmem_relinquish(); }
+    if (warp == W_WARP) { tmem_alloc(tmem_slot, 2 * TILE_R); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -137,168 +140,197 @@ __global__ void __launch_bounds__(NTHREADS, 1) rows_pointwise_tc_kernel(Params p
     const int64_t ntiles = (p.Nrows + TILE_R - 1) / TILE_R;
 
     if (warp < PWARPS) {
-        // ================================ producers + epilogue ================================
-        const int ml = lane >> 1, h = lane & 1;               // row within the warp's 16, 8-channel half
-        const int m = warp * 16 + ml;
-        const uint32_t offb0 = swz64_offset((uint32_t)m, (uint32_t)h), offb1 = swz64_offset((uint32_t)m, (uint32_t)(2 + h));
+        // ===================================== producers =====================================
+        // A warp has 16 rows of the tile, four at a time: lane = row rg of the four, channels 4j..4j+3 of the stage's 32.  A warp's
+        // load then reads whole 128-byte lines (two lanes of 32 bytes per row met 16 lines per load, and the L1 was what the
+        // kernel waited for).
+        const int rg = lane >> 3, j = lane & 7, m0 = warp * 16 + rg;
         const uint32_t stages32 = smem_u32(stages);
         int st_i = 0;
-        uint32_t st_ph = 0, tcount = 0;
-        bool alive = true;
+        uint32_t st_ph = 0;
 
-        // 8 channels of 16-channel block `b16` of the row into the current stage (two blocks per stage)
-        auto publish = [&](const float4& a0, const float4& a1, int b16) -> bool {
-            if ((b16 & 1) == 0) {
-                if (!mbar_try_wait(&empty[st_i], st_ph ^ 1u)) {
-                    int ok = 1;
-                    if (lane == 0) ok = mbar_wait(&empty[st_i], st_ph ^ 1u, abort_flag) ? 1 : 0;
-                    ok = __shfl_sync(0xffffffffu, ok, 0);
-                    if (!ok) return false;
-                }
-            }
-            const uint32_t st = stages32 + (uint32_t)st_i * (uint32_t)sbytes;
-            uint32_t hi[4], lo[4];
-            if (NSPLIT == 1) {
-                hi[0] = pack_bf16x2(a0.x, a0.y); hi[1] = pack_bf16x2(a0.z, a0.w);
-                hi[2] = pack_bf16x2(a1.x, a1.y); hi[3] = pack_bf16x2(a1.z, a1.w);
-            } else {
-                split_bf16x2(a0.x, a0.y, hi[0], lo[0]); split_bf16x2(a0.z, a0.w, hi[1], lo[1]);
-                split_bf16x2(a1.x, a1.y, hi[2], lo[2]); split_bf16x2(a1.z, a1.w, hi[3], lo[3]);
-            }
-            const uint32_t ob = (b16 & 1) ? offb1 : offb0;
-            sts_f4(st + ob, make_float4(__uint_as_float(hi[0]), __uint_as_float(hi[1]), __uint_as_float(hi[2]), __uint_as_float(hi[3])));
-            if (NSPLIT == 2)
-                sts_f4(st + ROW_TILE_BYTES + ob, make_float4(__uint_as_float(lo[0]), __uint_as_float(lo[1]), __uint_as_float(lo[2]), __uint_as_float(lo[3])));
-            if ((b16 & 1) == 0) return true;                  // the stage is complete with the odd block
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&full[st_i]);
-            if (++st_i == S) { st_i = 0; st_ph ^= 1u; }
-            return true;
-        };
-
-        for (int64_t tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x, ++tcount) {
-            const int64_t r0 = tile * TILE_R;
-            const int64_t row = r0 + m;
-            const bool valid = row < p.Nrows;
-            int v0 = -1, v1 = -1, v2 = -1, beg = 0, end = 0;
-            float inv_n = 0.f;
+        // what the warp's rows are made of, a row per lane; the next tile's is loaded while this one's rows are
+        struct Source { int v[3]; int beg, n; float inv_n; };
+        auto source = [&](int64_t tile, Source& s) {
+            const int64_t row = tile * TILE_R + warp * 16 + lane;
+            const bool valid = lane < 16 && row < p.Nrows;
             if (MODE == 0) {
-                if (valid) {
-                    v0 = __ldg(p.face + 3 * row); v1 = __ldg(p.face + 3 * row + 1); v2 = __ldg(p.face + 3 * row + 2);
-                    if (v0 < 0 || v0 >= p.Nv) v0 = -1;            // a bad index contributes nothing
-                    if (v1 < 0 || v1 >= p.Nv) v1 = -1;
-                    if (v2 < 0 || v2 >= p.Nv) v2 = -1;
-                }
-            } else if (valid) {
-                beg = __ldg(p.rowptr + row); end = __ldg(p.rowptr + row + 1);
-                if (end > beg) inv_n = 1.f / (float)__ldg(p.nfCount + row);
-            }
-            for (int b16 = 0; b16 < 2 * p.nkb && alive; ++b16) {
-                const int c = b16 * 16 + h * 8;
-                float4 a0 = zero4(), a1 = zero4();
-                if (c < C) {
-                    if (MODE == 0) {
-                        // the k-ascending FMA chain of the stand-alone vertex2facet kernel
-                        const int vs[3] = {v0, v1, v2};
 #pragma unroll
-                        for (int k = 0; k < 3; ++k) {
-                            if (vs[k] >= 0) {
-                                const float4* x = reinterpret_cast<const float4*>(p.vin + (int64_t)vs[k] * C + c);
-                                const float4* f = reinterpret_cast<const float4*>(p.vfilt + (int64_t)k * C + c);
-                                fma4(a0, ldg4(f), ldg4(x));
-                                fma4(a1, ldg4(f + 1), ldg4(x + 1));
+                for (int k = 0; k < 3; ++k) {
+                    s.v[k] = valid ? __ldg(p.face + 3 * row + k) : -1;
+                    if (s.v[k] < 0 || s.v[k] >= p.Nv) s.v[k] = -1;            // a bad index contributes nothing
+                }
+            } else if (MODE == 1) {
+                s.beg = valid ? __ldg(p.rowptr + row) : 0;
+                s.n = valid ? __ldg(p.rowptr + row + 1) - s.beg : 0;
+                s.inv_n = s.n > 0 ? 1.f / (float)__ldg(p.nfCount + row) : 0.f;
+            }
+        };
+        Source cur, nxt;
+        source(blockIdx.x, nxt);
+        for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+            const int64_t row0 = tile * TILE_R + m0;             // rows row0 + 4k
+            cur = nxt;
+            source(tile + gridDim.x, nxt);
+            int id[4], beg[4], n[4], most[4];
+            if (MODE == 1) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    beg[k] = __shfl_sync(0xffffffffu, cur.beg, 4 * k + rg);
+                    n[k] = __shfl_sync(0xffffffffu, cur.n, 4 * k + rg);
+                    most[k] = __reduce_max_sync(0xffffffffu, n[k]);
+                    id[k] = j < n[k] ? __ldg(p.entries + beg[k] + j) >> 2 : 0;
+                }
+            }
+            for (int kb = 0; kb < p.nkb; ++kb) {
+                float4 a[4];
+                const int c = kb * KB + 4 * j;
+                const bool in = c < C;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) a[k] = zero4();
+                if (MODE == 0) {
+                    // the k-ascending FMA chain of the stand-alone vertex2facet kernel, the loads of two rows ahead of it
+                    float4 fl[3];
+#pragma unroll
+                    for (int t = 0; t < 3; ++t) fl[t] = in ? ldg4(reinterpret_cast<const float4*>(p.vfilt + (int64_t)t * C + c)) : zero4();
+#pragma unroll
+                    for (int k0 = 0; k0 < 4; k0 += 2) {
+                        int v[2][3];
+                        float4 x[2][3];
+#pragma unroll
+                        for (int k = 0; k < 2; ++k)
+#pragma unroll
+                            for (int t = 0; t < 3; ++t) {
+                                v[k][t] = __shfl_sync(0xffffffffu, cur.v[t], 4 * (k0 + k) + rg);
+                                if (!in) v[k][t] = -1;
+                                if (v[k][t] >= 0) x[k][t] = ldg4(reinterpret_cast<const float4*>(p.vin + (int64_t)v[k][t] * C + c));
                             }
+#pragma unroll
+                        for (int k = 0; k < 2; ++k)
+#pragma unroll
+                            for (int t = 0; t < 3; ++t)
+                                if (v[k][t] >= 0) fma4(a[k0 + k], fl[t], x[k][t]);
+                    }
+                } else if (MODE == 1) {
+                    // ascending CSR entries, then one scaling: the arithmetic of the stand-alone gather kernel
+                    const float* base = p.wx + c;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+#pragma unroll
+                        for (int e0 = 0; e0 < 8; e0 += 4) {
+                            if (e0 >= most[k]) break;
+                            float4 x[4];
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const int f = __shfl_sync(0xffffffffu, id[k], (lane & 24) + e0 + e);
+                                if (in && e0 + e < n[k]) x[e] = ldg4(reinterpret_cast<const float4*>(base + (int64_t)f * C));
+                            }
+#pragma unroll
+                            for (int e = 0; e < 4; ++e)
+                                if (in && e0 + e < n[k]) add4(a[k], x[e]);
                         }
-                    } else if (MODE == 2) {
-                        if (valid) {
-                            const float4* x = reinterpret_cast<const float4*>(p.rows + row * C + c);
-                            a0 = ldg4(x); a1 = ldg4(x + 1);
-                            if (p.mask) {
-                                const float4* mk = reinterpret_cast<const float4*>(p.mask + row * C + c);
-                                const float4 m0 = ldg4(mk), m1 = ldg4(mk + 1);
-                                if (p.bn_mean) {
-                                    auto through = [&](float4& a, const float4& x, int o) {
-                                        const float4 mu = ldg4(reinterpret_cast<const float4*>(p.bn_mean + c) + o);
-                                        const float4 sc = ldg4(reinterpret_cast<const float4*>(p.bn_scale + c) + o);
-                                        const float4 k1 = ldg4(reinterpret_cast<const float4*>(p.bn_k1 + c) + o);
-                                        const float4 k2 = ldg4(reinterpret_cast<const float4*>(p.bn_k2 + c) + o);
-                                        a.x = fmaf(sc.x, a.x, fmaf(k2.x, x.x - mu.x, k1.x));
-                                        a.y = fmaf(sc.y, a.y, fmaf(k2.y, x.y - mu.y, k1.y));
-                                        a.z = fmaf(sc.z, a.z, fmaf(k2.z, x.z - mu.z, k1.z));
-                                        a.w = fmaf(sc.w, a.w, fmaf(k2.w, x.w - mu.w, k1.w));
-                                    };
-                                    through(a0, m0, 0);
-                                    through(a1, m1, 1);
-                                }
-                                if (p.relu_mask) {
-                                a0 = make_float4(m0.x > 0.f ? a0.x : 0.f, m0.y > 0.f ? a0.y : 0.f, m0.z > 0.f ? a0.z : 0.f,
-                                                 m0.w > 0.f ? a0.w : 0.f);
-                                a1 = make_float4(m1.x > 0.f ? a1.x : 0.f, m1.y > 0.f ? a1.y : 0.f, m1.z > 0.f ? a1.z : 0.f,
-                                                 m1.w > 0.f ? a1.w : 0.f);
-                                }
-                            }
-                            if (p.masked_out) {
-                                float4* mo = reinterpret_cast<float4*>(p.masked_out + row * C + c);
-                                mo[0] = a0; mo[1] = a1;
-                            }
+                        if (in)
+                            for (int e = 8; e < n[k]; ++e)
+                                add4(a[k], ldg4(reinterpret_cast<const float4*>(base + (int64_t)(__ldg(p.entries + beg[k] + e) >> 2) * C)));
+                        const float inv_n = __shfl_sync(0xffffffffu, cur.inv_n, 4 * k + rg);
+                        if (n[k] > 0) a[k] = scale4(a[k], inv_n);
+                    }
+                } else {
+                    float4 mk[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        mk[k] = zero4();
+                        if (!in || row0 + 4 * k >= p.Nrows) continue;
+                        a[k] = ldg4(reinterpret_cast<const float4*>(p.rows + (row0 + 4 * k) * C + c));
+                        if (p.mask) mk[k] = ldg4(reinterpret_cast<const float4*>(p.mask + (row0 + 4 * k) * C + c));
+                    }
+                    if (p.bn_mean && in) {
+                        const float4 mu = ldg4(reinterpret_cast<const float4*>(p.bn_mean + c)), sc = ldg4(reinterpret_cast<const float4*>(p.bn_scale + c));
+                        const float4 k1 = ldg4(reinterpret_cast<const float4*>(p.bn_k1 + c)), k2 = ldg4(reinterpret_cast<const float4*>(p.bn_k2 + c));
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            a[k].x = fmaf(sc.x, a[k].x, fmaf(k2.x, mk[k].x - mu.x, k1.x));
+                            a[k].y = fmaf(sc.y, a[k].y, fmaf(k2.y, mk[k].y - mu.y, k1.y));
+                            a[k].z = fmaf(sc.z, a[k].z, fmaf(k2.z, mk[k].z - mu.z, k1.z));
+                            a[k].w = fmaf(sc.w, a[k].w, fmaf(k2.w, mk[k].w - mu.w, k1.w));
                         }
+                    }
+                    if (p.mask && p.relu_mask) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            a[k] = make_float4(mk[k].x > 0.f ? a[k].x : 0.f, mk[k].y > 0.f ? a[k].y : 0.f, mk[k].z > 0.f ? a[k].z : 0.f,
+                                               mk[k].w > 0.f ? a[k].w : 0.f);
+                    }
+                }
+                float* const side = MODE == 2 ? p.masked_out : p.feat_out;
+                if (side && in) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (row0 + 4 * k < p.Nrows) *reinterpret_cast<float4*>(side + (row0 + 4 * k) * C + c) = a[k];
+                }
+                if (!warp_wait(&empty[st_i], st_ph ^ 1u, abort_flag, lane)) { tile = ntiles; break; }
+                const uint32_t st = stages32 + (uint32_t)st_i * (uint32_t)sbytes + (uint32_t)(j & 1) * 8u;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const uint32_t at = st + swz64_offset((uint32_t)(m0 + 4 * k), (uint32_t)(j >> 1));
+                    uint32_t h0, h1, l0, l1;
+                    if (NSPLIT == 1) {
+                        h0 = pack_bf16x2(a[k].x, a[k].y); h1 = pack_bf16x2(a[k].z, a[k].w);
                     } else {
-                        // ascending CSR entries, then one scaling: the arithmetic of the stand-alone gather kernel
-                        for (int e = beg; e < end; ++e) {
-                            const int64_t f = __ldg(p.entries + e) >> 2;
-                            const float4* x = reinterpret_cast<const float4*>(p.wx + f * C + c);
-                            add4(a0, ldg4(x));
-                            add4(a1, ldg4(x + 1));
-                        }
-                        if (end > beg) { a0 = scale4(a0, inv_n); a1 = scale4(a1, inv_n); }
+                        split_bf16x2(a[k].x, a[k].y, h0, l0); split_bf16x2(a[k].z, a[k].w, h1, l1);
+                        sts_u2(at + ROW_TILE_BYTES, l0, l1);
                     }
-                    if (MODE != 2 && p.feat_out && valid) {
-                        float4* fo = reinterpret_cast<float4*>(p.feat_out + row * C + c);
-                        fo[0] = a0; fo[1] = a1;
-                    }
+                    sts_u2(at, h0, h1);
                 }
-                if (!publish(a0, a1, b16)) { alive = false; break; }
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full[st_i]);
+                if (++st_i == S) { st_i = 0; st_ph ^= 1u; }
             }
-            if (!alive) break;
-            // ---- epilogue: accumulator rows = output channels, columns = rows of the tile
-            int ok = 1;
-            if (lane == 0) ok = mbar_wait(acc_full, tcount & 1u, abort_flag) ? 1 : 0;
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            if (!ok) { alive = false; break; }
+        }
+    } else if (warp < W_WARP) {
+        // ========== epilogue: accumulator rows = output channels, columns = rows of the tile ==========
+        const int q = warp & 3;
+        const int co = q * 32 + lane;
+        const float bv = (p.bias && co < Cout) ? __ldg(p.bias + co) : 0.f;
+        float ev_m = 0.f, ev_s = 1.f, ev_b = 0.f;
+        if (p.ev_var && co < Cout) {
+            ev_m = __ldg(p.ev_mean + co);
+            ev_s = 1.f / sqrtf(__ldg(p.ev_var + co) + p.ev_eps);
+            if (p.ev_gamma) ev_s *= __ldg(p.ev_gamma + co);
+            if (p.ev_beta) ev_b = __ldg(p.ev_beta + co);
+        }
+        uint32_t tcount = 0;
+        for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++tcount) {
+            const int64_t r0 = tile * TILE_R;
+            const uint32_t b = tcount & 1u;
+            if (!warp_wait(&acc_full[b], (tcount >> 1) & 1u, abort_flag, lane)) break;
             tc_fence_after();
-            const int q = warp & 3, g = warp >> 2;
-            const int co = q * 32 + lane;
-            const float bv = (p.bias && co < Cout) ? __ldg(p.bias + co) : 0.f;
-            float ev_m = 0.f, ev_s = 1.f, ev_b = 0.f;
-            if (p.ev_var && co < Cout) {
-                ev_m = __ldg(p.ev_mean + co);
-                ev_s = 1.f / sqrtf(__ldg(p.ev_var + co) + p.ev_eps);
-                if (p.ev_gamma) ev_s *= __ldg(p.ev_gamma + co);
-                if (p.ev_beta) ev_b = __ldg(p.ev_beta + co);
-            }
+            if (q * 32 < Cout) {
 #pragma unroll 1
-            for (int half = 0; half < 2; ++half) {
-                const int col = g * 64 + half * 32;
-                uint32_t r[32];
-                tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)col, r);
-                tmem_ld_wait();
-                if (co < Cout) {
-                    const int64_t left = p.Nrows - (r0 + col);
-                    const int cnt = left < 32 ? (int)left : 32;              // rows of this half (<= 0: none)
-                    float* o = p.out + (r0 + col) * p.out_stride + co;
+                for (int col = 0; col < TILE_R; col += 32) {
+                    uint32_t r[32];
+                    tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + b * TILE_R + (uint32_t)col, r);
+                    tmem_ld_wait();
+                    if (co < Cout) {
+                        const int64_t left = p.Nrows - (r0 + col);
+                        const int cnt = left < 32 ? (int)left : 32;              // rows of this group (<= 0: none)
+                        float* o = p.out + (r0 + col) * p.out_stride + co;
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        float v = __uint_as_float(r[j]) + bv;
-                        if (p.relu) v = fmaxf(v, 0.f);
-                        v = fmaf(v - ev_m, ev_s, ev_b);
-                        if (j < cnt) __stcs(o + (int64_t)j * p.out_stride, v);
+                        for (int j = 0; j < 32; ++j) {
+                            float v = __uint_as_float(r[j]) + bv;
+                            if (p.relu) v = fmaxf(v, 0.f);
+                            v = fmaf(v - ev_m, ev_s, ev_b);
+                            if (j < cnt) __stcs(o + (int64_t)j * p.out_stride, v);
+                        }
                     }
                 }
             }
             tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_free[b]);
         }
-    } else if (warp == PWARPS) {
+    } else if (warp == W_WARP) {
         // ================================ weight loader (TMA engine) ==========================
         if (elect_one()) {
             const uint32_t bytes = (uint32_t)(NSPLIT * W_TILE_BYTES);
@@ -325,9 +357,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) rows_pointwise_tc_kernel(Params p
             constexpr uint32_t idesc = instr_desc(FMT_BF16, UM, TILE_R);
             const uint64_t dbase = smem_desc_kmajor(smem_u32(stages), 64, SWZ_64B);
             int s = 0;
-            uint32_t ph = 0;
+            uint32_t ph = 0, tcount = 0;
             bool alive = true;
-            for (int64_t tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x) {
+            for (int64_t tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x, ++tcount) {
+                const uint32_t acc = tmem_base + (tcount & 1u) * TILE_R;
+                if (!mbar_wait(&acc_free[tcount & 1u], ((tcount >> 1) & 1u) ^ 1u, abort_flag)) break;
+                tc_fence_after();
                 for (int kb = 0; kb < p.nkb; ++kb) {
                     if (!mbar_wait(&full[s], ph, abort_flag)) { alive = false; break; }
                     tc_fence_after();
@@ -338,19 +373,19 @@ __global__ void __launch_bounds__(NTHREADS, 1) rows_pointwise_tc_kernel(Params p
                         const uint64_t adv = (uint64_t)(ks * 2);
                         const uint32_t first = (kb | ks) != 0;
                         if (NSPLIT == 1) {
-                            mma_f16(tmem_base, w_hi + adv, rows_hi + adv, idesc, first);
+                            mma_f16(acc, w_hi + adv, rows_hi + adv, idesc, first);
                         } else {
                             const uint64_t rows_lo = rows_hi + (uint64_t)(ROW_TILE_BYTES >> 4);
                             const uint64_t w_lo = w_hi + (uint64_t)(W_TILE_BYTES >> 4);
-                            mma_f16(tmem_base, w_lo + adv, rows_hi + adv, idesc, first);
-                            mma_f16(tmem_base, w_hi + adv, rows_lo + adv, idesc, 1u);
-                            mma_f16(tmem_base, w_hi + adv, rows_hi + adv, idesc, 1u);
+                            mma_f16(acc, w_lo + adv, rows_hi + adv, idesc, first);
+                            mma_f16(acc, w_hi + adv, rows_lo + adv, idesc, 1u);
+                            mma_f16(acc, w_hi + adv, rows_hi + adv, idesc, 1u);
                         }
                     }
                     tc_commit(&empty[s]);
                     if (++s == S) { s = 0; ph ^= 1u; }
                 }
-                if (alive) tc_commit(acc_full);
+                if (alive) tc_commit(&acc_full[tcount & 1u]);
             }
         }
     }
@@ -358,7 +393,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) rows_pointwise_tc_kernel(Params p
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == PWARPS) tmem_dealloc(tmem_base, TILE_R);
+    if (warp == W_WARP) tmem_dealloc(tmem_base, 2 * TILE_R);
     if (tid == 0 && abort_flag[0] && p.async_err) {
         *p.async_err = 4;
         __threadfence_system();
