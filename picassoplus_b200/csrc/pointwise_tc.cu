@@ -8,12 +8,15 @@
 //   vertex2facet:  feat[f, c] = sum_{k<3} filter[k, c] * input[face[f, k], c]        (r = 1)
 //   facet2vertex:  feat[v, c] = (sum over the CSR entries (f, corner) of v of wx[f, c]) / nfCount[v]
 //                  (wx = the per-face products of the facet2vertex forward pass)
-// Per CTA (persistent) and per tile of 256 rows, the same roles as the facet2facet forward kernel:
-// 16 producer warps gather and combine the operand rows (thread = row x 8 channels) and write them
-// as 64-byte swizzled K-major bf16 rows (one stage = 32 channels); one thread streams the
-// pre-swizzled weight blocks with 1-D bulk copies; one thread issues tcgen05.mma (M = 128 output
-// channels, N = 256 rows, K = 16 per instruction, fp32 accumulation in TMEM); the producer warps
-// drain the accumulator, add the bias, apply the activation and store out[row, co] coalesced.
+// Per CTA (persistent) and per tile of 256 rows:
+//   * 16 producer warps gather and combine the operand rows (whole 128-byte lines per load, four rows per warp at a time) and write
+//     them as 64-byte swizzled K-major bf16 rows (one stage = 32 channels);
+//   * one thread streams the pre-swizzled weight blocks with 1-D bulk copies, one issues tcgen05.mma (M = 128 output channels,
+//     N = 256 rows, K = 16 per instruction, fp32 accumulation in TMEM, two accumulators);
+//   * 8 epilogue warps drain the other accumulator meanwhile, add the bias, apply the activation and store out[row, co] coalesced.
+// What bounds it: memory, and the epilogue's instructions per value.  978 000 rows 64 -> 64 in fp32 mode: 240 us with the
+// producers doing the epilogue, 235 with four warps of its own, 107 with eight and no per-value predicates (no epilogue at
+// all: 75); gradient rows 128 -> 128 with mask and masked copy 397 -> 330 us (5.9 TB/s).
 // Precision modes: bf16 operands (one product per term) or bf16 hi + lo operands (three products,
 // about 1e-5 relative: the fp32 mode).  All waits are bounded (tc_ptx.cuh).
 #include "common.cuh"
@@ -34,12 +37,13 @@ using namespace ptx;
 constexpr int TILE_R = 256;                 // rows per tile (UMMA N)
 constexpr int UM = 128;                     // output channels per launch (UMMA M), zero-padded
 constexpr int PWARPS = 16;
-constexpr int EWARPS = 4;                   // epilogue: one warp per TMEM quadrant
-constexpr int W_WARP = PWARPS + EWARPS, MMA_WARP = W_WARP + 1;
-constexpr int NTHREADS = (MMA_WARP + 1) * 32;
+// epilogue warps: two per TMEM quadrant; one for facet2vertex rows, whose gathers need the registers
+template <int MODE> constexpr int EWARPS_OF = MODE == 1 ? 4 : 8;
+template <int MODE> constexpr int NTHREADS = (PWARPS + EWARPS_OF<MODE> + 2) * 32;
 constexpr int ROW_TILE_BYTES = TILE_R * 64;
 constexpr int W_TILE_BYTES = UM * 64;
 constexpr int KB = 32;                      // channels per stage (one 64-byte bf16 operand row)
+constexpr int IDS = 8;                      // entries of a facet2vertex row that are kept in registers
 
 // weight image: Wimg[kb][split][co 0..127][32 bf16, 64B-swizzled], element (co, k) = Wd[kb*32 + k][co0 + co]
 // at wd[k * sk + n * sn]: (sk, sn) = (Cout, 1) for the layer's weights as they are, (1, Cin) for their transpose
@@ -110,7 +114,8 @@ __host__ __device__ inline size_t stage_bytes(int nsplit) { return (size_t)nspli
 
 // MODE 0: vertex2facet rows, MODE 1: facet2vertex rows, MODE 2: rows of a gradient masked by an activation
 template <int NSPLIT, int MODE>
-__global__ void __launch_bounds__(NTHREADS, 1) rows_pointwise_tc_kernel(Params p) {
+__global__ void __launch_bounds__(NTHREADS<MODE>, 1) rows_pointwise_tc_kernel(Params p) {
+    constexpr int EWARPS = EWARPS_OF<MODE>, W_WARP = PWARPS + EWARPS;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -144,16 +149,19 @@ __global__ void __launch_bounds__(NTHREADS, 1) rows_pointwise_tc_kernel(Params p
         // A warp has 16 rows of the tile, four at a time: lane = row rg of the four, channels 4j..4j+3 of the stage's 32.  A warp's
         // load then reads whole 128-byte lines (two lanes of 32 bytes per row met 16 lines per load, and the L1 was what the
         // kernel waited for).
-        const int rg = lane >> 3, j = lane & 7, m0 = warp * 16 + rg;
+        // facet2vertex rows keep the two lanes: their gathers come from L2, a line is wanted by three vertices, and what the small
+        // L1 can hold meanwhile is 64 bytes of every row of the tile, not 128 (128 channels: 499 against 574 us).
+        const int rg = lane >> 3, j = lane & 7, m0 = MODE == 1 ? warp * 16 + (lane >> 1) : warp * 16 + rg;
         const uint32_t stages32 = smem_u32(stages);
         int st_i = 0;
         uint32_t st_ph = 0;
 
-        // what the warp's rows are made of, a row per lane; the next tile's is loaded while this one's rows are
+        // what the rows are made of: vertex2facet a row of the warp per lane, facet2vertex the thread's own row; the next tile's is
+        // loaded while this one's rows are
         struct Source { int v[3]; int beg, n; float inv_n; };
         auto source = [&](int64_t tile, Source& s) {
-            const int64_t row = tile * TILE_R + warp * 16 + lane;
-            const bool valid = lane < 16 && row < p.Nrows;
+            const int64_t row = tile * TILE_R + (MODE == 1 ? m0 : warp * 16 + lane);
+            const bool valid = (MODE == 1 || lane < 16) && row < p.Nrows;
             if (MODE == 0) {
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
@@ -169,18 +177,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) rows_pointwise_tc_kernel(Params p
         Source cur, nxt;
         source(blockIdx.x, nxt);
         for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-            const int64_t row0 = tile * TILE_R + m0;             // rows row0 + 4k
+            const int64_t row0 = tile * TILE_R + m0;             // rows row0 + 4k; facet2vertex: row0
             cur = nxt;
             source(tile + gridDim.x, nxt);
-            int id[4], beg[4], n[4], most[4];
+            int id[MODE == 1 ? IDS : 1];
             if (MODE == 1) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    beg[k] = __shfl_sync(0xffffffffu, cur.beg, 4 * k + rg);
-                    n[k] = __shfl_sync(0xffffffffu, cur.n, 4 * k + rg);
-                    most[k] = __reduce_max_sync(0xffffffffu, n[k]);
-                    id[k] = j < n[k] ? __ldg(p.entries + beg[k] + j) >> 2 : 0;
-                }
+                for (int e = 0; e < IDS; ++e) id[e] = e < cur.n ? __ldg(p.entries + cur.beg + e) >> 2 : 0;
             }
             for (int kb = 0; kb < p.nkb; ++kb) {
                 float4 a[4];
@@ -212,28 +215,33 @@ __global__ void __launch_bounds__(NTHREADS, 1) rows_pointwise_tc_kernel(Params p
                                 if (v[k][t] >= 0) fma4(a[k0 + k], fl[t], x[k][t]);
                     }
                 } else if (MODE == 1) {
-                    // ascending CSR entries, then one scaling: the arithmetic of the stand-alone gather kernel
-                    const float* base = p.wx + c;
+                    // ascending CSR entries, then one scaling: the arithmetic of the stand-alone gather kernel.  The rows of four
+                    // entries are on their way at a time; a[2i], a[2i + 1] = channels kb*32 + 16i + 8h ..+7
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
+                    for (int i = 0; i < 2; ++i) {
+                        const int ci = kb * KB + 16 * i + 8 * (lane & 1);
+                        if (ci >= C) continue;
+                        const float* base = p.wx + ci;
 #pragma unroll
-                        for (int e0 = 0; e0 < 8; e0 += 4) {
-                            if (e0 >= most[k]) break;
-                            float4 x[4];
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const int f = __shfl_sync(0xffffffffu, id[k], (lane & 24) + e0 + e);
-                                if (in && e0 + e < n[k]) x[e] = ldg4(reinterpret_cast<const float4*>(base + (int64_t)f * C));
-                            }
+                        for (int e0 = 0; e0 < IDS; e0 += 4) {
+                            if (e0 >= cur.n) break;
+                            float4 x[4][2];
 #pragma unroll
                             for (int e = 0; e < 4; ++e)
-                                if (in && e0 + e < n[k]) add4(a[k], x[e]);
+                                if (e0 + e < cur.n) {
+                                    const float4* src = reinterpret_cast<const float4*>(base + (int64_t)id[e0 + e] * C);
+                                    x[e][0] = ldg4(src); x[e][1] = ldg4(src + 1);
+                                }
+#pragma unroll
+                            for (int e = 0; e < 4; ++e)
+                                if (e0 + e < cur.n) { add4(a[2 * i], x[e][0]); add4(a[2 * i + 1], x[e][1]); }
                         }
-                        if (in)
-                            for (int e = 8; e < n[k]; ++e)
-                                add4(a[k], ldg4(reinterpret_cast<const float4*>(base + (int64_t)(__ldg(p.entries + beg[k] + e) >> 2) * C)));
-                        const float inv_n = __shfl_sync(0xffffffffu, cur.inv_n, 4 * k + rg);
-                        if (n[k] > 0) a[k] = scale4(a[k], inv_n);
+                        for (int e = IDS; e < cur.n; ++e) {
+                            const float4* src = reinterpret_cast<const float4*>(base + (int64_t)(__ldg(p.entries + cur.beg + e) >> 2) * C);
+                            add4(a[2 * i], ldg4(src));
+                            add4(a[2 * i + 1], ldg4(src + 1));
+                        }
+                        if (cur.n > 0) { a[2 * i] = scale4(a[2 * i], cur.inv_n); a[2 * i + 1] = scale4(a[2 * i + 1], cur.inv_n); }
                     }
                 } else {
                     float4 mk[4];
@@ -263,16 +271,23 @@ __global__ void __launch_bounds__(NTHREADS, 1) rows_pointwise_tc_kernel(Params p
                     }
                 }
                 float* const side = MODE == 2 ? p.masked_out : p.feat_out;
-                if (side && in) {
+                if (MODE == 1) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const int ci = kb * KB + 16 * (k >> 1) + 8 * (lane & 1) + 4 * (k & 1);
+                        if (side && ci < C && row0 < p.Nrows) *reinterpret_cast<float4*>(side + row0 * C + ci) = a[k];
+                    }
+                } else if (side && in) {
 #pragma unroll
                     for (int k = 0; k < 4; ++k)
                         if (row0 + 4 * k < p.Nrows) *reinterpret_cast<float4*>(side + (row0 + 4 * k) * C + c) = a[k];
                 }
                 if (!warp_wait(&empty[st_i], st_ph ^ 1u, abort_flag, lane)) { tile = ntiles; break; }
-                const uint32_t st = stages32 + (uint32_t)st_i * (uint32_t)sbytes + (uint32_t)(j & 1) * 8u;
+                const uint32_t st = stages32 + (uint32_t)st_i * (uint32_t)sbytes;
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    const uint32_t at = st + swz64_offset((uint32_t)(m0 + 4 * k), (uint32_t)(j >> 1));
+                    const uint32_t at = MODE == 1 ? st + swz64_offset((uint32_t)m0, (uint32_t)(2 * (k >> 1) + (lane & 1))) + (uint32_t)(k & 1) * 8u
+                                                  : st + swz64_offset((uint32_t)(m0 + 4 * k), (uint32_t)(j >> 1)) + (uint32_t)(j & 1) * 8u;
                     uint32_t h0, h1, l0, l1;
                     if (NSPLIT == 1) {
                         h0 = pack_bf16x2(a[k].x, a[k].y); h1 = pack_bf16x2(a[k].z, a[k].w);
@@ -308,21 +323,25 @@ __global__ void __launch_bounds__(NTHREADS, 1) rows_pointwise_tc_kernel(Params p
             tc_fence_after();
             if (q * 32 < Cout) {
 #pragma unroll 1
-                for (int col = 0; col < TILE_R; col += 32) {
+                for (int col = ((warp - PWARPS) >> 2) * 32; col < TILE_R; col += EWARPS / 4 * 32) {
                     uint32_t r[32];
                     tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + b * TILE_R + (uint32_t)col, r);
                     tmem_ld_wait();
-                    if (co < Cout) {
-                        const int64_t left = p.Nrows - (r0 + col);
-                        const int cnt = left < 32 ? (int)left : 32;              // rows of this group (<= 0: none)
-                        float* o = p.out + (r0 + col) * p.out_stride + co;
+                    const int64_t left = p.Nrows - (r0 + col);               // rows of this group that exist
+                    float* const o = p.out + (r0 + col) * p.out_stride + co;
+                    if (co >= Cout || left <= 0) continue;
+                    auto value = [&](int j) {
+                        float v = __uint_as_float(r[j]) + bv;
+                        return p.relu ? fmaxf(v, 0.f) : v;
+                    };
+                    // a warp's instructions per value are what an epilogue takes its time for: the whole group without predicates
+                    if (left >= 32 && !p.ev_var) {
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            float v = __uint_as_float(r[j]) + bv;
-                            if (p.relu) v = fmaxf(v, 0.f);
-                            v = fmaf(v - ev_m, ev_s, ev_b);
-                            if (j < cnt) __stcs(o + (int64_t)j * p.out_stride, v);
-                        }
+                        for (int j = 0; j < 32; ++j) o[(uint32_t)(j * p.out_stride)] = value(j);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j)
+                            if (j < left) o[(uint32_t)(j * p.out_stride)] = fmaf(value(j) - ev_m, ev_s, ev_b);
                     }
                 }
             }
@@ -426,6 +445,18 @@ static int set_extra(Params& p, const pb200_pointwise_extra* x, const char* wher
 }
 
 template <int MODE>
+static int launch(const char* label, const Params& p, const Plan& pl, int grid, cudaStream_t stream) {
+    if (pl.nsplit == 2) {
+        PB_CUDA(cudaFuncSetAttribute(rows_pointwise_tc_kernel<2, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
+        PB_LAUNCH(label, (rows_pointwise_tc_kernel<2, MODE>), grid, NTHREADS<MODE>, pl.smem, stream, p);
+    } else {
+        PB_CUDA(cudaFuncSetAttribute(rows_pointwise_tc_kernel<1, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
+        PB_LAUNCH(label, (rows_pointwise_tc_kernel<1, MODE>), grid, NTHREADS<MODE>, pl.smem, stream, p);
+    }
+    return PB200_OK;
+}
+
+template <int MODE>
 static int run(Params p, int Cout, const float* wd, const float* bias, float* out, int precision, void* ws,
                cudaStream_t stream, bool transposed = false) {
     int rc = tc::check_async_error("pointwise fusion");
@@ -446,14 +477,18 @@ static int run(Params p, int Cout, const float* wd, const float* bias, float* ou
         p.ev_mean = all.ev_var ? all.ev_mean + co0 : nullptr; p.ev_var = all.ev_var ? all.ev_var + co0 : nullptr;
         p.ev_gamma = all.ev_gamma ? all.ev_gamma + co0 : nullptr; p.ev_beta = all.ev_beta ? all.ev_beta + co0 : nullptr;
         const char* label = MODE == 0 ? "v2f_pointwise_tc" : (MODE == 1 ? "f2v_pointwise_tc" : "masked_rows_tc");
-        if (co0 > 0) { p.masked_out = nullptr; p.feat_out = nullptr; }      // by-products are written by the first chunk's launch
-        if (pl.nsplit == 2) {
-            PB_CUDA(cudaFuncSetAttribute(rows_pointwise_tc_kernel<2, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
-            PB_LAUNCH(label, (rows_pointwise_tc_kernel<2, MODE>), grid, NTHREADS, pl.smem, stream, p);
-        } else {
-            PB_CUDA(cudaFuncSetAttribute(rows_pointwise_tc_kernel<1, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
-            PB_LAUNCH(label, (rows_pointwise_tc_kernel<1, MODE>), grid, NTHREADS, pl.smem, stream, p);
+        if (co0 > 0 && MODE != 2 && p.feat_out) {
+            // the first chunk's launch has written the gathered rows: the others read them (978 000 faces, 256 output
+            // channels from 128: 99 us per chunk instead of 176)
+            p.rows = p.feat_out; p.mask = nullptr; p.feat_out = nullptr;
+            int rc2 = launch<2>(label, p, pl, grid, stream);
+            if (rc2) return rc2;
+            p.feat_out = all.feat_out;
+            continue;
         }
+        if (co0 > 0) p.masked_out = nullptr;                                // by-products are written by the first chunk's launch
+        rc = launch<MODE>(label, p, pl, grid, stream);
+        if (rc) return rc;
     }
     return PB200_OK;
 }
