@@ -1,6 +1,7 @@
 // facet2vertex: forward as a vertex-centred pull over the CSR (segmented sum in a fixed
 // order, no atomics); backward as a face-centred gather that yields the input gradient
 // and per-thread filter-gradient partials in one pass.
+#include <type_traits>
 #include "common.cuh"
 
 namespace pb {
@@ -284,62 +285,81 @@ f2v_bwd_tile_kernel(int64_t Nf, int CV, int K, const int32_t* __restrict__ face,
         if (ak[n] >= 0) partial[((int64_t)blockIdx.x * K + ak[n]) * CV + cg0 + ac[n]] = acc[n];
 }
 
-// The same two phases, register-blocked for whole 128-channel chunks (lane = float4 channel
-// group) and K <= 32, so that the shared-memory pipe is not the limit: every 16-byte shared
-// load of a warp is either 512 distinct bytes or one broadcast address.
-//   phase 1  warp w owns faces w, w+8, w+16, w+24 of the tile: a filter row read from shared
-//            memory is used for all four faces;
-//   phase 2  warp g owns the coefficients 4g..4g+3: a row of t read from shared memory feeds
-//            four accumulators.
-// The index chain of the gather (face -> vtMap -> nfCount) is resolved by 96 threads one hop
-// per tile for the block's next three tiles, so that phase 1 finds output vertex and 1/nfCount
-// of every corner in shared memory and issues its twelve gradOutput row loads at once.
+// The same two phases register-blocked, for K <= 32: a face's channels lie on LPF lanes (float4 each; LPF = 4, 8, 16, 32, chunks of
+// 32 behind that), a warp has 32 / LPF faces side by side and four such passes per tile.
+//   phase 1  a filter row read from shared memory is used for the four passes' faces;
+//   phase 2  a warp owns four coefficients and, while K leaves warps over, a share of the tile's faces: a row of t read from shared
+//            memory feeds four accumulators.
+// What bounds it: shared memory (70 % busy at 128 channels) and the three barriers of a tile; packed multiply-adds on coefficients
+// kept twice changed nothing.  A kernel without register blocking served all widths that are no multiple of 128 before:
+// 1 954 000 faces, 64 channels, K = 16 960 -> 606 us; 977 000 faces, 48 channels, K = 9 408 -> 286 us, 100 channels 817 -> 561.
+// The index chain of the gather (face -> vtMap -> nfCount) is resolved one hop per tile for the block's next three tiles, so that
+// phase 1 finds output vertex and 1/nfCount of every corner in shared memory and issues its twelve gradOutput row loads at once.
+template <int LPF> constexpr int F2VB_FACES = 32 * (32 / LPF);         // faces of a tile
+// floats of a coefficient row; a pad keeps the rows of faces side by side in a warp off one another's banks
+template <int LPF> __host__ __device__ constexpr int f2vb_pitch(int K) { return (K + 3) / 4 * 4 + (LPF < 32 ? 4 : 0); }
+template <int LPF>
+static size_t f2vb_smem(int K) {
+    return sizeof(float4) * ((size_t)(K + 3) / 4 * 4 * LPF + F2VB_FACES<LPF> * LPF) + sizeof(float) * 2 * F2VB_FACES<LPF> * f2vb_pitch<LPF>(K) +
+           2 * F2VB_FACES<LPF> * 3 * 8;
+}
+
+template <int LPF>
 __global__ void __launch_bounds__(256, 2)
 f2v_bwd_blocked_kernel(int64_t Nf, int CV, int K, const int32_t* __restrict__ face, const int32_t* __restrict__ vtMap,
                        const int32_t* __restrict__ nfCount, const float* __restrict__ coeff,
                        const float4* __restrict__ in, const float4* __restrict__ filt, const float4* __restrict__ gout,
                        float4* __restrict__ gin, float4* __restrict__ partial) {
     extern __shared__ float4 smem[];
-    const int KP = (K + 3) / 4 * 4;                            // coeff row pitch (floats), pad columns zero
-    const int KG = KP / 4;                                     // groups of 4 coefficients (<= 8)
-    float4* sfilt = smem;                                      // [KP][32], rows K..KP-1 zero
-    float4* st = smem + KP * 32;                               // [TF][32]   t = input * gt
-    float4* scoef0 = st + F2VB_TF * 32;                        // [2][TF][KG], double-buffered (asynchronous copies)
-    int* svo = reinterpret_cast<int*>(scoef0 + 2 * F2VB_TF * KG);   // [2][96] output vertex of (face, corner), -1 = none
-    float* srn = reinterpret_cast<float*>(svo + 2 * 96);       // [2][96] 1 / nfCount of that vertex
+    constexpr int FPW = 32 / LPF, TF = F2VB_FACES<LPF>, NE = TF * 3, NI = (NE + 255) / 256;
+    const int KG = (K + 3) / 4, CP = f2vb_pitch<LPF>(K);            // groups of 4 coefficients (<= 8)
+    float4* sfilt = smem;                                      // [4 KG][LPF], rows K.. zero
+    float4* st = smem + 4 * KG * LPF;                          // [TF][LPF]   t = input * gt
+    float* scoef0 = reinterpret_cast<float*>(st + TF * LPF);   // [2][TF][CP], double-buffered (asynchronous copies)
+    int* svo = reinterpret_cast<int*>(scoef0 + 2 * TF * CP);   // [2][NE] output vertex of (face, corner), -1 = none
+    float* srn = reinterpret_cast<float*>(svo + 2 * NE);       // [2][NE] 1 / nfCount of that vertex
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int cg = blockIdx.y * 32 + lane;                     // this lane's channel group
-    for (int i = threadIdx.x; i < KP * 32; i += blockDim.x) {
-        const int k = i >> 5;
-        sfilt[i] = k < K ? filt[k * CV + blockIdx.y * 32 + (i & 31)] : zero4();
+    const int l = lane % LPF, fs = lane / LPF;                 // channel group, face among the warp's
+    const int cg = blockIdx.y * LPF + l;
+    const bool on = cg < CV;
+    for (int i = threadIdx.x; i < 4 * KG * LPF; i += blockDim.x) {
+        const int k = i / LPF, c = blockIdx.y * LPF + i % LPF;
+        sfilt[i] = k < K && c < CV ? filt[k * CV + c] : zero4();
     }
-    for (int i = threadIdx.x; i < 2 * F2VB_TF * KG; i += blockDim.x) scoef0[i] = zero4();
-    float4 acc[4] = {zero4(), zero4(), zero4(), zero4()};     // coefficients 4*warp .. 4*warp+3
-    const int64_t ntiles = (Nf + F2VB_TF - 1) / F2VB_TF;
-    // index pipeline of thread e < 96 (entry e = 3*face + corner of a tile): vertex id of the
-    // tile three steps ahead, output vertex two steps ahead, 1/nfCount one step ahead
-    const bool ix = threadIdx.x < 96;
-    auto hop_face = [&](int64_t tile) -> int {
-        const int64_t e = tile * (F2VB_TF * 3) + threadIdx.x;
-        return (ix && tile < ntiles && e < Nf * 3) ? __ldg(face + e) : -1;
+    for (int i = threadIdx.x; i < 2 * TF * CP; i += blockDim.x) scoef0[i] = 0.f;
+    // phase 2: coefficients 4g..4g+3, faces fs + FPW * (slice + slices * i)
+    const int slices = 8 / KG, g2 = warp % KG, slice = warp / KG;
+    float4 acc[4] = {zero4(), zero4(), zero4(), zero4()};
+    const int64_t ntiles = (Nf + TF - 1) / TF;
+    // index pipeline (entry e = 3*face + corner of a tile): vertex id of the tile three steps ahead, output vertex two steps
+    // ahead, 1/nfCount one step ahead
+    auto hop_face = [&](int64_t tile, int i) -> int {
+        const int e = threadIdx.x + 256 * i;
+        const int64_t at = tile * NE + e;
+        return (e < NE && tile < ntiles && at < Nf * 3) ? __ldg(face + at) : -1;
     };
     auto hop_vo = [&](int vi) -> int { return vi < 0 ? -1 : (vtMap ? __ldg(vtMap + vi) : vi); };
     auto hop_rn = [&](int vo) -> float { return vo < 0 ? 0.f : __frcp_rn((float)__ldg(nfCount + vo)); };
+    auto park = [&](int b, int i, int vo, float rn) {
+        const int e = threadIdx.x + 256 * i;
+        if (e < NE) { svo[b * NE + e] = vo; srn[b * NE + e] = rn; }
+    };
     const int64_t tstep = gridDim.x;
-    int vo1 = hop_vo(hop_face(blockIdx.x));                                   // first tile: resolved up front
-    float rn1 = hop_rn(vo1);
-    if (ix) { svo[threadIdx.x] = vo1; srn[threadIdx.x] = rn1; }
-    vo1 = hop_vo(hop_face(blockIdx.x + tstep));                               // second tile
-    int vi2 = hop_face(blockIdx.x + 2 * tstep);                               // third tile
-    auto fetch_coef = [&](int64_t tile, int b) {               // the pad columns stay zero
-        if (tile < ntiles) {
-            const int64_t f0 = tile * F2VB_TF;
-            const int nf_tile = Nf - f0 < F2VB_TF ? (int)(Nf - f0) : F2VB_TF;
-            float* sc = reinterpret_cast<float*>(scoef0 + b * F2VB_TF * KG);
-            for (int i = threadIdx.x; i < nf_tile * K; i += blockDim.x) {
-                const int fl = i / K;
-                cp_async4(sc + fl * KP + (i - fl * K), coeff + f0 * K + i);
-            }
+    int vo1[NI], vi2[NI];
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+        const int vo = hop_vo(hop_face(blockIdx.x, i));        // first tile: resolved up front
+        park(0, i, vo, hop_rn(vo));
+        vo1[i] = hop_vo(hop_face(blockIdx.x + tstep, i));      // second tile
+        vi2[i] = hop_face(blockIdx.x + 2 * tstep, i);          // third tile
+    }
+    auto fetch_coef = [&](int64_t tile, int b) {               // a lane per coefficient; the pad columns stay zero
+        if (tile < ntiles && lane < K) {
+            const int64_t f0 = tile * TF;
+            const int nf_tile = Nf - f0 < TF ? (int)(Nf - f0) : TF;
+            const float* src = coeff + f0 * K + lane;
+            float* sc = scoef0 + b * TF * CP + lane;
+            for (int fl = warp; fl < nf_tile; fl += 8) cp_async4(sc + fl * CP, src + fl * K);
         }
         cp_async_commit();
     };
@@ -347,84 +367,92 @@ f2v_bwd_blocked_kernel(int64_t Nf, int CV, int K, const int32_t* __restrict__ fa
     fetch_coef(blockIdx.x, 0);
     int buf = 0;
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += tstep, buf ^= 1) {
-        const int64_t f0 = tile * F2VB_TF;
-        const int nf_tile = Nf - f0 < F2VB_TF ? (int)(Nf - f0) : F2VB_TF;
+        const int64_t f0 = tile * TF;
+        const int nf_tile = Nf - f0 < TF ? (int)(Nf - f0) : TF;
         // one hop for each of the next three tiles (results are used in the next iteration)
-        const float rn_next = hop_rn(vo1);
-        const int vo_next = hop_vo(vi2);
-        const int vi_next = hop_face(tile + 3 * tstep);
+        float rn_next[NI];
+        int vo_next[NI], vi_next[NI];
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            rn_next[i] = hop_rn(vo1[i]);
+            vo_next[i] = hop_vo(vi2[i]);
+            vi_next[i] = hop_face(tile + 3 * tstep, i);
+        }
         __syncthreads();                                       // previous tile fully consumed
         fetch_coef(tile + tstep, buf ^ 1);                     // the next tile's coefficient rows, asynchronously
         cp_async_wait<1>();                                    // this tile's rows have landed (own copies) ...
         __syncthreads();                                       // ... and everybody else's
-        const float4* scoef = scoef0 + buf * F2VB_TF * KG;
-        // ---- phase 1: faces warp, warp+8, warp+16, warp+24
-        // all sixteen row loads of the warp's four faces are issued first; the filter sums below need
-        // only the coefficients and run while the rows are on their way
-        float4 gt[4], x[4], w[4], gr[4][3];
+        const float* scoef = scoef0 + buf * TF * CP;
+        // ---- phase 1: faces (warp + 8 i) * FPW + fs
+        // all sixteen row loads of the thread are issued first; the filter sums below need only the coefficients and run
+        // while the rows are on their way
+        float4 x[4], w[4], gr[4][3];
         float rn[4][3];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int fl = warp + 8 * i;
+            const int fl = (warp + 8 * i) * FPW + fs;
             x[i] = zero4(); w[i] = zero4();
 #pragma unroll
             for (int j = 0; j < 3; ++j) { gr[i][j] = zero4(); rn[i][j] = 0.f; }
-            if (fl < nf_tile) {
+            if (on && fl < nf_tile) {
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
-                    const int vo = svo[buf * 96 + fl * 3 + j];
-                    rn[i][j] = srn[buf * 96 + fl * 3 + j];
+                    const int vo = svo[buf * NE + fl * 3 + j];
+                    rn[i][j] = srn[buf * NE + fl * 3 + j];
                     if (vo >= 0) gr[i][j] = ldg4(gout + (int64_t)vo * CV + cg);
                 }
                 x[i] = ldg4(in + (f0 + fl) * CV + cg);
             }
         }
-        for (int g = 0; g < KG; ++g) {
-            float4 cf[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) cf[i] = scoef[(warp + 8 * i) * KG + g];   // rows past the tile are stale or zero: unused
-            const float4 f0v = sfilt[(4 * g) * 32 + lane], f1v = sfilt[(4 * g + 1) * 32 + lane];
-            const float4 f2v = sfilt[(4 * g + 2) * 32 + lane], f3v = sfilt[(4 * g + 3) * 32 + lane];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                fma4s(w[i], cf[i].x, f0v); fma4s(w[i], cf[i].y, f1v); fma4s(w[i], cf[i].z, f2v); fma4s(w[i], cf[i].w, f3v);
-            }
+        for (int g = 0; g < KG; ++g) {                         // rows past the tile are stale or zero: unused
+                            const float4 fa = sfilt[4 * g * LPF + l], fb = sfilt[(4 * g + 1) * LPF + l];
+                            const float4 fc = sfilt[(4 * g + 2) * LPF + l], fd = sfilt[(4 * g + 3) * LPF + l];
+            #pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                const float4 cf = *reinterpret_cast<const float4*>(scoef + ((warp + 8 * i) * FPW + fs) * CP + 4 * g);
+                                fma4s(w[i], cf.x, fa); fma4s(w[i], cf.y, fb); fma4s(w[i], cf.z, fc); fma4s(w[i], cf.w, fd);
+                            }
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            gt[i] = zero4();
+            const int fl = (warp + 8 * i) * FPW + fs;
+            float4 gt = zero4();
 #pragma unroll
-            for (int j = 0; j < 3; ++j) fma4s(gt[i], rn[i][j], gr[i][j]);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int fl = warp + 8 * i;
-            if (fl < nf_tile) {
-                __stcs(gin + (f0 + fl) * CV + cg, mul4(gt[i], w[i]));
-                st[fl * 32 + lane] = mul4(x[i], gt[i]);
-            }
+            for (int j = 0; j < 3; ++j) fma4s(gt, rn[i][j], gr[i][j]);
+            if (on && fl < nf_tile) __stcs(gin + (f0 + fl) * CV + cg, mul4(gt, w[i]));
+            if (fl < nf_tile) st[fl * LPF + l] = mul4(x[i], gt);
         }
         __syncthreads();
         // the next tile's corners go to the other index buffer (its readers are behind the barrier above)
-        if (ix) { svo[(buf ^ 1) * 96 + threadIdx.x] = vo1; srn[(buf ^ 1) * 96 + threadIdx.x] = rn_next; }
-        vo1 = vo_next; vi2 = vi_next;
-        // ---- phase 2: coefficients 4*warp .. 4*warp+3, faces in order
-        if (warp < KG) {
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            park(buf ^ 1, i, vo1[i], rn_next[i]);
+            vo1[i] = vo_next[i]; vi2[i] = vi_next[i];
+        }
+        // ---- phase 2, faces in order
+        if (slice < slices) {
 #pragma unroll 4
-            for (int fl = 0; fl < nf_tile; ++fl) {
-                const float4 c = scoef[fl * KG + warp];
-                const float4 t = st[fl * 32 + lane];
+            for (int fl = slice * FPW + fs; fl < nf_tile; fl += slices * FPW) {
+                const float4 t = st[fl * LPF + l];
+                const float4 c = *reinterpret_cast<const float4*>(scoef + fl * CP + 4 * g2);
                 fma4s(acc[0], c.x, t); fma4s(acc[1], c.y, t); fma4s(acc[2], c.z, t); fma4s(acc[3], c.w, t);
             }
         }
     }
     cp_async_wait<0>();
-    if (warp < KG) {
+    __syncthreads();                                           // the sums of the slices, in slice order, and of the side-by-side faces
+    float4* sums = st;                                         // [slices * KG][4][32]: st has as many
+    if (slice < slices)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int k = 4 * warp + j;
-            if (k < K) partial[((int64_t)blockIdx.x * K + k) * CV + cg] = acc[j];
-        }
+        for (int j = 0; j < 4; ++j) sums[(warp * 4 + j) * 32 + lane] = acc[j];
+    __syncthreads();
+    for (int i = threadIdx.x; i < K * LPF; i += blockDim.x) {
+        const int k = i / LPF, c = i % LPF;
+        float4 s = zero4();
+        for (int v = 0; v < slices; ++v)
+#pragma unroll
+            for (int q = 0; q < FPW; ++q) add4(s, sums[((v * KG + k / 4) * 4 + k % 4) * 32 + q * LPF + c]);
+        if (blockIdx.y * LPF + c < CV) partial[((int64_t)blockIdx.x * K + k) * CV + blockIdx.y * LPF + c] = s;
     }
 }
 
@@ -604,17 +632,29 @@ int pb200_facet2vertex_backward(int64_t Nf, int64_t NvIn, int64_t NvOut, int C, 
     bool vec = p.vec && aligned16(gradOutput) && aligned16(input) && aligned16(filter) && aligned16(gradInput);
     if (vec) {
         int CV = C / 4;
+        // K <= 32: lanes of a face as many as hold its channels.  Behind 128 channels chunks of 128 on blockIdx.y
+        if (K <= 32) {
+            auto run = [&](auto lpf) {
+                constexpr int LPF = decltype(lpf)::value;
+                const int chunks = (int)ceil_div(CV, LPF);
+                int64_t gx = ceil_div(2 * (int64_t)sm_count(), chunks);              // two blocks per SM
+                if (gx > ceil_div(Nf, F2VB_FACES<LPF>)) gx = ceil_div(Nf, F2VB_FACES<LPF>);
+                if (gx > p.grid_x) gx = p.grid_x;
+                const size_t smemb = f2vb_smem<LPF>(K);
+                PB_CUDA(cudaFuncSetAttribute(f2v_bwd_blocked_kernel<LPF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemb));
+                PB_LAUNCH("f2v_bwd", f2v_bwd_blocked_kernel<LPF>, dim3((unsigned)gx, chunks), 256, smemb, stream, Nf, CV, K, face, vtMap,
+                          nfCount, coeff, (const float4*)input, (const float4*)filter, (const float4*)gradOutput, (float4*)gradInput,
+                          (float4*)partial);
+                return reduce_partials(partial, (int)gx, (int64_t)K * Cr, gradFilter, stream);
+            };
+            if (CV <= 4) return run(std::integral_constant<int, 4>{});
+            if (CV <= 8) return run(std::integral_constant<int, 8>{});
+            if (CV <= 16) return run(std::integral_constant<int, 16>{});
+            return run(std::integral_constant<int, 32>{});
+        }
         dim3 grid(p.grid_x, (unsigned)ceil_div(CV, 32));
         const int KP = (K + 3) / 4 * 4 + 4;
         size_t smem = sizeof(float4) * (32 * (size_t)K + F2VB_TF * 32) + sizeof(float) * F2VB_TF * KP;
-        if (CV % 32 == 0 && K <= 32) {
-            const int KPb = (K + 3) / 4 * 4;
-            const size_t smemb = sizeof(float4) * ((size_t)KPb * 32 + F2VB_TF * 32 + 2 * F2VB_TF * (KPb / 4)) + 2 * 96 * 8;
-            PB_LAUNCH("f2v_bwd", f2v_bwd_blocked_kernel, grid, 256, smemb, stream, Nf, CV, K, face, vtMap, nfCount, coeff,
-                      (const float4*)input, (const float4*)filter, (const float4*)gradOutput, (float4*)gradInput,
-                      (float4*)partial);
-            return reduce_partials(partial, p.grid_x, (int64_t)K * Cr, gradFilter, stream);
-        }
         const int cvc = CV < 32 ? CV : 32;
         const int nacc = (int)ceil_div((int64_t)K * cvc, 256);
 #define PB_F2VB_LAUNCH(N)                                                                                        \
