@@ -387,18 +387,16 @@ f2v_bwd_blocked_kernel(int64_t Nf, int CV, int K, const int32_t* __restrict__ fa
         // all sixteen row loads of the thread are issued first; the filter sums below need only the coefficients and run
         // while the rows are on their way
         float4 x[4], w[4], gr[4][3];
-        float rn[4][3];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int fl = (warp + 8 * i) * FPW + fs;
             x[i] = zero4(); w[i] = zero4();
 #pragma unroll
-            for (int j = 0; j < 3; ++j) { gr[i][j] = zero4(); rn[i][j] = 0.f; }
+            for (int j = 0; j < 3; ++j) gr[i][j] = zero4();
             if (on && fl < nf_tile) {
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
                     const int vo = svo[buf * NE + fl * 3 + j];
-                    rn[i][j] = srn[buf * NE + fl * 3 + j];
                     if (vo >= 0) gr[i][j] = ldg4(gout + (int64_t)vo * CV + cg);
                 }
                 x[i] = ldg4(in + (f0 + fl) * CV + cg);
@@ -418,7 +416,7 @@ f2v_bwd_blocked_kernel(int64_t Nf, int CV, int K, const int32_t* __restrict__ fa
             const int fl = (warp + 8 * i) * FPW + fs;
             float4 gt = zero4();
 #pragma unroll
-            for (int j = 0; j < 3; ++j) fma4s(gt, rn[i][j], gr[i][j]);
+            for (int j = 0; j < 3; ++j) fma4s(gt, srn[buf * NE + fl * 3 + j], gr[i][j]);
             if (on && fl < nf_tile) __stcs(gin + (f0 + fl) * CV + cg, mul4(gt, w[i]));
             if (fl < nf_tile) st[fl * LPF + l] = mul4(x[i], gt);
         }
@@ -431,10 +429,12 @@ f2v_bwd_blocked_kernel(int64_t Nf, int CV, int K, const int32_t* __restrict__ fa
         }
         // ---- phase 2, faces in order
         if (slice < slices) {
+            const int first = slice * FPW + fs, step = slices * FPW;
+            const float* cp = scoef + first * CP + 4 * g2;
+            const float4* tp = st + first * LPF + l;
 #pragma unroll 4
-            for (int fl = slice * FPW + fs; fl < nf_tile; fl += slices * FPW) {
-                const float4 t = st[fl * LPF + l];
-                const float4 c = *reinterpret_cast<const float4*>(scoef + fl * CP + 4 * g2);
+            for (int fl = first; fl < nf_tile; fl += step, cp += step * CP, tp += step * LPF) {
+                const float4 c = *reinterpret_cast<const float4*>(cp), t = *tp;
                 fma4s(acc[0], c.x, t); fma4s(acc[1], c.y, t); fma4s(acc[2], c.z, t); fma4s(acc[3], c.w, t);
             }
         }
