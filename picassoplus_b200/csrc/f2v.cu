@@ -58,11 +58,10 @@ f2v_fwd_face_kernel(int64_t Nf, int CV, int K, const float* __restrict__ coeff, 
     }
 }
 
-// The same for whole 128-channel chunks (lane = float4 channel group) and K <= 32, register-
-// blocked so that the shared-memory pipe is not the limit: warp w owns faces w, w+8, ..., w+56
-// of the tile, and a filter row read from shared memory (512 distinct bytes per warp) is used
-// for all eight; the coefficient loads are one broadcast address per warp.  The coefficient
-// rows of the next tile arrive by 4-byte asynchronous copies while this tile is computed.
+// The same register-blocked, for K <= 32: a face's channels lie on LPF lanes (float4 each; LPF = 4, 8, 16, 32, chunks of 128
+// channels behind that), a warp has 32 / LPF faces side by side, and a filter row read from shared memory is used for all FB such
+// passes of the warp.  The coefficient rows of the next tile arrive by 4-byte asynchronous copies while this one is
+// computed.  (The kernel above took 389 us for 1 758 000 faces of 64 channels, K = 16, bound by its shared-memory reads.)
 __device__ __forceinline__ void cp_async4(void* dst_smem, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src)
                  : "memory");
@@ -71,64 +70,70 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+template <int LPF> constexpr int F2VF_PASSES = LPF >= 16 ? 8 : 4;
+template <int LPF> constexpr int F2VF_FACES = 8 * F2VF_PASSES<LPF> * (32 / LPF);         // faces of a tile
+// floats of a coefficient row; a pad keeps the rows of faces side by side in a warp off one another's banks
+template <int LPF> __host__ __device__ constexpr int f2v_pitch(int K) { return (K + 3) / 4 * 4 + (LPF < 32 ? 4 : 0); }
+
+template <int LPF>
 __global__ void __launch_bounds__(256)
 f2v_fwd_face_blocked_kernel(int64_t Nf, int CV, int K, const float* __restrict__ coeff, const float4* __restrict__ in,
                             const float4* __restrict__ filt, float4* __restrict__ wx) {
     extern __shared__ float4 smem[];
-    constexpr int FB = F2VF_TF / 8;                            // faces per warp
-    const int KP = (K + 3) / 4 * 4, KG = KP / 4;               // coeff row pitch, pad columns zero
-    float4* sfilt = smem;                                      // [KP][32], rows K..KP-1 zero
-    float4* scoef0 = smem + KP * 32;                           // [2][TF][KG], double-buffered
+    constexpr int FB = F2VF_PASSES<LPF>, FPW = 32 / LPF, TF = F2VF_FACES<LPF>;
+    const int KG = (K + 3) / 4, CP = f2v_pitch<LPF>(K);
+    float4* sfilt = smem;                                      // [4 KG][LPF], rows K.. zero
+    float* scoef0 = reinterpret_cast<float*>(smem + 4 * KG * LPF);     // [2][TF][CP], double-buffered, pad columns zero
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int cg = blockIdx.y * 32 + lane;
-    for (int i = threadIdx.x; i < KP * 32; i += blockDim.x) {
-        const int k = i >> 5;
-        sfilt[i] = k < K ? filt[k * CV + blockIdx.y * 32 + (i & 31)] : zero4();
+    const int l = lane % LPF, fs = lane / LPF;                 // channel group, face among the warp's
+    const int cg = blockIdx.y * LPF + l;
+    const bool on = cg < CV;
+    for (int i = threadIdx.x; i < 4 * KG * LPF; i += blockDim.x) {
+        const int k = i / LPF, c = blockIdx.y * LPF + i % LPF;
+        sfilt[i] = k < K && c < CV ? filt[k * CV + c] : zero4();
     }
-    for (int i = threadIdx.x; i < 2 * F2VF_TF * KG; i += blockDim.x) scoef0[i] = zero4();
+    for (int i = threadIdx.x; i < 2 * TF * CP; i += blockDim.x) scoef0[i] = 0.f;
     __syncthreads();
-    const int64_t ntiles = (Nf + F2VF_TF - 1) / F2VF_TF;
-    auto fetch_coef = [&](int64_t tile, int buf) {             // the pad columns stay zero
-        if (tile < ntiles) {
-            const int64_t f0 = tile * F2VF_TF;
-            const int nf_tile = Nf - f0 < F2VF_TF ? (int)(Nf - f0) : F2VF_TF;
-            float* sc = reinterpret_cast<float*>(scoef0 + buf * F2VF_TF * KG);
-            for (int i = threadIdx.x; i < nf_tile * K; i += blockDim.x) {
-                const int fl = i / K;
-                cp_async4(sc + fl * KP + (i - fl * K), coeff + f0 * K + i);
-            }
+    const int64_t ntiles = (Nf + TF - 1) / TF;
+    auto fetch_coef = [&](int64_t tile, int buf) {             // a lane per coefficient
+        if (tile < ntiles && lane < K) {
+            const int64_t f0 = tile * TF;
+            const int nf_tile = Nf - f0 < TF ? (int)(Nf - f0) : TF;
+            const float* src = coeff + f0 * K + lane;
+            float* sc = scoef0 + buf * TF * CP + lane;
+            for (int fl = warp; fl < nf_tile; fl += 8) cp_async4(sc + fl * CP, src + fl * K);
         }
         cp_async_commit();
     };
     fetch_coef(blockIdx.x, 0);
     int buf = 0;
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, buf ^= 1) {
-        const int64_t f0 = tile * F2VF_TF;
-        const int nf_tile = Nf - f0 < F2VF_TF ? (int)(Nf - f0) : F2VF_TF;
+        const int64_t f0 = tile * TF;
+        const int nf_tile = Nf - f0 < TF ? (int)(Nf - f0) : TF;
         fetch_coef(tile + gridDim.x, buf ^ 1);                 // its readers finished behind the barrier below
         cp_async_wait<1>();                                    // this tile's rows have landed (own copies) ...
         __syncthreads();                                       // ... and everybody else's
-        const float4* scoef = scoef0 + buf * F2VF_TF * KG;
+        const float* scoef = scoef0 + buf * TF * CP + (warp * FPW + fs) * CP;
         float4 x[FB], w[FB];
 #pragma unroll
         for (int i = 0; i < FB; ++i) {
-            const int fl = warp + 8 * i;
+            const int fl = (warp + 8 * i) * FPW + fs;
             w[i] = zero4();
-            x[i] = fl < nf_tile ? ldg4(in + (f0 + fl) * CV + cg) : zero4();
+            x[i] = on && fl < nf_tile ? ldg4(in + (f0 + fl) * CV + cg) : zero4();
         }
         for (int g = 0; g < KG; ++g) {
-            const float4 f0v = sfilt[(4 * g) * 32 + lane], f1v = sfilt[(4 * g + 1) * 32 + lane];
-            const float4 f2v = sfilt[(4 * g + 2) * 32 + lane], f3v = sfilt[(4 * g + 3) * 32 + lane];
+            const float4 fa = sfilt[4 * g * LPF + l], fb = sfilt[(4 * g + 1) * LPF + l];
+            const float4 fc = sfilt[(4 * g + 2) * LPF + l], fd = sfilt[(4 * g + 3) * LPF + l];
 #pragma unroll
-            for (int i = 0; i < FB; ++i) {
-                const float4 cf = scoef[(warp + 8 * i) * KG + g];        // rows past the tile are stale or zero: unused
-                fma4s(w[i], cf.x, f0v); fma4s(w[i], cf.y, f1v); fma4s(w[i], cf.z, f2v); fma4s(w[i], cf.w, f3v);
+            for (int i = 0; i < FB; ++i) {                     // rows past the tile are stale or zero: unused
+                const float4 cf = *reinterpret_cast<const float4*>(scoef + 8 * i * FPW * CP + 4 * g);
+                fma4s(w[i], cf.x, fa); fma4s(w[i], cf.y, fb); fma4s(w[i], cf.z, fc); fma4s(w[i], cf.w, fd);
             }
         }
 #pragma unroll
         for (int i = 0; i < FB; ++i) {
-            const int fl = warp + 8 * i;
-            if (fl < nf_tile) wx[(f0 + fl) * CV + cg] = mul4(w[i], x[i]);
+            const int fl = (warp + 8 * i) * FPW + fs;
+            if (on && fl < nf_tile) wx[(f0 + fl) * CV + cg] = mul4(w[i], x[i]);
         }
         __syncthreads();                                       // this tile's buffer may be refilled now
     }
@@ -296,11 +301,9 @@ f2v_bwd_tile_kernel(int64_t Nf, int CV, int K, const int32_t* __restrict__ face,
 // The index chain of the gather (face -> vtMap -> nfCount) is resolved one hop per tile for the block's next three tiles, so that
 // phase 1 finds output vertex and 1/nfCount of every corner in shared memory and issues its twelve gradOutput row loads at once.
 template <int LPF> constexpr int F2VB_FACES = 32 * (32 / LPF);         // faces of a tile
-// floats of a coefficient row; a pad keeps the rows of faces side by side in a warp off one another's banks
-template <int LPF> __host__ __device__ constexpr int f2vb_pitch(int K) { return (K + 3) / 4 * 4 + (LPF < 32 ? 4 : 0); }
 template <int LPF>
 static size_t f2vb_smem(int K) {
-    return sizeof(float4) * ((size_t)(K + 3) / 4 * 4 * LPF + F2VB_FACES<LPF> * LPF) + sizeof(float) * 2 * F2VB_FACES<LPF> * f2vb_pitch<LPF>(K) +
+    return sizeof(float4) * ((size_t)(K + 3) / 4 * 4 * LPF + F2VB_FACES<LPF> * LPF) + sizeof(float) * 2 * F2VB_FACES<LPF> * f2v_pitch<LPF>(K) +
            2 * F2VB_FACES<LPF> * 3 * 8;
 }
 
@@ -312,7 +315,7 @@ f2v_bwd_blocked_kernel(int64_t Nf, int CV, int K, const int32_t* __restrict__ fa
                        float4* __restrict__ gin, float4* __restrict__ partial) {
     extern __shared__ float4 smem[];
     constexpr int FPW = 32 / LPF, TF = F2VB_FACES<LPF>, NE = TF * 3, NI = (NE + 255) / 256;
-    const int KG = (K + 3) / 4, CP = f2vb_pitch<LPF>(K);            // groups of 4 coefficients (<= 8)
+    const int KG = (K + 3) / 4, CP = f2v_pitch<LPF>(K);            // groups of 4 coefficients (<= 8)
     float4* sfilt = smem;                                      // [4 KG][LPF], rows K.. zero
     float4* st = smem + 4 * KG * LPF;                          // [TF][LPF]   t = input * gt
     float* scoef0 = reinterpret_cast<float*>(st + TF * LPF);   // [2][TF][CP], double-buffered (asynchronous copies)
@@ -542,12 +545,19 @@ int f2v_face_products(int64_t Nf, int C, int K, const float* input, const float*
     const int CV = C / 4;
     float4* wx = (float4*)wx_;
     if (Nf <= 0) return PB200_OK;
-    if (CV % 32 == 0 && K <= 32) {
-        const int KPb = (K + 3) / 4 * 4;
-        const size_t smemb = sizeof(float4) * ((size_t)KPb * 32 + 2 * F2VF_TF * (KPb / 4));
-        dim3 gridf(persistent_blocks(Nf, F2VF_TF, 4), (unsigned)(CV / 32));
-        PB_LAUNCH("f2v_fwd_face", f2v_fwd_face_blocked_kernel, gridf, 256, smemb, stream, Nf, CV, K, coeff,
-                  (const float4*)input, (const float4*)filter, wx);
+    if (K <= 32) {
+        auto run = [&](auto lpf) {
+            constexpr int LPF = decltype(lpf)::value, TF = F2VF_FACES<LPF>;
+            const size_t smemb = sizeof(float4) * (size_t)((K + 3) / 4 * 4) * LPF + sizeof(float) * 2 * TF * f2v_pitch<LPF>(K);
+            PB_CUDA(cudaFuncSetAttribute(f2v_fwd_face_blocked_kernel<LPF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemb));
+            PB_LAUNCH("f2v_fwd_face", f2v_fwd_face_blocked_kernel<LPF>, dim3(persistent_blocks(Nf, TF, 4), (unsigned)ceil_div(CV, LPF)),
+                      256, smemb, stream, Nf, CV, K, coeff, (const float4*)input, (const float4*)filter, wx);
+            return PB200_OK;
+        };
+        if (CV <= 4) return run(std::integral_constant<int, 4>{});
+        if (CV <= 8) return run(std::integral_constant<int, 8>{});
+        if (CV <= 16) return run(std::integral_constant<int, 16>{});
+        return run(std::integral_constant<int, 32>{});
     } else {
         const int KP = (K + 3) / 4 * 4 + 4;
         size_t smem = sizeof(float4) * 32 * (size_t)K + sizeof(float) * F2VF_TF * KP;
