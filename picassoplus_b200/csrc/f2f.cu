@@ -10,6 +10,14 @@ int f2f_simt_forward(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, const fl
 int f2f_simt_backward(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, const float* gout, const float* input,
                       const float* filter, const float* bary, const int32_t* cum, float* gin, float* gfilter,
                       void* ws, cudaStream_t stream, bool want_gin, bool want_gfilter);
+namespace small {
+bool supported(int Cin, int Cout, int F);
+int forward(int64_t Nf, int Cin, int Cout, int F, const float* input, const float* filter, const float* bary, const int32_t* cum,
+            float* output, cudaStream_t stream);
+size_t workspace_bytes(int64_t Nf, int Cin, int Cout, int F);
+int backward_filter(int64_t Nf, int Cin, int Cout, int F, const float* gout, const float* input, const float* bary, const int32_t* cum,
+                    float* gfilter, void* ws, cudaStream_t stream);
+}  // namespace small
 namespace tc {
 bool fwd_supported(int Cin, int Cout, int F);
 size_t fwd_workspace_bytes(int64_t NiK, int Cin, int Cout, int F, int precision);
@@ -58,6 +66,17 @@ static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 static bool use_tc_fwd(int Cin, int Cout, int F, int precision) {
     return precision != PB200_PREC_FP32_FFMA && tc::fwd_supported(Cin, Cout, F);
 }
+// Few input channels: fp32 kernels of their own in every tensor-core mode.  A mesh of less than a thousand faces stays on the
+// tensor-core kernels, as the tests of the dispatch have it: a call is launches there (960 faces 25 us against 9).  The filter
+// gradient's products outgrow the multiply-add units where the tensor cores' padding wastes less (1 758 000 faces, three channels:
+// 16 bases, 32 outputs 358 against 876 us, 25 bases, 64 outputs 1376 against 1066); forward there are no partial sums to keep and the
+// line lies further out (278 against 907 us, 1006 against 1168).
+static bool use_small(int64_t Nf, int Cin, int Cout, int F, int precision) {
+    return precision != PB200_PREC_FP32_FFMA && Nf >= 1024 && small::supported(Cin, Cout, F) && Cin * Cout * F <= 5000;
+}
+static bool use_small_gf(int64_t Nf, int Cin, int Cout, int F, int precision) {
+    return use_small(Nf, Cin, Cout, F, precision) && Cin * Cout * F <= 3600;
+}
 static bool use_tc_gf(int64_t Nf, int Cin, int Cout, int F, int precision) {
     return precision != PB200_PREC_FP32_FFMA && tc::gfilter::supported(Cin, Cout, F) &&
            tc::gfilter::fits(Nf, Cin, Cout, F, precision);
@@ -74,6 +93,7 @@ extern "C" {
 
 size_t pb200_facet2facet_forward_workspace_bytes(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, int precision) {
     if (!f2f_sizes_ok(Nf, NiK, Cin, Cout, F)) return 0;
+    if (use_small(Nf, Cin, Cout, F, precision)) return 256;
     if (use_tc_fwd(Cin, Cout, F, precision)) return tc::fwd_workspace_bytes(NiK, Cin, Cout, F, precision);
     return f2f_simt_fwd_ws(Nf, Cin, Cout, F);
 }
@@ -91,6 +111,7 @@ int pb200_facet2facet_forward(int64_t Nf, int64_t NiK, int Cin, int Cout, int F,
                "facet2facet_forward: null pointer");
     PB_REQUIRE(workspace && workspace_bytes >= pb200_facet2facet_forward_workspace_bytes(Nf, NiK, Cin, Cout, F, precision),
                PB200_EWORKSPACE, "facet2facet_forward: workspace too small");
+    if (use_small(Nf, Cin, Cout, F, precision)) return small::forward(Nf, Cin, Cout, F, input, filter, bary, numInterior, output, stream);
     if (use_tc_fwd(Cin, Cout, F, precision)) {
         PB_REQUIRE(NiK == 0 || aligned16(input), PB200_EINVAL, "facet2facet_forward: input must be 16-byte aligned");
         PB_REQUIRE(aligned16(workspace), PB200_EINVAL, "facet2facet_forward: workspace must be 16-byte aligned");
@@ -173,6 +194,7 @@ static size_t gin_ws(int Cin, int Cout, int F, int precision) {
 
 // room for the partial sums of either filter-gradient kernel
 static size_t gf_ws(int64_t Nf, int Cin, int Cout, int F, int precision) {
+    if (use_small_gf(Nf, Cin, Cout, F, precision)) return small::workspace_bytes(Nf, Cin, Cout, F);
     const size_t a = tc::gfilter::workspace_bytes(Nf, Cin, Cout, F, precision);
     const size_t b = tc::onef::supported(Cin, Cout, F, precision) ? tc::onef::workspace_bytes(Nf, Cin, Cout, F, precision) : 0;
     return a > b ? a : b;
@@ -180,12 +202,13 @@ static size_t gf_ws(int64_t Nf, int Cin, int Cout, int F, int precision) {
 
 size_t pb200_facet2facet_backward_workspace_bytes(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, int precision) {
     if (!f2f_sizes_ok(Nf, NiK, Cin, Cout, F)) return 0;
-    const bool tg = use_tc_gin(Cin, Cout, F, precision), tf = use_tc_gf(Nf, Cin, Cout, F, precision);
+    const bool tg = use_tc_gin(Cin, Cout, F, precision), sf = use_small_gf(Nf, Cin, Cout, F, precision);
+    const bool tf = sf || use_tc_gf(Nf, Cin, Cout, F, precision);
     size_t n = (tg && tf) ? 0 : f2f_simt_bwd_ws(Nf, Cin, Cout, F);
     if (tg) n += gin_ws(Cin, Cout, F, precision);
     if (tf) n += gf_ws(Nf, Cin, Cout, F, precision);
     if (tg || tf) n += tc::padded_bary_bytes(NiK, F);
-    if (tf) n += tc::padded_input_bytes(NiK, Cin);
+    if (tf && !sf) n += tc::padded_input_bytes(NiK, Cin);
     return n;
 }
 
@@ -211,7 +234,8 @@ static int f2f_backward_impl(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, 
                "facet2facet_backward: null pointer");
     PB_REQUIRE(workspace && workspace_bytes >= pb200_facet2facet_backward_workspace_bytes(Nf, NiK, Cin, Cout, F, precision),
                PB200_EWORKSPACE, "facet2facet_backward: workspace too small");
-    const bool tg = use_tc_gin(Cin, Cout, F, precision), tf = use_tc_gf(Nf, Cin, Cout, F, precision);
+    const bool tg = use_tc_gin(Cin, Cout, F, precision), sf = use_small_gf(Nf, Cin, Cout, F, precision);
+    const bool tf = sf || use_tc_gf(Nf, Cin, Cout, F, precision);
     if (tg || tf)
         PB_REQUIRE(aligned16(gradOutput) && aligned16(workspace) && (NiK == 0 || (aligned16(input) && aligned16(bary))),
                    PB200_EINVAL, "facet2facet_backward: gradOutput, input, bary and workspace must be 16-byte aligned");
@@ -221,7 +245,7 @@ static int f2f_backward_impl(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, 
     // both tensor-core kernels read bary rows with 16-byte loads: rows padded to 4 floats
     const float* bary_p = bary;
     const int Fp = tc::padded_F(F);
-    if ((tg || tf) && F % 4 != 0 && NiK > 0) {
+    if (((tg && want_gin) || (tf && !sf)) && F % 4 != 0 && NiK > 0) {
         if (baryPadded) {
             PB_REQUIRE(aligned16(baryPadded), PB200_EINVAL, "facet2facet_backward: baryPadded must be 16-byte aligned");
             bary_p = baryPadded;
@@ -243,7 +267,10 @@ static int f2f_backward_impl(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, 
         }
         w += gin_ws(Cin, Cout, F, precision);
     }
-    if (tf && one_each && tc::onef::supported(Cin, Cout, F, precision)) {
+    if (sf) {
+        int rc = small::backward_filter(Nf, Cin, Cout, F, gradOutput, input, bary, numInterior, gradFilter, w, stream);
+        if (rc) return rc;
+    } else if (tf && one_each && tc::onef::supported(Cin, Cout, F, precision)) {
         int rc = tc::onef::backward_filter(Nf, Cin, Cout, F, gradOutput, input, bary_p, gradFilter, precision, w, stream);
         if (rc) return rc;
     } else if (tf) {
