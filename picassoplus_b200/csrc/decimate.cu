@@ -61,6 +61,26 @@ __device__ __forceinline__ void warp_append(bool pred, uint32_t value, uint32_t*
     if (pred) list[base + __popc(m & ((1u << lane) - 1u))] = value;
 }
 
+// SWEEP values per lane, those with what[j] == wanted, with one addition to the counter
+constexpr int SWEEP = 4;
+__device__ __forceinline__ void warp_append_all(const int (&what)[SWEEP], int wanted, const uint32_t (&value)[SWEEP],
+                                                uint32_t* __restrict__ list, int32_t* counter) {
+    const int lane = threadIdx.x & 31;
+    unsigned m[SWEEP];
+    int total = 0;
+#pragma unroll
+    for (int j = 0; j < SWEEP; ++j) { m[j] = __ballot_sync(0xffffffffu, what[j] == wanted); total += __popc(m[j]); }
+    if (total == 0) return;
+    int32_t base = 0;
+    if (lane == 0) base = atomicAdd(counter, total);
+    base = __shfl_sync(0xffffffffu, base, 0);
+#pragma unroll
+    for (int j = 0; j < SWEEP; ++j) {
+        if (what[j] == wanted) list[base + __popc(m[j] & ((1u << lane) - 1u))] = value[j];
+        base += __popc(m[j]);
+    }
+}
+
 // counter[key] += 1 for the lanes with key >= 0, one atomic per distinct key of the warp; called by whole warps
 __device__ __forceinline__ void warp_count(int key, int32_t* counter) {
     const int lane = threadIdx.x & 31;
@@ -648,13 +668,20 @@ __device__ bool grid_select(const Cluster& p, const uint32_t* list, int n, bool 
     for (int shift = 64 - bits; shift >= 0; shift -= bits) {
         const bool empty = shift < 32 && shift >= ubits;
         if (!empty) {
-            for (int i = tid; i < n; i += nt) {
-                const uint32_t u = __ldcg(list + i);
-                const int s = sample_of(p.ulo[u], p.nvIn, p.B);
-                if (__ldcg(&p.rest[s]) < 0) continue;
-                const u64 key = p.key[u];
-                if (shift + bits >= 64 || (key >> (shift + bits)) == __ldcg(&p.prefix[s]))
-                    atomicAdd(&p.hist[((int64_t)s << bits) + (int)((key >> shift) & (u64)(bins - 1))], 1);
+            // one atomic per distinct digit of a warp: the upper digits are the costs' exponents, the same for most
+            for (int i0 = tid - (int)(threadIdx.x & 31); i0 < n; i0 += nt) {
+                const int i = i0 + (int)(threadIdx.x & 31);
+                int at = -1;
+                if (i < n) {
+                    const uint32_t u = __ldcg(list + i);
+                    const int s = sample_of(p.ulo[u], p.nvIn, p.B);
+                    if (__ldcg(&p.rest[s]) >= 0) {
+                        const u64 key = p.key[u];
+                        if (shift + bits >= 64 || (key >> (shift + bits)) == __ldcg(&p.prefix[s]))
+                            at = (s << bits) + (int)((key >> shift) & (u64)(bins - 1));
+                    }
+                }
+                warp_count(at, p.hist);
             }
             if (!grid_barrier(p.barrier, p.status)) return false;
         }
@@ -688,10 +715,11 @@ __device__ bool grid_select(const Cluster& p, const uint32_t* list, int n, bool 
     return true;
 }
 
-__global__ void __launch_bounds__(GRID_THREADS, 3) cluster_grid_kernel(Cluster p) {
+__global__ void __launch_bounds__(GRID_THREADS, 2) cluster_grid_kernel(Cluster p) {
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
     // the barrier's give-up flag shares the word: nobody raises it before everybody has passed the first barrier
     if (__ldcg(p.status) != 0) return;
+    const int lane = threadIdx.x & 31;
     const int nu = p.ustart[p.Nv];
     const int ubits = bit_length(nu);
     int32_t* live = p.counters;             // [3] in turn
@@ -714,21 +742,50 @@ __global__ void __launch_bounds__(GRID_THREADS, 3) cluster_grid_kernel(Cluster p
     };
     while (n > TAIL || (from == nullptr && n > 0)) {
         if (tid == 0) live[(slot + 1) % 3] = 0;
-        for (int i = tid; i < n; i += nt) {
-            const uint32_t u = from ? __ldcg(from + i) : (uint32_t)i;
-            if (from || eligible(u)) post_edge(p, u, vmin);
+        // SWEEP edges of a thread at a time: their chains of loads overlap, and the lists' counters see one addition per batch of a warp
+        for (int i0 = tid; i0 < n; i0 += SWEEP * nt) {
+            uint32_t u[SWEEP];
+            int lo[SWEEP], hi[SWEEP];
+            u64 k[SWEEP];
+            bool on[SWEEP];
+#pragma unroll
+            for (int j = 0; j < SWEEP; ++j) {
+                on[j] = i0 + j * nt < n;
+                u[j] = !on[j] ? 0u : from ? __ldcg(from + i0 + j * nt) : (uint32_t)(i0 + j * nt);
+            }
+#pragma unroll
+            for (int j = 0; j < SWEEP; ++j) {
+                on[j] = on[j] && (from || eligible(u[j]));
+                lo[j] = on[j] ? p.ulo[u[j]] : 0; hi[j] = on[j] ? p.uhi[u[j]] : 0; k[j] = on[j] ? p.key[u[j]] : 0;
+            }
+#pragma unroll
+            for (int j = 0; j < SWEEP; ++j) on[j] = on[j] && !is_covered(p.covered, lo[j]) && !is_covered(p.covered, hi[j]);
+            u64 a[SWEEP], b[SWEEP];
+#pragma unroll
+            for (int j = 0; j < SWEEP; ++j) { a[j] = on[j] ? __ldcg(&vmin[lo[j]]) : 0; b[j] = on[j] ? __ldcg(&vmin[hi[j]]) : 0; }
+#pragma unroll
+            for (int j = 0; j < SWEEP; ++j) {                   // slots only fall: a key above what is there need not be posted
+                if (k[j] < a[j]) atomicMin(&vmin[lo[j]], k[j]);
+                if (k[j] < b[j]) atomicMin(&vmin[hi[j]], k[j]);
+            }
         }
         if (!grid_barrier(p.barrier, p.status)) return;
-        for (int i0 = blockIdx.x * blockDim.x; i0 < n; i0 += nt) {
-            const int i = i0 + threadIdx.x;
-            int what = 0;
-            uint32_t u = 0;
-            if (i < n) {
-                u = from ? __ldcg(from + i) : (uint32_t)i;
-                if (from || eligible(u)) what = take_edge(p, u, vmin, vnext);
+        for (int i0 = tid - lane; i0 < n; i0 += SWEEP * nt) {
+            uint32_t u[SWEEP];
+            int what[SWEEP];
+#pragma unroll
+            for (int j = 0; j < SWEEP; ++j) {
+                const int i = i0 + j * nt + lane;
+                u[j] = i >= n ? 0u : from ? __ldcg(from + i) : (uint32_t)i;
+                what[j] = i < n && (from || eligible(u[j])) ? 1 : 0;
             }
-            took(what == 2, u);
-            warp_append(what == 1, u, out, &live[slot]);
+#pragma unroll
+            for (int j = 0; j < SWEEP; ++j) what[j] = what[j] ? take_edge(p, u[j], vmin, vnext) : 0;
+            warp_append_all(what, 2, u, p.taken, ntaken);
+#pragma unroll
+            for (int j = 0; j < SWEEP; ++j)
+                if (__any_sync(0xffffffffu, what[j] == 2)) warp_count(what[j] == 2 ? sample_of(p.ulo[u[j]], p.nvIn, p.B) : -1, p.matched);
+            warp_append_all(what, 1, u, out, &live[slot]);
         }
         if (!grid_barrier(p.barrier, p.status)) return;
         n = __ldcg(&live[slot]);

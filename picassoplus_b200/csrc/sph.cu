@@ -10,6 +10,19 @@ namespace pb {
 
 constexpr int SPH_BLOCK = 128;
 
+// the block's rows, K of K + 1 floats each in shared memory, to consecutive addresses.  Element j + SPH_BLOCK lies SPH_BLOCK / K rows
+// and SPH_BLOCK % K columns further on: no division per element (with a 64-bit one the kernel took 137 us for 4.4 million points
+// of 16 components)
+__device__ __forceinline__ void write_rows(const float* stage, int rows, int K, float* dst) {
+    const int drow = SPH_BLOCK / K, dcol = SPH_BLOCK - drow * K;
+    int r = (int)threadIdx.x / K, k = (int)threadIdx.x - r * K;
+    for (int j = threadIdx.x; j < rows * K; j += SPH_BLOCK) {
+        dst[j] = stage[r * (K + 1) + k];
+        r += drow; k += dcol;
+        if (k >= K) { k -= K; ++r; }
+    }
+}
+
 __global__ void __launch_bounds__(SPH_BLOCK)
 sph_harm_kernel(int64_t N, int L, const float* __restrict__ xyz, SphConst cst, float* __restrict__ out) {
     extern __shared__ float stage[];            // [SPH_BLOCK][K+1]
@@ -22,12 +35,7 @@ sph_harm_kernel(int64_t N, int L, const float* __restrict__ xyz, SphConst cst, f
         sph_eval(xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], L, c, stage + threadIdx.x * KP);
     }
     __syncthreads();
-    int64_t npts = N - base < SPH_BLOCK ? N - base : SPH_BLOCK;
-    float* dst = out + base * K;
-    for (int64_t j = threadIdx.x; j < npts * K; j += SPH_BLOCK) {
-        int p = (int)(j / K), k = (int)(j - (int64_t)p * K);
-        dst[j] = stage[p * KP + k];
-    }
+    write_rows(stage, (int)(N - base < SPH_BLOCK ? N - base : SPH_BLOCK), K, out + base * K);
 }
 
 // out[f] = mean over the samples k of face f of the components of xyz[k] (0 for a face without samples): the two
@@ -58,12 +66,7 @@ face_mean_sph_harm_kernel(int64_t Nf, int64_t NiK, int L, const float* __restric
         for (int k = 0; k < K; ++k) acc[k] *= inv;
     }
     __syncthreads();
-    const int64_t nrows = Nf - base < SPH_BLOCK ? Nf - base : SPH_BLOCK;
-    float* dst = out + base * K;
-    for (int64_t j = threadIdx.x; j < nrows * K; j += SPH_BLOCK) {
-        int r = (int)(j / K), k = (int)(j - (int64_t)r * K);
-        dst[j] = stage[r * KP + k];
-    }
+    write_rows(stage, (int)(Nf - base < SPH_BLOCK ? Nf - base : SPH_BLOCK), K, out + base * K);
 }
 
 // The three-row vertex2facet filter of a layer, corners (3,K) @ weights (K,C), and its gradient corners^T @ gradFilter:
