@@ -191,16 +191,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_gfilter_kernel(Par
                 __syncwarp();
                 if (lane == 0) mbar_arrive(acc_free);
             }
-            if (!warp_wait(&raw_full[rr.i], rr.ph, abort_flag, lane)) { alive = false; break; }
+            // (the warp that reports the weights has seen the rows arrive)
+            const int slot = gr.i;
+            if (!warp_wait(&g_full[slot], gr.ph, abort_flag, lane)) { alive = false; break; }
             float x[FS];
             {
                 const uint32_t a = x32 + (uint32_t)rr.i * raw_bytes, pitch = (uint32_t)p.R * 4u;
 #pragma unroll
                 for (int k = 0; k < FS; ++k) x[k] = lds_f32(a + k * pitch);
             }
-            const int slot = gr.i;
-            if (!warp_wait(&g_full[slot], gr.ph, abort_flag, lane) ||
-                (st >= p.nbuf && !warp_wait(&done[(st - p.nbuf) & 7], (uint32_t)((st - p.nbuf) >> 3) & 1u, abort_flag, lane))) {
+            if (st >= p.nbuf && !warp_wait(&done[(st - p.nbuf) & 7], (uint32_t)((st - p.nbuf) >> 3) & 1u, abort_flag, lane)) {
                 alive = false;
                 break;
             }
