@@ -66,13 +66,13 @@ static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 static bool use_tc_fwd(int Cin, int Cout, int F, int precision) {
     return precision != PB200_PREC_FP32_FFMA && tc::fwd_supported(Cin, Cout, F);
 }
-// Few input channels: fp32 kernels of their own in every tensor-core mode.  A mesh of less than a thousand faces stays on the
-// tensor-core kernels, as the tests of the dispatch have it: a call is launches there (960 faces 25 us against 9).  The filter
+// Few input channels: fp32 kernels of their own in every tensor-core mode.  A mesh of less than 4096 faces stays on the
+// tensor-core kernels, as the tests of the dispatch have it: a step is host work there, and a call launches (4000 faces 26 us against 9).  The filter
 // gradient's products outgrow the multiply-add units where the tensor cores' padding wastes less (1 758 000 faces, three channels:
 // 16 bases, 32 outputs 358 against 876 us, 25 bases, 64 outputs 1376 against 1066); forward there are no partial sums to keep and the
 // line lies further out (278 against 907 us, 1006 against 1168).
 static bool use_small(int64_t Nf, int Cin, int Cout, int F, int precision) {
-    return precision != PB200_PREC_FP32_FFMA && Nf >= 1024 && small::supported(Cin, Cout, F) && Cin * Cout * F <= 5000;
+    return precision != PB200_PREC_FP32_FFMA && Nf >= 4096 && small::supported(Cin, Cout, F) && Cin * Cout * F <= 5000;
 }
 static bool use_small_gf(int64_t Nf, int Cin, int Cout, int F, int precision) {
     return use_small(Nf, Cin, Cout, F, precision) && Cin * Cout * F <= 3600;

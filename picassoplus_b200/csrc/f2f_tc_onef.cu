@@ -22,6 +22,7 @@
 // f2f_tc_gfilter.cu) with reductions that nothing waits for; each address has one thread that adds, so the order is fixed.
 // A second kernel adds the chunks in order.  All waits are bounded.
 #include <math.h>
+#include <string.h>
 #include <type_traits>
 #include "common.cuh"
 #include "tc_ptx.cuh"
@@ -431,7 +432,7 @@ static size_t smem_bytes(const Params& p, int nsplit, int faces) {
 // The split of the work, everything but the pointers: the way (which tensor is expanded, its channel blocks, tiles per CTA) with
 // the least estimated time.  A stage of a CTA takes the longest of its products (half a clock per column), the building of the
 // expanded operand (about 100 clocks per tile and 250 besides) and its rows (about 24 bytes per clock from L2).
-static bool plan(int64_t Nf, int Cin, int Cout, int F, int precision, Params& p) {
+static void make_plan(int64_t Nf, int Cin, int Cout, int F, int precision, Params& p) {
     const int nsplit = operand_mode(precision).nsplit, fs = nsplit == 2 ? FACES<2> : FACES<1>, products = nsplit == 2 ? 3 : 2;
     const int sms = sm_count(), Fp = (F + 3) / 4 * 4;
     p = Params();
@@ -482,20 +483,29 @@ static bool plan(int64_t Nf, int Cin, int Cout, int F, int precision, Params& p)
     if (chunks > pay) chunks = pay;
     if (chunks > p.nstages) chunks = p.nstages;
     p.chunks = chunks < 1 ? 1 : (int)chunks;
-    return smem_bytes(p, nsplit, fs) <= 227 * 1024;
+}
+
+// A call wants its plan several times (workspace, checks, launch), and a training loop the same one every step
+static const Params& plan(int64_t Nf, int Cin, int Cout, int F, int precision) {
+    static thread_local int64_t key[6] = {-1, 0, 0, 0, 0, 0};
+    static thread_local Params last;
+    const int64_t now[6] = {Nf, Cin, Cout, F, precision, sm_count()};
+    if (memcmp(key, now, sizeof(key)) != 0) {
+        make_plan(Nf, Cin, Cout, F, precision, last);
+        memcpy(key, now, sizeof(key));
+    }
+    return last;
 }
 
 // bf16 operands (hi + lo or single); rows of both tensors in pieces of 16 bytes
 bool supported(int Cin, int Cout, int F, int precision) {
     if (precision != PB200_PREC_FP32 && precision != PB200_PREC_BF16) return false;
-    if (Cin < 4 || Cout < 4 || Cin % 4 != 0 || Cout % 4 != 0 || F < 1 || F > MAX_F) return false;
-    Params p;
-    return plan(1, Cin, Cout, F, precision, p);
+    // (blocks of 128 channels, 32 bases and rings of four fit into shared memory)
+    return Cin >= 4 && Cout >= 4 && Cin % 4 == 0 && Cout % 4 == 0 && F >= 1 && F <= MAX_F;
 }
 
 size_t workspace_bytes(int64_t Nf, int Cin, int Cout, int F, int precision) {
-    Params p;
-    plan(Nf, Cin, Cout, F, precision, p);
+    const Params& p = plan(Nf, Cin, Cout, F, precision);
     return align_up((size_t)p.nb1 * p.nb2 * p.groups * p.chunks * sum_cols(p) * ROWS * sizeof(float), 256);
 }
 
@@ -512,8 +522,7 @@ int backward_filter(int64_t Nf, int Cin, int Cout, int F, const float* gout, con
                     int precision, void* ws, cudaStream_t stream) {
     int rc = check_async_error("facet2facet_backward");
     if (rc) return rc;
-    Params p;
-    PB_REQUIRE(plan(Nf, Cin, Cout, F, precision, p), PB200_EINVAL, "facet2facet_backward: no plan for the filter gradient");
+    Params p = plan(Nf, Cin, Cout, F, precision);
     p.x = p.swap ? gout : input;
     p.g = p.swap ? input : gout;
     p.w = w; p.sums = (float*)ws; p.out = gfilter;

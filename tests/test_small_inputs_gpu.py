@@ -8,8 +8,8 @@ from conftest import rel_err
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nf,cin,cout,F", [(1024, 3, 32, 16), (1025, 1, 4, 1), (1087, 2, 16, 9), (1151, 3, 33, 25), (1279, 4, 28, 32),
-                                            (1281, 3, 48, 16), (5000, 3, 100, 9), (1500, 1, 130, 25), (1100, 3, 7, 7), (2049, 3, 64, 25),
+@pytest.mark.parametrize("nf,cin,cout,F", [(4096, 3, 32, 16), (4097, 1, 4, 1), (4159, 2, 16, 9), (4223, 3, 33, 25), (4351, 4, 28, 32),
+                                            (4353, 3, 48, 16), (5000, 3, 100, 9), (4500, 1, 130, 25), (4200, 3, 7, 7), (8193, 3, 64, 25),
                                             (90000, 3, 32, 16)])
 def test_small_inputs(nf, cin, cout, F):
     from picassoplus_b200.mesh.pi_modules import conv3d
