@@ -12,10 +12,14 @@
 //     slices to drain one; the two warps of a quadrant in a group take the slice's channel quadruples in turn, load a
 //     quadruple's columns together, hand the accumulator back as soon as the last columns are in registers, and store 16 bytes
 //     per quadruple;
-//   * a slice holds a multiple of four channels (NQ), its filter image exactly the rows the product reads;
-//   * a work item is a tile of 128 faces and a run of slices: few tiles are spread over the chip by splitting their slices.
-// Loaders, filter stream and MMA issue as in f2f_tc_gin.cu.  What bounds it now: the three products per term at 64 channels
-// and more (bf16 hi + lo), the epilogue below and in bf16 mode.  All waits are bounded.
+//   * a slice holds as many channels as fill the accumulator (NQ; drained in groups of G), its filter image exactly the rows the
+//     product reads, and a filter stage as many K-blocks as fit twice (a hand-over per K-block cost the bf16 mode a third);
+//   * a work item is a tile of 128 faces and a run of slices: few tiles are spread over the chip by splitting their slices;
+//   * the next item's rows and weights are asked towards L2 while this one's are copied.
+// Loaders, filter stream and MMA issue as in f2f_tc_gin.cu.  Now 735 us for the product above, and 1683 for 930 000 faces, 128 -> 128,
+// 25 bases (bf16 1260 -> 857).  What bounds it: the three products per term at 128 channels (0.96 of what the board sustains), the
+// epilogue and the row copies below.  More row loaders leave the epilogue too few registers (four: 735 -> 960 us).  All
+// waits are bounded.
 #include "common.cuh"
 #include "tc_ptx.cuh"
 #include "tc_runtime.cuh"

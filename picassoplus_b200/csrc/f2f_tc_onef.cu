@@ -21,6 +21,10 @@
 // The accumulators are added to the CTA's sums in global memory every 4096 faces (the tensor core's adder truncates, see
 // f2f_tc_gfilter.cu) with reductions that nothing waits for; each address has one thread that adds, so the order is fixed.
 // A second kernel adds the chunks in order.  All waits are bounded.
+// Now 685 us for the case above (bf16 1964 -> 372), 2074 for 930 000 faces, 128 -> 128, 25 bases (2524 before; bf16 2335 -> 1490).
+// What bounds it: hand-overs -- a stage without any work takes 490 clocks, with 64 channels 880 of which 384 are products, with
+// 128 channels 1090 (576 products; two operand buffers are what fits beside three accumulators).  Two or four groups on one
+// stage are slower (697 -> 814, 1196 us), two bulk-copy warps the same.
 #include <math.h>
 #include <string.h>
 #include <type_traits>
