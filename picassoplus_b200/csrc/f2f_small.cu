@@ -18,6 +18,9 @@ namespace small {
 
 constexpr int NT = 256;
 constexpr int MAX_C = 4, MAX_F = 32;
+// Samples whose rows are loaded together (1 758 000 faces, 16 bases, 32 outputs, one at a time: forward 279 us, filter gradient 358; two:
+// 244 and 329; four take the filter gradient a block per SM in registers: 249 and 426)
+constexpr int AT = 2;
 
 // floats of an A row: a multiple of four, and 4 (mod 8), so that rows read side by side lie on different banks
 __host__ __device__ __forceinline__ int a_pitch(int F, int C) { return ((F + 3) / 4 * 4 * C) | 4; }
@@ -48,22 +51,28 @@ __device__ __forceinline__ void face_rows(const Params& p, int64_t f0, float* sa
             for (int c = 0; c < C; ++c) a[j][c] = 0.f;
         if (f < p.Nf) {
             const int k0 = f > 0 ? __ldg(p.cum + f - 1) : 0, k1 = __ldg(p.cum + f);
-            for (int k = k0; k < k1; ++k) {
-                float b[4], x[C];
-                const float* src = p.bary + (int64_t)k * F + 4 * q;
-                if (vec) {
-                    const float4 v = ldg4(reinterpret_cast<const float4*>(src));
-                    b[0] = v.x; b[1] = v.y; b[2] = v.z; b[3] = v.w;
-                } else {
+            for (int k = k0; k < k1; k += AT) {                    // the rows of AT samples are on their way together
+                float b[AT][4], x[AT][C];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) b[j] = 4 * q + j < F ? __ldg(src + j) : 0.f;
+                for (int t = 0; t < AT; ++t) {
+                    const bool on = k + t < k1;
+                    const float* src = p.bary + (int64_t)(k + t) * F + 4 * q;
+                    if (vec) {
+                        const float4 v = on ? ldg4(reinterpret_cast<const float4*>(src)) : zero4();
+                        b[t][0] = v.x; b[t][1] = v.y; b[t][2] = v.z; b[t][3] = v.w;
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) b[t][j] = on && 4 * q + j < F ? __ldg(src + j) : 0.f;
+                    }
+#pragma unroll
+                    for (int c = 0; c < C; ++c) x[t][c] = on ? __ldg(p.in + (int64_t)(k + t) * C + c) : 0.f;
                 }
 #pragma unroll
-                for (int c = 0; c < C; ++c) x[c] = __ldg(p.in + (int64_t)k * C + c);
+                for (int t = 0; t < AT; ++t)
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
+                    for (int j = 0; j < 4; ++j)
 #pragma unroll
-                    for (int c = 0; c < C; ++c) a[j][c] = fmaf(b[j], x[c], a[j][c]);
+                        for (int c = 0; c < C; ++c) a[j][c] = fmaf(b[t][j], x[t][c], a[j][c]);
             }
             const float w = k1 > k0 ? 1.f / (float)(k1 - k0) : 0.f;
 #pragma unroll
