@@ -11,6 +11,7 @@
 
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
@@ -53,9 +54,12 @@ bool misaligned(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_pt
 // boundary (a slice of a larger tensor) is moved to fresh storage.
 Tensor aligned(const Tensor& t) { return misaligned(t) ? t.clone() : t; }
 
-// Everything a call needs from the current device: guard, stream, allocation.
+// Everything a call needs from the current device: guard, stream, allocation.  Autocast stays out: AutoDispatchBelow... leaves its
+// keys on, and a product that torch rounds to half precision under it would come back as half the bytes that the kernels behind
+// it read and write.  The kernels choose their operands' precision themselves.
 struct Scope {
     c10::cuda::CUDAGuard guard;
+    c10::impl::ExcludeDispatchKeyGuard no_autocast{c10::DispatchKey::AutocastCUDA};
     at::TensorOptions f32;
     void* stream;
     explicit Scope(const Tensor& t)
@@ -65,9 +69,17 @@ struct Scope {
     Tensor bytes(size_t n) const { return at::empty({(int64_t)(n > 0 ? n : 1)}, f32.dtype(at::kByte)); }
 };
 
-const float* fp(const Tensor& t) { return t.defined() ? static_cast<const float*>(t.data_ptr()) : nullptr; }
-float* fpm(const Tensor& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
-const int32_t* ip(const Tensor& t) { return t.defined() ? static_cast<const int32_t*>(t.data_ptr()) : nullptr; }
+// Addresses for a kernel: whatever way a tensor came in, one of another type, device or layout goes no further
+void* address(const Tensor& t, at::ScalarType type) {
+    if (!t.defined()) return nullptr;
+    if (t.scalar_type() != type || !t.is_cuda() || t.get_device() != c10::cuda::current_device() || !t.is_contiguous())
+        fail(std::string("expected a contiguous ") + c10::toString(type) + " tensor on the call's CUDA device, got " +
+             c10::toString(t.scalar_type()) + " on " + t.device().str());
+    return t.data_ptr();
+}
+const float* fp(const Tensor& t) { return static_cast<const float*>(address(t, at::kFloat)); }
+float* fpm(const Tensor& t) { return static_cast<float*>(address(t, at::kFloat)); }
+const int32_t* ip(const Tensor& t) { return static_cast<const int32_t*>(address(t, at::kInt)); }
 Tensor or_undefined(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
 SavedVariable keep(const Tensor& t) { return SavedVariable(t, /*is_output=*/false); }
 
@@ -482,7 +494,7 @@ struct Tail {
 // Mean and 1 / deviation of every channel
 struct NormStats { Tensor mean, invstd; };
 void bump(const Tensor& t) { if (t.defined()) t.unsafeGetTensorImpl()->bump_version(); }
-int64_t* counter(const Tensor& t) { return t.defined() ? static_cast<int64_t*>(t.data_ptr()) : nullptr; }
+int64_t* counter(const Tensor& t) { return static_cast<int64_t*>(address(t, at::kLong)); }
 
 // Statistics of activated rows with torch's own reduction (norm.cu says why); it moves the running statistics too.
 NormStats batch_stats(const Scope& s, const Tail& t, const Tensor& act) {
@@ -899,9 +911,9 @@ Tensor f2f_layer(const Tensor& input, const Tensor& filter, const Tensor& bary, 
         node = node_for<F2FLayer>(input, filter, bias0, t.gamma, t.beta);
     at::AutoDispatchBelowADInplaceOrView below;
     check_f2f(input, filter, bary);
+    Scope s(input);
     const Tensor cum = at::cumsum(counts, 0, at::kInt), bias = flat(bias0);
     check(cum, "num_texture", 1, at::kInt);
-    Scope s(input);
     Tensor act = f2f_forward(s, aligned(input), filter, bary, cum, precision), out;
     const NormStats st = bias_act_norm(s, t, act, bias, out);
     if (node) {
