@@ -647,6 +647,9 @@ static int launch_bwd_coop(int64_t Np, int64_t Mp, int64_t Nout, int nb, int F, 
                            cudaStream_t stream) {
     if (Np > 0) {
         const int nlong = Nout > LONG_ROW ? long_blocks(Np) : 0;
+        // beside the 17 KB that the long rows are staged in, a filter table above 31 KB needs more than the default 48 KB
+        PB_CUDA(cudaFuncSetAttribute(conv_bwd_input_coop_kernel<TT, CV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(sizeof(float4) * F * CV)));
         PB_LAUNCH("pcloud_conv_bwd_input", (conv_bwd_input_coop_kernel<TT, CV>), nlong + persistent_blocks(Np * Lanes<CV>::LN, 256, 8), 256,
                   sizeof(float4) * F * CV, stream, Np, Mp, F, T, (const float4*)gout, (const float4*)filter, nnCount, nnIndex, bin,
                   coeff, rowptr, members, nlong, (float4*)gin);
@@ -738,6 +741,8 @@ int pb200_pcloud_conv3d_backward(int64_t Np, int64_t Mp, int64_t Nout, int F, in
         }
         if (Np > 0) {
             const int nlong = Nout > LONG_ROW ? long_blocks(Np) : 0;
+            PB_CUDA(cudaFuncSetAttribute(conv_bwd_input_vec_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(sizeof(float) * F * C)));
             PB_LAUNCH("pcloud_conv_bwd_input", conv_bwd_input_vec_kernel, nlong + persistent_blocks(Np * CV, 256, 8), 256,
                       sizeof(float) * F * C, stream, Np, Mp, F, CV, T, (const float4*)gradOutput, (const float4*)filter, nnCount,
                       nnIndex, binIndex, binCoeff, rowptr_in, members_in, nlong, (float4*)gradInput);

@@ -60,6 +60,39 @@ def test_matches_oracle_and_reference(Np, Mp, knn, F, C, r, T, shuffle):
         assert rel_err(out, r_out) <= TOL and rel_err(gin, r_gin) <= TOL and rel_err(gf, r_gf) <= TOL
 
 
+@pytest.mark.parametrize("F,C,T", [
+    (33, 256, 3), (33, 256, 0),          # vector kernels, a filter table of 34 KB beside the staged pairs
+    (65, 128, 0), (65, 128, 3),          # cooperative kernels, 33 KB
+    (12, 1024, 0),                       # the largest table and the widest rows: 48 KB, one group of lanes per block
+    (17, 64, 3), (17, 64, 0), (9, 32, 2), (9, 48, 3),
+    (9, 128, 5), (9, 20, 4),             # more bins than are staged
+])
+def test_input_points_with_many_pairs(F, C, T):
+    """Padded neighbour lists name a few input points over and over: rows of 64 (walked with the others), 65, 256, 257, 300 and
+    thousands of pairs, several of them in one block's range of points, one in another's."""
+    from oracle import mesh_oracle as mo
+    from picassoplus_b200.point.pi_modules import conv3d
+    d = pcloud_inputs(2500, 600, 16, F, C, 1, T, seed=29, shuffle=True)
+    n = d["nn_index"].shape[0]
+    at = 0
+    for point, pairs in ((0, 1500), (7, 64), (8, 65), (9, 256), (10, 257), (1023, 300), (2047, 100), (2499, 700)):
+        d["nn_index"][:, 1][d["nn_index"][:, 1] == point] = 3
+        d["nn_index"][at:at + pairs, 1] = point
+        at += pairs
+    assert at < n
+    dbl = lambda t: None if t is None else t.double()                               # noqa: E731
+    want_in, want_filter = mo.pcloud_conv3d_backward(d["g_out"].double(), d["x"].double(), d["filt"].double(), d["nn_count"],
+                                                     d["nn_index"], d["bin_index"], dbl(d["bin_coeff"]))
+    c = _dev(d)
+    args = [c[k] for k in ("g_out", "x", "filt", "nn_count", "nn_index", "bin_index", "bin_coeff")]
+    gin, gf = conv3d._backward(*args)
+    assert rel_err(gin, want_in) <= 1e-5 and rel_err(gf, want_filter) <= 1e-5
+    for point in (0, 8, 257, 2499):
+        assert rel_err(gin[point], want_in[point]) <= 1e-4
+    again = conv3d._backward(*args)
+    assert torch.equal(again[0], gin) and torch.equal(again[1], gf)
+
+
 @pytest.mark.parametrize("name", sorted(PCLOUD_GOLDEN_CASES))
 def test_against_committed_reference_fixtures(name):
     from picassoplus_b200.point.pi_modules import conv3d
