@@ -1238,20 +1238,53 @@ Tensor on_device(const std::vector<int64_t>& values, const Tensor& like) {
     return at::tensor(values, at::TensorOptions().dtype(at::kInt)).to(like.device());
 }
 std::vector<int64_t> on_host(const Tensor& t) {
-    const Tensor h = t.cpu();
+    const Tensor h = t.cpu().contiguous();
     const int32_t* p = h.data_ptr<int32_t>();
     return std::vector<int64_t>(p, p + h.numel());
 }
 
 // The pass loop of mesh_decimation (picasso/mesh/pi_modules/decimate.py:5-48) with one synchronisation per pass: the host
 // reads the samples' new sizes, which it needs to allocate the result, and decides on the next pass by them.
-// nv_host / mf_host / target_host: the samples' sizes where the caller knows them already (empty: read here).
+// target_in: vertices to keep, one number per sample or one for all.  Without it the sizes are known to the caller already:
+// nv_host / mf_host / target_host are the values of nv_in / mf_in and the target.
 std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, std::vector<int64_t>, std::vector<int64_t>>
 mesh_decimation(const Tensor& vertex_in, const Tensor& face_in, const Tensor& geometry_in, const Tensor& nv_in, const Tensor& mf_in,
                 const OptTensor& target_in, bool use_area, double wgt_bnd, std::vector<int64_t> nv_host, std::vector<int64_t> mf_host,
                 std::vector<int64_t> target_host) {
     c10::InferenceMode inference(false);
     at::NoGradGuard no_grad;
+    if (nv_in.dim() != 1 || mf_in.dim() != 1) fail("nvIn and mfIn must have dimension of 1");
+    const int64_t B = nv_in.size(0);
+    if (target_in.has_value()) {
+        const Tensor& t = *target_in;
+        if (t.dim() > 1) fail("the vertices to keep must have dimension of 1");
+        if (t.dim() == 1 && t.device() != nv_in.device()) fail("the vertices to keep must be on the device of nvIn");
+        if (nv_in.device() == mf_in.device() && nv_in.device() == t.device()) {                   // one copy to the host
+            const std::vector<int64_t> all = on_host(at::cat({nv_in.to(at::kInt), mf_in.to(at::kInt), t.reshape({-1}).to(at::kInt)}));
+            nv_host.assign(all.begin(), all.begin() + B);
+            mf_host.assign(all.begin() + B, all.begin() + B + mf_in.size(0));
+            target_host.assign(all.begin() + B + mf_in.size(0), all.end());
+        } else {
+            nv_host = on_host(nv_in.to(at::kInt));
+            mf_host = on_host(mf_in.to(at::kInt));
+            target_host = on_host(t.reshape({-1}).to(at::kInt));
+        }
+    }
+    if (target_host.size() == 1) target_host.assign(B, target_host[0]);
+    if ((int64_t)nv_host.size() != B || (int64_t)target_host.size() != B)
+        fail("nvIn and the vertices to keep must have one entry per sample");
+    auto sum = [](const std::vector<int64_t>& v) { int64_t t = 0; for (int64_t x : v) t += x; return t; };
+    auto more = [&] { for (int64_t k = 0; k < B; ++k) if (nv_host[k] > target_host[k]) return true; return false; };
+    Tensor rep, map;
+    if (!more()) {
+        const auto i32 = vertex_in.options().dtype(at::kInt).requires_grad(false);
+        rep = at::zeros({vertex_in.size(0)}, i32);
+        map = at::arange(vertex_in.size(0), i32);
+        return {vertex_in, face_in, geometry_in, nv_in, mf_in, rep, map, nv_host, mf_host};
+    }
+    if (mf_in.size(0) != B || (int64_t)mf_host.size() != B) fail("mfIn must have one entry per sample");
+    for (int64_t k = 0; k < B; ++k)
+        if (nv_host[k] < 0 || mf_host[k] < 0) fail("mesh_simplify: nvIn / mfIn must not be negative");
     Tensor vertex = vertex_in.contiguous(), face = face_in.contiguous(), geometry = geometry_in.contiguous();
     check(vertex, "vertexIn", 2, at::kFloat);
     check(face, "faceIn", 2, at::kInt);
@@ -1259,22 +1292,16 @@ mesh_decimation(const Tensor& vertex_in, const Tensor& face_in, const Tensor& ge
     if (vertex.size(1) < 3) fail("The shape of input vertex should be (Nv, 3+)).");
     if (face.size(1) != 3) fail("The shape of input face should be (Nf, 3)).");
     if (geometry.size(0) != face.size(0) || geometry.size(1) != 5) fail("The shape of input face normals should be (Nf, 5)).");
+    for (const Tensor& t : {face, geometry, nv_in, mf_in})
+        if (t.device() != vertex.device()) fail("vertexIn, faceIn, planeIn, nvIn and mfIn must be on one CUDA device");
+    if (sum(nv_host) != vertex.size(0) || sum(mf_host) != face.size(0))
+        fail("mesh_simplify: nvIn / mfIn must be the samples' vertex and face counts");
     Scope s(vertex);
     const auto i32 = s.f32.dtype(at::kInt);
-    const int64_t D = vertex.size(1), B = nv_in.size(0);
-    Tensor nv = nv_in, mf = mf_in, rep, map;
-    if (nv_host.empty()) {
-        const std::vector<int64_t> all = on_host(at::cat({nv_in.to(at::kInt), mf_in.to(at::kInt), target_in.value().to(at::kInt)}));
-        nv_host.assign(all.begin(), all.begin() + B);
-        mf_host.assign(all.begin() + B, all.begin() + 2 * B);
-        target_host.assign(all.begin() + 2 * B, all.end());
-    }
-    auto sum = [](const std::vector<int64_t>& v) { int64_t t = 0; for (int64_t x : v) t += x; return t; };
-    auto more = [&] { for (int64_t k = 0; k < B; ++k) if (nv_host[k] > target_host[k]) return true; return false; };
-    const bool any = more();
-    if (any && (sum(nv_host) != vertex.size(0) || sum(mf_host) != face.size(0)))
-        fail("mesh_simplify: nvIn / mfIn must be the samples' vertex and face counts");
-    const Tensor target = target_in.has_value() ? target_in->to(vertex.device(), at::kInt).contiguous() : on_device(target_host, vertex);
+    const int64_t D = vertex.size(1);
+    Tensor nv = nv_in, mf = mf_in;
+    const bool there = target_in.has_value() && target_in->dim() == 1 && target_in->size(0) == B;
+    const Tensor target = there ? target_in->to(at::kInt).contiguous() : on_device(target_host, vertex);
     while (more()) {
         const int64_t Nv = vertex.size(0), Nf = face.size(0);
         const Tensor sizes = at::empty({2 * B + 1}, i32), vt_replace = at::empty({Nv}, i32), vt_map = at::empty({Nv}, i32);
@@ -1322,7 +1349,7 @@ mesh_decimation(const Tensor& vertex_in, const Tensor& face_in, const Tensor& ge
         nv = sizes.narrow(0, 0, B);
         mf = sizes.narrow(0, B, B);
     }
-    if (!rep.defined()) {
+    if (!rep.defined()) {                  // not even the first pass found an edge
         rep = at::zeros({vertex.size(0)}, i32);
         map = at::arange(vertex.size(0), i32);
         return {vertex_in, face_in, geometry_in, nv, mf, rep, map, nv_host, mf_host};

@@ -136,6 +136,10 @@ def combine_clusters_(repA, mapA, repB, mapB):
 def mesh_decimation_(vertexIn, faceIn, geometryIn, nvIn, mfIn, nvOut, useArea=True, wgtBnd=5):
     '''Decimates every sample of the batch to nvOut vertices (decimate.py:5-48): passes of `simplify`
     until every sample has shed its vertices, clusters merged across the passes; the loop runs natively with one
-    synchronisation per pass.
+    synchronisation per pass.  nvOut: one number per sample, or one for all of them.
     Returns vertexOut, faceOut, geometryOut, nvOut, mfOut, vtReplace, vtMap.'''
+    if not isinstance(nvOut, torch.Tensor):
+        nvOut = torch.tensor(nvOut)
+    if nvOut.is_floating_point():
+        nvOut = nvOut.ceil()             # whole vertices are removed: those above the number, rounded down
     return _lib.ops.mesh_decimation(vertexIn, faceIn, geometryIn, nvIn, mfIn, nvOut, bool(useArea), float(wgtBnd), [], [], [])[:7]
