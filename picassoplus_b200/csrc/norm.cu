@@ -360,10 +360,12 @@ segment_pieces_kernel(int64_t N, int C, int B, const int64_t* __restrict__ ends,
 }
 
 __global__ void __launch_bounds__(32 * 8)
-segment_finish_kernel(int C, int B, const int64_t* __restrict__ ends, const float* __restrict__ pieces, float* __restrict__ out) {
+segment_finish_kernel(int64_t N, int C, int B, const int64_t* __restrict__ ends, const float* __restrict__ pieces, float* __restrict__ out) {
     __shared__ float red[8][32];
     const int s = blockIdx.x, c = blockIdx.y * 32 + threadIdx.x;
-    const int64_t b = s > 0 ? ends[s - 1] : 0, e = ends[s];
+    // with deferred validation the ends may be anything yet: pieces exist for rows 0 .. N - 1 only
+    const int64_t before = s > 0 ? ends[s - 1] : 0, end = ends[s];
+    const int64_t b = before < 0 ? 0 : before < N ? before : N, e = end < 0 ? 0 : end < N ? end : N;
     float a = 0.f;
     if (c < C && e > b)
         for (int64_t k = b / SEG_ROWS + threadIdx.y; k <= (e - 1) / SEG_ROWS; k += 8) a += pieces[(k + s) * C + c];
@@ -371,7 +373,7 @@ segment_finish_kernel(int C, int B, const int64_t* __restrict__ ends, const floa
     __syncthreads();
     if (threadIdx.y == 0 && c < C) {
         for (int w = 1; w < 8; ++w) a += red[w][threadIdx.x];
-        out[(int64_t)s * C + c] = a / (float)(e - b);           // a sample without rows: 0 / 0, as the mean of nothing is
+        out[(int64_t)s * C + c] = a / (float)(end - before);           // a sample without rows: 0 / 0, as the mean of nothing is
     }
 }
 
@@ -490,7 +492,7 @@ int pb200_segment_mean(int64_t N, int B, int C, const float* rows, const int64_t
     if (N > 0)
         PB_LAUNCH("segment_pieces", segment_pieces_kernel, dim3((unsigned)ceil_div(N, SEG_ROWS), (unsigned)ceil_div(C, 32)), 256, 0, stream,
                   N, C, B, ends, rows, pieces);
-    PB_LAUNCH("segment_finish", segment_finish_kernel, dim3((unsigned)B, (unsigned)ceil_div(C, 32)), dim3(32, 8), 0, stream, C, B, ends,
+    PB_LAUNCH("segment_finish", segment_finish_kernel, dim3((unsigned)B, (unsigned)ceil_div(C, 32)), dim3(32, 8), 0, stream, N, C, B, ends,
               pieces, out);
     return PB200_OK;
 }

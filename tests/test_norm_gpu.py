@@ -96,3 +96,24 @@ def test_global_mean(lengths, C):
     assert rel_err(gx, torch.repeat_interleave(g / nv[:, None], nv.long(), 0)) <= 1e-6
     with pytest.raises(RuntimeError):
         GlobalPool3d("avg")(x, nv + 1)
+
+
+@pytest.mark.parametrize("lengths", [[300, 900, 1200], [100, -4000, 500], [5000000, 1, 1], [-5, 1000, 5]])
+def test_global_mean_of_wrong_counts_with_deferred_validation(lengths):
+    """Counts that do not add up to the rows are reported at the next check; until then nothing behind the rows is read.
+    (Samples in front of the first wrong row keep their mean while the totals rise; a negative count makes the search over them
+    meaningless.)"""
+    from picassoplus_b200 import topology
+    from picassoplus_b200.mesh.layers import GlobalPool3d
+    x = torch.randn(1000, 40, device="cuda").requires_grad_()
+    nv = torch.tensor(lengths, device="cuda", dtype=torch.int32)
+    topology.set_validation("deferred")
+    try:
+        out = GlobalPool3d("avg")(x, nv)
+        torch.autograd.grad(out, x, torch.ones_like(out))
+        if 0 < lengths[0] < 1000 and min(lengths) >= 0:
+            assert rel_err(out[0], x[:lengths[0]].double().mean(0)) <= 1e-5
+        with pytest.raises(RuntimeError, match="add up"):
+            topology.check_deferred()
+    finally:
+        topology.set_validation("sync")
