@@ -1382,7 +1382,7 @@ level_prepare(const Tensor& vertex, const Tensor& face, const OptTensor& vt_map,
 
 // -------------------------------------------------------------------------------------------------- topology cache
 // Structures derived from index tensors (CSRs, sample means, running totals), found again by the tensors they were made
-// from.  An entry is named by kind, addresses and two numbers; it is good while the index tensors' storages are the ones it
+// from.  An entry is named by kind, addresses, row counts, row strides, types and two numbers; it is good while the index tensors' storages are the ones it
 // was made from (weak references: the cache does not keep a batch's tensors alive, and memory that was freed and handed out
 // again is another storage) and their version counters have not moved.  Entries of storages that are gone are dropped at
 // the next insertion: a program that brings a new batch every step holds the structures of the batches it holds, no more.
@@ -1404,7 +1404,7 @@ struct TopologyCache {
         int64_t bytes;
         c10::cuda::CUDAStream stream;
     };
-    using Key = std::array<int64_t, 8>;
+    using Key = std::array<int64_t, 12>;
     struct Hash {
         size_t operator()(const Key& k) const {
             uint64_t h = 0x9e3779b97f4a7c15ull;
@@ -1418,8 +1418,9 @@ struct TopologyCache {
     int64_t bytes = 0, budget = 2ll << 30;
 
     static Key key(int kind, const Tensor& a, const OptTensor& b, int64_t m, int64_t n) {
-        return {kind, a.device().index(), (int64_t)a.data_ptr(), a.size(0), b.has_value() ? (int64_t)b->data_ptr() : -1,
-                b.has_value() ? b->size(0) : -1, m, n};
+        Key k{kind, a.device().index(), (int64_t)a.data_ptr(), a.size(0), a.stride(0), (int64_t)a.scalar_type(), m, n, -1, -1, -1, -1};
+        if (b.has_value()) k[8] = (int64_t)b->data_ptr(), k[9] = b->size(0), k[10] = b->stride(0), k[11] = (int64_t)b->scalar_type();
+        return k;
     }
     void erase(List::iterator it) {
         bytes -= it->second.bytes;

@@ -6,8 +6,8 @@ operator calls per step in the reference's encoder blocks,
 picasso/networks/pi2_blocks.py:88-92), so the CSR is built once per (face, vtMap) pair
 and looked up afterwards.
 
-Cache policy (TopologyCache in csrc/torch_ops.cpp).  An entry is named by the storage of the index
-tensors (device, data pointer, length) and good while those storages live and their version counters
+Cache policy (TopologyCache in csrc/torch_ops.cpp).  An entry is named by the memory of the index
+tensors (device, data pointer, length, stride, type) and good while those storages live and their version counters
 stand still.  A lookup whose versions differ (the tensors were overwritten in place, as a streaming
 loader does with its device buffers) rebuilds the structure and REPLACES the entry, so stale entries
 never pile up; entries whose tensors are gone are dropped at the next insertion, so neither do those of
@@ -343,7 +343,7 @@ class SampleEnds:
 def sample_ends(counts: torch.Tensor, n_rows: int) -> torch.Tensor:
     """Cached running totals of the samples' row counts; same cache, budget and validation modes as vertex_csr.  They must
     add up to n_rows."""
-    hit = _ops.cache_find(_SAMPLES, counts, None, n_rows, counts.element_size())
+    hit = _ops.cache_find(_SAMPLES, counts, None, n_rows, 0)
     if hit is not None:
         return hit.ends
     ends = torch.cumsum(counts.detach(), 0, dtype=torch.int64)
@@ -355,7 +355,7 @@ def sample_ends(counts: torch.Tensor, n_rows: int) -> torch.Tensor:
             _deferred.append((bad.to(torch.int32), msg))
     elif bool(bad.item()):
         raise RuntimeError(msg)
-    _store(_SAMPLES, counts, None, n_rows, counts.element_size(), SampleEnds(ends))
+    _store(_SAMPLES, counts, None, n_rows, 0, SampleEnds(ends))
     return ends
 
 

@@ -117,3 +117,27 @@ def test_global_mean_of_wrong_counts_with_deferred_validation(lengths):
             topology.check_deferred()
     finally:
         topology.set_validation("sync")
+
+
+def test_global_mean_of_two_views_of_one_count_table():
+    """Row and column of a table share address, length and storage; so do two types' views of one buffer."""
+    from picassoplus_b200.mesh.layers import GlobalPool3d
+    pool = GlobalPool3d("avg")
+    x = torch.randn(10, 8, device="cuda")
+
+    def want(lengths):
+        return torch.stack([p.mean(0) for p in torch.split(x.double(), lengths)])
+    table = torch.tensor([[3, 5, 2], [2, 1, 1], [5, 1, 1]], device="cuda", dtype=torch.int32)
+    assert rel_err(pool(x, table[0]), want([3, 5, 2])) <= 1e-6
+    assert rel_err(pool(x, table[:, 0]), want([3, 2, 5])) <= 1e-6
+    table = torch.tensor([[3, 5, 2], [2, 1, 1], [4, 1, 1]], device="cuda", dtype=torch.int32)
+    pool(x, table[0])
+    with pytest.raises(RuntimeError, match="add up"):
+        pool(x, table[:, 0])
+    counts = torch.tensor([10, 0, 0], device="cuda", dtype=torch.int64)
+    assert rel_err(pool(x, counts[:1]), want([10])) <= 1e-6
+    assert rel_err(pool(x, counts.view(torch.int32)[:1]), want([10])) <= 1e-6
+    ones = torch.full((5,), 2, device="cuda", dtype=torch.int32)
+    assert rel_err(pool(x, ones), want([2] * 5)) <= 1e-6
+    with pytest.raises(RuntimeError, match="add up"):
+        pool(x, ones.view(torch.float32))
