@@ -9,6 +9,8 @@
 // Functions), backward runs on the engine's thread without the GIL.
 #include <torch/extension.h>
 
+#include <c10/core/Event.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
@@ -1387,7 +1389,8 @@ level_prepare(const Tensor& vertex, const Tensor& face, const OptTensor& vt_map,
 // again is another storage) and their version counters have not moved.  Entries of storages that are gone are dropped at
 // the next insertion: a program that brings a new batch every step holds the structures of the batches it holds, no more.
 // Otherwise least recently used ones go when the bytes exceed the budget.  A structure used on a stream other than the one
-// it was made on is recorded there, so that dropping it is safe at any time.  All calls run under the GIL.
+// it was made on waits there for its kernels and is recorded there, so that dropping it is safe at any time.  One made while a
+// graph is captured exists when that graph has run and is good inside that capture only.  All calls run under the GIL.
 struct TopologyCache {
     struct Source {
         c10::weak_intrusive_ptr<c10::StorageImpl> storage;
@@ -1403,6 +1406,9 @@ struct TopologyCache {
         py::object value;
         int64_t bytes;
         c10::cuda::CUDAStream stream;
+        unsigned long long capture;              // id of the capture it was made in, 0: none
+        c10::Event ready;                        // behind the kernels that make it
+        bool complete = false;                   // seen to have passed
     };
     using Key = std::array<int64_t, 12>;
     struct Hash {
@@ -1413,7 +1419,7 @@ struct TopologyCache {
         }
     };
     using List = std::list<std::pair<Key, Entry>>;
-    List order;                                  // least recently used first
+    List recent;                                 // least recently used first
     std::unordered_map<Key, List::iterator, Hash> at;
     int64_t bytes = 0, budget = 2ll << 30;
 
@@ -1422,18 +1428,42 @@ struct TopologyCache {
         if (b.has_value()) k[8] = (int64_t)b->data_ptr(), k[9] = b->size(0), k[10] = b->stride(0), k[11] = (int64_t)b->scalar_type();
         return k;
     }
+    static unsigned long long capture_id(c10::cuda::CUDAStream stream) {
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        unsigned long long id = 0;
+        C10_CUDA_CHECK(cudaStreamGetCaptureInfo(stream.stream(), &status, &id));
+        return status == cudaStreamCaptureStatusActive ? id : 0;
+    }
+    // orders work on `now` behind the kernels that make e; false: they belong to another capture
+    static bool order(Entry& e, c10::cuda::CUDAStream now) {
+        if (e.capture != 0) {
+            if (capture_id(now) != e.capture) return false;
+            if (now != e.stream) e.ready.block(now.unwrap());
+            return true;
+        }
+        if (now == e.stream || e.complete) return true;
+        c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);     // a capture elsewhere must not mind the query
+        e.complete = e.ready.query();
+        if (!e.complete && capture_id(now) != 0) {       // a captured stream cannot wait for what lies outside: the host does
+            e.ready.synchronize();
+            e.complete = true;
+        }
+        if (!e.complete) e.ready.block(now.unwrap());
+        return true;
+    }
     void erase(List::iterator it) {
         bytes -= it->second.bytes;
         at.erase(it->first);
-        order.erase(it);
+        recent.erase(it);
     }
     Entry* find(const Key& k, const Tensor& a, const OptTensor& b) {
         auto it = at.find(k);
         if (it == at.end()) return nullptr;
         Entry& e = it->second->second;
         if (!e.sources[0].is(a) || (b.has_value() && !e.sources[1].is(*b))) return nullptr;
-        order.splice(order.end(), order, it->second);
         const auto now = c10::cuda::getCurrentCUDAStream(a.device().index());
+        if (!order(e, now)) return nullptr;
+        recent.splice(recent.end(), recent, it->second);
         if (now != e.stream)
             for (const Tensor& t : e.tensors) t.record_stream(now);
         return &e;
@@ -1441,18 +1471,20 @@ struct TopologyCache {
     void put(const Key& k, const Tensor& a, const OptTensor& b, std::vector<Tensor> tensors, py::object value, int64_t size) {
         auto old = at.find(k);
         if (old != at.end()) erase(old->second);
-        for (auto it = order.begin(); it != order.end();) {
+        for (auto it = recent.begin(); it != recent.end();) {
             auto here = it++;
             bool gone = false;
             for (const Source& src : here->second.sources) gone |= src.storage.expired();
             if (gone) erase(here);
         }
         if (budget <= 0) return;
-        Entry e{{Source(a)}, std::move(tensors), std::move(value), size, c10::cuda::getCurrentCUDAStream(a.device().index())};
+        const auto now = c10::cuda::getCurrentCUDAStream(a.device().index());
+        Entry e{{Source(a)}, std::move(tensors), std::move(value), size, now, capture_id(now), c10::Event(c10::DeviceType::CUDA)};
         if (b.has_value()) e.sources.emplace_back(*b);
-        at[k] = order.insert(order.end(), {k, std::move(e)});
+        e.ready.record(now.unwrap());
+        at[k] = recent.insert(recent.end(), {k, std::move(e)});
         bytes += size;
-        while (!order.empty() && bytes > budget) erase(order.begin());
+        while (!recent.empty() && bytes > budget) erase(recent.begin());
     }
 };
 TopologyCache& cache() {
@@ -1470,12 +1502,12 @@ void cache_put(int kind, const Tensor& a, const OptTensor& b, int64_t m, int64_t
 void cache_budget(int64_t n) {
     TopologyCache& c = cache();
     c.budget = n;
-    while (!c.order.empty() && c.bytes > c.budget) c.erase(c.order.begin());
+    while (!c.recent.empty() && c.bytes > c.budget) c.erase(c.recent.begin());
 }
-py::tuple cache_stats() { return py::make_tuple(cache().order.size(), cache().bytes, cache().budget); }
+py::tuple cache_stats() { return py::make_tuple(cache().recent.size(), cache().bytes, cache().budget); }
 void cache_clear() {
     cache().at.clear();
-    cache().order.clear();
+    cache().recent.clear();
     cache().bytes = 0;
 }
 
