@@ -1363,6 +1363,7 @@ mesh_decimation(const Tensor& vertex_in, const Tensor& face_in, const Tensor& ge
 std::tuple<OptTensor, OptTensor, Tensor, Tensor, Tensor, Tensor, Tensor>
 level_prepare(const Tensor& vertex, const Tensor& face, const OptTensor& vt_map, int64_t nv_out, int L, bool orient, bool want_geometry,
               bool want_normals) {
+    c10::InferenceMode inference(false);         // the structure is kept (topology.py)
     at::NoGradGuard no_grad;
     Scope s(face);
     const auto i32 = s.f32.dtype(at::kInt);

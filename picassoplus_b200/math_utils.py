@@ -36,7 +36,8 @@ def corner_basis(L: int, device) -> torch.Tensor:
     handed out, so every stream may read it."""
     table = _corners.get((L, device))
     if table is None:
-        table = sph_harm_coeff(L, torch.eye(3, device=device))
+        with torch.inference_mode(False):                 # autograd graphs of later calls keep it
+            table = sph_harm_coeff(L, torch.eye(3, device=device))
         if torch.cuda.is_current_stream_capturing():      # memory of a graph's pool: good for this graph only
             return table
         torch.cuda.current_stream(device).synchronize()

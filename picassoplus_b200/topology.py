@@ -22,6 +22,10 @@ per cache miss, which also answers whether `vtMap` is the identity) and a bad in
 RuntimeError.  `set_validation("deferred")` removes that synchronisation: status words are
 kept and `check_deferred()` reads them all at a point where the caller synchronises anyway
 (the end of a step).  Bad indices are never dereferenced in either mode.
+
+Streams and modes.  A structure found on another stream than the one that made it is waited for there; one made inside a
+graph capture is found inside that capture only.  Structures outlive the call that makes them and end up in autograd
+graphs, so they are ordinary tensors also when that call runs under torch.inference_mode.
 """
 from __future__ import annotations
 
@@ -112,7 +116,7 @@ def _bad_index_message(nv_in, nv_out):
 def build_vertex_csr(face: torch.Tensor, vt_map: Optional[torch.Tensor], nv_in: int, nv_out: int) -> VertexCSR:
     """Uncached build.  Validates every index: in 'sync' mode a bad one raises RuntimeError here
     (one device synchronisation), in 'deferred' mode at the next check_deferred()."""
-    with torch.cuda.device(face.device):
+    with torch.inference_mode(False), torch.cuda.device(face.device):
         rowptr, entries, status = _launch_build(face, vt_map, nv_in, nv_out)
         if _validation == "deferred":
             with _lock:
@@ -133,7 +137,7 @@ def vertex_csr(face: torch.Tensor, vt_map: Optional[torch.Tensor], nv_in: int, n
     may_be_identity = vt_map is not None and nv_in == nv_out and vt_map.shape[0] == nv_in
     if may_be_identity and _validation == "sync":
         base = _ops.cache_find(_VERTEX, face, None, nv_in, nv_out)
-        with torch.cuda.device(face.device):
+        with torch.inference_mode(False), torch.cuda.device(face.device):
             ident = (vt_map == torch.arange(nv_in, dtype=vt_map.dtype, device=vt_map.device)).all().to(torch.int32)
             if base is None:
                 # build the identity CSR and test vtMap in the same synchronisation
@@ -203,7 +207,7 @@ def cluster_csr(vt_replace: torch.Tensor, vt_map: torch.Tensor, nv_out: int) -> 
     if hit is not None:
         return hit
     dev = vt_replace.device
-    with torch.cuda.device(dev):
+    with torch.inference_mode(False), torch.cuda.device(dev):
         key = torch.empty(max(nv_in, 1), dtype=torch.int32, device=dev)
         rowptr = torch.empty(nv_out + 1, dtype=torch.int32, device=dev)
         members = torch.empty(max(nv_in, 1), dtype=torch.int32, device=dev)
@@ -243,7 +247,7 @@ def pair_csr(nn_index: torch.Tensor, column: int, n_rows: int) -> PairCSR:
     if hit is not None:
         return hit
     dev = nn_index.device
-    with torch.cuda.device(dev):
+    with torch.inference_mode(False), torch.cuda.device(dev):
         rowptr = torch.empty(n_rows + 1, dtype=torch.int32, device=dev)
         members = torch.empty(max(npairs, 1), dtype=torch.int32, device=dev)
         status = torch.empty(1, dtype=torch.int32, device=dev)
@@ -285,7 +289,7 @@ def pad_rows(rows: torch.Tensor):
         return None
     Fp = _lib.query("pb200_padded_row_floats", F)
     dev = rows.device
-    with torch.cuda.device(dev):
+    with torch.inference_mode(False), torch.cuda.device(dev):
         out = torch.empty(n, Fp, dtype=torch.float32, device=dev)
         _lib.call("pb200_pad_rows", n, F, ptr(rows), ptr(out), stream_ptr(dev))
     return out
@@ -299,13 +303,12 @@ def face_means(sample_rows: torch.Tensor, num_interior: torch.Tensor) -> FaceMea
     if hit is not None:
         return hit
     dev = sample_rows.device
-    with torch.cuda.device(dev):
+    with torch.inference_mode(False), torch.cuda.device(dev):
         check_num_interior(num_interior, nik)
         rows = torch.empty(nf, sample_rows.shape[1], dtype=torch.float32, device=dev)
         _lib.call("pb200_face_mean_rows", nf, nik, sample_rows.shape[1], ptr(sample_rows), ptr(num_interior), ptr(rows),
                   stream_ptr(dev))
-        one_each = torch.arange(1, nf + 1, dtype=torch.int32, device=dev)
-    fm = FaceMeans(rows, one_each)
+        fm = FaceMeans(rows, torch.arange(1, nf + 1, dtype=torch.int32, device=dev))
     _store(_MEANS, sample_rows, num_interior, sample_rows.shape[1], 0, fm)
     return fm
 
@@ -320,12 +323,11 @@ def face_means_sph_harm(L: int, sample_xyz: torch.Tensor, num_interior: torch.Te
     if sample_xyz.dim() != 2 or sample_xyz.shape[1] != 3 or sample_xyz.dtype != torch.float32 or not sample_xyz.is_contiguous():
         raise RuntimeError("sample_xyz must be a contiguous float32 tensor of shape (NiK, 3)")
     dev = sample_xyz.device
-    with torch.cuda.device(dev):
+    with torch.inference_mode(False), torch.cuda.device(dev):
         check_num_interior(num_interior, nik)
         rows = torch.empty(nf, (L + 1) ** 2, dtype=torch.float32, device=dev)
         _lib.call("pb200_face_mean_sph_harm", nf, nik, int(L), ptr(sample_xyz), ptr(num_interior), ptr(rows), stream_ptr(dev))
-        one_each = torch.arange(1, nf + 1, dtype=torch.int32, device=dev)
-    fm = FaceMeans(rows, one_each)
+        fm = FaceMeans(rows, torch.arange(1, nf + 1, dtype=torch.int32, device=dev))
     _store(_MEANS_SH, sample_xyz, num_interior, L, 0, fm)
     return fm
 
@@ -346,9 +348,10 @@ def sample_ends(counts: torch.Tensor, n_rows: int) -> torch.Tensor:
     hit = _ops.cache_find(_SAMPLES, counts, None, n_rows, 0)
     if hit is not None:
         return hit.ends
-    ends = torch.cumsum(counts.detach(), 0, dtype=torch.int64)
-    bad = ends[-1:] != n_rows if counts.shape[0] else torch.full((1,), n_rows != 0, device=counts.device)
-    bad = bad | (counts < 0).any()
+    with torch.inference_mode(False):
+        ends = torch.cumsum(counts.detach(), 0, dtype=torch.int64)
+        bad = ends[-1:] != n_rows if counts.shape[0] else torch.full((1,), n_rows != 0, device=counts.device)
+        bad = bad | (counts < 0).any()
     msg = "the samples' row counts must be non-negative and add up to the number of rows"
     if _validation == "deferred":
         with _lock:
@@ -364,7 +367,7 @@ def check_num_interior(num_interior: torch.Tensor, nik: int) -> None:
     device: raises in 'sync' mode, queues the status word in 'deferred' mode.  The facet2facet
     kernels trust numInterior as the reference does; run this once per array."""
     dev = num_interior.device
-    with torch.cuda.device(dev):
+    with torch.inference_mode(False), torch.cuda.device(dev):
         status = torch.empty(1, dtype=torch.int32, device=dev)
         _lib.call("pb200_check_num_interior", num_interior.shape[0], int(nik), ptr(num_interior), ptr(status),
                   stream_ptr(dev))
