@@ -1457,7 +1457,10 @@ struct TopologyCache {
         at.erase(it->first);
         recent.erase(it);
     }
+    // what inference mode made counts no versions: nothing tells whether it has been overwritten since
+    static bool versioned(const Tensor& a, const OptTensor& b) { return !a.is_inference() && !(b.has_value() && b->is_inference()); }
     Entry* find(const Key& k, const Tensor& a, const OptTensor& b) {
+        if (!versioned(a, b)) return nullptr;
         auto it = at.find(k);
         if (it == at.end()) return nullptr;
         Entry& e = it->second->second;
@@ -1478,7 +1481,7 @@ struct TopologyCache {
             for (const Source& src : here->second.sources) gone |= src.storage.expired();
             if (gone) erase(here);
         }
-        if (budget <= 0) return;
+        if (budget <= 0 || !versioned(a, b)) return;
         const auto now = c10::cuda::getCurrentCUDAStream(a.device().index());
         Entry e{{Source(a)}, std::move(tensors), std::move(value), size, now, capture_id(now), c10::Event(c10::DeviceType::CUDA)};
         if (b.has_value()) e.sources.emplace_back(*b);

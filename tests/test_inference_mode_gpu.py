@@ -1,5 +1,6 @@
-"""Training on meshes that an evaluation under torch.inference_mode has seen first: what is kept between calls (adjacency, clusters,
-groupings, per-face means, basis tables) is made of ordinary tensors and can be saved for a backward pass."""
+"""torch.inference_mode.  Training on meshes that an evaluation under it has seen first: what is kept between calls (adjacency,
+clusters, groupings, per-face means, basis tables) is made of ordinary tensors and can be saved for a backward pass.  Index tensors
+made under it count no versions: their structures are made anew on every call."""
 import pytest
 import torch
 
@@ -54,3 +55,18 @@ def test_training_after_an_evaluation():
     want = torch.autograd.grad(loss, leaves + [d["x"]])
     assert all(torch.equal(a, b) for a, b in zip(got, want))
     assert abs(float(seen) - float(loss.detach())) <= 1e-4 * abs(float(seen)) + 1e-2      # running statistics inside or behind the kernel
+
+
+def test_counts_made_under_inference_mode():
+    from picassoplus_b200 import topology
+    from picassoplus_b200.mesh.layers import GlobalPool3d
+    pool, x = GlobalPool3d("avg"), torch.randn(10, 8, device="cuda")
+    topology.clear_cache()
+    with torch.inference_mode():
+        nv = torch.tensor([4, 6], device="cuda", dtype=torch.int32)
+        first = pool(x, nv)
+        nv.copy_(torch.tensor([3, 7], dtype=torch.int32))
+        second = pool(x, nv)
+    for got, n in ((first, 4), (second, 3), (pool(x, nv), 3)):
+        assert torch.allclose(got, torch.stack([x[:n].mean(0), x[n:].mean(0)]), atol=1e-6)
+    assert topology.cache_stats()["slots"] == 0
