@@ -48,10 +48,10 @@ class SphHarmCoeff(nn.Module):
         return sph_harm_coeff(self.l, cart_coords)
 
 
-def _norm_args(bn, rows, device, needs_grad):
+def _norm_args(bn, rows, device):
     """How the native layers run the module's batch norm: (mode, weight, bias, running mean, running var, batches, momentum,
     eps) with mode 1 = statistics of the batch, 2 = running statistics, or None when the torch module has to run itself (a
-    subclass or a hook, cumulative averages, parameters elsewhere, inference statistics under autograd, a single row)."""
+    subclass or a hook, cumulative averages, parameters elsewhere, a single row)."""
     if (type(bn) is not nn.BatchNorm1d or bn._forward_hooks or bn._forward_pre_hooks or bn._backward_hooks or
             bn._backward_pre_hooks or _has_global_hooks()):
         return None
@@ -66,7 +66,7 @@ def _norm_args(bn, rows, device, needs_grad):
         if rows < 2 or (mean is not None and (bn.momentum is None or batches.device != device or batches.dtype != torch.int64)):
             return None
         return 1, weight, bias, mean, var, batches, bn.momentum or 0.0, bn.eps
-    return None if needs_grad else (2, weight, bias, mean, var, None, 0.0, bn.eps)
+    return 2, weight, bias, mean, var, None, 0.0, bn.eps
 
 
 _has_global_hooks = nn.modules.module._has_any_global_hook
@@ -99,8 +99,12 @@ class _PointwiseTail(nn.Module):
         _norm_args allows it, by the torch module behind it otherwise."""
         norm = _NO_NORM
         if self.with_bn:
-            needs_grad = torch.is_grad_enabled() and (x.requires_grad or any(q.requires_grad for q in self._parameters.values()))
-            norm = _norm_args(self._modules["BatchNorm"], rows, x.device, needs_grad)
+            norm = _norm_args(self._modules["BatchNorm"], rows, x.device)
+            # running statistics inside the kernel have no backward pass: neither for what is in front of them nor for their own
+            # weight and bias, which may train while the layer's weights are frozen
+            if norm is not None and norm[0] == 2 and torch.is_grad_enabled() and \
+                    (x.requires_grad or any(q.requires_grad for q in self.parameters())):
+                norm = None
         relu = self.activation_fn is not None
         if norm is None:
             return self.BatchNorm(run(relu, *_NO_NORM))

@@ -141,3 +141,36 @@ def test_global_mean_of_two_views_of_one_count_table():
     assert rel_err(pool(x, ones), want([2] * 5)) <= 1e-6
     with pytest.raises(RuntimeError, match="add up"):
         pool(x, ones.view(torch.float32))
+
+
+@pytest.mark.parametrize("frozen", [True, False])
+@pytest.mark.parametrize("kind", ["rows", "facet", "mesh", "point"])
+def test_inference_statistics_under_autograd(kind, frozen):
+    """eval() with gradients on, the layer's own weights frozen or not: weight and bias of the batch norm have their gradients."""
+    from cases import conv_inputs, pcloud_inputs
+    from picassoplus_b200.mesh.layers import F2FConv3d, PerItemConv3d, V2FConv3d
+    from picassoplus_b200.point.layers import PCloudConv3d
+    torch.manual_seed(3)
+    on = lambda d: {k: (v.cuda() if isinstance(v, torch.Tensor) else v) for k, v in d.items()}      # noqa: E731
+    d = on(conv_inputs("ico2x3", 16, 1, 16, 24, seed=13))
+    q = on(pcloud_inputs(500, 300, 12, 17, 16, 1, 3, seed=23))
+    m, args = {"rows": (PerItemConv3d(16, 24), (d["x_v"],)), "facet": (F2FConv3d(16, 24, 3), (d["tex"], d["bary"], d["counts"])),
+               "mesh": (V2FConv3d(16, 24, 3), (d["x_v"], d["face"])),
+               "point": (PCloudConv3d(16, 24, 17), (q["x"], q["nn_count"], q["nn_index"], q["bin_index"], q["bin_coeff"]))}[kind]
+    m = m.cuda()
+    for _ in range(2):
+        m(*args)                                            # running statistics
+    m.eval()
+    own = [p for n, p in m.named_parameters() if not n.startswith("BatchNorm")]
+    for p in own:
+        p.requires_grad_(not frozen)
+    bn = m.BatchNorm
+    out = m(*args)
+    g = torch.randn_like(out)
+    grads = torch.autograd.grad(out, [bn.weight, bn.bias] + ([] if frozen else own), g)
+    with torch.no_grad():
+        whole = m(*args)
+    xhat = (out - bn.bias) / bn.weight
+    assert rel_err(whole, out) <= 1e-5
+    assert rel_err(grads[0], (g * xhat).sum(0)) <= 1e-4 and rel_err(grads[1], g.sum(0)) <= 1e-5
+    assert all(bool(t.abs().sum() > 0) for t in grads)
