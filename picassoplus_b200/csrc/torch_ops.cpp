@@ -1534,7 +1534,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("avg_pool", &avg_pool);
     m.def("unpool", &unpool);
     m.def("segment_mean", &segment_mean);
-    m.def("mesh_decimation", &mesh_decimation);
+    // it waits for the GPU once per pass: other threads of the interpreter go on meanwhile
+    m.def("mesh_decimation", &mesh_decimation, py::call_guard<py::gil_scoped_release>());
     m.def("level_prepare", &level_prepare);
     m.def("cache_find", &cache_find);
     m.def("cache_put", &cache_put);

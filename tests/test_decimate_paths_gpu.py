@@ -72,3 +72,27 @@ def test_face_across_samples():
     args = [on(dev, a) for a in (v, f, geo, np.cumsum(nv).astype(np.int32), np.cumsum(mf).astype(np.int32), nv // 2)]
     with pytest.raises(RuntimeError, match="two samples"):
         dm().simplify(*args, True, 1.0)
+
+
+def test_other_threads_go_on_while_the_gpu_is_waited_for():
+    """A loader thread prepares a batch behind a long kernel; the main thread's interpreter runs meanwhile."""
+    import threading
+    import time
+    dev = torch.device("cuda")
+    v, f, geo, nv, mf = batch([synth.icosphere(3)])
+    args = [on(dev, a) for a in (v, f, geo, nv, mf, nv // 4)]
+    want = dm().mesh_decimation_(*args)
+    got, ticks = [], 0
+    torch.cuda.synchronize()
+
+    def load():
+        torch.cuda._sleep(600_000_000)                       # some 0.3 s
+        got.extend(dm().mesh_decimation_(*args))
+    loader = threading.Thread(target=load)
+    loader.start()
+    while loader.is_alive():
+        time.sleep(0.001)
+        ticks += 1
+    loader.join()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    assert ticks >= 50
