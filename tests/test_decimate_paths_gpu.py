@@ -27,6 +27,14 @@ def fan(n):
     return v, np.stack([np.zeros(n, np.int64), 1 + i, 1 + (i + 1) % n], 1)
 
 
+def book(n):
+    """n pages that share one edge: with few vertices to keep, all of them join the cluster of its two ends."""
+    a = np.linspace(0, 2 * np.pi, n, endpoint=False)
+    v = np.concatenate([[[0, 0, 0], [0, 0, 1]], np.stack([np.cos(a), np.sin(a), np.full(n, 0.5)], 1)])
+    i = np.arange(n)
+    return v, np.stack([np.zeros(n, np.int64), np.ones(n, np.int64), 2 + i], 1)
+
+
 # 96 x 96: 16 245 faces, one block's sample at most; 98 x 98: the grid
 @pytest.mark.parametrize("sizes", [(96, 20, 33), (98, 20, 33), (130, 120, 8)])
 @pytest.mark.parametrize("frac", [0.05, 0.3, 0.45, 0.75])
@@ -46,6 +54,33 @@ def test_hub_vertices(n, frac):
     remove = np.floor(nv * frac).astype(np.int32)
     check_against_oracle(torch.device("cuda"), [v, f, geo, np.cumsum(nv).astype(np.int32), np.cumsum(mf).astype(np.int32), remove],
                          False, 1.0)
+
+
+@pytest.mark.parametrize("n,D", [(16, 3), (17, 3), (18, 40), (33, 3), (300, 5), (2000, 3)])
+def test_large_clusters(n, D):
+    """Clusters around and above what a thread sorts by itself, several of them, rows wider than a warp."""
+    v, f, geo, nv, mf = batch([book(n), synth.icosphere(1), book(n + 40), fan(30), book(19)])
+    if D > 3:
+        v = np.concatenate([v, np.random.default_rng(n).standard_normal((v.shape[0], D - 3))], 1).astype(np.float32)
+    remove = (nv - 3).astype(np.int32)
+    got, _ = check_against_oracle(torch.device("cuda"), [v, f, geo, np.cumsum(nv).astype(np.int32), np.cumsum(mf).astype(np.int32),
+                                                         remove], False, 1.0)
+    assert int(got["vtReplace"].max()) >= n - 3
+
+
+def test_time_of_large_clusters_is_not_quadratic():
+    """A cluster of 3000: some 0.1 s where a thread walks the whole list for every member."""
+    import time
+    dev = torch.device("cuda")
+    v, f, geo, nv, mf = batch([book(3000)])
+    args = [on(dev, a) for a in (v, f, geo, nv, mf, (nv - 3).astype(np.int32))]
+    best = 1e9
+    for _ in range(4):
+        t0 = time.perf_counter()
+        dm().simplify(*args, False, 1.0)
+        torch.cuda.synchronize()
+        best = min(best, time.perf_counter() - t0)
+    assert best < 0.15
 
 
 @pytest.mark.parametrize("sizes,stride", [((40, 30), 4), ((110,), 16)])
