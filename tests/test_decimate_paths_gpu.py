@@ -47,7 +47,7 @@ def test_samples_and_grid(sizes, frac):
                          True, 5.0)
 
 
-@pytest.mark.parametrize("n", [15, 16, 17, 33, 500])
+@pytest.mark.parametrize("n", [15, 16, 17, 33, 500, 2500])
 @pytest.mark.parametrize("frac", [0.2, 0.8])
 def test_hub_vertices(n, frac):
     v, f, geo, nv, mf = batch([fan(n), fan(7), synth.icosphere(1)])
@@ -56,7 +56,7 @@ def test_hub_vertices(n, frac):
                          False, 1.0)
 
 
-@pytest.mark.parametrize("n,D", [(16, 3), (17, 3), (18, 40), (33, 3), (300, 5), (2000, 3)])
+@pytest.mark.parametrize("n,D", [(16, 3), (17, 3), (18, 40), (33, 3), (300, 5), (2000, 3), (20000, 3)])
 def test_large_clusters(n, D):
     """Clusters around and above what a thread sorts by itself, several of them, rows wider than a warp."""
     v, f, geo, nv, mf = batch([book(n), synth.icosphere(1), book(n + 40), fan(30), book(19)])
@@ -68,19 +68,18 @@ def test_large_clusters(n, D):
     assert int(got["vtReplace"].max()) >= n - 3
 
 
-def test_time_of_large_clusters_is_not_quadratic():
-    """A cluster of 3000: some 0.1 s where a thread walks the whole list for every member."""
+@pytest.mark.parametrize("mesh,keep", [(book, 3), (fan, 100000)])
+def test_time_of_large_clusters_and_hubs_is_not_quadratic(mesh, keep):
+    """200 000 pages of a book, a fan of 200 000 triangles: some 0.1 s where the work grows with the lists, minutes with their square."""
     import time
     dev = torch.device("cuda")
-    v, f, geo, nv, mf = batch([book(3000)])
-    args = [on(dev, a) for a in (v, f, geo, nv, mf, (nv - 3).astype(np.int32))]
-    best = 1e9
-    for _ in range(4):
+    for n in (2000, 200000):
+        v, f, geo, nv, mf = batch([mesh(n)])
+        args = [on(dev, a) for a in (v, f, geo, nv, mf, (nv - min(keep, n // 2)).astype(np.int32))]
         t0 = time.perf_counter()
         dm().simplify(*args, False, 1.0)
         torch.cuda.synchronize()
-        best = min(best, time.perf_counter() - t0)
-    assert best < 0.15
+        assert time.perf_counter() - t0 < (0.25 if n == 2000 else 3)
 
 
 @pytest.mark.parametrize("sizes,stride", [((40, 30), 4), ((110,), 16)])
