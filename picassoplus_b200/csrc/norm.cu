@@ -39,6 +39,10 @@ template <int V> __device__ __forceinline__ void store(float* p, const Vec<V>& x
     else *p = x.v[0];
 }
 
+// ReLU as torch has it: a NaN stays one, forward and backward
+__device__ __forceinline__ float relu_of(float x) { return x > 0.f || x != x ? x : 0.f; }
+__device__ __forceinline__ float relu_grad(float g, float act) { return act <= 0.f ? 0.f : g; }
+
 struct Moments { float n, mean, m2; };
 __device__ __forceinline__ void merge(Moments& a, const Moments& b) {
     const float n = a.n + b.n, d = b.mean - a.mean, f = b.n > 0.f ? __fdividef(b.n, n) : 0.f;      // no branch: loads run ahead
@@ -67,7 +71,7 @@ stats_kernel(int64_t N, int C, float* __restrict__ rows, const float* __restrict
         const int64_t step = (int64_t)gridDim.x * TEAMS;
         auto take = [&](Vec<V> x, int64_t r) {
 #pragma unroll
-            for (int j = 0; j < V; ++j) { x.v[j] += b[j]; if (relu) x.v[j] = fmaxf(x.v[j], 0.f); }
+            for (int j = 0; j < V; ++j) { x.v[j] += b[j]; if (relu) x.v[j] = relu_of(x.v[j]); }
             store<V>(rows + r * C + c, x);
             if (n == 0)
 #pragma unroll
@@ -89,7 +93,7 @@ stats_kernel(int64_t N, int C, float* __restrict__ rows, const float* __restrict
 #pragma unroll
     for (int j = 0; j < V; ++j) {
         Moments m{(float)n, shift[j], 0.f};
-        if (n > 0) { m.mean = shift[j] + s1[j] / (float)n; m.m2 = fmaxf(s2[j] - s1[j] * s1[j] / (float)n, 0.f); }
+        if (n > 0) { m.mean = shift[j] + s1[j] / (float)n; m.m2 = relu_of(s2[j] - s1[j] * s1[j] / (float)n); }    // (a NaN stays one)
         red[team][lane][j] = m;
     }
     __syncthreads();
@@ -275,7 +279,7 @@ bwd_apply_kernel(int64_t N, int C, const float* __restrict__ g, const float* __r
 #pragma unroll
             for (int j = 0; j < V; ++j) {
                 if (BN) d.v[j] = fmaf(s[j], d.v[j], fmaf(a2[j], x.v[j] - m[j], a1[j]));
-                if (relu) d.v[j] = x.v[j] > 0.f ? d.v[j] : 0.f;
+                if (relu) d.v[j] = relu_grad(d.v[j], x.v[j]);
                 sum[j] += d.v[j];
             }
             store<V>(gm + r * C + c, d);

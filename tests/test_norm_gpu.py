@@ -174,3 +174,41 @@ def test_inference_statistics_under_autograd(kind, frozen):
     assert rel_err(whole, out) <= 1e-5
     assert rel_err(grads[0], (g * xhat).sum(0)) <= 1e-4 and rel_err(grads[1], g.sum(0)) <= 1e-5
     assert all(bool(t.abs().sum() > 0) for t in grads)
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("with_bn", [True, False])
+@pytest.mark.parametrize("kind", ["facet", "point"])
+def test_nan_and_infinity_spread_as_in_torch(kind, with_bn, value):
+    """One bad value in the input: the native layer's outputs and gradients are NaN, infinite or finite where those of the separate
+    operators are (ReLU lets a NaN through in both directions)."""
+    from cases import conv_inputs, pcloud_inputs
+    from picassoplus_b200.mesh import layers
+    from picassoplus_b200.point.layers import PCloudConv3d
+    torch.manual_seed(3)
+    on = lambda d: {k: (v.cuda() if isinstance(v, torch.Tensor) else v) for k, v in d.items()}      # noqa: E731
+    if kind == "facet":
+        d = on(conv_inputs("ico2x3", 16, 1, 16, 24, seed=13))
+        x = d["tex"]
+        m, args = layers.F2FConv3d(16, 24, 3, with_bn=with_bn), (d["bary"], d["counts"])
+    else:
+        d = on(pcloud_inputs(500, 300, 12, 17, 16, 1, 3, seed=23))
+        x = d["x"]
+        m, args = PCloudConv3d(16, 24, 17, with_bn=with_bn), tuple(d[k] for k in ("nn_count", "nn_index", "bin_index", "bin_coeff"))
+    m = m.cuda()
+    x[7, 3] = value
+    upstream = torch.randn(args[1 if kind == "facet" else 0].shape[0], 24, device="cuda")    # (of a constant one a batch norm keeps only noise)
+    results = []
+    for native in (True, False):
+        layers.set_fusion(native)
+        try:
+            out = m(x, *args)
+            results.append([out, *torch.autograd.grad(out, [m.biases], upstream)])
+        finally:
+            layers.set_fusion(True)
+    for a, b in zip(*results):
+        assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(torch.isposinf(a), torch.isposinf(b))
+        ok = torch.isfinite(b)
+        assert rel_err(a[ok], b[ok]) <= 1e-4
+    if with_bn:
+        assert bool(torch.isnan(results[0][0]).any())
