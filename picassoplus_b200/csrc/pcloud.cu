@@ -339,7 +339,8 @@ template <int CV> struct Lanes {
 };
 
 // The bins and weights of the pair a lane fetched (TT of 1 or 3), handed to the group's lanes by shuffles.  A bin outside
-// [0, F) becomes bin 0 with weight 0.
+// [0, F) becomes `none` with weight 0: bin 0 where filter rows are read, -1 where gradients are added (a weight of 0 in a real
+// bin is added there like any other: 0 x NaN is NaN).
 template <int TT>
 struct LaneBins {
     int f[TT == 3 ? 3 : 1];
@@ -347,13 +348,13 @@ struct LaneBins {
 };
 
 template <int TT>
-__device__ __forceinline__ void load_bins(LaneBins<TT>& b, bool have, int64_t p, int F, const int32_t* __restrict__ bin,
+__device__ __forceinline__ void load_bins(LaneBins<TT>& b, bool have, int64_t p, int F, int none, const int32_t* __restrict__ bin,
                                           const float* __restrict__ coeff) {
 #pragma unroll
     for (int t = 0; t < (TT == 3 ? 3 : 1); ++t) {
         b.f[t] = have ? __ldg(bin + p * (TT == 3 ? 3 : 1) + t) : -1;
         b.c[t] = TT == 3 ? (have ? __ldg(coeff + p * 3 + t) : 0.f) : 1.f;
-        if ((unsigned)b.f[t] >= (unsigned)F) { b.f[t] = 0; b.c[t] = 0.f; }
+        if ((unsigned)b.f[t] >= (unsigned)F) { b.f[t] = none; b.c[t] = 0.f; }
     }
 }
 
@@ -411,7 +412,7 @@ conv_fwd_coop_kernel(int64_t Np, int64_t Mp, int F, int T, const float4* __restr
                 p_mine = __ldg(members + e + ln);
                 in_mine = __ldg(nnIndex + 2 * (int64_t)p_mine + 1);
             }
-            if constexpr (TT != 0) load_bins<TT>(mybins, have, p_mine, F, bin, coeff);
+            if constexpr (TT != 0) load_bins<TT>(mybins, have, p_mine, F, 0, bin, coeff);
             const int n = e1 - e < LN ? e1 - e : LN;
             for (int j = 0; j < n; j += U) {
                 float4 x[U][VPL];
@@ -470,7 +471,7 @@ conv_bwd_input_coop_kernel(int64_t Np, int64_t Mp, int F, int T, const float4* _
             p_mine = 0, o_mine = -1, rn_mine = 0.f;
             if (have) p_mine = __ldg(members + e);
             if (have) o_mine = __ldg(nnIndex + 2 * (int64_t)p_mine);
-            if constexpr (TT != 0) load_bins<TT>(mybins, have, p_mine, F, bin, coeff);
+            if constexpr (TT != 0) load_bins<TT>(mybins, have, p_mine, F, 0, bin, coeff);
             if (o_mine >= Mp) o_mine = -1;
             if (o_mine >= 0) rn_mine = 1.f / (float)__ldg(nnCount + o_mine);
         };
@@ -550,7 +551,7 @@ conv_bwd_filter_coop_kernel(int64_t Np, int64_t Mp, int64_t Nout, int pairs_per_
             o_mine = __ldg(nnIndex + 2 * (q + cg));
             in_mine = __ldg(nnIndex + 2 * (q + cg) + 1);
         }
-        if constexpr (TT != 0) load_bins<TT>(mybins, have, q + cg, F, bin, coeff);
+        if constexpr (TT != 0) load_bins<TT>(mybins, have, q + cg, F, -1, bin, coeff);
         if (o_mine >= 0 && o_mine < Mp) rn_mine = 1.f / (float)__ldg(nnCount + o_mine);
         const int n = q1 - q < CV ? (int)(q1 - q) : CV;
         for (int j = 0; j < n; j += 4) {
@@ -576,7 +577,7 @@ conv_bwd_filter_coop_kernel(int64_t Np, int64_t Mp, int64_t Nout, int pairs_per_
                     for (int t = 0; t < (TT == 3 ? 3 : 1); ++t) {
                         const int f = __shfl_sync(mask, mybins.f[t], src);
                         const float c = __shfl_sync(mask, mybins.c[t], src);
-                        if (ok[u] && c != 0.f) fma4s(mine[f * CV + cg], c, d);
+                        if (ok[u] && f >= 0) fma4s(mine[f * CV + cg], c, d);
                     }
                 } else if (ok[u]) {
                     const int64_t p = q + j + u;

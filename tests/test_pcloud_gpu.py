@@ -93,6 +93,26 @@ def test_input_points_with_many_pairs(F, C, T):
     assert torch.equal(again[0], gin) and torch.equal(again[1], gf)
 
 
+@pytest.mark.parametrize("C", [32, 64, 128, 48])
+@pytest.mark.parametrize("T", [0, 3])
+def test_nan_reaches_every_bin_of_its_pairs(C, T):
+    """A NaN row of the upstream gradient is in the filter gradient of all bins that its pairs name, those of weight 0 among them, and
+    in no other; bins outside the table take no part."""
+    from picassoplus_b200.point.pi_modules import conv3d
+    d = pcloud_inputs(400, 200, 12, 17, C, 1, T, seed=31)
+    if T:
+        d["bin_coeff"][::2, 1] = 0
+    d["bin_index"].view(-1)[::7] = 17
+    d["bin_index"].view(-1)[3::7] = -1
+    row = int(d["nn_index"][40, 0])
+    d["g_out"][row] = float("nan")
+    named = d["bin_index"][d["nn_index"][:, 0] == row].flatten()
+    named = set(int(b) for b in named if 0 <= b < 17)
+    c = _dev(d)
+    _, gf = conv3d._backward(*[c[k] for k in ("g_out", "x", "filt", "nn_count", "nn_index", "bin_index", "bin_coeff")])
+    assert len(named) < 17 and set(torch.isnan(gf).flatten(1).any(1).nonzero().flatten().tolist()) == named
+
+
 @pytest.mark.parametrize("name", sorted(PCLOUD_GOLDEN_CASES))
 def test_against_committed_reference_fixtures(name):
     from picassoplus_b200.point.pi_modules import conv3d
