@@ -95,12 +95,14 @@ def facet2facet_shared_rows(face_rows, filter, bary_sh, cum):
     bary_sh: the (NiK, F) sample weights, or their per-face means as topology.face_means / face_means_sph_harm
     return them (then cum is not looked at)."""
     fm = bary_sh if isinstance(bary_sh, FaceMeans) else face_means(bary_sh, cum)
+    if not _lib.native_calls():                   # the general operator over one sample per face
+        return conv3d.f2f_Function.apply(face_rows.contiguous(), filter.contiguous(), fm.rows, fm.one_each)
     return _lib.ops.facet2facet_shared_rows(face_rows, filter, fm.rows, fm.one_each, fm.rows_padded, conv3d._f2f_precision)
 
 
 def conv_block(x, Wv, Wf, Wo, face, cum, bary_sh, coeff, nf_count, vt_map, sh_eye):
     """One native autograd node for the three operators: forward and backward run without the interpreter."""
-    if sh_eye.requires_grad:                      # its gradient comes from the product with Wv: operator by operator
+    if sh_eye.requires_grad or not _lib.native_calls():      # (its gradient comes from the product with Wv) operator by operator
         y = conv3d.vertex2facet(x, (sh_eye @ Wv).reshape(3, x.shape[1], 1), face)
         z = facet2facet_shared_rows(y, Wf, bary_sh, cum)
         return conv3d.facet2vertex(z, Wo, coeff, face, nf_count, vt_map)

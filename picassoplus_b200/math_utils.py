@@ -36,8 +36,13 @@ def corner_basis(L: int, device) -> torch.Tensor:
     handed out, so every stream may read it."""
     table = _corners.get((L, device))
     if table is None:
-        with torch.inference_mode(False):                 # autograd graphs of later calls keep it
-            table = sph_harm_coeff(L, torch.eye(3, device=device))
+        tracer = torch._C._get_tracing_state()
+        torch._C._set_tracing_state(None)                 # a constant to a tracer, not the steps that make it
+        try:
+            with torch.inference_mode(False):             # autograd graphs of later calls keep it
+                table = sph_harm_coeff(L, torch.eye(3, device=device))
+        finally:
+            torch._C._set_tracing_state(tracer)
         if torch.cuda.is_current_stream_capturing():      # memory of a graph's pool: good for this graph only
             return table
         torch.cuda.current_stream(device).synchronize()

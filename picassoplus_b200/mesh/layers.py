@@ -92,7 +92,7 @@ class _PointwiseTail(nn.Module):
         return x
 
     def _fusable(self, x, channels, multiplier):
-        return _fusion and fused.eligible(x, channels, multiplier, self.activation_fn)
+        return _fusion and fused.eligible(x, channels, multiplier, self.activation_fn) and _lib.native_calls()
 
     def _native(self, rows, x, run):
         """run(relu, norm mode, norm arrays ..., precision) = the whole layer as one native call; batch norm included where
@@ -127,7 +127,8 @@ class F2FConv3d(_PointwiseTail):
     def forward(self, input_texture, bary_coeff, num_texture):
         assert self.in_channels == input_texture.shape[-1]
         assert self.num_basis == bary_coeff.shape[-1]
-        if input_texture.is_cuda and _fusion and _plain_activation(self.activation_fn) and num_texture.shape[0] > 0:
+        if (input_texture.is_cuda and _fusion and _plain_activation(self.activation_fn) and num_texture.shape[0] > 0 and
+                _lib.native_calls()):
             bary_coeff.requires_grad = False
             return self._native(num_texture.shape[0], input_texture, lambda *tail: _lib.ops.f2f_layer(
                 input_texture, self.weights, bary_coeff, num_texture, self.biases, *tail, conv3d._f2f_precision))
@@ -256,7 +257,8 @@ class GlobalPool3d(nn.Module):
 
     def forward(self, inputs, nv_in):
         if self.method == 'avg':
-            if inputs.is_cuda and inputs.dtype == torch.float32 and inputs.dim() == 2 and nv_in.dim() == 1 and nv_in.device == inputs.device:
+            if (inputs.is_cuda and inputs.dtype == torch.float32 and inputs.dim() == 2 and nv_in.dim() == 1 and
+                    nv_in.device == inputs.device and _lib.native_calls()):
                 return _lib.ops.segment_mean(inputs.contiguous(), sample_ends(nv_in, inputs.shape[0]))
             return torch.segment_reduce(inputs, 'mean', lengths=nv_in.to(torch.int64))
         if self.method == 'max':

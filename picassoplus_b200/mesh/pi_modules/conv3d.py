@@ -211,7 +211,8 @@ def facet2vertex_backward(grad_output, input, filter, coeff, face, nfCount, vtMa
 
 # ------------------------------------------------------------------ autograd Functions
 # The three calls facet2facet / vertex2facet / facet2vertex go through the native nodes of _torch_ops (same kernels, same
-# gradients, a tenth of the host time); the Function classes are the reference's names for callers that use them directly.
+# gradients, a tenth of the host time); the Function classes are the reference's names for callers that use them directly, and
+# run where native nodes may not (_lib.native_calls).
 class f2f_Function(torch.autograd.Function):
     @staticmethod
     def forward(ctx, textureIn, filter, baryCoeff, numTexture):
@@ -240,6 +241,8 @@ def facet2facet(textureIn, filter, baryCoeff, numTexture):
     Output:
         output:      (concat_NfIn, out_channels) float32
     '''
+    if not _lib.native_calls():
+        return f2f_Function.apply(textureIn, filter, baryCoeff, numTexture)
     baryCoeff.requires_grad = False
     numTexture.requires_grad = False
     return _ops.facet2facet(textureIn, filter, baryCoeff, numTexture, _f2f_precision)
@@ -269,6 +272,8 @@ def vertex2facet(input, filter, face):
     Output:
         output: (concat_NfIn, in_channels*multiplier) float32
     '''
+    if not _lib.native_calls():
+        return v2f_Function.apply(input, filter, face)
     face.requires_grad = False
     rowptr = entries = None
     if torch.is_grad_enabled() and (input.requires_grad or filter.requires_grad):
@@ -308,6 +313,8 @@ def facet2vertex(input, filter, coeff, face, nfCount, vtMap):
     Output:
         output:  (concat_NvOut, in_channels*multiplier) float32
     '''
+    if not _lib.native_calls():
+        return f2v_Function.apply(input, filter, coeff, face, nfCount, vtMap)
     coeff.requires_grad = False
     face.requires_grad = False
     nfCount.requires_grad = False

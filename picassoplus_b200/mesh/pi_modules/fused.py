@@ -81,18 +81,29 @@ def rows_layer(rows, weights, biases, tail):
     return _lib.ops.rows_layer(rows, weights, biases, *tail, _precision)
 
 
+def _tail(outputs, biases, relu):
+    outputs = outputs if biases is None else outputs + biases
+    return torch.relu(outputs) if relu else outputs
+
+
 def rows_pointwise(rows, weights, biases, relu):
     """out = act(rows @ weights + biases): the pointwise layer (the reference's PerItemConv3d, picasso/mesh/layers.py:198-240)
     without normalisation."""
+    if not _lib.native_calls():
+        return _tail(rows @ weights, biases, relu)
     return rows_layer(rows, weights, biases, (relu, *_NO_NORM))
 
 
 def vertex2facet_pointwise(input, filter, face, depth_weights, biases, relu):
     if tuple(filter.shape) != (3, input.shape[1], 1):
         raise RuntimeError("filter must have shape (3, C, 1) and depth_weights (C, out_channels)")
+    if not _lib.native_calls():
+        return _tail(conv3d.vertex2facet(input, filter, face) @ depth_weights, biases, relu)
     eye = torch.eye(3, device=input.device)       # the filter itself stands for the product of basis and weights
     return vertex2facet_layer(input, face, eye, filter.reshape(3, -1), depth_weights, biases, (relu, *_NO_NORM))
 
 
 def facet2vertex_pointwise(input, filter, coeff, face, nf_count, vt_map, depth_weights, biases, relu):
+    if not _lib.native_calls():
+        return _tail(conv3d.facet2vertex(input, filter, coeff, face, nf_count, vt_map) @ depth_weights, biases, relu)
     return facet2vertex_layer(input, filter, coeff, face, nf_count, vt_map, depth_weights, biases, (relu, *_NO_NORM))

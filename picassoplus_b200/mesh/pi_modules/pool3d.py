@@ -111,6 +111,8 @@ class MaxPoolFunction(torch.autograd.Function):
 
 
 def maxPool(input, vt_replace, vt_map, vt_out):
+    if not _lib.native_calls():
+        return MaxPoolFunction.apply(input, vt_replace, vt_map, vt_out)
     _pool_checks(input, vt_replace, vt_map, vt_out)
     vt_replace.requires_grad = False
     vt_map.requires_grad = False
@@ -138,6 +140,8 @@ class AvgPoolFunction(torch.autograd.Function):
 
 
 def avgPool(input, vt_replace, vt_map, vt_out):
+    if not _lib.native_calls():
+        return AvgPoolFunction.apply(input, vt_replace, vt_map, vt_out)
     _pool_checks(input, vt_replace, vt_map, vt_out)
     vt_replace.requires_grad = False
     vt_map.requires_grad = False

@@ -66,6 +66,8 @@ class InterpolateFunction(torch.autograd.Function):
 
 
 def interpolate(input, vt_replace, vt_map):
+    if not _lib.native_calls():
+        return InterpolateFunction.apply(input, vt_replace, vt_map)
     _check(input, "input", 2, torch.float32)
     _check(vt_replace, "vt_replace", 1, torch.int32)
     _check(vt_map, "vt_map", 1, torch.int32)

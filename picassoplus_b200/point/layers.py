@@ -24,7 +24,8 @@ class PCloudConv3d(_PointwiseTail):
         self._init_tail(out_channels, activation_fn, with_bn, bn_momentum)
 
     def forward(self, inputs, nn_count, nn_index, filt_index, filt_coeff=None):
-        if _layers._fusion and inputs.is_cuda and _layers._plain_activation(self.activation_fn) and nn_count.shape[0] > 0:
+        if (_layers._fusion and inputs.is_cuda and _layers._plain_activation(self.activation_fn) and nn_count.shape[0] > 0 and
+                _lib.native_calls()):
             pairs = (nn_count, nn_index, filt_index, filt_coeff)
             return self._native(nn_count.shape[0], inputs, lambda *tail: _lib.ops.point_layer(
                 inputs, self.spatial_weights, *pairs, *conv3d.groupings(inputs, *pairs), self.depth_weights, self.biases, *tail))

@@ -122,6 +122,8 @@ def groupings(input, nn_count, nn_index, bin_index, bin_coeff):
 
 
 def conv3d(input, filter, nn_count, nn_index, bin_index):
+    if not _lib.native_calls():
+        return ConvFunction.apply(input, filter, nn_count, nn_index, bin_index)
     return _lib.ops.point_conv(input, filter, nn_count, nn_index, bin_index, None,
                                *groupings(input, nn_count, nn_index, bin_index, None))
 
@@ -145,5 +147,7 @@ class FuzzyConv3dFunction(torch.autograd.Function):
 
 
 def fuzzyconv3d(input, filter, nn_count, nn_index, bin_index, bin_coeff):
+    if not _lib.native_calls():
+        return FuzzyConv3dFunction.apply(input, filter, nn_count, nn_index, bin_index, bin_coeff)
     return _lib.ops.point_conv(input, filter, nn_count, nn_index, bin_index, bin_coeff,
                                *groupings(input, nn_count, nn_index, bin_index, bin_coeff))
