@@ -28,8 +28,17 @@ def set_fusion(on: bool) -> None:
     _fusion = bool(on)
 
 
+_has_global_hooks = nn.modules.module._has_any_global_hook
+
+
+def _hooked(module):
+    """Whether calling the module runs a hook, which a native call in its place would leave out."""
+    return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks or
+                _has_global_hooks())
+
+
 def _plain_activation(fn):
-    return fn is None or type(fn) is nn.ReLU
+    return fn is None or (type(fn) is nn.ReLU and not _hooked(fn))
 
 
 def _filter_variable_(shape, stddev=1.0, use_xavier=True):
@@ -52,8 +61,7 @@ def _norm_args(bn, rows, device):
     """How the native layers run the module's batch norm: (mode, weight, bias, running mean, running var, batches, momentum,
     eps) with mode 1 = statistics of the batch, 2 = running statistics, or None when the torch module has to run itself (a
     subclass or a hook, cumulative averages, parameters elsewhere, a single row)."""
-    if (type(bn) is not nn.BatchNorm1d or bn._forward_hooks or bn._forward_pre_hooks or bn._backward_hooks or
-            bn._backward_pre_hooks or _has_global_hooks()):
+    if type(bn) is not nn.BatchNorm1d or _hooked(bn):
         return None
     p, b = bn._parameters, bn._buffers
     weight, bias, mean, var, batches = p["weight"], p["bias"], b["running_mean"], b["running_var"], b["num_batches_tracked"]
@@ -69,7 +77,6 @@ def _norm_args(bn, rows, device):
     return 2, weight, bias, mean, var, None, 0.0, bn.eps
 
 
-_has_global_hooks = nn.modules.module._has_any_global_hook
 _NO_NORM = (0, None, None, None, None, None, 0.0, 0.0)
 
 

@@ -142,3 +142,22 @@ def test_saved_tensors_elsewhere(kind, train):
         assert torch.equal(a, b)
     for a, b in zip(torch.autograd.grad(checkpoint(call, x, use_reentrant=False), leaves, g), want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("kind", ["facet", "point"])
+def test_hooks_on_the_activation_run(kind):
+    """Facet and point layers call their activation module; with a hook on it, or on all modules, they still do."""
+    call = Call(kind)
+    call.m.activation_fn = nn.ReLU()
+    with torch.no_grad():
+        want, seen = call(call.x), []
+        handle = call.m.activation_fn.register_forward_hook(lambda module, args, out: seen.append(out))
+        out = call(call.x)
+        handle.remove()
+        assert len(seen) == 1 and close(out, want) and bool((seen[0] >= 0).all())
+        handle = nn.modules.module.register_module_forward_hook(lambda module, args, out: seen.append(type(module)))
+        call(call.x)
+        handle.remove()
+        assert nn.ReLU in seen and nn.BatchNorm1d in seen
+        n = len(seen)
+        assert torch.equal(call(call.x), want) and len(seen) == n
