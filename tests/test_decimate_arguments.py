@@ -77,6 +77,16 @@ def test_forms_of_the_target():
         for sizes in ((cn, cm), (cn.long(), cm.long())):
             got = dm.mesh_decimation_(v, f, g, *sizes, t)
             assert all(torch.equal(a, b) for a, b in zip(got, want))
-    got = MeshHierarchy([target(20)], True, 5.0)(v, f, cn, cm)[1]
     want = dm.mesh_decimation_(v, f, g, cn, cm, 20, True, 5.0)
-    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    for t in (target(20), target(20)[0], torch.tensor([19.5, 20.]), target(20, 20).cuda()):
+        got = MeshHierarchy([t], True, 5.0)(v, f, cn, cm)[1]
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("stride", [1.1, 1.5, 2, 2.7, 3, 4, 5, 7, 10, 41, 47, 55, 61, 83])
+def test_vertices_kept_per_stride(stride):
+    """The whole range of counts: those of tensor / stride on the GPU, to the vertex."""
+    n = torch.arange(0, 300001, dtype=torch.int32, device="cuda")
+    want = torch.clip((n.to(torch.float) / float(stride)).to(torch.int), min=4).tolist()
+    assert MeshHierarchy([stride], [4], True, 1.0)._target(0, n.tolist()) == want
