@@ -492,6 +492,10 @@ struct Tail {
     Tensor gamma, beta, running_mean, running_var, batches;
     double momentum = 0, eps = 0;
 };
+void check_tail(const Tail& t, int64_t Cout) {
+    for (const Tensor* x : {&t.gamma, &t.beta, &t.running_mean, &t.running_var})
+        if (x->defined() && x->numel() != Cout) fail("batch normalisation must have one value per output channel");
+}
 
 // Mean and 1 / deviation of every channel
 struct NormStats { Tensor mean, invstd; };
@@ -564,6 +568,7 @@ void masked_gradient(const Scope& s, const Tensor& g, const Tensor& act, const N
 struct Staged { Tensor out, act, features; NormStats stats; };
 template <typename Launch>
 Staged run_stage(const Scope& s, const Tail& t, int64_t rows, int64_t C, int64_t Cout, bool keep_features, Launch&& launch) {
+    check_tail(t, Cout);
     Staged r;
     r.act = s.floats({rows, Cout});
     pb200_pointwise_extra x = {};
@@ -625,7 +630,13 @@ StageGrads stage_backward(const Scope& s, const Tensor& g_in, const Tensor& act,
     return r;
 }
 
-Tensor flat(const Tensor& bias) { return bias.defined() ? bias.reshape({-1}).contiguous() : bias; }
+// one value per output channel; a single value stands for all
+Tensor flat(const Tensor& bias, int64_t Cout) {
+    if (!bias.defined()) return bias;
+    if (bias.numel() == 1 && Cout != 1) return bias.reshape({1}).expand({Cout}).contiguous();
+    if (bias.numel() != Cout) fail("biases must have one value per output channel");
+    return bias.reshape({-1}).contiguous();
+}
 void check_stage(const Tensor& weights, int64_t C) {
     check(weights, "depth_weights", 2, at::kFloat);
     if (weights.size(0) != C) fail("depth_weights must have shape (channels, out_channels)");
@@ -780,7 +791,7 @@ Tensor v2f_layer(const Tensor& x_in, const Tensor& face, const OptTensor& rowptr
     if (spatial.size(0) != K || spatial.size(1) != C) fail("spatial_weights must have shape (number of bases, channels)");
     if (Nf > 0 && face.size(1) != 3) fail("face must have shape (NfIn, 3)");
     Scope s(x_in);
-    const Tensor x = aligned(x_in), bias = flat(bias0);
+    const Tensor x = aligned(x_in), bias = flat(bias0, Cout);
     // the library product, whose rounding the separate modules share (norm.cu says why bits matter between layers)
     const Tensor filter = at::matmul(corners, spatial).view({3, C, 1});
     const size_t nb = pb200_vertex2facet_pointwise_workspace_bytes((int)C, precision);
@@ -824,7 +835,7 @@ Tensor f2v_layer(const Tensor& x_in, const Tensor& face, const Tensor& nf_count,
     const int64_t Nf = x_in.size(0), C = x_in.size(1), K = filter_in.size(0), NvOut = nf_count.size(0), Cout = weights.size(1);
     if (filter_in.size(2) != 1) fail("filter must have shape (K, C, 1)");
     Scope s(x_in);
-    const Tensor x = aligned(x_in), filter = aligned(filter_in), bias = flat(bias0);
+    const Tensor x = aligned(x_in), filter = aligned(filter_in), bias = flat(bias0, Cout);
     const size_t nb = pb200_facet2vertex_pointwise_workspace_bytes(Nf, (int)C, precision);
     Tensor ws = s.bytes(nb);
     Staged r = run_stage(s, t, NvOut, C, Cout, (bool)node, [&](float* out, const pb200_pointwise_extra* extra) {
@@ -864,7 +875,7 @@ Tensor rows_layer(const Tensor& rows_in, const Tensor& weights, const OptTensor&
     const int64_t N = rows_in.size(0), C = rows_in.size(1), Cout = weights.size(1);
     if (weights.size(0) != C) fail("weights must have shape (in_channels, out_channels)");
     Scope s(rows_in);
-    const Tensor rows = aligned(rows_in), bias = flat(bias0);
+    const Tensor rows = aligned(rows_in), bias = flat(bias0, Cout);
     const size_t nb = pb200_masked_rows_matmul_workspace_bytes((int)C, precision);
     Tensor ws = s.bytes(nb);
     Staged r = run_stage(s, t, N, C, Cout, false, [&](float* out, const pb200_pointwise_extra* extra) {
@@ -889,6 +900,7 @@ Tensor rows_layer(const Tensor& rows_in, const Tensor& weights, const OptTensor&
 // act <- activation(act + bias) in place, out = its normalisation (act itself without one); the statistics used
 NormStats bias_act_norm(const Scope& s, const Tail& t, const Tensor& act, const Tensor& bias, Tensor& out) {
     const int64_t rows = act.size(0), C = act.size(1);
+    check_tail(t, C);
     Tensor partial = s.floats({pb200_norm_parts(rows, (int)C), 3, C});
     int parts = 0;
     call(pb200_bias_act_stats(rows, (int)C, fpm(act), fp(bias), t.relu, fpm(partial), &parts, s.stream), "pb200_bias_act_stats");
@@ -914,7 +926,7 @@ Tensor f2f_layer(const Tensor& input, const Tensor& filter, const Tensor& bary, 
     at::AutoDispatchBelowADInplaceOrView below;
     check_f2f(input, filter, bary);
     Scope s(input);
-    const Tensor cum = at::cumsum(counts, 0, at::kInt), bias = flat(bias0);
+    const Tensor cum = at::cumsum(counts, 0, at::kInt), bias = flat(bias0, filter.size(0));
     check(cum, "num_texture", 1, at::kInt);
     Tensor act = f2f_forward(s, aligned(input), filter, bary, cum, precision), out;
     const NormStats st = bias_act_norm(s, t, act, bias, out);
@@ -1220,7 +1232,7 @@ Tensor point_layer(const Tensor& input, const Tensor& filter, const Tensor& nn_c
     Scope s(input);
     Tensor feats = pairs_forward(s, input, filter, q, out_rowptr, out_members);
     Tensor act = at::matmul(feats, weights), out;
-    const NormStats st = bias_act_norm(s, t, act, flat(bias0), out);
+    const NormStats st = bias_act_norm(s, t, act, flat(bias0, weights.size(1)), out);
     if (node) {
         node->keep_pairs(input, filter, q, or_undefined(in_rowptr), or_undefined(in_members));
         node->features = keep(feats);

@@ -161,3 +161,34 @@ def test_hooks_on_the_activation_run(kind):
         assert nn.ReLU in seen and nn.BatchNorm1d in seen
         n = len(seen)
         assert torch.equal(call(call.x), want) and len(seen) == n
+
+
+@pytest.mark.parametrize("kind", ["rows", "mesh", "facet", "point"])
+@pytest.mark.parametrize("train", [False, True])
+def test_widths_of_bias_and_batch_norm(kind, train):
+    """A batch norm or a bias of another width is refused, as the separate operators refuse it; one value of the bias stands for all."""
+    call = Call(kind).train(train)
+    layer = call.m.V2F_conv3d if kind == "mesh" else call.m
+    bias, norm = layer.biases, layer.BatchNorm
+    with torch.no_grad():
+        bias.fill_(0.25)
+        want = call(call.x)
+        for width in (bias.shape[1] - 8, bias.shape[1] + 8):
+            layer.BatchNorm = nn.BatchNorm1d(width).cuda().train(train)
+            with pytest.raises(RuntimeError):
+                call(call.x)
+            layer.BatchNorm = norm
+            layer.biases = nn.Parameter(torch.zeros(1, width, device="cuda"))
+            with pytest.raises(RuntimeError):
+                call(call.x)
+            layer.biases = bias
+    layer.biases = nn.Parameter(torch.full((1, 1), 0.25, device="cuda"))
+    if not train:
+        with torch.no_grad():
+            assert torch.equal(call(call.x), want)
+    out = call(call.x)
+    g = torch.randn_like(out)
+    got, = torch.autograd.grad(out, [layer.biases], g)
+    layer.biases = bias
+    each, = torch.autograd.grad(call(call.x), [bias], g)
+    assert got.shape == (1, 1) and abs(float(got - each.sum())) <= 1e-3 * float(each.abs().sum())
