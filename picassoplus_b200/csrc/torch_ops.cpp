@@ -785,7 +785,7 @@ Tensor v2f_layer(const Tensor& x_in, const Tensor& face, const OptTensor& rowptr
     at::AutoDispatchBelowADInplaceOrView below;
     check(x_in, "input", 2, at::kFloat);
     check(face, "face", 2, at::kInt);
-    check(spatial, "spatial_weights", 2, at::kFloat);
+    check(spatial.contiguous(), "spatial_weights", 2, at::kFloat);
     check_stage(weights_in, x_in.size(1));
     const int64_t Nv = x_in.size(0), C = x_in.size(1), Nf = face.size(0), Cout = weights_in.size(1), K = corners.size(1);
     if (spatial.size(0) != K || spatial.size(1) != C) fail("spatial_weights must have shape (number of bases, channels)");
@@ -1218,18 +1218,19 @@ Tensor point_conv(const Tensor& input, const Tensor& filter, const Tensor& nn_co
 
 Tensor point_layer(const Tensor& input, const Tensor& filter, const Tensor& nn_count, const Tensor& nn_index, const Tensor& bin_index,
                    const OptTensor& bin_coeff, const Tensor& out_rowptr, const Tensor& out_members, const OptTensor& in_rowptr,
-                   const OptTensor& in_members, const Tensor& weights, const Tensor& bias0, bool relu, int norm_mode, const OptTensor& gamma,
+                   const OptTensor& in_members, const Tensor& weights_in, const Tensor& bias0, bool relu, int norm_mode, const OptTensor& gamma,
                    const OptTensor& beta, const OptTensor& running_mean, const OptTensor& running_var, const OptTensor& batches,
                    double momentum, double eps) {
     const Tail t = make_tail(TAIL_ARGS);
     const Pairs q{nn_count, nn_index, bin_index, or_undefined(bin_coeff)};
     check_pairs(input, filter, q);
-    check_stage(weights, filter.size(1) * filter.size(2));
     std::shared_ptr<PointLayer> node;
-    if (torch::autograd::compute_requires_grad(input, filter, weights, bias0, t.gamma, t.beta))
-        node = node_for<PointLayer>(input, filter, weights, bias0, t.gamma, t.beta);
+    if (torch::autograd::compute_requires_grad(input, filter, weights_in, bias0, t.gamma, t.beta))
+        node = node_for<PointLayer>(input, filter, weights_in, bias0, t.gamma, t.beta);
     at::AutoDispatchBelowADInplaceOrView below;
     Scope s(input);
+    const Tensor weights = weights_in.contiguous();
+    check_stage(weights, filter.size(1) * filter.size(2));
     Tensor feats = pairs_forward(s, input, filter, q, out_rowptr, out_members);
     Tensor act = at::matmul(feats, weights), out;
     const NormStats st = bias_act_norm(s, t, act, flat(bias0, weights.size(1)), out);

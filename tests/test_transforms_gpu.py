@@ -192,3 +192,19 @@ def test_widths_of_bias_and_batch_norm(kind, train):
     layer.biases = bias
     each, = torch.autograd.grad(call(call.x), [bias], g)
     assert got.shape == (1, 1) and abs(float(got - each.sum())) <= 1e-3 * float(each.abs().sum())
+
+
+@pytest.mark.parametrize("kind,name", [("mesh", "spatial_weights"), ("point", "depth_weights")])
+def test_strided_weights(kind, name):
+    """Weights that go into a torch product may have any strides (a transposed parameter, a slice of a larger one)."""
+    call = Call(kind)
+    layer = call.m.V2F_conv3d if kind == "mesh" else call.m
+    w = getattr(layer, name)
+    out = call(call.x)
+    g = torch.randn_like(out)
+    want, = torch.autograd.grad(out, [w], g)
+    other = nn.Parameter(w.detach().t().contiguous().t())
+    assert not other.is_contiguous()
+    setattr(layer, name, other)
+    got = call(call.x)
+    assert close(got.detach(), out.detach()) and close(torch.autograd.grad(got, [other], g)[0], want)
