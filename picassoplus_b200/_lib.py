@@ -33,12 +33,14 @@ except ImportError as e:
 
 from torch.autograd import forward_ad as _forward_ad  # noqa: E402
 
+_tracing_state = _torch._C._get_tracing_state
+
 
 def native_calls() -> bool:
     """Whether the calls of `ops` may stand for operators and layers.  Their nodes belong to reverse mode alone: a tracer would
     not see them and keep their result as a constant, forward mode would lose its tangents.  There the autograd Functions and
     torch's own operators run, which are traced, and refuse what they cannot do."""
-    return _torch._C._get_tracing_state() is None and _forward_ad._current_level < 0
+    return _tracing_state() is None and _forward_ad._current_level < 0
 
 
 i64, i32, vp, sz, f32 = C.c_int64, C.c_int, C.c_void_p, C.c_size_t, C.c_float

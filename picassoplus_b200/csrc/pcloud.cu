@@ -169,6 +169,8 @@ constexpr int LONG_ROW = 64;
 // memory, then the block's groups of CV lanes walk equal consecutive parts of them, four row gathers in flight; the groups'
 // sums are added in group order.
 constexpr int LONG_SCAN = 1024, STAGE = 256, STAGED_BINS = 3;
+// beside the 17 KB that they are staged in, a filter table above this needs more than the default 48 KB
+constexpr size_t UNASKED_TABLE = 30 * 1024;
 static inline int long_blocks(int64_t Np) { return (int)ceil_div(Np, LONG_SCAN); }
 
 __device__ __noinline__ void bwd_input_long_rows(int64_t first, int64_t Np, int64_t Mp, int F, int CV, int T,
@@ -648,9 +650,9 @@ static int launch_bwd_coop(int64_t Np, int64_t Mp, int64_t Nout, int nb, int F, 
                            cudaStream_t stream) {
     if (Np > 0) {
         const int nlong = Nout > LONG_ROW ? long_blocks(Np) : 0;
-        // beside the 17 KB that the long rows are staged in, a filter table above 31 KB needs more than the default 48 KB
-        PB_CUDA(cudaFuncSetAttribute(conv_bwd_input_coop_kernel<TT, CV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(sizeof(float4) * F * CV)));
+        if (sizeof(float4) * F * CV > UNASKED_TABLE)
+            PB_CUDA(cudaFuncSetAttribute(conv_bwd_input_coop_kernel<TT, CV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(sizeof(float4) * F * CV)));
         PB_LAUNCH("pcloud_conv_bwd_input", (conv_bwd_input_coop_kernel<TT, CV>), nlong + persistent_blocks(Np * Lanes<CV>::LN, 256, 8), 256,
                   sizeof(float4) * F * CV, stream, Np, Mp, F, T, (const float4*)gout, (const float4*)filter, nnCount, nnIndex, bin,
                   coeff, rowptr, members, nlong, (float4*)gin);
@@ -742,8 +744,9 @@ int pb200_pcloud_conv3d_backward(int64_t Np, int64_t Mp, int64_t Nout, int F, in
         }
         if (Np > 0) {
             const int nlong = Nout > LONG_ROW ? long_blocks(Np) : 0;
-            PB_CUDA(cudaFuncSetAttribute(conv_bwd_input_vec_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(sizeof(float) * F * C)));
+            if (sizeof(float) * F * C > UNASKED_TABLE)
+                PB_CUDA(cudaFuncSetAttribute(conv_bwd_input_vec_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)(sizeof(float) * F * C)));
             PB_LAUNCH("pcloud_conv_bwd_input", conv_bwd_input_vec_kernel, nlong + persistent_blocks(Np * CV, 256, 8), 256,
                       sizeof(float) * F * C, stream, Np, Mp, F, CV, T, (const float4*)gradOutput, (const float4*)filter, nnCount,
                       nnIndex, binIndex, binCoeff, rowptr_in, members_in, nlong, (float4*)gradInput);

@@ -24,6 +24,7 @@
 #include <stdexcept>
 #include <string>
 #include <unordered_map>
+#include <utility>
 #include <vector>
 
 #include "../../include/picasso_b200.h"
@@ -59,14 +60,17 @@ Tensor aligned(const Tensor& t) { return misaligned(t) ? t.clone() : t; }
 // Everything a call needs from the current device: guard, stream, allocation.  Autocast stays out: AutoDispatchBelow... leaves its
 // keys on, and a product that torch rounds to half precision under it would come back as half the bytes that the kernels behind
 // it read and write.  The kernels choose their operands' precision themselves.
+thread_local c10::DeviceIndex call_device = -1;              // of the innermost Scope
 struct Scope {
     c10::cuda::CUDAGuard guard;
+    const c10::DeviceIndex outer = std::exchange(call_device, guard.current_device().index());
     c10::impl::ExcludeDispatchKeyGuard no_autocast{c10::DispatchKey::AutocastCUDA};
     at::TensorOptions f32;
     void* stream;
     explicit Scope(const Tensor& t)
         : guard(t.device()), f32(t.options().dtype(at::kFloat).requires_grad(false)),
           stream(c10::cuda::getCurrentCUDAStream(t.device().index()).stream()) {}
+    ~Scope() { call_device = outer; }
     Tensor floats(at::IntArrayRef shape) const { return at::empty(shape, f32); }
     Tensor bytes(size_t n) const { return at::empty({(int64_t)(n > 0 ? n : 1)}, f32.dtype(at::kByte)); }
 };
@@ -74,7 +78,7 @@ struct Scope {
 // Addresses for a kernel: whatever way a tensor came in, one of another type, device or layout goes no further
 void* address(const Tensor& t, at::ScalarType type) {
     if (!t.defined()) return nullptr;
-    if (t.scalar_type() != type || !t.is_cuda() || t.get_device() != c10::cuda::current_device() || !t.is_contiguous())
+    if (t.scalar_type() != type || !t.is_cuda() || t.get_device() != call_device || !t.is_contiguous())
         fail(std::string("expected a contiguous ") + c10::toString(type) + " tensor on the call's CUDA device, got " +
              c10::toString(t.scalar_type()) + " on " + t.device().str());
     return t.data_ptr();
@@ -1422,7 +1426,7 @@ struct TopologyCache {
         c10::cuda::CUDAStream stream;
         unsigned long long capture;              // id of the capture it was made in, 0: none
         c10::Event ready;                        // behind the kernels that make it
-        bool complete = false;                   // seen to have passed
+        bool complete = false;                   // they are known to have run
     };
     using Key = std::array<int64_t, 12>;
     struct Hash {
@@ -1485,7 +1489,7 @@ struct TopologyCache {
             for (const Tensor& t : e.tensors) t.record_stream(now);
         return &e;
     }
-    void put(const Key& k, const Tensor& a, const OptTensor& b, std::vector<Tensor> tensors, py::object value, int64_t size) {
+    void put(const Key& k, const Tensor& a, const OptTensor& b, std::vector<Tensor> tensors, py::object value, int64_t size, bool complete) {
         auto old = at.find(k);
         if (old != at.end()) erase(old->second);
         for (auto it = recent.begin(); it != recent.end();) {
@@ -1498,7 +1502,8 @@ struct TopologyCache {
         const auto now = c10::cuda::getCurrentCUDAStream(a.device().index());
         Entry e{{Source(a)}, std::move(tensors), std::move(value), size, now, capture_id(now), c10::Event(c10::DeviceType::CUDA)};
         if (b.has_value()) e.sources.emplace_back(*b);
-        e.ready.record(now.unwrap());
+        e.complete = complete && e.capture == 0;
+        if (!e.complete) e.ready.record(now.unwrap());
         at[k] = recent.insert(recent.end(), {k, std::move(e)});
         bytes += size;
         while (!recent.empty() && bytes > budget) erase(recent.begin());
@@ -1512,9 +1517,10 @@ py::object cache_find(int kind, const Tensor& a, const OptTensor& b, int64_t m, 
     TopologyCache::Entry* e = cache().find(TopologyCache::key(kind, a, b, m, n), a, b);
     return e ? e->value : py::object(py::none());
 }
+// complete: the caller has waited for the kernels that make the structure
 void cache_put(int kind, const Tensor& a, const OptTensor& b, int64_t m, int64_t n, std::vector<Tensor> tensors, py::object value,
-               int64_t bytes) {
-    cache().put(TopologyCache::key(kind, a, b, m, n), a, b, std::move(tensors), std::move(value), bytes);
+               int64_t bytes, bool complete) {
+    cache().put(TopologyCache::key(kind, a, b, m, n), a, b, std::move(tensors), std::move(value), bytes, complete);
 }
 void cache_budget(int64_t n) {
     TopologyCache& c = cache();

@@ -29,6 +29,7 @@ graphs, so they are ordinary tensors also when that call runs under torch.infere
 """
 from __future__ import annotations
 
+import contextlib
 import threading
 from typing import List, Optional
 
@@ -90,10 +91,22 @@ class VertexCSR:
         return [self.rowptr, self.entries]
 
 
-def _store(kind, a, b, m, n, value, shared=False):
-    """Puts a structure made from the index tensors a (and b) into the cache; shared: its arrays belong to another entry."""
+def _store(kind, a, b, m, n, value, shared=False, validated=True):
+    """Puts a structure made from the index tensors a (and b) into the cache; shared: its arrays belong to another entry.
+    validated: a status word behind its kernels is looked at, in 'sync' mode before this call."""
     tensors = value._tensors()
-    _ops.cache_put(kind, a, b, m, n, tensors, value, 0 if shared else sum(t.numel() * t.element_size() for t in tensors))
+    _ops.cache_put(kind, a, b, m, n, tensors, value, 0 if shared else sum(t.numel() * t.element_size() for t in tensors),
+                   validated and _validation == "sync")
+
+
+def _building(device):
+    """The device of a structure that is made; not under inference mode, for it is kept."""
+    if not torch.is_inference_mode_enabled():
+        return torch.cuda.device(device)
+    stack = contextlib.ExitStack()
+    stack.enter_context(torch.inference_mode(False))
+    stack.enter_context(torch.cuda.device(device))
+    return stack
 
 
 def _launch_build(face, vt_map, nv_in, nv_out):
@@ -116,7 +129,7 @@ def _bad_index_message(nv_in, nv_out):
 def build_vertex_csr(face: torch.Tensor, vt_map: Optional[torch.Tensor], nv_in: int, nv_out: int) -> VertexCSR:
     """Uncached build.  Validates every index: in 'sync' mode a bad one raises RuntimeError here
     (one device synchronisation), in 'deferred' mode at the next check_deferred()."""
-    with torch.inference_mode(False), torch.cuda.device(face.device):
+    with _building(face.device):
         rowptr, entries, status = _launch_build(face, vt_map, nv_in, nv_out)
         if _validation == "deferred":
             with _lock:
@@ -137,7 +150,7 @@ def vertex_csr(face: torch.Tensor, vt_map: Optional[torch.Tensor], nv_in: int, n
     may_be_identity = vt_map is not None and nv_in == nv_out and vt_map.shape[0] == nv_in
     if may_be_identity and _validation == "sync":
         base = _ops.cache_find(_VERTEX, face, None, nv_in, nv_out)
-        with torch.inference_mode(False), torch.cuda.device(face.device):
+        with _building(face.device):
             ident = (vt_map == torch.arange(nv_in, dtype=vt_map.dtype, device=vt_map.device)).all().to(torch.int32)
             if base is None:
                 # build the identity CSR and test vtMap in the same synchronisation
@@ -207,7 +220,7 @@ def cluster_csr(vt_replace: torch.Tensor, vt_map: torch.Tensor, nv_out: int) -> 
     if hit is not None:
         return hit
     dev = vt_replace.device
-    with torch.inference_mode(False), torch.cuda.device(dev):
+    with _building(dev):
         key = torch.empty(max(nv_in, 1), dtype=torch.int32, device=dev)
         rowptr = torch.empty(nv_out + 1, dtype=torch.int32, device=dev)
         members = torch.empty(max(nv_in, 1), dtype=torch.int32, device=dev)
@@ -247,7 +260,7 @@ def pair_csr(nn_index: torch.Tensor, column: int, n_rows: int) -> PairCSR:
     if hit is not None:
         return hit
     dev = nn_index.device
-    with torch.inference_mode(False), torch.cuda.device(dev):
+    with _building(dev):
         rowptr = torch.empty(n_rows + 1, dtype=torch.int32, device=dev)
         members = torch.empty(max(npairs, 1), dtype=torch.int32, device=dev)
         status = torch.empty(1, dtype=torch.int32, device=dev)
@@ -289,7 +302,7 @@ def pad_rows(rows: torch.Tensor):
         return None
     Fp = _lib.query("pb200_padded_row_floats", F)
     dev = rows.device
-    with torch.inference_mode(False), torch.cuda.device(dev):
+    with _building(dev):
         out = torch.empty(n, Fp, dtype=torch.float32, device=dev)
         _lib.call("pb200_pad_rows", n, F, ptr(rows), ptr(out), stream_ptr(dev))
     return out
@@ -303,13 +316,13 @@ def face_means(sample_rows: torch.Tensor, num_interior: torch.Tensor) -> FaceMea
     if hit is not None:
         return hit
     dev = sample_rows.device
-    with torch.inference_mode(False), torch.cuda.device(dev):
+    with _building(dev):
         check_num_interior(num_interior, nik)
         rows = torch.empty(nf, sample_rows.shape[1], dtype=torch.float32, device=dev)
         _lib.call("pb200_face_mean_rows", nf, nik, sample_rows.shape[1], ptr(sample_rows), ptr(num_interior), ptr(rows),
                   stream_ptr(dev))
         fm = FaceMeans(rows, torch.arange(1, nf + 1, dtype=torch.int32, device=dev))
-    _store(_MEANS, sample_rows, num_interior, sample_rows.shape[1], 0, fm)
+    _store(_MEANS, sample_rows, num_interior, sample_rows.shape[1], 0, fm, validated=False)
     return fm
 
 
@@ -323,12 +336,12 @@ def face_means_sph_harm(L: int, sample_xyz: torch.Tensor, num_interior: torch.Te
     if sample_xyz.dim() != 2 or sample_xyz.shape[1] != 3 or sample_xyz.dtype != torch.float32 or not sample_xyz.is_contiguous():
         raise RuntimeError("sample_xyz must be a contiguous float32 tensor of shape (NiK, 3)")
     dev = sample_xyz.device
-    with torch.inference_mode(False), torch.cuda.device(dev):
+    with _building(dev):
         check_num_interior(num_interior, nik)
         rows = torch.empty(nf, (L + 1) ** 2, dtype=torch.float32, device=dev)
         _lib.call("pb200_face_mean_sph_harm", nf, nik, int(L), ptr(sample_xyz), ptr(num_interior), ptr(rows), stream_ptr(dev))
         fm = FaceMeans(rows, torch.arange(1, nf + 1, dtype=torch.int32, device=dev))
-    _store(_MEANS_SH, sample_xyz, num_interior, L, 0, fm)
+    _store(_MEANS_SH, sample_xyz, num_interior, L, 0, fm, validated=False)
     return fm
 
 
@@ -348,7 +361,7 @@ def sample_ends(counts: torch.Tensor, n_rows: int) -> torch.Tensor:
     hit = _ops.cache_find(_SAMPLES, counts, None, n_rows, 0)
     if hit is not None:
         return hit.ends
-    with torch.inference_mode(False):
+    with _building(counts.device):
         ends = torch.cumsum(counts.detach(), 0, dtype=torch.int64)
         bad = ends[-1:] != n_rows if counts.shape[0] else torch.full((1,), n_rows != 0, device=counts.device)
         bad = bad | (counts < 0).any()
@@ -367,7 +380,7 @@ def check_num_interior(num_interior: torch.Tensor, nik: int) -> None:
     device: raises in 'sync' mode, queues the status word in 'deferred' mode.  The facet2facet
     kernels trust numInterior as the reference does; run this once per array."""
     dev = num_interior.device
-    with torch.inference_mode(False), torch.cuda.device(dev):
+    with _building(dev):
         status = torch.empty(1, dtype=torch.int32, device=dev)
         _lib.call("pb200_check_num_interior", num_interior.shape[0], int(nik), ptr(num_interior), ptr(status),
                   stream_ptr(dev))
