@@ -251,9 +251,13 @@ def kernel_models(d):
         "f2f_bwd_gfilter_tc": dict(bytes=4 * Ci * Ns + 4 * K * Ns + 4 * Nf + 4 * Co * Nf,
                                    flops=2 * Q * Ns + 2 * Q * Co * Nf),
         "face_mean_rows": dict(bytes=4 * K * NiK + 4 * Nf + 4 * K * Nf),
-        # forward for one sample per face: a plain product over the input rows, the sum over the bases in the epilogue
+        # one sample per face: a plain product over the input rows with the sum over the bases in the epilogue, on the general
+        # input-gradient kernel and on the kernels of its own
         "f2f_fwd_one_sample_tc": dict(bytes=4 * Ci * Nf + 4 * K * Nf + 4 * Co * Nf, flops=2 * Q * Co * Nf + 2 * K * Co * Nf),
     }
+    m["f2f_fwd_one_tc"] = m["f2f_fwd_one_sample_tc"]
+    m["f2f_bwd_gin_one_tc"] = dict(bytes=4 * Co * Nf + 4 * K * Nf + 4 * Ci * Nf, flops=2 * Q * Co * Nf + 2 * Q * Nf)
+    m["f2f_bwd_gfilter_one_tc"] = dict(bytes=4 * Ci * Nf + 4 * K * Nf + 4 * Co * Nf, flops=2 * Q * Nf + 2 * Q * Co * Nf)
     return m
 
 

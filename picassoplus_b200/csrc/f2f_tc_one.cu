@@ -376,7 +376,7 @@ static int launch(const char* label, const Params& p, int grid, size_t smem, cud
 // forward = true: the operator's forward pass (filter (Cn, Ck, F)); false: its input gradient (filter (Ck, Cn, F))
 int run(int64_t Nf, int Cn, int Ck, int F, const float* rows, const float* filter, const float* w, int Fp, float* out, int precision,
         void* ws, cudaStream_t stream, bool forward) {
-    const char* label = forward ? "f2f_fwd_one_sample_tc" : "f2f_bwd_gin_tc";
+    const char* label = forward ? "f2f_fwd_one_tc" : "f2f_bwd_gin_one_tc";
     int rc = check_async_error(forward ? "facet2facet_forward" : "facet2facet_backward");
     if (rc) return rc;
     const Plan pl = plan(Cn, Ck, F, precision);

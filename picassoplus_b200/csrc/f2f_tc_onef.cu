@@ -517,7 +517,7 @@ template <int NSPLIT>
 static int launch(const Params& p, cudaStream_t stream) {
     const size_t smem = smem_bytes(p, NSPLIT, FACES<NSPLIT>);
     PB_CUDA(cudaFuncSetAttribute(f2f_one_sample_gfilter_kernel<NSPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PB_LAUNCH("f2f_bwd_gfilter_tc", (f2f_one_sample_gfilter_kernel<NSPLIT>), p.nb1 * p.nb2 * p.groups * p.chunks, NTHREADS, smem, stream, p);
+    PB_LAUNCH("f2f_bwd_gfilter_one_tc", (f2f_one_sample_gfilter_kernel<NSPLIT>), p.nb1 * p.nb2 * p.groups * p.chunks, NTHREADS, smem, stream, p);
     return PB200_OK;
 }
 
@@ -535,7 +535,7 @@ int backward_filter(int64_t Nf, int Cin, int Cout, int F, const float* gout, con
     rc = operand_mode(precision).nsplit == 2 ? launch<2>(p, stream) : launch<1>(p, stream);
     if (rc) return rc;
     const int64_t items = (int64_t)p.nb1 * p.nb2 * p.tiles * p.N * 2;
-    PB_LAUNCH("f2f_bwd_gfilter_reduce", f2f_one_sample_gfilter_reduce_kernel, persistent_blocks(items, 1, 16), 256, 0, stream, p);
+    PB_LAUNCH("f2f_bwd_gfilter_one_reduce", f2f_one_sample_gfilter_reduce_kernel, persistent_blocks(items, 1, 16), 256, 0, stream, p);
     return PB200_OK;
 }
 

@@ -48,3 +48,25 @@ def test_one_sample_backward(nf, cin, cout, F, precision, gate):
     assert rel_err(gf, want_gf.reshape(cout, cin, F)) <= gate
     assert torch.equal(gin, again[0]) and torch.equal(gf, again[1])
     assert _lib.query("pb200_async_error") == 0
+
+
+@pytest.mark.parametrize("precision,F,cin,names", [
+    (_lib.PREC_FP32, 16, 64, {"f2f_bwd_gin_one_tc", "f2f_bwd_gfilter_one_tc", "f2f_bwd_gfilter_one_reduce"}),
+    (_lib.PREC_BF16, 25, 128, {"f2f_bwd_gin_one_tc", "f2f_bwd_gfilter_one_tc", "f2f_bwd_gfilter_one_reduce"}),
+    (_lib.PREC_FP32, 7, 48, {"f2f_gA_sgemm", "f2f_bwd_gfilter_one_tc"}),            # a basis count the product kernels are not built for
+    (_lib.PREC_TF32, 16, 64, {"f2f_bwd_gin_tc", "f2f_bwd_gfilter_tc"}),            # tf32 operands: the general kernels
+])
+def test_which_kernels_run(precision, F, cin, names):
+    x, go = torch.randn(300, cin, device="cuda"), torch.randn(300, 64, device="cuda")
+    w, filt = torch.rand(300, F, device="cuda"), torch.randn(64, cin, F, device="cuda")
+    _lib.prof_reset()
+    _lib.prof_enable(True)
+    try:
+        one_sample_backward(go, x, filt, w, precision)
+        torch.cuda.synchronize()
+    finally:
+        _lib.prof_enable(False)
+    ran = {n for n, _, _ in _lib.prof_read(64)}
+    _lib.prof_reset()
+    others = {"f2f_bwd_gin_tc", "f2f_bwd_gin_one_tc", "f2f_bwd_gfilter_tc", "f2f_bwd_gfilter_one_tc"} - names
+    assert names <= ran and not others & ran, ran
