@@ -406,13 +406,13 @@ f2v_bwd_blocked_kernel(int64_t Nf, int CV, int K, const int32_t* __restrict__ fa
             }
         }
         for (int g = 0; g < KG; ++g) {                         // rows past the tile are stale or zero: unused
-                            const float4 fa = sfilt[4 * g * LPF + l], fb = sfilt[(4 * g + 1) * LPF + l];
-                            const float4 fc = sfilt[(4 * g + 2) * LPF + l], fd = sfilt[(4 * g + 3) * LPF + l];
-            #pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const float4 cf = *reinterpret_cast<const float4*>(scoef + ((warp + 8 * i) * FPW + fs) * CP + 4 * g);
-                                fma4s(w[i], cf.x, fa); fma4s(w[i], cf.y, fb); fma4s(w[i], cf.z, fc); fma4s(w[i], cf.w, fd);
-                            }
+            const float4 fa = sfilt[4 * g * LPF + l], fb = sfilt[(4 * g + 1) * LPF + l];
+            const float4 fc = sfilt[(4 * g + 2) * LPF + l], fd = sfilt[(4 * g + 3) * LPF + l];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 cf = *reinterpret_cast<const float4*>(scoef + ((warp + 8 * i) * FPW + fs) * CP + 4 * g);
+                fma4s(w[i], cf.x, fa); fma4s(w[i], cf.y, fb); fma4s(w[i], cf.z, fc); fma4s(w[i], cf.w, fd);
+            }
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
