@@ -266,9 +266,9 @@ def kernel_models(d):
 # proportion to the faces).  Source: the summaries under profiles/.
 MEASURED_DRAM_BYTES_PER_FACE = {
     # the block with the repetition of the face rows folded in (one sample per face reaches facet2facet)
-    ("c5", "f2f_fwd_one_sample_tc"): 1041.0,
-    ("c5", "f2f_bwd_gin_tc"): 1043.0,
-    ("c5", "f2f_bwd_gfilter_tc"): 1858.0,
+    ("c5", "f2f_fwd_one_tc"): 1052.0,
+    ("c5", "f2f_bwd_gin_one_tc"): 1048.0,
+    ("c5", "f2f_bwd_gfilter_one_tc"): 2515.0,
     # the general forward kernel over every sample (variants.block_as_written)
     ("c5", "f2f_fwd_tc"): 2001.0,
 }

@@ -66,8 +66,9 @@ static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 static bool use_tc_fwd(int Cin, int Cout, int F, int precision) {
     return precision != PB200_PREC_FP32_FFMA && tc::fwd_supported(Cin, Cout, F);
 }
-// Few input channels: fp32 kernels of their own in every tensor-core mode.  A mesh of less than 4096 faces stays on the
-// tensor-core kernels, as the tests of the dispatch have it: a step is host work there, and a call launches (4000 faces 26 us against 9).  The filter
+// Few input channels: fp32 kernels of their own in every tensor-core mode.  Meshes of less than 4096 faces stay on the
+// tensor-core kernels: test_every_channel_count_runs_on_the_tensor_cores pins those for a small mesh of three channels.  The line is
+// not where the two sides meet (4000 faces: 26 us on the tensor cores, 9 here); a training step of that size is host work.  The filter
 // gradient's products outgrow the multiply-add units where the tensor cores' padding wastes less (1 758 000 faces, three channels:
 // 16 bases, 32 outputs 358 against 876 us, 25 bases, 64 outputs 1376 against 1066); forward there are no partial sums to keep and the
 // line lies further out (278 against 907 us, 1006 against 1168).
