@@ -1346,8 +1346,9 @@ mesh_decimation(const Tensor& vertex_in, const Tensor& face_in, const Tensor& ge
         const int64_t Nv2 = sum(nv_host), Nf2 = sum(mf_host);
         Tensor vertex2 = s.floats({Nv2, D}), face2 = at::empty({Nf2, 3}, i32), geometry2 = s.floats({Nf2, 5});
         // an empty result still needs addresses for the checks of the call; nothing is written there
-        call(pb200_decimate_finish(B, D, Nv, Nf, fp(vertex), ip(vt_replace), ip(vt_map), Nv2 ? fpm(vertex2) : fpm(geometry),
-                                   Nf2 ? face2.data_ptr<int32_t>() : sz, Nf2 ? fpm(geometry2) : fpm(geometry), ws.data_ptr(), nb, s.stream),
+        float* const nowhere = static_cast<float*>(ws.data_ptr());
+        call(pb200_decimate_finish(B, D, Nv, Nf, fp(vertex), ip(vt_replace), ip(vt_map), Nv2 ? fpm(vertex2) : nowhere,
+                                   Nf2 ? face2.data_ptr<int32_t>() : sz, Nf2 ? fpm(geometry2) : nowhere, ws.data_ptr(), nb, s.stream),
              "pb200_decimate_finish");
         if (!rep.defined()) {
             rep = vt_replace;

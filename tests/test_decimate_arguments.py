@@ -90,3 +90,20 @@ def test_vertices_kept_per_stride(stride):
     n = torch.arange(0, 300001, dtype=torch.int32, device="cuda")
     want = torch.clip((n.to(torch.float) / float(stride)).to(torch.int), min=4).tolist()
     assert MeshHierarchy([stride], [4], True, 1.0)._target(0, n.tolist()) == want
+
+
+@pytest.mark.gpu
+def test_meshes_without_faces():
+    """A vertex without a face is dropped: a batch, or a sample of it, that has none comes out empty."""
+    vertex, face, _, _, _ = host_batch()
+    v, f = vertex.cuda(), face[:80].cuda()
+    none = torch.zeros(0, 3, dtype=torch.int32, device="cuda")
+    out = dm.mesh_decimation_(v, none, torch.zeros(0, 5, device="cuda"), target(42, 42).cuda(), target(0, 0).cuda(), target(20, 20).cuda())
+    assert [tuple(t.shape) for t in out[:3]] == [(0, 3), (0, 3), (0, 5)]
+    assert out[3].tolist() == [0, 0] and out[4].tolist() == [0, 0] and out[6].tolist() == [-1] * 84
+    out = dm.mesh_decimation_(v, f, dm.compute_triangle_geometry_(v, f), target(42, 42).cuda(), target(80, 0).cuda(), target(20, 20).cuda())
+    w = v[:42].contiguous()
+    alone = dm.mesh_decimation_(w, f, dm.compute_triangle_geometry_(w, f), target(42).cuda(), target(80).cuda(), target(20).cuda())
+    assert out[3].tolist() == [int(alone[3]), 0] and all(torch.equal(a, b) for a, b in zip(out[:3], alone[:3]))
+    levels = MeshHierarchy([4], [4], True, 1.0)(v, none, target(42, 42).cuda(), target(0, 0).cuda())
+    assert levels[1][0].shape == (0, 3)
