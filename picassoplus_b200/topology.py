@@ -112,6 +112,8 @@ def _building(device):
 def _launch_build(face, vt_map, nv_in, nv_out):
     dev = face.device
     nf = face.shape[0]
+    if nf > 0 and (face.dim() != 2 or face.shape[1] != 3):
+        raise RuntimeError("face must have shape (NfIn, 3)")
     rowptr = torch.empty(nv_out + 1, dtype=torch.int32, device=dev)
     entries = torch.empty(max(3 * nf, 1), dtype=torch.int32, device=dev)
     status = torch.empty(1, dtype=torch.int32, device=dev)
@@ -256,6 +258,8 @@ def pair_csr(nn_index: torch.Tensor, column: int, n_rows: int) -> PairCSR:
     """Cached grouping of the neighbour pairs of a point-cloud convolution by their output point
     (column 0) or input point (column 1); same cache, budget and validation modes as vertex_csr."""
     npairs = nn_index.shape[0]
+    if npairs > 0 and (nn_index.dim() != 2 or nn_index.shape[1] != 2):
+        raise RuntimeError("nn_index must have shape (pairs, 2)")
     hit = _ops.cache_find(_PAIRS, nn_index, None, column, n_rows)
     if hit is not None:
         return hit

@@ -93,6 +93,28 @@ def test_input_points_with_many_pairs(F, C, T):
     assert torch.equal(again[0], gin) and torch.equal(again[1], gf)
 
 
+def test_pairs_and_faces_of_another_width_are_refused():
+    """Rows of one or three indices are told before the grouping reads them as rows of two, faces of two or four before the adjacency
+    reads them as triangles."""
+    from picassoplus_b200.mesh.layers import F2VConv3d, V2FConv3d
+    from picassoplus_b200.mesh.pi_modules import conv3d as mesh_conv
+    from picassoplus_b200.point.layers import PCloudConv3d
+    d = _dev(pcloud_inputs(200, 60, 12, 9, 8, 1, 0, seed=3))
+    layer = PCloudConv3d(8, 16, 9).cuda()
+    for index in (d["nn_index"][:, :1].contiguous(), torch.cat([d["nn_index"], d["nn_index"][:, :1]], 1)):
+        with pytest.raises(RuntimeError, match="pairs, 2"):
+            layer(d["x"], d["nn_count"], index, d["bin_index"])
+    x, ones = torch.randn(30, 8, device="cuda"), torch.ones(30, dtype=torch.int32, device="cuda")
+    for width in (2, 4):
+        face = torch.zeros(20, width, dtype=torch.int32, device="cuda")
+        rows, coeff = torch.randn(20, 8, device="cuda"), torch.rand(20, 9, device="cuda")
+        for call in (lambda: V2FConv3d(8, 16, 2).cuda()(x, face), lambda: F2VConv3d(8, 16, 2).cuda()(rows, face, ones, ones * 0, coeff),
+                     lambda: mesh_conv.vertex2facet(x.requires_grad_(), torch.randn(3, 8, 1, device="cuda"), face),
+                     lambda: mesh_conv.facet2vertex(rows, torch.randn(9, 8, 1, device="cuda"), coeff, face, ones, ones * 0)):
+            with pytest.raises(RuntimeError, match="NfIn, 3"):
+                call()
+
+
 @pytest.mark.parametrize("C", [32, 64, 128, 48])
 @pytest.mark.parametrize("T", [0, 3])
 def test_nan_reaches_every_bin_of_its_pairs(C, T):
