@@ -108,6 +108,7 @@ Tensor v2f_forward(const Scope& s, const Tensor& input, const Tensor& filter, co
 void v2f_backward(const Scope& s, const Tensor& g, const Tensor& input, const Tensor& filter, const Tensor& face,
                   const Tensor& rowptr, const Tensor& entries, Tensor& gin, Tensor& gf) {
     const int64_t Nv = input.size(0), C = input.size(1), r = filter.size(2), Nf = face.size(0);
+    if (!rowptr.defined()) fail("face holds an index outside the vertex range");       // (topology.for_backward)
     gin = s.floats({Nv, C});
     gf = s.floats({3, C, r});
     const size_t nb = pb200_vertex2facet_backward_workspace_bytes(Nf, Nv, (int)C, (int)r);
@@ -1120,6 +1121,7 @@ Tensor pairs_forward(const Scope& s, const Tensor& input, const Tensor& filter, 
 void pairs_backward(const Scope& s, const Tensor& g, const Tensor& input, const Tensor& filter, const Pairs& q, const Tensor& rowptr,
                     const Tensor& members, Tensor& gin, Tensor& gf) {
     const int64_t Np = input.size(0), C = input.size(1), F = filter.size(0), r = filter.size(2), Mp = q.nn_count.size(0), n = q.nn_index.size(0);
+    if (!rowptr.defined()) fail("nn_index holds an index outside the input points");    // (topology.for_backward)
     gin = s.floats({Np, C});
     gf = s.floats({F, C, r});
     const size_t nb = pb200_pcloud_conv3d_backward_workspace_bytes(n, (int)F, (int)C, (int)r);

@@ -11,7 +11,7 @@ from __future__ import annotations
 import torch
 
 from ... import _lib
-from ...topology import vertex_csr, ptr, stream_ptr
+from ...topology import for_backward, vertex_csr, ptr, stream_ptr
 
 _ops = _lib.ops
 
@@ -278,8 +278,9 @@ def vertex2facet(input, filter, face):
     rowptr = entries = None
     if torch.is_grad_enabled() and (input.requires_grad or filter.requires_grad):
         _check(face, "face", 2, torch.int32)
-        csr = vertex_csr(face, None, input.shape[0], input.shape[0])
-        rowptr, entries = csr.rowptr, csr.entries
+        csr = for_backward(vertex_csr, face, None, input.shape[0], input.shape[0])
+        if csr is not None:
+            rowptr, entries = csr.rowptr, csr.entries
     return _ops.vertex2facet(input, filter, face, rowptr, entries)
 
 

@@ -12,7 +12,7 @@ from __future__ import annotations
 import torch
 
 from ... import _lib
-from ...topology import ptr, stream_ptr, vertex_csr
+from ...topology import for_backward, ptr, stream_ptr, vertex_csr
 from . import conv3d
 
 _precision = _lib.PREC_FP32
@@ -62,8 +62,9 @@ def vertex2facet_layer(input, face, corners, spatial_weights, depth_weights, bia
     if torch.is_grad_enabled():
         conv3d._check(input, "input", 2, torch.float32)
         conv3d._check(face, "face", 2, torch.int32)
-        csr = vertex_csr(face, None, input.shape[0], input.shape[0])
-        rowptr, entries = csr.rowptr, csr.entries
+        csr = for_backward(vertex_csr, face, None, input.shape[0], input.shape[0])
+        if csr is not None:
+            rowptr, entries = csr.rowptr, csr.entries
     return _lib.ops.v2f_layer(input, face, rowptr, entries, corners, spatial_weights, depth_weights, biases, *tail, _precision)
 
 

@@ -12,7 +12,7 @@ import torch
 
 from ... import _lib
 from ...mesh.pi_modules.conv3d import _check
-from ...topology import pair_csr, ptr, stream_ptr
+from ...topology import for_backward, pair_csr, ptr, stream_ptr
 
 
 def _checks(input, filter, nn_count, nn_index, bin_index, bin_coeff):
@@ -116,7 +116,9 @@ def groupings(input, nn_count, nn_index, bin_index, bin_coeff):
     _check(nn_index, "nn_index", 2, torch.int32)
     by_out = pair_csr(nn_index, 0, nn_count.shape[0])
     if torch.is_grad_enabled():
-        by_in = pair_csr(nn_index, 1, input.shape[0])
+        by_in = for_backward(pair_csr, nn_index, 1, input.shape[0])
+        if by_in is None:
+            return by_out.rowptr, by_out.members, None, None
         return by_out.rowptr, by_out.members, by_in.rowptr, by_in.members
     return by_out.rowptr, by_out.members, None, None
 

@@ -21,7 +21,8 @@ default mode the status word is read back right after the build (ONE device sync
 per cache miss, which also answers whether `vtMap` is the identity) and a bad index raises
 RuntimeError.  `set_validation("deferred")` removes that synchronisation: status words are
 kept and `check_deferred()` reads them all at a point where the caller synchronises anyway
-(the end of a step).  Bad indices are never dereferenced in either mode.
+(the end of a step).  Bad indices are never dereferenced in either mode.  Arrays that only a backward pass
+reads are made ahead of it, in the forward pass; a bad index in them is reported by the backward pass.
 
 Streams and modes.  A structure found on another stream than the one that made it is waited for there; one made inside a
 graph capture is found inside that capture only.  Structures outlive the call that makes them and end up in autograd
@@ -78,6 +79,10 @@ def check_deferred() -> None:
     for code, (_, msg) in zip(codes, items):
         if code != 0:
             raise RuntimeError(msg)
+
+
+class BadIndex(RuntimeError):
+    """An index array holds an index outside its range."""
 
 
 class VertexCSR:
@@ -137,7 +142,7 @@ def build_vertex_csr(face: torch.Tensor, vt_map: Optional[torch.Tensor], nv_in: 
             with _lock:
                 _deferred.append((status, _bad_index_message(nv_in, nv_out)))
         elif int(status.item()) != 0:
-            raise RuntimeError(_bad_index_message(nv_in, nv_out))
+            raise BadIndex(_bad_index_message(nv_in, nv_out))
     return VertexCSR(rowptr, entries)
 
 
@@ -159,7 +164,7 @@ def vertex_csr(face: torch.Tensor, vt_map: Optional[torch.Tensor], nv_in: int, n
                 rowptr, entries, status = _launch_build(face, None, nv_in, nv_out)
                 code, is_ident = torch.stack([status[0], ident]).tolist()
                 if code != 0:
-                    raise RuntimeError(_bad_index_message(nv_in, nv_out))
+                    raise BadIndex(_bad_index_message(nv_in, nv_out))
                 base = VertexCSR(rowptr, entries)
                 _store(_VERTEX, face, None, nv_in, nv_out, base)
             else:
@@ -194,10 +199,19 @@ def prepare_level(vertex: torch.Tensor, face: torch.Tensor, vt_map: Optional[tor
         with _lock:
             _deferred.append((status, _bad_index_message(nv_in, nv_out)))
     elif int(status.item()) != 0:
-        raise RuntimeError(_bad_index_message(nv_in, nv_out))
+        raise BadIndex(_bad_index_message(nv_in, nv_out))
     csr = VertexCSR(rowptr, entries)
     _store(_VERTEX, face, vt_map, nv_in, nv_out, csr)
     return dict(geometry=geometry, normals=normals, coeff=coeff, nf_count=nf_count, csr=csr)
+
+
+def for_backward(structure, *args):
+    """structure(*args) that only a backward pass reads, or None when it raises BadIndex: the forward pass, in which such an index
+    contributes nothing, is not refused for it; the node's backward pass is."""
+    try:
+        return structure(*args)
+    except BadIndex:
+        return None
 
 
 class ClusterCSR:
@@ -278,7 +292,7 @@ def pair_csr(nn_index: torch.Tensor, column: int, n_rows: int) -> PairCSR:
             with _lock:
                 _deferred.append((status, msg))
         elif int(status.item()) != 0:
-            raise RuntimeError(msg)
+            raise BadIndex(msg)
     csr = PairCSR(rowptr, members)
     _store(_PAIRS, nn_index, None, column, n_rows, csr)
     return csr

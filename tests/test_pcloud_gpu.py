@@ -93,6 +93,29 @@ def test_input_points_with_many_pairs(F, C, T):
     assert torch.equal(again[0], gin) and torch.equal(again[1], gf)
 
 
+def test_a_bad_index_that_only_the_backward_pass_looks_up():
+    """An input point or vertex outside the range contributes nothing to a forward pass, under autograd or not; the backward pass, which
+    sorts by it, refuses it."""
+    from picassoplus_b200.mesh.layers import V2FConv3d
+    from picassoplus_b200.mesh.pi_modules import conv3d as mesh_conv
+    from picassoplus_b200.point.layers import PCloudConv3d
+    from picassoplus_b200.point.pi_modules import conv3d
+    d = _dev(pcloud_inputs(200, 60, 12, 9, 8, 1, 0, seed=3))
+    layer, x, w = PCloudConv3d(8, 16, 9).cuda().eval(), d["x"].requires_grad_(), torch.randn(9, 8, 1, device="cuda", requires_grad=True)
+    d["nn_index"][5, 1] = 200
+    pairs = d["nn_count"], d["nn_index"], d["bin_index"]
+    face = torch.randint(0, 200, (50, 3), dtype=torch.int32, device="cuda")
+    face[7, 2] = 200
+    faces, f = V2FConv3d(8, 16, 2).cuda().eval(), torch.randn(3, 8, 1, device="cuda", requires_grad=True)
+    for call in (lambda: layer(x, *pairs), lambda: conv3d.conv3d(x, w, *pairs), lambda: faces(x, face), lambda: mesh_conv.vertex2facet(x, f, face)):
+        with torch.no_grad():
+            want = call()
+        out = call()
+        assert rel_err(out, want) <= 1e-5
+        with pytest.raises(RuntimeError, match="outside"):
+            torch.autograd.grad(out, [x], torch.ones_like(out))
+
+
 def test_pairs_and_faces_of_another_width_are_refused():
     """Rows of one or three indices are told before the grouping reads them as rows of two, faces of two or four before the adjacency
     reads them as triangles."""
