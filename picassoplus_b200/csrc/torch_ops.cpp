@@ -105,10 +105,14 @@ Tensor v2f_forward(const Scope& s, const Tensor& input, const Tensor& filter, co
     return out;
 }
 
+// what a backward pass says of an adjacency that could not be made (topology.for_backward)
+constexpr const char* BAD_FACE = "face holds an index outside the vertex range";
+constexpr const char* BAD_PAIR = "nn_index holds an index outside the input points";
+
 void v2f_backward(const Scope& s, const Tensor& g, const Tensor& input, const Tensor& filter, const Tensor& face,
                   const Tensor& rowptr, const Tensor& entries, Tensor& gin, Tensor& gf) {
     const int64_t Nv = input.size(0), C = input.size(1), r = filter.size(2), Nf = face.size(0);
-    if (!rowptr.defined()) fail("face holds an index outside the vertex range");       // (topology.for_backward)
+    if (!rowptr.defined()) fail(BAD_FACE);
     gin = s.floats({Nv, C});
     gf = s.floats({3, C, r});
     const size_t nb = pb200_vertex2facet_backward_workspace_bytes(Nf, Nv, (int)C, (int)r);
@@ -659,6 +663,7 @@ struct V2FLayer : Node {
         std::lock_guard<std::mutex> lock(mutex_);
         const Tensor x = input.unpack(), eye = corners.unpack();
         Scope s(x);
+        if (!rowptr.unpack().defined()) fail(BAD_FACE);
         StageGrads r = stage_backward(s, upstream(grads), act.unpack(shared_from_this()), features.unpack(), weights.unpack(), NormStats{mean.unpack(), invstd.unpack()},
                                       gamma.unpack(), relu,
                                       task_should_compute_output(0) || task_should_compute_output(1), precision);
@@ -1121,7 +1126,7 @@ Tensor pairs_forward(const Scope& s, const Tensor& input, const Tensor& filter, 
 void pairs_backward(const Scope& s, const Tensor& g, const Tensor& input, const Tensor& filter, const Pairs& q, const Tensor& rowptr,
                     const Tensor& members, Tensor& gin, Tensor& gf) {
     const int64_t Np = input.size(0), C = input.size(1), F = filter.size(0), r = filter.size(2), Mp = q.nn_count.size(0), n = q.nn_index.size(0);
-    if (!rowptr.defined()) fail("nn_index holds an index outside the input points");    // (topology.for_backward)
+    if (!rowptr.defined()) fail(BAD_PAIR);
     gin = s.floats({Np, C});
     gf = s.floats({F, C, r});
     const size_t nb = pb200_pcloud_conv3d_backward_workspace_bytes(n, (int)F, (int)C, (int)r);
@@ -1176,6 +1181,7 @@ struct PointLayer : PairsNode {
                      g = aligned(upstream(grads));
         const NormStats st{mean.unpack(), invstd.unpack()};
         Scope s(x);
+        if (!rowptr.unpack().defined()) fail(BAD_PAIR);
         NormGrads n;
         if (st.mean.defined()) {
             n = norm_backward(s, g, a, st, gamma.unpack());

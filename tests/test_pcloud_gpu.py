@@ -114,6 +114,9 @@ def test_a_bad_index_that_only_the_backward_pass_looks_up():
         assert rel_err(out, want) <= 1e-5
         with pytest.raises(RuntimeError, match="outside"):
             torch.autograd.grad(out, [x], torch.ones_like(out))
+    for m, rest in ((layer, pairs), (faces, (face,))):        # also where only the layer's weights have a gradient
+        with pytest.raises(RuntimeError, match="outside"):
+            torch.autograd.grad(m(x.detach(), *rest).sum(), [m.depth_weights])
 
 
 def test_pairs_and_faces_of_another_width_are_refused():
