@@ -265,7 +265,7 @@ class GlobalPool3d(nn.Module):
     def forward(self, inputs, nv_in):
         if self.method == 'avg':
             if (inputs.is_cuda and inputs.dtype == torch.float32 and inputs.dim() == 2 and nv_in.dim() == 1 and
-                    nv_in.device == inputs.device and _lib.native_calls()):
+                    nv_in.shape[0] > 0 and nv_in.device == inputs.device and _lib.native_calls()):
                 return _lib.ops.segment_mean(inputs.contiguous(), sample_ends(nv_in, inputs.shape[0]))
             return torch.segment_reduce(inputs, 'mean', lengths=nv_in.to(torch.int64))
         if self.method == 'max':

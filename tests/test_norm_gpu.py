@@ -96,6 +96,8 @@ def test_global_mean(lengths, C):
     assert rel_err(gx, torch.repeat_interleave(g / nv[:, None], nv.long(), 0)) <= 1e-6
     with pytest.raises(RuntimeError):
         GlobalPool3d("avg")(x, nv + 1)
+    with pytest.raises(RuntimeError):
+        GlobalPool3d("avg")(x[:0], nv[:0])                  # no samples at all: torch's operator refuses them
 
 
 @pytest.mark.parametrize("lengths", [[300, 900, 1200], [100, -4000, 500], [5000000, 1, 1], [-5, 1000, 5]])
