@@ -655,7 +655,7 @@ void check_stage(const Tensor& weights, int64_t C) {
 
 struct V2FLayer : Node {
     SavedVariable input, filter, corners, face, rowptr, entries, weights, act, features, mean, invstd, gamma;
-    bool relu = false;
+    bool relu = false, sorted = true;                          // sorted: there are rowptr and entries
     int precision = 0;
     variable_list apply(variable_list&& grads) override {
         variable_list out(6);
@@ -663,7 +663,7 @@ struct V2FLayer : Node {
         std::lock_guard<std::mutex> lock(mutex_);
         const Tensor x = input.unpack(), eye = corners.unpack();
         Scope s(x);
-        if (!rowptr.unpack().defined()) fail(BAD_FACE);
+        if (!sorted) fail(BAD_FACE);
         StageGrads r = stage_backward(s, upstream(grads), act.unpack(shared_from_this()), features.unpack(), weights.unpack(), NormStats{mean.unpack(), invstd.unpack()},
                                       gamma.unpack(), relu,
                                       task_should_compute_output(0) || task_should_compute_output(1), precision);
@@ -817,6 +817,7 @@ Tensor v2f_layer(const Tensor& x_in, const Tensor& face, const OptTensor& rowptr
         node->corners = keep(corners);
         node->face = keep(face);
         node->rowptr = keep(or_undefined(rowptr));
+        node->sorted = rowptr.has_value();
         node->entries = keep(or_undefined(entries));
         node->weights = keep(weights_in);
         node->features = keep(r.features);
@@ -1139,6 +1140,7 @@ void pairs_backward(const Scope& s, const Tensor& g, const Tensor& input, const 
 
 struct PairsNode : Node {
     SavedVariable input, filter, nn_count, nn_index, bin_index, bin_coeff, rowptr, members;
+    bool sorted = true;                                        // there are rowptr and members
     void keep_pairs(const Tensor& x, const Tensor& f, const Pairs& q, const Tensor& by_in_rowptr, const Tensor& by_in_members) {
         input = keep(x);
         filter = keep(f);
@@ -1147,6 +1149,7 @@ struct PairsNode : Node {
         bin_index = keep(q.bin_index);
         bin_coeff = keep(q.bin_coeff);
         rowptr = keep(by_in_rowptr);
+        sorted = by_in_rowptr.defined();
         members = keep(by_in_members);
     }
     void pairs_gradient(const Scope& s, const Tensor& g, const Tensor& x, Tensor& gin, Tensor& gf) {
@@ -1181,7 +1184,7 @@ struct PointLayer : PairsNode {
                      g = aligned(upstream(grads));
         const NormStats st{mean.unpack(), invstd.unpack()};
         Scope s(x);
-        if (!rowptr.unpack().defined()) fail(BAD_PAIR);
+        if (!sorted) fail(BAD_PAIR);
         NormGrads n;
         if (st.mean.defined()) {
             n = norm_backward(s, g, a, st, gamma.unpack());
