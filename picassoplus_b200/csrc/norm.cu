@@ -40,7 +40,11 @@ template <int V> __device__ __forceinline__ void store(float* p, const Vec<V>& x
 }
 
 // ReLU as torch has it: a NaN stays one, forward and backward
-__device__ __forceinline__ float relu_of(float x) { return x > 0.f || x != x ? x : 0.f; }
+__device__ __forceinline__ float relu_of(float x) {
+    float y;
+    asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(y) : "f"(x));
+    return y;
+}
 __device__ __forceinline__ float relu_grad(float g, float act) { return act <= 0.f ? 0.f : g; }
 
 struct Moments { float n, mean, m2; };
