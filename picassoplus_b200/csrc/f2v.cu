@@ -290,172 +290,283 @@ f2v_bwd_tile_kernel(int64_t Nf, int CV, int K, const int32_t* __restrict__ face,
         if (ak[n] >= 0) partial[((int64_t)blockIdx.x * K + ak[n]) * CV + cg0 + ac[n]] = acc[n];
 }
 
-// The same two phases register-blocked, for K <= 32: a face's channels lie on LPF lanes (float4 each; LPF = 4, 8, 16, 32, chunks of
-// 32 behind that), a warp has 32 / LPF faces side by side and four such passes per tile.
-//   phase 1  a filter row read from shared memory is used for the four passes' faces;
-//   phase 2  a warp owns four coefficients and, while K leaves warps over, a share of the tile's faces: a row of t read from shared
-//            memory feeds four accumulators.
-// What bounds it: shared memory (70 % busy at 128 channels) and the three barriers of a tile; packed multiply-adds on coefficients
-// kept twice changed nothing.  A kernel without register blocking served all widths that are no multiple of 128 before:
-// 1 954 000 faces, 64 channels, K = 16 960 -> 606 us; 977 000 faces, 48 channels, K = 9 408 -> 286 us, 100 channels 817 -> 561.
-// The index chain of the gather (face -> vtMap -> nfCount) is resolved one hop per tile for the block's next three tiles, so that
-// phase 1 finds output vertex and 1/nfCount of every corner in shared memory and issues its twelve gradOutput row loads at once.
-template <int LPF> constexpr int F2VB_FACES = 32 * (32 / LPF);         // faces of a tile
-template <int LPF>
-static size_t f2vb_smem(int K) {
-    return sizeof(float4) * ((size_t)(K + 3) / 4 * 4 * LPF + F2VB_FACES<LPF> * LPF) + sizeof(float) * 2 * F2VB_FACES<LPF> * f2v_pitch<LPF>(K) +
-           2 * F2VB_FACES<LPF> * 3 * 8;
+// K <= 32: a lane keeps NC channels for the whole kernel, with their K filter values and K filter-gradient sums in registers, and
+// walks faces: the only operands of the 2 K multiply-adds of a face and channel that come out of shared memory are the K coefficients,
+// read once for both sums and broadcast to the warp.  Coefficients, filter and sums go in pairs (k, k + 1), so that the products are
+// packed (fma.rn.f32x2) without an operand kept twice.  A face's channels lie on LPF lanes (4, 8, 16, 32; chunks behind that on
+// blockIdx.y), a warp has FPW = 32 / LPF faces side by side and four such passes per stage.  Warps share nothing: each has a ring of
+// stages of its own (three gradOutput rows, the input row and the coefficients of every face) that asynchronous copies fill, and
+// resolves the index chain face -> vtMap -> nfCount one hop per stage ahead of them.
+// What bounds it: instructions (126 per warp and face at 16 coefficients, 64 of them multiply-adds) with 8 to 12 warps per SM.  A kernel
+// that read filter, coefficients and products from shared memory for every step (register blocks of 4 faces, three block barriers per
+// tile) took, per call with a cold L2: 879 000 faces, 64 channels, K = 16 247 us (now 148, copy floor 98); 464 000 faces, 128 channels,
+// K = 25 308 (257, floor 101); 879 000 faces, 48 channels, K = 9 226 (165), 32 channels, K = 25 200 (136), 16 channels, K = 16 118 (60).
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void* dst_smem, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src), "n"(BYTES)
+                 : "memory");
+}
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void* dst_smem, const void* src, bool on) {      // off: zeros
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src),
+                 "n"(BYTES), "r"(on ? BYTES : 0) : "memory");
+}
+__device__ __forceinline__ uint64_t pair2(float lo, float hi) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float2 unpair2(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
 
-template <int LPF>
-__global__ void __launch_bounds__(256, 2)
-f2v_bwd_blocked_kernel(int64_t Nf, int CV, int K, const int32_t* __restrict__ face, const int32_t* __restrict__ vtMap,
-                       const int32_t* __restrict__ nfCount, const float* __restrict__ coeff,
-                       const float4* __restrict__ in, const float4* __restrict__ filt, const float4* __restrict__ gout,
-                       float4* __restrict__ gin, float4* __restrict__ partial) {
-    extern __shared__ float4 smem[];
-    constexpr int FPW = 32 / LPF, TF = F2VB_FACES<LPF>, NE = TF * 3, NI = (NE + 255) / 256;
-    const int KG = (K + 3) / 4, CP = f2v_pitch<LPF>(K);            // groups of 4 coefficients (<= 8)
-    float4* sfilt = smem;                                      // [4 KG][LPF], rows K.. zero
-    float4* st = smem + 4 * KG * LPF;                          // [TF][LPF]   t = input * gt
-    float* scoef0 = reinterpret_cast<float*>(st + TF * LPF);   // [2][TF][CP], double-buffered (asynchronous copies)
-    int* svo = reinterpret_cast<int*>(scoef0 + 2 * TF * CP);   // [2][NE] output vertex of (face, corner), -1 = none
-    float* srn = reinterpret_cast<float*>(svo + 2 * NE);       // [2][NE] 1 / nfCount of that vertex
+// Shape by the number of coefficient pairs P.  Registers decide: filter and sums take 4 P NC of them, so up to 16 coefficients a lane holds
+// four channels, above that two (25 coefficients, 4 channels: 269 instead of 257 us, with nothing left to overlap loads).  Two stages:
+// a third one, or longer ones, take from the L1 that serves the gradOutput rows which neighbouring faces share (16 coefficients: 148
+// us with 2 x 4 passes, 171 with 3 x 4, 179 with 2 x 6).
+template <int P> constexpr int F2VL_NC = P <= 8 ? 4 : 2;                              // channels of a lane
+template <int P> constexpr int F2VL_BLOCKS = P <= 8 ? 2 : P <= 13 ? 3 : 2;            // blocks per SM
+constexpr int F2VL_WARPS = 4, F2VL_PASSES = 4, F2VL_STAGES = 2;
+template <int LPF> constexpr int F2VL_FACES = F2VL_PASSES * (32 / LPF);             // faces of a stage
+// floats of a coefficient row: quads, and rows of faces side by side on different banks
+template <int P> constexpr int F2VL_PITCH = (2 * P + 3) / 4 * 4 % 16 == 0 ? (2 * P + 3) / 4 * 4 + 4 : (2 * P + 3) / 4 * 4;
+template <int NC> struct F2VLVec { using type = float2; };
+template <> struct F2VLVec<4> { using type = float4; };
+template <int P, int LPF> struct F2VLStage {
+    typename F2VLVec<F2VL_NC<P>>::type row[F2VL_PASSES][4][32];                            // gradOutput of the corners 0..2, input; a lane's own channels
+    alignas(16) float coef[F2VL_FACES<LPF> * F2VL_PITCH<P>];
+    int4 vo[F2VL_FACES<LPF>];                                  // output vertices of the corners (-1: none) ...
+    float4 rn[F2VL_FACES<LPF>];                                // ... and 1 / nfCount of them
+};
+
+template <int P, int LPF>
+__global__ void __launch_bounds__(32 * F2VL_WARPS, F2VL_BLOCKS<P>)
+f2v_bwd_lane_kernel(int64_t Nf, int C, int K, const int32_t* __restrict__ face, const int32_t* __restrict__ vtMap,
+                    const int32_t* __restrict__ nfCount, const float* __restrict__ coeff, const float* __restrict__ in,
+                    const float* __restrict__ filt, const float* __restrict__ gout, float* __restrict__ gin,
+                    float* __restrict__ partial) {
+    extern __shared__ __align__(16) unsigned char f2vl_smem[];
+    using Stage = F2VLStage<P, LPF>;
+    constexpr int FPW = 32 / LPF, TF = F2VL_FACES<LPF>, NE = 3 * TF, NI = (NE + 31) / 32, CP = F2VL_PITCH<P>, D = F2VL_STAGES;
+    constexpr int NC = F2VL_NC<P>;
+    using Vec = typename F2VLVec<NC>::type;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int l = lane % LPF, fs = lane / LPF;                 // channel group, face among the warp's
-    const int cg = blockIdx.y * LPF + l;
-    const bool on = cg < CV;
-    for (int i = threadIdx.x; i < 4 * KG * LPF; i += blockDim.x) {
-        const int k = i / LPF, c = blockIdx.y * LPF + i % LPF;
-        sfilt[i] = k < K && c < CV ? filt[k * CV + c] : zero4();
-    }
-    for (int i = threadIdx.x; i < 2 * TF * CP; i += blockDim.x) scoef0[i] = 0.f;
-    // phase 2: coefficients 4g..4g+3, faces fs + FPW * (slice + slices * i)
-    const int slices = 8 / KG, g2 = warp % KG, slice = warp / KG;
-    float4 acc[4] = {zero4(), zero4(), zero4(), zero4()};
+    const int l = lane % LPF, fs = lane / LPF;                 // channel pair, face among the warp's
+    const bool on = (blockIdx.y * LPF + l) * NC < C;
+    const int ch = on ? (blockIdx.y * LPF + l) * NC : 0;        // lanes without channels follow and store nothing
+    Stage* ring = reinterpret_cast<Stage*>(f2vl_smem) + warp * D;
+
+    uint64_t f2[NC][P], acc[NC][P];
+#pragma unroll
+    for (int p = 0; p < P; ++p)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const float lo = 2 * p < K ? __ldg(filt + (2 * p) * C + ch + c) : 0.f;
+            const float hi = 2 * p + 1 < K ? __ldg(filt + (2 * p + 1) * C + ch + c) : 0.f;
+            f2[c][p] = pair2(lo, hi);
+            acc[c][p] = 0;
+        }
+    for (int s = 0; s < D; ++s)                                // columns K.. stay zero
+        for (int i = lane; i < TF * CP; i += 32) ring[s].coef[i] = 0.f;
+    __syncwarp();
+
     const int64_t ntiles = (Nf + TF - 1) / TF;
-    // index pipeline (entry e = 3*face + corner of a tile): vertex id of the tile three steps ahead, output vertex two steps
-    // ahead, 1/nfCount one step ahead
+    const int tstep = gridDim.x * F2VL_WARPS;
+    const int64_t tile0 = (int64_t)blockIdx.x * F2VL_WARPS + warp;
+    const bool quads = K == 2 * P && P % 2 == 0 && (reinterpret_cast<uintptr_t>(coeff) & 15) == 0;
+    const int row_bytes = C * 4;
+    const char* const gout_lane = reinterpret_cast<const char*>(gout + ch);
+
     auto hop_face = [&](int64_t tile, int i) -> int {
-        const int e = threadIdx.x + 256 * i;
+        const int e = lane + 32 * i;
         const int64_t at = tile * NE + e;
-        return (e < NE && tile < ntiles && at < Nf * 3) ? __ldg(face + at) : -1;
+        return (e < NE && at < Nf * 3) ? __ldg(face + at) : -1;
     };
     auto hop_vo = [&](int vi) -> int { return vi < 0 ? -1 : (vtMap ? __ldg(vtMap + vi) : vi); };
-    auto hop_rn = [&](int vo) -> float { return vo < 0 ? 0.f : __frcp_rn((float)__ldg(nfCount + vo)); };
-    auto park = [&](int b, int i, int vo, float rn) {
-        const int e = threadIdx.x + 256 * i;
-        if (e < NE) { svo[b * NE + e] = vo; srn[b * NE + e] = rn; }
+    auto hop_n = [&](int vo) -> int { return vo < 0 ? 0 : __ldg(nfCount + vo); };
+    auto park = [&](Stage& s, int i, int vo, int n) {
+        const int e = lane + 32 * i;
+        if (e < NE) {
+            reinterpret_cast<int*>(s.vo)[e + e / 3] = vo;
+            reinterpret_cast<float*>(s.rn)[e + e / 3] = vo < 0 ? 0.f : __frcp_rn((float)n);
+        }
     };
-    const int64_t tstep = gridDim.x;
-    int vo1[NI], vi2[NI];
+    // The copies of a tile, whose corners are parked.  `whole`: all its faces and corners are there; otherwise zeros stand for
+    // what is not.
+    auto fetch = [&](Stage& s, int64_t tile, bool whole) {
+        const int64_t f0 = tile * TF;
+        if (whole) {
+            const char* in_lane = reinterpret_cast<const char*>(in + (f0 + fs) * C + ch);
 #pragma unroll
-    for (int i = 0; i < NI; ++i) {
-        const int vo = hop_vo(hop_face(blockIdx.x, i));        // first tile: resolved up front
-        park(0, i, vo, hop_rn(vo));
-        vo1[i] = hop_vo(hop_face(blockIdx.x + tstep, i));      // second tile
-        vi2[i] = hop_face(blockIdx.x + 2 * tstep, i);          // third tile
-    }
-    auto fetch_coef = [&](int64_t tile, int b) {               // a lane per coefficient; the pad columns stay zero
-        if (tile < ntiles && lane < K) {
-            const int64_t f0 = tile * TF;
+            for (int p = 0; p < F2VL_PASSES; ++p) {
+                const int4 vo = s.vo[p * FPW + fs];
+                cp_async<4 * NC>(&s.row[p][0][lane], gout_lane + (int64_t)vo.x * row_bytes);
+                cp_async<4 * NC>(&s.row[p][1][lane], gout_lane + (int64_t)vo.y * row_bytes);
+                cp_async<4 * NC>(&s.row[p][2][lane], gout_lane + (int64_t)vo.z * row_bytes);
+                cp_async<4 * NC>(&s.row[p][3][lane], in_lane);
+                in_lane += FPW * row_bytes;
+            }
+        } else if (tile < ntiles) {
+#pragma unroll 1
+            for (int p = 0; p < F2VL_PASSES; ++p) {
+                const int fl = p * FPW + fs;
+                const int* vo = reinterpret_cast<const int*>(s.vo + fl);
+#pragma unroll 1
+                for (int j = 0; j < 3; ++j)
+                    cp_async<4 * NC>(&s.row[p][j][lane], vo[j] >= 0 ? gout_lane + (int64_t)vo[j] * row_bytes : gout_lane, vo[j] >= 0);
+                const bool there = f0 + fl < Nf;
+                cp_async<4 * NC>(&s.row[p][3][lane], there ? in + (f0 + fl) * C + ch : in, there);
+            }
+        }
+        if (tile < ntiles) {
             const int nf_tile = Nf - f0 < TF ? (int)(Nf - f0) : TF;
-            const float* src = coeff + f0 * K + lane;
-            float* sc = scoef0 + b * TF * CP + lane;
-            for (int fl = warp; fl < nf_tile; fl += 8) cp_async4(sc + fl * CP, src + fl * K);
+            if (quads) {
+                constexpr int Q = P / 2 > 0 ? P / 2 : 1;       // quads of a row
+#pragma unroll
+                for (int i0 = 0; i0 < TF * Q; i0 += 32) {
+                    const int i = i0 + lane, fl = i / Q, q = i % Q;
+                    const bool there = i < nf_tile * Q;
+                    if (i < TF * Q) cp_async<16>(s.coef + fl * CP + 4 * q, coeff + (there ? f0 * K + 4 * i : 0), there);
+                }
+            } else if (lane < K) {
+                const float* src = coeff + f0 * K + lane;
+                if (whole) {
+#pragma unroll
+                    for (int fl = 0; fl < TF; ++fl, src += K) cp_async<4>(s.coef + fl * CP + lane, src);
+                } else
+#pragma unroll 1
+                    for (int fl = 0; fl < TF; ++fl, src += K) cp_async<4>(s.coef + fl * CP + lane, fl < nf_tile ? src : coeff, fl < nf_tile);
+            }
         }
         cp_async_commit();
     };
-    __syncthreads();                                           // the zero fill above is complete
-    fetch_coef(blockIdx.x, 0);
-    int buf = 0;
-    for (int64_t tile = blockIdx.x; tile < ntiles; tile += tstep, buf ^= 1) {
-        const int64_t f0 = tile * TF;
-        const int nf_tile = Nf - f0 < TF ? (int)(Nf - f0) : TF;
-        // one hop for each of the next three tiles (results are used in the next iteration)
-        float rn_next[NI];
-        int vo_next[NI], vi_next[NI];
+    auto all_there = [&](int64_t tile, const int (&vo)[NI]) {
+        bool mine = true;
+#pragma unroll
+        for (int i = 0; i < NI; ++i) mine = mine && (vo[i] >= 0 || lane + 32 * i >= NE);
+        return __all_sync(0xffffffffu, mine) && (tile + 1) * TF <= Nf;
+    };
+
+    // prologue: the first D - 1 tiles resolved up front, then the chain of the three behind them
+    int vo0[NI], n0[NI], vo1[NI], vi2[NI];
+    bool whole[D];
+#pragma unroll
+    for (int s = 0; s < D - 1; ++s) {
+        int vo[NI];
 #pragma unroll
         for (int i = 0; i < NI; ++i) {
-            rn_next[i] = hop_rn(vo1[i]);
+            vo[i] = hop_vo(hop_face(tile0 + s * tstep, i));
+            park(ring[s], i, vo[i], hop_n(vo[i]));
+        }
+        whole[s] = all_there(tile0 + s * tstep, vo);
+    }
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+        vo0[i] = hop_vo(hop_face(tile0 + (D - 1) * tstep, i));
+        n0[i] = hop_n(vo0[i]);
+        vo1[i] = hop_vo(hop_face(tile0 + D * tstep, i));
+        vi2[i] = hop_face(tile0 + (D + 1) * tstep, i);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int s = 0; s < D - 1; ++s) fetch(ring[s], tile0 + s * tstep, whole[s]);
+
+    int now = 0, next = D - 1;                                 // stages: of this tile, of tile + (D - 1) tstep
+    for (int64_t tile = tile0; tile < ntiles; tile += tstep) {
+        int n_next[NI], vo_next[NI], vi_next[NI];
+        const bool next_whole = all_there(tile + (D - 1) * tstep, vo0);
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            park(ring[next], i, vo0[i], n0[i]);
+            n_next[i] = hop_n(vo1[i]);
             vo_next[i] = hop_vo(vi2[i]);
-            vi_next[i] = hop_face(tile + 3 * tstep, i);
+            vi_next[i] = hop_face(tile + (D + 2) * tstep, i);
         }
-        __syncthreads();                                       // previous tile fully consumed
-        fetch_coef(tile + tstep, buf ^ 1);                     // the next tile's coefficient rows, asynchronously
-        cp_async_wait<1>();                                    // this tile's rows have landed (own copies) ...
-        __syncthreads();                                       // ... and everybody else's
-        const float* scoef = scoef0 + buf * TF * CP;
-        // ---- phase 1: faces (warp + 8 i) * FPW + fs
-        // all sixteen row loads of the thread are issued first; the filter sums below need only the coefficients and run
-        // while the rows are on their way
-        float4 x[4], w[4], gr[4][3];
+        cp_async_wait<D - 2>();                                // this tile's copies have landed (own ones) ...
+        __syncwarp();                                          // ... and the other lanes'; the next corners are parked
+        fetch(ring[next], tile + (D - 1) * tstep, next_whole);
+        const Stage& s = ring[now];
+        const int64_t f0 = tile * TF;
+        const int left = on ? (int)(Nf - f0 < TF ? Nf - f0 : TF) - fs : 0;          // this lane stores while p FPW < left
+        char* gin_lane = reinterpret_cast<char*>(gin + (f0 + fs) * C + ch);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int fl = (warp + 8 * i) * FPW + fs;
-            x[i] = zero4(); w[i] = zero4();
+        for (int p = 0; p < F2VL_PASSES; ++p) {
+            const float4 rn = s.rn[p * FPW + fs];
+            const Vec g0 = s.row[p][0][lane], g1 = s.row[p][1][lane], g2 = s.row[p][2][lane], x = s.row[p][3][lane];
+            float gt[NC];
+            uint64_t t[NC], w[NC];
 #pragma unroll
-            for (int j = 0; j < 3; ++j) gr[i][j] = zero4();
-            if (on && fl < nf_tile) {
+            for (int c = 0; c < NC; ++c) {
+                auto at = [&](const Vec& v) { return reinterpret_cast<const float*>(&v)[c]; };
+                gt[c] = fmaf(rn.z, at(g2), fmaf(rn.y, at(g1), rn.x * at(g0)));
+                const float tc = at(x) * gt[c];
+                t[c] = pair2(tc, tc);
+            }
+            const float* cf = s.coef + (p * FPW + fs) * CP;
 #pragma unroll
-                for (int j = 0; j < 3; ++j) {
-                    const int vo = svo[buf * NE + fl * 3 + j];
-                    if (vo >= 0) gr[i][j] = ldg4(gout + (int64_t)vo * CV + cg);
+            for (int q = 0; q < P; q += 2) {
+                const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(cf + 2 * q);
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    if (q == 0) w[c] = mul2(k.x, f2[c][0]);
+                    else fma2(w[c], k.x, f2[c][q]);
+                    fma2(acc[c][q], k.x, t[c]);
+                    if (q + 1 < P) {
+                        fma2(w[c], k.y, f2[c][q + 1]);
+                        fma2(acc[c][q + 1], k.y, t[c]);
+                    }
                 }
-                x[i] = ldg4(in + (f0 + fl) * CV + cg);
             }
-        }
-        for (int g = 0; g < KG; ++g) {                         // rows past the tile are stale or zero: unused
-            const float4 fa = sfilt[4 * g * LPF + l], fb = sfilt[(4 * g + 1) * LPF + l];
-            const float4 fc = sfilt[(4 * g + 2) * LPF + l], fd = sfilt[(4 * g + 3) * LPF + l];
+            Vec g;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float4 cf = *reinterpret_cast<const float4*>(scoef + ((warp + 8 * i) * FPW + fs) * CP + 4 * g);
-                fma4s(w[i], cf.x, fa); fma4s(w[i], cf.y, fb); fma4s(w[i], cf.z, fc); fma4s(w[i], cf.w, fd);
+            for (int c = 0; c < NC; ++c) {
+                const float2 a = unpair2(w[c]);
+                reinterpret_cast<float*>(&g)[c] = gt[c] * (a.x + a.y);
             }
+            if (p * FPW < left) __stcs(reinterpret_cast<Vec*>(gin_lane), g);
+            gin_lane += FPW * row_bytes;
         }
+        __syncwarp();                                          // this stage may be filled again
+        now = now + 1 == D ? 0 : now + 1;
+        next = next + 1 == D ? 0 : next + 1;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int fl = (warp + 8 * i) * FPW + fs;
-            float4 gt = zero4();
-#pragma unroll
-            for (int j = 0; j < 3; ++j) fma4s(gt, srn[buf * NE + fl * 3 + j], gr[i][j]);
-            if (on && fl < nf_tile) __stcs(gin + (f0 + fl) * CV + cg, mul4(gt, w[i]));
-            if (fl < nf_tile) st[fl * LPF + l] = mul4(x[i], gt);
-        }
-        __syncthreads();
-        // the next tile's corners go to the other index buffer (its readers are behind the barrier above)
-#pragma unroll
-        for (int i = 0; i < NI; ++i) {
-            park(buf ^ 1, i, vo1[i], rn_next[i]);
-            vo1[i] = vo_next[i]; vi2[i] = vi_next[i];
-        }
-        // ---- phase 2, faces in order
-        if (slice < slices) {
-            const int first = slice * FPW + fs, step = slices * FPW;
-            const float* cp = scoef + first * CP + 4 * g2;
-            const float4* tp = st + first * LPF + l;
-#pragma unroll 4
-            for (int fl = first; fl < nf_tile; fl += step, cp += step * CP, tp += step * LPF) {
-                const float4 c = *reinterpret_cast<const float4*>(cp), t = *tp;
-                fma4s(acc[0], c.x, t); fma4s(acc[1], c.y, t); fma4s(acc[2], c.z, t); fma4s(acc[3], c.w, t);
-            }
-        }
+        for (int i = 0; i < NI; ++i) { vo0[i] = vo1[i]; n0[i] = n_next[i]; vo1[i] = vo_next[i]; vi2[i] = vi_next[i]; }
     }
     cp_async_wait<0>();
-    __syncthreads();                                           // the sums of the slices, in slice order, and of the side-by-side faces
-    float4* sums = st;                                         // [slices * KG][4][32]: st has as many
-    if (slice < slices)
+    __syncthreads();                                           // the sums of the faces side by side, then of the warps, in order
+    Vec* sums = reinterpret_cast<Vec*>(f2vl_smem);             // [warp][2 P][32]: a warp's ring is longer
+    static_assert(sizeof(Stage) * D >= sizeof(Vec) * 2 * P * 32, "the sums reuse the ring");
 #pragma unroll
-        for (int j = 0; j < 4; ++j) sums[(warp * 4 + j) * 32 + lane] = acc[j];
+    for (int p = 0; p < P; ++p) {
+        Vec a, b;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const float2 v = unpair2(acc[c][p]);
+            reinterpret_cast<float*>(&a)[c] = v.x;
+            reinterpret_cast<float*>(&b)[c] = v.y;
+        }
+        sums[(warp * 2 * P + 2 * p) * 32 + lane] = a;
+        sums[(warp * 2 * P + 2 * p + 1) * 32 + lane] = b;
+    }
     __syncthreads();
-    for (int i = threadIdx.x; i < K * LPF; i += blockDim.x) {
-        const int k = i / LPF, c = i % LPF;
-        float4 s = zero4();
-        for (int v = 0; v < slices; ++v)
+    const float* flat = reinterpret_cast<const float*>(sums);
+    for (int i = threadIdx.x; i < K * LPF * NC; i += blockDim.x) {
+        const int k = i / (LPF * NC), c = i % (LPF * NC), co = blockIdx.y * LPF * NC + c;
+        float t = 0.f;
+        for (int v = 0; v < F2VL_WARPS; ++v)
 #pragma unroll
-            for (int q = 0; q < FPW; ++q) add4(s, sums[((v * KG + k / 4) * 4 + k % 4) * 32 + q * LPF + c]);
-        if (blockIdx.y * LPF + c < CV) partial[((int64_t)blockIdx.x * K + k) * CV + blockIdx.y * LPF + c] = s;
+            for (int q = 0; q < FPW; ++q) t += flat[((v * 2 * P + k) * 32 + q * LPF) * NC + c];
+        if (co < C) partial[((int64_t)blockIdx.x * K + k) * C + co] = t;
     }
 }
 
@@ -642,25 +753,33 @@ int pb200_facet2vertex_backward(int64_t Nf, int64_t NvIn, int64_t NvOut, int C, 
     bool vec = p.vec && aligned16(gradOutput) && aligned16(input) && aligned16(filter) && aligned16(gradInput);
     if (vec) {
         int CV = C / 4;
-        // K <= 32: lanes of a face as many as hold its channels.  Behind 128 channels chunks of 128 on blockIdx.y
         if (K <= 32) {
-            auto run = [&](auto lpf) {
-                constexpr int LPF = decltype(lpf)::value;
-                const int chunks = (int)ceil_div(CV, LPF);
-                int64_t gx = ceil_div(2 * (int64_t)sm_count(), chunks);              // two blocks per SM
-                if (gx > ceil_div(Nf, F2VB_FACES<LPF>)) gx = ceil_div(Nf, F2VB_FACES<LPF>);
+            auto run = [&](auto pairs, auto lpf) {
+                constexpr int P = decltype(pairs)::value, LPF = decltype(lpf)::value;
+                const int chunks = (int)ceil_div(C, F2VL_NC<P> * LPF);
+                const size_t smemb = sizeof(F2VLStage<P, LPF>) * F2VL_STAGES * F2VL_WARPS;
+                const int fit = (int)(228 * 1024 / (smemb + 1024));                // blocks that an SM's shared memory holds
+                int64_t gx = (int64_t)(fit < F2VL_BLOCKS<P> ? fit : F2VL_BLOCKS<P>) * sm_count() / chunks;
+                if (gx < 1) gx = 1;
+                if (gx > ceil_div(Nf, F2VL_WARPS * F2VL_FACES<LPF>)) gx = ceil_div(Nf, F2VL_WARPS * F2VL_FACES<LPF>);
                 if (gx > p.grid_x) gx = p.grid_x;
-                const size_t smemb = f2vb_smem<LPF>(K);
-                PB_CUDA(cudaFuncSetAttribute(f2v_bwd_blocked_kernel<LPF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemb));
-                PB_LAUNCH("f2v_bwd", f2v_bwd_blocked_kernel<LPF>, dim3((unsigned)gx, chunks), 256, smemb, stream, Nf, CV, K, face, vtMap,
-                          nfCount, coeff, (const float4*)input, (const float4*)filter, (const float4*)gradOutput, (float4*)gradInput,
-                          (float4*)partial);
+                PB_CUDA(cudaFuncSetAttribute(f2v_bwd_lane_kernel<P, LPF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemb));
+                PB_LAUNCH("f2v_bwd", (f2v_bwd_lane_kernel<P, LPF>), dim3((unsigned)gx, chunks), 32 * F2VL_WARPS, smemb, stream, Nf, C, K,
+                          face, vtMap, nfCount, coeff, input, filter, gradOutput, gradInput, partial);
                 return reduce_partials(partial, (int)gx, (int64_t)K * Cr, gradFilter, stream);
             };
-            if (CV <= 4) return run(std::integral_constant<int, 4>{});
-            if (CV <= 8) return run(std::integral_constant<int, 8>{});
-            if (CV <= 16) return run(std::integral_constant<int, 16>{});
-            return run(std::integral_constant<int, 32>{});
+            auto width = [&](auto pairs) {
+                constexpr int NC = F2VL_NC<decltype(pairs)::value>;
+                if (C <= 4 * NC) return run(pairs, std::integral_constant<int, 4>{});
+                if (C <= 8 * NC) return run(pairs, std::integral_constant<int, 8>{});
+                if (C <= 16 * NC) return run(pairs, std::integral_constant<int, 16>{});
+                return run(pairs, std::integral_constant<int, 32>{});
+            };
+            if (K <= 4) return width(std::integral_constant<int, 2>{});
+            if (K <= 10) return width(std::integral_constant<int, 5>{});
+            if (K <= 16) return width(std::integral_constant<int, 8>{});
+            if (K <= 26) return width(std::integral_constant<int, 13>{});
+            return width(std::integral_constant<int, 16>{});
         }
         dim3 grid(p.grid_x, (unsigned)ceil_div(CV, 32));
         const int KP = (K + 3) / 4 * 4 + 4;
