@@ -63,6 +63,43 @@ __device__ __forceinline__ void add4(float4& acc, const float4& a) {
 }
 __device__ __forceinline__ float4 zero4() { return make_float4(0.f, 0.f, 0.f, 0.f); }
 
+// ---- packed pairs: two fp32 operations in one instruction, each rounded as its own ------
+__device__ __forceinline__ uint64_t pair2(float lo, float hi) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float2 unpair2(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ void add2(uint64_t& acc, uint64_t a) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(a)); }
+struct F4x2 { uint64_t a, b; };          // a float4 as two pairs
+__device__ __forceinline__ F4x2 ldg4x2(const float4* p) {
+    const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2*>(p));
+    return F4x2{v.x, v.y};
+}
+__device__ __forceinline__ F4x2 pair4(const float4& v) { return F4x2{pair2(v.x, v.y), pair2(v.z, v.w)}; }
+__device__ __forceinline__ float4 unpair4(const F4x2& v) {
+    const float2 a = unpair2(v.a), b = unpair2(v.b);
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void add2(F4x2& acc, const F4x2& v) { add2(acc.a, v.a); add2(acc.b, v.b); }
+__device__ __forceinline__ void add2_if(bool on, F4x2& acc, const F4x2& v) {
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %4, 0;\n\t@p add.rn.f32x2 %0, %0, %2;\n\t@p add.rn.f32x2 %1, %1, %3;\n\t}"
+        : "+l"(acc.a), "+l"(acc.b) : "l"(v.a), "l"(v.b), "r"((int)on));
+}
+__device__ __forceinline__ void fma2(F4x2& acc, const F4x2& x, const F4x2& y) { fma2(acc.a, x.a, y.a); fma2(acc.b, x.b, y.b); }
+
 // The vectorised kernels give each item (a face or a vertex) to a team of TL threads
 // (TL a power of two <= 32); a thread owns one float4 channel group of the item, and
 // gridDim.y walks channel chunks of 32 groups (128 channels).

@@ -1,17 +1,25 @@
 // vertex2facet: forward (pure gather) and backward (vertex-centred pull over the CSR that
 // yields the input gradient and the filter gradient in one pass, no float atomics).
 #include "common.cuh"
+#include "row_walk.cuh"
 
 #include <mutex>
 
 namespace pb {
 
+// Rows in flight and blocks per SM of the backward kernel: six rows, three sums, filter and filter gradient fill the 85 registers of
+// three blocks; most vertices have six faces (batch of 32 height fields, 128 channels: 2.49 ms; eight rows 3.02, four rows and four
+// blocks 3.19).
+constexpr int V2F_BWD_BATCH = 6, V2F_BWD_BLOCKS = 3;
+
 // ------------------------------------------------------------------- forward, vectorised
-// r == 1, C % 4 == 0.  A team of TL threads owns one face; a thread owns one float4 of
-// channels.  HBM traffic per face: 12 B of indices, 16*CV B written; the three vertex rows
-// are gathers that mostly hit L2 (every vertex row is shared by ~6 faces).
+// r == 1, C % 4 == 0.  A team of TL threads owns two faces behind one another at a time; a thread owns one float4 of
+// channels.  HBM traffic per face: 12 B of indices, 16*CV B written; the three vertex rows are gathers that mostly hit L2
+// (every vertex row is shared by ~6 faces; two faces in a row mostly share an edge).  What bounds it is the latency of index
+// and row loads: the next pair's indices are asked for before this pair's six rows are used (one face at a time, eight blocks
+// per SM: 172 us for 1.76 M faces of 64 channels, now 122, copy floor 110; 7.4 M faces of 128 channels 1.51 ms, now 1.05).
 template <int TL>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 v2f_fwd_vec_kernel(int64_t Nf, int CV, const int32_t* __restrict__ face, const float4* __restrict__ in,
                    const float4* __restrict__ filt, float4* __restrict__ out) {
     const int lane = threadIdx.x % TL;
@@ -20,16 +28,27 @@ v2f_fwd_vec_kernel(int64_t Nf, int CV, const int32_t* __restrict__ face, const f
     if (cg >= CV) return;
     const float4 f0 = filt[cg], f1 = filt[CV + cg], f2 = filt[2 * CV + cg];
     const int teams = blockDim.x / TL;
-    for (int64_t f = (int64_t)blockIdx.x * teams + team; f < Nf; f += (int64_t)gridDim.x * teams) {
-        int v0 = __ldg(face + 3 * f), v1 = __ldg(face + 3 * f + 1), v2 = __ldg(face + 3 * f + 2);
-        float4 x0 = ldg4(in + (int64_t)v0 * CV + cg);
-        float4 x1 = ldg4(in + (int64_t)v1 * CV + cg);
-        float4 x2 = ldg4(in + (int64_t)v2 * CV + cg);
-        float4 o = zero4();
-        fma4(o, f0, x0);      // same k-ascending fused-multiply-add chain as the reference
-        fma4(o, f1, x1);
-        fma4(o, f2, x2);
-        __stcs(out + f * CV + cg, o);
+    const int64_t step = 2 * (int64_t)gridDim.x * teams;
+    int64_t f = 2 * ((int64_t)blockIdx.x * teams + team);
+    int n[6];
+    auto indices = [&](int64_t at) {                           // past the end: vertex 0, read and not used
+#pragma unroll
+        for (int j = 0; j < 6; ++j) n[j] = 3 * at + j < 3 * Nf ? __ldg(face + 3 * at + j) : 0;
+    };
+    if (f < Nf) indices(f);
+    for (; f < Nf; f += step) {
+        float4 x[6];
+#pragma unroll
+        for (int j = 0; j < 6; ++j) x[j] = ldg4(in + (int64_t)n[j] * CV + cg);
+        indices(f + step);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            float4 o = zero4();
+            fma4(o, f0, x[3 * u]);      // same k-ascending fused-multiply-add chain as the reference
+            fma4(o, f1, x[3 * u + 1]);
+            fma4(o, f2, x[3 * u + 2]);
+            if (f + u < Nf) __stcs(out + (f + u) * CV + cg, o);
+        }
     }
 }
 
@@ -53,14 +72,18 @@ __global__ void v2f_fwd_generic_kernel(int64_t Nf, int C, int r, const int32_t* 
 }
 
 // ------------------------------------------------------------------ backward, vectorised
-// A team owns one vertex v: it loads input[v] once, walks the CSR row of v in ascending
-// (face, corner) order, and for every incident corner (f,k) reads gradOutput[f]:
-//     gradInput[v] += g * filter[k]            (fixed order -> deterministic)
-//     gradFilter[k] += g * input[v]            (per-thread registers)
+// A team owns one vertex v: it walks the CSR row of v in ascending (face, corner) order and sums the gradOutput rows of its
+// corners by the corner's number k in the face, s[k] = sum over (f, k) of gradOutput[f]; then
+//     gradInput[v]   = sum_k s[k] * filter[k]        (fixed order -> deterministic)
+//     gradFilter[k] += s[k] * input[v]               (per-thread registers)
 // The per-thread filter-gradient partials are summed over the teams of the block in team
 // order and written to partial[blockIdx.x][3][C]; a second kernel adds the blocks in order.
+// What bounds it: instructions per corner and the threefold row gather from L2.  Sums by corner number cost a corner two packed
+// additions; multiplying every row by its filter row and by input[v] cost it twelve instructions, and bounds, entries and rows
+// one behind another three latencies per vertex: 980 000 vertices, 64 channels 341 us (now 248, copy floor 146); 4.15 M
+// vertices, 128 channels 3.13 ms (2.49, floor 1.24).
 template <int TL>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(256, V2F_BWD_BLOCKS)
 v2f_bwd_vec_kernel(int64_t Nv, int CV, const int32_t* __restrict__ rowptr, const int32_t* __restrict__ entries,
                    const float4* __restrict__ gout, const float4* __restrict__ in, const float4* __restrict__ filt,
                    float4* __restrict__ gin, float4* __restrict__ partial) {
@@ -68,51 +91,33 @@ v2f_bwd_vec_kernel(int64_t Nv, int CV, const int32_t* __restrict__ rowptr, const
     const int lane = threadIdx.x % TL;
     const int team = threadIdx.x / TL;
     const int teams = blockDim.x / TL;
+    constexpr int B = V2F_BWD_BATCH;
     const int cg = blockIdx.y * 32 + lane;
     const bool active = cg < CV;
-    float4 gf0 = zero4(), gf1 = zero4(), gf2 = zero4();
-    if (active) {
-        const float4 f0 = filt[cg], f1 = filt[CV + cg], f2 = filt[2 * CV + cg];
-        for (int64_t v = (int64_t)blockIdx.x * teams + team; v < Nv; v += (int64_t)gridDim.x * teams) {
-            int beg = __ldg(rowptr + v), end = __ldg(rowptr + v + 1);
-            float4 acc = zero4();
-            if (end > beg) {
-                float4 x = ldg4(in + v * CV + cg);
-                auto accumulate = [&](int ent, const float4& g) {
-                    const int k = ent & 3;
-                    const float4 fk = (k == 0) ? f0 : ((k == 1) ? f1 : f2);
-                    fma4(acc, g, fk);
-                    const float4 t = mul4(g, x);
-                    if (k == 0) add4(gf0, t); else if (k == 1) add4(gf1, t); else add4(gf2, t);
-                };
-                // four gradOutput rows in flight at a time, added in entry order
-                int e = beg;
-                for (; e + 3 < end; e += 4) {
-                    int ent[4];
-                    float4 g[4];
+    F4x2 gf0{0, 0}, gf1{0, 0}, gf2{0, 0}, f0{0, 0}, f1{0, 0}, f2{0, 0};
+    if (active) { f0 = pair4(filt[cg]); f1 = pair4(filt[CV + cg]); f2 = pair4(filt[2 * CV + cg]); }
+    RowWalk<TL, B> walk(rowptr, entries, (int64_t)blockIdx.x * teams + team, (int64_t)gridDim.x * teams, Nv);
+    for (; walk.v < Nv; walk.step()) {
+        const F4x2 x = active ? ldg4x2(in + walk.v * CV + cg) : F4x2{0, 0};
+        F4x2 s0{0, 0}, s1{0, 0}, s2{0, 0};
+        walk.rows([&](const int (&ent)[B]) {
+            F4x2 g[B];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) ent[u] = __ldg(entries + e + u);
+            for (int u = 0; u < B; ++u) g[u] = active && ent[u] >= 0 ? ldg4x2(gout + (int64_t)(ent[u] >> 2) * CV + cg) : F4x2{0, 0};
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) g[u] = ldg4(gout + (int64_t)(ent[u] >> 2) * CV + cg);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) accumulate(ent[u], g[u]);
-                }
-                for (; e + 1 < end; e += 2) {
-                    const int ent0 = __ldg(entries + e), ent1 = __ldg(entries + e + 1);
-                    const float4 g0 = ldg4(gout + (int64_t)(ent0 >> 2) * CV + cg);
-                    const float4 g1 = ldg4(gout + (int64_t)(ent1 >> 2) * CV + cg);
-                    accumulate(ent0, g0);
-                    accumulate(ent1, g1);
-                }
-                if (e < end) {
-                    const int ent = __ldg(entries + e);
-                    accumulate(ent, ldg4(gout + (int64_t)(ent >> 2) * CV + cg));
-                }
+            for (int u = 0; u < B; ++u) {              // a missing entry (-1) is no corner 0, 1, 2
+                const int k = ent[u] & 3;
+                add2_if(k == 0, s0, g[u]);
+                add2_if(k == 1, s1, g[u]);
+                add2_if(k == 2, s2, g[u]);
             }
-            gin[v * CV + cg] = acc;
-        }
+        });
+        F4x2 acc{0, 0};
+        fma2(acc, s0, f0); fma2(acc, s1, f1); fma2(acc, s2, f2);
+        fma2(gf0, s0, x); fma2(gf1, s1, x); fma2(gf2, s2, x);
+        if (active) gin[walk.v * CV + cg] = unpair4(acc);
     }
-    red[0][threadIdx.x] = gf0; red[1][threadIdx.x] = gf1; red[2][threadIdx.x] = gf2;
+    red[0][threadIdx.x] = unpair4(gf0); red[1][threadIdx.x] = unpair4(gf1); red[2][threadIdx.x] = unpair4(gf2);
     __syncthreads();
     if (team == 0 && active) {
         float4 s0 = zero4(), s1 = zero4(), s2 = zero4();
@@ -205,7 +210,7 @@ int pb200_vertex2facet_forward(int64_t Nf, int64_t Nv, int C, int r, const float
     if (vec_ok(C, r) && aligned16(input) && aligned16(filter) && aligned16(output)) {
         int CV = C / 4;
         TeamGeom g = team_geom(CV);
-        dim3 grid(persistent_blocks(Nf, g.teams, 8), g.chunks);
+        dim3 grid(persistent_blocks(ceil_div(Nf, 2), g.teams, 4), g.chunks);
         PB_DISPATCH_TL(g.TL, PB_LAUNCH("v2f_fwd", v2f_fwd_vec_kernel<TL>, grid, 256, 0, stream, Nf, CV, face,
                                        (const float4*)input, (const float4*)filter, (float4*)output));
     } else {
@@ -244,11 +249,14 @@ int pb200_vertex2facet_backward(int64_t Nf, int64_t Nv, int C, int r, const floa
     if (vec) {
         int CV = C / 4;
         TeamGeom g = team_geom(CV);
-        dim3 grid(p.grid_x, g.chunks);
+        int gx = V2F_BWD_BLOCKS * sm_count() / g.chunks;       // the blocks that run side by side
+        if (gx < 1) gx = 1;
+        if (gx > p.grid_x) gx = p.grid_x;
+        dim3 grid(gx, g.chunks);
         PB_DISPATCH_TL(g.TL, PB_LAUNCH("v2f_bwd", v2f_bwd_vec_kernel<TL>, grid, 256, 0, stream, Nv, CV, rowptr,
                                        entries, (const float4*)gradOutput, (const float4*)input,
                                        (const float4*)filter, (float4*)gradInput, (float4*)partial));
-        return reduce_partials(partial, p.grid_x, 3 * Cr, gradFilter, stream);
+        return reduce_partials(partial, gx, 3 * Cr, gradFilter, stream);
     }
     // generic path (any C, r): plan for the non-vector layout even if only alignment failed
     V2FBwdPlan q = p;

@@ -1,0 +1,52 @@
+"""The kernels that walk the faces of a vertex (vertex2facet backward, facet2vertex forward) and vertex2facet forward against the fp64
+formulas where the work is split: vertices with no face, with as many as a batch holds (5 to 9), with more (17, 33, 70), odd numbers of
+faces, and every number of lanes per row."""
+import pytest
+import torch
+
+from conftest import rel_err
+from picassoplus_b200.mesh.pi_modules import conv3d
+
+pytestmark = pytest.mark.gpu
+
+DEGREES = [0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 12, 13, 16, 17, 33, 70]
+
+
+def _faces(copies, seed):
+    """Faces whose vertex v has exactly DEGREES[v % 16] corners, in random order and corner position (one corner more where needed)."""
+    ids = torch.cat([torch.full((d,), v + 16 * c) for c in range(copies) for v, d in enumerate(DEGREES)])
+    g = torch.Generator().manual_seed(seed)
+    ids = ids[torch.randperm(ids.numel(), generator=g)]
+    ids = ids[:ids.numel() // 3 * 3]
+    return ids.view(-1, 3).int().cuda(), 16 * copies
+
+
+@pytest.mark.parametrize("C", [4, 8, 12, 16, 32, 64, 100, 128, 132])
+@pytest.mark.parametrize("copies,odd", [(1, False), (1, True), (40, False), (300, True)])
+def test_rows(copies, odd, C):
+    face, nv = _faces(copies, C + copies)
+    if (face.shape[0] % 2 == 1) != odd:
+        face = face[:-1].contiguous()
+    nf, g = face.shape[0], torch.Generator(device="cuda").manual_seed(C)
+    x, w = torch.randn(nv, C, device="cuda", generator=g), torch.randn(3, C, 1, device="cuda", generator=g)
+    go = torch.randn(nf, C, device="cuda", generator=g)
+    vid = face.long()
+    picked = x.double()[vid]                                                      # (nf, 3, C)
+    out = conv3d.vertex2facet_forward(x, w, face)
+    assert rel_err(out, (picked * w.double()[None, :, :, 0]).sum(1)) <= 1e-6
+    gin, gw = conv3d.vertex2facet_backward(go, x, w, face)
+    want = torch.zeros(nv, C, dtype=torch.float64, device="cuda")
+    want.index_add_(0, vid.reshape(-1), (go.double()[:, None] * w.double()[None, :, :, 0]).reshape(-1, C))
+    # sums of up to 70 terms of unit size: 70 * 2^-24 of the largest
+    assert rel_err(gin, want) <= 5e-6 and rel_err(gw[:, :, 0], (go.double()[:, None] * picked).sum(0)) <= 5e-6
+    K = 9
+    coeff, filt = torch.randn(nf, K, device="cuda", generator=g), torch.randn(K, C, 1, device="cuda", generator=g)
+    vt = torch.arange(nv, dtype=torch.int32, device="cuda")
+    count = torch.bincount(vid.reshape(-1), minlength=nv).int()
+    rows = conv3d.facet2vertex_forward(go, filt, coeff, face, count, vt)
+    want = torch.zeros(nv, C, dtype=torch.float64, device="cuda")
+    prod = (coeff.double() @ filt.double()[:, :, 0]) * go.double()
+    want.index_add_(0, vid.reshape(-1), prod.repeat_interleave(3, 0))
+    assert rel_err(rows, want / count.clamp(min=1).double()[:, None]) <= 5e-6
+    again = conv3d.vertex2facet_backward(go, x, w, face)
+    assert torch.equal(gin, again[0]) and torch.equal(gw, again[1])
