@@ -20,6 +20,7 @@
 // 25 bases (bf16 1260 -> 857).  What bounds it: the three products per term at 128 channels (0.96 of what the board sustains), the
 // epilogue and the row copies below.  More row loaders leave the epilogue too few registers (four: 735 -> 960 us).  All
 // waits are bounded.
+#include <cuda.h>
 #include "common.cuh"
 #include "tc_ptx.cuh"
 #include "tc_runtime.cuh"
@@ -39,10 +40,15 @@ using namespace ptx;
 constexpr int TILE_M = 128;
 constexpr int NCOLS = 256;                       // accumulator columns
 constexpr int EWARPS = 16;                       // epilogue warps: 2 groups x 4 TMEM quadrants x 2
-constexpr int GWARPS = 2;                        // row loaders
-constexpr int NTHREADS = (EWARPS + 2 + GWARPS) * 32;
+constexpr int GWARPS = 1;                        // row converters
+constexpr int NTHREADS = (EWARPS + 3 + GWARPS) * 32;
+// Registers per thread: at launch, of the epilogue's four warpgroups, of the two that hold filter stream, issue, row stream and converters
+constexpr int REGS_LAUNCH = 96, REGS_EPILOGUE = 104, REGS_OTHER = 64;
+static_assert(NTHREADS % 128 == 0 && EWARPS * 32 * REGS_EPILOGUE + (NTHREADS - EWARPS * 32) * REGS_OTHER == NTHREADS * REGS_LAUNCH,
+              "the shares are what the block is launched with");
 constexpr int KTILE_BYTES = TILE_M * 64;         // 32 channels of the tile's rows
 constexpr int MAX_CK = 256;                      // contracted channels per launch
+constexpr int MAX_GBUFS = 3;                     // tile buffers
 
 struct Params {
     int64_t Nf;
@@ -80,13 +86,13 @@ __device__ __forceinline__ float weighted(const float* v, const float (&b)[(F + 
 }
 
 template <int NSPLIT, int F>
-__global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p) {
+__global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p, const __grid_constant__ CUtensorMap rows_map) {
     constexpr int nq = NQ<F>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int S = p.nstages, KST = p.kst;
-    const uint32_t gtile_bytes = (uint32_t)NSPLIT * KST * KTILE_BYTES;
+    const uint32_t gtile_bytes = 2u * KST * KTILE_BYTES;
     const uint32_t w_bytes = (uint32_t)p.nmma * 64, wblk_bytes = NSPLIT * w_bytes, wstage_bytes = wblk_bytes * p.kb;
     uint8_t* gtile = smem;
     uint8_t* wst = smem + (size_t)p.gbufs * gtile_bytes;
@@ -95,15 +101,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
     uint64_t* w_empty = bars + S;             // [S]
     uint64_t* acc_full = bars + 2 * S;        // [2]
     uint64_t* acc_empty = bars + 2 * S + 2;   // [2]
-    uint64_t* g_full = bars + 2 * S + 4;      // [2] row tile buffer written
-    uint64_t* g_empty = bars + 2 * S + 6;     // [2] all products of the item done with the buffer
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S + 8);
+    uint64_t* raw_full = bars + 2 * S + 4;    // [MAX_GBUFS] rows in the tile buffer as they are in memory
+    uint64_t* g_full = raw_full + MAX_GBUFS;  // [MAX_GBUFS] converted
+    uint64_t* g_empty = g_full + MAX_GBUFS;   // [MAX_GBUFS] all products of the item done with the buffer
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(g_empty + MAX_GBUFS);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     if (tid == 0) {
         for (int s = 0; s < S; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], 1); }
         for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], EWARPS / 2); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&g_full[b], GWARPS); mbar_init(&g_empty[b], 1); }
+        for (int b = 0; b < MAX_GBUFS; ++b) { mbar_init(&raw_full[b], 1); mbar_init(&g_full[b], GWARPS); mbar_init(&g_empty[b], 1); }
         abort_flag[0] = 0;
         abort_flag[1] = p.wait_budget;
         fence_barrier_init();
@@ -114,6 +121,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     const int64_t nitems = (p.Nf + TILE_M - 1) / TILE_M * p.groups;
+    if (warp < EWARPS) registers_take<REGS_EPILOGUE>();
+    else registers_keep<REGS_OTHER>();
 
     if (warp < EWARPS) {
         // ===================== epilogue (thread = face) =====================
@@ -188,62 +197,67 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
                 }
             }
         }
-    } else if (warp >= EWARPS + 2) {
-        // ===================== row loaders =====================
-        // a task is one 16-byte operand chunk (8 channels) of one row; consecutive lanes take consecutive chunks
-        const int gt = tid - (EWARPS + 2) * 32;
-        const int cpr = KST * 4, ntasks = TILE_M * cpr;
-        constexpr int U = 6;                                      // tasks in flight per thread
+    } else if (warp >= EWARPS + 3) {
+        // ===================== row converters =====================
+        // a task is 32 channels of 32 rows: a lane turns its row's 32 floats, which lie in the two 64-byte slots of that row
+        // (channels 0..15 and 16..31), into bf16 hi and lo in the same two slots
+        const int gw = warp - (EWARPS + 3);
         uint32_t icount = 0;
         for (int64_t item = blockIdx.x; item < nitems; item += gridDim.x, ++icount) {
-            const int64_t f0 = item / p.groups * TILE_M;
-            const uint32_t gb = p.gbufs == 2 ? (icount & 1u) : 0u;
-            const uint32_t gph = p.gbufs == 2 ? ((icount >> 1) & 1u) : (icount & 1u);
-            uint8_t* const gdst = gtile + (size_t)gb * gtile_bytes;
-            if (warp == EWARPS + 2 && lane < 2) {                 // the next item's rows and weights, on their way to L2
-                const int64_t n0 = (item + gridDim.x) / p.groups * TILE_M;
-                if (n0 < p.Nf && n0 != f0) {
-                    const int64_t n = p.Nf - n0 < TILE_M ? p.Nf - n0 : TILE_M;
-                    if (lane == 0 && p.stride == p.Ck) prefetch_l2(p.rows + n0 * p.stride, (uint32_t)(n * p.stride * 4));
-                    if (lane == 1) prefetch_l2(p.w + n0 * p.Fp, (uint32_t)(n * p.Fp * 4));
-                }
-            }
-            int ok = 1;
-            if (lane == 0) ok = mbar_wait(&g_empty[gb], gph ^ 1u, abort_flag) ? 1 : 0;
-            if (!__shfl_sync(0xffffffffu, ok, 0)) break;
-            for (int base = 0; base < ntasks; base += U * GWARPS * 32) {
-                float4 u[U], w[U];
+            const uint32_t gb = icount % p.gbufs, gph = icount / p.gbufs & 1u;
+            const uint32_t tile = smem_u32(gtile) + gb * gtile_bytes;
+            if (!warp_wait(&raw_full[gb], gph, abort_flag, lane)) break;
+            for (int task = gw; task < 4 * KST; task += GWARPS) {
+                const uint32_t rr = (uint32_t)(task & 3) * 32 + lane, sw = rr >> 1 & 3u;
+                const uint32_t first = tile + (uint32_t)(task >> 2) * KTILE_BYTES + rr * 64, second = first + (uint32_t)KST * KTILE_BYTES;
+                float4 v[8];
 #pragma unroll
-                for (int j = 0; j < U; ++j) {
-                    const int idx = base + j * GWARPS * 32 + gt;
-                    const int rr = idx / cpr, c = idx - rr * cpr;
-                    const int64_t fr = f0 + rr;
-                    const float4* src = reinterpret_cast<const float4*>(p.rows + fr * p.stride);
-                    u[j] = zero4(); w[j] = zero4();
-                    if (idx < ntasks && fr < p.Nf && c * 8 < p.Ck) u[j] = ldg4(src + 2 * c);
-                    if (idx < ntasks && fr < p.Nf && c * 8 + 4 < p.Ck) w[j] = ldg4(src + 2 * c + 1);
-                }
+                for (uint32_t c = 0; c < 4; ++c) { v[c] = lds_f4(first + ((c ^ sw) << 4)); v[4 + c] = lds_f4(second + ((c ^ sw) << 4)); }
 #pragma unroll
-                for (int j = 0; j < U; ++j) {
-                    const int idx = base + j * GWARPS * 32 + gt;
-                    if (idx >= ntasks) continue;
-                    const int rr = idx / cpr, c = idx - rr * cpr;
-                    uint8_t* dst = gdst + (size_t)(c >> 2) * KTILE_BYTES + swz64_offset((uint32_t)rr, (uint32_t)(c & 3));
+                for (uint32_t c = 0; c < 4; ++c) {
+                    const float4 a = v[2 * c], b = v[2 * c + 1];
                     uint32_t hi[4], lo[4];
                     if (NSPLIT == 1) {
-                        hi[0] = pack_bf16x2(u[j].x, u[j].y); hi[1] = pack_bf16x2(u[j].z, u[j].w);
-                        hi[2] = pack_bf16x2(w[j].x, w[j].y); hi[3] = pack_bf16x2(w[j].z, w[j].w);
+                        hi[0] = pack_bf16x2(a.x, a.y); hi[1] = pack_bf16x2(a.z, a.w);
+                        hi[2] = pack_bf16x2(b.x, b.y); hi[3] = pack_bf16x2(b.z, b.w);
                     } else {
-                        split_bf16x2(u[j].x, u[j].y, hi[0], lo[0]); split_bf16x2(u[j].z, u[j].w, hi[1], lo[1]);
-                        split_bf16x2(w[j].x, w[j].y, hi[2], lo[2]); split_bf16x2(w[j].z, w[j].w, hi[3], lo[3]);
-                        *reinterpret_cast<uint4*>(dst + (size_t)KST * KTILE_BYTES) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                        split_bf16x2(a.x, a.y, hi[0], lo[0]); split_bf16x2(a.z, a.w, hi[1], lo[1]);
+                        split_bf16x2(b.x, b.y, hi[2], lo[2]); split_bf16x2(b.z, b.w, hi[3], lo[3]);
+                        sts_u4(second + ((c ^ sw) << 4), lo[0], lo[1], lo[2], lo[3]);
                     }
-                    *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                    sts_u4(first + ((c ^ sw) << 4), hi[0], hi[1], hi[2], hi[3]);
                 }
             }
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) mbar_arrive(&g_full[gb]);
+        }
+    } else if (warp == EWARPS + 2) {
+        // ===================== row stream (TMA engine) =====================
+        if (elect_one()) {
+            uint32_t icount = 0;
+            bool alive = true;
+            for (int64_t item = blockIdx.x; item < nitems; item += gridDim.x, ++icount) {
+                const int64_t f0 = item / p.groups * TILE_M;
+                const uint32_t gb = icount % p.gbufs, gph = icount / p.gbufs & 1u;
+                const int64_t n0 = (item + gridDim.x) / p.groups * TILE_M;
+                if (n0 < p.Nf && n0 != f0) {                      // the next item's rows and weights, on their way to L2
+                    const int64_t n = p.Nf - n0 < TILE_M ? p.Nf - n0 : TILE_M;
+                    if (p.stride == p.Ck) prefetch_l2(p.rows + n0 * p.stride, (uint32_t)(n * p.stride * 4));
+                    prefetch_l2(p.w + n0 * p.Fp, (uint32_t)(n * p.Fp * 4));
+                }
+                if (!mbar_wait(&g_empty[gb], gph ^ 1u, abort_flag)) { alive = false; break; }
+                mbar_arrive_expect_tx(&raw_full[gb], gtile_bytes);
+                uint8_t* const dst = gtile + (size_t)gb * gtile_bytes;
+                for (int ks = 0; ks < KST; ++ks) {
+                    tile_g2s(dst + (size_t)ks * KTILE_BYTES, &rows_map, ks * 32, (int)f0, &raw_full[gb]);
+                    tile_g2s(dst + (size_t)(KST + ks) * KTILE_BYTES, &rows_map, ks * 32 + 16, (int)f0, &raw_full[gb]);
+                }
+            }
+            if (!alive) {                                         // let copies in flight land before shared memory is released
+                const long long t0 = clock64();
+                while (clock64() - t0 < 2000000) { }
+            }
         }
     } else if (warp == EWARPS) {
         // ===================== filter stream (TMA engine) =====================
@@ -278,8 +292,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
             for (int64_t item = blockIdx.x; item < nitems && alive; item += gridDim.x, ++icount) {
                 const int s0 = (int)(item % p.groups) * p.per_group;
                 const int s1 = s0 + p.per_group < p.nslices ? s0 + p.per_group : p.nslices;
-                const uint32_t gb = p.gbufs == 2 ? (icount & 1u) : 0u;
-                const uint32_t gph = p.gbufs == 2 ? ((icount >> 1) & 1u) : (icount & 1u);
+                const uint32_t gb = icount % p.gbufs, gph = icount / p.gbufs & 1u;
                 const uint64_t dg_tile = dg_base + (uint64_t)((gb * gtile_bytes) >> 4);
                 if (!mbar_wait(&g_full[gb], gph, abort_flag)) break;
                 for (int slice = s0; slice < s1 && alive; ++slice, ++sc) {
@@ -345,9 +358,10 @@ static Plan plan(int Cn, int CkAll, int F, int precision) {
     pl.nslices = (Cn + pl.nq - 1) / pl.nq;
     pl.kst = (Ck + 31) / 32;
     const size_t budget = 226 * 1024;
-    const size_t gt = (size_t)pl.nsplit * pl.kst * KTILE_BYTES, ws = (size_t)pl.nsplit * pl.nmma * 64;
-    // a second tile buffer takes the row copy off the critical path, when at least three filter stages still fit beside it
+    const size_t gt = (size_t)2 * pl.kst * KTILE_BYTES, ws = (size_t)pl.nsplit * pl.nmma * 64;
+    // a second tile buffer takes the row copy off the critical path, when at least three filter blocks still fit beside it
     pl.gbufs = (2 * gt + 1024 + 384 + 3 * ws <= budget) ? 2 : 1;
+    if (3 * gt + 1024 + 384 + 2 * pl.kst * ws <= budget) pl.gbufs = 3;
     const size_t fixed = pl.gbufs * gt + 1024 + 384;
     pl.nblocks = (int)((budget - fixed) / ws);
     if (pl.nblocks > 16) pl.nblocks = 16;
@@ -366,10 +380,39 @@ bool supported(int Cn, int Ck, int F, int precision) {
 
 size_t workspace_bytes(int Cn, int Ck, int F, int precision) { return align_up(plan(Cn, Ck, F, precision).wimg_bytes, 256); }
 
+// Tensor map of (Nf, channels) floats with `stride` floats between rows: boxes of 16 channels x 128 rows, laid down as 64-byte rows with
+// the 64-byte swizzle, the layout of the product's operand
+static int map_rows(CUtensorMap* map, const float* rows, int64_t Nf, int channels, int stride, const char* label) {
+    typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                               const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const Encode encode = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess)
+            fn = nullptr;
+        return (Encode)fn;
+    }();
+    PB_REQUIRE(encode, PB200_ECUDA, "%s: the driver has no cuTensorMapEncodeTiled", label);
+    const cuuint64_t dims[2] = {(cuuint64_t)channels, (cuuint64_t)Nf}, strides[1] = {(cuuint64_t)stride * 4};
+    const cuuint32_t box[2] = {16, TILE_M}, step[2] = {1, 1};
+    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(rows), dims, strides, box, step,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    PB_REQUIRE(r == CUDA_SUCCESS, PB200_ECUDA, "%s: cuTensorMapEncodeTiled failed (%d) for %lld rows of %d floats", label, (int)r,
+               (long long)Nf, channels);
+    return PB200_OK;
+}
+
 template <int NSPLIT, int F>
-static int launch(const char* label, const Params& p, int grid, size_t smem, cudaStream_t stream) {
+static int launch(const char* label, const Params& p, const CUtensorMap& map, int grid, size_t smem, cudaStream_t stream) {
     PB_CUDA(cudaFuncSetAttribute(f2f_one_sample_tc_kernel<NSPLIT, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PB_LAUNCH(label, (f2f_one_sample_tc_kernel<NSPLIT, F>), grid, NTHREADS, smem, stream, p);
+    static const int regs = [] {                                  // a kernel built with fewer would wait for registers that are not there
+        cudaFuncAttributes a;
+        return cudaFuncGetAttributes(&a, f2f_one_sample_tc_kernel<NSPLIT, F>) == cudaSuccess ? a.numRegs : 0;
+    }();
+    PB_REQUIRE(regs == REGS_LAUNCH, PB200_ECUDA, "%s: built with %d registers per thread instead of %d", label, regs, REGS_LAUNCH);
+    PB_LAUNCH(label, (f2f_one_sample_tc_kernel<NSPLIT, F>), grid, NTHREADS, smem, stream, p, map);
     return PB200_OK;
 }
 
@@ -414,12 +457,15 @@ int run(int64_t Nf, int Cn, int Ck, int F, const float* rows, const float* filte
         p.w = w; p.Fp = Fp; p.wimg = (const uint8_t*)ws; p.out = out;
         p.async_err = async_error_word();
         p.wait_budget = wait_budget_kclocks();
+        CUtensorMap map;
+        rc = map_rows(&map, p.rows, Nf, chunk, Ck, label);
+        if (rc) return rc;
         const bool two = pl.nsplit == 2;
         switch (F) {
-            case 4: rc = two ? launch<2, 4>(label, p, grid, pl.smem, stream) : launch<1, 4>(label, p, grid, pl.smem, stream); break;
-            case 9: rc = two ? launch<2, 9>(label, p, grid, pl.smem, stream) : launch<1, 9>(label, p, grid, pl.smem, stream); break;
-            case 16: rc = two ? launch<2, 16>(label, p, grid, pl.smem, stream) : launch<1, 16>(label, p, grid, pl.smem, stream); break;
-            default: rc = two ? launch<2, 25>(label, p, grid, pl.smem, stream) : launch<1, 25>(label, p, grid, pl.smem, stream); break;
+            case 4: rc = two ? launch<2, 4>(label, p, map, grid, pl.smem, stream) : launch<1, 4>(label, p, map, grid, pl.smem, stream); break;
+            case 9: rc = two ? launch<2, 9>(label, p, map, grid, pl.smem, stream) : launch<1, 9>(label, p, map, grid, pl.smem, stream); break;
+            case 16: rc = two ? launch<2, 16>(label, p, map, grid, pl.smem, stream) : launch<1, 16>(label, p, map, grid, pl.smem, stream); break;
+            default: rc = two ? launch<2, 25>(label, p, map, grid, pl.smem, stream) : launch<1, 25>(label, p, map, grid, pl.smem, stream); break;
         }
         if (rc) return rc;
     }

@@ -89,6 +89,13 @@ __device__ __forceinline__ bool elect_one() {
     return r != 0;
 }
 
+// Registers per thread of the calling warpgroup (four warps, all of which call it): a share of what the block was launched
+// with.  `give` waits until others have let go of enough, so the shares of a block must add up to its launch's registers.
+template <int N>
+__device__ __forceinline__ void registers_keep() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void registers_take() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+
 // -------------------------------------------------------------------- bulk (TMA) copies
 // bring a piece of memory towards L2; address 16-byte aligned, size a multiple of 16
 __device__ __forceinline__ void prefetch_l2(const void* src, uint32_t bytes) {
@@ -100,6 +107,15 @@ __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, u
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                      smem_u32(dst_smem)),
                  "l"(src_gmem), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+
+// tiled copy of the box at (x, y) of a two-dimensional tensor map; what lies outside the tensor arrives as zeros and counts as
+// bytes like the rest.  x * element size a multiple of 16 bytes.
+__device__ __forceinline__ void tile_g2s(void* dst_smem, const void* map, int x, int y, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                     smem_u32(dst_smem)),
+                 "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
                  : "memory");
 }
 
@@ -300,6 +316,10 @@ __device__ __forceinline__ void sts_f4(uint32_t a, const float4& v) {
 
 __device__ __forceinline__ void sts_u2(uint32_t a, uint32_t x, uint32_t y) {
     asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(a), "r"(x), "r"(y) : "memory");
+}
+
+__device__ __forceinline__ void sts_u4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
 
 __device__ __forceinline__ float to_tf32_rna(float x) {
