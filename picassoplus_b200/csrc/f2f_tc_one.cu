@@ -8,19 +8,29 @@
 // SAMPLES of a face; with one sample half of them did nothing but read the same columns again, and the other half's chain of
 // TMEM loads and sums per slice was three times as long as the slice's products at 64 channels (two scenes of 880 000 faces,
 // 64 -> 64, 16 bases: 924 us, products alone 300 us).  Here
-//   * 16 epilogue warps (thread = face) in two groups of eight, one group per accumulator, so a group has the time of two
-//     slices to drain one; the two warps of a quadrant in a group take the slice's channel quadruples in turn, load a
-//     quadruple's columns together, hand the accumulator back as soon as the last columns are in registers, and store 16 bytes
-//     per quadruple;
+//   * 16 epilogue warps (thread = face) drain one of two accumulators together: the four warps of a TMEM quadrant take the slice's
+//     channel quadruples in turn, load a quadruple's columns together, hand the accumulator back as soon as their last columns
+//     are in registers, and store 16 bytes per quadruple (eight warps per accumulator: 316 instead of 288 us for 880 000 faces, 64 ->
+//     64, 16 bases, and 5 % more on most other shapes);
 //   * a slice holds as many channels as fill the accumulator (NQ; drained in groups of G), its filter image exactly the rows the
 //     product reads, and a filter stage as many K-blocks as fit twice (a hand-over per K-block cost the bf16 mode a third);
-//   * a work item is a tile of 128 faces and a run of slices: few tiles are spread over the chip by splitting their slices;
+//   * a tile's rows arrive by tiled bulk copies of 16 channels x 128 rows, swizzled as the operand wants it, in the operand buffer
+//     itself: the 32 floats of a row's K-block take the two 64-byte slots that its bf16 hi and lo go to, and one warp converts them in
+//     place.  (Two warps that loaded rows into registers were slower than a tile's products: 64 meshes, 64 -> 128 channels, both
+//     directions 179 -> 124 us; 1.76 M faces, 64 -> 64: 1 620 -> 1 246.)  The registers of the block are dealt out by role;
+//   * with many products per slice CTAs work in pairs (cta_group::2): each keeps its own tile and accumulators and half of every
+//     filter block, the CTA of rank 0 issues, and its peer's filter stream, converter and epilogue report to its barriers;
+//   * a work item is a tile of 128 faces (a pair of them) and a run of slices: few tiles are spread over the chip by splitting
+//     their slices;
 //   * the next item's rows and weights are asked towards L2 while this one's are copied.
-// Loaders, filter stream and MMA issue as in f2f_tc_gin.cu.  Now 735 us for the product above, and 1683 for 930 000 faces, 128 -> 128,
-// 25 bases (bf16 1260 -> 857).  What bounds it: the three products per term at 128 channels (0.96 of what the board sustains), the
-// epilogue and the row copies below.  More row loaders leave the epilogue too few registers (four: 735 -> 960 us).  All
-// waits are bounded.
+// Per call with a cold L2, before (register loaders, no pairs) and now: 464 000 faces, 128 -> 128, 25 bases 832 -> 763 us, 16 bases 544 ->
+// 468, 9 bases 413 -> 314; 880 000 faces, 64 -> 64, 16 bases 380 -> 288; 464 000 faces, 32 -> 32, 16 bases 130 -> 75; bf16, 128 -> 128, 25
+// bases 441 -> 400.  What bounds it: the three products per term at 128 channels (0.91 of the burst rate), below that the round
+// trips between issue and epilogue, some 1 300 clocks per slice.  Measured and left: one commit per slice for both its last
+// filter stage and its accumulator (1 313 -> 1 242 us at 64 channels, 29.6 -> 31.1 ms at 128, 25 bases); 16-byte stores at 25 bases (the
+// second sum does not fit the registers: 755 -> 789 us); probing the barriers without sleeping (nothing).  All waits are bounded.
 #include <cuda.h>
+#include <type_traits>
 #include "common.cuh"
 #include "tc_ptx.cuh"
 #include "tc_runtime.cuh"
@@ -52,6 +62,7 @@ constexpr int MAX_GBUFS = 3;                     // tile buffers
 
 struct Params {
     int64_t Nf;
+    int nitems;                      // pairs of tiles x slice groups
     int Cn, Ck;
     int nslices, kst, nmma;
     int nstages, kb, gbufs;          // filter stages, K-blocks of 32 channels in one stage (divides kst)
@@ -85,7 +96,29 @@ __device__ __forceinline__ float weighted(const float* v, const float (&b)[(F + 
     return s;
 }
 
-template <int NSPLIT, int F>
+// The barriers that the issuing thread waits on lie in the CTA of rank 0 and are arrived at from both
+template <bool PAIR>
+__device__ __forceinline__ void arrive_first(uint64_t* bar) {
+    if constexpr (PAIR) mbar_arrive_at(at_rank(bar, 0));
+    else mbar_arrive(bar);
+}
+template <bool PAIR>
+__device__ __forceinline__ bool wait_first(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    if constexpr (PAIR) return mbar_wait_cluster(bar, parity, abort_flag);
+    else return mbar_wait(bar, parity, abort_flag);
+}
+template <bool PAIR>
+__device__ __forceinline__ void multiply(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    if constexpr (PAIR) mma_f16_pair(d_tmem, a_desc, b_desc, idesc, accumulate);
+    else mma_f16(d_tmem, a_desc, b_desc, idesc, accumulate);
+}
+template <bool PAIR>
+__device__ __forceinline__ void commit(uint64_t* bar) {
+    if constexpr (PAIR) tc_commit_pair(bar);
+    else tc_commit(bar);
+}
+
+template <int NSPLIT, int F, bool PAIR>
 __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p, const __grid_constant__ CUtensorMap rows_map) {
     constexpr int nq = NQ<F>;
     extern __shared__ uint8_t smem_raw[];
@@ -93,49 +126,55 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int S = p.nstages, KST = p.kst;
     const uint32_t gtile_bytes = 2u * KST * KTILE_BYTES;
-    const uint32_t w_bytes = (uint32_t)p.nmma * 64, wblk_bytes = NSPLIT * w_bytes, wstage_bytes = wblk_bytes * p.kb;
+    constexpr int NB = PAIR ? 2 : 1;          // CTAs of a product: each has its own tile and its share of a filter block's rows
+    const uint32_t w_bytes = (uint32_t)p.nmma * 64 / NB, wblk_bytes = NSPLIT * w_bytes, wstage_bytes = wblk_bytes * p.kb;
+    const uint32_t rank = PAIR ? cluster_rank() : 0;
     uint8_t* gtile = smem;
     uint8_t* wst = smem + (size_t)p.gbufs * gtile_bytes;
     uint64_t* bars = reinterpret_cast<uint64_t*>(wst + (size_t)S * wstage_bytes);
     uint64_t* w_full = bars;                  // [S]
     uint64_t* w_empty = bars + S;             // [S]
-    uint64_t* acc_full = bars + 2 * S;        // [2]
-    uint64_t* acc_empty = bars + 2 * S + 2;   // [2]
-    uint64_t* raw_full = bars + 2 * S + 4;    // [MAX_GBUFS] rows in the tile buffer as they are in memory
-    uint64_t* g_full = raw_full + MAX_GBUFS;  // [MAX_GBUFS] converted
+    uint64_t* w_peer = bars + 2 * S;          // [S] rank 0: the peer's half has landed
+    uint64_t* acc_full = bars + 3 * S;        // [2]
+    uint64_t* acc_empty = bars + 3 * S + 2;   // [2] rank 0: both blocks' epilogues
+    uint64_t* raw_full = bars + 3 * S + 4;    // [MAX_GBUFS] rows in the tile buffer as they are in memory
+    uint64_t* g_full = raw_full + MAX_GBUFS;  // [MAX_GBUFS] converted; rank 0: in both blocks
     uint64_t* g_empty = g_full + MAX_GBUFS;   // [MAX_GBUFS] all products of the item done with the buffer
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(g_empty + MAX_GBUFS);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     if (tid == 0) {
-        for (int s = 0; s < S; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], 1); }
-        for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], EWARPS / 2); }
-        for (int b = 0; b < MAX_GBUFS; ++b) { mbar_init(&raw_full[b], 1); mbar_init(&g_full[b], GWARPS); mbar_init(&g_empty[b], 1); }
+        for (int s = 0; s < S; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], 1); mbar_init(&w_peer[s], 1); }
+        for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], NB * EWARPS); }
+        for (int b = 0; b < MAX_GBUFS; ++b) { mbar_init(&raw_full[b], 1); mbar_init(&g_full[b], NB * GWARPS); mbar_init(&g_empty[b], 1); }
         abort_flag[0] = 0;
         abort_flag[1] = p.wait_budget;
         fence_barrier_init();
     }
-    if (warp == EWARPS) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+    if constexpr (PAIR) { __syncthreads(); cluster_sync(); }      // the peer's barriers are there
+    if (warp == EWARPS) {
+        if constexpr (PAIR) tmem_alloc_pair(tmem_slot, 512);
+        else { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    const int64_t nitems = (p.Nf + TILE_M - 1) / TILE_M * p.groups;
+    const int nitems = p.nitems, item0 = blockIdx.x / NB, item_step = gridDim.x / NB;
     if (warp < EWARPS) registers_take<REGS_EPILOGUE>();
     else registers_keep<REGS_OTHER>();
 
     if (warp < EWARPS) {
         // ===================== epilogue (thread = face) =====================
-        const int q = warp & 3, sub = (warp >> 2) & 1;
-        const uint32_t mine = (uint32_t)(warp >> 3);              // accumulator of this group
+        const int q = warp & 3, sub = warp >> 2;
         const int r = q * 32 + lane;
-        const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + mine * NCOLS;
+        const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16);
         const bool vec = p.Cn % G<F> == 0 && (reinterpret_cast<uintptr_t>(p.out) & (4 * G<F> - 1)) == 0;
         uint32_t sc = 0;
         bool alive = true;
-        for (int64_t item = blockIdx.x; item < nitems && alive; item += gridDim.x) {
-            const int64_t f = item / p.groups * TILE_M + r;
-            const int s0 = (int)(item % p.groups) * p.per_group;
+        for (int item = item0; item < nitems && alive; item += item_step) {
+            const int64_t f = (int64_t)(item / p.groups * NB + rank) * TILE_M + r;
+            const int s0 = item % p.groups * p.per_group;
             const int s1 = s0 + p.per_group < p.nslices ? s0 + p.per_group : p.nslices;
             const bool valid = f < p.Nf;
             float b[(F + 3) / 4 * 4];
@@ -169,24 +208,24 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
                 }
             };
             for (int slice = s0; slice < s1; ++slice, ++sc) {
-                if ((sc & 1u) != mine) continue;
+                const uint32_t a = sc & 1u;
                 int ok = 1;
-                if (lane == 0) ok = mbar_wait(&acc_full[mine], (sc >> 1) & 1u, abort_flag) ? 1 : 0;
+                if (lane == 0) ok = mbar_wait(&acc_full[a], (sc >> 1) & 1u, abort_flag) ? 1 : 0;
                 if (!__shfl_sync(0xffffffffu, ok, 0)) { alive = false; break; }
                 tc_fence_after();
                 const int c0 = slice * nq;
                 int left = (p.Cn - c0 + G<F> - 1) / G<F>;         // steps of the slice that exist
                 if (left > nq / G<F>) left = nq / G<F>;
                 auto hand_back = [&](int k) {                     // after the loads of this warp's last quadruple
-                    if (k + 2 < left) return;
+                    if (k + EWARPS / 4 < left) return;
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&acc_empty[mine]);
+                    if (lane == 0) arrive_first<PAIR>(&acc_empty[a]);
                 };
                 if (sub >= left) hand_back(left);                 // nothing of this slice for this warp
-                for (int k = sub; k < left; k += 2) {
+                for (int k = sub; k < left; k += EWARPS / 4) {
                     float s[G<F>], v[G<F> * F];
-                    const uint32_t t = tbase + (uint32_t)(k * G<F> * F);
+                    const uint32_t t = tbase + a * NCOLS + (uint32_t)(k * G<F> * F);
                     if constexpr (F == 16) { tmem_ld32f(t, v); tmem_ld32f(t + 32, v + 32); }
                     else tmem_ld_row<G<F> * F>(t, v);
                     tmem_ld_wait();
@@ -203,7 +242,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
         // (channels 0..15 and 16..31), into bf16 hi and lo in the same two slots
         const int gw = warp - (EWARPS + 3);
         uint32_t icount = 0;
-        for (int64_t item = blockIdx.x; item < nitems; item += gridDim.x, ++icount) {
+        for (int item = item0; item < nitems; item += item_step, ++icount) {
             const uint32_t gb = icount % p.gbufs, gph = icount / p.gbufs & 1u;
             const uint32_t tile = smem_u32(gtile) + gb * gtile_bytes;
             if (!warp_wait(&raw_full[gb], gph, abort_flag, lane)) break;
@@ -230,17 +269,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
             }
             fence_proxy_async();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&g_full[gb]);
+            if (lane == 0) arrive_first<PAIR>(&g_full[gb]);
         }
     } else if (warp == EWARPS + 2) {
         // ===================== row stream (TMA engine) =====================
         if (elect_one()) {
             uint32_t icount = 0;
             bool alive = true;
-            for (int64_t item = blockIdx.x; item < nitems; item += gridDim.x, ++icount) {
-                const int64_t f0 = item / p.groups * TILE_M;
+            for (int item = item0; item < nitems; item += item_step, ++icount) {
+                const int64_t f0 = (int64_t)(item / p.groups * NB + rank) * TILE_M;
                 const uint32_t gb = icount % p.gbufs, gph = icount / p.gbufs & 1u;
-                const int64_t n0 = (item + gridDim.x) / p.groups * TILE_M;
+                const int64_t n0 = (int64_t)((item + item_step) / p.groups * NB + rank) * TILE_M;
                 if (n0 < p.Nf && n0 != f0) {                      // the next item's rows and weights, on their way to L2
                     const int64_t n = p.Nf - n0 < TILE_M ? p.Nf - n0 : TILE_M;
                     if (p.stride == p.Ck) prefetch_l2(p.rows + n0 * p.stride, (uint32_t)(n * p.stride * 4));
@@ -265,13 +304,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
             int s = 0;
             uint32_t ph = 0;
             bool alive = true;
-            for (int64_t item = blockIdx.x; item < nitems && alive; item += gridDim.x) {
-                const int s0 = (int)(item % p.groups) * p.per_group;
+            for (int item = item0; item < nitems && alive; item += item_step) {
+                const int s0 = item % p.groups * p.per_group;
                 const int s1 = s0 + p.per_group < p.nslices ? s0 + p.per_group : p.nslices;
                 for (int blk = s0 * KST; blk < s1 * KST; blk += p.kb) {
                     if (!mbar_wait(&w_empty[s], ph ^ 1u, abort_flag)) { alive = false; break; }
                     mbar_arrive_expect_tx(&w_full[s], wstage_bytes);
-                    bulk_g2s(wst + (size_t)s * wstage_bytes, p.wimg + (size_t)blk * wblk_bytes, wstage_bytes, &w_full[s]);
+                    const uint8_t* src = p.wimg + (size_t)blk * NB * wblk_bytes + (size_t)rank * w_bytes;
+                    if (!PAIR) bulk_g2s(wst + (size_t)s * wstage_bytes, src, wstage_bytes, &w_full[s]);
+                    else for (int i = 0; i < p.kb * NSPLIT; ++i)  // [K-block][hi, lo][rows]: this CTA's half of the rows
+                        bulk_g2s(wst + (size_t)s * wstage_bytes + (size_t)i * w_bytes, src + (size_t)i * NB * w_bytes, w_bytes, &w_full[s]);
                     if (++s == S) { s = 0; ph ^= 1u; }
                 }
             }
@@ -281,27 +323,42 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
             }
         }
     } else {
-        // ===================== MMA issue =====================
-        if (elect_one()) {
-            const uint32_t idesc = instr_desc(FMT_BF16, TILE_M, (uint32_t)p.nmma);
+        // ===================== MMA issue (rank 0), word that the filter has landed (rank 1) =====================
+        if (PAIR && rank != 0) {
+            if (elect_one()) {
+                int s = 0;
+                uint32_t ph = 0;
+                bool alive = true;
+                for (int item = item0; item < nitems && alive; item += item_step) {
+                    const int s0 = item % p.groups * p.per_group;
+                    const int s1 = s0 + p.per_group < p.nslices ? s0 + p.per_group : p.nslices;
+                    for (int blk = s0 * KST; blk < s1 * KST; blk += p.kb) {
+                        if (!mbar_wait(&w_full[s], ph, abort_flag)) { alive = false; break; }
+                        arrive_first<PAIR>(&w_peer[s]);
+                        if (++s == S) { s = 0; ph ^= 1u; }
+                    }
+                }
+            }
+        } else if (elect_one()) {
+            const uint32_t idesc = instr_desc(FMT_BF16, NB * TILE_M, (uint32_t)p.nmma);
             const uint64_t dg_base = smem_desc_kmajor(smem_u32(gtile), 64, SWZ_64B);
             const uint64_t dw_base = smem_desc_kmajor(smem_u32(wst), 64, SWZ_64B);
             int s = 0;
             uint32_t ph = 0, icount = 0, sc = 0;
             bool alive = true;
-            for (int64_t item = blockIdx.x; item < nitems && alive; item += gridDim.x, ++icount) {
-                const int s0 = (int)(item % p.groups) * p.per_group;
+            for (int item = item0; item < nitems && alive; item += item_step, ++icount) {
+                const int s0 = item % p.groups * p.per_group;
                 const int s1 = s0 + p.per_group < p.nslices ? s0 + p.per_group : p.nslices;
                 const uint32_t gb = icount % p.gbufs, gph = icount / p.gbufs & 1u;
                 const uint64_t dg_tile = dg_base + (uint64_t)((gb * gtile_bytes) >> 4);
-                if (!mbar_wait(&g_full[gb], gph, abort_flag)) break;
+                if (!wait_first<PAIR>(&g_full[gb], gph, abort_flag)) break;
                 for (int slice = s0; slice < s1 && alive; ++slice, ++sc) {
                     const uint32_t a = sc & 1u;
-                    if (!mbar_wait(&acc_empty[a], ((sc >> 1) & 1u) ^ 1u, abort_flag)) { alive = false; break; }
+                    if (!wait_first<PAIR>(&acc_empty[a], ((sc >> 1) & 1u) ^ 1u, abort_flag)) { alive = false; break; }
                     tc_fence_after();
                     const uint32_t d_tmem = tmem_base + a * NCOLS;
                     for (int ks0 = 0; ks0 < KST; ks0 += p.kb) {
-                        if (!mbar_wait(&w_full[s], ph, abort_flag)) { alive = false; break; }
+                        if (!mbar_wait(&w_full[s], ph, abort_flag) || (PAIR && !mbar_wait_cluster(&w_peer[s], ph, abort_flag))) { alive = false; break; }
                         tc_fence_after();
                         for (int kk = 0; kk < p.kb; ++kk) {
                             const int ks = ks0 + kk;
@@ -312,30 +369,34 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
                                 const uint64_t adv = (uint64_t)(k2 * 2);
                                 const uint32_t first = (ks | k2) != 0;
                                 if (NSPLIT == 1) {
-                                    mma_f16(d_tmem, dg_hi + adv, dw_hi + adv, idesc, first);
+                                    multiply<PAIR>(d_tmem, dg_hi + adv, dw_hi + adv, idesc, first);
                                 } else {
                                     const uint64_t dg_lo = dg_hi + (uint64_t)(((uint32_t)KST * KTILE_BYTES) >> 4);
                                     const uint64_t dw_lo = dw_hi + (uint64_t)(w_bytes >> 4);
-                                    mma_f16(d_tmem, dg_lo + adv, dw_hi + adv, idesc, first);
-                                    mma_f16(d_tmem, dg_hi + adv, dw_lo + adv, idesc, 1u);
-                                    mma_f16(d_tmem, dg_hi + adv, dw_hi + adv, idesc, 1u);
+                                    multiply<PAIR>(d_tmem, dg_lo + adv, dw_hi + adv, idesc, first);
+                                    multiply<PAIR>(d_tmem, dg_hi + adv, dw_lo + adv, idesc, 1u);
+                                    multiply<PAIR>(d_tmem, dg_hi + adv, dw_hi + adv, idesc, 1u);
                                 }
                             }
                         }
-                        tc_commit(&w_empty[s]);
+                        commit<PAIR>(&w_empty[s]);
                         if (++s == S) { s = 0; ph ^= 1u; }
                     }
-                    if (alive) tc_commit(&acc_full[a]);
+                    if (alive) commit<PAIR>(&acc_full[a]);
                 }
-                if (alive) tc_commit(&g_empty[gb]);
+                if (alive) commit<PAIR>(&g_empty[gb]);
             }
         }
     }
     __syncwarp();
     tc_fence_before();
     __syncthreads();
+    if constexpr (PAIR) cluster_sync();                           // nothing of this CTA is used by its peer any more
     tc_fence_after();
-    if (warp == EWARPS) tmem_dealloc(tmem_base, 512);
+    if (warp == EWARPS) {
+        if constexpr (PAIR) tmem_dealloc_pair(tmem_base, 512);
+        else tmem_dealloc(tmem_base, 512);
+    }
     if (tid == 0 && *abort_flag && p.async_err) {
         *p.async_err = 2;
         __threadfence_system();
@@ -343,7 +404,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
 }
 
 // ---------------------------------------------------------------------------- host side
-struct Plan { int nsplit, nq, nslices, kst, nmma, nblocks, gbufs; size_t smem, wimg_bytes; };
+struct Plan { bool pair; int nsplit, nq, nslices, kst, nmma, nblocks, gbufs; size_t smem, wimg_bytes; };
+
+// K-blocks of 32 contracted channels from which CTAs work in pairs, three products per term.  A pair halves the traffic of the filter
+// blocks, from L2 and from shared memory, and pays with a round trip between two SMs per slice: worth it where a slice is 24
+// products long (464 000 faces, 128 -> 128: 25 bases 851 -> 761 us, 16 bases 529 -> 466, 9 bases 343 -> 312; 3 000 faces 27.6 -> 25.6),
+// not at 18 (96 -> 96, 16 bases: 294 -> 306), 12 (880 000 faces, 64 -> 64: 288 -> 331) or 8 (bf16, 128 -> 128, 25 bases: 400 -> 542).
+constexpr int PAIR_FROM = 4;
 
 static int nq_of(int F) { return F == 4 ? NQ<4> : F == 9 ? NQ<9> : F == 16 ? NQ<16> : NQ<25>; }
 
@@ -353,20 +420,21 @@ static Plan plan(int Cn, int CkAll, int F, int precision) {
     pl.nsplit = operand_mode(precision).nsplit;
     pl.nq = nq_of(F);
     const int g = F == 25 ? G<25> : G<4>, cn = (Cn + g - 1) / g * g;
-    if (pl.nq > cn) pl.nmma = (cn * F + 15) / 16 * 16;
-    else pl.nmma = (pl.nq * F + 15) / 16 * 16;
-    pl.nslices = (Cn + pl.nq - 1) / pl.nq;
     pl.kst = (Ck + 31) / 32;
+    pl.pair = pl.nsplit == 2 && pl.kst >= PAIR_FROM;
+    const int step = pl.pair ? 32 : 16;                           // columns of a product
+    pl.nmma = ((pl.nq > cn ? cn : pl.nq) * F + step - 1) / step * step;
+    pl.nslices = (Cn + pl.nq - 1) / pl.nq;
     const size_t budget = 226 * 1024;
-    const size_t gt = (size_t)2 * pl.kst * KTILE_BYTES, ws = (size_t)pl.nsplit * pl.nmma * 64;
+    const size_t gt = (size_t)2 * pl.kst * KTILE_BYTES, wblk = (size_t)pl.nsplit * pl.nmma * 64, ws = pl.pair ? wblk / 2 : wblk;
     // a second tile buffer takes the row copy off the critical path, when at least three filter blocks still fit beside it
-    pl.gbufs = (2 * gt + 1024 + 384 + 3 * ws <= budget) ? 2 : 1;
-    if (3 * gt + 1024 + 384 + 2 * pl.kst * ws <= budget) pl.gbufs = 3;
-    const size_t fixed = pl.gbufs * gt + 1024 + 384;
+    pl.gbufs = (2 * gt + 1024 + 640 + 3 * ws <= budget) ? 2 : 1;
+    if (3 * gt + 1024 + 640 + 2 * pl.kst * ws <= budget) pl.gbufs = 3;
+    const size_t fixed = pl.gbufs * gt + 1024 + 640;
     pl.nblocks = (int)((budget - fixed) / ws);
     if (pl.nblocks > 16) pl.nblocks = 16;
     pl.smem = fixed + pl.nblocks * ws;
-    pl.wimg_bytes = (size_t)pl.nslices * pl.kst * ws;
+    pl.wimg_bytes = (size_t)pl.nslices * pl.kst * wblk;
     return pl;
 }
 
@@ -404,15 +472,22 @@ static int map_rows(CUtensorMap* map, const float* rows, int64_t Nf, int channel
     return PB200_OK;
 }
 
-template <int NSPLIT, int F>
+template <int NSPLIT, int F, bool PAIR>
 static int launch(const char* label, const Params& p, const CUtensorMap& map, int grid, size_t smem, cudaStream_t stream) {
-    PB_CUDA(cudaFuncSetAttribute(f2f_one_sample_tc_kernel<NSPLIT, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PB_CUDA(cudaFuncSetAttribute(f2f_one_sample_tc_kernel<NSPLIT, F, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     static const int regs = [] {                                  // a kernel built with fewer would wait for registers that are not there
         cudaFuncAttributes a;
-        return cudaFuncGetAttributes(&a, f2f_one_sample_tc_kernel<NSPLIT, F>) == cudaSuccess ? a.numRegs : 0;
+        return cudaFuncGetAttributes(&a, f2f_one_sample_tc_kernel<NSPLIT, F, PAIR>) == cudaSuccess ? a.numRegs : 0;
     }();
     PB_REQUIRE(regs == REGS_LAUNCH, PB200_ECUDA, "%s: built with %d registers per thread instead of %d", label, regs, REGS_LAUNCH);
-    PB_LAUNCH(label, (f2f_one_sample_tc_kernel<NSPLIT, F>), grid, NTHREADS, smem, stream, p, map);
+    cudaLaunchAttribute two;
+    two.id = cudaLaunchAttributeClusterDimension;
+    two.val.clusterDim.x = 2; two.val.clusterDim.y = two.val.clusterDim.z = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid); c.blockDim = dim3(NTHREADS); c.dynamicSmemBytes = smem; c.stream = stream;
+    c.attrs = &two; c.numAttrs = PAIR ? 1 : 0;
+    LaunchScope scope(label, stream);
+    PB_CUDA(cudaLaunchKernelEx(&c, f2f_one_sample_tc_kernel<NSPLIT, F, PAIR>, p, map));
     return PB200_OK;
 }
 
@@ -424,8 +499,8 @@ int run(int64_t Nf, int Cn, int Ck, int F, const float* rows, const float* filte
     if (rc) return rc;
     const Plan pl = plan(Cn, Ck, F, precision);
     const int64_t s_ck = forward ? (int64_t)F : (int64_t)Cn * F, s_cn = forward ? (int64_t)Ck * F : (int64_t)F;
-    const int64_t ntiles = ceil_div(Nf, TILE_M);
-    const int sms = sm_count();
+    const int nb = pl.pair ? 2 : 1, sms = sm_count() / nb;        // CTAs, and those that work on items of their own
+    const int64_t ntiles = ceil_div(Nf, nb * TILE_M);
     // Slice groups of a tile.  With fewer tiles than SMs a tile's slices go to as many CTAs as there are.  With a few tiles per
     // SM the last wave is short of tiles: groups are halved while that evens it out, but a group keeps enough products (two
     // slices of three, four of one) for the copy of the next item's rows to hide behind.
@@ -440,14 +515,15 @@ int run(int64_t Nf, int Cn, int Ck, int F, const float* rows, const float* filte
     const int per_group = (int)ceil_div(pl.nslices, groups);
     groups = (int)ceil_div(pl.nslices, per_group);
     const int64_t items = ntiles * groups;
-    const int grid = (int)(items < sms ? items : sms);
+    PB_REQUIRE(items < 0x7fffffff / 2, PB200_EINVAL, "%s: %lld faces are too many", label, (long long)Nf);
+    const int grid = nb * (int)(items < sms ? items : sms);
     for (int k0 = 0; k0 < Ck; k0 += MAX_CK) {
         const int chunk = Ck - k0 < MAX_CK ? Ck - k0 : MAX_CK;
         const int kst = (chunk + 31) / 32;
         rc = gin::prep_filter_bf16(F, Cn, k0, chunk, pl.nq, pl.nslices, kst, pl.nsplit, pl.nmma, s_ck, s_cn, filter, (uint8_t*)ws, stream);
         if (rc) return rc;
         Params p;
-        p.Nf = Nf; p.Cn = Cn; p.Ck = chunk;
+        p.Nf = Nf; p.nitems = (int)items; p.Cn = Cn; p.Ck = chunk;
         p.nslices = pl.nslices; p.kst = kst; p.nmma = pl.nmma; p.gbufs = pl.gbufs;
         p.kb = kst;
         while (p.kb > 1 && (kst % p.kb != 0 || pl.nblocks < 2 * p.kb)) --p.kb;
@@ -461,11 +537,16 @@ int run(int64_t Nf, int Cn, int Ck, int F, const float* rows, const float* filte
         rc = map_rows(&map, p.rows, Nf, chunk, Ck, label);
         if (rc) return rc;
         const bool two = pl.nsplit == 2;
+        auto go = [&](auto f) {
+            constexpr int FF = decltype(f)::value;
+            if (pl.pair) return launch<2, FF, true>(label, p, map, grid, pl.smem, stream);
+            return two ? launch<2, FF, false>(label, p, map, grid, pl.smem, stream) : launch<1, FF, false>(label, p, map, grid, pl.smem, stream);
+        };
         switch (F) {
-            case 4: rc = two ? launch<2, 4>(label, p, map, grid, pl.smem, stream) : launch<1, 4>(label, p, map, grid, pl.smem, stream); break;
-            case 9: rc = two ? launch<2, 9>(label, p, map, grid, pl.smem, stream) : launch<1, 9>(label, p, map, grid, pl.smem, stream); break;
-            case 16: rc = two ? launch<2, 16>(label, p, map, grid, pl.smem, stream) : launch<1, 16>(label, p, map, grid, pl.smem, stream); break;
-            default: rc = two ? launch<2, 25>(label, p, map, grid, pl.smem, stream) : launch<1, 25>(label, p, map, grid, pl.smem, stream); break;
+            case 4: rc = go(std::integral_constant<int, 4>{}); break;
+            case 9: rc = go(std::integral_constant<int, 9>{}); break;
+            case 16: rc = go(std::integral_constant<int, 16>{}); break;
+            default: rc = go(std::integral_constant<int, 25>{}); break;
         }
         if (rc) return rc;
     }

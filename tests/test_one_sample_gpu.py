@@ -50,6 +50,33 @@ def test_one_sample_backward(nf, cin, cout, F, precision, gate):
     assert _lib.query("pb200_async_error") == 0
 
 
+@pytest.mark.parametrize("nf", [1, 127, 128, 129, 255, 256, 257, 511, 40001])
+@pytest.mark.parametrize("cin,cout,F", [(100, 20, 4), (128, 48, 9), (100, 128, 16), (260, 36, 25), (64, 64, 16), (512, 12, 9)])
+@pytest.mark.parametrize("precision,gate", [(_lib.PREC_FP32, 2e-5), (_lib.PREC_BF16, 2e-2)])
+def test_one_sample_forward(nf, cin, cout, F, precision, gate):
+    """Around the 128 rows of a tile and the 256 of a pair of CTAs (from 97 contracted channels on), contracted channels that fill no
+    K-block, more than one launch holds, and rows behind the last face."""
+    g = torch.Generator(device="cuda").manual_seed(nf + cin)
+    x = torch.randn(nf, cin, device="cuda", generator=g)
+    w = torch.rand(nf, F, device="cuda", generator=g)
+    filt = torch.randn(cout, cin, F, device="cuda", generator=g) / (cin * F) ** 0.5
+    wp = torch.nn.functional.pad(w, (0, -F % 4)).contiguous()
+    need = _lib.query("pb200_facet2facet_one_sample_forward_workspace_bytes", nf, cin, cout, F, precision)
+    ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+    out = torch.full((nf + 1, cout), 7., device="cuda")
+
+    def run():
+        _lib.call("pb200_facet2facet_one_sample_forward", nf, cin, cout, F, ptr(x), ptr(filt), ptr(w), ptr(wp), ptr(out), precision, ptr(ws),
+                  need, stream_ptr(x.device))
+        return out.clone()
+
+    got = run()
+    want = ((x.double() @ filt.double().transpose(1, 2).reshape(cout, F, cin).reshape(-1, cin).T).reshape(nf, cout, F) * w.double()[:, None]).sum(2)
+    assert rel_err(got[:nf], want) <= gate
+    assert torch.equal(got, run()) and bool((got[nf] == 7).all())
+    assert _lib.query("pb200_async_error") == 0
+
+
 @pytest.mark.parametrize("precision,F,cin,names", [
     (_lib.PREC_FP32, 16, 64, {"f2f_bwd_gin_one_tc", "f2f_bwd_gfilter_one_tc", "f2f_bwd_gfilter_one_reduce"}),
     (_lib.PREC_BF16, 25, 128, {"f2f_bwd_gin_one_tc", "f2f_bwd_gfilter_one_tc", "f2f_bwd_gfilter_one_reduce"}),
