@@ -359,6 +359,22 @@ int pb200_facet2facet_one_sample_backward(int64_t Nf, int Cin, int Cout, int F, 
                                           const int32_t* oneEach, float* gradInput, float* gradFilter, int precision,
                                           void* workspace, size_t workspace_bytes, void* stream);
 
+/* What a layer makes of facet2facet: act = activation(facet2facet + bias) (bias may be NULL) and the statistics of its rows, as
+ * pb200_bias_act_stats leaves them (partial: pb200_norm_parts(Nf, Cout) * 3 * Cout floats); workspace of
+ * pb200_facet2facet_forward_workspace_bytes. */
+int pb200_facet2facet_layer_forward(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, const float* input, const float* filter,
+                                    const float* bary, const int32_t* numInterior, const float* bias, int relu, float* act,
+                                    float* partial, int* nparts, int precision, void* workspace, size_t workspace_bytes, void* stream);
+
+/* Gradients of filter and bias of that layer in one pass, for samples that need no gradient: gradOutput goes back through the
+ * normalisation (norm, NULL without one) and the activation on the way.  For what ..._fused says 1 to. */
+int pb200_facet2facet_layer_gradient_fused(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, const float* bary, int precision);
+size_t pb200_facet2facet_layer_filter_gradient_workspace_bytes(int64_t Nf, int Cout, int F);
+int pb200_facet2facet_layer_filter_gradient(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, const float* gradOutput, const float* act,
+                                            int relu, const pb200_norm_gradient* norm, const float* input, const float* bary,
+                                            const int32_t* numInterior, float* gradFilter, float* gradBias, int precision,
+                                            void* workspace, size_t workspace_bytes, void* stream);
+
 /* The filter gradient alone (same workspace), for samples that are data and need no gradient. */
 int pb200_facet2facet_filter_gradient(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, const float* gradOutput,
                                       const float* input, const float* bary, const float* baryPadded, const int32_t* numInterior,

@@ -18,6 +18,14 @@ size_t workspace_bytes(int64_t Nf, int Cin, int Cout, int F);
 int backward_filter(int64_t Nf, int Cin, int Cout, int F, const float* gout, const float* input, const float* bary, const int32_t* cum,
                     float* gfilter, void* ws, cudaStream_t stream);
 }  // namespace small
+namespace rgb {
+bool supported(int Cin, int Cout, int F, const float* bary);
+int forward(int64_t Nf, int Cout, int F, const float* input, const float* filter, const float* bary, const int32_t* cum, const float* bias,
+            int relu, float* output, float* stats, int most, int* nparts, cudaStream_t stream);
+size_t workspace_bytes(int64_t Nf, int Cout, int F);
+int backward_filter(int64_t Nf, int Cout, int F, const float* gout, const float* act, int relu, const pb200_norm_gradient* norm,
+                    const float* input, const float* bary, const int32_t* cum, float* gfilter, float* gbias, void* ws, cudaStream_t stream);
+}  // namespace rgb
 namespace tc {
 bool fwd_supported(int Cin, int Cout, int F);
 size_t fwd_workspace_bytes(int64_t NiK, int Cin, int Cout, int F, int precision);
@@ -112,7 +120,11 @@ int pb200_facet2facet_forward(int64_t Nf, int64_t NiK, int Cin, int Cout, int F,
                "facet2facet_forward: null pointer");
     PB_REQUIRE(workspace && workspace_bytes >= pb200_facet2facet_forward_workspace_bytes(Nf, NiK, Cin, Cout, F, precision),
                PB200_EWORKSPACE, "facet2facet_forward: workspace too small");
-    if (use_small(Nf, Cin, Cout, F, precision)) return small::forward(Nf, Cin, Cout, F, input, filter, bary, numInterior, output, stream);
+    if (use_small(Nf, Cin, Cout, F, precision)) {
+        if (rgb::supported(Cin, Cout, F, bary))
+            return rgb::forward(Nf, Cout, F, input, filter, bary, numInterior, nullptr, 0, output, nullptr, 0, nullptr, stream);
+        return small::forward(Nf, Cin, Cout, F, input, filter, bary, numInterior, output, stream);
+    }
     if (use_tc_fwd(Cin, Cout, F, precision)) {
         PB_REQUIRE(NiK == 0 || aligned16(input), PB200_EINVAL, "facet2facet_forward: input must be 16-byte aligned");
         PB_REQUIRE(aligned16(workspace), PB200_EINVAL, "facet2facet_forward: workspace must be 16-byte aligned");
@@ -120,6 +132,45 @@ int pb200_facet2facet_forward(int64_t Nf, int64_t NiK, int Cin, int Cout, int F,
                            stream);
     }
     return f2f_simt_forward(Nf, NiK, Cin, Cout, F, input, filter, bary, numInterior, output, workspace, stream);
+}
+
+int pb200_facet2facet_layer_forward(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, const float* input, const float* filter,
+                                    const float* bary, const int32_t* numInterior, const float* bias, int relu, float* act,
+                                    float* partial, int* nparts, int precision, void* workspace, size_t workspace_bytes, void* stream) {
+    PB_REQUIRE(f2f_sizes_ok(Nf, NiK, Cin, Cout, F) && Nf > 0, PB200_EINVAL, "facet2facet_layer_forward: bad sizes (F must be in 1..50)");
+    PB_REQUIRE(partial && nparts, PB200_EINVAL, "facet2facet_layer_forward: null pointer");
+    if (use_small(Nf, Cin, Cout, F, precision) && rgb::supported(Cin, Cout, F, bary)) {
+        PB_REQUIRE(filter && numInterior && act && (NiK == 0 || (input && bary)), PB200_EINVAL, "facet2facet_layer_forward: null pointer");
+        return rgb::forward(Nf, Cout, F, input, filter, bary, numInterior, bias, relu, act, partial, pb200_norm_parts(Nf, Cout), nparts,
+                            (cudaStream_t)stream);
+    }
+    const int rc = pb200_facet2facet_forward(Nf, NiK, Cin, Cout, F, input, filter, bary, numInterior, act, precision, workspace, workspace_bytes,
+                                             stream);
+    return rc ? rc : pb200_bias_act_stats(Nf, Cout, act, bias, relu, partial, nparts, stream);
+}
+
+int pb200_facet2facet_layer_gradient_fused(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, const float* bary, int precision) {
+    return Nf > 0 && f2f_sizes_ok(Nf, NiK, Cin, Cout, F) && use_small_gf(Nf, Cin, Cout, F, precision) &&
+                   rgb::supported(Cin, Cout, F, bary) ? 1 : 0;
+}
+
+int pb200_facet2facet_layer_filter_gradient(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, const float* gradOutput, const float* act,
+                                            int relu, const pb200_norm_gradient* norm, const float* input, const float* bary,
+                                            const int32_t* numInterior, float* gradFilter, float* gradBias, int precision,
+                                            void* workspace, size_t workspace_bytes, void* stream) {
+    PB_REQUIRE(pb200_facet2facet_layer_gradient_fused(Nf, NiK, Cin, Cout, F, bary, precision), PB200_EINVAL,
+               "facet2facet_layer_filter_gradient: sizes that the fused gradient is not for");
+    PB_REQUIRE(gradOutput && act && gradFilter && gradBias && numInterior && (NiK == 0 || (input && bary)) &&
+                   (!norm || (norm->mean && norm->scale && norm->k1 && norm->k2)),
+               PB200_EINVAL, "facet2facet_layer_filter_gradient: null pointer");
+    PB_REQUIRE(workspace && workspace_bytes >= rgb::workspace_bytes(Nf, Cout, F), PB200_EWORKSPACE,
+               "facet2facet_layer_filter_gradient: workspace too small");
+    return rgb::backward_filter(Nf, Cout, F, gradOutput, act, relu, norm, input, bary, numInterior, gradFilter, gradBias, workspace,
+                                (cudaStream_t)stream);
+}
+
+size_t pb200_facet2facet_layer_filter_gradient_workspace_bytes(int64_t Nf, int Cout, int F) {
+    return Nf > 0 && Cout > 0 && F > 0 ? rgb::workspace_bytes(Nf, Cout, F) : 0;
 }
 
 // One sample per face: output[f,co] = sum_d weights[f,d] * (sum_ci input[f,ci] * filter[co,ci,d]).  The inner
@@ -269,7 +320,9 @@ static int f2f_backward_impl(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, 
         w += gin_ws(Cin, Cout, F, precision);
     }
     if (sf) {
-        int rc = small::backward_filter(Nf, Cin, Cout, F, gradOutput, input, bary, numInterior, gradFilter, w, stream);
+        int rc = rgb::supported(Cin, Cout, F, bary)
+                     ? rgb::backward_filter(Nf, Cout, F, gradOutput, nullptr, 0, nullptr, input, bary, numInterior, gradFilter, nullptr, w, stream)
+                     : small::backward_filter(Nf, Cin, Cout, F, gradOutput, input, bary, numInterior, gradFilter, w, stream);
         if (rc) return rc;
     } else if (tf && one_each && tc::onef::supported(Cin, Cout, F, precision)) {
         int rc = tc::onef::backward_filter(Nf, Cin, Cout, F, gradOutput, input, bary_p, gradFilter, precision, w, stream);

@@ -19,6 +19,7 @@
 // Layout: a team of TL = min(32, C/V) threads takes a row, a thread V = 4 (16-byte loads, C % 4 == 0 and aligned rows)
 // or 1 channels of it; four rows of a thread are in flight; gridDim.y walks chunks of 32 thread columns.
 #include "common.cuh"
+#include "moments.cuh"
 
 namespace pb {
 namespace norm {
@@ -37,22 +38,6 @@ template <int V> __device__ __forceinline__ Vec<V> load(const float* p) {
 template <int V> __device__ __forceinline__ void store(float* p, const Vec<V>& x) {
     if (V == 4) *reinterpret_cast<float4*>(p) = make_float4(x.v[0], x.v[1 % V], x.v[2 % V], x.v[3 % V]);
     else *p = x.v[0];
-}
-
-// ReLU as torch has it: a NaN stays one, forward and backward
-__device__ __forceinline__ float relu_of(float x) {
-    float y;
-    asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float relu_grad(float g, float act) { return act <= 0.f ? 0.f : g; }
-
-struct Moments { float n, mean, m2; };
-__device__ __forceinline__ void merge(Moments& a, const Moments& b) {
-    const float n = a.n + b.n, d = b.mean - a.mean, f = b.n > 0.f ? __fdividef(b.n, n) : 0.f;      // no branch: loads run ahead
-    a.mean = fmaf(d, f, a.mean);
-    a.m2 += b.m2 + d * d * a.n * f;
-    a.n = n;
 }
 
 constexpr int THREADS = 256;
@@ -96,9 +81,7 @@ stats_kernel(int64_t N, int C, float* __restrict__ rows, const float* __restrict
     }
 #pragma unroll
     for (int j = 0; j < V; ++j) {
-        Moments m{(float)n, shift[j], 0.f};
-        if (n > 0) { m.mean = shift[j] + s1[j] / (float)n; m.m2 = relu_of(s2[j] - s1[j] * s1[j] / (float)n); }    // (a NaN stays one)
-        red[team][lane][j] = m;
+        red[team][lane][j] = moments((float)n, shift[j], s1[j], s2[j]);
     }
     __syncthreads();
     if (team == 0 && active) {

@@ -762,9 +762,24 @@ struct F2FLayer : Node {
             out[3] = n.gamma;
             out[4] = n.beta;
         }
+        const Tensor w = filter.unpack();
+        const int64_t Nf = a.size(0), NiK = x.size(0), Cin = x.size(1), Cout = w.size(0), F = w.size(2);
+        const Tensor weights = aligned(bary.unpack());
+        if (!task_should_compute_output(0) &&
+            pb200_facet2facet_layer_gradient_fused(Nf, NiK, (int)Cin, (int)Cout, (int)F, fp(weights), precision)) {
+            out[1] = s.floats(w.sizes());
+            out[2] = s.floats({1, Cout});
+            const size_t nb = pb200_facet2facet_layer_filter_gradient_workspace_bytes(Nf, (int)Cout, (int)F);
+            const Tensor ws = s.bytes(nb), samples = aligned(x), ends = cum.unpack();
+            call(pb200_facet2facet_layer_filter_gradient(Nf, NiK, (int)Cin, (int)Cout, (int)F, fp(g), fp(a), relu,
+                                                         st.mean.defined() ? &n.factors : nullptr, fp(samples), fp(weights), ip(ends), fpm(out[1]),
+                                                         fpm(out[2]), precision, ws.data_ptr(), nb, s.stream),
+                 "pb200_facet2facet_layer_filter_gradient");
+            return out;
+        }
         Tensor gm;
         masked_gradient(s, g, a, n, relu, gm, out[2]);
-        f2f_backward(s, gm, aligned(x), filter.unpack(), aligned(bary.unpack()), Tensor(), cum.unpack(), precision, out[0], out[1],
+        f2f_backward(s, gm, aligned(x), w, weights, Tensor(), cum.unpack(), precision, out[0], out[1],
                      task_should_compute_output(0));
         return out;
     }
@@ -908,13 +923,10 @@ Tensor rows_layer(const Tensor& rows_in, const Tensor& weights, const OptTensor&
     return r.out;
 }
 
-// act <- activation(act + bias) in place, out = its normalisation (act itself without one); the statistics used
-NormStats bias_act_norm(const Scope& s, const Tail& t, const Tensor& act, const Tensor& bias, Tensor& out) {
-    const int64_t rows = act.size(0), C = act.size(1);
-    check_tail(t, C);
-    Tensor partial = s.floats({pb200_norm_parts(rows, (int)C), 3, C});
-    int parts = 0;
-    call(pb200_bias_act_stats(rows, (int)C, fpm(act), fp(bias), t.relu, fpm(partial), &parts, s.stream), "pb200_bias_act_stats");
+// out = the normalisation of activated rows (act itself without one) by the statistics of the batch, from their partials, or the
+// running ones; the batch's statistics
+NormStats normalise_by(const Scope& s, const Tail& t, const Tensor& act, int parts, const Tensor& partial, Tensor& out) {
+    const int64_t C = act.size(1);
     out = act;
     NormStats st;
     if (t.mode == NORM_BATCH) {
@@ -928,6 +940,16 @@ NormStats bias_act_norm(const Scope& s, const Tail& t, const Tensor& act, const 
     return st;
 }
 
+// act <- activation(act + bias) in place, out = its normalisation (act itself without one); the statistics used
+NormStats bias_act_norm(const Scope& s, const Tail& t, const Tensor& act, const Tensor& bias, Tensor& out) {
+    const int64_t rows = act.size(0), C = act.size(1);
+    check_tail(t, C);
+    Tensor partial = s.floats({pb200_norm_parts(rows, (int)C), 3, C});
+    int parts = 0;
+    call(pb200_bias_act_stats(rows, (int)C, fpm(act), fp(bias), t.relu, fpm(partial), &parts, s.stream), "pb200_bias_act_stats");
+    return normalise_by(s, t, act, parts, partial, out);
+}
+
 // facet2facet over the samples of every face (`counts` per face), then bias, ReLU or nothing, normalisation
 Tensor f2f_layer(const Tensor& input, const Tensor& filter, const Tensor& bary, const Tensor& counts, const Tensor& bias0, TAIL_PARAMS) {
     const Tail t = make_tail(TAIL_ARGS);
@@ -939,8 +961,17 @@ Tensor f2f_layer(const Tensor& input, const Tensor& filter, const Tensor& bary, 
     Scope s(input);
     const Tensor cum = at::cumsum(counts, 0, at::kInt), bias = flat(bias0, filter.size(0));
     check(cum, "num_texture", 1, at::kInt);
-    Tensor act = f2f_forward(s, aligned(input), filter, bary, cum, precision), out;
-    const NormStats st = bias_act_norm(s, t, act, bias, out);
+    const int64_t NiK = input.size(0), Cin = input.size(1), Cout = filter.size(0), F = filter.size(2), Nf = cum.size(0);
+    check_tail(t, Cout);
+    const Tensor x = aligned(input), act = s.floats({Nf, Cout}), partial = s.floats({pb200_norm_parts(Nf, (int)Cout), 3, Cout});
+    const size_t nb = pb200_facet2facet_forward_workspace_bytes(Nf, NiK, (int)Cin, (int)Cout, (int)F, precision);
+    const Tensor ws = s.bytes(nb);
+    int parts = 0;
+    call(pb200_facet2facet_layer_forward(Nf, NiK, (int)Cin, (int)Cout, (int)F, fp(x), fp(filter), fp(bary), ip(cum), fp(bias), relu, fpm(act),
+                                         fpm(partial), &parts, precision, ws.data_ptr(), nb, s.stream),
+         "pb200_facet2facet_layer_forward");
+    Tensor out;
+    const NormStats st = normalise_by(s, t, act, parts, partial, out);
     if (node) {
         node->input = keep(input);
         node->filter = keep(filter);
