@@ -62,7 +62,7 @@ def _ops_command(out: str):
             [a for d in (inc, os.path.join(inc, "torch", "csrc", "api", "include"), os.path.join(cuda, "include"),
                          sysconfig.get_paths()["include"]) for a in ("-isystem", d)] +
             [os.path.join(CSRC, "torch_ops.cpp"), "-o", out, "-L" + PKG, "-l:libpicasso_b200.so", "-L" + lib, "-lc10", "-lc10_cuda",
-             "-ltorch_cpu", "-ltorch", "-ltorch_python", "-L" + os.path.join(cuda, "lib64"), "-lcudart", "-Wl,-rpath,$ORIGIN:" + lib])
+             "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", "-L" + os.path.join(cuda, "lib64"), "-lcudart", "-Wl,-rpath,$ORIGIN:" + lib])
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
