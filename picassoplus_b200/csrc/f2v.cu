@@ -667,6 +667,16 @@ int f2v_face_products(int64_t Nf, int C, int K, const float* input, const float*
     return PB200_OK;
 }
 
+// The vertex stage on its own: sums of the faces' products, over nfCount (C % 4 == 0, 16-byte aligned rows).
+int f2v_gather(int64_t NvOut, int C, const int32_t* rowptr, const int32_t* entries, const int32_t* nfCount, const float* wx, float* output,
+               cudaStream_t stream) {
+    const TeamGeom g = team_geom(C / 4);
+    const dim3 grid(persistent_blocks(NvOut, g.teams, 4), g.chunks);
+    PB_DISPATCH_TL(g.TL, PB_LAUNCH("f2v_fwd_gather", f2v_fwd_gather_kernel<TL>, grid, 256, 0, stream, NvOut, C / 4, rowptr, entries, nfCount,
+                                   (const float4*)wx, (float4*)output));
+    return PB200_OK;
+}
+
 }  // namespace pb
 
 using namespace pb;
@@ -694,14 +704,10 @@ int pb200_facet2vertex_forward(int64_t Nf, int64_t NvOut, int C, int r, int K, c
     if (vec_ok(C, r) && kt_ok(K) && aligned16(input) && aligned16(filter) && aligned16(output))
         PB_REQUIRE(vec, PB200_EWORKSPACE, "facet2vertex_forward: workspace missing, misaligned or too small");
     if (vec) {
-        int CV = C / 4;
-        float4* wx = (float4*)workspace;
-        int rc = f2v_face_products(Nf, C, K, input, filter, coeff, (float*)wx, stream);
+        float* wx = (float*)workspace;
+        int rc = f2v_face_products(Nf, C, K, input, filter, coeff, wx, stream);
         if (rc) return rc;
-        TeamGeom g = team_geom(CV);
-        dim3 grid(persistent_blocks(NvOut, g.teams, 4), g.chunks);
-        PB_DISPATCH_TL(g.TL, PB_LAUNCH("f2v_fwd_gather", f2v_fwd_gather_kernel<TL>, grid, 256, 0, stream, NvOut, CV,
-                                       rowptr, entries, nfCount, (const float4*)wx, (float4*)output));
+        return f2v_gather(NvOut, C, rowptr, entries, nfCount, wx, output, stream);
     } else {
         int grid = persistent_blocks(NvOut * C * r, 256, 16);
         PB_LAUNCH("f2v_fwd_generic", f2v_fwd_generic_kernel, grid, 256, 0, stream, NvOut, C, r, K, rowptr, entries,

@@ -590,13 +590,25 @@ void masked_gradient(const Scope& s, const Tensor& g, const Tensor& act, const N
 // The pointwise stage of a forward pass.  `launch` runs the operator's layer entry with the extras it is handed; what
 // the backward pass needs stays in `act`, `features` and `stats`.
 struct Staged { Tensor out, act, features; NormStats stats; };
+// What a pass that keeps no features may spend on gathered rows (2 M rows of 128 channels); larger ones gather inside the product.
+constexpr int64_t GATHER_BYTES = int64_t(1) << 30;
 template <typename Launch>
-Staged run_stage(const Scope& s, const Tail& t, int64_t rows, int64_t C, int64_t Cout, bool keep_features, Launch&& launch) {
+Staged run_stage(const Scope& s, const Tail& t, int64_t rows, int64_t C, int64_t Cout, bool keep_features, bool gathers, Launch&& launch) {
     check_tail(t, Cout);
     Staged r;
     r.act = s.floats({rows, Cout});
     pb200_pointwise_extra x = {};
-    if (keep_features) { r.features = s.floats({rows, C}); x.features = fpm(r.features); }
+    Workspace scratch;
+    if (keep_features) {
+        r.features = s.floats({rows, C});
+        x.features = fpm(r.features);
+    } else if (gathers && pb200_layer_wants_features(rows) && rows <= GATHER_BYTES / 4 / C) {
+        try {
+            scratch = s.bytes((size_t)(4 * rows * C));
+            x.features = static_cast<float*>(scratch.data_ptr());
+        } catch (const c10::OutOfMemoryError&) {      // the kernel that needs no room for them is still there
+        }
+    }
     if (t.mode == NORM_RUNNING) {
         x.mean = fp(t.running_mean); x.var = fp(t.running_var); x.gamma = fp(t.gamma); x.beta = fp(t.beta); x.eps = (float)t.eps;
     }
@@ -837,7 +849,7 @@ Tensor v2f_layer(const Tensor& x_in, const Tensor& face, const OptTensor& rowptr
     const Tensor filter = at::matmul(corners, spatial).view({3, C, 1});
     const size_t nb = pb200_vertex2facet_pointwise_workspace_bytes((int)C, precision);
     const Workspace ws = s.bytes(nb);
-    Staged r = run_stage(s, t, Nf, C, Cout, (bool)node, [&](float* out, const pb200_pointwise_extra* extra) {
+    Staged r = run_stage(s, t, Nf, C, Cout, (bool)node, true, [&](float* out, const pb200_pointwise_extra* extra) {
         call(pb200_vertex2facet_layer_forward(Nf, Nv, (int)C, (int)Cout, fp(x), fp(filter), ip(face), fp(weights_in), fp(bias), relu, out,
                                               precision, extra, ws.data_ptr(), nb, s.stream),
              "pb200_vertex2facet_layer_forward");
@@ -880,7 +892,7 @@ Tensor f2v_layer(const Tensor& x_in, const Tensor& face, const Tensor& nf_count,
     const Tensor x = aligned(x_in), filter = aligned(filter_in), bias = flat(bias0, Cout);
     const size_t nb = pb200_facet2vertex_pointwise_workspace_bytes(Nf, (int)C, precision);
     const Workspace ws = s.bytes(nb);
-    Staged r = run_stage(s, t, NvOut, C, Cout, (bool)node, [&](float* out, const pb200_pointwise_extra* extra) {
+    Staged r = run_stage(s, t, NvOut, C, Cout, (bool)node, true, [&](float* out, const pb200_pointwise_extra* extra) {
         call(pb200_facet2vertex_layer_forward(Nf, NvOut, (int)C, (int)K, (int)Cout, fp(x), fp(filter), fp(coeff), ip(nf_count), ip(rowptr),
                                               ip(entries), fp(weights), fp(bias), relu, out, precision, extra, ws.data_ptr(), nb, s.stream),
              "pb200_facet2vertex_layer_forward");
@@ -920,7 +932,7 @@ Tensor rows_layer(const Tensor& rows_in, const Tensor& weights, const OptTensor&
     const Tensor rows = aligned(rows_in), bias = flat(bias0, Cout);
     const size_t nb = pb200_masked_rows_matmul_workspace_bytes((int)C, precision);
     const Workspace ws = s.bytes(nb);
-    Staged r = run_stage(s, t, N, C, Cout, false, [&](float* out, const pb200_pointwise_extra* extra) {
+    Staged r = run_stage(s, t, N, C, Cout, false, false, [&](float* out, const pb200_pointwise_extra* extra) {
         call(pb200_rows_layer_forward(N, (int)C, (int)Cout, fp(rows), fp(weights), fp(bias), relu, out, precision, extra, ws.data_ptr(), nb,
                                       s.stream),
              "pb200_rows_layer_forward");

@@ -50,3 +50,44 @@ def test_rows(copies, odd, C):
     assert rel_err(rows, want / count.clamp(min=1).double()[:, None]) <= 5e-6
     again = conv3d.vertex2facet_backward(go, x, w, face)
     assert torch.equal(gin, again[0]) and torch.equal(gw, again[1])
+
+
+@pytest.mark.parametrize("train", [False, True])
+@pytest.mark.parametrize("rows", [99999, 100000, 100003])
+@pytest.mark.parametrize("C,cout", [(8, 72), (64, 128), (136, 136)])
+def test_layers_where_the_gather_leaves_the_product(C, cout, rows, train):
+    """Layers over 100 000 rows and more gather in a kernel of their own: the bits of the fused kernel, which takes each part of a call
+    that is split in two, with and without the features kept for a backward pass."""
+    from picassoplus_b200 import _lib
+    from picassoplus_b200.mesh.pi_modules import fused
+    g = torch.Generator(device="cuda").manual_seed(rows + C)
+    randn = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    half = 50000
+    weights, bias, filt = randn(C, cout), randn(1, cout), randn(3, C, 1)
+    x = randn(4000, C)
+    face = torch.randint(4000, (rows, 3), device="cuda", generator=g).int()
+    whole = fused.vertex2facet_pointwise(x, filt, face, weights.requires_grad_(train), bias, True)
+    with torch.no_grad():
+        parts = [fused.vertex2facet_pointwise(x, filt, f.contiguous(), weights, bias, True) for f in (face[:half], face[half:])]
+    assert torch.equal(whole, torch.cat(parts))
+    if train:
+        go = randn(rows, cout)
+        grad, = torch.autograd.grad(whole, weights, go)
+        rows64 = (x.double()[face.long()] * filt.double()[:, :, 0]).sum(1)
+        # operands of a bf16 high and low part: 2^-16 of each product
+        assert rel_err(grad, rows64.t() @ (go.double() * (whole > 0))) <= 1e-4
+    # vertices: the first have no faces, the last have many
+    degree = torch.arange(rows, device="cuda") % 11
+    rowptr = torch.cat([degree.new_zeros(1), degree.cumsum(0)]).int()
+    nf, K = 30000, 9
+    entries = (torch.randint(nf, (int(rowptr[-1]),), device="cuda", generator=g) * 4).int()
+    xf, coeff, wf = randn(nf, C), randn(nf, K), randn(K, C, 1)
+    fake = torch.zeros(nf, 3, dtype=torch.int32, device="cuda")
+    tail = (1, *fused._NO_NORM)
+
+    def layer(lo, hi):
+        return _lib.ops.f2v_layer(xf, fake, degree[lo:hi].int(), torch.zeros(hi - lo, dtype=torch.int32, device="cuda"),
+                                  rowptr[lo:hi + 1].clone(), entries, coeff, wf, weights, bias, *tail, fused._precision)
+    whole = layer(0, rows)
+    with torch.no_grad():
+        assert torch.equal(whole, torch.cat([layer(0, half), layer(half, rows)]))
