@@ -49,7 +49,7 @@ using namespace ptx;
 
 constexpr int TILE_M = 128;
 constexpr int NCOLS = 256;                       // accumulator columns
-constexpr int EWARPS = 16;                       // epilogue warps: 2 groups x 4 TMEM quadrants x 2
+constexpr int EWARPS = 16;                       // epilogue warps: four per TMEM quadrant
 constexpr int GWARPS = 1;                        // row converters
 constexpr int NTHREADS = (EWARPS + 3 + GWARPS) * 32;
 // Registers per thread: at launch, of the epilogue's four warpgroups, of the two that hold filter stream, issue, row stream and converters

@@ -31,7 +31,7 @@ __device__ __forceinline__ void set_zero(float4& a) { a = zero4(); }
 __device__ __forceinline__ float quot(float x, float c) {
     const float r = __frcp_rn(c), q = x * r;
     const uint32_t u = __float_as_uint(x) & 0x7fffffffu;       // 2^-60 <= |x| < infinity, or zero
-    if ((u - 0x21800000u < 0x5e000000u || u == 0) && c >= 1.f && c <= 16777216.f) return fmaf(fmaf(-q, c, x), r, q);
+    if ((u - 0x21800000u < 0x5e000000u || u == 0) && c >= 1.f && c <= 16777216.f) return u ? fmaf(fmaf(-q, c, x), r, q) : x;
     return x / c;
 }
 __device__ __forceinline__ float4 quot(const float4& x, float c) { return make_float4(quot(x.x, c), quot(x.y, c), quot(x.z, c), quot(x.w, c)); }

@@ -173,3 +173,12 @@ def test_level_prepare_matches_the_separate_calls(kind, L, orient):
     n = int(ref_csr.rowptr[-1])
     assert torch.equal(got["csr"].entries[:n], ref_csr.entries[:n])
     assert topology.vertex_csr(face, vt_map, d["vt_map"].shape[0], d["nv_out"]) is got["csr"]     # served from the cache
+
+
+@pytest.mark.parametrize("C", [5, 64])
+def test_average_gradient_keeps_the_sign_of_zero(C):
+    """A gradient of -0 over any member count is -0, as the division gives it."""
+    from picassoplus_b200.mesh.pi_modules import pool3d
+    d = _dev(cluster_inputs(300, 90, C, seed=3, ties=False))
+    got = pool3d.avg_backward(torch.full((90, C), -0.0, device="cuda"), d["x"], d["vt_replace"], d["vt_map"])
+    assert torch.signbit(got[d["vt_map"] >= 0]).all()
