@@ -166,16 +166,15 @@ __global__ void triangle_geometry_kernel(int64_t Nf, int64_t Nv, int vstride, co
 // per-vertex corner counts that seed the vertex CSR (= the reference's nfCount).  The vertex rows of
 // a face are read once for all of it; the K coefficients are staged through shared memory so the
 // global store is coalesced.
-constexpr int PREP_BLOCK = 128;
-
-__global__ void __launch_bounds__(PREP_BLOCK)
+template <int L>
+__global__ void __launch_bounds__(SPH_BLOCK)
 level_prepare_kernel(int64_t Nf, int64_t NvIn, int64_t NvOut, int vstride, const float* __restrict__ vertex,
-                     const int32_t* __restrict__ face, const int32_t* __restrict__ vtMap, int L, int orient, SphConst cst,
+                     const int32_t* __restrict__ face, const int32_t* __restrict__ vtMap, int orient, SphConst cst,
                      float* __restrict__ geom, float* __restrict__ normal_out, float* __restrict__ coeff,
-                     int32_t* __restrict__ cnt, int32_t* __restrict__ status) {
-    extern __shared__ float stage[];            // [PREP_BLOCK][K+1]
-    const int K = (L + 1) * (L + 1), KP = K + 1;
-    const int64_t base = (int64_t)blockIdx.x * PREP_BLOCK;
+                     int32_t* __restrict__ cnt, int32_t* __restrict__ status, bool vec) {
+    constexpr int K = (L + 1) * (L + 1);
+    __shared__ __align__(16) float stage[SPH_BLOCK * sph_pitch<K>];
+    const int64_t base = (int64_t)blockIdx.x * SPH_BLOCK;
     const int64_t f = base + threadIdx.x;
     if (f < Nf) {
         const int i0 = face[3 * f], i1 = face[3 * f + 1], i2 = face[3 * f + 2];
@@ -211,7 +210,9 @@ level_prepare_kernel(int64_t Nf, int64_t NvIn, int64_t NvOut, int vstride, const
             if (geom) { float* g = geom + f * 5; g[0] = g[1] = g[2] = g[3] = g[4] = 0.f; }
         }
         if (normal_out) { normal_out[3 * f] = nx; normal_out[3 * f + 1] = ny; normal_out[3 * f + 2] = nz; }
-        sph_eval(nx, ny, nz, L, cst.c, stage + threadIdx.x * KP);
+        float o[K];
+        sph_eval(nx, ny, nz, L, cst.c, o);
+        put_row<K>(stage, o);
         if (cnt && ok) {
             const int vi[3] = {i0, i1, i2};
 #pragma unroll
@@ -223,12 +224,7 @@ level_prepare_kernel(int64_t Nf, int64_t NvIn, int64_t NvOut, int vstride, const
         }
     }
     __syncthreads();
-    const int64_t nfb = Nf - base < PREP_BLOCK ? Nf - base : PREP_BLOCK;
-    float* dst = coeff + base * K;
-    for (int64_t j = threadIdx.x; j < nfb * K; j += PREP_BLOCK) {
-        const int p = (int)(j / K), k = (int)(j - (int64_t)p * K);
-        dst[j] = stage[p * KP + k];
-    }
+    write_rows<K>(stage, (int)(Nf - base < SPH_BLOCK ? Nf - base : SPH_BLOCK), coeff + base * K, vec);
 }
 
 // ------------------------------------------------------------------------ row expansion
@@ -420,10 +416,9 @@ int pb200_level_prepare(int64_t Nf, int64_t NvIn, int64_t NvOut, int vstride, co
     PB_CUDA(cudaMemsetAsync(w.cursor, 0, sizeof(int32_t) * (NvOut + 1), stream));
     if (Nf > 0) {
         static const SphConst cst = make_sph_const();
-        const int K = (L + 1) * (L + 1);
-        PB_LAUNCH("level_prepare", level_prepare_kernel, (unsigned)ceil_div(Nf, PREP_BLOCK), PREP_BLOCK,
-                  sizeof(float) * PREP_BLOCK * (K + 1), stream, Nf, NvIn, NvOut, vstride, vertex, face, vtMap, L, orient, cst,
-                  geometry, normals, coeff, w.cursor, status);
+        PB_DISPATCH_DEGREE(L, PB_LAUNCH("level_prepare", level_prepare_kernel<DEG>, (unsigned)ceil_div(Nf, SPH_BLOCK), SPH_BLOCK, 0, stream,
+                                        Nf, NvIn, NvOut, vstride, vertex, face, vtMap, orient, cst, geometry, normals, coeff, w.cursor,
+                                        status, aligned16(coeff)));
     }
     // the corner counts are the reference's nfCount
     return pb::finish_vertex_csr(Nf, NvIn, NvOut, face, vtMap, rowptr, entries, nfCount, w, stream);

@@ -8,65 +8,54 @@
 
 namespace pb {
 
-constexpr int SPH_BLOCK = 128;
-
-// the block's rows, K of K + 1 floats each in shared memory, to consecutive addresses.  Element j + SPH_BLOCK lies SPH_BLOCK / K rows
-// and SPH_BLOCK % K columns further on: no division per element (with a 64-bit one the kernel took 137 us for 4.4 million points
-// of 16 components)
-__device__ __forceinline__ void write_rows(const float* stage, int rows, int K, float* dst) {
-    const int drow = SPH_BLOCK / K, dcol = SPH_BLOCK - drow * K;
-    int r = (int)threadIdx.x / K, k = (int)threadIdx.x - r * K;
-    for (int j = threadIdx.x; j < rows * K; j += SPH_BLOCK) {
-        dst[j] = stage[r * (K + 1) + k];
-        r += drow; k += dcol;
-        if (k >= K) { k -= K; ++r; }
-    }
-}
-
+template <int L>
 __global__ void __launch_bounds__(SPH_BLOCK)
-sph_harm_kernel(int64_t N, int L, const float* __restrict__ xyz, SphConst cst, float* __restrict__ out) {
-    extern __shared__ float stage[];            // [SPH_BLOCK][K+1]
-    const int K = (L + 1) * (L + 1);
-    const int KP = K + 1;
-    const float* c = cst.c;
-    int64_t base = (int64_t)blockIdx.x * SPH_BLOCK;
-    int64_t i = base + threadIdx.x;
+sph_harm_kernel(int64_t N, const float* __restrict__ xyz, SphConst cst, float* __restrict__ out, bool vec) {
+    constexpr int K = (L + 1) * (L + 1);
+    __shared__ __align__(16) float stage[SPH_BLOCK * sph_pitch<K>];
+    const int64_t base = (int64_t)blockIdx.x * SPH_BLOCK;
+    const int64_t i = base + threadIdx.x;
     if (i < N) {
-        sph_eval(xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], L, c, stage + threadIdx.x * KP);
+        float o[K];
+        sph_eval(xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], L, cst.c, o);
+        put_row<K>(stage, o);
     }
     __syncthreads();
-    write_rows(stage, (int)(N - base < SPH_BLOCK ? N - base : SPH_BLOCK), K, out + base * K);
+    write_rows<K>(stage, (int)(N - base < SPH_BLOCK ? N - base : SPH_BLOCK), out + base * K, vec);
 }
 
 // out[f] = mean over the samples k of face f of the components of xyz[k] (0 for a face without samples): the two
 // steps sph_harm + per-face mean of the rows in one pass, without the (samples, K) array in between.  A thread walks
-// its face's samples in ascending order and adds each evaluation to its row in shared memory, so the result has the
+// its face's samples in ascending order and adds each evaluation to its sums, so the result has the
 // bits of the two-step path.
+template <int L>
 __global__ void __launch_bounds__(SPH_BLOCK)
-face_mean_sph_harm_kernel(int64_t Nf, int64_t NiK, int L, const float* __restrict__ xyz, const int32_t* __restrict__ cum,
-                          SphConst cst, float* __restrict__ out) {
-    extern __shared__ float stage[];            // [SPH_BLOCK][K+1] sums, then [SPH_BLOCK][K+1] one evaluation
-    const int K = (L + 1) * (L + 1);
-    const int KP = K + 1;
-    const float* c = cst.c;
-    float* acc = stage + threadIdx.x * KP;
-    float* one = stage + (SPH_BLOCK + threadIdx.x) * KP;
+face_mean_sph_harm_kernel(int64_t Nf, int64_t NiK, const float* __restrict__ xyz, const int32_t* __restrict__ cum,
+                          SphConst cst, float* __restrict__ out, bool vec) {
+    constexpr int K = (L + 1) * (L + 1);
+    __shared__ __align__(16) float stage[SPH_BLOCK * sph_pitch<K>];
     const int64_t base = (int64_t)blockIdx.x * SPH_BLOCK;
     const int64_t f = base + threadIdx.x;
     if (f < Nf) {
         int64_t k0 = f > 0 ? cum[f - 1] : 0, k1 = cum[f];
         if (k0 < 0) k0 = 0;
         if (k1 > NiK) k1 = NiK;
+        float acc[K];
+#pragma unroll
         for (int k = 0; k < K; ++k) acc[k] = 0.f;
         for (int64_t i = k0; i < k1; ++i) {
-            sph_eval(xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], L, c, one);
-            for (int k = 0; k < K; ++k) acc[k] += one[k];
+            float one[K];
+            sph_eval(xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], L, cst.c, one);
+#pragma unroll
+            for (int k = 0; k < K; ++k) acc[k] = __fadd_rn(acc[k], one[k]);        // not contracted with a component's last product
         }
         const float inv = k1 > k0 ? 1.f / (float)(k1 - k0) : 0.f;
+#pragma unroll
         for (int k = 0; k < K; ++k) acc[k] *= inv;
+        put_row<K>(stage, acc);
     }
     __syncthreads();
-    write_rows(stage, (int)(Nf - base < SPH_BLOCK ? Nf - base : SPH_BLOCK), K, out + base * K);
+    write_rows<K>(stage, (int)(Nf - base < SPH_BLOCK ? Nf - base : SPH_BLOCK), out + base * K, vec);
 }
 
 // The three-row vertex2facet filter of a layer, corners (3,K) @ weights (K,C), and its gradient corners^T @ gradFilter:
@@ -97,6 +86,8 @@ __global__ void corner_filter_bwd_kernel(int K, int C, const float* __restrict__
 
 using namespace pb;
 
+static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 extern "C" int pb200_corner_filter(int K, int C, const float* corners, const float* weights, float* filter, void* stream) {
     PB_REQUIRE(K > 0 && C > 0 && K <= (1 << 15) && C <= (1 << 15), PB200_EINVAL, "corner_filter: bad sizes");
     PB_REQUIRE(corners && weights && filter, PB200_EINVAL, "corner_filter: null pointer");
@@ -122,10 +113,8 @@ extern "C" int pb200_face_mean_sph_harm(int64_t Nf, int64_t NiK, int L, const fl
     if (Nf == 0) return PB200_OK;
     PB_REQUIRE(numInterior && out && (NiK == 0 || xyz), PB200_EINVAL, "face_mean_sph_harm: null pointer");
     static const SphConst cst = make_sph_const();
-    int K = (L + 1) * (L + 1);
-    size_t smem = sizeof(float) * 2 * SPH_BLOCK * (K + 1);
-    PB_LAUNCH("face_mean_sph_harm", face_mean_sph_harm_kernel, (unsigned)ceil_div(Nf, SPH_BLOCK), SPH_BLOCK, smem, stream, Nf,
-              NiK, L, xyz, numInterior, cst, out);
+    PB_DISPATCH_DEGREE(L, PB_LAUNCH("face_mean_sph_harm", face_mean_sph_harm_kernel<DEG>, (unsigned)ceil_div(Nf, SPH_BLOCK), SPH_BLOCK, 0,
+                                    stream, Nf, NiK, xyz, numInterior, cst, out, aligned16(out)));
     return PB200_OK;
 }
 
@@ -136,8 +125,7 @@ extern "C" int pb200_sph_harm_coeff(int64_t N, int L, const float* xyz, float* o
     if (N == 0) return PB200_OK;
     PB_REQUIRE(xyz && out, PB200_EINVAL, "sph_harm_coeff: null pointer");
     static const SphConst cst = make_sph_const();
-    int K = (L + 1) * (L + 1);
-    size_t smem = sizeof(float) * SPH_BLOCK * (K + 1);
-    PB_LAUNCH("sph_harm", sph_harm_kernel, (unsigned)ceil_div(N, SPH_BLOCK), SPH_BLOCK, smem, stream, N, L, xyz, cst, out);
+    PB_DISPATCH_DEGREE(L, PB_LAUNCH("sph_harm", sph_harm_kernel<DEG>, (unsigned)ceil_div(N, SPH_BLOCK), SPH_BLOCK, 0, stream, N, xyz, cst,
+                                    out, aligned16(out)));
     return PB200_OK;
 }

@@ -93,4 +93,48 @@ __device__ __forceinline__ void sph_eval(float x, float y, float z, int L, const
     }
 }
 
+// The way of a block's components to memory, for the kernels that evaluate them (one thread per row of K).  What bounds those is
+// instructions, of the angles, divisions and sines before all, then the stores.  The degree is a constant of the kernel, so components
+// stay in registers, go to shared memory and on from there in 16-byte pieces (a run-time degree and single floats before): 4.4 million
+// points, degree 1 / 3 / 4 / 5: 60 / 98 / 131 / 162 -> 50 / 70 / 84 / 110 us; means of 4.4 million points over 1.76 M faces, degree 3 / 4: 164 / 250
+// -> 111 / 133 us.  Same operations per component, same bits.
+constexpr int SPH_BLOCK = 128;
+
+// Floats of a row in shared memory: rows of whole quads are an odd number of quads apart, others, which have an odd length, follow one
+// another; either way neighbouring threads' rows start in other banks.
+template <int K> constexpr int sph_pitch = K % 4 == 0 ? 4 * (K / 4 | 1) : K;
+
+template <int K>
+__device__ __forceinline__ void put_row(float* stage, const float (&o)[K]) {
+    float* const row = stage + threadIdx.x * sph_pitch<K>;
+    if (K % 4 == 0) {
+#pragma unroll
+        for (int k = 0; k + 3 < K; k += 4) *reinterpret_cast<float4*>(row + k) = make_float4(o[k], o[k + 1], o[k + 2], o[k + 3]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < K; ++k) row[k] = o[k];
+    }
+}
+
+// the block's rows to consecutive addresses, from a multiple of SPH_BLOCK rows on; vec: out is 16-byte aligned
+template <int K>
+__device__ __forceinline__ void write_rows(const float* stage, int rows, float* dst, bool vec) {
+    constexpr int P = sph_pitch<K>;
+    auto at = [](int j) { return P == K ? j : j / K * P + j % K; };
+    const int n = rows * K, quads = vec ? n / 4 : 0;
+    for (int q = threadIdx.x; q < quads; q += SPH_BLOCK)
+        reinterpret_cast<float4*>(dst)[q] = *reinterpret_cast<const float4*>(stage + at(4 * q));
+    for (int j = 4 * quads + threadIdx.x; j < n; j += SPH_BLOCK) dst[j] = stage[at(j)];
+}
+
+#define PB_DISPATCH_DEGREE(L, ...)                              \
+    switch (L) {                                                \
+        case 0: { constexpr int DEG = 0; __VA_ARGS__; } break;  \
+        case 1: { constexpr int DEG = 1; __VA_ARGS__; } break;  \
+        case 2: { constexpr int DEG = 2; __VA_ARGS__; } break;  \
+        case 3: { constexpr int DEG = 3; __VA_ARGS__; } break;  \
+        case 4: { constexpr int DEG = 4; __VA_ARGS__; } break;  \
+        default: { constexpr int DEG = 5; __VA_ARGS__; } break; \
+    }
+
 }  // namespace pb

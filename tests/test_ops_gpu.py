@@ -557,3 +557,22 @@ def test_error_behaviour_of_the_shared_rows_entries(mods):
     assert _lib.query("pb200_padded_row_floats", 25) == 28 and _lib.query("pb200_padded_row_floats", 16) == 16
     # nothing of the above has left the device in a bad state
     assert torch.isfinite(one_sample_forward(x, w, b)).all()
+
+
+@pytest.mark.parametrize("L", range(6))
+@pytest.mark.parametrize("N", [1, 127, 128, 129, 1000])
+def test_sph_harm_rows_at_any_address(L, N):
+    """Rows leave in 16-byte pieces where the result allows it: the same values at an address that does not, nothing behind the last
+    row, and the oracle's components (2e-6 absolute, the fp32 angles' rounding in components of size one)."""
+    from oracle import mesh_oracle as mo
+    from picassoplus_b200 import _lib
+    K = (L + 1) ** 2
+    xyz = torch.randn(N, 3, generator=torch.Generator().manual_seed(N + L))
+    x, rows = xyz.cuda(), []
+    for shift in (0, 1):
+        buf = torch.full((N * K + 8,), 7.0, device="cuda")
+        _lib.call("pb200_sph_harm_coeff", N, L, x.data_ptr(), buf[shift:].data_ptr(), torch.cuda.current_stream().cuda_stream)
+        rows.append(buf[shift:shift + N * K].view(N, K))
+        assert (buf[:shift] == 7).all() and (buf[shift + N * K:] == 7).all()
+    assert torch.equal(*rows)
+    assert max_abs(rows[0], mo.sph_harm_coeff(L, xyz)) <= 2e-6
