@@ -62,7 +62,8 @@ f2v_fwd_face_kernel(int64_t Nf, int CV, int K, const float* __restrict__ coeff, 
 // The same register-blocked, for K <= 32: a face's channels lie on LPF lanes (float4 each; LPF = 4, 8, 16, 32, chunks of 128
 // channels behind that), a warp has 32 / LPF faces side by side, and a filter row read from shared memory is used for all FB such
 // passes of the warp.  The coefficient rows of the next tile arrive by 4-byte asynchronous copies while this one is
-// computed.  (The kernel above took 389 us for 1 758 000 faces of 64 channels, K = 16, bound by its shared-memory reads.)
+// computed.  (The kernel above took 389 us for 1 758 000 faces of 64 channels, K = 16, bound by its shared-memory reads; this one takes
+// 183.  Measured and left: packed multiply-adds with the coefficients paired in registers, 202, or stored in pairs, 224.)
 __device__ __forceinline__ void cp_async4(void* dst_smem, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src)
                  : "memory");
