@@ -217,3 +217,22 @@ def test_bad_arguments(device):
     # the library still works afterwards
     outs = dm().simplify(c["vertex"], c["face"], c["geometry"], c["nv_cum"], c["mf_cum"], c["remove"], True, 5.0)
     assert int(outs[5].sum()) < c["vertex"].shape[0]
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("shape", ["plane", "crease", "tilted", "line"])
+def test_quadrics_of_every_rank(shape, axis, device):
+    """Systems whose columns have no pivot, in every place: planes and folds across each axis, a plane across none, a mesh squeezed to a
+    line (zero normals).  Bit for bit the sequential restatement, costs included."""
+    v, f = planar_grid(24)
+    if shape == "crease":
+        v[:, 2] = np.abs(v[:, 0] - 0.5)
+    elif shape == "tilted":
+        v[:, 2] = np.float32(0.3) * v[:, 0] + np.float32(0.7) * v[:, 1]
+    elif shape == "line":
+        v[:, 1] = 0
+    v = np.ascontiguousarray(np.roll(v, axis, axis=1))
+    geo = c_oracle.triangle_geometry(v, f)
+    arrs = [v, f, geo, np.array([v.shape[0]], np.int32), np.array([f.shape[0]], np.int32), np.array([v.shape[0] // 2], np.int32)]
+    for weight in (0.0, 5.0):
+        check_against_oracle(device, arrs, True, weight)
