@@ -108,7 +108,8 @@ int pb200_build_vertex_csr(int64_t Nf, int64_t NvIn, int64_t NvOut, const int32_
 /* ---- vertex2facet -------------------------------------------------------------------
  * output[f, c*r+m] = sum_{k<3} filter[k,c,m] * input[face[f,k], c]
  * Replaces vertex2facetConv3dLauncher (mesh_conv3d_gpu.cu:176-195,261-266; binding
- * mesh_conv3d.cpp:123-152).  input (Nv,C), filter (3,C,r), face (Nf,3), output (Nf,C*r). */
+ * mesh_conv3d.cpp:123-152).  input (Nv,C), filter (3,C,r), face (Nf,3), output (Nf,C*r).
+ * A corner outside [0,Nv) is not read and contributes nothing. */
 int pb200_vertex2facet_forward(int64_t Nf, int64_t Nv, int C, int r, const float* input,
                                const float* filter, const int32_t* face, float* output, void* stream);
 

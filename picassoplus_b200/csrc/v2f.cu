@@ -18,9 +18,10 @@ constexpr int V2F_BWD_BATCH = 6, V2F_BWD_BLOCKS = 3;
 // (every vertex row is shared by ~6 faces; two faces in a row mostly share an edge).  What bounds it is the latency of index
 // and row loads: the next pair's indices are asked for before this pair's six rows are used (one face at a time, eight blocks
 // per SM: 172 us for 1.76 M faces of 64 channels, now 122, copy floor 110; 7.4 M faces of 128 channels 1.51 ms, now 1.05).
+// A corner outside the vertices is not read and contributes nothing: forward passes run on indices that nothing has checked yet.
 template <int TL>
 __global__ void __launch_bounds__(256, 4)
-v2f_fwd_vec_kernel(int64_t Nf, int CV, const int32_t* __restrict__ face, const float4* __restrict__ in,
+v2f_fwd_vec_kernel(int64_t Nf, uint32_t Nv, int CV, const int32_t* __restrict__ face, const float4* __restrict__ in,
                    const float4* __restrict__ filt, float4* __restrict__ out) {
     const int lane = threadIdx.x % TL;
     const int team = threadIdx.x / TL;
@@ -31,12 +32,29 @@ v2f_fwd_vec_kernel(int64_t Nf, int CV, const int32_t* __restrict__ face, const f
     const int64_t step = 2 * (int64_t)gridDim.x * teams;
     int64_t f = 2 * ((int64_t)blockIdx.x * teams + team);
     int n[6];
-    auto indices = [&](int64_t at) {                           // past the end: vertex 0, read and not used
+    auto indices = [&](int64_t at) {                           // past the end: no vertex
 #pragma unroll
-        for (int j = 0; j < 6; ++j) n[j] = 3 * at + j < 3 * Nf ? __ldg(face + 3 * at + j) : 0;
+        for (int j = 0; j < 6; ++j) n[j] = 3 * at + j < 3 * Nf ? __ldg(face + 3 * at + j) : -1;
     };
     if (f < Nf) indices(f);
     for (; f < Nf; f += step) {
+        bool all = true;                                       // the team's faces: uniform among its threads
+#pragma unroll
+        for (int j = 0; j < 6; ++j) all = all && (uint32_t)n[j] < Nv;
+        if (!all) {                                            // the last face of an odd number, a bad index
+#pragma unroll 1
+            for (int64_t g = f; g < Nf && g < f + 2; ++g) {
+                float4 o = zero4();
+#pragma unroll 1
+                for (int k = 0; k < 3; ++k) {
+                    const int v = __ldg(face + 3 * g + k);
+                    if ((uint32_t)v < Nv) fma4(o, ldg4(filt + (int64_t)k * CV + cg), ldg4(in + (int64_t)v * CV + cg));
+                }
+                __stcs(out + g * CV + cg, o);
+            }
+            indices(f + step);
+            continue;
+        }
         float4 x[6];
 #pragma unroll
         for (int j = 0; j < 6; ++j) x[j] = ldg4(in + (int64_t)n[j] * CV + cg);
@@ -47,13 +65,13 @@ v2f_fwd_vec_kernel(int64_t Nf, int CV, const int32_t* __restrict__ face, const f
             fma4(o, f0, x[3 * u]);      // same k-ascending fused-multiply-add chain as the reference
             fma4(o, f1, x[3 * u + 1]);
             fma4(o, f2, x[3 * u + 2]);
-            if (f + u < Nf) __stcs(out + (f + u) * CV + cg, o);
+            __stcs(out + (f + u) * CV + cg, o);
         }
     }
 }
 
 // ---------------------------------------------------------------------- forward, generic
-__global__ void v2f_fwd_generic_kernel(int64_t Nf, int C, int r, const int32_t* __restrict__ face,
+__global__ void v2f_fwd_generic_kernel(int64_t Nf, uint32_t Nv, int C, int r, const int32_t* __restrict__ face,
                                        const float* __restrict__ in, const float* __restrict__ filt,
                                        float* __restrict__ out) {
     const int Cr = C * r;
@@ -65,8 +83,10 @@ __global__ void v2f_fwd_generic_kernel(int64_t Nf, int C, int r, const int32_t* 
         int c = co / r;
         float acc = 0.f;
 #pragma unroll
-        for (int k = 0; k < 3; ++k)
-            acc = fmaf(__ldg(filt + k * Cr + co), __ldg(in + (int64_t)face[3 * f + k] * C + c), acc);
+        for (int k = 0; k < 3; ++k) {
+            const int v = face[3 * f + k];
+            if ((uint32_t)v < Nv) acc = fmaf(__ldg(filt + k * Cr + co), __ldg(in + (int64_t)v * C + c), acc);
+        }
         out[i] = acc;
     }
 }
@@ -207,15 +227,16 @@ int pb200_vertex2facet_forward(int64_t Nf, int64_t Nv, int C, int r, const float
     PB_REQUIRE(Nf >= 0 && Nv >= 0 && C > 0 && r > 0, PB200_EINVAL, "vertex2facet_forward: bad sizes");
     if (Nf == 0) return PB200_OK;
     PB_REQUIRE(input && filter && face && output, PB200_EINVAL, "vertex2facet_forward: null pointer");
+    const uint32_t vertices = Nv < (1LL << 31) ? (uint32_t)Nv : 1u << 31;         // indices are 32-bit
     if (vec_ok(C, r) && aligned16(input) && aligned16(filter) && aligned16(output)) {
         int CV = C / 4;
         TeamGeom g = team_geom(CV);
         dim3 grid(persistent_blocks(ceil_div(Nf, 2), g.teams, 4), g.chunks);
-        PB_DISPATCH_TL(g.TL, PB_LAUNCH("v2f_fwd", v2f_fwd_vec_kernel<TL>, grid, 256, 0, stream, Nf, CV, face,
-                                       (const float4*)input, (const float4*)filter, (float4*)output));
+        PB_DISPATCH_TL(g.TL, PB_LAUNCH("v2f_fwd", v2f_fwd_vec_kernel<TL>, grid, 256, 0, stream, Nf, vertices, CV,
+                                       face, (const float4*)input, (const float4*)filter, (float4*)output));
     } else {
         int grid = persistent_blocks(Nf * C * r, 256, 16);
-        PB_LAUNCH("v2f_fwd_generic", v2f_fwd_generic_kernel, grid, 256, 0, stream, Nf, C, r, face, input, filter, output);
+        PB_LAUNCH("v2f_fwd_generic", v2f_fwd_generic_kernel, grid, 256, 0, stream, Nf, vertices, C, r, face, input, filter, output);
     }
     return PB200_OK;
 }

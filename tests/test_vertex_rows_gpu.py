@@ -91,3 +91,45 @@ def test_layers_where_the_gather_leaves_the_product(C, cout, rows, train):
     whole = layer(0, rows)
     with torch.no_grad():
         assert torch.equal(whole, torch.cat([layer(0, half), layer(half, rows)]))
+
+
+BAD = [-1, -2 ** 31, 2 ** 31 - 1]                  # and the number of vertices
+
+
+@pytest.mark.parametrize("C,r", [(4, 1), (12, 1), (64, 1), (132, 1), (5, 1), (8, 2)])
+@pytest.mark.parametrize("nf", [1, 2, 7, 5001])
+def test_corner_outside_the_vertices(nf, C, r):
+    """It contributes nothing to vertex2facet, not even its product with an infinite filter value."""
+    g = torch.Generator(device="cuda").manual_seed(nf + C)
+    nv = 60
+    x, w = torch.randn(nv, C, device="cuda", generator=g), torch.randn(3, C, r, device="cuda", generator=g)
+    face = torch.randint(nv, (nf, 3), device="cuda", generator=g).int()
+    for i, bad in enumerate(BAD + [nv]):
+        face[i % nf, i % 3] = bad
+    w[0, 0, 0] = float("inf")                       # of a corner that the first face does not have
+    good = (face >= 0) & (face < nv)
+    picked = x.double()[face.long().clamp(0, nv - 1)].repeat_interleave(r, 2)                    # (nf, 3, C * r)
+    want = torch.where(good[:, :, None], picked * w.double().view(1, 3, C * r), 0.0).sum(1)
+    out = conv3d.vertex2facet_forward(x, w, face).double()
+    assert bool(out[0].isfinite().all()) and torch.equal(out.isfinite(), want.isfinite())
+    # three products of unit size, each rounded once
+    assert rel_err(out.nan_to_num(0, 0, 0), want.nan_to_num(0, 0, 0)) <= 1e-6
+
+
+@pytest.mark.parametrize("C,cout", [(8, 24), (64, 136)])
+def test_layer_over_a_corner_outside_the_vertices(C, cout):
+    """The vertex2facet layer tolerates one forward at any size, under autograd or not, with the same result; its backward pass refuses it."""
+    from picassoplus_b200.mesh.layers import V2FConv3d
+    g = torch.Generator(device="cuda").manual_seed(C)
+    rows, half, nv = 100003, 50000, 4000
+    layer, x = V2FConv3d(C, cout, 2).cuda().eval(), torch.randn(nv, C, device="cuda", generator=g).requires_grad_()
+    face = torch.randint(nv, (rows, 3), device="cuda", generator=g).int()
+    for i, bad in enumerate(BAD + [nv]):
+        face[i::20000, i % 3] = bad
+    with torch.no_grad():
+        want = torch.cat([layer(x, f.contiguous()) for f in (face[:half], face[half:])])         # gathered inside the product
+        assert torch.equal(layer(x, face), want)
+    out = layer(x, face)
+    assert rel_err(out, want) <= 1e-5               # normalised by a kernel of its own
+    with pytest.raises(RuntimeError, match="outside"):
+        torch.autograd.grad(out, [x], torch.ones_like(out))
