@@ -293,6 +293,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
                     tile_g2s(dst + (size_t)(KST + ks) * KTILE_BYTES, &rows_map, ks * 32 + 16, (int)f0, &raw_full[gb]);
                 }
             }
+            // The commits behind the last accumulator are waited for by nobody else, and in a pair they arrive in both CTAs: none leaves
+            // its shared memory to another block while one is on its way.  A buffer that was never used is free from the start.
+            for (int i = 0; i < p.gbufs && alive; ++i, ++icount)
+                alive = mbar_wait(&g_empty[icount % p.gbufs], (icount / p.gbufs & 1u) ^ 1u, abort_flag);
             if (!alive) {                                         // let copies in flight land before shared memory is released
                 const long long t0 = clock64();
                 while (clock64() - t0 < 2000000) { }
@@ -316,6 +320,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
                         bulk_g2s(wst + (size_t)s * wstage_bytes + (size_t)i * w_bytes, src + (size_t)i * NB * w_bytes, w_bytes, &w_full[s]);
                     if (++s == S) { s = 0; ph ^= 1u; }
                 }
+            }
+            for (int i = 0; i < S && alive; ++i) {                // the last commits of every stage, as above
+                alive = mbar_wait(&w_empty[s], ph ^ 1u, abort_flag);
+                if (++s == S) { s = 0; ph ^= 1u; }
             }
             if (!alive) {                                         // let copies in flight land before shared memory is released
                 const long long t0 = clock64();
@@ -391,7 +399,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
     __syncwarp();
     tc_fence_before();
     __syncthreads();
-    if constexpr (PAIR) cluster_sync();                           // nothing of this CTA is used by its peer any more
+    if constexpr (PAIR) cluster_sync();                           // both have drained their barriers: nothing of this CTA is used any more
     tc_fence_after();
     if (warp == EWARPS) {
         if constexpr (PAIR) tmem_dealloc_pair(tmem_base, 512);
