@@ -92,6 +92,14 @@ __global__ void v2f_fwd_generic_kernel(int64_t Nf, uint32_t Nv, int C, int r, co
 }
 
 // ------------------------------------------------------------------ backward, vectorised
+__device__ __forceinline__ bool finite4(const float4& a) { return isfinite(a.x) && isfinite(a.y) && isfinite(a.z) && isfinite(a.w); }
+__device__ __forceinline__ void take_where_infinite(float4& a, const float4& b) {
+    if (!isfinite(a.x)) a.x = b.x;
+    if (!isfinite(a.y)) a.y = b.y;
+    if (!isfinite(a.z)) a.z = b.z;
+    if (!isfinite(a.w)) a.w = b.w;
+}
+
 // A team owns one vertex v: it walks the CSR row of v in ascending (face, corner) order and sums the gradOutput rows of its
 // corners by the corner's number k in the face, s[k] = sum over (f, k) of gradOutput[f]; then
 //     gradInput[v]   = sum_k s[k] * filter[k]        (fixed order -> deterministic)
@@ -137,7 +145,31 @@ v2f_bwd_vec_kernel(int64_t Nv, int CV, const int32_t* __restrict__ rowptr, const
         fma2(gf0, s0, x); fma2(gf1, s1, x); fma2(gf2, s2, x);
         if (active) gin[walk.v * CV + cg] = unpair4(acc);
     }
-    red[0][threadIdx.x] = unpair4(gf0); red[1][threadIdx.x] = unpair4(gf1); red[2][threadIdx.x] = unpair4(gf2);
+    float4 r0 = unpair4(gf0), r1 = unpair4(gf1), r2 = unpair4(gf2);
+    // The loop above also multiplies the empty sums of corner numbers that a vertex does not have, which is right for finite factors.
+    // With an infinite filter value, or where a sum came out infinite, a thread does its channels again, corner by corner.  (Keeping
+    // note in the loop of the corner numbers that occur cost every call 15 %: 245 -> 286 us, 2.14 -> 2.48 ms.)
+    const float4 w0 = unpair4(f0), w1 = unpair4(f1), w2 = unpair4(f2);
+    const bool filters = finite4(w0) && finite4(w1) && finite4(w2), sums = finite4(r0) && finite4(r1) && finite4(r2);
+    if (active && !(filters && sums)) {
+        float4 q0 = zero4(), q1 = zero4(), q2 = zero4();
+#pragma unroll 1
+        for (int64_t v = (int64_t)blockIdx.x * teams + team; v < Nv; v += (int64_t)gridDim.x * teams) {
+            const int end = __ldg(rowptr + v + 1);
+            float4 acc = zero4();
+#pragma unroll 1
+            for (int e = __ldg(rowptr + v); e < end; ++e) {
+                const int ent = __ldg(entries + e), k = ent & 3;
+                const float4 g = ldg4(gout + (int64_t)(ent >> 2) * CV + cg);
+                fma4(acc, g, k == 0 ? w0 : k == 1 ? w1 : w2);
+                const float4 t = mul4(g, ldg4(in + v * CV + cg));
+                if (k == 0) add4(q0, t); else if (k == 1) add4(q1, t); else add4(q2, t);
+            }
+            if (!filters) gin[v * CV + cg] = acc;
+        }
+        take_where_infinite(r0, q0); take_where_infinite(r1, q1); take_where_infinite(r2, q2);
+    }
+    red[0][threadIdx.x] = r0; red[1][threadIdx.x] = r1; red[2][threadIdx.x] = r2;
     __syncthreads();
     if (team == 0 && active) {
         float4 s0 = zero4(), s1 = zero4(), s2 = zero4();

@@ -133,3 +133,25 @@ def test_layer_over_a_corner_outside_the_vertices(C, cout):
     assert rel_err(out, want) <= 1e-5               # normalised by a kernel of its own
     with pytest.raises(RuntimeError, match="outside"):
         torch.autograd.grad(out, [x], torch.ones_like(out))
+
+
+@pytest.mark.parametrize("C", [4, 8, 64, 100, 132, 6])
+def test_rows_that_take_no_part(C):
+    """An infinite row of a vertex without faces, or in the corner numbers that a vertex is not, stays out of the filter gradient, and an
+    infinite filter value out of the input gradient of the vertices that it does not meet."""
+    inf, nan = float("inf"), float("nan")
+    g = torch.Generator(device="cuda").manual_seed(C)
+    # 0: no face; 1: corner 0 of every face and nothing else; 2 to 9: corners 1 and 2
+    face = torch.randint(2, 10, (40, 3), device="cuda", generator=g).int()
+    face[:, 0] = 1
+    x, w = torch.randn(10, C, device="cuda", generator=g), torch.randn(3, C, 1, device="cuda", generator=g)
+    go = torch.randn(40, C, device="cuda", generator=g)
+    x[0], x[1, 0] = nan, inf
+    w[0, 1], w[2, 2] = inf, nan
+    gin, gw = conv3d.vertex2facet_backward(go, x, w, face)
+    assert bool((gin[0] == 0).all())                                              # no face
+    assert bool(gin[2:, 1].isfinite().all()) and bool(gin[1, 2].isfinite())       # filters of corners that these vertices are not
+    assert not bool(gin[1, 1].isfinite()) and bool(gin[face[0, 2].long(), 2].isnan())
+    want = (go.double()[:, None] * x.double()[face.long()]).sum(0)                # (3, C)
+    assert not bool(want[0, 0].isfinite()) and bool(gw[1:, 0].isfinite().all()) and not bool(gw[0, 0].isfinite())
+    assert rel_err(gw[:, 1:, 0], want[:, 1:]) <= 5e-6
