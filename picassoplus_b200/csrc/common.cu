@@ -111,9 +111,9 @@ reduce_partials_sliced_kernel(const float* __restrict__ partial, int nparts, int
     }
 }
 
-int reduce_partials(const float* partial, int nparts, int64_t n, float* out, cudaStream_t stream) {
+int reduce_partials(const float* partial, int nparts, int64_t n, float* out, cudaStream_t stream, int sliced_from) {
     if (n <= 0) return PB200_OK;
-    if (nparts >= 256) {
+    if (nparts >= sliced_from) {
         PB_LAUNCH("reduce_partials", reduce_partials_sliced_kernel, (unsigned)ceil_div(n, RP_WIDTH), dim3(RP_WIDTH, RP_SLICES), 0, stream,
                   partial, nparts, n, out);
         return PB200_OK;

@@ -759,7 +759,7 @@ int pb200_facet2vertex_backward(int64_t Nf, int64_t NvIn, int64_t NvOut, int C, 
                 PB_CUDA(cudaFuncSetAttribute(f2v_bwd_lane_kernel<P, LPF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemb));
                 PB_LAUNCH("f2v_bwd", (f2v_bwd_lane_kernel<P, LPF>), dim3((unsigned)gx, chunks), 32 * F2VL_WARPS, smemb, stream, Nf, C, K,
                           face, vtMap, nfCount, coeff, input, filter, gradOutput, gradInput, partial);
-                return reduce_partials(partial, (int)gx, (int64_t)K * Cr, gradFilter, stream);
+                return reduce_partials(partial, (int)gx, (int64_t)K * Cr, gradFilter, stream, FEW_PARTIALS);
             };
             auto width = [&](auto pairs) {
                 constexpr int NC = F2VL_NC<decltype(pairs)::value>;

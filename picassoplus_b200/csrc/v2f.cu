@@ -309,7 +309,7 @@ int pb200_vertex2facet_backward(int64_t Nf, int64_t Nv, int C, int r, const floa
         PB_DISPATCH_TL(g.TL, PB_LAUNCH("v2f_bwd", v2f_bwd_vec_kernel<TL>, grid, 256, 0, stream, Nv, CV, rowptr,
                                        entries, (const float4*)gradOutput, (const float4*)input,
                                        (const float4*)filter, (float4*)gradInput, (float4*)partial));
-        return reduce_partials(partial, gx, 3 * Cr, gradFilter, stream);
+        return reduce_partials(partial, gx, 3 * Cr, gradFilter, stream, FEW_PARTIALS);
     }
     // generic path (any C, r): plan for the non-vector layout even if only alignment failed
     V2FBwdPlan q = p;
