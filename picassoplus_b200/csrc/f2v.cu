@@ -299,14 +299,14 @@ f2v_bwd_tile_kernel(int64_t Nf, int CV, int K, const int32_t* __restrict__ face,
 // K <= 32: a lane keeps NC channels for the whole kernel, with their K filter values and K filter-gradient sums in registers, and
 // walks faces: the only operands of the 2 K multiply-adds of a face and channel that come out of shared memory are the K coefficients,
 // read once for both sums and broadcast to the warp.  Coefficients, filter and sums go in pairs (k, k + 1), so that the products are
-// packed (fma.rn.f32x2) without an operand kept twice.  A face's channels lie on LPF lanes (4, 8, 16, 32; chunks behind that on
-// blockIdx.y), a warp has FPW = 32 / LPF faces side by side and four such passes per stage.  Warps share nothing: each has a ring of
+// packed (fma.rn.f32x2) without an operand kept twice.  A face's channels lie on LPF lanes (4, 8, 16, 32; chunks of one width
+// behind that on blockIdx.y), a warp has FPW = 32 / LPF faces side by side and four such passes per stage.  Warps share nothing: each has a ring of
 // stages of its own (three gradOutput rows, the input row and the coefficients of every face) that asynchronous copies fill, and
 // resolves the index chain face -> vtMap -> nfCount one hop per stage ahead of them.
 // What bounds it: instructions (126 per warp and face at 16 coefficients, 64 of them multiply-adds) with 8 to 12 warps per SM.  A kernel
 // that read filter, coefficients and products from shared memory for every step (register blocks of 4 faces, three block barriers per
 // tile) took, per call with a cold L2: 879 000 faces, 64 channels, K = 16 247 us (now 148, copy floor 98); 464 000 faces, 128 channels,
-// K = 25 308 (257, floor 101); 879 000 faces, 48 channels, K = 9 226 (165), 32 channels, K = 25 200 (136), 16 channels, K = 16 118 (60).
+// K = 25 308 (248, floor 101); 879 000 faces, 48 channels, K = 9 226 (136), 32 channels, K = 25 200 (136), 16 channels, K = 16 118 (60).
 template <int BYTES>
 __device__ __forceinline__ void cp_async(void* dst_smem, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src), "n"(BYTES)
@@ -338,7 +338,7 @@ template <int P, int LPF> struct F2VLStage {
 
 template <int P, int LPF>
 __global__ void __launch_bounds__(32 * F2VL_WARPS, F2VL_BLOCKS<P>)
-f2v_bwd_lane_kernel(int64_t Nf, int C, int K, const int32_t* __restrict__ face, const int32_t* __restrict__ vtMap,
+f2v_bwd_lane_kernel(int64_t Nf, int C, int K, int width, const int32_t* __restrict__ face, const int32_t* __restrict__ vtMap,
                     const int32_t* __restrict__ nfCount, const float* __restrict__ coeff, const float* __restrict__ in,
                     const float* __restrict__ filt, const float* __restrict__ gout, float* __restrict__ gin,
                     float* __restrict__ partial) {
@@ -349,8 +349,12 @@ f2v_bwd_lane_kernel(int64_t Nf, int C, int K, const int32_t* __restrict__ face, 
     using Vec = typename F2VLVec<NC>::type;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int l = lane % LPF, fs = lane / LPF;                 // channel pair, face among the warp's
-    const bool on = (blockIdx.y * LPF + l) * NC < C;
-    const int ch = on ? (blockIdx.y * LPF + l) * NC : 0;        // lanes without channels follow and store nothing
+    const int c0 = blockIdx.y * width, here = C - c0 < width ? C - c0 : width;       // channels of this block
+    const bool on = l * NC < here;
+    // Lanes without channels follow on zeros of their own: they copy nothing and store nothing.  (When they copied channel 0 as well, one
+    // address for several places of shared memory, the memory unit took the copies apart: 879 000 faces, 100 channels, 25 coefficients
+    // 615 us, now 473; 136 channels, 16 coefficients, with an even share per chunk besides, 1 050 and 534.)
+    const int ch = on ? c0 + l * NC : 0;
     Stage* ring = reinterpret_cast<Stage*>(f2vl_smem) + warp * D;
 
     uint64_t f2[NC][P], acc[NC][P];
@@ -363,8 +367,11 @@ f2v_bwd_lane_kernel(int64_t Nf, int C, int K, const int32_t* __restrict__ face, 
             f2[c][p] = pair2(lo, hi);
             acc[c][p] = 0;
         }
-    for (int s = 0; s < D; ++s)                                // columns K.. stay zero
+    for (int s = 0; s < D; ++s) {                              // columns K.. stay zero
         for (int i = lane; i < TF * CP; i += 32) ring[s].coef[i] = 0.f;
+        if (!on)
+            for (int i = 0; i < 4 * F2VL_PASSES; ++i) ring[s].row[i / 4][i % 4][lane] = Vec{};
+    }
     __syncwarp();
 
     const int64_t ntiles = (Nf + TF - 1) / TF;
@@ -392,7 +399,7 @@ f2v_bwd_lane_kernel(int64_t Nf, int C, int K, const int32_t* __restrict__ face, 
     // what is not.
     auto fetch = [&](Stage& s, int64_t tile, bool whole) {
         const int64_t f0 = tile * TF;
-        if (whole) {
+        if (whole && on) {
             const char* in_lane = reinterpret_cast<const char*>(in + (f0 + fs) * C + ch);
 #pragma unroll
             for (int p = 0; p < F2VL_PASSES; ++p) {
@@ -403,7 +410,7 @@ f2v_bwd_lane_kernel(int64_t Nf, int C, int K, const int32_t* __restrict__ face, 
                 cp_async<4 * NC>(&s.row[p][3][lane], in_lane);
                 in_lane += FPW * row_bytes;
             }
-        } else if (tile < ntiles) {
+        } else if (tile < ntiles && on) {
 #pragma unroll 1
             for (int p = 0; p < F2VL_PASSES; ++p) {
                 const int fl = p * FPW + fs;
@@ -548,12 +555,12 @@ f2v_bwd_lane_kernel(int64_t Nf, int C, int K, const int32_t* __restrict__ face, 
     __syncthreads();
     const float* flat = reinterpret_cast<const float*>(sums);
     for (int i = threadIdx.x; i < K * LPF * NC; i += blockDim.x) {
-        const int k = i / (LPF * NC), c = i % (LPF * NC), co = blockIdx.y * LPF * NC + c;
+        const int k = i / (LPF * NC), c = i % (LPF * NC);
         float t = 0.f;
         for (int v = 0; v < F2VL_WARPS; ++v)
 #pragma unroll
             for (int q = 0; q < FPW; ++q) t += flat[((v * 2 * P + k) * 32 + q * LPF) * NC + c];
-        if (co < C) partial[((int64_t)blockIdx.x * K + k) * C + co] = t;
+        if (c < here) partial[((int64_t)blockIdx.x * K + k) * C + c0 + c] = t;
     }
 }
 
@@ -749,7 +756,7 @@ int pb200_facet2vertex_backward(int64_t Nf, int64_t NvIn, int64_t NvOut, int C, 
         if (K <= 32) {
             auto run = [&](auto pairs, auto lpf) {
                 constexpr int P = decltype(pairs)::value, LPF = decltype(lpf)::value;
-                const int chunks = (int)ceil_div(C, F2VL_NC<P> * LPF);
+                const int chunks = (int)ceil_div(C, F2VL_NC<P> * LPF), width = (int)ceil_div(C, F2VL_NC<P> * chunks) * F2VL_NC<P>;
                 const size_t smemb = sizeof(F2VLStage<P, LPF>) * F2VL_STAGES * F2VL_WARPS;
                 const int fit = (int)(228 * 1024 / (smemb + 1024));                // blocks that an SM's shared memory holds
                 int64_t gx = (int64_t)(fit < F2VL_BLOCKS<P> ? fit : F2VL_BLOCKS<P>) * sm_count() / chunks;
@@ -757,7 +764,7 @@ int pb200_facet2vertex_backward(int64_t Nf, int64_t NvIn, int64_t NvOut, int C, 
                 if (gx > ceil_div(Nf, F2VL_WARPS * F2VL_FACES<LPF>)) gx = ceil_div(Nf, F2VL_WARPS * F2VL_FACES<LPF>);
                 if (gx > p.grid_x) gx = p.grid_x;
                 PB_CUDA(cudaFuncSetAttribute(f2v_bwd_lane_kernel<P, LPF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemb));
-                PB_LAUNCH("f2v_bwd", (f2v_bwd_lane_kernel<P, LPF>), dim3((unsigned)gx, chunks), 32 * F2VL_WARPS, smemb, stream, Nf, C, K,
+                PB_LAUNCH("f2v_bwd", (f2v_bwd_lane_kernel<P, LPF>), dim3((unsigned)gx, chunks), 32 * F2VL_WARPS, smemb, stream, Nf, C, K, width,
                           face, vtMap, nfCount, coeff, input, filter, gradOutput, gradInput, partial);
                 return reduce_partials(partial, (int)gx, (int64_t)K * Cr, gradFilter, stream, FEW_PARTIALS);
             };

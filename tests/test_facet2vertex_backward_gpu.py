@@ -11,7 +11,7 @@ from picassoplus_b200.topology import ptr, stream_ptr
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("C", [4, 16, 24, 32, 48, 64, 100, 128, 132, 256])
+@pytest.mark.parametrize("C", [4, 16, 24, 32, 48, 64, 100, 128, 132, 136, 200, 256])
 @pytest.mark.parametrize("nf,K", [(1, 1), (31, 9), (129, 4), (257, 16), (1025, 17), (3000, 25), (700, 32), (333, 36)])
 def test_facet2vertex_backward(nf, K, C):
     g = torch.Generator(device="cuda").manual_seed(nf * 1000 + C)
