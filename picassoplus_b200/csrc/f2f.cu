@@ -19,7 +19,11 @@ int backward_filter(int64_t Nf, int Cin, int Cout, int F, const float* gout, con
                     float* gfilter, void* ws, cudaStream_t stream);
 }  // namespace small
 namespace rgb {
-bool supported(int Cin, int Cout, int F, const float* bary);
+bool supported(int Cin, int F, const float* bary);
+bool forward_alone(int Cout, int F);
+bool gradient_alone(int Cout);
+bool layer_forward(int Cout);
+bool layer_gradient(int Cout);
 int forward(int64_t Nf, int Cout, int F, const float* input, const float* filter, const float* bary, const int32_t* cum, const float* bias,
             int relu, float* output, float* stats, int most, int* nparts, cudaStream_t stream);
 size_t workspace_bytes(int64_t Nf, int Cout, int F);
@@ -121,7 +125,7 @@ int pb200_facet2facet_forward(int64_t Nf, int64_t NiK, int Cin, int Cout, int F,
     PB_REQUIRE(workspace && workspace_bytes >= pb200_facet2facet_forward_workspace_bytes(Nf, NiK, Cin, Cout, F, precision),
                PB200_EWORKSPACE, "facet2facet_forward: workspace too small");
     if (use_small(Nf, Cin, Cout, F, precision)) {
-        if (rgb::supported(Cin, Cout, F, bary))
+        if (rgb::supported(Cin, F, bary) && rgb::forward_alone(Cout, F))
             return rgb::forward(Nf, Cout, F, input, filter, bary, numInterior, nullptr, 0, output, nullptr, 0, nullptr, stream);
         return small::forward(Nf, Cin, Cout, F, input, filter, bary, numInterior, output, stream);
     }
@@ -139,7 +143,7 @@ int pb200_facet2facet_layer_forward(int64_t Nf, int64_t NiK, int Cin, int Cout, 
                                     float* partial, int* nparts, int precision, void* workspace, size_t workspace_bytes, void* stream) {
     PB_REQUIRE(f2f_sizes_ok(Nf, NiK, Cin, Cout, F) && Nf > 0, PB200_EINVAL, "facet2facet_layer_forward: bad sizes (F must be in 1..50)");
     PB_REQUIRE(partial && nparts, PB200_EINVAL, "facet2facet_layer_forward: null pointer");
-    if (use_small(Nf, Cin, Cout, F, precision) && rgb::supported(Cin, Cout, F, bary)) {
+    if (use_small(Nf, Cin, Cout, F, precision) && rgb::supported(Cin, F, bary) && rgb::layer_forward(Cout)) {
         PB_REQUIRE(filter && numInterior && act && (NiK == 0 || (input && bary)), PB200_EINVAL, "facet2facet_layer_forward: null pointer");
         return rgb::forward(Nf, Cout, F, input, filter, bary, numInterior, bias, relu, act, partial, pb200_norm_parts(Nf, Cout), nparts,
                             (cudaStream_t)stream);
@@ -151,7 +155,7 @@ int pb200_facet2facet_layer_forward(int64_t Nf, int64_t NiK, int Cin, int Cout, 
 
 int pb200_facet2facet_layer_gradient_fused(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, const float* bary, int precision) {
     return Nf > 0 && f2f_sizes_ok(Nf, NiK, Cin, Cout, F) && use_small_gf(Nf, Cin, Cout, F, precision) &&
-                   rgb::supported(Cin, Cout, F, bary) ? 1 : 0;
+                   rgb::supported(Cin, F, bary) && rgb::layer_gradient(Cout) ? 1 : 0;
 }
 
 int pb200_facet2facet_layer_filter_gradient(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, const float* gradOutput, const float* act,
@@ -320,7 +324,7 @@ static int f2f_backward_impl(int64_t Nf, int64_t NiK, int Cin, int Cout, int F, 
         w += gin_ws(Cin, Cout, F, precision);
     }
     if (sf) {
-        int rc = rgb::supported(Cin, Cout, F, bary)
+        int rc = rgb::supported(Cin, F, bary) && rgb::gradient_alone(Cout)
                      ? rgb::backward_filter(Nf, Cout, F, gradOutput, nullptr, 0, nullptr, input, bary, numInterior, gradFilter, nullptr, w, stream)
                      : small::backward_filter(Nf, Cin, Cout, F, gradOutput, input, bary, numInterior, gradFilter, w, stream);
         if (rc) return rc;

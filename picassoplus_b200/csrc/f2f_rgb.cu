@@ -1,5 +1,5 @@
-// facet2facet for colours: three input channels and bases in whole quads (F = 4, 8, 12, 16; rows of 16-byte multiples), forward and
-// filter gradient, in fp32, with the layer around them.  f2f_small.cu has the formulas and serves the other sizes.
+// facet2facet for colours: three input channels and 4 or 16 bases (one or four quads, rows of 16-byte multiples), forward and filter
+// gradient, in fp32, with the layer around them.  f2f_small.cu has the formulas and serves the other sizes.
 //
 // A warp works by itself through batches of eight faces:
 //   * a lane makes the A values of one face and quad of bases, so that a sample's weights are read in whole sectors; the samples
@@ -11,10 +11,11 @@
 // activation is the gradient kernel's prologue: a lane is a channel, its factors and sums are registers.
 // What bounds it: instructions (about 100 per face and warp, 24 of them multiply-adds at 16 bases and 32 outputs) with 12 warps per SM.
 // 1 758 000 faces, 4.4 million samples, 16 bases, 32 outputs: forward 255 us with bias, ReLU and statistics (247 without, and 77 for
-// those, before), gradient 288 us with normalisation, ReLU and bias gradient (325 and 96); a layer's training step 1 064 -> 844 us,
-// with 64 outputs 1 700 -> 1 345, with 16 738 -> 613.  With 9 and 25 bases, whose rows have to be read in single floats, these kernels
-// are the slower ones (956 -> 1 019, 1 499 -> 2 362 us).  Measured and left: samples through shared memory by asynchronous copies (350, 384
-// us), five blocks per SM (spills: 490, 410), two outputs per lane at 32 outputs (348, 556).
+// those, before), gradient 288 us with normalisation, ReLU and bias gradient (325 and 96); a layer's training step 1 064 -> 826 us,
+// with 64 outputs 1 700 -> 1 330, with 16 738 -> 587.  Measured and left: 9 and 25 bases, whose rows have to be read in single floats
+// (956 -> 1 019, 1 499 -> 2 362 us); 8 and 12, whose rows leave quads of the warp idle (800 000 faces, 33 outputs, forward 97 -> 173 us and
+// 136 -> 173, gradient 136 -> 235 and 159 -> 237); samples through shared memory by asynchronous copies (350, 384 us), five blocks per SM
+// (spills: 490, 410), two outputs per lane at 32 outputs (348, 556).
 #include <type_traits>
 #include "common.cuh"
 #include "moments.cuh"
@@ -23,14 +24,14 @@ namespace pb {
 namespace rgb {
 
 constexpr int WARPS = 4, NT = 32 * WARPS;
-constexpr int C = 3, MAX_F = 16;
+constexpr int C = 3;
 constexpr int AHEAD = 4;                 // samples of a face that are loaded a batch ahead; further ones when their turn comes
 
 constexpr int BF = 8;                    // faces of a batch: what a warp makes rows of at once with four quads
 
 struct Params {
     int64_t Nf;
-    int F, Cout;
+    int Cout;
     int lpf;                             // lanes of a face: 16 (two faces side by side) or 32
     const float* in;
     const float* bary;
@@ -49,7 +50,7 @@ struct Params {
 // The A values of a warp's batches: lane = (face, quad of bases)
 template <int Q>
 struct Rows {
-    static constexpr int M4 = 4 * Q * C, AP = M4 | 4;         // floats of a row and its pitch
+    static constexpr int F = 4 * Q, M = F * C, AP = M | 4;    // bases, floats of a row and its pitch
     const Params& p;
     int step, fl, q;                                           // batches from one of the warp's to the next
     uint64_t b[AHEAD][2];                                      // the first samples of this batch's face: weights, channels
@@ -66,16 +67,16 @@ struct Rows {
     __device__ __forceinline__ void range(int64_t batch, int& a, int& e) const {
         const int64_t f = batch * BF + fl;
         a = e = 0;
-        if (fl < BF && f < p.Nf && 4 * q < p.F) {
+        if (fl < BF && f < p.Nf) {
             if (f > 0) a = __ldg(p.cum + f - 1);
             e = __ldg(p.cum + f);
         }
     }
     __device__ __forceinline__ void ask(int a, int e) {
-        const float* src = p.bary + (int64_t)a * p.F + 4 * q;
+        const float* src = p.bary + (int64_t)a * F + 4 * q;
         const float* in = p.in + (int64_t)a * C;
 #pragma unroll
-        for (int t = 0; t < AHEAD; ++t, src += p.F, in += C) {
+        for (int t = 0; t < AHEAD; ++t, src += F, in += C) {
             const bool on = a + t < e;
             b[t][0] = b[t][1] = 0;
 #pragma unroll
@@ -129,11 +130,10 @@ struct Rows {
 template <int Q, int NO>
 __global__ void __launch_bounds__(NT, 4 * Q * C * NO <= 48 ? 3 : 2) f2f_rgb_fwd_kernel(Params p) {
     using R = Rows<Q>;
-    constexpr int PAIRS = R::M4 / 2;
+    constexpr int F = R::F, PAIRS = R::M / 2;
     __shared__ __align__(16) float rows[WARPS][BF * R::AP];
     __shared__ norm::Moments red[WARPS * 2][32 * NO];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l = lane % p.lpf, fs = lane / p.lpf, fpw = 32 / p.lpf;
-    const int M = p.F * C;
     uint64_t w[NO][PAIRS];
     float bias[NO], shift[NO], s1[NO], s2[NO];
     int co[NO];
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(NT, 4 * Q * C * NO <= 48 ? 3 : 2) f2f_rgb_fwd_
     for (int o = 0; o < NO; ++o) {
         co[o] = (blockIdx.y * NO + o) * p.lpf + l;
         const bool on = co[o] < p.Cout;
-        auto value = [&](int m) { return on && m < M ? __ldg(p.filter + ((int64_t)co[o] * C + m % C) * p.F + m / C) : 0.f; };
+        auto value = [&](int m) { return on ? __ldg(p.filter + ((int64_t)co[o] * C + m % C) * F + m / C) : 0.f; };
 #pragma unroll
         for (int i = 0; i < PAIRS; ++i) w[o][i] = pair2(value(2 * i), value(2 * i + 1));
         bias[o] = on && p.bias ? __ldg(p.bias + co[o]) : 0.f;
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(NT, 4 * Q * C * NO <= 48 ? 3 : 2) f2f_rgb_fwd_
 template <int Q, int NO>
 __global__ void __launch_bounds__(NT, 4 * Q * C * NO <= 48 ? 3 : 2) f2f_rgb_gfilter_kernel(Params p) {
     using R = Rows<Q>;
-    constexpr int M4 = R::M4, PAIRS = M4 / 2;
+    constexpr int F = R::F, M = R::M, PAIRS = M / 2;
     __shared__ __align__(16) float rows[WARPS][BF * R::AP];
     constexpr int MS = 8;
     __shared__ float red[MS * NT * NO];
@@ -263,38 +263,48 @@ __global__ void __launch_bounds__(NT, 4 * Q * C * NO <= 48 ? 3 : 2) f2f_rgb_gfil
         }
     }
     // the sums of the warps, in order, MS values of (d, ci) at a time; the column sums are the value behind the last
-    float* const out = p.out + (int64_t)blockIdx.x * p.Cout * C * p.F;
-    const int M = p.F * C, width = NO * p.lpf, mine = (warp * fpw + fs) * width + l;
+    float* const out = p.out + (int64_t)blockIdx.x * p.Cout * M;
+    const int width = NO * p.lpf, mine = (warp * fpw + fs) * width + l;
 #pragma unroll
-    for (int m0 = 0; m0 <= M4; m0 += MS) {
+    for (int m0 = 0; m0 <= M; m0 += MS) {
         __syncthreads();
 #pragma unroll
         for (int j = 0; j < MS; ++j) {
             const int m = m0 + j;
-            if (m > M4) break;
+            if (m > M) break;
 #pragma unroll
             for (int o = 0; o < NO; ++o) {
                 float v = sum[o];
-                if (m < M4) { const float2 e = unpair2(acc[o][m < M4 ? m / 2 : 0]); v = m % 2 ? e.y : e.x; }
+                if (m < M) { const float2 e = unpair2(acc[o][m < M ? m / 2 : 0]); v = m % 2 ? e.y : e.x; }
                 red[j * NT * NO + mine + o * p.lpf] = v;
             }
         }
         __syncthreads();
         for (int i = threadIdx.x; i < MS * width; i += NT) {
             const int j = i / width, c = i - j * width, at = blockIdx.y * width + c, m = m0 + j;
-            if (at >= p.Cout || (m >= M && m != M4)) continue;
+            if (at >= p.Cout || m > M) continue;
             float t = red[j * NT * NO + c];
             for (int k = 1; k < WARPS * fpw; ++k) t += red[j * NT * NO + k * width + c];
-            if (m < M) out[((int64_t)at * C + m % C) * p.F + m / C] = t;
+            if (m < M) out[((int64_t)at * C + m % C) * F + m / C] = t;
             else if (p.sums) p.sums[(int64_t)blockIdx.x * p.Cout + at] = t;
         }
     }
 }
 
 // ---------------------------------------------------------------------------- host side
-bool supported(int Cin, int Cout, int F, const float* bary) {
-    return Cin == C && Cout >= 1 && F >= 4 && F <= MAX_F && F % 4 == 0 && (reinterpret_cast<uintptr_t>(bary) & 15) == 0;
+bool supported(int Cin, int F, const float* bary) {
+    return Cin == C && (F == 4 || F == 16) && (reinterpret_cast<uintptr_t>(bary) & 15) == 0;
 }
+// Where these kernels are the faster ones, over 4 096 to 1 000 000 faces and 1 to 400 outputs (f2f_small.cu -> these, 400 000 faces):
+//   the operator alone: forward with 16 bases and up to 16 outputs (55 -> 45 us; 24 outputs 64 -> 68; 4 bases 20 -> 31), gradient with 12 to 32
+//     outputs (4 bases 62 -> 56, 16 bases 95 -> 81; 40 outputs 73 -> 81 and 108 -> 134, 3 outputs and 16 bases 58 -> 62);
+//   the layer forward from 4 outputs on (8 outputs 95 -> 58; with less the statistics' few rows hold the grid down: 50 -> 71);
+//   the layer's gradients too, except where a second column of 64 outputs is nearly empty and f2f_small.cu reads rows in 16-byte
+//     pieces (80 outputs, 4 bases 262 -> 296; 75 outputs 361 -> 318, 128 341 -> 313).
+bool forward_alone(int Cout, int F) { return F == 16 && Cout <= 16; }
+bool gradient_alone(int Cout) { return Cout >= 12 && Cout <= 32; }
+bool layer_forward(int Cout) { return Cout >= 4; }
+bool layer_gradient(int Cout) { return Cout >= 4 && (Cout <= 64 || Cout > 100 || Cout % 4 != 0); }
 
 // Calls go(Q, NO): quads of a row, two outputs per lane where there are more than a warp's
 template <typename Go>
@@ -302,7 +312,7 @@ static int with_shape(int F, int Cout, Go&& go) {
     const std::integral_constant<int, 1> one{};
     const std::integral_constant<int, 2> two{};
     const std::integral_constant<int, 4> four{};
-    if (F <= 4) return Cout > 32 ? go(one, two) : go(one, one);
+    if (F == 4) return Cout > 32 ? go(one, two) : go(one, one);
     return Cout > 32 ? go(four, two) : go(four, one);
 }
 
@@ -316,7 +326,7 @@ static int blocks_per_sm(Kernel k) {
 int forward(int64_t Nf, int Cout, int F, const float* input, const float* filter, const float* bary, const int32_t* cum, const float* bias,
             int relu, float* output, float* stats, int most, int* nparts, cudaStream_t stream) {
     Params p = {};
-    p.Nf = Nf; p.F = F; p.Cout = Cout; p.lpf = Cout <= 16 ? 16 : 32;
+    p.Nf = Nf; p.Cout = Cout; p.lpf = Cout <= 16 ? 16 : 32;
     p.in = input; p.bary = bary; p.cum = cum; p.filter = filter; p.bias = bias; p.relu = relu; p.out = output; p.stats = stats;
     return with_shape(F, Cout, [&](auto q, auto no) {
         constexpr int Q = decltype(q)::value, NO = decltype(no)::value;
@@ -338,7 +348,7 @@ size_t workspace_bytes(int64_t Nf, int Cout, int F) {
 int backward_filter(int64_t Nf, int Cout, int F, const float* gout, const float* act, int relu, const pb200_norm_gradient* norm,
                     const float* input, const float* bary, const int32_t* cum, float* gfilter, float* gbias, void* ws, cudaStream_t stream) {
     Params p = {};
-    p.Nf = Nf; p.F = F; p.Cout = Cout; p.lpf = Cout <= 16 ? 16 : 32;
+    p.Nf = Nf; p.Cout = Cout; p.lpf = Cout <= 16 ? 16 : 32;
     p.in = input; p.bary = bary; p.cum = cum; p.gout = gout; p.act = act; p.relu = relu; p.out = (float*)ws;
     if (norm) p.norm = *norm;
     return with_shape(F, Cout, [&](auto q, auto no) {

@@ -10,7 +10,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("nf,cin,cout,F", [(4096, 3, 32, 16), (4097, 1, 4, 1), (4159, 2, 16, 9), (4223, 3, 33, 25), (4351, 4, 28, 32),
                                             (4353, 3, 48, 16), (5000, 3, 100, 9), (4500, 1, 130, 25), (4200, 3, 7, 7), (8193, 3, 64, 25),
-                                            (90000, 3, 32, 16)])
+                                            (90000, 3, 32, 16), (4099, 3, 16, 8), (4101, 3, 33, 8), (4096, 3, 32, 12), (4200, 3, 64, 12),
+                                            (4111, 3, 12, 4), (4111, 3, 11, 16), (4105, 3, 33, 16)])
 def test_small_inputs(nf, cin, cout, F):
     from picassoplus_b200.mesh.pi_modules import conv3d
     g = torch.Generator(device="cuda").manual_seed(nf + F)
