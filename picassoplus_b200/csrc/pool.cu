@@ -26,8 +26,8 @@ __device__ __forceinline__ void upd(float& best, int& arg, float v, int m) { if 
 __device__ __forceinline__ void set_zero(float& a) { a = 0.f; }
 __device__ __forceinline__ void set_zero(float4& a) { a = zero4(); }
 // x / c for a member count c: quotient by the reciprocal and one correction by its exact remainder (Markstein's division), rounded as
-// the division is (compared for every mantissa and the counts 1 to 12 288 and up to 2^24).  The values it is not for -- tiny, infinite
-// and NaN ones, counts that are none -- are divided.  A division takes some sixty instructions: it was what average pooling did.
+// the division is.  The values it is not for -- tiny, infinite and NaN ones, counts that are none -- are divided.  A division goes a long
+// way round for a numerator of zero, and every second value behind a ReLU is one.
 __device__ __forceinline__ float quot(float x, float c) {
     const float r = __frcp_rn(c), q = x * r;
     const uint32_t u = __float_as_uint(x) & 0x7fffffffu;       // 2^-60 <= |x| < infinity, or zero
@@ -35,6 +35,16 @@ __device__ __forceinline__ float quot(float x, float c) {
     return x / c;
 }
 __device__ __forceinline__ float4 quot(const float4& x, float c) { return make_float4(quot(x.x, c), quot(x.y, c), quot(x.z, c), quot(x.w, c)); }
+// for gradients, whose values are seldom zero: one branch for the four that are of the ordinary kind (490 000 vertices of 32 channels to a
+// quarter 24.2 -> 22.9 us)
+__device__ __forceinline__ float quot_of_gradient(float x, float c) { return quot(x, c); }
+__device__ __forceinline__ float4 quot_of_gradient(const float4& x, float c) {
+    auto plain = [](float v) { return (__float_as_uint(v) & 0x7fffffffu) - 0x21800000u < 0x5e000000u; };
+    if (!(plain(x.x) && plain(x.y) && plain(x.z) && plain(x.w) && c >= 1.f && c <= 16777216.f)) return quot(x, c);
+    const float r = __frcp_rn(c);
+    auto one = [&](float v) { const float q = v * r; return fmaf(fmaf(-q, c, v), r, q); };
+    return make_float4(one(x.x), one(x.y), one(x.z), one(x.w));
+}
 __device__ __forceinline__ void accum(float& a, float x) { a += x; }
 __device__ __forceinline__ void accum(float4& a, const float4& x) { add4(a, x); }
 
@@ -150,26 +160,33 @@ __device__ __forceinline__ float cluster_size(int m, const int32_t* __restrict__
     return (float)(__ldg(vtReplace + (rep < 0 ? -(int64_t)rep : m)) + 1);
 }
 
-__global__ void avg_pool_fwd_kernel(int64_t NvOut, int C, const float* __restrict__ in, const int32_t* __restrict__ vtReplace,
-                                    const int32_t* __restrict__ rowptr, const int32_t* __restrict__ members, float* __restrict__ out) {
-    const int64_t total = NvOut * C;
+template <int VEC>
+__global__ void avg_pool_fwd_kernel(int64_t NvIn, int64_t NvOut, int CVn, const float* __restrict__ in,
+                                    const int32_t* __restrict__ vtReplace, const int32_t* __restrict__ rowptr,
+                                    const int32_t* __restrict__ members, float* __restrict__ out) {
+    const int64_t total = NvOut * CVn;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t vo = i / C;
-        const int c = (int)(i - vo * C);
-        float acc = 0.f;
-        for (int e = rowptr[vo]; e < rowptr[vo + 1]; ++e) {
+        const int64_t vo = i / CVn;
+        const int c = (int)(i - vo * CVn);
+        const int beg = rowptr[vo], end = rowptr[vo + 1];
+        typename Vec<VEC>::T acc;
+        set_zero(acc);
+        for (int e = beg; e < end; ++e) {
             const int m = members[e];
-            acc += __ldg(in + (int64_t)m * C + c) / cluster_size(m, vtReplace);
+            accum(acc, quot(Vec<VEC>::ld(in, (int64_t)m * CVn + c), cluster_size(m, vtReplace)));
         }
-        out[i] = acc;
+        Vec<VEC>::st(out, i, acc);
     }
 }
 
-// The same for channels in quads: a team of TL lanes takes a coarse vertex, its members' rows come B at a time and its next cluster's
-// members are asked for meanwhile (row_walk.cuh).  Two levels of one scene (123 000 vertices of 64 channels, 30 800 of 128): 45 us
-// member after member with a division for every value, now 25, 43 with the divisions.  (Max pooling by teams: 223 us instead of 215
-// for three levels of 980 000 vertices, 14.1 instead of 14.5 for three of 41 000.)
+// The same for channels in quads where there are few of them: a team of TL lanes takes a coarse vertex, its members' rows come B at a
+// time and its next cluster's members are asked for meanwhile (row_walk.cuh).
 constexpr int POOL_BATCH = 4;                                  // most clusters have as many members
+// Quads of the result up to which the teams are the faster ones: a chain of loads per member then, memory and idle lanes of the teams
+// above.  Clusters of four, rows of half zeros, thread per quad -> teams: 10 000 vertices of 64 channels 5.2 -> 4.8 us, 41 000 of 32 8.2 -> 9.3,
+// 123 000 of 48 10 -> 14, 490 000 of 64 and 100 45.7 -> 53.2 and 67 -> 82; clusters of one, 100 000 of 100 27 -> 39; of ten, 41 000 of 32 16.4
+// -> 13.3, of 100 22.0 -> 23.6.  (The division for every value in place of quot: 41 000 of 32 18.6 us, 490 000 of 64 97.6.)
+constexpr int64_t POOL_TEAMS = 100000;
 template <int TL>
 __global__ void __launch_bounds__(256)
 avg_pool_fwd_team_kernel(int64_t NvOut, int CV, const float4* __restrict__ in, const int32_t* __restrict__ vtReplace,
@@ -213,7 +230,7 @@ __global__ void avg_pool_bwd_kernel(int64_t NvIn, int CVn, const float* __restri
             const int rep = vtReplace[v];
             const int64_t mapid = rep < 0 ? -(int64_t)rep : v;
             const float count = (float)(vtReplace[mapid] + 1);
-            r = quot(Vec<VEC>::ld(gout, (int64_t)vo * CVn + c), count);
+            r = quot_of_gradient(Vec<VEC>::ld(gout, (int64_t)vo * CVn + c), count);
         }
         Vec<VEC>::st(gin, i, r);
     }
@@ -332,13 +349,13 @@ int pb200_mesh_avg_pool_forward(int64_t NvIn, int64_t NvOut, int C, const float*
     PB_REQUIRE(rowptr && output && (NvIn == 0 || (input && members && vtReplace)), PB200_EINVAL,
                "mesh_avg_pool_forward: null pointer");
     const bool vec = C % 4 == 0 && aligned16(input) && aligned16(output);
-    if (vec) {
-        const TeamGeom g = team_geom(C / 4);
+    const int CVn = vec ? C / 4 : C;
+    if (vec && NvOut * CVn < POOL_TEAMS) {
+        const TeamGeom g = team_geom(CVn);
         PB_DISPATCH_TL(g.TL, PB_LAUNCH("mesh_avg_pool_fwd", avg_pool_fwd_team_kernel<TL>, dim3(persistent_blocks(NvOut, g.teams, 8), g.chunks), 256,
-                                       0, stream, NvOut, C / 4, (const float4*)input, vtReplace, rowptr, members, (float4*)output));
+                                       0, stream, NvOut, CVn, (const float4*)input, vtReplace, rowptr, members, (float4*)output));
     } else {
-        PB_LAUNCH("mesh_avg_pool_fwd", avg_pool_fwd_kernel, persistent_blocks(NvOut * C, 256, 16), 256, 0, stream, NvOut, C, input, vtReplace,
-                  rowptr, members, output);
+        PB_POOL_LAUNCH("mesh_avg_pool_fwd", avg_pool_fwd_kernel, NvOut * CVn, vec, NvIn, NvOut, CVn, input, vtReplace, rowptr, members, output);
     }
     return PB200_OK;
 }

@@ -182,3 +182,25 @@ def test_average_gradient_keeps_the_sign_of_zero(C):
     d = _dev(cluster_inputs(300, 90, C, seed=3, ties=False))
     got = pool3d.avg_backward(torch.full((90, C), -0.0, device="cuda"), d["x"], d["vt_replace"], d["vt_map"])
     assert torch.signbit(got[d["vt_map"] >= 0]).all()
+
+
+@pytest.mark.parametrize("C", [4, 48, 64, 100, 9])
+def test_average_of_many_and_of_few_clusters(C):
+    """Either side of the line between a thread per quad and teams gives the same bits, for clusters of no, one, four, five and forty members."""
+    from picassoplus_b200.mesh.pi_modules import pool3d
+    sizes = torch.tensor([0, 1, 4, 5, 40], device="cuda").repeat(3000)
+    key = torch.repeat_interleave(torch.arange(sizes.numel(), device="cuda"), sizes)
+    first = torch.cumsum(sizes, 0) - sizes
+    lead = torch.arange(key.numel(), device="cuda") == first[key]
+    # the first vertex cannot be pointed at (its negative is no index): it stands alone
+    rep = torch.where(lead, sizes[key] - 1, -first[key]).int()
+    key = torch.where(lead, key, -1).int()
+    x = torch.relu(torch.randn(key.numel(), C, device="cuda", generator=torch.Generator(device="cuda").manual_seed(C)))
+    whole = pool3d.avg_forward(x, rep, key, torch.zeros(sizes.numel(), 3, device="cuda"))
+    part, rows = 500, int(sizes[:500].sum())                    # 15 000 clusters against 500 of them
+    few = pool3d.avg_forward(x[:rows].contiguous(), rep[:rows].contiguous(), key[:rows].contiguous(), torch.zeros(part, 3, device="cuda"))
+    assert torch.equal(whole[:part], few) and bool((whole[::5] == 0).all())
+    want = torch.zeros(sizes.numel(), C, dtype=torch.float64, device="cuda")
+    owner = torch.repeat_interleave(torch.arange(sizes.numel(), device="cuda"), sizes)
+    want.index_add_(0, owner, x.double())
+    assert rel_err(whole, want / sizes.clamp(min=1).double()[:, None]) <= 1e-6
