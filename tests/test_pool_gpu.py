@@ -184,6 +184,43 @@ def test_average_gradient_keeps_the_sign_of_zero(C):
     assert torch.signbit(got[d["vt_map"] >= 0]).all()
 
 
+SPECIAL = [0.0, 2.0 ** -149, 2.0 ** -126, 2.0 ** -127, 2.0 ** -61, float(np.nextafter(np.float32(2.0 ** -60), np.float32(0))), 2.0 ** -60,
+           float(np.nextafter(np.float32(2.0 ** -60), np.float32(1))), 2.0 ** -36, 1.0, 3.0, float(np.finfo(np.float32).max), float("inf"), float("nan")]
+
+
+def _quotients(x, count, pool3d):
+    """x / count by average pooling's gradient and forward pass: every vertex a cluster of its own that claims `count` members."""
+    nv = x.shape[0]
+    rep = torch.full((nv,), count - 1, dtype=torch.int32, device="cuda")
+    key = torch.arange(nv, dtype=torch.int32, device="cuda")
+    return pool3d.avg_backward(x, x, rep, key), pool3d.avg_forward(x, rep, key, torch.zeros(nv, 3, device="cuda"))
+
+
+def _same_bits(a, b):
+    number = ~a.isnan()
+    return torch.equal(number, ~b.isnan()) and torch.equal(a.view(torch.int32)[number], b.view(torch.int32)[number])
+
+
+@pytest.mark.parametrize("count", [1, 2, 3, 4, 5, 6, 7, 9, 10, 11, 13, 15, 17, 23, 31, 49, 63, 97, 255, 1021, 4095, 12288, 65537, 8388607,
+                                   16777215, 16777216, 16777218, 2147483647])
+def test_quotients_have_the_bits_of_the_division(count):
+    """Every mantissa, at exponents all over the range, for a member count; and the values around the edges of the short form."""
+    from picassoplus_b200.mesh.pi_modules import pool3d
+    g = torch.Generator(device="cuda").manual_seed(count % 1000)
+    mantissa = torch.arange(1 << 23, dtype=torch.int32, device="cuda")
+    exponent = torch.randint(1, 255, mantissa.shape, dtype=torch.int32, device="cuda", generator=g)
+    sign = torch.randint(0, 2, mantissa.shape, dtype=torch.int32, device="cuda", generator=g)
+    edges = torch.tensor(SPECIAL + [-v for v in SPECIAL], device="cuda").repeat(256, 1)[:, :28].contiguous()
+    divisor = torch.tensor(float(count), device="cuda")
+    for x in (((exponent << 23) | mantissa | (sign << 31)).view(torch.float32).view(-1, 64), ((127 << 23) | mantissa).view(torch.float32).view(-1, 64),
+              edges, edges[:, :27].contiguous()):
+        want = x / divisor
+        back, forward = _quotients(x, count, pool3d)
+        assert _same_bits(back, want) and _same_bits(forward, want + 0.0)       # a sum from +0 has no -0
+    few = x[:100]
+    assert _same_bits(_quotients(few, count, pool3d)[1], few / divisor + 0.0)
+
+
 @pytest.mark.parametrize("C", [4, 48, 64, 100, 9])
 def test_average_of_many_and_of_few_clusters(C):
     """Either side of the line between a thread per quad and teams gives the same bits, for clusters of no, one, four, five and forty members."""
