@@ -592,6 +592,20 @@ void masked_gradient(const Scope& s, const Tensor& g, const Tensor& act, const N
 struct Staged { Tensor out, act, features; NormStats stats; };
 // What a pass that keeps no features may spend on gathered rows (2 M rows of 128 channels); larger ones gather inside the product.
 constexpr int64_t GATHER_BYTES = int64_t(1) << 30;
+// Whether that much can be had without making room: from what the allocator holds and nobody uses, else from a device that has
+// plenty.  An allocation that fails gives every cached block back to the driver first, and a pass would pay for that call after call.
+bool has_room(size_t bytes) {
+    using c10::CachingAllocator::StatType;
+    constexpr auto ALL = static_cast<size_t>(StatType::AGGREGATE);
+    const auto stats = c10::cuda::CUDACachingAllocator::getDeviceStats(call_device);
+    const int64_t reserved = stats.reserved_bytes[ALL].current, need = (int64_t)bytes;
+    if (reserved - stats.active_bytes[ALL].current >= need) return true;
+    size_t free = 0, total = 0;
+    c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
+    if (cudaMemGetInfo(&free, &total) != cudaSuccess) return false;
+    const double allowed = c10::cuda::CUDACachingAllocator::getMemoryFraction(call_device) * (double)total - (double)reserved;
+    return (double)free >= 4. * (double)need && allowed >= 4. * (double)need;
+}
 template <typename Launch>
 Staged run_stage(const Scope& s, const Tail& t, int64_t rows, int64_t C, int64_t Cout, bool keep_features, bool gathers, Launch&& launch) {
     check_tail(t, Cout);
@@ -602,11 +616,13 @@ Staged run_stage(const Scope& s, const Tail& t, int64_t rows, int64_t C, int64_t
     if (keep_features) {
         r.features = s.floats({rows, C});
         x.features = fpm(r.features);
-    } else if (gathers && pb200_layer_wants_features(rows) && rows <= GATHER_BYTES / 4 / C) {
+    } else if (gathers && rows <= GATHER_BYTES / 4 / C) {
         try {
-            scratch = s.bytes((size_t)(4 * rows * C));
-            x.features = static_cast<float*>(scratch.data_ptr());
-        } catch (const c10::OutOfMemoryError&) {      // the kernel that needs no room for them is still there
+            if (has_room((size_t)(4 * rows * C))) {
+                scratch = s.bytes((size_t)(4 * rows * C));
+                x.features = static_cast<float*>(scratch.data_ptr());
+            }
+        } catch (const c10::Error&) {      // no memory after all, an allocator without figures: the kernel that needs no room is still there
         }
     }
     if (t.mode == NORM_RUNNING) {
@@ -849,7 +865,7 @@ Tensor v2f_layer(const Tensor& x_in, const Tensor& face, const OptTensor& rowptr
     const Tensor filter = at::matmul(corners, spatial).view({3, C, 1});
     const size_t nb = pb200_vertex2facet_pointwise_workspace_bytes((int)C, precision);
     const Workspace ws = s.bytes(nb);
-    Staged r = run_stage(s, t, Nf, C, Cout, (bool)node, true, [&](float* out, const pb200_pointwise_extra* extra) {
+    Staged r = run_stage(s, t, Nf, C, Cout, (bool)node, pb200_layer_wants_features(Nf), [&](float* out, const pb200_pointwise_extra* extra) {
         call(pb200_vertex2facet_layer_forward(Nf, Nv, (int)C, (int)Cout, fp(x), fp(filter), ip(face), fp(weights_in), fp(bias), relu, out,
                                               precision, extra, ws.data_ptr(), nb, s.stream),
              "pb200_vertex2facet_layer_forward");
@@ -892,7 +908,7 @@ Tensor f2v_layer(const Tensor& x_in, const Tensor& face, const Tensor& nf_count,
     const Tensor x = aligned(x_in), filter = aligned(filter_in), bias = flat(bias0, Cout);
     const size_t nb = pb200_facet2vertex_pointwise_workspace_bytes(Nf, (int)C, precision);
     const Workspace ws = s.bytes(nb);
-    Staged r = run_stage(s, t, NvOut, C, Cout, (bool)node, true, [&](float* out, const pb200_pointwise_extra* extra) {
+    Staged r = run_stage(s, t, NvOut, C, Cout, (bool)node, pb200_layer_wants_features(NvOut), [&](float* out, const pb200_pointwise_extra* extra) {
         call(pb200_facet2vertex_layer_forward(Nf, NvOut, (int)C, (int)K, (int)Cout, fp(x), fp(filter), fp(coeff), ip(nf_count), ip(rowptr),
                                               ip(entries), fp(weights), fp(bias), relu, out, precision, extra, ws.data_ptr(), nb, s.stream),
              "pb200_facet2vertex_layer_forward");

@@ -155,3 +155,28 @@ def test_rows_that_take_no_part(C):
     want = (go.double()[:, None] * x.double()[face.long()]).sum(0)                # (3, C)
     assert not bool(want[0, 0].isfinite()) and bool(gw[1:, 0].isfinite().all()) and not bool(gw[0, 0].isfinite())
     assert rel_err(gw[:, 1:, 0], want[:, 1:]) <= 5e-6
+
+
+def test_inference_takes_no_room_that_is_not_there():
+    """Gathered rows that a layer could do without are not asked for where they do not fit: no failed allocation, which would cost the
+    process its cached memory call after call, and the same results."""
+    from picassoplus_b200.mesh.layers import V2FConv3d
+    g = torch.Generator(device="cuda").manual_seed(0)
+    rows, nv, C = 400000, 20000, 256
+    layer, x = V2FConv3d(C, 128, 2).cuda().eval(), torch.randn(nv, C, device="cuda", generator=g)
+    face = torch.randint(nv, (rows, 3), device="cuda", generator=g).int()
+    scratch = 4 * rows * C
+    with torch.no_grad():
+        torch.cuda.reset_peak_memory_stats()
+        want = layer(x, face)
+        assert torch.cuda.max_memory_allocated() - torch.cuda.memory_allocated() > scratch          # the sizes do ask for them
+        torch.cuda.empty_cache()
+        figures = lambda: [torch.cuda.memory_stats()[k] for k in ("num_ooms", "num_alloc_retries")]
+        counts, total = figures(), torch.cuda.get_device_properties(0).total_memory
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + want.numel() * 4 + scratch // 2) / total)
+        try:
+            for _ in range(3):
+                assert torch.equal(layer(x, face), want)
+        finally:
+            torch.cuda.set_per_process_memory_fraction(1.0)
+        assert figures() == counts
