@@ -242,8 +242,10 @@ typedef struct {
     const float *mean, *var, *gamma, *beta;
     float eps;
 } pb200_pointwise_extra;
-/* 1 if the layers' forward passes over this many rows run faster when `features` of their extras is given */
+/* 1 if a facet2vertex layer's forward pass over this many rows runs faster when `features` of its extras is given, and for vertex2facet if
+ * it does where nobody wants the features themselves */
 int pb200_layer_wants_features(int64_t rows);
+int pb200_vertex2facet_layer_wants_features(int64_t rows, int C, int Cout);
 int pb200_vertex2facet_layer_forward(int64_t Nf, int64_t Nv, int C, int Cout, const float* input, const float* filter,
                                      const int32_t* face, const float* depthWeights, const float* bias, int relu,
                                      float* output, int precision, const pb200_pointwise_extra* extra, void* workspace,

@@ -92,6 +92,7 @@ SIGNATURES = {
     "pb200_facet2facet_backward_padded": (i32, [i64, i64, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, i32, vp, sz, vp]),
     "pb200_facet2facet_one_sample_backward": (i32, [i64, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, i32, vp, sz, vp]),
     "pb200_layer_wants_features": (i32, [i64]),
+    "pb200_vertex2facet_layer_wants_features": (i32, [i64, i32, i32]),
     "pb200_facet2facet_layer_forward": (i32, [i64, i64, i32, i32, i32, vp, vp, vp, vp, vp, i32, vp, vp, vp, i32, vp, sz, vp]),
     "pb200_facet2facet_layer_gradient_fused": (i32, [i64, i64, i32, i32, i32, vp, i32]),
     "pb200_facet2facet_layer_filter_gradient_workspace_bytes": (sz, [i64, i32, i32]),

@@ -426,10 +426,20 @@ __global__ void __launch_bounds__(NTHREADS<MODE>, 1) rows_pointwise_tc_kernel(Pa
 // From this many rows on, a call that is given room for its gathered rows (`features`) runs the operator's own kernel into it and the
 // product on those rows: same sums, same bits, one launch more.  The fused producers keep 512 threads' gathers in flight per SM beside
 // 130 KB of operand buffers, the operator's kernel 2048 with all of L1.  980 000 vertices 128 -> 128: 805 us fused, 335 + 160 apart;
-// 1.76 M faces 64 -> 128: 519 against 122 + 230; an inference pass of a 2 x 700^2 scene 3.74 against 3.22 ms.  Below about 100 000 rows
-// the gathered rows stay in L2, the gather takes 20 us or less, and the launch costs what it saves: a scene of 2 x 120^2 with its
-// backward pass 1 209 us fused, 1 278 with every gather apart, 1 222 with those from 100 000 rows on (spread of a side 20).
+// 1.76 M faces 64 -> 128: 519 against 122 + 230.  Below, the launch costs what it saves: a scene of 2 x 120^2 with its backward pass
+// 1 209 us fused, 1 278 with every gather apart, 1 222 with those from 100 000 rows on (spread of a side 20).
+// The line is one of rows for facet2vertex at 8 to 384 channels and as many outputs (122 500 rows 0.54 to 0.93 of the fused time, 108 900
+// up to 1.0), and for vertex2facet where the backward pass wants the rows (195 000 rows at most 1.01).
 constexpr int64_t GATHER_ALONE = 100000;
+// vertex2facet that would write its rows for the product alone: the fused kernel reads three rows of a face that its neighbours read too
+// and writes none, so the other way pays where the outputs are many or take more than one launch, and for wide rows where the vertices
+// outgrow L2.  Layers with their running statistics, fused -> apart: 195 000 faces 64 -> 64 channels 55 -> 64 us, 128 -> 16 75 -> 88, 64 -> 128
+// 73 -> 66, 102 800 128 -> 128 53 -> 61, 128 -> 256 108 -> 96; 448 000 32 -> 16 69 -> 83, 64 -> 64 122 -> 109; 879 000 32 -> 16 137 -> 146, 16 -> 32
+// 128 -> 131, 32 -> 64 152 -> 148; 1.76 M 16 -> 64 270 -> 241.
+static bool rows_for_product_alone(int64_t rows, int C, int Cout) {
+    if (C < 64) return rows * Cout >= 50000000;
+    return rows * Cout >= 17000000 || rows >= 600000;
+}
 struct Plan { int nsplit, nkb, nstages; size_t smem, wimg_bytes; };
 
 static Plan plan(int C, int precision) {
@@ -511,6 +521,9 @@ using namespace pb;
 extern "C" {
 
 int pb200_layer_wants_features(int64_t rows) { return rows >= pw::GATHER_ALONE; }
+int pb200_vertex2facet_layer_wants_features(int64_t rows, int C, int Cout) {
+    return rows >= pw::GATHER_ALONE && pw::rows_for_product_alone(rows, C, Cout);
+}
 
 size_t pb200_vertex2facet_pointwise_workspace_bytes(int C, int precision) {
     if (C <= 0) return 0;

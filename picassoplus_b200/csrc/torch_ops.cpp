@@ -865,7 +865,7 @@ Tensor v2f_layer(const Tensor& x_in, const Tensor& face, const OptTensor& rowptr
     const Tensor filter = at::matmul(corners, spatial).view({3, C, 1});
     const size_t nb = pb200_vertex2facet_pointwise_workspace_bytes((int)C, precision);
     const Workspace ws = s.bytes(nb);
-    Staged r = run_stage(s, t, Nf, C, Cout, (bool)node, pb200_layer_wants_features(Nf), [&](float* out, const pb200_pointwise_extra* extra) {
+    Staged r = run_stage(s, t, Nf, C, Cout, (bool)node, pb200_vertex2facet_layer_wants_features(Nf, (int)C, (int)Cout), [&](float* out, const pb200_pointwise_extra* extra) {
         call(pb200_vertex2facet_layer_forward(Nf, Nv, (int)C, (int)Cout, fp(x), fp(filter), ip(face), fp(weights_in), fp(bias), relu, out,
                                               precision, extra, ws.data_ptr(), nb, s.stream),
              "pb200_vertex2facet_layer_forward");
