@@ -187,13 +187,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
                 }
             }
             float* const row = p.out + f * p.Cn;
-            auto store = [&](int c, const float (&s)[G<F>]) {
+            // old: what the chunks of contracted channels before have left there, when the caller has it already
+            auto store = [&](int c, const float (&s)[G<F>], const float4* old) {
                 if (!valid || c >= p.Cn) return;
                 if (vec) {
                     if constexpr (G<F> == 4) {
                         float4 v = make_float4(s[0], s[1], s[2], s[3]);
                         float4* dst = reinterpret_cast<float4*>(row + c);
-                        if (p.accumulate) add4(v, *dst);
+                        if (p.accumulate) add4(v, old ? *old : *dst);
                         *dst = v;
                     } else {
                         float2 v = make_float2(s[0], s[1]);
@@ -209,13 +210,24 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
             };
             for (int slice = s0; slice < s1; ++slice, ++sc) {
                 const uint32_t a = sc & 1u;
+                const int c0 = slice * nq;
+                int left = (p.Cn - c0 + G<F> - 1) / G<F>;         // steps of the slice that exist
+                if (left > nq / G<F>) left = nq / G<F>;
+                // With few bases a quadruple is little work, and the loads of what is there already, one behind another, were what a
+                // slice took (4 bases, 320 -> 256 channels, 300 000 faces: bf16 1 025 us, 563 with the slice's loads ahead of the wait)
+                constexpr int AHEAD = F == 4 ? nq / G<F> / (EWARPS / 4) : 1;
+                float4 old[AHEAD];
+                if constexpr (F == 4) {
+#pragma unroll
+                    for (int i = 0; i < AHEAD; ++i) {
+                        const int c = c0 + G<F> * (sub + i * (EWARPS / 4));
+                        old[i] = p.accumulate && vec && valid && c < p.Cn ? *reinterpret_cast<const float4*>(row + c) : zero4();
+                    }
+                }
                 int ok = 1;
                 if (lane == 0) ok = mbar_wait(&acc_full[a], (sc >> 1) & 1u, abort_flag) ? 1 : 0;
                 if (!__shfl_sync(0xffffffffu, ok, 0)) { alive = false; break; }
                 tc_fence_after();
-                const int c0 = slice * nq;
-                int left = (p.Cn - c0 + G<F> - 1) / G<F>;         // steps of the slice that exist
-                if (left > nq / G<F>) left = nq / G<F>;
                 auto hand_back = [&](int k) {                     // after the loads of this warp's last quadruple
                     if (k + EWARPS / 4 < left) return;
                     tc_fence_before();
@@ -223,7 +235,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
                     if (lane == 0) arrive_first<PAIR>(&acc_empty[a]);
                 };
                 if (sub >= left) hand_back(left);                 // nothing of this slice for this warp
-                for (int k = sub; k < left; k += EWARPS / 4) {
+                auto step = [&](int k, const float4* have) {
                     float s[G<F>], v[G<F> * F];
                     const uint32_t t = tbase + a * NCOLS + (uint32_t)(k * G<F> * F);
                     if constexpr (F == 16) { tmem_ld32f(t, v); tmem_ld32f(t + 32, v + 32); }
@@ -232,7 +244,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
                     hand_back(k);
 #pragma unroll
                     for (int j = 0; j < G<F>; ++j) s[j] = weighted<F>(v + j * F, b);
-                    store(c0 + G<F> * k, s);
+                    store(c0 + G<F> * k, s, have);
+                };
+                if constexpr (F == 4) {
+#pragma unroll
+                    for (int i = 0; i < AHEAD; ++i)
+                        if (sub + i * (EWARPS / 4) < left) step(sub + i * (EWARPS / 4), &old[i]);
+                } else {
+                    for (int k = sub; k < left; k += EWARPS / 4) step(k, nullptr);
                 }
             }
         }
@@ -505,29 +524,30 @@ int run(int64_t Nf, int Cn, int Ck, int F, const float* rows, const float* filte
     const char* label = forward ? "f2f_fwd_one_tc" : "f2f_bwd_gin_one_tc";
     int rc = check_async_error(forward ? "facet2facet_forward" : "facet2facet_backward");
     if (rc) return rc;
-    const Plan pl = plan(Cn, Ck, F, precision);
     const int64_t s_ck = forward ? (int64_t)F : (int64_t)Cn * F, s_cn = forward ? (int64_t)Ck * F : (int64_t)F;
-    const int nb = pl.pair ? 2 : 1, sms = sm_count() / nb;        // CTAs, and those that work on items of their own
-    const int64_t ntiles = ceil_div(Nf, nb * TILE_M);
-    // Slice groups of a tile.  With fewer tiles than SMs a tile's slices go to as many CTAs as there are.  With a few tiles per
-    // SM the last wave is short of tiles: groups are halved while that evens it out, but a group keeps enough products (two
-    // slices of three, four of one) for the copy of the next item's rows to hide behind.
-    int groups = 1;
-    if (ntiles < sms) {
-        groups = (int)(sms / ntiles);
-        if (groups > pl.nslices) groups = pl.nslices;
-    } else {
-        const int keep = pl.nsplit == 2 ? 2 : 4;
-        while (ntiles * groups < 8LL * sms && pl.nslices >= 2 * groups * keep) groups *= 2;
-    }
-    const int per_group = (int)ceil_div(pl.nslices, groups);
-    groups = (int)ceil_div(pl.nslices, per_group);
-    const int64_t items = ntiles * groups;
-    PB_REQUIRE(items < 0x7fffffff / 2, PB200_EINVAL, "%s: %lld faces are too many", label, (long long)Nf);
-    const int grid = nb * (int)(items < sms ? items : sms);
     for (int k0 = 0; k0 < Ck; k0 += MAX_CK) {
         const int chunk = Ck - k0 < MAX_CK ? Ck - k0 : MAX_CK;
-        const int kst = (chunk + 31) / 32;
+        // a plan of its own for every chunk: the last one may be short
+        const Plan pl = plan(Cn, chunk, F, precision);
+        const int kst = pl.kst;
+        const int nb = pl.pair ? 2 : 1, sms = sm_count() / nb;        // CTAs, and those that work on items of their own
+        const int64_t ntiles = ceil_div(Nf, nb * TILE_M);
+        // Slice groups of a tile.  With fewer tiles than SMs a tile's slices go to as many CTAs as there are.  With a few tiles per
+        // SM the last wave is short of tiles: groups are halved while that evens it out, but a group keeps enough products (two
+        // slices of three, four of one) for the copy of the next item's rows to hide behind.
+        int groups = 1;
+        if (ntiles < sms) {
+            groups = (int)(sms / ntiles);
+            if (groups > pl.nslices) groups = pl.nslices;
+        } else {
+            const int keep = pl.nsplit == 2 ? 2 : 4;
+            while (ntiles * groups < 8LL * sms && pl.nslices >= 2 * groups * keep) groups *= 2;
+        }
+        const int per_group = (int)ceil_div(pl.nslices, groups);
+        groups = (int)ceil_div(pl.nslices, per_group);
+        const int64_t items = ntiles * groups;
+        PB_REQUIRE(items < 0x7fffffff / 2, PB200_EINVAL, "%s: %lld faces are too many", label, (long long)Nf);
+        const int grid = nb * (int)(items < sms ? items : sms);
         rc = gin::prep_filter_bf16(F, Cn, k0, chunk, pl.nq, pl.nslices, kst, pl.nsplit, pl.nmma, s_ck, s_cn, filter, (uint8_t*)ws, stream);
         if (rc) return rc;
         Params p;
