@@ -59,13 +59,15 @@ static_assert(NTHREADS % 128 == 0 && EWARPS * 32 * REGS_EPILOGUE + (NTHREADS - E
 constexpr int KTILE_BYTES = TILE_M * 64;         // 32 channels of the tile's rows
 constexpr int MAX_CK = 256;                      // contracted channels per launch
 constexpr int MAX_GBUFS = 3;                     // tile buffers
+constexpr int RAW_STAGES = 2, RAW_BYTES = 2 * KTILE_BYTES;       // where rows are not converted in place: K-blocks on their way
 
 struct Params {
     int64_t Nf;
     int nitems;                      // pairs of tiles x slice groups
     int Cn, Ck;
     int nslices, kst, nmma;
-    int nstages, kb, gbufs;          // filter stages, K-blocks of 32 channels in one stage (divides kst)
+    int nstages, kb, gbufs;          // filter stages, K-blocks of 32 channels in one stage (divides kst), tile buffers
+    int staged;                      // one operand: rows come through stages of one K-block (see plan)
     int groups, per_group;           // slice groups of a tile, slices of a group
     const float* rows;
     int stride;                      // floats per row
@@ -125,28 +127,32 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int S = p.nstages, KST = p.kst;
-    const uint32_t gtile_bytes = 2u * KST * KTILE_BYTES;
+    const bool staged = NSPLIT == 1 && p.staged;
+    const uint32_t gtile_bytes = (staged ? 1u : 2u) * KST * KTILE_BYTES;
     constexpr int NB = PAIR ? 2 : 1;          // CTAs of a product: each has its own tile and its share of a filter block's rows
     const uint32_t w_bytes = (uint32_t)p.nmma * 64 / NB, wblk_bytes = NSPLIT * w_bytes, wstage_bytes = wblk_bytes * p.kb;
     const uint32_t rank = PAIR ? cluster_rank() : 0;
     uint8_t* gtile = smem;
-    uint8_t* wst = smem + (size_t)p.gbufs * gtile_bytes;
+    uint8_t* raw = smem + (size_t)p.gbufs * gtile_bytes;
+    uint8_t* wst = raw + (staged ? RAW_STAGES * RAW_BYTES : 0);
     uint64_t* bars = reinterpret_cast<uint64_t*>(wst + (size_t)S * wstage_bytes);
     uint64_t* w_full = bars;                  // [S]
     uint64_t* w_empty = bars + S;             // [S]
     uint64_t* w_peer = bars + 2 * S;          // [S] rank 0: the peer's half has landed
     uint64_t* acc_full = bars + 3 * S;        // [2]
     uint64_t* acc_empty = bars + 3 * S + 2;   // [2] rank 0: both blocks' epilogues
-    uint64_t* raw_full = bars + 3 * S + 4;    // [MAX_GBUFS] rows in the tile buffer as they are in memory
+    uint64_t* raw_full = bars + 3 * S + 4;    // [MAX_GBUFS] rows in the tile buffer (a K-block of them in a stage) as they are in memory
     uint64_t* g_full = raw_full + MAX_GBUFS;  // [MAX_GBUFS] converted; rank 0: in both blocks
     uint64_t* g_empty = g_full + MAX_GBUFS;   // [MAX_GBUFS] all products of the item done with the buffer
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(g_empty + MAX_GBUFS);
+    uint64_t* raw_empty = g_empty + MAX_GBUFS;   // [RAW_STAGES] a stage's rows are in the tile buffer
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(raw_empty + RAW_STAGES);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     if (tid == 0) {
         for (int s = 0; s < S; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], 1); mbar_init(&w_peer[s], 1); }
         for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], NB * EWARPS); }
         for (int b = 0; b < MAX_GBUFS; ++b) { mbar_init(&raw_full[b], 1); mbar_init(&g_full[b], NB * GWARPS); mbar_init(&g_empty[b], 1); }
+        for (int b = 0; b < RAW_STAGES; ++b) mbar_init(&raw_empty[b], GWARPS);
         abort_flag[0] = 0;
         abort_flag[1] = p.wait_budget;
         fence_barrier_init();
@@ -258,44 +264,66 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
     } else if (warp >= EWARPS + 3) {
         // ===================== row converters =====================
         // a task is 32 channels of 32 rows: a lane turns its row's 32 floats, which lie in the two 64-byte slots of that row
-        // (channels 0..15 and 16..31), into bf16 hi and lo in the same two slots
+        // (channels 0..15 and 16..31), into bf16 hi and lo in the same two slots, or from a stage into the tile buffer's one
         const int gw = warp - (EWARPS + 3);
-        uint32_t icount = 0;
-        for (int item = item0; item < nitems; item += item_step, ++icount) {
+        auto convert = [&](uint32_t rr, uint32_t from, uint32_t from2, uint32_t to, uint32_t to2) {
+            const uint32_t sw = rr >> 1 & 3u;
+            float4 v[8];
+#pragma unroll
+            for (uint32_t c = 0; c < 4; ++c) { v[c] = lds_f4(from + ((c ^ sw) << 4)); v[4 + c] = lds_f4(from2 + ((c ^ sw) << 4)); }
+#pragma unroll
+            for (uint32_t c = 0; c < 4; ++c) {
+                const float4 a = v[2 * c], b = v[2 * c + 1];
+                uint32_t hi[4], lo[4];
+                if (NSPLIT == 1) {
+                    hi[0] = pack_bf16x2(a.x, a.y); hi[1] = pack_bf16x2(a.z, a.w);
+                    hi[2] = pack_bf16x2(b.x, b.y); hi[3] = pack_bf16x2(b.z, b.w);
+                } else {
+                    split_bf16x2(a.x, a.y, hi[0], lo[0]); split_bf16x2(a.z, a.w, hi[1], lo[1]);
+                    split_bf16x2(b.x, b.y, hi[2], lo[2]); split_bf16x2(b.z, b.w, hi[3], lo[3]);
+                    sts_u4(to2 + ((c ^ sw) << 4), lo[0], lo[1], lo[2], lo[3]);
+                }
+                sts_u4(to + ((c ^ sw) << 4), hi[0], hi[1], hi[2], hi[3]);
+            }
+        };
+        uint32_t icount = 0, blocks = 0;
+        bool alive = true;
+        for (int item = item0; item < nitems && alive; item += item_step, ++icount) {
             const uint32_t gb = icount % p.gbufs, gph = icount / p.gbufs & 1u;
             const uint32_t tile = smem_u32(gtile) + gb * gtile_bytes;
-            if (!warp_wait(&raw_full[gb], gph, abort_flag, lane)) break;
-            for (int task = gw; task < 4 * KST; task += GWARPS) {
-                const uint32_t rr = (uint32_t)(task & 3) * 32 + lane, sw = rr >> 1 & 3u;
-                const uint32_t first = tile + (uint32_t)(task >> 2) * KTILE_BYTES + rr * 64, second = first + (uint32_t)KST * KTILE_BYTES;
-                float4 v[8];
-#pragma unroll
-                for (uint32_t c = 0; c < 4; ++c) { v[c] = lds_f4(first + ((c ^ sw) << 4)); v[4 + c] = lds_f4(second + ((c ^ sw) << 4)); }
-#pragma unroll
-                for (uint32_t c = 0; c < 4; ++c) {
-                    const float4 a = v[2 * c], b = v[2 * c + 1];
-                    uint32_t hi[4], lo[4];
-                    if (NSPLIT == 1) {
-                        hi[0] = pack_bf16x2(a.x, a.y); hi[1] = pack_bf16x2(a.z, a.w);
-                        hi[2] = pack_bf16x2(b.x, b.y); hi[3] = pack_bf16x2(b.z, b.w);
-                    } else {
-                        split_bf16x2(a.x, a.y, hi[0], lo[0]); split_bf16x2(a.z, a.w, hi[1], lo[1]);
-                        split_bf16x2(b.x, b.y, hi[2], lo[2]); split_bf16x2(b.z, b.w, hi[3], lo[3]);
-                        sts_u4(second + ((c ^ sw) << 4), lo[0], lo[1], lo[2], lo[3]);
+            if (staged) {
+                if (!warp_wait(&g_empty[gb], gph ^ 1u, abort_flag, lane)) break;
+                for (int ks = 0; ks < KST; ++ks, ++blocks) {
+                    const uint32_t st = blocks % RAW_STAGES;
+                    if (!warp_wait(&raw_full[st], blocks / RAW_STAGES & 1u, abort_flag, lane)) { alive = false; break; }
+                    for (uint32_t part = gw; part < 4; part += GWARPS) {
+                        const uint32_t rr = part * 32 + lane, from = smem_u32(raw) + st * RAW_BYTES + rr * 64;
+                        const uint32_t to = tile + (uint32_t)ks * KTILE_BYTES + rr * 64;
+                        convert(rr, from, from + KTILE_BYTES, to, to);
                     }
-                    sts_u4(first + ((c ^ sw) << 4), hi[0], hi[1], hi[2], hi[3]);
+                    fence_proxy_async();                          // these reads before the next copy, these writes before the products
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&raw_empty[st]);
                 }
+                if (!alive) break;
+            } else {
+                if (!warp_wait(&raw_full[gb], gph, abort_flag, lane)) break;
+                for (int task = gw; task < 4 * KST; task += GWARPS) {
+                    const uint32_t rr = (uint32_t)(task & 3) * 32 + lane;
+                    const uint32_t first = tile + (uint32_t)(task >> 2) * KTILE_BYTES + rr * 64, second = first + (uint32_t)KST * KTILE_BYTES;
+                    convert(rr, first, second, first, second);
+                }
+                fence_proxy_async();
+                __syncwarp();
             }
-            fence_proxy_async();
-            __syncwarp();
             if (lane == 0) arrive_first<PAIR>(&g_full[gb]);
         }
     } else if (warp == EWARPS + 2) {
         // ===================== row stream (TMA engine) =====================
         if (elect_one()) {
-            uint32_t icount = 0;
+            uint32_t icount = 0, blocks = 0;
             bool alive = true;
-            for (int item = item0; item < nitems; item += item_step, ++icount) {
+            for (int item = item0; item < nitems && alive; item += item_step, ++icount) {
                 const int64_t f0 = (int64_t)(item / p.groups * NB + rank) * TILE_M;
                 const uint32_t gb = icount % p.gbufs, gph = icount / p.gbufs & 1u;
                 const int64_t n0 = (int64_t)((item + item_step) / p.groups * NB + rank) * TILE_M;
@@ -303,6 +331,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
                     const int64_t n = p.Nf - n0 < TILE_M ? p.Nf - n0 : TILE_M;
                     if (p.stride == p.Ck) prefetch_l2(p.rows + n0 * p.stride, (uint32_t)(n * p.stride * 4));
                     prefetch_l2(p.w + n0 * p.Fp, (uint32_t)(n * p.Fp * 4));
+                }
+                if (staged) {
+                    for (int ks = 0; ks < KST; ++ks, ++blocks) {
+                        const uint32_t st = blocks % RAW_STAGES;
+                        if (!mbar_wait(&raw_empty[st], (blocks / RAW_STAGES & 1u) ^ 1u, abort_flag)) { alive = false; break; }
+                        mbar_arrive_expect_tx(&raw_full[st], RAW_BYTES);
+                        tile_g2s(raw + st * RAW_BYTES, &rows_map, ks * 32, (int)f0, &raw_full[st]);
+                        tile_g2s(raw + st * RAW_BYTES + KTILE_BYTES, &rows_map, ks * 32 + 16, (int)f0, &raw_full[st]);
+                    }
+                    continue;
                 }
                 if (!mbar_wait(&g_empty[gb], gph ^ 1u, abort_flag)) { alive = false; break; }
                 mbar_arrive_expect_tx(&raw_full[gb], gtile_bytes);
@@ -431,7 +469,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) f2f_one_sample_tc_kernel(Params p
 }
 
 // ---------------------------------------------------------------------------- host side
-struct Plan { bool pair; int nsplit, nq, nslices, kst, nmma, nblocks, gbufs; size_t smem, wimg_bytes; };
+struct Plan { bool pair, staged; int nsplit, nq, nslices, kst, nmma, nblocks, gbufs; size_t smem, wimg_bytes; };
 
 // K-blocks of 32 contracted channels from which CTAs work in pairs, three products per term.  A pair halves the traffic of the filter
 // blocks, from L2 and from shared memory, and pays with a round trip between two SMs per slice: worth it where a slice is 24
@@ -457,7 +495,15 @@ static Plan plan(int Cn, int CkAll, int F, int precision) {
     // a second tile buffer takes the row copy off the critical path, when at least three filter blocks still fit beside it
     pl.gbufs = (2 * gt + 1024 + 640 + 3 * ws <= budget) ? 2 : 1;
     if (3 * gt + 1024 + 640 + 2 * pl.kst * ws <= budget) pl.gbufs = 3;
-    const size_t fixed = pl.gbufs * gt + 1024 + 640;
+    size_t fixed = pl.gbufs * gt + 1024 + 640;
+    // One operand fills half of what its rows take on the way.  Where that leaves a single buffer, rows come through stages of one K-block
+    // instead of in place, and two buffers of the operand alone fit (bf16, 256 -> 256, 25 bases, 40 000 faces: 198 us in place, 169
+    // so; 192 -> 64, 9 bases, 300 000 faces 214 and 140).
+    pl.staged = pl.nsplit == 1 && pl.gbufs == 1;
+    if (pl.staged) {
+        pl.gbufs = 2;
+        fixed = (size_t)2 * pl.kst * KTILE_BYTES + RAW_STAGES * RAW_BYTES + 1024 + 640;
+    }
     pl.nblocks = (int)((budget - fixed) / ws);
     if (pl.nblocks > 16) pl.nblocks = 16;
     pl.smem = fixed + pl.nblocks * ws;
@@ -552,7 +598,7 @@ int run(int64_t Nf, int Cn, int Ck, int F, const float* rows, const float* filte
         if (rc) return rc;
         Params p;
         p.Nf = Nf; p.nitems = (int)items; p.Cn = Cn; p.Ck = chunk;
-        p.nslices = pl.nslices; p.kst = kst; p.nmma = pl.nmma; p.gbufs = pl.gbufs;
+        p.nslices = pl.nslices; p.kst = kst; p.nmma = pl.nmma; p.gbufs = pl.gbufs; p.staged = pl.staged;
         p.kb = kst;
         while (p.kb > 1 && (kst % p.kb != 0 || pl.nblocks < 2 * p.kb)) --p.kb;
         p.nstages = pl.nblocks / p.kb;
