@@ -476,17 +476,21 @@ struct Plan { bool pair, staged; int nsplit, nq, nslices, kst, nmma, nblocks, gb
 // products long (464 000 faces, 128 -> 128: 25 bases 851 -> 761 us, 16 bases 529 -> 466, 9 bases 343 -> 312; 3 000 faces 27.6 -> 25.6),
 // not at 18 (96 -> 96, 16 bases: 294 -> 306), 12 (880 000 faces, 64 -> 64: 288 -> 331) or 8 (bf16, 128 -> 128, 25 bases: 400 -> 542).
 constexpr int PAIR_FROM = 4;
+// Five and seven blocks make a round trip each, as no larger filter stage divides them.  Five still pair where CTAs have several tiles,
+// because only a pair's smaller filter blocks leave room for a second tile buffer (160 -> 128, 16 bases, alone -> in pairs: 40 000 faces 135 ->
+// 89 us, 10 000 34 -> 45); seven never (224 -> 128, 16 bases: 40 000 faces 179 -> 194, 10 000 44 -> 54).
+static bool in_pairs(int kst, bool several_tiles) { return kst >= PAIR_FROM && kst != 7 && (kst != 5 || several_tiles); }
 
 static int nq_of(int F) { return F == 4 ? NQ<4> : F == 9 ? NQ<9> : F == 16 ? NQ<16> : NQ<25>; }
 
-static Plan plan(int Cn, int CkAll, int F, int precision) {
+static Plan plan(int Cn, int CkAll, int F, int precision, bool several_tiles) {
     Plan pl;
     const int Ck = CkAll < MAX_CK ? CkAll : MAX_CK;
     pl.nsplit = operand_mode(precision).nsplit;
     pl.nq = nq_of(F);
     const int g = F == 25 ? G<25> : G<4>, cn = (Cn + g - 1) / g * g;
     pl.kst = (Ck + 31) / 32;
-    pl.pair = pl.nsplit == 2 && pl.kst >= PAIR_FROM;
+    pl.pair = pl.nsplit == 2 && in_pairs(pl.kst, several_tiles);
     const int step = pl.pair ? 32 : 16;                           // columns of a product
     pl.nmma = ((pl.nq > cn ? cn : pl.nq) * F + step - 1) / step * step;
     pl.nslices = (Cn + pl.nq - 1) / pl.nq;
@@ -515,11 +519,15 @@ static Plan plan(int Cn, int CkAll, int F, int precision) {
 bool supported(int Cn, int Ck, int F, int precision) {
     if (precision != PB200_PREC_FP32 && precision != PB200_PREC_BF16) return false;
     if (!(F == 4 || F == 9 || F == 16 || F == 25) || Cn < 1 || Ck < 4 || Ck % 4 != 0) return false;
-    const Plan pl = plan(Cn, Ck, F, precision);
-    return pl.nblocks >= 2 && pl.smem <= 227 * 1024;
+    for (const bool several : {false, true}) {
+        const Plan pl = plan(Cn, Ck, F, precision, several);
+        if (pl.nblocks < 2 || pl.smem > 227 * 1024) return false;
+    }
+    return true;
 }
 
-size_t workspace_bytes(int Cn, int Ck, int F, int precision) { return align_up(plan(Cn, Ck, F, precision).wimg_bytes, 256); }
+// the image of a pair, whose columns are rounded further up, is no smaller than the other
+size_t workspace_bytes(int Cn, int Ck, int F, int precision) { return align_up(plan(Cn, Ck, F, precision, true).wimg_bytes, 256); }
 
 // Tensor map of (Nf, channels) floats with `stride` floats between rows: boxes of 16 channels x 128 rows, laid down as 64-byte rows with
 // the 64-byte swizzle, the layout of the product's operand
@@ -574,7 +582,7 @@ int run(int64_t Nf, int Cn, int Ck, int F, const float* rows, const float* filte
     for (int k0 = 0; k0 < Ck; k0 += MAX_CK) {
         const int chunk = Ck - k0 < MAX_CK ? Ck - k0 : MAX_CK;
         // a plan of its own for every chunk: the last one may be short
-        const Plan pl = plan(Cn, chunk, F, precision);
+        const Plan pl = plan(Cn, chunk, F, precision, ceil_div(Nf, TILE_M) > sm_count());
         const int kst = pl.kst;
         const int nb = pl.pair ? 2 : 1, sms = sm_count() / nb;        // CTAs, and those that work on items of their own
         const int64_t ntiles = ceil_div(Nf, nb * TILE_M);

@@ -52,7 +52,7 @@ def test_one_sample_backward(nf, cin, cout, F, precision, gate):
 
 @pytest.mark.parametrize("nf", [1, 127, 128, 129, 255, 256, 257, 511, 40001])
 @pytest.mark.parametrize("cin,cout,F", [(100, 20, 4), (128, 48, 9), (100, 128, 16), (260, 36, 25), (64, 64, 16), (512, 12, 9),
-                                          (192, 48, 25), (256, 40, 9), (252, 132, 4)])
+                                          (192, 48, 25), (256, 40, 9), (252, 132, 4), (160, 36, 16), (220, 20, 9)])
 @pytest.mark.parametrize("precision,gate", [(_lib.PREC_FP32, 2e-5), (_lib.PREC_BF16, 2e-2)])
 def test_one_sample_forward(nf, cin, cout, F, precision, gate):
     """Around the 128 rows of a tile and the 256 of a pair of CTAs (from 97 contracted channels on), contracted channels that fill no
