@@ -167,7 +167,7 @@ int pb200_facet2vertex_forward(int64_t Nf, int64_t NvOut, int C, int r, int K, c
 /* gt[f,co] = sum_{j<3, vo_j>=0} gradOutput[vo_j,co] / nfCount[vo_j];
  * gradInput[f,c] = sum_m gt[f,co]*w[f,co];  gradFilter[k,c,m] = sum_f coeff[f,k]*input[f,c]*gt[f,co]
  * Replaces facet2vertexConv3dGradLauncher (mesh_conv3d_gpu.cu:338-426,434-458; binding
- * mesh_conv3d.cpp:75-122).  vtMap may be NULL (identity). */
+ * mesh_conv3d.cpp:75-122).  vtMap may be NULL (identity).  Corners whose vertex or output vertex is out of range are skipped. */
 size_t pb200_facet2vertex_backward_workspace_bytes(int64_t Nf, int C, int r, int K);
 int pb200_facet2vertex_backward(int64_t Nf, int64_t NvIn, int64_t NvOut, int C, int r, int K,
                                 const float* gradOutput, const float* input, const float* filter,

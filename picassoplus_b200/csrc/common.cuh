@@ -39,6 +39,8 @@ int sm_count();           // SMs of the current device (cached per device)
     do { cudaError_t _e = (call); if (_e != cudaSuccess) return pb::cuda_fail(_e, #call); } while (0)
 
 static inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
+// n as the bound of 32-bit indices: (uint32_t)index < index_range(n) also refuses negative ones
+static inline uint32_t index_range(int64_t n) { return n < (1LL << 31) ? (uint32_t)n : 1u << 31; }
 static inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 static inline int pow2_ceil(int x) { int p = 1; while (p < x) p <<= 1; return p; }
 

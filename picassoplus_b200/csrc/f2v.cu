@@ -199,6 +199,20 @@ __global__ void f2v_fwd_generic_kernel(int64_t NvOut, int C, int r, int K, const
     }
 }
 
+// What the backward kernels know of the index arrays: a corner whose vertex, or its output vertex, is outside its range has none and
+// nothing is read for it, as in the adjacency.  (With deferred validation they run on indices that nobody has looked at yet.)
+struct OutVertex {
+    const int32_t* vtMap;                // null: the same vertex
+    uint32_t NvIn, NvOut;
+    __device__ __forceinline__ int mapped(int vi) const {      // not yet looked at: whoever waits for it does (one of the next hops)
+        if ((uint32_t)vi >= NvIn) return -1;
+        return vtMap ? __ldg(vtMap + vi) : vi;
+    }
+    __device__ __forceinline__ int within(int vo) const { return (uint32_t)vo < NvOut ? vo : -1; }
+    __device__ __forceinline__ int operator()(int vi) const { return within(mapped(vi)); }
+};
+
+
 // ------------------------------------------------------------------- backward, vectorised
 // r == 1, C % 4 == 0, any K <= 64.  A block walks tiles of 32 faces; per tile
 //   phase 1  item = (face, float4 channel group): gt = sum over the three corners of
@@ -213,7 +227,7 @@ constexpr int F2VB_TF = 32;
 
 template <int NACC>
 __global__ void __launch_bounds__(256)
-f2v_bwd_tile_kernel(int64_t Nf, int CV, int K, const int32_t* __restrict__ face, const int32_t* __restrict__ vtMap,
+f2v_bwd_tile_kernel(int64_t Nf, int CV, int K, const int32_t* __restrict__ face, OutVertex out_vertex,
                     const int32_t* __restrict__ nfCount, const float* __restrict__ coeff,
                     const float4* __restrict__ in, const float4* __restrict__ filt, const float4* __restrict__ gout,
                     float4* __restrict__ gin, float4* __restrict__ partial) {
@@ -256,8 +270,7 @@ f2v_bwd_tile_kernel(int64_t Nf, int CV, int K, const int32_t* __restrict__ face,
             float4 gt = zero4();
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
-                int vi = __ldg(face + 3 * f + j);
-                int vo = vtMap ? __ldg(vtMap + vi) : vi;
+                const int vo = out_vertex(__ldg(face + 3 * f + j));
                 if (vo >= 0) {
                     float rn = __frcp_rn((float)__ldg(nfCount + vo));
                     fma4s(gt, rn, ldg4(gout + (int64_t)vo * CV + cg));
@@ -338,7 +351,7 @@ template <int P, int LPF> struct F2VLStage {
 
 template <int P, int LPF>
 __global__ void __launch_bounds__(32 * F2VL_WARPS, F2VL_BLOCKS<P>)
-f2v_bwd_lane_kernel(int64_t Nf, int C, int K, int width, const int32_t* __restrict__ face, const int32_t* __restrict__ vtMap,
+f2v_bwd_lane_kernel(int64_t Nf, int C, int K, int width, const int32_t* __restrict__ face, OutVertex out_vertex,
                     const int32_t* __restrict__ nfCount, const float* __restrict__ coeff, const float* __restrict__ in,
                     const float* __restrict__ filt, const float* __restrict__ gout, float* __restrict__ gin,
                     float* __restrict__ partial) {
@@ -386,7 +399,7 @@ f2v_bwd_lane_kernel(int64_t Nf, int C, int K, int width, const int32_t* __restri
         const int64_t at = tile * NE + e;
         return (e < NE && at < Nf * 3) ? __ldg(face + at) : -1;
     };
-    auto hop_vo = [&](int vi) -> int { return vi < 0 ? -1 : (vtMap ? __ldg(vtMap + vi) : vi); };
+    auto hop_vo = [&](int vi) -> int { return out_vertex(vi); };
     auto hop_n = [&](int vo) -> int { return vo < 0 ? 0 : __ldg(nfCount + vo); };
     auto park = [&](Stage& s, int i, int vo, int n) {
         const int e = lane + 32 * i;
@@ -482,8 +495,9 @@ f2v_bwd_lane_kernel(int64_t Nf, int C, int K, int width, const int32_t* __restri
 #pragma unroll
         for (int i = 0; i < NI; ++i) {
             park(ring[next], i, vo0[i], n0[i]);
+            vo1[i] = out_vertex.within(vo1[i]);
             n_next[i] = hop_n(vo1[i]);
-            vo_next[i] = hop_vo(vi2[i]);
+            vo_next[i] = out_vertex.mapped(vi2[i]);
             vi_next[i] = hop_face(tile + (D + 2) * tstep, i);
         }
         cp_async_wait<D - 2>();                                // this tile's copies have landed (own ones) ...
@@ -565,20 +579,19 @@ f2v_bwd_lane_kernel(int64_t Nf, int C, int K, int width, const int32_t* __restri
 }
 
 // ---------------------------------------------------------------------- backward, generic
-__device__ __forceinline__ float f2v_gt(const int32_t* __restrict__ face, const int32_t* __restrict__ vtMap,
+__device__ __forceinline__ float f2v_gt(const int32_t* __restrict__ face, const OutVertex& out_vertex,
                                         const int32_t* __restrict__ nfCount, const float* __restrict__ gout,
                                         int64_t f, int Cr, int co) {
     float gt = 0.f;
     for (int j = 0; j < 3; ++j) {
-        int vi = face[3 * f + j];
-        int vo = vtMap ? vtMap[vi] : vi;
+        const int vo = out_vertex(face[3 * f + j]);
         if (vo >= 0) gt += __ldg(gout + (int64_t)vo * Cr + co) / (float)nfCount[vo];
     }
     return gt;
 }
 
 __global__ void f2v_bwd_input_generic_kernel(int64_t Nf, int C, int r, int K, const int32_t* __restrict__ face,
-                                             const int32_t* __restrict__ vtMap, const int32_t* __restrict__ nfCount,
+                                             OutVertex out_vertex, const int32_t* __restrict__ nfCount,
                                              const float* __restrict__ coeff, const float* __restrict__ filt,
                                              const float* __restrict__ gout, float* __restrict__ gin) {
     const int Cr = C * r;
@@ -592,7 +605,7 @@ __global__ void f2v_bwd_input_generic_kernel(int64_t Nf, int C, int r, int K, co
             int co = c * r + m;
             float w = 0.f;
             for (int k = 0; k < K; ++k) w = fmaf(__ldg(coeff + f * K + k), __ldg(filt + k * Cr + co), w);
-            acc = fmaf(f2v_gt(face, vtMap, nfCount, gout, f, Cr, co), w, acc);
+            acc = fmaf(f2v_gt(face, out_vertex, nfCount, gout, f, Cr, co), w, acc);
         }
         gin[i] = acc;
     }
@@ -600,7 +613,7 @@ __global__ void f2v_bwd_input_generic_kernel(int64_t Nf, int C, int r, int K, co
 
 // thread = output channel co, blockIdx.x = chunk of faces (walked in order), blockIdx.z = k
 __global__ void f2v_bwd_filter_generic_kernel(int64_t Nf, int C, int r, int K, int64_t faces_per_chunk,
-                                              const int32_t* __restrict__ face, const int32_t* __restrict__ vtMap,
+                                              const int32_t* __restrict__ face, OutVertex out_vertex,
                                               const int32_t* __restrict__ nfCount, const float* __restrict__ coeff,
                                               const float* __restrict__ in, const float* __restrict__ gout,
                                               float* __restrict__ partial) {
@@ -613,7 +626,7 @@ __global__ void f2v_bwd_filter_generic_kernel(int64_t Nf, int C, int r, int K, i
     int64_t f1 = f0 + faces_per_chunk < Nf ? f0 + faces_per_chunk : Nf;
     float acc = 0.f;
     for (int64_t f = f0; f < f1; ++f) {
-        float gt = f2v_gt(face, vtMap, nfCount, gout, f, Cr, co);
+        float gt = f2v_gt(face, out_vertex, nfCount, gout, f, Cr, co);
         acc = fmaf(__ldg(coeff + f * K + k) * __ldg(in + f * C + c), gt, acc);
     }
     partial[((int64_t)blockIdx.x * K + k) * Cr + co] = acc;
@@ -748,6 +761,7 @@ int pb200_facet2vertex_backward(int64_t Nf, int64_t NvIn, int64_t NvOut, int C, 
                "facet2vertex_backward: null pointer");
     PB_REQUIRE(workspace && workspace_bytes >= pb200_facet2vertex_backward_workspace_bytes(Nf, C, r, K),
                PB200_EWORKSPACE, "facet2vertex_backward: workspace too small");
+    const OutVertex out_vertex{vtMap, index_range(vtMap ? NvIn : NvOut), index_range(NvOut)};
     F2VBwdPlan p = f2v_bwd_plan(Nf, C, r, K);
     float* partial = (float*)workspace;
     bool vec = p.vec && aligned16(gradOutput) && aligned16(input) && aligned16(filter) && aligned16(gradInput);
@@ -765,7 +779,7 @@ int pb200_facet2vertex_backward(int64_t Nf, int64_t NvIn, int64_t NvOut, int C, 
                 if (gx > p.grid_x) gx = p.grid_x;
                 PB_CUDA(cudaFuncSetAttribute(f2v_bwd_lane_kernel<P, LPF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemb));
                 PB_LAUNCH("f2v_bwd", (f2v_bwd_lane_kernel<P, LPF>), dim3((unsigned)gx, chunks), 32 * F2VL_WARPS, smemb, stream, Nf, C, K, width,
-                          face, vtMap, nfCount, coeff, input, filter, gradOutput, gradInput, partial);
+                          face, out_vertex, nfCount, coeff, input, filter, gradOutput, gradInput, partial);
                 return reduce_partials(partial, (int)gx, (int64_t)K * Cr, gradFilter, stream, FEW_PARTIALS);
             };
             auto width = [&](auto pairs) {
@@ -787,7 +801,7 @@ int pb200_facet2vertex_backward(int64_t Nf, int64_t NvIn, int64_t NvOut, int C, 
         const int cvc = CV < 32 ? CV : 32;
         const int nacc = (int)ceil_div((int64_t)K * cvc, 256);
 #define PB_F2VB_LAUNCH(N)                                                                                        \
-        PB_LAUNCH("f2v_bwd", f2v_bwd_tile_kernel<N>, grid, 256, smem, stream, Nf, CV, K, face, vtMap, nfCount,   \
+        PB_LAUNCH("f2v_bwd", f2v_bwd_tile_kernel<N>, grid, 256, smem, stream, Nf, CV, K, face, out_vertex, nfCount,   \
                   coeff, (const float4*)input, (const float4*)filter, (const float4*)gradOutput,                \
                   (float4*)gradInput, (float4*)partial)
         if (smem > 48 * 1024) {
@@ -808,12 +822,12 @@ int pb200_facet2vertex_backward(int64_t Nf, int64_t NvIn, int64_t NvOut, int C, 
         q.grid_x = (int)ceil_div(Nf, q.faces_per_chunk);
     }
     int gi = persistent_blocks(Nf * C, 256, 16);
-    PB_LAUNCH("f2v_bwd_input_generic", f2v_bwd_input_generic_kernel, gi, 256, 0, stream, Nf, C, r, K, face, vtMap,
+    PB_LAUNCH("f2v_bwd_input_generic", f2v_bwd_input_generic_kernel, gi, 256, 0, stream, Nf, C, r, K, face, out_vertex,
               nfCount, coeff, filter, gradOutput, gradInput);
     PB_REQUIRE(K <= 65535, PB200_EINVAL, "facet2vertex_backward: K too large");
     dim3 gridf(q.grid_x, (unsigned)ceil_div(Cr, 128), K);
     PB_LAUNCH("f2v_bwd_filter_generic", f2v_bwd_filter_generic_kernel, gridf, 128, 0, stream, Nf, C, r, K,
-              q.faces_per_chunk, face, vtMap, nfCount, coeff, input, gradOutput, partial);
+              q.faces_per_chunk, face, out_vertex, nfCount, coeff, input, gradOutput, partial);
     return reduce_partials(partial, q.grid_x, (int64_t)K * Cr, gradFilter, stream);
 }
 

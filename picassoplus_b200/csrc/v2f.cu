@@ -205,7 +205,7 @@ __global__ void v2f_bwd_input_generic_kernel(int64_t Nv, int C, int r, const int
 }
 
 // thread = output channel co, block row = a contiguous chunk of faces walked in order
-__global__ void v2f_bwd_filter_generic_kernel(int64_t Nf, int C, int r, int64_t faces_per_chunk,
+__global__ void v2f_bwd_filter_generic_kernel(int64_t Nf, uint32_t Nv, int C, int r, int64_t faces_per_chunk,
                                               const int32_t* __restrict__ face, const float* __restrict__ in,
                                               const float* __restrict__ gout, float* __restrict__ partial) {
     const int Cr = C * r;
@@ -217,9 +217,10 @@ __global__ void v2f_bwd_filter_generic_kernel(int64_t Nf, int C, int r, int64_t 
     float a0 = 0.f, a1 = 0.f, a2 = 0.f;
     for (int64_t f = f0; f < f1; ++f) {
         float g = __ldg(gout + f * Cr + co);
-        a0 = fmaf(g, __ldg(in + (int64_t)face[3 * f] * C + c), a0);
-        a1 = fmaf(g, __ldg(in + (int64_t)face[3 * f + 1] * C + c), a1);
-        a2 = fmaf(g, __ldg(in + (int64_t)face[3 * f + 2] * C + c), a2);
+        const int v0 = face[3 * f], v1 = face[3 * f + 1], v2 = face[3 * f + 2];
+        if ((uint32_t)v0 < Nv) a0 = fmaf(g, __ldg(in + (int64_t)v0 * C + c), a0);
+        if ((uint32_t)v1 < Nv) a1 = fmaf(g, __ldg(in + (int64_t)v1 * C + c), a1);
+        if ((uint32_t)v2 < Nv) a2 = fmaf(g, __ldg(in + (int64_t)v2 * C + c), a2);
     }
     float* p = partial + (int64_t)blockIdx.x * 3 * Cr;
     p[co] = a0; p[Cr + co] = a1; p[2 * Cr + co] = a2;
@@ -259,7 +260,7 @@ int pb200_vertex2facet_forward(int64_t Nf, int64_t Nv, int C, int r, const float
     PB_REQUIRE(Nf >= 0 && Nv >= 0 && C > 0 && r > 0, PB200_EINVAL, "vertex2facet_forward: bad sizes");
     if (Nf == 0) return PB200_OK;
     PB_REQUIRE(input && filter && face && output, PB200_EINVAL, "vertex2facet_forward: null pointer");
-    const uint32_t vertices = Nv < (1LL << 31) ? (uint32_t)Nv : 1u << 31;         // indices are 32-bit
+    const uint32_t vertices = index_range(Nv);
     if (vec_ok(C, r) && aligned16(input) && aligned16(filter) && aligned16(output)) {
         int CV = C / 4;
         TeamGeom g = team_geom(CV);
@@ -324,7 +325,7 @@ int pb200_vertex2facet_backward(int64_t Nf, int64_t Nv, int C, int r, const floa
     PB_LAUNCH("v2f_bwd_input_generic", v2f_bwd_input_generic_kernel, gi, 256, 0, stream, Nv, C, r, rowptr, entries,
               gradOutput, filter, gradInput);
     dim3 gridf(q.grid_x, (unsigned)ceil_div(Cr, 128));
-    PB_LAUNCH("v2f_bwd_filter_generic", v2f_bwd_filter_generic_kernel, gridf, 128, 0, stream, Nf, C, r,
+    PB_LAUNCH("v2f_bwd_filter_generic", v2f_bwd_filter_generic_kernel, gridf, 128, 0, stream, Nf, index_range(Nv), C, r,
               q.faces_per_chunk, face, input, gradOutput, partial);
     return reduce_partials(partial, q.grid_x, 3 * Cr, gradFilter, stream);
 }
