@@ -30,7 +30,21 @@ NVCC_FLAGS = [
 
 # Per-file flags.  The decimation kernels round every float operation on its own (no fused
 # multiply-add) so that their edge costs, and with them the clustering, are reproducible by plain C.
-FILE_FLAGS = {"decimate.cu": ["--fmad=false"]}
+FILE_FLAGS = {"decimate.cu": ["--fmad=false"], "f2f_tc_one.cu": ["-Xptxas", "-v"]}
+# Registers per thread that kernels have to be built with: f2f_tc_one.cu deals out what its blocks are launched with, and its
+# calls refuse a kernel that was built with fewer.
+REGISTERS = {"f2f_tc_one.cu": ("f2f_one_sample_tc_kernel", 96)}
+
+
+def wrong_registers(ptxas: str, kernel: str, count: int):
+    """Lines of the assembler's report that give a kernel of this name another number of registers."""
+    wrong, name = [], ""
+    for line in ptxas.splitlines():
+        if "Compiling entry function" in line:
+            name = line
+        elif "Used " in line and kernel in name and f"Used {count} registers" not in line:
+            wrong.append(name + line)
+    return wrong
 
 
 def _nvcc() -> str:
@@ -93,6 +107,11 @@ def build(force: bool = False, verbose: bool = False) -> str:
         with ThreadPoolExecutor(max_workers=min(8, len(jobs))) as ex:
             for cmd, r in ex.map(run, jobs):
                 check(cmd, r)
+                src = os.path.basename(cmd[-3])
+                if src in REGISTERS and wrong_registers(r.stdout + r.stderr, *REGISTERS[src]):
+                    os.remove(cmd[-1])
+                    raise RuntimeError(f"{src}: {REGISTERS[src][0]} is not built with {REGISTERS[src][1]} registers:\n" +
+                                       "\n".join(wrong_registers(r.stdout + r.stderr, *REGISTERS[src])))
     if jobs or not os.path.exists(LIB):
         cmd = [nvcc, "-shared", "-o", LIB] + objs + ["-cudart", "static",
                "-gencode", "arch=compute_100a,code=sm_100a"]

@@ -556,7 +556,7 @@ static int map_rows(CUtensorMap* map, const float* rows, int64_t Nf, int channel
 template <int NSPLIT, int F, bool PAIR>
 static int launch(const char* label, const Params& p, const CUtensorMap& map, int grid, size_t smem, cudaStream_t stream) {
     PB_CUDA(cudaFuncSetAttribute(f2f_one_sample_tc_kernel<NSPLIT, F, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    static const int regs = [] {                                  // a kernel built with fewer would wait for registers that are not there
+    static const int regs = [] {                                  // built with fewer it would wait for registers that are not there (build.py refuses to)
         cudaFuncAttributes a;
         return cudaFuncGetAttributes(&a, f2f_one_sample_tc_kernel<NSPLIT, F, PAIR>) == cudaSuccess ? a.numRegs : 0;
     }();

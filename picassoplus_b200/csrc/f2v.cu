@@ -64,8 +64,9 @@ f2v_fwd_face_kernel(int64_t Nf, int CV, int K, const float* __restrict__ coeff, 
 // passes of the warp.  The coefficient rows of the next tile arrive by 4-byte asynchronous copies while this one is
 // computed.  (The kernel above took 389 us for 1 758 000 faces of 64 channels, K = 16, bound by its shared-memory reads; this one takes
 // 183.  Measured and left: packed multiply-adds with the coefficients paired in registers, 202, or stored in pairs, 224.)
-__device__ __forceinline__ void cp_async4(void* dst_smem, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src)
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void* dst_smem, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src), "n"(BYTES)
                  : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
@@ -103,7 +104,7 @@ f2v_fwd_face_blocked_kernel(int64_t Nf, int CV, int K, const float* __restrict__
             const int nf_tile = Nf - f0 < TF ? (int)(Nf - f0) : TF;
             const float* src = coeff + f0 * K + lane;
             float* sc = scoef0 + buf * TF * CP + lane;
-            for (int fl = warp; fl < nf_tile; fl += 8) cp_async4(sc + fl * CP, src + fl * K);
+            for (int fl = warp; fl < nf_tile; fl += 8) cp_async<4>(sc + fl * CP, src + fl * K);
         }
         cp_async_commit();
     };
@@ -320,11 +321,6 @@ f2v_bwd_tile_kernel(int64_t Nf, int CV, int K, const int32_t* __restrict__ face,
 // that read filter, coefficients and products from shared memory for every step (register blocks of 4 faces, three block barriers per
 // tile) took, per call with a cold L2: 879 000 faces, 64 channels, K = 16 247 us (now 148, copy floor 98); 464 000 faces, 128 channels,
 // K = 25 308 (248, floor 101); 879 000 faces, 48 channels, K = 9 226 (136), 32 channels, K = 25 200 (136), 16 channels, K = 16 118 (60).
-template <int BYTES>
-__device__ __forceinline__ void cp_async(void* dst_smem, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src), "n"(BYTES)
-                 : "memory");
-}
 template <int BYTES>
 __device__ __forceinline__ void cp_async(void* dst_smem, const void* src, bool on) {      // off: zeros
     asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src),

@@ -133,7 +133,7 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 }
 
 // Registers per thread of the calling warpgroup (four warps, all of which call it): a share of what the block was launched
-// with.  `give` waits until others have let go of enough, so the shares of a block must add up to its launch's registers.
+// with.  `registers_take` waits until others have let go of enough, so the shares of a block must add up to its launch's registers.
 template <int N>
 __device__ __forceinline__ void registers_keep() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N>

@@ -37,3 +37,15 @@ def test_host_side_argument_checks():
     assert _lib.query("pb200_vertex_csr_workspace_bytes", 1000, 600) > 4 * 3000
     assert _lib.query("pb200_facet2facet_backward_workspace_bytes", 1000, 2500, 32, 64, 16, 0) > 0
     assert _lib.launch_count() == 0                # nothing was launched by the checks above
+
+
+def test_build_refuses_other_register_counts():
+    """The report of the assembler on the kernels that deal out their registers is read for every one of them."""
+    from picassoplus_b200 import build
+    report = """ptxas info    : Compiling entry function '_ZN2pb3one24f2f_one_sample_tc_kernelILi2ELi9ELb1EEEv' for 'sm_100a'
+ptxas info    : Used {} registers, used 1 barriers
+ptxas info    : Compiling entry function '_ZN2pb3one5otherEv' for 'sm_100a'
+ptxas info    : Used 40 registers"""
+    name, count = build.REGISTERS["f2f_tc_one.cu"]
+    assert not build.wrong_registers(report.format(count), name, count)
+    assert len(build.wrong_registers(report.format(88), name, count)) == 1
