@@ -602,7 +602,10 @@ bool has_room(size_t bytes) {
     if (reserved - stats.active_bytes[ALL].current >= need) return true;
     size_t free = 0, total = 0;
     c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
-    if (cudaMemGetInfo(&free, &total) != cudaSuccess) return false;
+    if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
     const double allowed = c10::cuda::CUDACachingAllocator::getMemoryFraction(call_device) * (double)total - (double)reserved;
     return (double)free >= 4. * (double)need && allowed >= 4. * (double)need;
 }

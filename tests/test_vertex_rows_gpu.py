@@ -180,3 +180,22 @@ def test_inference_takes_no_room_that_is_not_there():
         finally:
             torch.cuda.set_per_process_memory_fraction(1.0)
         assert figures() == counts
+
+
+def test_inference_over_many_rows_is_captured():
+    """The question for room and the rows themselves inside a graph capture: the replay has the results of the plain call."""
+    from picassoplus_b200.mesh.layers import V2FConv3d
+    g = torch.Generator(device="cuda").manual_seed(1)
+    rows, nv, C = 200000, 20000, 64
+    layer, x = V2FConv3d(C, 128, 2).cuda().eval(), torch.randn(nv, C, device="cuda", generator=g)
+    face = torch.randint(nv, (rows, 3), device="cuda", generator=g).int()
+    with torch.no_grad():
+        want = layer(x, face)
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()                    # nothing at hand: the device is asked
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = layer(x, face)
+        out.zero_()
+        graph.replay()
+        assert torch.equal(out, want)
